@@ -289,6 +289,77 @@ int jb200_lsf_step_norm(const void* m_bf16, const double* stats, const double* p
                         const float* var_scale, float alpha_min, float alpha_max, const float* h_in, float* h_out,
                         float* x, const float* w_norm, float eps, void* xn_bf16, int B, int C, void* stream);
 
+/* ---- whole layers in one call --------------------------------------------------------------- */
+
+/* Device pointers and scalars of one block (JarvisBlock, jarvis_engine/jarvis_model.py:399-441): the f32 parameters, the
+ * prepared packed weights (jb200_prepare_weights) and their scales.  gamma = sigmoid(gamma_raw). */
+typedef struct jb200_layer {
+  const float* w_norm1;          /* [C] */
+  const float* w_norm2;          /* [C] */
+  const float* w_router;         /* [E][C] */
+  const float* gamma;            /* [H] */
+  const float* var_scale;        /* [1] */
+  const uint8_t* w_qkv;          /* [3C][C/4], scales a_qkv [3] */
+  const float* a_qkv;
+  const uint8_t* w_out;          /* [C][C/4], [1] */
+  const float* a_out;
+  const uint8_t* w1;             /* [E][hidden][C/4], [E] */
+  const float* a1;
+  const uint8_t* w2;             /* [E][C][hidden/4], [E] */
+  const float* a2;
+  const float* mu;               /* [1] ReflectivePenalty.mu_t (jarvis_model.py:329-351), or NULL: no penalty wanted */
+  float eps1, eps2, alpha_min, alpha_max, balance_alpha;
+  float reflect_lam, reflect_tau;
+} jb200_layer;
+
+/* One call of jb200_forward_layers.  Pointer arrays live on the HOST and hold one device pointer per layer; an array
+ * or an entry may be NULL (no state in / not wanted out).  s_out[l] may be s_in[l], h_out[l] may be h_in[l]. */
+typedef struct jb200_forward {
+  int B, T, C, H, E, hidden;     /* top-2 experts; C % 128 == 0, C <= 1024, C == 64 H */
+  const int64_t* ids;            /* [B*T] token ids, or NULL: x already holds the residual stream */
+  const float* table;            /* [vocab][C] embedding (with ids) */
+  int vocab;
+  float* x;                      /* f32 [B*T][C] residual stream, updated in place */
+  const float* cos_tab;          /* f32 [n_pos][32] */
+  const float* sin_tab;
+  int n_pos;
+  const int32_t* pos0;           /* [B] or NULL (pos0_scalar), as jb200_attn_scan */
+  int pos0_scalar;
+  const float* const* s_in;      /* f32 [B][H][64][64] */
+  float* const* s_out;
+  const float* const* h_in;      /* f32 [B][C] */
+  float* const* h_out;           /* required */
+  double* acc;                   /* f64 [n_layers][2 + E], i32 [n_layers][E]: zeroed by the call, then the sums of */
+  int32_t* hist;                 /*   jb200_moe_scatter_combine / jb200_router_top2 */
+  float* scalars;                /* f32 [n_layers][3]: l_balance, act_mean, act_var of every layer */
+  float* reflect;                /* f32 [n_layers]: lam * ((mu - act_mean)^2 + relu(act_var - tau)); or NULL */
+  void* routing;                 /* n_layers blocks of jb200_routing_layout bytes: the routing results of every layer */
+  const float* w_final;          /* [C] or NULL: RMSNorm after the last layer -> hidden_out bf16 [B*T][C] */
+  float eps_final;
+  void* hidden_out;
+  void* workspace;               /* jb200_forward_workspace_bytes, 256-byte aligned */
+} jb200_forward;
+
+/* Bytes of one layer's routing block; offsets[7] (may be NULL) receives the byte offsets of topk_idx (i64 [N][2]), gates
+ * (f32 [N][2]), expert_counts, expert_offsets, scatter_map, gather_map, gate_idx_map (see jb200_moe_metadata). */
+size_t jb200_routing_layout(int N, int E, size_t* offsets);
+size_t jb200_forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden);
+
+/* The blocks of the model, one after another (Jarvis.forward's loop, jarvis_engine/jarvis_model.py:498-516): embedding,
+ * then per layer norm1, q|k|v, attention scan or step, output projection + residual, norm2 + router, dispatch, the
+ * two expert matrices, combine, LSF + residual, and the final norm.  Enqueues the kernels of the single-stage entry
+ * points with their results; one call instead of ~14 per layer keeps the host (about 15 us per call from Python) out
+ * of the way of short forwards. */
+int jb200_forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, void* stream);
+
+/* Training / evaluation loss from bf16 logits (jarvis_engine/jarvis_model.py:536-545): cross entropy averaged over the
+ * rows whose target is not -100, plus the sums of n_aux entries of aux_a (stride stride_a) and aux_b (stride 1), e.g.
+ * l_balance and the reflective penalty of every layer.  logits: row stride ld >= V elements, 16-byte aligned rows;
+ * targets: i64 [n_rows] (one outside [0, V) other than -100 makes the loss NaN); row_loss: f32 [n_rows] scratch;
+ * loss: f32 [1]. */
+int jb200_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
+                        const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, void* stream);
+
 /* ---- expert parallelism over peer memory (no counterpart: the reference is single-GPU) ------------------- */
 
 /* Device buffers that other processes on the node can map (CUDA IPC).  alloc: cudaMalloc on the current device and

@@ -23,6 +23,24 @@ _I = C.c_int
 _Z = C.c_size_t
 _F = C.c_float
 
+
+
+class Layer(C.Structure):
+    """jb200_layer"""
+    _fields_ = [(n, _P) for n in ("w_norm1", "w_norm2", "w_router", "gamma", "var_scale", "w_qkv", "a_qkv", "w_out", "a_out",
+                                  "w1", "a1", "w2", "a2", "mu")] + \
+               [(n, _F) for n in ("eps1", "eps2", "alpha_min", "alpha_max", "balance_alpha", "reflect_lam", "reflect_tau")]
+
+
+class Forward(C.Structure):
+    """jb200_forward"""
+    _fields_ = [(n, _I) for n in ("B", "T", "C", "H", "E", "hidden")] + \
+               [("ids", _P), ("table", _P), ("vocab", _I), ("x", _P), ("cos_tab", _P), ("sin_tab", _P), ("n_pos", _I),
+                ("pos0", _P), ("pos0_scalar", _I), ("s_in", _P), ("s_out", _P), ("h_in", _P), ("h_out", _P), ("acc", _P),
+                ("hist", _P), ("scalars", _P), ("reflect", _P), ("routing", _P), ("w_final", _P), ("eps_final", _F), ("hidden_out", _P),
+                ("workspace", _P)]
+
+
 # name -> (restype, argtypes); must list every function declared in include/jarvis_b200.h
 PROTOTYPES = {
     "jb200_last_error": (C.c_char_p, []),
@@ -57,6 +75,10 @@ PROTOTYPES = {
     "jb200_lsf_scan_scratch_bytes": (_Z, [_I, _I, _I]),
     "jb200_lsf_step_norm": (_I, [_P, _P, _P, _P, _I, C.c_longlong, C.c_longlong, _F, _P, _P, _F, _F, _P, _P, _P, _P, _F, _P,
                                  _I, _I, _P]),
+    "jb200_cross_entropy": (_I, [_P, _I, _I, _I, _P, _P, _P, _I, _P, _I, _P, _P]),
+    "jb200_routing_layout": (_Z, [_I, _I, C.POINTER(_Z)]),
+    "jb200_forward_workspace_bytes": (_Z, [_I] * 6),
+    "jb200_forward_layers": (_I, [_P, _I, C.POINTER(Forward), _P]),
     "jb200_peer_buffer_alloc": (_I, [_Z, _P, _P]),
     "jb200_peer_buffer_open": (_I, [_P, _P]),
     "jb200_peer_buffer_close": (_I, [_P]),

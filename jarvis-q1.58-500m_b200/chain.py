@@ -1,0 +1,236 @@
+"""Whole layers in one ctypes call (jb200_forward_layers): the descriptor table of a list of blocks and its checks.
+
+A forward is ~14 launches per layer.  Issued through ops.* each costs ~15 us of Python; here the loop over the layers
+runs in C++ and Python pays for one call, a handful of allocations and the check that no parameter has changed.
+"""
+from __future__ import annotations
+
+import ctypes as C
+import operator
+from typing import List, Optional
+
+import torch
+
+from . import _lib, ops
+
+_data_ptr = torch.Tensor.data_ptr
+_version = operator.attrgetter("_version")
+
+
+def supported(blocks) -> bool:
+    """Shapes jb200_forward_layers takes, all parameters on one CUDA device."""
+    a = blocks[0].attn
+    d_model = a.q_proj.weight.shape[1]
+    hidden, E, dev = blocks[0].moe.w1[0].weight.shape[0], blocks[0].moe.num_experts, blocks[0].norm1.weight.device
+    if d_model % 128 or d_model > 1024 or hidden % 128 or E not in (4, 8) or dev.type != "cuda":
+        return False
+    return all(b.attn.n_heads == a.n_heads and b.attn.head_dim == 64 and b.attn.q_proj.weight.shape[1] == d_model and
+               b.moe.num_experts == E and b.moe.top_k == 2 and b.moe.w1[0].weight.shape[0] == hidden and
+               b.attn.rotary.base == a.rotary.base and all(p.device == dev for p in b.parameters()) for b in blocks)
+
+
+class LayerTable:
+    """jb200_layer array of `blocks`, valid as long as every parameter it was built from is the same unmodified tensor in
+    the same place (identity, storage and version are compared on every call: 16 tensors per layer, ~0.1 us each)."""
+
+    def __init__(self, blocks):
+        from .modules import ReflectivePenalty, _f32
+        self.blocks = list(blocks)
+        self.n = len(self.blocks)
+        b0 = self.blocks[0]
+        self.C, self.H, self.E = b0.norm1.weight.numel(), b0.attn.n_heads, b0.moe.num_experts
+        self.hidden = b0.moe.w1[0].weight.shape[0]
+        self.device = b0.norm1.weight.device
+        self.array = (_lib.Layer * self.n)()
+        self._keep = []
+        self._sizes = {}
+        self.has_reflect = all(type(b.reflect) is ReflectivePenalty for b in self.blocks)
+        self._watch(self.blocks)
+        for d, b in zip(self.array, self.blocks):
+            at, moe, lq = b.attn, b.moe, b.liquid
+            qkv, a_qkv = at.qkv_packed()
+            out, a_out = at.out_proj.packed()
+            (w1, a1), (w2, a2) = moe.packed()
+            gamma = torch.sigmoid(at.gamma_raw.detach().float())
+            tensors = dict(w_norm1=_f32(b.norm1.weight), w_norm2=_f32(b.norm2.weight), w_router=_f32(moe.router.weight),
+                           gamma=gamma, var_scale=_f32(lq.var_scale, scalar=True), w_qkv=qkv, a_qkv=a_qkv, w_out=out,
+                           a_out=a_out, w1=w1, a1=a1, w2=w2, a2=a2)
+            if self.has_reflect:
+                tensors["mu"] = _f32(b.reflect.mu_t, scalar=True)
+                d.reflect_lam, d.reflect_tau = b.reflect.lam, b.reflect.tau_max
+            for name, t in tensors.items():
+                setattr(d, name, t.data_ptr())
+            self._keep.append(tensors)
+            d.eps1, d.eps2, d.balance_alpha = b.norm1.eps, b.norm2.eps, moe.balance_alpha
+            d.alpha_min, d.alpha_max = lq.alpha_min, lq.alpha_max
+
+    def _watch(self, blocks):
+        slots, mods, self._flags, self._consts = [], [], [], []
+        for b in blocks:
+            at, moe = b.attn, b.moe
+            mods += [(b, "norm1"), (b, "norm2"), (b, "attn"), (b, "moe"), (b, "liquid"), (b, "reflect"), (moe, "router"),
+                     (moe, "w1"), (moe, "w2")] + [(at, n) for n in ("q_proj", "k_proj", "v_proj", "out_proj", "rotary")]
+            slots += [(m, "weight") for m in (b.norm1, b.norm2, moe.router, at.q_proj, at.k_proj, at.v_proj, at.out_proj)]
+            slots += [(at, "gamma_raw"), (b.liquid, "var_scale")]
+            for lst in (moe.w1, moe.w2):
+                mods += [(lst, str(i)) for i in range(len(lst))]
+                slots += [(m, "weight") for m in lst]
+            self._flags.append((at.__dict__, moe.__dict__))
+            self._consts.append((b.norm1, b.norm2, moe, b.liquid, b.reflect))
+        self._slots = [(m._parameters, n) for m, n in slots]
+        if self.has_reflect:
+            self._slots += [(b.reflect._buffers, "mu_t") for b in blocks]
+        self._mods = [(m._modules, n) for m, n in mods]
+        self._mod_objs = [d[n] for d, n in self._mods]
+        self._params = [d[n] for d, n in self._slots]
+        self._ptrs = list(map(_data_ptr, self._params))
+        self._versions = list(map(_version, self._params))
+        self._const_vals = self._read_consts()
+
+    def _read_consts(self):
+        return [(a.eps, b.eps, m.balance_alpha, q.alpha_min, q.alpha_max, getattr(r, "lam", None), getattr(r, "tau_max", None))
+                for a, b, m, q, r in self._consts]
+
+    def current(self) -> bool:
+        try:
+            now = [d[n] for d, n in self._slots]
+            return (all(map(operator.is_, now, self._params)) and list(map(_data_ptr, now)) == self._ptrs and
+                    list(map(_version, now)) == self._versions and
+                    all(map(operator.is_, [d[n] for d, n in self._mods], self._mod_objs)) and
+                    self._read_consts() == self._const_vals)
+        except (KeyError, AttributeError):
+            return False
+
+    def local(self) -> bool:
+        """No hook that needs the per-kernel path: statistics or experts shared with other GPUs, fused prologue, training."""
+        for at, moe in self._flags:
+            if moe["stats_group"] is not None or moe["_ep"] is not None or at["fuse_prologue"] or moe["training"]:
+                return False
+        return True
+
+    def sizes(self, B: int, T: int):
+        key = (B, T)
+        got = self._sizes.get(key)
+        if got is None:
+            lib = _lib.load()
+            off = (C.c_size_t * 7)()
+            rb = lib.jb200_routing_layout(B * T, self.E, off)
+            got = (lib.jb200_forward_workspace_bytes(B, T, self.C, self.H, self.E, self.hidden), rb, tuple(off))
+            if len(self._sizes) >= 256:
+                self._sizes.clear()
+            self._sizes[key] = got
+        return got
+
+
+def table_of(owner, blocks) -> Optional[LayerTable]:
+    """The (cached) table of `blocks`, kept on `owner`; None when they need the per-kernel path."""
+    tab = owner.__dict__.get("_layer_table")
+    if tab is None or tab.n != len(blocks) or not all(map(operator.is_, tab.blocks, blocks)) or not tab.current():
+        if not supported(blocks):
+            return None
+        tab = LayerTable(blocks)
+        owner.__dict__["_layer_table"] = tab
+    return tab if tab.local() else None
+
+
+def _f32_list(ts: Optional[List[Optional[torch.Tensor]]]):
+    if ts is None:
+        return None
+    return [t if t is None or (t.dtype is torch.float32 and t.is_contiguous()) else t.float().contiguous() for t in ts]
+
+
+def _pointers(n, ts):
+    return (C.c_void_p * n)(*[None if t is None else t.data_ptr() for t in ts])
+
+
+def _rows_of(n, base, stride):
+    return (C.c_void_p * n)(*range(base, base + n * stride, stride))
+
+
+class Result:
+    """What a call leaves: h / S (lists, one tensor per layer; S None when not wanted), scalars f32 (n, 3), reflect f32 (n,)
+    and hidden (normalised rows after the last layer, bf16)."""
+    __slots__ = ("h", "S", "scalars", "reflect", "hidden")
+
+
+def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0, max_position=None, h_in=None, s_in=None,
+        want_state=False, inplace=False, final_norm=None) -> Result:
+    """One jb200_forward_layers call on the current stream.  x: f32 (B*T, C), updated in place (written from `ids` and the
+    embedding `table` when given).  h_in / s_in: lists with one f32 tensor or None per layer, or None."""
+    n, dev = tab.n, tab.device
+    if not (x.is_cuda and x.dtype is torch.float32 and x.is_contiguous()):
+        raise RuntimeError("forward: expected a contiguous f32 CUDA residual stream (this path has no CPU fallback)")
+    ws_bytes, routing_bytes, _ = tab.sizes(B, T)
+    acc_bytes = n * (2 + tab.E) * 8
+    hist_off = acc_bytes
+    head = (acc_bytes + n * tab.E * 4 + 255) // 256 * 256
+    work = torch.empty(head + ws_bytes, dtype=torch.uint8, device=dev)
+    routing = torch.empty(n * routing_bytes, dtype=torch.uint8, device=dev)
+    res = Result()
+    aux = torch.empty(4 * n, dtype=torch.float32, device=dev)
+    res.scalars, res.reflect = aux[:3 * n].view(n, 3), aux[3 * n:] if tab.has_reflect else None
+    f = _lib.Forward()
+    f.B, f.T, f.C, f.H, f.E, f.hidden = B, T, tab.C, tab.H, tab.E, tab.hidden
+    if ids is not None:
+        f.ids, f.table, f.vocab = ids.data_ptr(), table.data_ptr(), table.shape[0]
+    f.x = x.data_ptr()
+    if torch.is_tensor(start_pos):
+        if not (start_pos.is_cuda and start_pos.dtype is torch.int32 and start_pos.is_contiguous() and start_pos.numel() == B):
+            raise RuntimeError("forward: per-sequence positions must be a contiguous int32 CUDA tensor with one entry per sequence")
+        # without the caller's bound the table is sized from the positions themselves (a host read)
+        end = (max_position if max_position is not None else int(start_pos.max())) + T
+        f.pos0 = start_pos.data_ptr()
+    else:
+        f.pos0_scalar = int(start_pos)
+        end = f.pos0_scalar + T
+    cos, sin = tab.blocks[0].attn.rotary.half_tables(end, dev)
+    f.cos_tab, f.sin_tab, f.n_pos = cos.data_ptr(), sin.data_ptr(), cos.shape[0]
+    h_in, s_in = _f32_list(h_in), _f32_list(s_in)
+    if h_in is not None:
+        h_ptrs = _pointers(n, h_in)
+        f.h_in = C.addressof(h_ptrs)
+    if s_in is not None:
+        s_ptrs = _pointers(n, s_in)
+        f.s_in = C.addressof(s_ptrs)
+    if inplace and h_in is not None and None not in h_in:
+        res.h, ho_ptrs = h_in, h_ptrs
+    else:
+        h_all = torch.empty((n, B, tab.C), dtype=torch.float32, device=dev)
+        res.h, ho_ptrs = list(h_all.unbind(0)), _rows_of(n, h_all.data_ptr(), B * tab.C * 4)
+    f.h_out = C.addressof(ho_ptrs)
+    res.S = None
+    if inplace and s_in is not None and None not in s_in:
+        res.S, so_ptrs = s_in, s_ptrs
+        f.s_out = C.addressof(so_ptrs)
+    elif want_state:
+        s_all = torch.empty((n, B, tab.H, 64, 64), dtype=torch.float32, device=dev)
+        res.S, so_ptrs = list(s_all.unbind(0)), _rows_of(n, s_all.data_ptr(), B * tab.H * 64 * 64 * 4)
+        f.s_out = C.addressof(so_ptrs)
+    base = work.data_ptr()
+    f.acc, f.hist, f.workspace = base, base + hist_off, base + head
+    f.scalars, f.routing = aux.data_ptr(), routing.data_ptr()
+    f.reflect = aux.data_ptr() + 12 * n if tab.has_reflect else None
+    res.hidden = None
+    if final_norm is not None:
+        res.hidden = torch.empty((B * T, tab.C), dtype=torch.bfloat16, device=dev)
+        f.w_final, f.eps_final, f.hidden_out = final_norm[0].data_ptr(), final_norm[1], res.hidden.data_ptr()
+    _lib.check(_lib.load().jb200_forward_layers(tab.array, n, C.byref(f), ops._stream()), "jb200_forward_layers")
+    for i, (_, moe) in enumerate(tab._flags):
+        moe["_routing"] = (routing, i, B * T, tab)      # the views are built when somebody looks at them
+    return res
+
+
+def routing_views(src):
+    """(topk_idx, gates, (counts, offsets, scatter, gather, gate_idx)) of one layer from its block of a call's routing buffer."""
+    buf, layer, N, tab = src
+    nbytes, off = None, (C.c_size_t * 7)()
+    nbytes = _lib.load().jb200_routing_layout(N, tab.E, off)
+
+    def view(i, count, dtype, *shape):
+        size = torch.empty((), dtype=dtype).element_size()
+        at = layer * nbytes + off[i]
+        return buf[at:at + count * size].view(dtype).view(*shape)
+    i32, E = torch.int32, tab.E
+    return (view(0, 2 * N, torch.int64, N, 2), view(1, 2 * N, torch.float32, N, 2),
+            (view(2, E, i32, E), view(3, E + 1, i32, E + 1), view(4, 2 * N, i32, N, 2), view(5, 2 * N, i32, 2 * N),
+             view(6, 2 * N, i32, 2 * N)))

@@ -53,6 +53,83 @@ int cuda_fail(cudaError_t e, const char* what) {
   return JB200_ERR_CUDA;
 }
 
+namespace {
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled_fn() {
+  static std::atomic<EncodeTiledFn> fn{nullptr};
+  EncodeTiledFn f = fn.load(std::memory_order_acquire);
+  if (!f) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess) {
+      f = reinterpret_cast<EncodeTiledFn>(p);
+      fn.store(f, std::memory_order_release);
+    }
+  }
+  return f;
+}
+
+struct MapKey {        // every field is set for every entry (unused dimensions to zero), so keys compare bytewise
+  uint64_t ptr, dims[3], strides[2];
+  uint32_t box[3], dt, rank, swizzle, promotion, pad;
+};
+struct MapEntry {
+  MapKey key;
+  CUtensorMap map;
+};
+constexpr int MAP_CACHE = 64;
+thread_local MapEntry g_maps[MAP_CACHE];   // zero keys match nothing: rank is never 0
+}  // namespace
+
+int encode_tiled(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const void* ptr, const cuuint64_t* dims,
+                 const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle,
+                 CUtensorMapL2promotion promotion, const char* what) {
+  MapKey k;
+  memset(&k, 0, sizeof(k));
+  k.ptr = reinterpret_cast<uint64_t>(ptr);
+  for (int i = 0; i < rank; ++i) { k.dims[i] = dims[i]; k.box[i] = box[i]; }
+  for (int i = 0; i + 1 < rank; ++i) k.strides[i] = strides[i];
+  k.dt = uint32_t(dt); k.rank = uint32_t(rank); k.swizzle = uint32_t(swizzle); k.promotion = uint32_t(promotion);
+  uint64_t h = 1469598103934665603ull;
+  const uint64_t* w = reinterpret_cast<const uint64_t*>(&k);
+  for (size_t i = 0; i < sizeof(k) / 8; ++i) h = (h ^ w[i]) * 1099511628211ull;
+  MapEntry& e = g_maps[(h >> 40) % MAP_CACHE];
+  if (memcmp(&e.key, &k, sizeof(k)) != 0) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) {
+      set_error("%s: cuTensorMapEncodeTiled entry point not available", what);
+      return JB200_ERR_CUDA;
+    }
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult cr = fn(&e.map, dt, cuuint32_t(rank), const_cast<void*>(ptr), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) {
+      memset(&e.key, 0, sizeof(e.key));
+      set_error("%s: cuTensorMapEncodeTiled failed (%d)", what, int(cr));
+      return JB200_ERR_CUDA;
+    }
+    e.key = k;
+  }
+  *tm = e.map;
+  return JB200_OK;
+}
+
+int set_max_smem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
+    set_error("set_max_smem: cudaGetDevice failed");
+    return JB200_ERR_CUDA;
+  }
+  if ((done->load(std::memory_order_acquire) >> dev) & 1ull) return JB200_OK;
+  JB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  done->fetch_or(1ull << dev, std::memory_order_release);
+  return JB200_OK;
+}
+
 unsigned int* device_status_ptr() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
@@ -118,7 +195,7 @@ extern "C" {
 
 const char* jb200_last_error(void) { return g_err; }
 
-int jb200_abi_version(void) { return 11; }
+int jb200_abi_version(void) { return 12; }
 
 long long jb200_kernel_launches(int reset) {
   return reset ? g_launches.exchange(0) : g_launches.load();
@@ -336,8 +413,24 @@ int jb200_lsf_step_norm(const void* m_bf16, const double* stats, const double* p
                         int E, long long n_tokens, long long n_elems, float balance_alpha, float* scalars,
                         const float* var_scale, float alpha_min, float alpha_max, const float* h_in, float* h_out,
                         float* x, const float* w_norm, float eps, void* xn_bf16, int B, int C, void* stream) {
-  return launch_lsf_step_norm(m_bf16, stats, probs_sum, top1_hist, E, n_tokens, n_elems, balance_alpha, scalars,
-                              var_scale, alpha_min, alpha_max, h_in, h_out, x, w_norm, eps, xn_bf16, B, C,
+  const LsfStats st = {stats, probs_sum, top1_hist, E, n_tokens, n_elems, balance_alpha, scalars, nullptr, 0.f, 0.f, nullptr};
+  return launch_lsf_step_norm(m_bf16, st, var_scale, alpha_min, alpha_max, h_in, h_out, x, w_norm, eps, xn_bf16, B, C,
+                              static_cast<cudaStream_t>(stream));
+}
+
+size_t jb200_routing_layout(int N, int E, size_t* offsets) { return routing_layout(N, E, offsets); }
+
+size_t jb200_forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden) {
+  return forward_workspace_bytes(B, T, C, H, E, hidden);
+}
+
+int jb200_forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, void* stream) {
+  return forward_layers(layers, n_layers, f, static_cast<cudaStream_t>(stream));
+}
+
+int jb200_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
+                        const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, void* stream) {
+  return launch_cross_entropy(logits, ld, n_rows, V, targets, row_loss, aux_a, stride_a, aux_b, n_aux, loss,
                               static_cast<cudaStream_t>(stream));
 }
 

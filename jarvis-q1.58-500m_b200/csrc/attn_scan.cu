@@ -1060,34 +1060,12 @@ attn_decode_stream_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
   if (t == 0) bulk_wait_group<0>();
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 int make_map(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld) {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      set_error("attn_scan: cuTensorMapEncodeTiled entry point not available");
-      return JB200_ERR_CUDA;
-    }
-    fn = reinterpret_cast<EncodeTiledFn>(f);
-  }
   const cuuint64_t gdim[2] = {cuuint64_t(cols), cuuint64_t(rows)};
   const cuuint64_t gstride[1] = {cuuint64_t(ld) * 2};
   const cuuint32_t box[2] = {cuuint32_t(D), cuuint32_t(CH)};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult cr = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (cr != CUDA_SUCCESS) {
-    set_error("attn_scan: cuTensorMapEncodeTiled failed (%d)", int(cr));
-    return JB200_ERR_CUDA;
-  }
-  return JB200_OK;
+  return encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, gdim, gstride, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "attn_scan");
 }
 
 }  // namespace
@@ -1162,7 +1140,7 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
       // the state streams through shared memory as bulk copies: two CTAs per SM walk the (sequence, head) pairs
       const int sms = sm_count();
       if (sms <= 0) return JB200_ERR_CUDA;
-      JB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(DEC_SMEM_BYTES)));
+      JB_MAX_SMEM(attn_decode_stream_kernel, DEC_SMEM_BYTES);
       const int grid = B * H < 2 * sms ? B * H : 2 * sms;
       launch_dep(attn_decode_stream_kernel, grid, 256, DEC_SMEM_BYTES, stream, reinterpret_cast<const __nv_bfloat16*>(q),
                  reinterpret_cast<const __nv_bfloat16*>(k), reinterpret_cast<const __nv_bfloat16*>(v), ld_qkv, dp);
@@ -1201,16 +1179,16 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   p.n_split = 0; p.split_chunk = 0; p.handoff = nullptr; p.ctrl = nullptr;
   if (!o) {
     // state only: the k/v pass over every piece, then the fold
-    JB_CUDA(cudaFuncSetAttribute(attn_state_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(STATE_SMEM_BYTES)));
+    JB_MAX_SMEM(attn_state_pass_kernel, STATE_SMEM_BYTES);
     launch_dep(attn_state_pass_kernel, dim3(H, B, p.nseg), STATE_THREADS, STATE_SMEM_BYTES, stream, tk, tv, p);
     JB_LAUNCH_CHECK("attn_state_pass_kernel");
     launch_dep(attn_fold_states_kernel, dim3(H, B), 256, 0, stream, p);
     JB_LAUNCH_CHECK("attn_fold_states_kernel");
     return JB200_OK;
   }
-  JB_CUDA(cudaFuncSetAttribute(attn_scan_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(PIPE_SMEM_BYTES)));
+  JB_MAX_SMEM(attn_scan_pipe_kernel, PIPE_SMEM_BYTES);
   if (p.nseg > 1) {
-    JB_CUDA(cudaFuncSetAttribute(attn_state_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(STATE_SMEM_BYTES)));
+    JB_MAX_SMEM(attn_state_pass_kernel, STATE_SMEM_BYTES);
     launch_dep(attn_state_pass_kernel, dim3(H, B, p.nseg - 1), STATE_THREADS, STATE_SMEM_BYTES, stream, tk, tv, p);
     JB_LAUNCH_CHECK("attn_state_pass_kernel");
   }

@@ -1,0 +1,156 @@
+// Whole layers in one host call: the launch sequence of JarvisBlock.forward (jarvis_engine/jarvis_model.py:428-441) and
+// of the model's loop around it (:498-516), issued from C++ over one caller-owned workspace.  A forward is a few
+// hundred launches; issued one by one from Python they cost ~15 us each (5 ms for 24 layers), more than the GPU
+// needs for anything below a few thousand tokens, issued here ~2 us each.
+#include "common.cuh"
+#include "launchers.h"
+
+namespace jb {
+
+namespace {
+
+inline size_t up(size_t n, size_t a) { return (n + a - 1) / a * a; }
+
+struct Routing {
+  size_t idx, gates, counts, offsets, scatter, gather, gate_idx, bytes;
+  Routing(int N, int E) {
+    size_t o = 0;
+    auto take = [&](size_t n) { const size_t at = o; o += up(n, 16); return at; };
+    idx = take(size_t(N) * 2 * 8);
+    gates = take(size_t(N) * 2 * 4);
+    counts = take(size_t(E) * 4);
+    offsets = take(size_t(E + 1) * 4);
+    scatter = take(size_t(N) * 2 * 4);
+    gather = take(size_t(N) * 2 * 4);
+    gate_idx = take(size_t(N) * 2 * 4);
+    bytes = o;
+  }
+};
+
+// Buffers of one layer, reused by the next: a kernel only ever overlaps its immediate predecessor, and nothing below
+// writes what its predecessor still reads.
+struct Workspace {
+  size_t xn, qkv, o, hid, y, out, attn, lsf, meta, bytes;
+  Workspace(int B, int T, int C, int H, int E, int hidden) {
+    const size_t N = size_t(B) * T;
+    size_t p = 0;
+    auto take = [&](size_t n) { const size_t at = p; p += up(n, 256); return at; };
+    xn = take(N * C * 2);
+    qkv = take(N * 3 * C * 2);          // later the dispatched rows [2N][C]
+    o = take(N * C * 2);                // later the MoE output
+    hid = take(N * 2 * hidden * 2);
+    y = take(N * 2 * C * 2);
+    out = o;
+    attn = take(T > 1 ? attn_scan_scratch_bytes(B, T, H) : 0);
+    lsf = take(T > 1 ? lsf_scan_scratch_bytes(B, T, C) : 0);
+    meta = take(moe_metadata_scratch_bytes(int(N), 2, E));
+    bytes = p;
+  }
+};
+
+#define JB_TRY(call)                    \
+  do {                                  \
+    const int rc__ = (call);            \
+    if (rc__ != JB200_OK) return rc__;  \
+  } while (0)
+
+}  // namespace
+
+size_t routing_layout(int N, int E, size_t* offsets) {
+  const Routing r(N > 0 ? N : 0, E > 0 ? E : 0);
+  if (offsets) {
+    const size_t all[7] = {r.idx, r.gates, r.counts, r.offsets, r.scatter, r.gather, r.gate_idx};
+    for (int i = 0; i < 7; ++i) offsets[i] = all[i];
+  }
+  return r.bytes;
+}
+
+size_t forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden) {
+  if (B <= 0 || T <= 0 || C <= 0 || H <= 0 || E <= 0 || hidden <= 0) return 0;
+  return Workspace(B, T, C, H, E, hidden).bytes;
+}
+
+int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, cudaStream_t st) {
+  JB_REQUIRE(layers && f && n_layers >= 1, "forward_layers: null pointer or no layers");
+  const int B = f->B, T = f->T, C = f->C, H = f->H, E = f->E, hidden = f->hidden;
+  JB_REQUIRE(B >= 1 && T >= 1 && size_t(B) * T < (size_t(1) << 30), "forward_layers: bad shape (B=%d, T=%d)", B, T);
+  JB_REQUIRE(C % 128 == 0 && C <= 1024 && C == 64 * H && hidden % 128 == 0 && (E == 4 || E == 8),
+             "forward_layers: d_model %d / heads %d / hidden %d / experts %d not supported", C, H, hidden, E);
+  JB_REQUIRE(f->x && f->cos_tab && f->sin_tab && f->h_out && f->acc && f->hist && f->scalars && f->routing && f->workspace,
+             "forward_layers: null pointer");
+  JB_REQUIRE((f->w_final == nullptr) == (f->hidden_out == nullptr), "forward_layers: w_final and hidden_out come together");
+  const int N = B * T;
+  const Workspace ws(B, T, C, H, E, hidden);
+  const Routing rl(N, E);
+  uint8_t* w = static_cast<uint8_t*>(f->workspace);
+  uint16_t *xn = reinterpret_cast<uint16_t*>(w + ws.xn), *qkv = reinterpret_cast<uint16_t*>(w + ws.qkv);
+  uint16_t *o = reinterpret_cast<uint16_t*>(w + ws.o), *hid = reinterpret_cast<uint16_t*>(w + ws.hid);
+  uint16_t *y = reinterpret_cast<uint16_t*>(w + ws.y), *out = reinterpret_cast<uint16_t*>(w + ws.out);
+  uint16_t* disp = qkv;
+  float* x = f->x;
+
+  const size_t acc_bytes = size_t(n_layers) * (2 + E) * sizeof(double), hist_bytes = size_t(n_layers) * E * sizeof(int32_t);
+  if (reinterpret_cast<uint8_t*>(f->acc) + acc_bytes == reinterpret_cast<uint8_t*>(f->hist)) {
+    JB_CUDA(cudaMemsetAsync(f->acc, 0, acc_bytes + hist_bytes, st));
+  } else {
+    JB_CUDA(cudaMemsetAsync(f->acc, 0, acc_bytes, st));
+    JB_CUDA(cudaMemsetAsync(f->hist, 0, hist_bytes, st));
+  }
+  if (f->ids) JB_TRY(launch_embedding(f->ids, f->table, f->vocab, x, N, C, st));
+  JB_TRY(launch_rmsnorm(x, 0, layers[0].w_norm1, layers[0].eps1, xn, 1, N, C, st));
+
+  for (int l = 0; l < n_layers; ++l) {
+    const jb200_layer& p = layers[l];
+    const bool last = l + 1 == n_layers;
+    const float* s_in = f->s_in ? f->s_in[l] : nullptr;
+    float* s_out = f->s_out ? f->s_out[l] : nullptr;
+    const float* h_in = f->h_in ? f->h_in[l] : nullptr;
+    float* h_out = f->h_out[l];
+    JB_REQUIRE(h_out != nullptr, "forward_layers: h_out of layer %d missing", l);
+    double* acc = f->acc + size_t(l) * (2 + E);
+    int32_t* hist = f->hist + size_t(l) * E;
+    float* scalars = f->scalars + size_t(l) * 3;
+    uint8_t* r = static_cast<uint8_t*>(f->routing) + size_t(l) * rl.bytes;
+    int64_t* idx = reinterpret_cast<int64_t*>(r + rl.idx);
+    float* gates = reinterpret_cast<float*>(r + rl.gates);
+    int *counts = reinterpret_cast<int*>(r + rl.counts), *offs = reinterpret_cast<int*>(r + rl.offsets);
+    int *scatter = reinterpret_cast<int*>(r + rl.scatter), *gather = reinterpret_cast<int*>(r + rl.gather);
+    int* gate_idx = reinterpret_cast<int*>(r + rl.gate_idx);
+
+    // x += attn(norm1(x))
+    JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st));
+    // a state updated in place needs one segment per sequence: later segments would read what the last one writes
+    void* attn_scratch = (T > 1 && !(s_in && s_in == s_out)) ? w + ws.attn : nullptr;
+    if (attn_scratch && ws.attn == ws.lsf) attn_scratch = nullptr;            // no scratch wanted at this shape
+    JB_TRY(launch_attn_scan(qkv, qkv + C, qkv + 2 * C, 3 * C, p.gamma, f->cos_tab, f->sin_tab, f->n_pos, f->pos0, f->pos0_scalar,
+                            s_in, o, C, s_out, attn_scratch, B, T, H, 64, 0, st));
+    JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st));
+
+    // moe(norm2(x))
+    JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st));
+    JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
+    JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
+    JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st));
+    JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st));
+    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st));
+
+    // x += lsf(moe), and the norm of what follows
+    const float* w_next = last ? f->w_final : layers[l + 1].w_norm1;
+    const float eps_next = last ? f->eps_final : layers[l + 1].eps1;
+    void* xn_next = last ? f->hidden_out : static_cast<void*>(xn);
+    const LsfStats stats = {acc, acc + 2, hist, E, N, (long long)N * C, p.balance_alpha, scalars,
+                            p.mu, p.reflect_lam, p.reflect_tau, (f->reflect && p.mu) ? f->reflect + l : nullptr};
+    if (T == 1) {
+      JB_TRY(launch_lsf_step_norm(out, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
+                                  w_next ? xn_next : nullptr, B, C, st));
+    } else {
+      void* lsf_scratch = (h_in && h_in == h_out) || ws.lsf == ws.meta ? nullptr : w + ws.lsf;
+      JB_TRY(launch_lsf_scan(out, 1, nullptr, nullptr, nullptr, p.var_scale, p.alpha_min, p.alpha_max, h_in, x, nullptr, 0,
+                             h_out, lsf_scratch, B, T, C, st, &stats));
+      if (w_next) JB_TRY(launch_rmsnorm(x, 0, w_next, eps_next, xn_next, 1, N, C, st));
+    }
+  }
+  return JB200_OK;
+}
+
+}  // namespace jb

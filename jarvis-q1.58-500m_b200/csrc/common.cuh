@@ -13,6 +13,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "jarvis_b200.h"
 
 namespace jb {
@@ -50,6 +52,23 @@ int sm_count();
 void count_launch();  // bumps the per-process kernel-launch counter (jb200_kernel_launches)
 int set_dependent_launch(int on);
 bool dependent_launch_enabled();  // programmatic dependent launch of the library's kernels (jb200_set_dependent_launch)
+
+// Tensor maps are pure functions of their arguments, and a forward encodes the same ones for every layer (~0.4 us of
+// host time each, ten per layer): the last few dozen of a thread are kept and compared by value.  dims / box: `rank`
+// entries, innermost first; strides: rank - 1 entries in bytes.  `what` names the caller in error messages.
+int encode_tiled(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const void* ptr, const cuuint64_t* dims,
+                 const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle,
+                 CUtensorMapL2promotion promotion, const char* what);
+
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per device and kernel (0.3 us a call): `done` is a static
+// bit mask of the call site, one bit per device ordinal.
+int set_max_smem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done);
+#define JB_MAX_SMEM(kernel, bytes)                                                                             \
+  do {                                                                                                         \
+    static std::atomic<unsigned long long> done__{0};                                                          \
+    const int rc__ = ::jb::set_max_smem(reinterpret_cast<const void*>(kernel), (bytes), &done__);              \
+    if (rc__ != JB200_OK) return rc__;                                                                         \
+  } while (0)
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

@@ -96,23 +96,6 @@ struct GemmParams {
   int rope_feats;            // out-features [0, rope_feats) are q and k heads (64 features each), the rest plain
 };
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-inline EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
-
 // Residual epilogue: the old values of a tile (128 KiB) are what its epilogue waits for longest.  Called by
 // an epilogue warp BEFORE it waits for the tile's accumulator, i.e. while the tile's MMAs still run: every
 // lane asks L2 for the 128-byte line (32 f32 features) of one token row of each chunk the warp will handle.

@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "jarvis_b200.h"
+
 namespace jb {
 
 size_t pack_ternary_scratch_bytes(int out_features, int in_features);
@@ -51,21 +53,40 @@ int launch_scatter_combine(const void* y_bf16, const float* gates, const int* sc
 int launch_moe_finalize(const double* stats, const double* probs_sum, const int* top1_hist, int E, long long n_tokens,
                         long long n_elems, float balance_alpha, float* scalars, cudaStream_t stream);
 
+// Accumulators of the MoE layer whose output an LSF call scans: the scan derives act_var from them and leaves the
+// layer's scalars (l_balance, act_mean, act_var), so that no launch of its own is needed for those.
+struct LsfStats {
+  const double* stats;       // [2] sum, sum of squares; null: not used
+  const double* probs_sum;   // [E]
+  const int* top1_hist;      // [E]
+  int E;
+  long long n_tokens, n_elems;
+  float balance_alpha;
+  float* scalars;            // [3] out
+  const float* mu;           // with reflect: the layer's reflective penalty is left there
+  float lam, tau;
+  float* reflect;            // [1] out or null
+};
 int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const float* alpha_scalar,
                     const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,
                     float* resid, void* out, int out_dtype, float* h_last, void* scratch, int B, int T, int D,
-                    cudaStream_t stream);
+                    cudaStream_t stream, const LsfStats* st = nullptr);
 size_t lsf_scan_scratch_bytes(int B, int T, int D);
-int launch_lsf_step_norm(const void* m_bf16, const double* stats, const double* probs_sum, const int* top1_hist, int E,
-                         long long n_tokens, long long n_elems, float balance_alpha, float* scalars,
-                         const float* var_scale, float alpha_min, float alpha_max, const float* h_in, float* h_out,
-                         float* x, const float* w_norm, float eps, void* xn_bf16, int B, int C, cudaStream_t stream);
+int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* var_scale, float alpha_min, float alpha_max,
+                         const float* h_in, float* h_out, float* x, const float* w_norm, float eps, void* xn_bf16, int B,
+                         int C, cudaStream_t stream);
 
 int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, const float* gamma,
                      const float* cos_tab, const float* sin_tab, int n_pos, const int32_t* pos0, int pos0_scalar,
                      const float* s_in, void* o, int ld_o, float* s_out, void* scratch, int B, int T, int H,
                      int head_dim, int flags, cudaStream_t stream);
 size_t attn_scan_scratch_bytes(int B, int T, int H);
+
+int launch_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
+                         const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, cudaStream_t stream);
+size_t routing_layout(int N, int E, size_t* offsets);
+size_t forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden);
+int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, cudaStream_t stream);
 
 int launch_peer_barrier(const void* const* peer_flags, int world, int rank, cudaStream_t stream);
 int launch_ep_pull_gather(const void* const* peer_offs, const void* const* peer_gmap, const void* const* peer_xn,

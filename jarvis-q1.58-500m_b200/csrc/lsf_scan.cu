@@ -53,7 +53,24 @@ struct LsfParams {
   int n_pre_tiles;         // tiles in the non-final segments = (nseg - 1) * seg_len / tile
   float* seg_end;          // [B][n_pre_tiles][D] end value of each of those tiles from a zero carry
   float* seg_prod;         // [B][n_pre_tiles][D] product of its decays (tensor mode)
+  LsfStats st;             // st.stats != null: act_var comes from the MoE layer's accumulators
 };
+
+// The scalar decay of a call (model semantics).  With st.stats the variance of the MoE output is derived here, as
+// moe_finalize_kernel would have, instead of in a launch of its own between the combine and the scan.
+__device__ __forceinline__ float lsf_decay(const LsfParams& p) {
+  if (p.alpha_s) return __ldg(p.alpha_s);
+  const float var = p.st.stats ? moe_act_var(p.st.stats, p.st.n_elems) : __ldg(p.act_var);
+  return lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), var);
+}
+// One thread of the whole grid leaves the MoE layer's scalars.
+__device__ __forceinline__ void lsf_leave_scalars(const LsfStats& st) {
+  if (st.stats && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) {
+    moe_finalize_scalars(st.stats, st.probs_sum, st.top1_hist, st.E, st.n_tokens, st.n_elems, st.balance_alpha, st.scalars);
+    if (st.reflect)
+      *st.reflect = reflect_penalty(st.lam, st.tau, __ldg(st.mu), moe_act_mean(st.stats, st.n_elems), moe_act_var(st.stats, st.n_elems));
+  }
+}
 
 template <typename T>
 __device__ __forceinline__ float2 ld2(const T* p);
@@ -90,12 +107,8 @@ __global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_ke
 
   float alpha = 0.f, pw[TPW];  // scalar mode: pw[i] = alpha^(i+1)
   if (!TENSOR_ALPHA) {
-    if (p.alpha_s) {
-      alpha = __ldg(p.alpha_s);
-    } else {
-      const float z = -__ldg(p.var_scale) * __ldg(p.act_var);
-      alpha = p.alpha_min + (p.alpha_max - p.alpha_min) * (1.0f / (1.0f + expf(-z)));
-    }
+    alpha = lsf_decay(p);
+    if (!ENDS_ONLY) lsf_leave_scalars(p.st);
     float a = alpha;
 #pragma unroll
     for (int i = 0; i < TPW; ++i) { pw[i] = a; a *= alpha; }
@@ -224,8 +237,8 @@ __global__ void __launch_bounds__(256) lsf_short_kernel(const LsfParams p) {
   TOut* out = reinterpret_cast<TOut*>(p.out);
   float alpha = 0.f;
   if (!TENSOR_ALPHA) {
-    if (p.alpha_s) alpha = __ldg(p.alpha_s);
-    else alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), __ldg(p.act_var));
+    alpha = lsf_decay(p);
+    lsf_leave_scalars(p.st);
   }
   float2 h = p.h0 ? *reinterpret_cast<const float2*>(p.h0 + size_t(b) * p.D + ch) : make_float2(0.f, 0.f);
   for (int t = 0; t < p.T; ++t) {
@@ -252,13 +265,7 @@ __global__ void __launch_bounds__(256) lsf_short_kernel(const LsfParams p) {
 // summation order, every rounding as in the three kernels: the results are theirs bit for bit.
 struct LsfStepParams {
   const __nv_bfloat16* m;      // [B][C] MoE output
-  const double* stats;         // [2] sum, sum of squares of the MoE output
-  const double* probs_sum;     // [E] or null
-  const int* top1_hist;        // [E] or null
-  int E;
-  long long n_tokens, n_elems;
-  float balance_alpha;
-  float* scalars;              // [3] out: l_balance, act_mean, act_var
+  LsfStats st;                 // accumulators of the MoE layer and where its scalars go
   const float* var_scale;
   float alpha_min, alpha_max;
   const float* h_in;           // [B][C] or null (zero membrane)
@@ -273,11 +280,10 @@ struct LsfStepParams {
 __global__ void __launch_bounds__(256) lsf_step_norm_kernel(const LsfStepParams p) {
   pdl_wait();
   pdl_trigger();
-  if (blockIdx.x == 0 && threadIdx.x == 0)
-    moe_finalize_scalars(p.stats, p.probs_sum, p.top1_hist, p.E, p.n_tokens, p.n_elems, p.balance_alpha, p.scalars);
+  lsf_leave_scalars(p.st);
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= p.B) return;
-  const float alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), moe_act_var(p.stats, p.n_elems));
+  const float alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), moe_act_var(p.st.stats, p.st.n_elems));
   const size_t base = size_t(row) * p.C;
   float v[4][8];
   float ss = 0.f;
@@ -394,13 +400,8 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
   const int t_end = min(p.T, t_begin + p.seg_len);
   const int n_tiles = (t_end - t_begin + LT_TOK - 1) / LT_TOK;
 
-  float alpha;
-  if (p.alpha_s) {
-    alpha = __ldg(p.alpha_s);
-  } else {
-    const float z = -__ldg(p.var_scale) * __ldg(p.act_var);
-    alpha = p.alpha_min + (p.alpha_max - p.alpha_min) * (1.0f / (1.0f + expf(-z)));
-  }
+  const float alpha = lsf_decay(p);
+  lsf_leave_scalars(p.st);
   float pw[TPW];   // alpha^(i+1)
   {
     float a = alpha;
@@ -505,22 +506,11 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
 }
 
 int make_lsf_map(CUtensorMap* tm, const void* ptr, CUtensorMapDataType dt, int elem, int B, int T, int D) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) {
-    set_error("lsf_scan: cuTensorMapEncodeTiled entry point not available");
-    return JB200_ERR_CUDA;
-  }
   const cuuint64_t gdim[3] = {cuuint64_t(D), cuuint64_t(T), cuuint64_t(B)};
   const cuuint64_t gstride[2] = {cuuint64_t(D) * elem, cuuint64_t(T) * D * elem};
   const cuuint32_t box[3] = {cuuint32_t(LSF_CH), cuuint32_t(LT_TOK), 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult cr = fn(tm, dt, 3, const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (cr != CUDA_SUCCESS) {
-    set_error("lsf_scan: cuTensorMapEncodeTiled failed (%d)", int(cr));
-    return JB200_ERR_CUDA;
-  }
-  return JB200_OK;
+  return encode_tiled(tm, dt, 3, ptr, gdim, gstride, box, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                      "lsf_scan");
 }
 
 template <bool FUSED>
@@ -552,8 +542,7 @@ int launch_tma(LsfParams p, cudaStream_t stream) {
     JB_LAUNCH_CHECK("lsf_scan_kernel<ends>");
   }
   dim3 grid((p.D + LSF_CH - 1) / LSF_CH, p.B, p.nseg);
-  JB_CUDA(cudaFuncSetAttribute(lsf_tma_kernel<FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(Cfg::smem_bytes(Cfg::STAGES_ALONE))));
+  JB_MAX_SMEM(lsf_tma_kernel<FUSED>, Cfg::smem_bytes(Cfg::STAGES_ALONE));
   launch_dep(lsf_tma_kernel<FUSED>, grid, LSF_THREADS, Cfg::smem_bytes(stages), stream, tm_m, tm_io, p, stages, status);
   JB_LAUNCH_CHECK("lsf_tma_kernel");
   return JB200_OK;
@@ -585,14 +574,14 @@ size_t lsf_scan_scratch_bytes(int B, int T, int D) {
 int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const float* alpha_scalar,
                     const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,
                     float* resid, void* out, int out_dtype, float* h_last, void* scratch, int B, int T, int D,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, const LsfStats* st) {
   JB_REQUIRE(B >= 0 && T >= 0 && D > 0, "lsf_scan: bad shape (%d, %d, %d)", B, T, D);
   JB_REQUIRE(D % 2 == 0, "lsf_scan: channel count (%d) must be even", D);
   JB_REQUIRE(B <= 65535, "lsf_scan: batch (%d) exceeds 65535", B);
   JB_REQUIRE((m_dtype == 0 || m_dtype == 1) && (out_dtype == 0 || out_dtype == 1), "lsf_scan: dtype must be 0 (f32) or 1 (bf16)");
   if (B == 0 || T == 0) return JB200_OK;
   JB_REQUIRE(m != nullptr, "lsf_scan: null input");
-  JB_REQUIRE(alpha_tensor || alpha_scalar || (act_var && var_scale), "lsf_scan: no decay given");
+  JB_REQUIRE(alpha_tensor || alpha_scalar || ((act_var || st) && var_scale), "lsf_scan: no decay given");
   JB_REQUIRE(out || resid || h_last, "lsf_scan: no output requested");
   const uintptr_t a8 = 7u, a4 = 3u;
   JB_REQUIRE((reinterpret_cast<uintptr_t>(m) & (m_dtype == 0 ? a8 : a4)) == 0, "lsf_scan: input pointer misaligned");
@@ -601,7 +590,7 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
   JB_REQUIRE(!resid || (reinterpret_cast<uintptr_t>(resid) & a8) == 0, "lsf_scan: residual pointer misaligned");
   JB_REQUIRE((!h0 || (reinterpret_cast<uintptr_t>(h0) & a8) == 0) && (!h_last || (reinterpret_cast<uintptr_t>(h_last) & a8) == 0),
              "lsf_scan: state pointer misaligned");
-  LsfParams p;
+  LsfParams p = {};
   p.m = m; p.alpha_t = alpha_tensor; p.alpha_s = alpha_scalar; p.act_var = act_var; p.var_scale = var_scale;
   p.alpha_min = alpha_min; p.alpha_max = alpha_max; p.h0 = h0; p.resid = resid; p.out = out; p.h_last = h_last;
   p.B = B; p.T = T; p.D = D;
@@ -609,6 +598,7 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
   p.nseg = 1;
   p.n_pre_tiles = 0;
   p.seg_end = p.seg_prod = nullptr;
+  if (st) p.st = *st;
   if (scratch) {
     JB_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & a8) == 0, "lsf_scan: scratch pointer misaligned");
     const int sms = sm_count();
@@ -638,23 +628,21 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
   return launch_t<true, float, bf>(p, stream);
 }
 
-int launch_lsf_step_norm(const void* m_bf16, const double* stats, const double* probs_sum, const int* top1_hist, int E,
-                         long long n_tokens, long long n_elems, float balance_alpha, float* scalars,
-                         const float* var_scale, float alpha_min, float alpha_max, const float* h_in, float* h_out,
-                         float* x, const float* w_norm, float eps, void* xn_bf16, int B, int C, cudaStream_t stream) {
+int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* var_scale, float alpha_min, float alpha_max,
+                         const float* h_in, float* h_out, float* x, const float* w_norm, float eps, void* xn_bf16, int B,
+                         int C, cudaStream_t stream) {
   JB_REQUIRE(B >= 0 && C > 0, "lsf_step_norm: bad shape (%d, %d)", B, C);
   JB_REQUIRE(C % 8 == 0 && C <= 1024, "lsf_step_norm: d_model (%d) must be a multiple of 8 and at most 1024", C);
-  JB_REQUIRE(E >= 0 && E <= 64 && n_tokens > 0 && n_elems > 0, "lsf_step_norm: bad counts");
+  JB_REQUIRE(st.E >= 0 && st.E <= 64 && st.n_tokens > 0 && st.n_elems > 0, "lsf_step_norm: bad counts");
   if (B == 0) return JB200_OK;
-  JB_REQUIRE(m_bf16 && stats && scalars && var_scale && h_out && x, "lsf_step_norm: null pointer");
+  JB_REQUIRE(m_bf16 && st.stats && st.scalars && var_scale && h_out && x, "lsf_step_norm: null pointer");
   JB_REQUIRE((w_norm == nullptr) == (xn_bf16 == nullptr), "lsf_step_norm: norm weight and normalised output come together");
   JB_REQUIRE(aligned16(m_bf16) && aligned16(h_out) && aligned16(x) && (!h_in || aligned16(h_in)) &&
                  (!w_norm || (aligned16(w_norm) && aligned16(xn_bf16))),
              "lsf_step_norm: pointers must be 16-byte aligned");
   LsfStepParams p;
   p.m = reinterpret_cast<const __nv_bfloat16*>(m_bf16);
-  p.stats = stats; p.probs_sum = probs_sum; p.top1_hist = top1_hist; p.E = E;
-  p.n_tokens = n_tokens; p.n_elems = n_elems; p.balance_alpha = balance_alpha; p.scalars = scalars;
+  p.st = st;
   p.var_scale = var_scale; p.alpha_min = alpha_min; p.alpha_max = alpha_max;
   p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;
   p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);

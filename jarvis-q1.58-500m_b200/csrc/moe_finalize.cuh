@@ -32,6 +32,12 @@ __device__ __forceinline__ void moe_finalize_scalars(const double* stats, const 
   }
 }
 
+// ReflectivePenalty of a layer (jarvis_model.py:329-351): lam * ((mu - act_mean)^2 + relu(act_var - tau)).
+__device__ __forceinline__ float reflect_penalty(float lam, float tau, float mu, float mean, float var) {
+  const float d = mu - mean, e = var - tau;
+  return lam * (d * d + (e > 0.f ? e : (e != e ? e : 0.f)));      // a NaN variance stays NaN, as with F.relu
+}
+
 // The decay of one LSF call from the variance of the MoE output (jarvis_model.py:297-298).
 __device__ __forceinline__ float lsf_alpha_from_var(float alpha_min, float alpha_max, float var_scale, float act_var) {
   return alpha_min + (alpha_max - alpha_min) * (1.0f / (1.0f + expf(var_scale * act_var)));

@@ -458,12 +458,12 @@ int launch_router_top2(const void* x_bf16, const float* w_router, int n_tokens, 
   const int blocks = (n_tokens + tpc - 1) / tpc;
   const size_t smem = size_t(E) * C * sizeof(float);
   if (E == 4) {
-    JB_CUDA(cudaFuncSetAttribute(router_top2_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    JB_MAX_SMEM(router_top2_kernel<4>, 160 * 1024);
     launch_dep(router_top2_kernel<4>, blocks, ROUTER_THREADS, smem, stream,
         reinterpret_cast<const __nv_bfloat16*>(x_bf16), w_router, n_tokens, C, tpc, topk_idx, gates, probs_out, probs_sum,
         top1_hist);
   } else {
-    JB_CUDA(cudaFuncSetAttribute(router_top2_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    JB_MAX_SMEM(router_top2_kernel<8>, 160 * 1024);
     launch_dep(router_top2_kernel<8>, blocks, ROUTER_THREADS, smem, stream,
         reinterpret_cast<const __nv_bfloat16*>(x_bf16), w_router, n_tokens, C, tpc, topk_idx, gates, probs_out, probs_sum,
         top1_hist);

@@ -368,36 +368,20 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
 
-  EncodeTiledFn enc = encode_tiled_fn();
-  if (!enc) {
-    set_error("ternary_linear: cuTensorMapEncodeTiled entry point not available");
-    return JB200_ERR_CUDA;
-  }
   CUtensorMap tmap;
   const cuuint64_t gdim[2] = {cuuint64_t(K), cuuint64_t(M)};
   const cuuint64_t gstride[1] = {cuuint64_t(K) * 2};
   const cuuint32_t box[2] = {cuuint32_t(BK), cuuint32_t(bn)};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult cr = enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x_bf16), gdim, gstride, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (cr != CUDA_SUCCESS) {
-    set_error("ternary_linear: cuTensorMapEncodeTiled failed (%d)", int(cr));
-    return JB200_ERR_CUDA;
-  }
-
-
+  int rc = encode_tiled(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x_bf16, gdim, gstride, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "ternary_linear");
+  if (rc != JB200_OK) return rc;
   CUtensorMap tmap_w = tmap;     // packed weights: the decoders read them with plain loads, the map is not used
   if (w_layout == 2) {
     const cuuint64_t wdim[2] = {cuuint64_t(K), cuuint64_t(N)};
     const cuuint32_t wbox[2] = {cuuint32_t(BK), cuuint32_t(BM)};
-    cr = enc(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint8_t*>(w_packed), wdim, gstride, wbox, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) {
-      set_error("dense_linear: cuTensorMapEncodeTiled failed for the weights (%d)", int(cr));
-      return JB200_ERR_CUDA;
-    }
+    rc = encode_tiled(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w_packed, wdim, gstride, wbox, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "dense_linear (weights)");
+    if (rc != JB200_OK) return rc;
   }
 
   // Residual epilogue of a single matrix: the tile is added to the f32 stream by TMA reductions (needs 16-byte
@@ -408,18 +392,13 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
     const cuuint64_t odim[2] = {cuuint64_t(N), cuuint64_t(M)};
     const cuuint64_t ostride[1] = {cuuint64_t(N) * 4};
     const cuuint32_t obox[2] = {32, 32};
-    cr = enc(&tmap_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, out, odim, ostride, obox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) {
-      set_error("ternary_linear: cuTensorMapEncodeTiled failed for the residual stream (%d)", int(cr));
-      return JB200_ERR_CUDA;
-    }
+    rc = encode_tiled(&tmap_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, out, odim, ostride, obox, CU_TENSOR_MAP_SWIZZLE_NONE,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "ternary_linear (residual stream)");
+    if (rc != JB200_OK) return rc;
     p.resid_stage_smem = 1;
   }
   const size_t smem_bytes = p.resid_stage_smem ? SMEM_BYTES_RESID : SMEM_BYTES;
-
-  // per device and cheap: set on every call rather than remembering which devices have seen it
-  JB_CUDA(cudaFuncSetAttribute(ternary_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM_BYTES_RESID)));
+  JB_MAX_SMEM(ternary_gemm_kernel, SMEM_BYTES_RESID);
   const long max_tiles = long((M + bn - 1) / bn + (G - 1)) * n_ft;
   const int grid = int(max_tiles < sms ? max_tiles : sms);
   launch_dep(ternary_gemm_kernel, grid, NUM_THREADS, smem_bytes, stream, tmap, tmap_w, tmap_out, p);

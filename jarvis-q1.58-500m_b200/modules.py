@@ -15,7 +15,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import ops
+from . import chain, ops
 
 # ----------------------------------------------------------------------------------------------
 # small pieces
@@ -270,7 +270,13 @@ class SparseMoELayer(nn.Module):
         self.stats_group = None
         self._n_total_hint = None   # global token count when known (avoids a host read per layer)
         self._ep = None             # parallel.PeerExpertParallelMoE: experts spread over the ranks of a group
-        self.last_routing = None  # (topk_idx, gates, metadata) of the most recent call, for inspection
+        self._routing = None      # what last_routing shows
+
+    @property
+    def last_routing(self):
+        """(topk_idx, gates, metadata) of the most recent call, for inspection."""
+        r = self._routing
+        return chain.routing_views(r) if r is not None and isinstance(r[-1], chain.LayerTable) else r
 
     def packed(self):
         return (self._p1.get([m.weight for m in self.w1], stack=True),
@@ -333,7 +339,7 @@ class SparseMoELayer(nn.Module):
             acc.copy_(both[:2 + E])
             hist.copy_(both[2 + E:2 + 2 * E].to(torch.int32))
             n_total = int(both[-1].item()) if self._n_total_hint is None else self._n_total_hint
-        self.last_routing = (idx, gates, meta)
+        self._routing = (idx, gates, meta)
         if not finalize:
             return out, n_total
         scalars = ops.moe_finalize(acc[:2], acc[2:], hist, E, n_total, n_total * C, self.balance_alpha, scalars=scalars)
@@ -437,7 +443,14 @@ class JarvisBlock(nn.Module):
                      inplace_state=False, scratch=None, cp=None):
         """x: f32 (B*T, C) residual stream, UPDATED IN PLACE.  Returns (h_last f32 (B, C), scalars f32
         [l_balance, act_mean, act_var], attention state or None).  cp (parallel.ContextParallel): this rank
-        holds one T-token slice of every sequence; states returned are those after the whole sequence."""
+        holds one T-token slice of every sequence; states returned are those after the whole sequence.
+        A call of its own (no `scratch` from a loop over layers) goes through one native call (chain.py); the
+        kernel-by-kernel form below is for what happens between the kernels of a layer on several GPUs."""
+        if scratch is None and cp is None:
+            tab = chain.table_of(self, [self])
+            if tab is not None:
+                r = self._chain(tab, x, B, T, h_prev, start_pos, attn_state, want_attn_state, inplace_state)
+                return r.h[0], r.scalars[0], None if r.S is None else r.S[0]
         C = x.shape[1]
         xn = ops.rmsnorm(x, _f32(self.norm1.weight), self.norm1.eps)
         o, state = self.attn.scan_rows(xn, B, T, start_pos, attn_state, want_attn_state, inplace_state, cp=cp)
@@ -493,11 +506,21 @@ class JarvisBlock(nn.Module):
             h_out=h_prev if (inplace_state and h_prev is not None and h_prev.dtype == torch.float32) else None)
         return h_last, scalars, state, xn_next
 
+    def _chain(self, tab, x, B, T, h_prev, start_pos, attn_state=None, want_state=False, inplace=False):
+        return chain.run(tab, x, B, T, start_pos=start_pos, max_position=self.attn.max_position,
+                         h_in=None if h_prev is None else [h_prev], s_in=None if attn_state is None else [attn_state],
+                         want_state=want_state, inplace=inplace)
+
     def forward(self, x, h_prev=None, start_pos: int = 0):
         B, T, C = x.shape
-        rows = x.reshape(B * T, C).float().clone()
-        h_last, sc, _ = self.forward_rows(rows, B, T, h_prev, start_pos)
-        l_reflect = self.reflect(sc[1], sc[2])
+        rows = x.reshape(B * T, C).to(torch.float32, copy=True)
+        tab = chain.table_of(self, [self]) if x.is_cuda else None
+        if tab is not None and tab.has_reflect:
+            r = self._chain(tab, rows, B, T, h_prev, start_pos)
+            h_last, sc, l_reflect = r.h[0], r.scalars[0], r.reflect[0]
+        else:
+            h_last, sc, _ = self.forward_rows(rows, B, T, h_prev, start_pos)
+            l_reflect = self.reflect(sc[1], sc[2])
         return rows.view(B, T, C).to(x.dtype), h_last.to(x.dtype), sc[0], l_reflect
 
 
@@ -526,8 +549,10 @@ class Jarvis(nn.Module):
         self.carry_attention_state = False
         self._cp = None
         self.logits_dtype = torch.bfloat16
+        self.use_chain = True      # False: every kernel by its own ops call (to put something between them)
         self._lm_head_bf16 = None
         self.last_aux = None
+        self._reflect = None
 
     def get_backend_status(self):
         n = len(self.blocks)
@@ -565,15 +590,42 @@ class Jarvis(nn.Module):
             self._lm_head_bf16 = (key, wp)
         return self._lm_head_bf16[1]
 
+    def _chain_table(self):
+        """The layers' descriptor table when the whole forward can go through one native call, else None."""
+        if not self.use_chain or self._cp is not None:
+            return None
+        return chain.table_of(self, list(self.blocks._modules.values()))
+
+    def _chain_rows(self, tab, idx, start_pos, h_in, s_in, want_state, max_position=None, inplace=False):
+        B, T = idx.shape
+        idx = ops._need(idx.contiguous(), torch.int64, "embedding.idx")
+        x = torch.empty((B * T, self.d_model), dtype=torch.float32, device=idx.device)
+        return chain.run(tab, x, B, T, ids=idx, table=_f32(self.tok_emb.weight), start_pos=start_pos, max_position=max_position,
+                         h_in=h_in, s_in=s_in, want_state=want_state, inplace=inplace,
+                         final_norm=(_f32(self.final_norm.weight), self.final_norm.eps))
+
     def hidden_rows(self, idx, persist_state=False):
         """Embedding + all blocks + final norm -> bf16 (B*T, C) hidden rows."""
         if self.training:
             raise RuntimeError("Jarvis (sm_100a): inference only; call .eval() first")
         B, T = idx.shape
-        x = ops.embedding(idx.contiguous(), _f32(self.tok_emb.weight)).view(B * T, self.d_model)
         start_pos = self._token_pos if persist_state else 0
         if persist_state:
             self._token_pos += T * (self._cp.world if self._cp is not None else 1)
+        tab = self._chain_table()
+        if tab is not None:
+            h_in = s_in = None
+            if persist_state:
+                h_in = [h if h is not None and h.shape[0] == B else None for h in self._h_states]
+                if self.carry_attention_state:
+                    s_in = [s if s is not None and s.shape[0] == B else None for s in self._attn_states]
+            r = self._chain_rows(tab, idx, start_pos, h_in, s_in, self.carry_attention_state)
+            self._h_states = r.h
+            self._attn_states = r.S if r.S is not None else [None] * tab.n
+            self.last_aux, self._reflect = r.scalars, r.reflect
+            return r.hidden
+        self._reflect = None
+        x = ops.embedding(idx.contiguous(), _f32(self.tok_emb.weight)).view(B * T, self.d_model)
         h_prevs = self._h_states if persist_state else [None] * len(self.blocks)
         s_prevs = self._attn_states if (persist_state and self.carry_attention_state) else [None] * len(self.blocks)
         new_h, new_s, aux = [], [], []
@@ -610,8 +662,13 @@ class Jarvis(nn.Module):
             raise RuntimeError("Jarvis (sm_100a): inference only; call .eval() first")
         B, T = idx.shape
         n = len(self.blocks)
-        x = ops.embedding(idx.contiguous(), _f32(self.tok_emb.weight)).view(B * T, self.d_model)
         pos = 0 if positions is None else positions
+        tab = self._chain_table()
+        if tab is not None:
+            r = self._chain_rows(tab, idx, pos, None if state is None else state["h"], None if state is None else state["S"],
+                                 True, max_position, inplace and state is not None)
+            return self._logits(r.hidden, B, T), {"h": r.h, "S": r.S}
+        x = ops.embedding(idx.contiguous(), _f32(self.tok_emb.weight)).view(B * T, self.d_model)
         hs = state["h"] if state is not None else [None] * n
         Ss = state["S"] if state is not None else [None] * n
         new_h, new_s = [], []
@@ -635,26 +692,26 @@ class Jarvis(nn.Module):
                 new_h.append(h_last)
                 new_s.append(S)
             hidden = ops.rmsnorm(x, _f32(self.final_norm.weight), self.final_norm.eps)
-        vocab = self.lm_head.weight.shape[0]
-        logits = ops.dense_linear(hidden, self._lm_head_weight()).view(B, T, -1)[..., :vocab]
-        return logits, {"h": new_h, "S": new_s}
+        return self._logits(hidden, B, T), {"h": new_h, "S": new_s}
+
+    def _logits(self, hidden, B, T):
+        """Dense bf16 lm_head on the same tcgen05 pipeline as the ternary layers (weight tiles by TMA); the padded
+        vocabulary columns are sliced off as a view."""
+        return ops.dense_linear(hidden, self._lm_head_weight()).view(B, T, -1)[..., :self.lm_head.weight.shape[0]]
 
     @torch.no_grad()
     def forward(self, idx, targets=None, persist_state=False):
         B, T = idx.shape
-        hidden = self.hidden_rows(idx, persist_state)
-        vocab = self.lm_head.weight.shape[0]
-        # dense bf16 lm_head on the same tcgen05 pipeline as the ternary layers (weight tiles by TMA); the padded
-        # vocabulary columns are sliced off as a view
-        logits = ops.dense_linear(hidden, self._lm_head_weight()).view(B, T, -1)[..., :vocab]
-        if self.logits_dtype != torch.bfloat16:
-            logits = logits.to(self.logits_dtype)
+        logits = self._logits(self.hidden_rows(idx, persist_state), B, T)
         loss = None
         if targets is not None:
-            ce = F.cross_entropy(logits.float().view(-1, logits.size(-1)), targets.view(-1))
-            aux = torch.stack(self.last_aux)
-            l_reflect = sum(b.reflect(sc[1], sc[2]) for b, sc in zip(self.blocks, self.last_aux))
-            loss = ce + aux[:, 0].sum() + l_reflect
+            aux = self.last_aux if torch.is_tensor(self.last_aux) else torch.stack(self.last_aux)
+            reflect = self._reflect
+            if reflect is None:
+                reflect = torch.stack([b.reflect(sc[1], sc[2]) for b, sc in zip(self.blocks, self.last_aux)])
+            loss = ops.cross_entropy(logits, targets, aux, reflect)
+        if self.logits_dtype != torch.bfloat16:
+            logits = logits.to(self.logits_dtype)
         return logits, loss
 
     def set_batch_split(self, group, global_tokens=None):

@@ -520,6 +520,27 @@ def lsf_step_norm(m: torch.Tensor, stats, probs_sum, top1_hist, E: int, n_tokens
     return xn, h_out
 
 
+def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, aux: torch.Tensor, reflect: torch.Tensor) -> torch.Tensor:
+    """mean over the targets other than -100 of -log softmax(logits)[target], + aux[:, 0].sum() + reflect.sum()
+    (Jarvis.forward with targets, jarvis_engine/jarvis_model.py:536-545).  logits: bf16 (B, T, V), the padded rows of
+    dense_linear; targets: int64 (B, T); aux: f32 (L, 3); reflect: f32 (L,) -> f32 scalar."""
+    lib = _lib.load()
+    B, T, V = logits.shape
+    ld = logits.stride(1)
+    if logits.dtype != torch.bfloat16 or logits.stride(2) != 1 or (B > 1 and logits.stride(0) != T * ld):
+        raise RuntimeError("cross_entropy: logits must be bf16 rows of one stride")
+    y = _need(targets.reshape(-1), torch.int64, "cross_entropy.targets")
+    if y.numel() != B * T:
+        raise RuntimeError("cross_entropy: one target per token is needed")
+    _need(aux, torch.float32, "cross_entropy.aux")
+    _need(reflect, torch.float32, "cross_entropy.reflect")
+    buf = torch.empty(B * T + 1, dtype=torch.float32, device=logits.device)
+    loss = buf[B * T]
+    _lib.check(lib.jb200_cross_entropy(_ptr(logits), ld, B * T, V, _ptr(y), _ptr(buf), _ptr(aux), aux.stride(0), _ptr(reflect),
+                                       reflect.numel(), _ptr(loss), _stream()), "jb200_cross_entropy")
+    return loss
+
+
 def sample(logits: torch.Tensor, u: torch.Tensor | None = None, *, temperature: float = 0.7, top_k: int = 50,
            top_p: float = 0.9, want_prob: bool = False):
     """One token per row of `logits` ((B, V) f32 or bf16, rows may be strided): temperature / top-k / top-p
