@@ -329,8 +329,7 @@ typedef struct jb200_forward {
   float* const* s_out;
   const float* const* h_in;      /* f32 [B][C] */
   float* const* h_out;           /* required */
-  double* acc;                   /* f64 [n_layers][2 + E], i32 [n_layers][E]: zeroed by the call, then the sums of */
-  int32_t* hist;                 /*   jb200_moe_scatter_combine / jb200_router_top2 */
+  void* accumulators;            /* n_layers * jb200_accumulator_bytes, 8-byte aligned: cleared and used by the call */
   float* scalars;                /* f32 [n_layers][3]: l_balance, act_mean, act_var of every layer */
   float* reflect;                /* f32 [n_layers]: lam * ((mu - act_mean)^2 + relu(act_var - tau)); or NULL */
   void* routing;                 /* n_layers blocks of jb200_routing_layout bytes: the routing results of every layer */
@@ -342,6 +341,7 @@ typedef struct jb200_forward {
 
 /* Bytes of one layer's routing block; offsets[7] (may be NULL) receives the byte offsets of topk_idx (i64 [N][2]), gates
  * (f32 [N][2]), expert_counts, expert_offsets, scatter_map, gather_map, gate_idx_map (see jb200_moe_metadata). */
+size_t jb200_accumulator_bytes(int E);
 size_t jb200_routing_layout(int N, int E, size_t* offsets);
 size_t jb200_forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden);
 

@@ -36,8 +36,7 @@ class Forward(C.Structure):
     """jb200_forward"""
     _fields_ = [(n, _I) for n in ("B", "T", "C", "H", "E", "hidden")] + \
                [("ids", _P), ("table", _P), ("vocab", _I), ("x", _P), ("cos_tab", _P), ("sin_tab", _P), ("n_pos", _I),
-                ("pos0", _P), ("pos0_scalar", _I), ("s_in", _P), ("s_out", _P), ("h_in", _P), ("h_out", _P), ("acc", _P),
-                ("hist", _P), ("scalars", _P), ("reflect", _P), ("routing", _P), ("w_final", _P), ("eps_final", _F), ("hidden_out", _P),
+                ("pos0", _P), ("pos0_scalar", _I), ("s_in", _P), ("s_out", _P), ("h_in", _P), ("h_out", _P), ("accumulators", _P), ("scalars", _P), ("reflect", _P), ("routing", _P), ("w_final", _P), ("eps_final", _F), ("hidden_out", _P),
                 ("workspace", _P)]
 
 
@@ -76,6 +75,7 @@ PROTOTYPES = {
     "jb200_lsf_step_norm": (_I, [_P, _P, _P, _P, _I, C.c_longlong, C.c_longlong, _F, _P, _P, _F, _F, _P, _P, _P, _P, _F, _P,
                                  _I, _I, _P]),
     "jb200_cross_entropy": (_I, [_P, _I, _I, _I, _P, _P, _P, _I, _P, _I, _P, _P]),
+    "jb200_accumulator_bytes": (_Z, [_I]),
     "jb200_routing_layout": (_Z, [_I, _I, C.POINTER(_Z)]),
     "jb200_forward_workspace_bytes": (_Z, [_I] * 6),
     "jb200_forward_layers": (_I, [_P, _I, C.POINTER(Forward), _P]),

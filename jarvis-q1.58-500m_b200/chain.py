@@ -41,6 +41,7 @@ class LayerTable:
         self.C, self.H, self.E = b0.norm1.weight.numel(), b0.attn.n_heads, b0.moe.num_experts
         self.hidden = b0.moe.w1[0].weight.shape[0]
         self.device = b0.norm1.weight.device
+        self.acc_bytes = _lib.load().jb200_accumulator_bytes(self.E)
         self.array = (_lib.Layer * self.n)()
         self._keep = []
         self._sizes = {}
@@ -161,9 +162,7 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
     if not (x.is_cuda and x.dtype is torch.float32 and x.is_contiguous()):
         raise RuntimeError("forward: expected a contiguous f32 CUDA residual stream (this path has no CPU fallback)")
     ws_bytes, routing_bytes, _ = tab.sizes(B, T)
-    acc_bytes = n * (2 + tab.E) * 8
-    hist_off = acc_bytes
-    head = (acc_bytes + n * tab.E * 4 + 255) // 256 * 256
+    head = (n * tab.acc_bytes + 255) // 256 * 256
     work = torch.empty(head + ws_bytes, dtype=torch.uint8, device=dev)
     routing = torch.empty(n * routing_bytes, dtype=torch.uint8, device=dev)
     res = Result()
@@ -207,7 +206,7 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
         res.S, so_ptrs = list(s_all.unbind(0)), _rows_of(n, s_all.data_ptr(), B * tab.H * 64 * 64 * 4)
         f.s_out = C.addressof(so_ptrs)
     base = work.data_ptr()
-    f.acc, f.hist, f.workspace = base, base + hist_off, base + head
+    f.accumulators, f.workspace = base, base + head
     f.scalars, f.routing = aux.data_ptr(), routing.data_ptr()
     f.reflect = aux.data_ptr() + 12 * n if tab.has_reflect else None
     res.hidden = None

@@ -418,6 +418,8 @@ int jb200_lsf_step_norm(const void* m_bf16, const double* stats, const double* p
                               static_cast<cudaStream_t>(stream));
 }
 
+size_t jb200_accumulator_bytes(int E) { return accumulator_bytes(E); }
+
 size_t jb200_routing_layout(int N, int E, size_t* offsets) { return routing_layout(N, E, offsets); }
 
 size_t jb200_forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden) {

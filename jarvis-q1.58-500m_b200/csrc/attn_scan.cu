@@ -73,6 +73,7 @@ struct AttnParams {
   float* handoff;          // [n_split][64][64] f32
   int* ctrl;               // [1 + n_split], zeroed before the launch
   unsigned int* status;
+  int settled;             // single-token step: state and positions were complete before the kernel ahead of this one started
 };
 
 __device__ __forceinline__ uint32_t swz(int row, int chunk16) {  // byte offset inside a swizzled [rows][128 B] tile
@@ -901,6 +902,10 @@ __device__ __forceinline__ float decode_update(float gamma, float s, float v, fl
   return __fmaf_rn(gamma, s, __fmul_rn(v, k));
 }
 
+// RoPE of a pair (d, d + 32), roundings spelled out for the same reason.
+__device__ __forceinline__ float rope_lo(float a, float b, float c, float s) { return __fmaf_rn(a, c, -__fmul_rn(b, s)); }
+__device__ __forceinline__ float rope_hi(float a, float b, float c, float s) { return __fmaf_rn(b, c, __fmul_rn(a, s)); }
+
 // One-token step (decode): S <- gamma*S + v (x) k', o = S q' for every (sequence, head).  Pure state
 // streaming: 2 x 16 KiB of fp32 state per (sequence, head) against 384 B of q, k, v, so the kernel is a
 // coalesced read-modify-write of S with the feature map + RoPE of the single token done in shared memory.
@@ -908,31 +913,39 @@ __device__ __forceinline__ float decode_update(float gamma, float s, float v, fl
 __global__ void __launch_bounds__(256)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                    const __nv_bfloat16* __restrict__ v, int ld_qkv, const AttnParams p) {
-  __shared__ float sq[D], sk[D], sv[D], rq[D], rk[D];
-  pdl_wait();
-  pdl_trigger();
+  __shared__ float sv[D], rq[D], rk[D];
   const int h = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
-  // the thread's 64 bytes of state first: they are in flight during the feature map of the token below
+  // What the token does not decide first: the thread's 64 bytes of state, the position and its angles.  In a chain they
+  // were written long before and are fetched while the projection still runs.
   const int row = t >> 2, c0 = (t & 3) * 16;
   const size_t so = (size_t(b) * p.H + h) * D * D + size_t(row) * D + c0;
   float4 st[4];
+  float cs = 0.f, sn = 0.f, gamma = 0.f;
+  auto fetch = [&]() {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    st[i] = p.s_in ? *reinterpret_cast<const float4*>(p.s_in + so + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float gamma = __ldg(p.gamma + h);
-  if (t < D) {
-    const size_t off = size_t(b) * ld_qkv + h * D + t;
-    sq[t] = elu1(__bfloat162float(q[off])) * 0.125f;
-    sk[t] = elu1(__bfloat162float(k[off]));
-    sv[t] = __bfloat162float(v[off]);
-  }
-  __syncthreads();
+    for (int i = 0; i < 4; ++i)
+      st[i] = p.s_in ? *reinterpret_cast<const float4*>(p.s_in + so + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    gamma = __ldg(p.gamma + h);
+    if (t < D / 2) {
+      int pos = p.pos0 ? p.pos0[b] : p.pos0_scalar;
+      pos = pos < 0 ? 0 : (pos >= p.n_pos ? p.n_pos - 1 : pos);
+      cs = __ldg(p.cos_tab + size_t(pos) * 32 + t);
+      sn = __ldg(p.sin_tab + size_t(pos) * 32 + t);
+    }
+  };
+  if (p.settled) fetch();
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+  if (!p.settled) fetch();
+  const size_t off = size_t(b) * ld_qkv + h * D;
   if (t < D / 2) {
-    int pos = p.pos0 ? p.pos0[b] : p.pos0_scalar;
-    pos = pos < 0 ? 0 : (pos >= p.n_pos ? p.n_pos - 1 : pos);
-    const float c = __ldg(p.cos_tab + size_t(pos) * 32 + t), sn = __ldg(p.sin_tab + size_t(pos) * 32 + t);
-    rq[t] = sq[t] * c - sq[t + 32] * sn;  rq[t + 32] = sq[t + 32] * c + sq[t] * sn;
-    rk[t] = sk[t] * c - sk[t + 32] * sn;  rk[t + 32] = sk[t + 32] * c + sk[t] * sn;
+    const float q0 = elu1(__bfloat162float(q[off + t])) * 0.125f, q1 = elu1(__bfloat162float(q[off + t + 32])) * 0.125f;
+    const float k0 = elu1(__bfloat162float(k[off + t])), k1 = elu1(__bfloat162float(k[off + t + 32]));
+    rq[t] = rope_lo(q0, q1, cs, sn);  rq[t + 32] = rope_hi(q0, q1, cs, sn);
+    rk[t] = rope_lo(k0, k1, cs, sn);  rk[t + 32] = rope_hi(k0, k1, cs, sn);
+  } else if (t < D / 2 + D) {
+    sv[t - 32] = __bfloat162float(v[off + t - 32]);
   }
   __syncthreads();
   const float vr = sv[row];
@@ -982,10 +995,6 @@ attn_decode_stream_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
     sm->abort_flag = 0;
     fence_mbar_init();
   }
-  pdl_wait();
-  pdl_trigger();
-  __syncthreads();
-  volatile uint32_t* abort_flag = &sm->abort_flag;
   const int n_units = p.B * p.H;
   const int n_my = (n_units - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);   // units u = blockIdx.x + i * gridDim.x
   auto unit_of = [&](int i) { return int(blockIdx.x) + i * int(gridDim.x); };
@@ -994,9 +1003,18 @@ attn_decode_stream_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
     mbar_arrive_expect_tx(smem_u32(&sm->full[s]), DEC_TILE_BYTES);
     bulk_load_1d(smem_u32(sm->tile[s]), p.s_in + size_t(unit_of(i)) * D * D, DEC_TILE_BYTES, smem_u32(&sm->full[s]));
   };
-  if (t == 0) {
-    for (int i = 0; i < DEC_STAGES && i < n_my; ++i) issue_load(i);
-  }
+  auto issue_first = [&]() {
+    if (t == 0) {
+      for (int i = 0; i < DEC_STAGES && i < n_my; ++i) issue_load(i);
+    }
+  };
+  if (p.settled) issue_first();      // the first state tiles travel while the projection still runs
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+  if (!p.settled) issue_first();
+  __syncthreads();
+  volatile uint32_t* abort_flag = &sm->abort_flag;
   // feature map + RoPE of the token of unit i into buffer i & 1: threads 0..31 the q / k pairs (d, d + 32), 32..95 v
   auto token_features = [&](int i) {
     if (t >= 96) return;
@@ -1008,8 +1026,8 @@ attn_decode_stream_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
       int pos = p.pos0 ? p.pos0[b] : p.pos0_scalar;
       pos = pos < 0 ? 0 : (pos >= p.n_pos ? p.n_pos - 1 : pos);
       const float c = __ldg(p.cos_tab + size_t(pos) * 32 + t), sn = __ldg(p.sin_tab + size_t(pos) * 32 + t);
-      sm->rq[buf][t] = q0 * c - q1 * sn;  sm->rq[buf][t + 32] = q1 * c + q0 * sn;
-      sm->rk[buf][t] = k0 * c - k1 * sn;  sm->rk[buf][t + 32] = k1 * c + k0 * sn;
+      sm->rq[buf][t] = rope_lo(q0, q1, c, sn);  sm->rq[buf][t + 32] = rope_hi(q0, q1, c, sn);
+      sm->rk[buf][t] = rope_lo(k0, k1, c, sn);  sm->rk[buf][t + 32] = rope_hi(k0, k1, c, sn);
     } else {
       sm->sv[buf][t - 32] = __bfloat162float(v[off + t - 32]);
     }
@@ -1109,7 +1127,7 @@ size_t attn_scan_scratch_bytes(int B, int T, int H) {
 int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, const float* gamma,
                      const float* cos_tab, const float* sin_tab, int n_pos, const int32_t* pos0, int pos0_scalar,
                      const float* s_in, void* o, int ld_o, float* s_out, void* scratch, int B, int T, int H,
-                     int head_dim, int flags, cudaStream_t stream) {
+                     int head_dim, int flags, cudaStream_t stream, bool settled) {
   JB_REQUIRE((flags & ~JB200_ATTN_QK_PREPARED) == 0, "attn_scan: unknown flags %d", flags);
   JB_REQUIRE(!(flags & JB200_ATTN_QK_PREPARED) || T > 1, "attn_scan: prepared q/k is for T > 1 (single-token steps take raw q, k)");
   JB_REQUIRE(head_dim == D, "attn_scan: head_dim (%d) must be %d", head_dim, D);
@@ -1134,7 +1152,7 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
     dp.gamma = gamma; dp.cos_tab = cos_tab; dp.sin_tab = sin_tab; dp.pos0 = pos0; dp.pos0_scalar = pos0_scalar;
     dp.n_pos = n_pos; dp.s_in = s_in; dp.s_out = s_out; dp.o = reinterpret_cast<__nv_bfloat16*>(o); dp.ld_o = ld_o;
     dp.B = B; dp.T = 1; dp.H = H; dp.seg_chunks = 1; dp.nseg = 1; dp.seg_state = nullptr; dp.n_pieces = 0; dp.qk_prepared = 0;
-    dp.wide_store = 0; dp.status = device_status_ptr();
+    dp.wide_store = 0; dp.settled = settled ? 1 : 0; dp.status = device_status_ptr();
     if (!dp.status) return JB200_ERR_CUDA;
     if (s_in && s_out && B * H >= 64) {
       // the state streams through shared memory as bulk copies: two CTAs per SM walk the (sequence, head) pairs

@@ -48,6 +48,19 @@ struct Workspace {
   }
 };
 
+// Which form of the ternary product a call of so many tokens runs (their results are the same bits): up to 16 tokens
+// mma.sync straight from the codes (24 layers of single-token steps 0.62 against 0.86 ms at 1 sequence, equal at 16), up to
+// MID_TOKENS the tcgen05 form that is built for latency (256 tokens 1.90 against 2.12 ms, 512 2.46 against 2.57, 777 2.91
+// against 2.86), beyond that the persistent pipeline.
+constexpr int SMALL_TOKENS = 16, MID_TOKENS = 640;
+// Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
+// tokens) that leaves the launch one wave.
+inline int mid_tile(int rows, int n_ft, int groups, int sms) {
+  int bn = rows <= 64 ? (rows + 15) / 16 * 16 : 64;
+  while (bn < 256 && long(n_ft) * groups * ((rows + bn - 1) / bn) > sms) bn += 16;
+  return bn;
+}
+
 #define JB_TRY(call)                    \
   do {                                  \
     const int rc__ = (call);            \
@@ -55,6 +68,8 @@ struct Workspace {
   } while (0)
 
 }  // namespace
+
+size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(E + 1) * 4 + 7) / 8 * 8; }
 
 size_t routing_layout(int N, int E, size_t* offsets) {
   const Routing r(N > 0 ? N : 0, E > 0 ? E : 0);
@@ -76,7 +91,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   JB_REQUIRE(B >= 1 && T >= 1 && size_t(B) * T < (size_t(1) << 30), "forward_layers: bad shape (B=%d, T=%d)", B, T);
   JB_REQUIRE(C % 128 == 0 && C <= 1024 && C == 64 * H && hidden % 128 == 0 && (E == 4 || E == 8),
              "forward_layers: d_model %d / heads %d / hidden %d / experts %d not supported", C, H, hidden, E);
-  JB_REQUIRE(f->x && f->cos_tab && f->sin_tab && f->h_out && f->acc && f->hist && f->scalars && f->routing && f->workspace,
+  JB_REQUIRE(f->x && f->cos_tab && f->sin_tab && f->h_out && f->accumulators && f->scalars && f->routing && f->workspace,
              "forward_layers: null pointer");
   JB_REQUIRE((f->w_final == nullptr) == (f->hidden_out == nullptr), "forward_layers: w_final and hidden_out come together");
   const int N = B * T;
@@ -88,16 +103,28 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   uint16_t *y = reinterpret_cast<uint16_t*>(w + ws.y), *out = reinterpret_cast<uint16_t*>(w + ws.out);
   uint16_t* disp = qkv;
   float* x = f->x;
+  const bool small = N <= SMALL_TOKENS;
+  const bool mid = !small && N <= MID_TOKENS;
+  const int sms = sm_count();
+  if (sms <= 0) return JB200_ERR_CUDA;
+  // an expert sees about half of the tokens: tiles and their stride for that, more tiles are looped over
+  const int half = N <= 32 ? N : (N + 1) / 2 + N / 16;
+  auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
+                      const int32_t* seg, const int64_t* ids, const int32_t* sc, int epi, void* dst, bool seg_settled) {
+    const int rows = seg ? half : M;
+    const int bn = mid_tile(rows, n_out / 128, G, sms);
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, (rows + bn - 1) / bn, true, seg_settled, st);
+  };
 
-  const size_t acc_bytes = size_t(n_layers) * (2 + E) * sizeof(double), hist_bytes = size_t(n_layers) * E * sizeof(int32_t);
-  if (reinterpret_cast<uint8_t*>(f->acc) + acc_bytes == reinterpret_cast<uint8_t*>(f->hist)) {
-    JB_CUDA(cudaMemsetAsync(f->acc, 0, acc_bytes + hist_bytes, st));
+  // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
+  uint8_t* acc0 = static_cast<uint8_t*>(f->accumulators);
+  const size_t acc_stride = accumulator_bytes(E);
+  if (f->ids) {
+    JB_TRY(launch_embed_norm(f->ids, f->table, f->vocab, layers[0].w_norm1, layers[0].eps1, x, xn, N, C, acc0, n_layers * acc_stride, st));
   } else {
-    JB_CUDA(cudaMemsetAsync(f->acc, 0, acc_bytes, st));
-    JB_CUDA(cudaMemsetAsync(f->hist, 0, hist_bytes, st));
+    JB_CUDA(cudaMemsetAsync(acc0, 0, n_layers * acc_stride, st));
+    JB_TRY(launch_rmsnorm(x, 0, layers[0].w_norm1, layers[0].eps1, xn, 1, N, C, st));
   }
-  if (f->ids) JB_TRY(launch_embedding(f->ids, f->table, f->vocab, x, N, C, st));
-  JB_TRY(launch_rmsnorm(x, 0, layers[0].w_norm1, layers[0].eps1, xn, 1, N, C, st));
 
   for (int l = 0; l < n_layers; ++l) {
     const jb200_layer& p = layers[l];
@@ -107,8 +134,9 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const float* h_in = f->h_in ? f->h_in[l] : nullptr;
     float* h_out = f->h_out[l];
     JB_REQUIRE(h_out != nullptr, "forward_layers: h_out of layer %d missing", l);
-    double* acc = f->acc + size_t(l) * (2 + E);
-    int32_t* hist = f->hist + size_t(l) * E;
+    double* acc = reinterpret_cast<double*>(acc0 + l * acc_stride);            // sum, sum of squares, P_e
+    int32_t* hist = reinterpret_cast<int32_t*>(acc + 2 + E);                   // top-1 counts
+    int32_t* ticket = hist + E;
     float* scalars = f->scalars + size_t(l) * 3;
     uint8_t* r = static_cast<uint8_t*>(f->routing) + size_t(l) * rl.bytes;
     int64_t* idx = reinterpret_cast<int64_t*>(r + rl.idx);
@@ -118,28 +146,61 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     int* gate_idx = reinterpret_cast<int*>(r + rl.gate_idx);
 
     // x += attn(norm1(x))
-    JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st));
+    if (small)
+      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, N, true, st));
+    else if (mid)
+      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, false));
+    else
+      JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
     void* attn_scratch = (T > 1 && !(s_in && s_in == s_out)) ? w + ws.attn : nullptr;
     if (attn_scratch && ws.attn == ws.lsf) attn_scratch = nullptr;            // no scratch wanted at this shape
     JB_TRY(launch_attn_scan(qkv, qkv + C, qkv + 2 * C, 3 * C, p.gamma, f->cos_tab, f->sin_tab, f->n_pos, f->pos0, f->pos0_scalar,
-                            s_in, o, C, s_out, attn_scratch, B, T, H, 64, 0, st));
-    JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st));
+                            s_in, o, C, s_out, attn_scratch, B, T, H, 64, 0, st, true));
+    if (small)
+      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, N, true, st));
+    else if (mid)
+      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, false));
+    else
+      JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st));
 
     // moe(norm2(x))
-    JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st));
-    JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
-    JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
-    JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st));
-    JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st));
-    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st));
+    if (N <= ROUTE_SMALL_MAX) {
+      JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, ticket, counts, offs,
+                                scatter, gather, gate_idx, st));
+      // every expert takes all rows where they are and stores the routed ones: no dispatch
+      if (small)
+        JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, N, true, st));
+      else
+        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, false));
+    } else {
+      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st));
+      JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
+      JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
+      if (mid)
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid, true));
+      else
+        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st));
+    }
+    if (small)
+      JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, N, true, st));
+    else if (mid)
+      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, true));
+    else
+      JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st));
 
-    // x += lsf(moe), and the norm of what follows
+    // combine, x += lsf(moe), and the norm of what follows
     const float* w_next = last ? f->w_final : layers[l + 1].w_norm1;
     const float eps_next = last ? f->eps_final : layers[l + 1].eps1;
     void* xn_next = last ? f->hidden_out : static_cast<void*>(xn);
     const LsfStats stats = {acc, acc + 2, hist, E, N, (long long)N * C, p.balance_alpha, scalars,
                             p.mu, p.reflect_lam, p.reflect_tau, (f->reflect && p.mu) ? f->reflect + l : nullptr};
+    if (N <= tail_max_tokens(C, T)) {
+      JB_TRY(launch_tail(y, gates, scatter, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
+                         w_next ? xn_next : nullptr, B, T, C, st));
+      continue;
+    }
+    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st));
     if (T == 1) {
       JB_TRY(launch_lsf_step_norm(out, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
                                   w_next ? xn_next : nullptr, B, C, st));

@@ -25,6 +25,18 @@ struct GemmRope {
 int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packed, const float* alpha,
                         int alpha_rows, int N, int G, const int32_t* seg_offsets, int epilogue, void* out,
                         int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope = nullptr);
+// The same product for a few tokens (small_gemm.cu), bit for bit.  idx / scatter ([M][2]): all M rows go through every group's
+// matrix and row n is stored at scatter[2n + k] where idx[2n + k] is the group; else seg as above.  tokens: about how many
+// rows a call holds (chooses the tile).  settled: weights and seg were complete before the kernel ahead of this one on the
+// stream began, so they may be read while it runs.
+int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
+                      int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
+                      int tokens, bool settled, cudaStream_t stream);
+// The same product again, latency form on tcgen05 (mid_gemm.cu): grid (N / 128, G, z), every CTA takes every z-th tile of
+// bn tokens of its group.  Arguments as launch_small_gemm.
+int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int z,
+                    bool settled, bool seg_settled, cudaStream_t stream);
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);
 void decode16_prepared_host(uint32_t w_canonical, uint32_t* out8);
@@ -76,14 +88,28 @@ int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* va
                          const float* h_in, float* h_out, float* x, const float* w_norm, float eps, void* xn_bf16, int B,
                          int C, cudaStream_t stream);
 
+// settled (T == 1): s_in and pos0 were complete before the kernel ahead of this one on the stream began.
 int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, const float* gamma,
                      const float* cos_tab, const float* sin_tab, int n_pos, const int32_t* pos0, int pos0_scalar,
                      const float* s_in, void* o, int ld_o, float* s_out, void* scratch, int B, int T, int H,
-                     int head_dim, int flags, cudaStream_t stream);
+                     int head_dim, int flags, cudaStream_t stream, bool settled = false);
 size_t attn_scan_scratch_bytes(int B, int T, int H);
 
+// Few tokens (moe_small.cu).
+constexpr int ROUTE_SMALL_MAX = 64;    // tokens
+constexpr int TAIL_MAX = 128;          // tokens: a warp each in the eight CTAs of a cluster
+int tail_max_tokens(int C, int T);     // tokens launch_tail takes at this width
+int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const float* w_norm, float eps, float* x, void* xn_bf16,
+                      int n_rows, int C, void* zero, size_t zero_bytes, cudaStream_t stream);
+int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router, int N, int C, int E,
+                       int64_t* idx, float* gates, double* probs_sum, int* hist, int* ticket, int* counts, int* offsets,
+                       int* scatter, int* gather, int* gate_idx, cudaStream_t stream);
+int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const LsfStats& st, const float* var_scale,
+                float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x, const float* w_norm, float eps,
+                void* xn_bf16, int B, int T, int C, cudaStream_t stream);
 int launch_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
                          const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, cudaStream_t stream);
+size_t accumulator_bytes(int E);
 size_t routing_layout(int N, int E, size_t* offsets);
 size_t forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden);
 int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, cudaStream_t stream);

@@ -1,0 +1,309 @@
+// Ternary linear layers for up to a few hundred tokens on the 5th-generation tensor cores: the latency form of
+// ternary_gemm_kernel.
+//
+// With one or two tiles per SM nothing amortises a pipeline's fill: ternary_gemm_kernel takes 11-18 us for products whose
+// arithmetic is ~1 us, because every K-block of its four-stage ring waits for a code load from L2, the decode, the MMA
+// and the stage's release one after another (~550 cycles), after TMEM, barriers and tensor maps have been set up.  Here
+//   - a CTA owns (out-feature tile, expert) and takes token tiles from a stride, so its weights are known from the grid: in
+//     a chain their codes are loaded and decoded into every stage there is before the grid dependency is waited for;
+//   - K-blocks travel in chunks of CK: one TMA copy, one barrier wait and one commit per chunk (issued singly they cost
+//     ~290, ~95 and ~100 cycles next to 4 x 40-48 cycles for a K-block's MMAs), with as many chunks in flight as fit
+//     (a smaller ring that lets two CTAs share an SM and prologues overlap measured 5-15 % slower);
+//   - code loads run four chunks ahead in registers that are never moved (a move waits for the load);
+//   - the eight decoder warps become the epilogue; the residual is added by reductions, nothing waits for old values.
+// What is left is the chain itself: 4 x 40-48 cycles per K-block.  Accumulation is the same chain of K = 16 steps as in
+// ternary_gemm_kernel: results are its bit for bit.
+#include "common.cuh"
+#include "gemm_shared.cuh"
+#include "launchers.h"
+
+namespace jb {
+
+namespace {
+
+constexpr int BM = 128, BK = 64, A_BYTES = BM * BK * 2;
+constexpr int CK = 2;                          // K-blocks per chunk (four: 1-3 % slower, the ring gets too coarse)
+constexpr int MAX_CHUNKS = 6, DEC_WARP0 = 2, THREADS = 320;
+constexpr int SLOTS = 4;                       // chunks whose codes are in registers
+
+struct MidParams {
+  const uint8_t* w;            // prepared [G][N][K/4]
+  const float* alpha;          // [G][N / alpha_rows]
+  const int32_t* seg;          // device [G+1] or null (every group takes rows [0, M))
+  const int64_t* idx;          // [M][2]: row n of group g goes to out row scatter[2n + k] where idx[2n + k] == g; null: row n
+  const int32_t* scatter;
+  void* out;
+  int M, N, K, alpha_rows, bn, chunks, epilogue;
+  int settled, seg_settled;    // weights / segments were complete before the kernel ahead of this one started
+  uint32_t tmem_cols;
+  unsigned int* status;
+};
+
+struct Ctl {
+  uint64_t full[MAX_CHUNKS], empty[MAX_CHUNKS], acc_full, acc_empty;
+  uint32_t tmem_base, abort_flag;
+};
+
+__global__ void __launch_bounds__(THREADS, 1)
+mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Ctl ctl;
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  const uint32_t base = (raw_addr + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - raw_addr);
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int S = p.chunks, n_ch = p.K / (BK * CK);
+  const uint32_t kb_bytes = uint32_t(p.bn) * BK * 2, b_bytes = kb_bytes * CK;
+  const uint32_t b_base = base + uint32_t(S) * (CK * A_BYTES);
+  const int ft = blockIdx.x, grp = blockIdx.y;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(smem_u32(&ctl.full[s]), 1 + 8);      // the producer's expectation and the eight decoder warps
+      mbar_init(smem_u32(&ctl.empty[s]), 1);
+    }
+    mbar_init(smem_u32(&ctl.acc_full), 1);
+    mbar_init(smem_u32(&ctl.acc_empty), 8);
+    ctl.abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 0) {
+    __syncwarp();                 // tcgen05.alloc is warp-collective: lane 0 rejoins from the barrier set-up first
+    tmem_alloc(smem_u32(&ctl.tmem_base), p.tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = ctl.tmem_base;
+  volatile uint32_t* abort_flag = &ctl.abort_flag;
+  int beg = 0, end = p.M;
+  auto segment = [&]() {
+    if (p.seg) {
+      beg = min(max(__ldg(p.seg + grp), 0), p.M);
+      end = min(max(__ldg(p.seg + grp + 1), 0), p.M);
+    }
+  };
+
+  if (warp == 0) {
+    // ---------------- TMA producer ----------------
+    if (p.seg_settled) segment();
+    pdl_wait();
+    pdl_trigger();
+    if (!p.seg_settled) segment();
+    int s = 0;
+    uint32_t ph = 1u;
+    bool ok = true;
+    for (int tok0 = beg + int(blockIdx.z) * p.bn; ok && tok0 < end; tok0 += int(gridDim.z) * p.bn) {
+#pragma unroll 1
+      for (int c = 0; c < n_ch; ++c) {
+        const uint32_t full = smem_u32(&ctl.full[s]);
+        if (!mbar_wait(smem_u32(&ctl.empty[s]), ph, abort_flag, p.status, JB200_STATUS_GEMM_PRODUCER)) { ok = false; break; }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(full, b_bytes);
+          tma_load_3d(b_base + uint32_t(s) * b_bytes, &tmap_x, 0, tok0, c * CK, full);
+        }
+        __syncwarp();
+        if (++s == S) { s = 0; ph ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    if (p.seg_settled) segment();
+    pdl_wait();
+    pdl_trigger();
+    if (!p.seg_settled) segment();
+    const uint32_t idesc = umma_idesc_bf16(BM, p.bn);
+    const uint64_t adesc0 = umma_desc_k_sw128(base), bdesc0 = umma_desc_k_sw128(b_base);
+    uint64_t ad = adesc0, bd = bdesc0;
+    int s = 0;
+    uint32_t ph = 0u, tile = 0u;
+    bool ok = true;
+    for (int tok0 = beg + int(blockIdx.z) * p.bn; ok && tok0 < end; tok0 += int(gridDim.z) * p.bn, ++tile) {
+      if (!mbar_wait(smem_u32(&ctl.acc_empty), (tile & 1u) ^ 1u, abort_flag, p.status, JB200_STATUS_GEMM_MMA)) break;
+      tc_fence_after_sync();
+#pragma unroll 1
+      for (int c = 0; c < n_ch; ++c) {
+        if (!mbar_wait(smem_u32(&ctl.full[s]), ph, abort_flag, p.status, JB200_STATUS_GEMM_MMA)) { ok = false; break; }
+        tc_fence_after_sync();
+        if (elect_one()) {
+#pragma unroll
+          for (int j = 0; j < CK; ++j) {
+            const uint64_t aj = ad + uint64_t(j) * (A_BYTES >> 4), bj = bd + uint64_t(j) * (kb_bytes >> 4);
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; ++kk)
+              umma_bf16_ss(tmem, aj + uint64_t(kk * 2), bj + uint64_t(kk * 2), idesc, (c | j | kk) != 0 ? 1u : 0u);
+          }
+          umma_commit(smem_u32(&ctl.empty[s]));
+          if (c + 1 == n_ch) umma_commit(smem_u32(&ctl.acc_full));
+        }
+        __syncwarp();
+        ad += (CK * A_BYTES) >> 4;
+        bd += b_bytes >> 4;
+        if (++s == S) { s = 0; ph ^= 1u; ad = adesc0; bd = bdesc0; }
+      }
+    }
+  } else {
+    // ---------------- decoders, then epilogue ----------------
+    const int par = (warp - DEC_WARP0) >> 2;                       // this thread decodes K-block par of every chunk,
+    const int r = ((warp - DEC_WARP0) & 3) * 32 + lane;             // weight row r of the tile
+    const uint8_t* wrow = p.w + (size_t(grp) * p.N + size_t(ft) * BM + r) * (size_t(p.K) / 4) + par * 16;
+    const uint32_t swz = uint32_t(r & 7);
+    uint4 code[SLOTS];
+    auto load_codes = [&](int u, int c) {
+      code[u] = c < n_ch ? __ldg(reinterpret_cast<const uint4*>(wrow + size_t(c * CK) * 16)) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    auto put = [&](const uint4& cw, uint8_t* arow) {       // 64 codes -> one swizzled 128-byte row
+      const uint32_t words[4] = {cw.x, cw.y, cw.z, cw.w};
+#pragma unroll
+      for (int wi = 0; wi < 4; ++wi) {
+        uint32_t v[8];
+        decode16_prepared(words[wi], v);
+        *reinterpret_cast<uint4*>(arow + ((uint32_t(2 * wi) ^ swz) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<uint4*>(arow + ((uint32_t(2 * wi + 1) ^ swz) << 4)) = make_uint4(v[4], v[5], v[6], v[7]);
+      }
+    };
+    // Chunk c of a tile goes to ring slot and phase of the running count over all tiles; code[c % SLOTS] is its codes.
+    int c = 0, s = 0;
+    uint32_t ph = 1u;
+    bool ok = true;
+    auto start_codes = [&]() {
+#pragma unroll
+      for (int u = 0; u < SLOTS; ++u) load_codes(u, u);
+    };
+    auto decode_to = [&](int limit, bool fresh) {
+#pragma unroll 1
+      while (c < limit) {
+#pragma unroll
+        for (int u = 0; u < SLOTS; ++u) {            // c % SLOTS == u: entered in the middle after an earlier call
+          if ((c & (SLOTS - 1)) != u || c >= limit) continue;
+          if (!fresh && !mbar_wait(smem_u32(&ctl.empty[s]), ph, abort_flag, p.status, JB200_STATUS_GEMM_DECODE)) { ok = false; c = limit; break; }
+          put(code[u], smem + size_t(s) * (CK * A_BYTES) + size_t(par) * A_BYTES + size_t(r) * 128);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&ctl.full[s]));
+          load_codes(u, c + SLOTS);
+          ++c;
+          if (++s == S) { s = 0; ph ^= 1u; }
+        }
+      }
+    };
+    const int fresh = S < n_ch ? S : n_ch;           // chunks that go into unused slots
+    if (p.settled) {
+      start_codes();
+      decode_to(fresh, true);
+    }
+    const float alpha = 0.5f * __ldg(p.alpha + size_t(grp) * (p.N / p.alpha_rows) + (ft * BM) / p.alpha_rows);   // codes decode to +-2
+    if (p.seg_settled) segment();
+    __syncwarp();
+    pdl_wait();
+    pdl_trigger();
+    if (!p.settled) {
+      start_codes();
+      decode_to(fresh, true);
+    }
+    if (!p.seg_settled) segment();
+    const int q4 = warp & 3;                         // TMEM lane quadrant of this warp
+    const int f0 = ft * BM + q4 * 32;
+    uint32_t tile = 0u;
+    for (int tok0 = beg + int(blockIdx.z) * p.bn; ok && tok0 < end; tok0 += int(gridDim.z) * p.bn, ++tile) {
+      if (tile > 0) {                                // a further tile: the same weights again
+        c = 0;
+        start_codes();
+      }
+      decode_to(n_ch, false);
+      if (!ok) break;
+      const int n = min(p.bn, end - tok0);
+      if (!mbar_wait(smem_u32(&ctl.acc_full), tile & 1u, abort_flag, p.status, JB200_STATUS_GEMM_EPILOGUE)) break;
+      tc_fence_after_sync();
+      __syncwarp();
+#pragma unroll 1
+      for (int c0 = par * 32; c0 < n; c0 += 64) {
+        // output row of token c0 + lane; -1: not stored
+        int row = c0 + lane < n ? tok0 + c0 + lane : -1;
+        if (p.idx && row >= 0) {
+          const longlong2 e = *reinterpret_cast<const longlong2*>(p.idx + 2 * row);
+          const int2 sc = *reinterpret_cast<const int2*>(p.scatter + 2 * row);
+          row = e.x == grp ? sc.x : (e.y == grp ? sc.y : -1);
+          if (row >= 2 * p.M) row = -1;
+        }
+        __syncwarp();
+        uint32_t v[32];
+        tmem_ld_32x32(tmem + (uint32_t(q4 * 32) << 16) + uint32_t(c0), v);
+        tmem_ld_wait();
+        if (p.epilogue == JB200_EPI_RESID_F32 || p.epilogue == JB200_EPI_F32) {
+          // lane = feature: a warp instruction covers 128 bytes of one token's row
+          float* o = reinterpret_cast<float*>(p.out) + f0 + lane;
+          const bool resid = p.epilogue == JB200_EPI_RESID_F32;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const int rj = __shfl_sync(0xffffffffu, row, j);
+            const float val = alpha * __uint_as_float(v[j]);
+            if (rj >= 0) {
+              if (resid) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + size_t(rj) * p.N), "f"(val) : "memory");
+              else o[size_t(rj) * p.N] = val;
+            }
+          }
+        } else {
+          const bool gelu = p.epilogue == JB200_EPI_GELU_BF16;
+          const int odd = lane & 1;
+          __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + f0 + (lane & ~1);
+#pragma unroll
+          for (int jj = 0; jj < 16; ++jj) {
+            float a = alpha * __uint_as_float(v[2 * jj]), b = alpha * __uint_as_float(v[2 * jj + 1]);
+            if (gelu) { a = gelu_erf(a); b = gelu_erf(b); }
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+            const uint32_t w2 = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);   // features (f & ~1, f | 1)
+            const int rj = __shfl_sync(0xffffffffu, row, 2 * jj + odd);            // token 2jj (even lanes) / 2jj + 1 (odd)
+            if (rj >= 0) *reinterpret_cast<uint32_t*>(o + size_t(rj) * p.N) = w2;
+          }
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl.acc_empty));
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, p.tmem_cols);
+  }
+}
+
+}  // namespace
+
+int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int z,
+                    bool settled, bool seg_settled, cudaStream_t stream) {
+  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn <= 256 && bn % 16 == 0 && z >= 1,
+             "mid_gemm: bad shape (M=%d, N=%d, K=%d, bn=%d)", M, N, K, bn);
+  MidParams p;
+  p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
+  p.M = M; p.N = N; p.K = K; p.alpha_rows = alpha_rows; p.bn = bn; p.epilogue = epilogue;
+  p.settled = settled ? 1 : 0;
+  p.seg_settled = seg_settled ? 1 : 0;
+  p.tmem_cols = bn <= 32 ? 32u : bn <= 64 ? 64u : bn <= 128 ? 128u : 256u;
+  p.status = device_status_ptr();
+  if (!p.status) return JB200_ERR_CUDA;
+  const int n_kb = K / BK, kb_bytes = A_BYTES + bn * BK * 2;
+  int S = (224 * 1024) / (CK * kb_bytes);
+  if (S > MAX_CHUNKS) S = MAX_CHUNKS;
+  if (S > n_kb / CK) S = n_kb / CK;
+  p.chunks = S;
+  CUtensorMap tmap;                            // [K-block][token][64]: one copy takes the same rows of CK K-blocks
+  const cuuint64_t gdim[3] = {cuuint64_t(BK), cuuint64_t(M), cuuint64_t(n_kb)};
+  const cuuint64_t gstride[2] = {cuuint64_t(K) * 2, cuuint64_t(BK) * 2};
+  const cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(bn), cuuint32_t(CK)};
+  const int rc = encode_tiled(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, x_bf16, gdim, gstride, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "mid_gemm");
+  if (rc != JB200_OK) return rc;
+  JB_MAX_SMEM(mid_gemm_kernel, 225 * 1024);
+  launch_dep(mid_gemm_kernel, dim3(N / BM, G, z), THREADS, size_t(S) * CK * kb_bytes + 1024, stream, tmap, p);
+  JB_LAUNCH_CHECK("mid_gemm_kernel");
+  return JB200_OK;
+}
+
+}  // namespace jb

@@ -32,6 +32,14 @@ __device__ __forceinline__ void moe_finalize_scalars(const double* stats, const 
   }
 }
 
+// l_balance alone, with the divisions by the token count taken out of the loop (for kernels whose last microsecond it is).
+__device__ __forceinline__ float moe_l_balance(const double* probs_sum, const int* top1_hist, int E, double inv_tokens,
+                                               float balance_alpha) {
+  double acc = 0.0;
+  for (int e = 0; e < E; ++e) acc += double(top1_hist[e]) * probs_sum[e];
+  return float(double(balance_alpha) * double(E) * (acc * inv_tokens * inv_tokens));
+}
+
 // ReflectivePenalty of a layer (jarvis_model.py:329-351): lam * ((mu - act_mean)^2 + relu(act_var - tau)).
 __device__ __forceinline__ float reflect_penalty(float lam, float tau, float mu, float mean, float var) {
   const float d = mu - mean, e = var - tau;

@@ -1,0 +1,602 @@
+// The glue of a block for few tokens (decode steps of small batches, short prompts), where every launch is latency: two
+// kernels in the place of five.
+//
+//   route_small_kernel  norm2 + top-2 router (jarvis_model.py:25-26, :218-224), a warp per token; the warp that finishes
+//                       last also makes the dispatch maps (sparse_model.cu:23-90)
+//   tail_step_kernel, tail_scan_kernel  combine of the expert rows, MoE statistics, LSF scan, residual add and the RMSNorm
+//                       that follows (sparse_model.cu:117-165, jarvis_model.py:244-250, :281-314, :430-436) in one
+//                       thread-block cluster: the decay of the scan depends on the variance of ALL combined rows, and
+//                       a cluster barrier does what the boundaries of two or three kernels (6 + 9 us, 6 + 8 + 5 us) did.
+// Everything a kernel needs that its predecessor on the stream did not make is fetched before the grid dependency is
+// waited for.  Every value is rounded and every sum ordered as in the kernels these stand for (rmsnorm_router_kernel,
+// meta_small_kernel, scatter_combine_kernel, lsf_step_norm_kernel, lsf_tma_kernel, lsf_short_kernel, rmsnorm_kernel): the
+// results are theirs bit for bit, so that a token's experts do not depend on how many others share its call.
+#include "common.cuh"
+#include "moe_finalize.cuh"
+#include "moe_router.cuh"
+#include "launchers.h"
+
+namespace jb {
+
+namespace {
+
+// Channel of element j of group i of a lane in the row kernels: (32 i + lane) * 8 + j, four groups for C = 1024.
+constexpr int GROUPS = 4;
+
+__device__ __forceinline__ void load8(const float* src, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void store8(float* dst, const float (&v)[8]) {
+  *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ uint4 norm8(const float (&v)[8], float r, float4 wa, float4 wb) {
+  return make_uint4(pack_bf16x2(v[0] * r * wa.x, v[1] * r * wa.y), pack_bf16x2(v[2] * r * wa.z, v[3] * r * wa.w),
+                    pack_bf16x2(v[4] * r * wb.x, v[5] * r * wb.y), pack_bf16x2(v[6] * r * wb.z, v[7] * r * wb.w));
+}
+
+struct RouteParams {
+  const float* x;              // [N][C]
+  const float* w_norm;
+  const float* w_router;       // [E][C]
+  __nv_bfloat16* xn;           // [N][C] out
+  int64_t* idx;                // [N][2]
+  float* gates;                // [N][2]
+  double* probs_sum;           // [E] accumulated
+  int* hist;                   // [E] accumulated
+  int* ticket;                 // zero on entry
+  int *counts, *offsets, *scatter, *gather, *gate_idx;
+  float eps;
+  int N, C;
+};
+
+// One warp per token and CTA: with all weights of the lane's channels in registers before the residual row arrives, the
+// chain is load - sum - norm - dot - sums - softmax.
+template <int E>
+__global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
+  __shared__ int h_acc[E];
+  const int lane = threadIdx.x, tok = blockIdx.x;
+  constexpr bool AHEAD = E <= 4;                 // eight experts' weights do not fit the registers: read where used
+  float wn[GROUPS][8];
+  float4 wr[GROUPS][AHEAD ? E : 1][2];
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < p.C) {
+      load8(p.w_norm + c, wn[i]);
+#pragma unroll
+      for (int e = 0; AHEAD && e < E; ++e) {
+        wr[i][e][0] = __ldg(reinterpret_cast<const float4*>(p.w_router + size_t(e) * p.C + c));
+        wr[i][e][1] = __ldg(reinterpret_cast<const float4*>(p.w_router + size_t(e) * p.C + c) + 1);
+      }
+    }
+  }
+  if (lane < E) h_acc[lane] = 0;
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+
+  float v[GROUPS][8], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < p.C) load8(p.x + size_t(tok) * p.C + c, v[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    if ((i * 32 + lane) * 8 < p.C) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss = __fmaf_rn(v[i][j], v[i][j], ss);
+    }
+  }
+  ss = warp_sum(ss);
+  const float r = rsqrtf(ss / float(p.C) + p.eps);
+  float acc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = 0.f;
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < p.C) {
+      const uint4 pk = norm8(v[i], r, make_float4(wn[i][0], wn[i][1], wn[i][2], wn[i][3]),
+                             make_float4(wn[i][4], wn[i][5], wn[i][6], wn[i][7]));
+      *reinterpret_cast<uint4*>(p.xn + size_t(tok) * p.C + c) = pk;
+      const float xv[8] = {bf16_lo(pk.x), bf16_hi(pk.x), bf16_lo(pk.y), bf16_hi(pk.y),
+                           bf16_lo(pk.z), bf16_hi(pk.z), bf16_lo(pk.w), bf16_hi(pk.w)};
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const float4* w = reinterpret_cast<const float4*>(p.w_router + size_t(e) * p.C + c);
+        acc[e] = AHEAD ? router_dot(acc[e], xv, wr[i][AHEAD ? e : 0][0], wr[i][AHEAD ? e : 0][1])
+                       : router_dot(acc[e], xv, __ldg(w), __ldg(w + 1));
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = warp_sum(acc[e]);
+  float pr[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) pr[e] = 0.f;
+  router_finish<E>(acc, lane, tok, p.idx, p.gates, nullptr, h_acc, pr);       // pr: the probabilities, in lane 0
+  int last = 0;
+  if (lane == 0) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      atomicAdd(p.probs_sum + e, double(pr[e]));
+      if (h_acc[e]) atomicAdd(p.hist + e, 1);
+    }
+    __threadfence();
+    last = atomicAdd(p.ticket, 1) == p.N - 1;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  // the last warp: stable counting sort of the 2 N assignments by expert, 32 at a time
+  __threadfence();
+  const int M = 2 * p.N;
+  const long long* ids = reinterpret_cast<const long long*>(p.idx);
+  int n_of = 0;                                  // lane e < E: assignments of expert e
+  for (int m0 = 0; m0 < M; m0 += 32) {
+    const int e = m0 + lane < M ? int(__ldcg(ids + m0 + lane)) : -1;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+      const unsigned b = __ballot_sync(0xffffffffu, e == q);
+      if (lane == q) n_of += __popc(b);
+    }
+  }
+  int incl = n_of;
+#pragma unroll
+  for (int o = 1; o < E; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  int at = incl - n_of;                          // lane e: next free slot of expert e
+  if (lane < E) {
+    p.counts[lane] = n_of;
+    p.offsets[lane] = at;
+    if (lane == E - 1) p.offsets[E] = incl;
+  }
+  for (int m0 = 0; m0 < M; m0 += 32) {
+    const int m = m0 + lane;
+    const int e = m < M ? int(__ldcg(ids + m)) : -1;
+    int slot = 0;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+      const unsigned b = __ballot_sync(0xffffffffu, e == q);
+      const int base = __shfl_sync(0xffffffffu, at, q);
+      if (e == q) slot = base + __popc(b & ((1u << lane) - 1u));
+      if (lane == q) at += __popc(b);
+    }
+    if (m < M) {
+      p.scatter[m] = slot;
+      p.gather[slot] = m >> 1;
+      p.gate_idx[slot] = m & 1;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+struct TailParams {
+  const __nv_bfloat16* y;      // [2N][C] expert outputs in dispatch order: the only input the kernel before this one made
+  const float* gates;          // [N][2]
+  const int* scatter;          // [N][2]
+  LsfStats st;                 // stats is not read: the sums are made here
+  double inv_tokens;
+  const float* var_scale;
+  float alpha_min, alpha_max;
+  const float* h_in;           // [B][C] or null
+  float* h_out;                // [B][C], may be h_in
+  float* x;                    // [N][C] residual stream
+  const float* w_norm;         // [C] or null
+  float eps;
+  __nv_bfloat16* xn;           // [N][C]
+  int B, T, N, C;
+};
+
+constexpr int MAX_CTAS = 8;
+constexpr int MAX_WARPS = TAIL_MAX / MAX_CTAS;         // tokens per CTA: one warp each
+
+// The combined row of one token: put(i, 8 values rounded to bf16) for every group; the sums of the unrounded ones over the warp.
+struct Combined { float s1, s2; };
+template <typename F>
+__device__ __forceinline__ Combined combine_row(const TailParams& p, int a, int b, float2 g, int lane, F&& put) {
+  a = min(max(a, 0), 2 * p.N - 1);
+  b = min(max(b, 0), 2 * p.N - 1);
+  uint4 ya[GROUPS], yb[GROUPS];
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < p.C) {
+      ya[i] = *reinterpret_cast<const uint4*>(p.y + size_t(a) * p.C + c);
+      yb[i] = *reinterpret_cast<const uint4*>(p.y + size_t(b) * p.C + c);
+    }
+  }
+  float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    if ((i * 32 + lane) * 8 < p.C) {
+      const uint32_t wa[4] = {ya[i].x, ya[i].y, ya[i].z, ya[i].w}, wb[4] = {yb[i].x, yb[i].y, yb[i].z, yb[i].w};
+      float acc[8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[2 * j] = __fmaf_rn(g.y, bf16_lo(wb[j]), __fmul_rn(g.x, bf16_lo(wa[j])));
+        acc[2 * j + 1] = __fmaf_rn(g.y, bf16_hi(wb[j]), __fmul_rn(g.x, bf16_hi(wa[j])));
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { s1 += acc[j]; s2 = __fmaf_rn(acc[j], acc[j], s2); }
+      put(i, make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
+                        pack_bf16x2(acc[6], acc[7])));
+    }
+  }
+  return {warp_sum(s1), warp_sum(s2)};
+}
+
+// Sums of the CTA's tokens (one per warp) -> every CTA of the cluster -> the decay of the call, the same bits everywhere.
+// Called by all threads after one cluster_arrive(); whatever `push` writes to other CTAs is visible to them when this
+// returns.
+template <typename F>
+__device__ __forceinline__ float tail_decay(const TailParams& p, Combined c, float var_scale, double (*part)[2], double (*all)[2],
+                                            float* s_alpha, int rank, int n_cta, F&& push) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+  if (lane == 0) { part[warp][0] = double(c.s1); part[warp][1] = double(c.s2); }
+  if (n_cta > 1) cluster_wait();               // the other CTAs have started: their shared memory may be written
+  push();
+  __syncthreads();
+  if (warp == 0) {
+    double a = lane < n_warps ? part[lane][0] : 0.0, b = lane < n_warps ? part[lane][1] : 0.0;
+#pragma unroll
+    for (int o = MAX_WARPS / 2; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (n_cta > 1) {
+      if (lane < 2 * n_cta)
+        cluster_st_f64(cluster_map(smem_u32(&all[rank][lane & 1]), uint32_t(lane >> 1)), (lane & 1) ? b : a);
+    } else if (lane == 0) {
+      all[0][0] = a;
+      all[0][1] = b;
+    }
+  }
+  if (n_cta > 1) {
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+  }
+  if (warp == 0) {
+    __syncwarp();
+    double s[2];
+    s[0] = lane < n_cta ? all[lane][0] : 0.0;
+    s[1] = lane < n_cta ? all[lane][1] : 0.0;
+#pragma unroll
+    for (int o = MAX_CTAS / 2; o > 0; o >>= 1) {
+      s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+      s[1] += __shfl_xor_sync(0xffffffffu, s[1], o);
+    }
+    if (lane == 0) {
+      const float mean = moe_act_mean(s, p.st.n_elems), var = moe_act_var(s, p.st.n_elems);
+      *s_alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, var);
+      if (rank == 0) {
+        p.st.scalars[1] = mean;
+        p.st.scalars[2] = var;
+        if (p.st.reflect) *p.st.reflect = reflect_penalty(p.st.lam, p.st.tau, __ldg(p.st.mu), mean, var);
+      }
+    }
+  }
+  __syncthreads();
+  return *s_alpha;
+}
+
+// One token per sequence (decode): a warp per token, its row in registers throughout.
+__global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailParams p, const int n_cta) {
+  __shared__ double s_part[MAX_WARPS][2], s_all[MAX_CTAS][2];
+  __shared__ float s_alpha;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = n_cta > 1 ? int(cluster_rank()) : 0;
+  const int n = rank + warp * n_cta;
+  const bool on = n < p.N;
+  if (n_cta > 1) cluster_arrive();
+  const float var_scale = __ldg(p.var_scale);
+  float x[GROUPS][8], h[GROUPS][8];
+  int2 sl = make_int2(0, 0);
+  float2 g = make_float2(0.f, 0.f);
+  if (on) {
+    sl = *reinterpret_cast<const int2*>(p.scatter + 2 * n);
+    g = *reinterpret_cast<const float2*>(p.gates + 2 * n);
+#pragma unroll
+    for (int i = 0; i < GROUPS; ++i) {
+      const int c = (i * 32 + lane) * 8;
+      if (c < p.C) {
+        load8(p.x + size_t(n) * p.C + c, x[i]);
+        if (p.h_in) {
+          load8(p.h_in + size_t(n) * p.C + c, h[i]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) h[i][j] = 0.f;
+        }
+      }
+    }
+  }
+  float l_bal = 0.f;
+  if (rank == 0 && tid == int(blockDim.x) - 1)
+    l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.inv_tokens, p.st.balance_alpha);
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+
+  uint4 m[GROUPS];
+  Combined c = {0.f, 0.f};
+  if (on) c = combine_row(p, sl.x, sl.y, g, lane, [&](int i, uint4 v) { m[i] = v; });
+  const float alpha = tail_decay(p, c, var_scale, s_part, s_all, &s_alpha, rank, n_cta, [] {});
+  if (rank == 0 && tid == int(blockDim.x) - 1) p.st.scalars[0] = l_bal;
+  if (!on) return;
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int ch = (i * 32 + lane) * 8;
+    if (ch < p.C) {
+      const uint32_t mw[4] = {m[i].x, m[i].y, m[i].z, m[i].w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        h[i][j] = lsf_step(alpha, h[i][j], (j & 1) ? bf16_hi(mw[j >> 1]) : bf16_lo(mw[j >> 1]));
+        x[i][j] = x[i][j] + h[i][j];
+        ss = __fmaf_rn(x[i][j], x[i][j], ss);
+      }
+      store8(p.h_out + size_t(n) * p.C + ch, h[i]);
+      store8(p.x + size_t(n) * p.C + ch, x[i]);
+    }
+  }
+  if (!p.w_norm) return;
+  ss = warp_sum(ss);
+  const float r = rsqrtf(ss / float(p.C) + p.eps);
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int ch = (i * 32 + lane) * 8;
+    if (ch < p.C)
+      *reinterpret_cast<uint4*>(p.xn + size_t(n) * p.C + ch) =
+          norm8(x[i], r, __ldg(reinterpret_cast<const float4*>(p.w_norm + ch)), __ldg(reinterpret_cast<const float4*>(p.w_norm + ch) + 1));
+  }
+}
+
+// Several tokens per sequence.  Rows are combined and normalised by the CTA that owns the token (token n: CTA n % n_cta, a
+// warp each), the scan runs where all tokens of a channel are (CTA k: channels [128 k, 128 k + 128)); the rows change
+// hands through distributed shared memory.  ms [N][128] bf16: combined rows of the CTA's channels; hs: their membranes; xr [N / n_cta][C] f32:
+// updated residual rows of the CTA's tokens.
+constexpr int SCAN_CH = 128, RUN = 16;         // channels per CTA; tokens per run (lsf_tma_kernel's warp runs)
+
+__global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailParams p, const int n_cta) {
+  extern __shared__ __align__(16) uint8_t tail_smem[];
+  __shared__ double s_part[MAX_WARPS][2], s_all[MAX_CTAS][2];
+  __shared__ float s_alpha;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, threads = blockDim.x;
+  const int N = p.N, B = p.B, T = p.T, C = p.C;
+  const int rank = n_cta > 1 ? int(cluster_rank()) : 0;
+  uint8_t* ms = tail_smem;                                                     // [N][256 bytes]
+  float* hs = reinterpret_cast<float*>(tail_smem + size_t(N) * SCAN_CH * 2);   // [B][128]: h_out may be h_in
+  float* xr = hs + size_t(B) * SCAN_CH;                                        // [ceil(N / n_cta)][C]
+  const int own = rank + warp * n_cta;                                         // this warp's token
+  const bool on = own < N;
+  if (n_cta > 1) cluster_arrive();
+  const float var_scale = __ldg(p.var_scale);
+  int2 sl = make_int2(0, 0);
+  float2 g = make_float2(0.f, 0.f);
+  if (on) {
+    sl = *reinterpret_cast<const int2*>(p.scatter + 2 * own);
+    g = *reinterpret_cast<const float2*>(p.gates + 2 * own);
+  }
+  for (int i = tid; i < B * SCAN_CH / 4; i += threads) {
+    const int b = i / (SCAN_CH / 4), q = i % (SCAN_CH / 4);
+    reinterpret_cast<float4*>(hs)[i] =
+        p.h_in ? *(reinterpret_cast<const float4*>(p.h_in + size_t(b) * C + rank * SCAN_CH) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float l_bal = 0.f;
+  if (rank == 0 && tid == threads - 1)
+    l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.inv_tokens, p.st.balance_alpha);
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+
+  uint4 m[GROUPS];
+  Combined cm = {0.f, 0.f};
+  if (on) cm = combine_row(p, sl.x, sl.y, g, lane, [&](int i, uint4 v) { m[i] = v; });
+  const float alpha = tail_decay(p, cm, var_scale, s_part, s_all, &s_alpha, rank, n_cta, [&] {
+    if (on) {
+#pragma unroll
+      for (int i = 0; i < GROUPS; ++i) {
+        const int c = (i * 32 + lane) * 8;
+        if (c < C) {
+          const uint32_t dst = smem_u32(ms) + uint32_t(own) * (SCAN_CH * 2) + uint32_t(c % SCAN_CH) * 2u;
+          cluster_st_128(n_cta > 1 ? cluster_map(dst, uint32_t(c / SCAN_CH)) : dst, m[i]);
+        }
+      }
+    }
+  });
+  if (rank == 0 && tid == threads - 1) p.st.scalars[0] = l_bal;
+
+  // ---- scan of the CTA's channels, two per thread: runs of 16 tokens from a zero carry, the carries along the runs,
+  // then every token's value, with the roundings of lsf_tma_kernel (T > 8) or lsf_short_kernel ----
+  const int pairs = SCAN_CH / 2, col = tid % pairs, slot = tid / pairs, slots = threads / pairs;
+  const int n_runs = T > 8 ? (T + RUN - 1) / RUN : 1, run_len = T > 8 ? RUN : T;
+  const float one_m = 1.0f - alpha;
+  float pw[RUN];
+  {
+    float a = alpha;
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) { pw[i] = a; a *= alpha; }
+  }
+  auto m_at = [&](int n) { return *reinterpret_cast<const uint32_t*>(ms + size_t(n) * (SCAN_CH * 2) + col * 4); };
+#pragma unroll 1
+  for (int w = slot; w < B * n_runs; w += slots) {           // (sequence, run)
+    const int b = w / n_runs, run = w - b * n_runs;
+    const size_t ch = size_t(rank) * SCAN_CH + col * 2;
+    float2 h = *reinterpret_cast<const float2*>(hs + b * SCAN_CH + col * 2);
+    float2 xv[RUN];              // the run's residual values, all in flight together
+#pragma unroll
+    for (int j = 0; j < RUN; ++j) {
+      const int t = run * RUN + j;
+      if (j < run_len && t < T) xv[j] = *reinterpret_cast<const float2*>(p.x + size_t(b * T + t) * C + ch);
+    }
+    // the carry into this run: the ends of the runs before it, each scanned from zero (at most seven)
+#pragma unroll 1
+    for (int q = 0; q < run; ++q) {
+      float2 e = make_float2(0.f, 0.f);
+#pragma unroll 4
+      for (int j = 0; j < RUN; ++j) {
+        const uint32_t v = m_at(b * T + q * RUN + j);
+        e.x = alpha * e.x + one_m * bf16_lo(v);
+        e.y = alpha * e.y + one_m * bf16_hi(v);
+      }
+      h.x = pw[RUN - 1] * h.x + e.x;
+      h.y = pw[RUN - 1] * h.y + e.y;
+    }
+    float2 loc = make_float2(0.f, 0.f);
+    float2 hv = h;
+#pragma unroll
+    for (int j = 0; j < RUN; ++j) {
+      const int t = run * RUN + j;
+      if (j < run_len && t < T) {
+        const int n = b * T + t;
+        const uint32_t v = m_at(n);
+        if (T > 8) {
+          loc.x = alpha * loc.x + one_m * bf16_lo(v);
+          loc.y = alpha * loc.y + one_m * bf16_hi(v);
+          hv.x = loc.x + pw[j] * h.x;
+          hv.y = loc.y + pw[j] * h.y;
+        } else {
+          hv.x = lsf_step(alpha, hv.x, bf16_lo(v));
+          hv.y = lsf_step(alpha, hv.y, bf16_hi(v));
+        }
+        xv[j].x = xv[j].x + hv.x;
+        xv[j].y = xv[j].y + hv.y;
+        *reinterpret_cast<float2*>(p.x + size_t(n) * C + ch) = xv[j];
+        const uint32_t dst = smem_u32(xr) + (uint32_t(n / n_cta) * uint32_t(C) + uint32_t(ch)) * 4u;
+        cluster_st_64(n_cta > 1 ? cluster_map(dst, uint32_t(n % n_cta)) : dst, xv[j]);
+        if (t == T - 1) *reinterpret_cast<float2*>(p.h_out + size_t(b) * C + ch) = hv;
+      }
+    }
+  }
+  if (n_cta > 1) { __syncwarp(); cluster_arrive(); cluster_wait(); } else __syncthreads();
+  if (!p.w_norm || !on) return;
+
+  // ---- the norm of the warp's token ----
+  const float* row = xr + size_t(warp) * C;
+  float v[GROUPS][8], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < C) {
+      load8(row + c, v[i]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss = __fmaf_rn(v[i][j], v[i][j], ss);
+    }
+  }
+  ss = warp_sum(ss);
+  const float r = rsqrtf(ss / float(C) + p.eps);
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < C)
+      *reinterpret_cast<uint4*>(p.xn + size_t(own) * C + c) =
+          norm8(v[i], r, __ldg(reinterpret_cast<const float4*>(p.w_norm + c)), __ldg(reinterpret_cast<const float4*>(p.w_norm + c) + 1));
+  }
+}
+
+// Embedding rows into the f32 residual stream (jarvis_model.py:498) and, while they are in registers, norm1 of the first
+// block; clears the chain's accumulators on the way.  One warp per token, C <= 1024.
+__global__ void __launch_bounds__(256)
+embed_norm_kernel(const int64_t* __restrict__ ids, const float* __restrict__ table, int vocab, const float* __restrict__ w_norm,
+                  float eps, float* __restrict__ x, __nv_bfloat16* __restrict__ xn, int n_rows, int C, uint32_t* __restrict__ zero,
+                  int n_zero) {
+  pdl_wait();
+  pdl_trigger();
+  const int gtid = blockIdx.x * 256 + threadIdx.x;
+  for (int i = gtid; i < n_zero; i += gridDim.x * 256) zero[i] = 0u;
+  const int row = gtid >> 5, lane = threadIdx.x & 31;
+  if (row >= n_rows) return;
+  long long id = ids[row];
+  id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);            // clamp instead of faulting on a bad id
+  const float* src = table + size_t(id) * C;
+  float v[GROUPS][8], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < C) load8(src + c, v[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < C) {
+      store8(x + size_t(row) * C + c, v[i]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss = __fmaf_rn(v[i][j], v[i][j], ss);
+    }
+  }
+  ss = warp_sum(ss);
+  const float r = rsqrtf(ss / float(C) + eps);
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const int c = (i * 32 + lane) * 8;
+    if (c < C)
+      *reinterpret_cast<uint4*>(xn + size_t(row) * C + c) =
+          norm8(v[i], r, __ldg(reinterpret_cast<const float4*>(w_norm + c)), __ldg(reinterpret_cast<const float4*>(w_norm + c) + 1));
+  }
+}
+
+}  // namespace
+
+int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const float* w_norm, float eps, float* x, void* xn_bf16,
+                      int n_rows, int C, void* zero, size_t zero_bytes, cudaStream_t stream) {
+  JB_REQUIRE(ids && table && w_norm && x && xn_bf16 && vocab > 0 && n_rows > 0, "embed_norm: null pointer or empty");
+  JB_REQUIRE(C % 8 == 0 && C <= 1024 && zero_bytes % 4 == 0, "embed_norm: row length %d", C);
+  JB_REQUIRE(aligned16(table) && aligned16(x) && aligned16(xn_bf16) && aligned16(w_norm), "embed_norm: pointers must be 16-byte aligned");
+  launch_dep(embed_norm_kernel, (n_rows + 7) / 8, 256, 0, stream, ids, table, vocab, w_norm, eps, x,
+             reinterpret_cast<__nv_bfloat16*>(xn_bf16), n_rows, C, reinterpret_cast<uint32_t*>(zero), int(zero_bytes / 4));
+  JB_LAUNCH_CHECK("embed_norm_kernel");
+  return JB200_OK;
+}
+
+int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router, int N, int C, int E,
+                       int64_t* idx, float* gates, double* probs_sum, int* hist, int* ticket, int* counts, int* offsets,
+                       int* scatter, int* gather, int* gate_idx, cudaStream_t stream) {
+  JB_REQUIRE(N >= 1 && N <= ROUTE_SMALL_MAX && C % 8 == 0 && C <= 1024 && (E == 4 || E == 8), "route_small: bad shape (N=%d, C=%d, E=%d)", N, C, E);
+  RouteParams p;
+  p.x = x; p.w_norm = w_norm; p.w_router = w_router; p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
+  p.idx = idx; p.gates = gates; p.probs_sum = probs_sum; p.hist = hist; p.ticket = ticket;
+  p.counts = counts; p.offsets = offsets; p.scatter = scatter; p.gather = gather; p.gate_idx = gate_idx;
+  p.eps = eps; p.N = N; p.C = C;
+  if (E == 4) launch_dep(route_small_kernel<4>, N, 32, 0, stream, p);
+  else launch_dep(route_small_kernel<8>, N, 32, 0, stream, p);
+  JB_LAUNCH_CHECK("route_small_kernel");
+  return JB200_OK;
+}
+
+int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const LsfStats& st, const float* var_scale,
+                float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x, const float* w_norm, float eps,
+                void* xn_bf16, int B, int T, int C, cudaStream_t stream) {
+  const int N = B * T;
+  JB_REQUIRE(N >= 1 && N <= tail_max_tokens(C, T) && C % 128 == 0 && C <= 1024, "tail: bad shape (B=%d, T=%d, C=%d)", B, T, C);
+  TailParams p;
+  p.y = reinterpret_cast<const __nv_bfloat16*>(y_bf16); p.gates = gates; p.scatter = scatter; p.st = st;
+  p.inv_tokens = 1.0 / double(st.n_tokens);
+  p.var_scale = var_scale; p.alpha_min = alpha_min; p.alpha_max = alpha_max;
+  p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;
+  p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
+  p.B = B; p.T = T; p.N = N; p.C = C;
+  if (T == 1) {
+    // a lone CTA while its SM can take the rows (4 KB in, 10 KB out each), else eight
+    const int n_cta = N <= 4 ? 1 : MAX_CTAS;
+    const int warps = (N + n_cta - 1) / n_cta;
+    if (n_cta == 1) launch_dep(tail_step_kernel, 1, 32 * warps, 0, stream, p, 1);
+    else launch_dep_cluster(tail_step_kernel, n_cta, 32 * warps, 0, n_cta, stream, p, n_cta);
+    JB_LAUNCH_CHECK("tail_step_kernel");
+    return JB200_OK;
+  }
+  const int n_cta = C / SCAN_CH, rows = (N + n_cta - 1) / n_cta;
+  const size_t smem = size_t(N) * SCAN_CH * 2 + (size_t(B) * SCAN_CH + size_t(rows) * C) * sizeof(float);
+  JB_MAX_SMEM(tail_scan_kernel, size_t(TAIL_MAX) * SCAN_CH * 2 + (size_t(TAIL_MAX / 2) * SCAN_CH + size_t(MAX_WARPS) * 1024) * sizeof(float));
+  if (n_cta == 1) launch_dep(tail_scan_kernel, 1, 32 * MAX_WARPS, smem, stream, p, 1);
+  else launch_dep_cluster(tail_scan_kernel, n_cta, 32 * MAX_WARPS, smem, n_cta, stream, p, n_cta);
+  JB_LAUNCH_CHECK("tail_scan_kernel");
+  return JB200_OK;
+}
+
+int tail_max_tokens(int C, int T) { return T == 1 ? TAIL_MAX : MAX_WARPS * (C / SCAN_CH); }
+
+}  // namespace jb

@@ -84,3 +84,33 @@ def test_cross_entropy_matches_torch(rows, V, ld):
     # f32 exponentials (2 ulp each) and an f32 logarithm and subtraction at magnitude |max| + log V <= 32: 32 * 2^-23 * 4
     assert abs(float(got) - float(want)) < 2e-5 * max(1.0, abs(float(want)))
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (4, 1), (5, 1), (8, 1), (9, 1), (16, 1), (17, 1), (33, 1), (64, 1), (65, 1), (128, 1),
+                                 (129, 1), (1, 2), (3, 3), (1, 16), (2, 20), (1, 64), (1, 65), (2, 64), (1, 128), (1, 129),
+                                 (1, 640), (1, 641)])
+def test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T):
+    """d_model 1024: the kernels for few tokens (GEMM forms up to 16, up to 640 and beyond, router up to 64, row cluster up to
+    128) against the kernel-by-kernel path; mixed routing, carried state, one expert without tokens at the smallest sizes."""
+    from jarvis_b200 import chain
+    torch.manual_seed(7)
+    blk = jm.ternary_init_(jm.JarvisBlock(1024, 16, max_seq_len=1024)).cuda().eval()
+    gen = torch.Generator(device="cuda").manual_seed(B * 1000 + T)
+    x = torch.randn(B * T, 1024, generator=gen, device="cuda")
+    h = torch.randn(B, 1024, generator=gen, device="cuda")
+    S = torch.randn(B, 16, 64, 64, generator=gen, device="cuda")
+    norm = (torch.rand(1024, generator=gen, device="cuda") + 0.5, 1e-6)
+    xa, xb = x.clone(), x.clone()
+    acc, hist = torch.zeros(6, dtype=torch.float64, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    ha, sa, Sa = blk.forward_rows(xa, B, T, h, 5, S, want_attn_state=True, scratch=(acc, hist, torch.zeros(3, device="cuda")))
+    r = chain.run(chain.table_of(blk, [blk]), xb, B, T, start_pos=5, h_in=[h], s_in=[S], want_state=True, final_norm=norm)
+    assert rel(xb, xa) < TOL and rel(r.h[0], ha) < TOL and rel(r.S[0], Sa) < TOL
+    assert rel(r.hidden.float(), ops.rmsnorm(xb, *norm).float()) < 4e-3        # one bf16 rounding of the same values
+    assert abs(float(r.scalars[0][0]) - float(sa[0])) < 1e-3 * abs(float(sa[0]))
+    assert abs(float(r.scalars[0][2]) - float(sa[2])) < 5e-3 * float(sa[2])
+    idx, gates, (counts, offsets, scatter, gather, gate_idx) = blk.moe.last_routing
+    want = ops.moe_metadata(idx.contiguous(), 4)
+    for got, ref in zip((counts, offsets, scatter, gather, gate_idx), want):
+        assert torch.equal(got, ref)                                          # dispatch order: bit-exact
+    assert int(torch.bincount(idx.flatten(), minlength=4).sum()) == 2 * B * T
+    assert _lib.device_status() == 0
