@@ -256,4 +256,7 @@ __device__ __forceinline__ void store_acc_chunk(const GemmParams& p, uint32_t ta
   }
 }
 
+// Many tokens: the CTA-pair kernel (pair_gemm.cu).  p: everything but bn and resid_stage_smem set, checked by the caller.
+int launch_pair_gemm(const GemmParams& p, const void* x_bf16, int sms, cudaStream_t stream);
+
 }  // namespace jb
