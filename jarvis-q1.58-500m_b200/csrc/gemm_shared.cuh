@@ -71,6 +71,36 @@ __device__ __forceinline__ float gelu_erf(float v) {
   return fmaf(hv, t, hv);
 }
 
+// The same for two values with the packed f32 instructions (each half rounds as the scalar one): 12 instructions for the pair
+// where two calls of gelu_erf take 20.  Clamping x^2 instead of x is the same function: beyond |x| = 8 tanh is 1 either way.
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f32x2_split(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t gelu_erf_x2(uint64_t v) {
+  float a, b;
+  f32x2_split(mul_f32x2(v, v), a, b);
+  const uint64_t x2 = f32x2(fminf(a, 64.0f), fminf(b, 64.0f));
+  uint64_t pz = fma_f32x2(f32x2(-0.0003515195915898722f, -0.0003515195915898722f), x2, f32x2(0.03700566448133039f, 0.03700566448133039f));
+  pz = fma_f32x2(pz, x2, f32x2(0.797507862407347f, 0.797507862407347f));
+  f32x2_split(mul_f32x2(pz, v), a, b);
+  asm("tanh.approx.f32 %0, %0;" : "+f"(a));
+  asm("tanh.approx.f32 %0, %0;" : "+f"(b));
+  const uint64_t hv = mul_f32x2(v, f32x2(0.5f, 0.5f));
+  return fma_f32x2(hv, f32x2(a, b), hv);
+}
 
 constexpr int MAX_GROUPS = 16;
 

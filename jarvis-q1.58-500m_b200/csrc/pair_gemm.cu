@@ -26,19 +26,25 @@ namespace {
 constexpr int BM = 128, BK = 64, BN = 256;             // tokens per CTA (256 per pair), K per stage, out-features per tile
 constexpr int A_BYTES = BM * BK * 2;                   // 16 KiB: this CTA's tokens
 constexpr int B_BYTES = (BN / 2) * BK * 2;             // 16 KiB: this CTA's half of the weights
-constexpr int STAGES = 6;
 constexpr int CODE_SLOTS = 3, CODE_KB = 4, CODE_BYTES = (BN / 2) * CODE_KB * 16;   // ring of codes: four K-blocks, 8 KiB a slot
 constexpr int DEC_GROUPS = 2;                          // of four warps, on alternate K-blocks (three or four: 3-8 % slower)
 constexpr int CODE_WARP = 2, DEC_WARP0 = 3, EPI_WARP0 = DEC_WARP0 + 4 * DEC_GROUPS, THREADS = 32 * (EPI_WARP0 + 8);
 constexpr uint32_t TMEM_COLS = 512;
 
+// The residual form trades one ring stage for a 4 KiB tile per epilogue warp, from which the memory system adds to x.
+constexpr int stages(bool resid) { return resid ? 5 : 6; }
+constexpr int OUT_BYTES = 32 * 32 * 4;
+
 struct PairCtl {
-  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], code_full[CODE_SLOTS], code_empty[CODE_SLOTS];
+  uint64_t full[6], empty[6], acc_full[2], acc_empty[2], code_full[CODE_SLOTS], code_empty[CODE_SLOTS];
   uint32_t tmem_base, abort_flag;
   int32_t seg[MAX_GROUPS + 1];
 };
-constexpr size_t SMEM_BYTES = 1024 + size_t(STAGES) * (A_BYTES + B_BYTES) + size_t(CODE_SLOTS) * CODE_BYTES + (sizeof(PairCtl) + 127) / 128 * 128;
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
+constexpr size_t CTL_BYTES = (sizeof(PairCtl) + 127) / 128 * 128;
+constexpr size_t smem_bytes(bool resid) {
+  return 1024 + size_t(stages(resid)) * (A_BYTES + B_BYTES) + size_t(CODE_SLOTS) * CODE_BYTES + (resid ? 8 * OUT_BYTES : 0) + CTL_BYTES;
+}
+static_assert(smem_bytes(false) <= 227 * 1024 && smem_bytes(true) <= 227 * 1024, "shared memory of one CTA");
 
 // ---- cta_group::2 forms of the wrappers in common.cuh ----
 __device__ __forceinline__ void pair_tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
@@ -112,13 +118,15 @@ __device__ __forceinline__ void st_global_256(void* p, const uint32_t* w) {
 __device__ __forceinline__ void store_row_chunk(const GemmParams& p, uint32_t (&v)[32], float alpha, size_t o) {
   if (p.epilogue == JB200_EPI_BF16 || p.epilogue == JB200_EPI_GELU_BF16) {
     uint32_t w[16];
-    if (p.epilogue == JB200_EPI_GELU_BF16) {
+    const bool gelu = p.epilogue == JB200_EPI_GELU_BF16;
+    const uint64_t al = f32x2(alpha, alpha);
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        w[j] = pack_bf16x2(gelu_erf(alpha * __uint_as_float(v[2 * j])), gelu_erf(alpha * __uint_as_float(v[2 * j + 1])));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) w[j] = pack_bf16x2(alpha * __uint_as_float(v[2 * j]), alpha * __uint_as_float(v[2 * j + 1]));
+    for (int j = 0; j < 16; ++j) {
+      uint64_t x = mul_f32x2(f32x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), al);
+      if (gelu) x = gelu_erf_x2(x);
+      float a, b;
+      f32x2_split(x, a, b);
+      w[j] = pack_bf16x2(a, b);
     }
     __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.out) + o;
     st_global_256(d, w);
@@ -129,7 +137,7 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, uint32_t (&
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(alpha * __uint_as_float(v[j]));
   if (p.epilogue == JB200_EPI_RESID_F32) {
-    // x += alpha * acc by the memory system: no load of the old values to wait for
+    // grouped calls (their tiles end inside a matrix, where a tile reduction would not be clipped)
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
@@ -182,16 +190,19 @@ __device__ __forceinline__ bool pair_tile(const PairCtl* ctl, const PairPlan& pl
   return false;
 }
 
+template <bool RESID>
 __global__ void __launch_bounds__(THREADS, 1)
 pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                 const __grid_constant__ GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ GemmParams p) {
+  constexpr int STAGES = stages(RESID);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw_addr);
   const uint32_t a_base = base, b_base = base + STAGES * A_BYTES;
   const uint32_t code_base = b_base + STAGES * B_BYTES;
-  PairCtl* ctl = reinterpret_cast<PairCtl*>(smem + size_t(STAGES) * (A_BYTES + B_BYTES) + size_t(CODE_SLOTS) * CODE_BYTES);
+  const uint32_t out_base = code_base + CODE_SLOTS * CODE_BYTES;
+  PairCtl* ctl = reinterpret_cast<PairCtl*>(smem + (out_base - base) + (RESID ? 8 * OUT_BYTES : 0));
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int rank = int(cluster_rank());
@@ -394,12 +405,33 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         uint32_t v[32];
         tmem_ld_32x32(t_lane + c0, v);
         tmem_ld_wait();
+        if (RESID) {
+          // x[token][feature] += alpha * acc by the memory system: the tile leaves as one TMA reduction, which clips rows past
+          // the matrix.  Rows of 128 bytes in the 128-byte swizzle: every 16-byte store of eight lanes covers all banks.
+          if (lane == 0) bulk_wait_group_read<0>();     // the previous reduction has read this warp's tile
+          __syncwarp();
+          const uint32_t stage = out_base + uint32_t(warp - EPI_WARP0) * OUT_BYTES, dst = stage + uint32_t(lane) * 128u;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
+                         ::"r"(dst + (uint32_t(j ^ (lane & 7)) << 4)), "f"(alpha * __uint_as_float(v[4 * j])),
+                           "f"(alpha * __uint_as_float(v[4 * j + 1])), "f"(alpha * __uint_as_float(v[4 * j + 2])),
+                           "f"(alpha * __uint_as_float(v[4 * j + 3])) : "memory");
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_2d(&tmap_out, f, tc.tok0 + rank * BM + q * 32, stage);
+            bulk_commit_group();
+          }
+          continue;
+        }
         if (on) store_row_chunk(p, v, alpha, size_t(tok) * p.N + f);
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) cluster_mbar_arrive(cluster_map(smem_u32(&ctl->acc_empty[acc]), 0u));
     }
+    if (RESID && lane == 0) bulk_wait_group<0>();       // every reduction has landed before the CTA ends
   }
 
   __syncwarp();
@@ -437,10 +469,22 @@ int launch_pair_gemm(const GemmParams& p, const void* x_bf16, int sms, cudaStrea
                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "ternary_linear (weights)");
   }
   if (rc != JB200_OK) return rc;
-  JB_MAX_SMEM(pair_gemm_kernel, SMEM_BYTES);
   const long tiles = (long((p.M + 2 * BM - 1) / (2 * BM)) + (p.G - 1)) * ((p.N + BN - 1) / BN) * 4;   // at most, with cut tiles
-  const int grid = 2 * int(tiles < pairs ? tiles : pairs);
-  launch_dep_cluster(pair_gemm_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, 2, stream, tmap, tmap_w, p);
+  const dim3 grid(2 * unsigned(tiles < pairs ? tiles : pairs));
+  CUtensorMap tmap_out = tmap;
+  if (p.epilogue == JB200_EPI_RESID_F32 && p.G == 1) {
+    const cuuint64_t odim[2] = {cuuint64_t(p.N), cuuint64_t(p.M)};
+    const cuuint64_t ostride[1] = {cuuint64_t(p.N) * 4};
+    const cuuint32_t obox[2] = {32, 32};
+    rc = encode_tiled(&tmap_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.out, odim, ostride, obox, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "ternary_linear (residual stream)");
+    if (rc != JB200_OK) return rc;
+    JB_MAX_SMEM(pair_gemm_kernel<true>, smem_bytes(true));
+    launch_dep_cluster(pair_gemm_kernel<true>, grid, dim3(THREADS), smem_bytes(true), 2, stream, tmap, tmap_w, tmap_out, p);
+  } else {
+    JB_MAX_SMEM(pair_gemm_kernel<false>, smem_bytes(false));
+    launch_dep_cluster(pair_gemm_kernel<false>, grid, dim3(THREADS), smem_bytes(false), 2, stream, tmap, tmap_w, tmap_out, p);
+  }
   JB_LAUNCH_CHECK("pair_gemm_kernel");
   return JB200_OK;
 }

@@ -1,0 +1,62 @@
+"""The CTA-pair GEMM (calls of more than 512 rows) at the sizes where it can go wrong: ragged token tiles and segments, empty
+segments, out-features that are odd multiples of 128, cut tiles of the last wave, one to many K-chunks.  Small-integer
+activations make every product and sum exact, so the comparison with a plain f32 matmul is exact; the GELU form is compared
+with the one-CTA kernel bit for bit."""
+import pytest
+import torch
+
+from jarvis_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _weights(G, N, K, gen, prepared):
+    w = torch.randint(-1, 2, (G, N, K), generator=gen, device="cuda").float()
+    packed = torch.stack([ops.pack_codes(w[g]) for g in range(G)])
+    return w, ops.prepare_weights(packed) if prepared else packed
+
+
+@pytest.mark.parametrize("M,N,K,prepared", [(513, 128, 256, True), (767, 384, 256, False), (1024, 1024, 1024, True),
+                                            (2331, 3072, 1024, True), (9473, 1024, 512, False), (19000, 256, 2048, True)])
+def test_single_matrix_forms_are_exact(M, N, K, prepared):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randint(-3, 4, (M, K), generator=gen, device="cuda").bfloat16()
+    w, packed = _weights(1, N, K, gen, prepared)
+    alpha = torch.tensor([0.25], device="cuda")
+    want = 0.25 * (x.float() @ w[0].t())                          # integers below 2^24 times a power of two
+    got = ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_F32, prepared=prepared)
+    assert torch.equal(got, want)
+    assert torch.equal(ops.ternary_linear(x, packed[0], alpha, prepared=prepared), want.bfloat16())
+    base = torch.randint(-8, 9, (M, N), generator=gen, device="cuda").float()
+    assert torch.equal(ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_RESID_F32, out=base.clone(), prepared=prepared), base + want)
+    a = ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_GELU_BF16, prepared=prepared)
+    b = ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_GELU_BF16, prepared=prepared, token_tile=128)
+    assert torch.equal(a, b)
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,cuts", [(513, 128, 256, [0, 0, 513, 513, 513]), (1500, 384, 512, [0, 1, 257, 900, 1500]),
+                                        (4662, 2048, 1024, [0, 1100, 2400, 3600, 4662]), (20000, 1024, 256, [0, 10000, 10001, 19999, 20000])])
+def test_grouped_forms_are_exact(M, N, K, cuts):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randint(-3, 4, (M, K), generator=gen, device="cuda").bfloat16()
+    w, packed = _weights(4, N, K, gen, True)
+    alpha = torch.tensor([0.25, 0.5, 1.0, 2.0], device="cuda")
+    offs = torch.tensor(cuts, dtype=torch.int32, device="cuda")
+    want = torch.cat([float(alpha[g]) * (x[cuts[g]:cuts[g + 1]].float() @ w[g].t()) for g in range(4)])
+    assert torch.equal(ops.ternary_linear_grouped(x, packed, alpha, offs, epilogue=ops.EPI_F32, prepared=True), want)
+    assert torch.equal(ops.ternary_linear_grouped(x, packed, alpha, offs, prepared=True), want.bfloat16())
+    out = want.clone()
+    assert torch.equal(ops.ternary_linear_grouped(x, packed, alpha, offs, epilogue=ops.EPI_RESID_F32, out=out, prepared=True), 2 * want)
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(513, 128, 256), (1111, 640, 1024), (3000, 50304, 256)])
+def test_dense_weights_are_exact(M, N, K):
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randint(-3, 4, (M, K), generator=gen, device="cuda").bfloat16()
+    w = torch.randint(-3, 4, (N, K), generator=gen, device="cuda").bfloat16()
+    want = x.float() @ w.float().t()
+    assert torch.equal(ops.dense_linear(x, w, out_dtype=torch.float32), want)
+    assert torch.equal(ops.dense_linear(x, w), want.bfloat16())
+    assert _lib.device_status() == 0
