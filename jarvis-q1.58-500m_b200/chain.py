@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import operator
+import weakref
 from typing import List, Optional
 
 import torch
@@ -35,9 +36,12 @@ class LayerTable:
 
     def __init__(self, blocks):
         from .modules import ReflectivePenalty, _f32
-        self.blocks = list(blocks)
-        self.n = len(self.blocks)
-        b0 = self.blocks[0]
+        blocks = list(blocks)
+        # weak: a block may own its table, and a cycle would keep a dropped model's memory until the next collection
+        self.blocks = [weakref.ref(b) for b in blocks]
+        self.n = len(blocks)
+        b0 = blocks[0]
+        self.rotary = b0.attn.rotary
         self.C, self.H, self.E = b0.norm1.weight.numel(), b0.attn.n_heads, b0.moe.num_experts
         self.hidden = b0.moe.w1[0].weight.shape[0]
         self.device = b0.norm1.weight.device
@@ -45,9 +49,9 @@ class LayerTable:
         self.array = (_lib.Layer * self.n)()
         self._keep = []
         self._sizes = {}
-        self.has_reflect = all(type(b.reflect) is ReflectivePenalty for b in self.blocks)
-        self._watch(self.blocks)
-        for d, b in zip(self.array, self.blocks):
+        self.has_reflect = all(type(b.reflect) is ReflectivePenalty for b in blocks)
+        self._watch(blocks)
+        for d, b in zip(self.array, blocks):
             at, moe, lq = b.attn, b.moe, b.liquid
             qkv, a_qkv = at.qkv_packed()
             out, a_out = at.out_proj.packed()
@@ -126,7 +130,7 @@ class LayerTable:
 def table_of(owner, blocks) -> Optional[LayerTable]:
     """The (cached) table of `blocks`, kept on `owner`; None when they need the per-kernel path."""
     tab = owner.__dict__.get("_layer_table")
-    if tab is None or tab.n != len(blocks) or not all(map(operator.is_, tab.blocks, blocks)) or not tab.current():
+    if tab is None or tab.n != len(blocks) or any(r() is not b for r, b in zip(tab.blocks, blocks)) or not tab.current():
         if not supported(blocks):
             return None
         tab = LayerTable(blocks)
@@ -182,7 +186,7 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
     else:
         f.pos0_scalar = int(start_pos)
         end = f.pos0_scalar + T
-    cos, sin = tab.blocks[0].attn.rotary.half_tables(end, dev)
+    cos, sin = tab.rotary.half_tables(end, dev)
     f.cos_tab, f.sin_tab, f.n_pos = cos.data_ptr(), sin.data_ptr(), cos.shape[0]
     h_in, s_in = _f32_list(h_in), _f32_list(s_in)
     if h_in is not None:
@@ -215,21 +219,25 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
         f.w_final, f.eps_final, f.hidden_out = final_norm[0].data_ptr(), final_norm[1], res.hidden.data_ptr()
     _lib.check(_lib.load().jb200_forward_layers(tab.array, n, C.byref(f), ops._stream()), "jb200_forward_layers")
     for i, (_, moe) in enumerate(tab._flags):
-        moe["_routing"] = (routing, i, B * T, tab)      # the views are built when somebody looks at them
+        moe["_routing"] = RoutingSource((routing, i, B * T, tab.E))      # the views are built when somebody looks at them
     return res
+
+
+class RoutingSource(tuple):
+    """(routing buffer, layer, tokens, experts): where a layer's last routing is, for routing_views."""
 
 
 def routing_views(src):
     """(topk_idx, gates, (counts, offsets, scatter, gather, gate_idx)) of one layer from its block of a call's routing buffer."""
-    buf, layer, N, tab = src
-    nbytes, off = None, (C.c_size_t * 7)()
-    nbytes = _lib.load().jb200_routing_layout(N, tab.E, off)
+    buf, layer, N, E = src
+    off = (C.c_size_t * 7)()
+    nbytes = _lib.load().jb200_routing_layout(N, E, off)
 
     def view(i, count, dtype, *shape):
         size = torch.empty((), dtype=dtype).element_size()
         at = layer * nbytes + off[i]
         return buf[at:at + count * size].view(dtype).view(*shape)
-    i32, E = torch.int32, tab.E
+    i32 = torch.int32
     return (view(0, 2 * N, torch.int64, N, 2), view(1, 2 * N, torch.float32, N, 2),
             (view(2, E, i32, E), view(3, E + 1, i32, E + 1), view(4, 2 * N, i32, N, 2), view(5, 2 * N, i32, 2 * N),
              view(6, 2 * N, i32, 2 * N)))

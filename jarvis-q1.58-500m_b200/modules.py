@@ -276,7 +276,7 @@ class SparseMoELayer(nn.Module):
     def last_routing(self):
         """(topk_idx, gates, metadata) of the most recent call, for inspection."""
         r = self._routing
-        return chain.routing_views(r) if r is not None and isinstance(r[-1], chain.LayerTable) else r
+        return chain.routing_views(r) if isinstance(r, chain.RoutingSource) else r
 
     def packed(self):
         return (self._p1.get([m.weight for m in self.w1], stack=True),
