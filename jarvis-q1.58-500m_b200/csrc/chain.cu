@@ -54,10 +54,11 @@ struct Workspace {
 // against 2.86), beyond that the persistent pipeline.
 constexpr int SMALL_TOKENS = 16, MID_TOKENS = 640;
 // Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
-// tokens) that leaves the launch one wave.
-inline int mid_tile(int rows, int n_ft, int groups, int sms) {
-  int bn = rows <= 64 ? (rows + 15) / 16 * 16 : 64;
-  while (bn < 256 && long(n_ft) * groups * ((rows + bn - 1) / bn) > sms) bn += 16;
+// tokens) that leaves the launch one wave.  `tail`: tiles that a call may have on top of its rows (segments that end
+// inside a tile).  Few rows are one tile, whichever expert they go to.
+inline int mid_tile(int rows, int longest, int n_ft, int tail, int sms) {
+  int bn = longest <= 64 ? (longest + 15) / 16 * 16 : 64;
+  while (bn < 256 && long(n_ft) * ((rows + bn - 1) / bn + tail) > sms) bn += 16;
   return bn;
 }
 
@@ -107,13 +108,11 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   const bool mid = !small && N <= MID_TOKENS;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
-  // an expert sees about half of the tokens: tiles and their stride for that, more tiles are looped over
-  const int half = N <= 32 ? N : (N + 1) / 2 + N / 16;
   auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
-                      const int32_t* seg, const int64_t* ids, const int32_t* sc, int epi, void* dst, bool seg_settled) {
-    const int rows = seg ? half : M;
-    const int bn = mid_tile(rows, n_out / 128, G, sms);
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, (rows + bn - 1) / bn, true, seg_settled, st);
+                      const int32_t* seg, const int64_t* ids, const int32_t* sc, int epi, void* dst) {
+    // grouped: M rows in all, at most N of them one expert's; every expert over all rows: G times M rows
+    const int bn = mid_tile(seg ? M : G * M, seg ? N : M, n_out / 128, seg ? G / 2 : 0, sms);
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, true, st);
   };
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
@@ -149,7 +148,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, N, true, st));
     else if (mid)
-      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, false));
+      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv));
     else
       JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
@@ -160,7 +159,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, N, true, st));
     else if (mid)
-      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, false));
+      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x));
     else
       JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st));
 
@@ -172,20 +171,20 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       if (small)
         JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, N, true, st));
       else
-        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, false));
+        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid));
     } else {
       JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st));
       JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
       JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
-        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid, true));
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid));
       else
         JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, N, true, st));
     else if (mid)
-      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, true));
+      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y));
     else
       JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st));
 

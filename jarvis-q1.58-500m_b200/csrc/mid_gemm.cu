@@ -4,8 +4,9 @@
 // With one or two tiles per SM nothing amortises a pipeline's fill: ternary_gemm_kernel takes 11-18 us for products whose
 // arithmetic is ~1 us, because every K-block of its four-stage ring waits for a code load from L2, the decode, the MMA
 // and the stage's release one after another (~550 cycles), after TMEM, barriers and tensor maps have been set up.  Here
-//   - a CTA owns (out-feature tile, expert) and takes token tiles from a stride, so its weights are known from the grid: in
-//     a chain their codes are loaded and decoded into every stage there is before the grid dependency is waited for;
+//   - the work is a list of (token tile, out-feature tile) items that every CTA reads off the segment offsets; those were
+//     complete before the kernel ahead on the stream began, so a CTA knows its weights at once and decodes them into every
+//     stage there is before the grid dependency is waited for;
 //   - K-blocks travel in chunks of CK: one TMA copy, one barrier wait and one commit per chunk (issued singly they cost
 //     ~290, ~95 and ~100 cycles next to 4 x 40-48 cycles for a K-block's MMAs), with as many chunks in flight as fit
 //     (a smaller ring that lets two CTAs share an SM and prologues overlap measured 5-15 % slower);
@@ -33,8 +34,8 @@ struct MidParams {
   const int64_t* idx;          // [M][2]: row n of group g goes to out row scatter[2n + k] where idx[2n + k] == g; null: row n
   const int32_t* scatter;
   void* out;
-  int M, N, K, alpha_rows, bn, chunks, epilogue;
-  int settled, seg_settled;    // weights / segments were complete before the kernel ahead of this one started
+  int M, N, K, G, n_ft, alpha_rows, bn, chunks, epilogue;
+  int settled;                 // weights and segments were complete before the kernel ahead of this one started
   uint32_t tmem_cols;
   unsigned int* status;
 };
@@ -42,6 +43,32 @@ struct MidParams {
 struct Ctl {
   uint64_t full[MAX_CHUNKS], empty[MAX_CHUNKS], acc_full, acc_empty;
   uint32_t tmem_base, abort_flag;
+  int32_t beg[MAX_GROUPS], end[MAX_GROUPS], first[MAX_GROUPS + 1];   // a group's rows and its first token tile
+};
+
+// The items of a CTA: a token tile (rows [tok0, end) of group grp, at most bn of them) and an out-feature tile, the latter
+// varying fastest.  The first one is worked out before the grid dependency is waited for; after it, only a CTA that has
+// another item pays for the division.
+struct Items {
+  int i, grp, tok0, end, ft;
+  __device__ __forceinline__ bool at(const MidParams& p, const Ctl& ctl) {
+    if (i >= ctl.first[p.G] * p.n_ft) return false;
+    const int t = i / p.n_ft;
+    ft = i - t * p.n_ft;
+    grp = 0;
+    while (t >= ctl.first[grp + 1]) ++grp;
+    tok0 = ctl.beg[grp] + (t - ctl.first[grp]) * p.bn;
+    end = ctl.end[grp];
+    return true;
+  }
+  __device__ __forceinline__ bool first(const MidParams& p, const Ctl& ctl) {
+    i = blockIdx.x;
+    return at(p, ctl);
+  }
+  __device__ __forceinline__ bool next(const MidParams& p, const Ctl& ctl) {
+    i += gridDim.x;
+    return at(p, ctl);
+  }
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -55,7 +82,6 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
   const int S = p.chunks, n_ch = p.K / (BK * CK);
   const uint32_t kb_bytes = uint32_t(p.bn) * BK * 2, b_bytes = kb_bytes * CK;
   const uint32_t b_base = base + uint32_t(S) * (CK * A_BYTES);
-  const int ft = blockIdx.x, grp = blockIdx.y;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -73,36 +99,53 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
     tmem_alloc(smem_u32(&ctl.tmem_base), p.tmem_cols);
     tmem_relinquish();
   }
+  if (!p.settled) {
+    pdl_wait();
+    pdl_trigger();
+  }
+  if (warp == 1) {
+    static_assert(MAX_GROUPS <= 32, "one lane per group");
+    int beg = 0, end = 0;
+    if (lane < p.G) {
+      beg = p.seg ? min(max(__ldg(p.seg + lane), 0), p.M) : 0;
+      end = p.seg ? min(max(__ldg(p.seg + lane + 1), 0), p.M) : p.M;
+    }
+    int tiles = end > beg ? (end - beg + p.bn - 1) / p.bn : 0;
+    for (int d = 1; d < MAX_GROUPS; d *= 2) {
+      const int u = __shfl_up_sync(0xffffffffu, tiles, d);
+      if (lane >= d) tiles += u;
+    }
+    if (lane < p.G) {
+      ctl.beg[lane] = beg;
+      ctl.end[lane] = end;
+      ctl.first[lane + 1] = tiles;
+    }
+    if (lane == 0) ctl.first[0] = 0;
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
-  int beg = 0, end = p.M;
-  auto segment = [&]() {
-    if (p.seg) {
-      beg = min(max(__ldg(p.seg + grp), 0), p.M);
-      end = min(max(__ldg(p.seg + grp + 1), 0), p.M);
-    }
-  };
-
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (p.seg_settled) segment();
-    pdl_wait();
-    pdl_trigger();
-    if (!p.seg_settled) segment();
+    Items it;
+    bool more = it.first(p, ctl);
+    if (p.settled) {
+      pdl_wait();
+      pdl_trigger();
+    }
     int s = 0;
     uint32_t ph = 1u;
     bool ok = true;
-    for (int tok0 = beg + int(blockIdx.z) * p.bn; ok && tok0 < end; tok0 += int(gridDim.z) * p.bn) {
+    for (; ok && more; more = it.next(p, ctl)) {
 #pragma unroll 1
       for (int c = 0; c < n_ch; ++c) {
         const uint32_t full = smem_u32(&ctl.full[s]);
         if (!mbar_wait(smem_u32(&ctl.empty[s]), ph, abort_flag, p.status, JB200_STATUS_GEMM_PRODUCER)) { ok = false; break; }
         if (elect_one()) {
           mbar_arrive_expect_tx(full, b_bytes);
-          tma_load_3d(b_base + uint32_t(s) * b_bytes, &tmap_x, 0, tok0, c * CK, full);
+          tma_load_3d(b_base + uint32_t(s) * b_bytes, &tmap_x, 0, it.tok0, c * CK, full);
         }
         __syncwarp();
         if (++s == S) { s = 0; ph ^= 1u; }
@@ -110,17 +153,19 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (p.seg_settled) segment();
-    pdl_wait();
-    pdl_trigger();
-    if (!p.seg_settled) segment();
+    Items it;
+    bool more = it.first(p, ctl);
+    if (p.settled) {
+      pdl_wait();
+      pdl_trigger();
+    }
     const uint32_t idesc = umma_idesc_bf16(BM, p.bn);
     const uint64_t adesc0 = umma_desc_k_sw128(base), bdesc0 = umma_desc_k_sw128(b_base);
     uint64_t ad = adesc0, bd = bdesc0;
     int s = 0;
     uint32_t ph = 0u, tile = 0u;
     bool ok = true;
-    for (int tok0 = beg + int(blockIdx.z) * p.bn; ok && tok0 < end; tok0 += int(gridDim.z) * p.bn, ++tile) {
+    for (; ok && more; more = it.next(p, ctl), ++tile) {
       if (!mbar_wait(smem_u32(&ctl.acc_empty), (tile & 1u) ^ 1u, abort_flag, p.status, JB200_STATUS_GEMM_MMA)) break;
       tc_fence_after_sync();
 #pragma unroll 1
@@ -148,7 +193,12 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
     // ---------------- decoders, then epilogue ----------------
     const int par = (warp - DEC_WARP0) >> 2;                       // this thread decodes K-block par of every chunk,
     const int r = ((warp - DEC_WARP0) & 3) * 32 + lane;             // weight row r of the tile
-    const uint8_t* wrow = p.w + (size_t(grp) * p.N + size_t(ft) * BM + r) * (size_t(p.K) / 4) + par * 16;
+    const uint8_t* wrow = nullptr;
+    float alpha = 0.f;
+    auto weights_of = [&](const Items& it) {
+      wrow = p.w + (size_t(it.grp) * p.N + size_t(it.ft) * BM + r) * (size_t(p.K) / 4) + par * 16;
+      alpha = 0.5f * __ldg(p.alpha + size_t(it.grp) * (p.N / p.alpha_rows) + (it.ft * BM) / p.alpha_rows);   // codes decode to +-2
+    };
     const uint32_t swz = uint32_t(r & 7);
     uint4 code[SLOTS];
     auto load_codes = [&](int u, int c) {
@@ -190,42 +240,40 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
       }
     };
     const int fresh = S < n_ch ? S : n_ch;           // chunks that go into unused slots
-    if (p.settled) {
+    Items it;
+    bool more = it.first(p, ctl);
+    if (more) {
+      weights_of(it);
       start_codes();
       decode_to(fresh, true);
     }
-    const float alpha = 0.5f * __ldg(p.alpha + size_t(grp) * (p.N / p.alpha_rows) + (ft * BM) / p.alpha_rows);   // codes decode to +-2
-    if (p.seg_settled) segment();
     __syncwarp();
-    pdl_wait();
-    pdl_trigger();
-    if (!p.settled) {
-      start_codes();
-      decode_to(fresh, true);
+    if (p.settled) {
+      pdl_wait();
+      pdl_trigger();
     }
-    if (!p.seg_settled) segment();
     const int q4 = warp & 3;                         // TMEM lane quadrant of this warp
-    const int f0 = ft * BM + q4 * 32;
     uint32_t tile = 0u;
-    for (int tok0 = beg + int(blockIdx.z) * p.bn; ok && tok0 < end; tok0 += int(gridDim.z) * p.bn, ++tile) {
-      if (tile > 0) {                                // a further tile: the same weights again
+    for (; ok && more; more = it.next(p, ctl), ++tile) {
+      if (tile > 0) {
         c = 0;
+        weights_of(it);
         start_codes();
       }
       decode_to(n_ch, false);
       if (!ok) break;
-      const int n = min(p.bn, end - tok0);
+      const int n = min(p.bn, it.end - it.tok0), f0 = it.ft * BM + q4 * 32;
       if (!mbar_wait(smem_u32(&ctl.acc_full), tile & 1u, abort_flag, p.status, JB200_STATUS_GEMM_EPILOGUE)) break;
       tc_fence_after_sync();
       __syncwarp();
 #pragma unroll 1
       for (int c0 = par * 32; c0 < n; c0 += 64) {
         // output row of token c0 + lane; -1: not stored
-        int row = c0 + lane < n ? tok0 + c0 + lane : -1;
+        int row = c0 + lane < n ? it.tok0 + c0 + lane : -1;
         if (p.idx && row >= 0) {
           const longlong2 e = *reinterpret_cast<const longlong2*>(p.idx + 2 * row);
           const int2 sc = *reinterpret_cast<const int2*>(p.scatter + 2 * row);
-          row = e.x == grp ? sc.x : (e.y == grp ? sc.y : -1);
+          row = e.x == it.grp ? sc.x : (e.y == it.grp ? sc.y : -1);
           if (row >= 2 * p.M) row = -1;
         }
         __syncwarp();
@@ -276,15 +324,15 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
 }  // namespace
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int z,
-                    bool settled, bool seg_settled, cudaStream_t stream) {
-  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn <= 256 && bn % 16 == 0 && z >= 1,
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, bool settled,
+                    cudaStream_t stream) {
+  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn <= 256 && bn % 16 == 0 &&
+                 G >= 1 && G <= MAX_GROUPS,
              "mid_gemm: bad shape (M=%d, N=%d, K=%d, bn=%d)", M, N, K, bn);
   MidParams p;
   p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
-  p.M = M; p.N = N; p.K = K; p.alpha_rows = alpha_rows; p.bn = bn; p.epilogue = epilogue;
+  p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / BM; p.alpha_rows = alpha_rows; p.bn = bn; p.epilogue = epilogue;
   p.settled = settled ? 1 : 0;
-  p.seg_settled = seg_settled ? 1 : 0;
   p.tmem_cols = bn <= 32 ? 32u : bn <= 64 ? 64u : bn <= 128 ? 128u : 256u;
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
@@ -300,8 +348,11 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   const int rc = encode_tiled(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, x_bf16, gdim, gstride, box, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "mid_gemm");
   if (rc != JB200_OK) return rc;
+  const int sms = sm_count();
+  if (sms <= 0) return JB200_ERR_CUDA;
+  const long tiles = seg ? (M + bn - 1) / bn + G - 1 : long(G) * ((M + bn - 1) / bn), items = tiles * (N / BM);   // at most
   JB_MAX_SMEM(mid_gemm_kernel, 225 * 1024);
-  launch_dep(mid_gemm_kernel, dim3(N / BM, G, z), THREADS, size_t(S) * CK * kb_bytes + 1024, stream, tmap, p);
+  launch_dep(mid_gemm_kernel, dim3(unsigned(items < sms ? items : sms)), THREADS, size_t(S) * CK * kb_bytes + 1024, stream, tmap, p);
   JB_LAUNCH_CHECK("mid_gemm_kernel");
   return JB200_OK;
 }
