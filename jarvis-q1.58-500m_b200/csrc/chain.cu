@@ -54,11 +54,10 @@ struct Workspace {
 // against 2.86), beyond that the persistent pipeline.
 constexpr int SMALL_TOKENS = 16, MID_TOKENS = 640;
 // Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
-// tokens) that leaves the launch one wave.  `tail`: tiles that a call may have on top of its rows (segments that end
-// inside a tile).  Few rows are one tile, whichever expert they go to.
-inline int mid_tile(int rows, int longest, int n_ft, int tail, int sms) {
-  int bn = longest <= 64 ? (longest + 15) / 16 * 16 : 64;
-  while (bn < 256 && long(n_ft) * ((rows + bn - 1) / bn + tail) > sms) bn += 16;
+// tokens) that leaves a launch of so many rows in each group one wave.
+inline int mid_tile(int rows, int groups, int n_ft, int sms) {
+  int bn = rows <= 64 ? (rows + 15) / 16 * 16 : 64;
+  while (bn < 256 && long(n_ft) * groups * ((rows + bn - 1) / bn) > sms) bn += 16;
   return bn;
 }
 
@@ -110,9 +109,17 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   if (sms <= 0) return JB200_ERR_CUDA;
   auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
                       const int32_t* seg, const int64_t* ids, const int32_t* sc, int epi, void* dst) {
-    // grouped: M rows in all, at most N of them one expert's; every expert over all rows: G times M rows
-    const int bn = mid_tile(seg ? M : G * M, seg ? N : M, n_out / 128, seg ? G / 2 : 0, sms);
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, true, st);
+    const int n_ft = n_out / 128;
+    if (!seg) {                                // every group over all rows
+      const int bn = mid_tile(M, G, n_ft, sms);
+      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn, true, st);
+    }
+    // Segments are known on the device alone: a tile for rows that are spread evenly, with an eighth to spare, and one for
+    // whatever they are (M / bn_max tiles and one cut short in every other group).
+    const int even = (M + G - 1) / G, bn = mid_tile(even + (even + 7) / 8, G, n_ft, sms);
+    int bn_max = bn;
+    while (bn_max < 256 && long(n_ft) * ((M + bn_max - 1) / bn_max + G - 1) > sms) bn_max += 16;
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn_max, true, st);
   };
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves

@@ -32,9 +32,10 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
 int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
                       int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
                       int tokens, bool settled, cudaStream_t stream);
-// The same product again, latency form on tcgen05 (mid_gemm.cu) with token tiles of bn rows.  Arguments as launch_small_gemm.
+// The same product again, latency form on tcgen05 (mid_gemm.cu) with token tiles of bn rows, or of bn_max rows
+// where the segments need more tiles of bn than there are SMs.  Arguments as launch_small_gemm.
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, bool settled,
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int bn_max, bool settled,
                     cudaStream_t stream);
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);

@@ -14,6 +14,8 @@
 //   - the eight decoder warps become the epilogue; the residual is added by reductions, nothing waits for old values.
 // What is left is the chain itself: 4 x 40-48 cycles per K-block.  Accumulation is the same chain of K = 16 steps as in
 // ternary_gemm_kernel: results are its bit for bit.
+#include <algorithm>
+
 #include "common.cuh"
 #include "gemm_shared.cuh"
 #include "launchers.h"
@@ -34,15 +36,21 @@ struct MidParams {
   const int64_t* idx;          // [M][2]: row n of group g goes to out row scatter[2n + k] where idx[2n + k] == g; null: row n
   const int32_t* scatter;
   void* out;
-  int M, N, K, G, n_ft, alpha_rows, bn, chunks, epilogue;
+  int M, N, K, G, n_ft, alpha_rows, epilogue;
+  int bn[2], chunks[2];        // token tile and ring: the first one where its items are one wave, else the second
   int settled;                 // weights and segments were complete before the kernel ahead of this one started
   uint32_t tmem_cols;
   unsigned int* status;
 };
 
+struct Maps {
+  CUtensorMap x[2];            // one box per token tile
+};
+
 struct Ctl {
   uint64_t full[MAX_CHUNKS], empty[MAX_CHUNKS], acc_full, acc_empty;
   uint32_t tmem_base, abort_flag;
+  int pick;
   int32_t beg[MAX_GROUPS], end[MAX_GROUPS], first[MAX_GROUPS + 1];   // a group's rows and its first token tile
 };
 
@@ -51,40 +59,37 @@ struct Ctl {
 // another item pays for the division.
 struct Items {
   int i, grp, tok0, end, ft;
-  __device__ __forceinline__ bool at(const MidParams& p, const Ctl& ctl) {
+  __device__ __forceinline__ bool at(const MidParams& p, const Ctl& ctl, int bn) {
     if (i >= ctl.first[p.G] * p.n_ft) return false;
     const int t = i / p.n_ft;
     ft = i - t * p.n_ft;
     grp = 0;
     while (t >= ctl.first[grp + 1]) ++grp;
-    tok0 = ctl.beg[grp] + (t - ctl.first[grp]) * p.bn;
+    tok0 = ctl.beg[grp] + (t - ctl.first[grp]) * bn;
     end = ctl.end[grp];
     return true;
   }
-  __device__ __forceinline__ bool first(const MidParams& p, const Ctl& ctl) {
+  __device__ __forceinline__ bool first(const MidParams& p, const Ctl& ctl, int bn) {
     i = blockIdx.x;
-    return at(p, ctl);
+    return at(p, ctl, bn);
   }
-  __device__ __forceinline__ bool next(const MidParams& p, const Ctl& ctl) {
+  __device__ __forceinline__ bool next(const MidParams& p, const Ctl& ctl, int bn) {
     i += gridDim.x;
-    return at(p, ctl);
+    return at(p, ctl, bn);
   }
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
-mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
+mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Ctl ctl;
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw_addr);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int S = p.chunks, n_ch = p.K / (BK * CK);
-  const uint32_t kb_bytes = uint32_t(p.bn) * BK * 2, b_bytes = kb_bytes * CK;
-  const uint32_t b_base = base + uint32_t(S) * (CK * A_BYTES);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
+    for (int s = 0; s < MAX_CHUNKS; ++s) {
       mbar_init(smem_u32(&ctl.full[s]), 1 + 8);      // the producer's expectation and the eight decoder warps
       mbar_init(smem_u32(&ctl.empty[s]), 1);
     }
@@ -92,7 +97,7 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
     mbar_init(smem_u32(&ctl.acc_empty), 8);
     ctl.abort_flag = 0;
     fence_mbar_init();
-    tma_prefetch_desc(&tmap_x);
+    tma_prefetch_desc(&maps.x[0]);
   }
   if (warp == 0) {
     __syncwarp();                 // tcgen05.alloc is warp-collective: lane 0 rejoins from the barrier set-up first
@@ -110,27 +115,41 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
       beg = p.seg ? min(max(__ldg(p.seg + lane), 0), p.M) : 0;
       end = p.seg ? min(max(__ldg(p.seg + lane + 1), 0), p.M) : p.M;
     }
-    int tiles = end > beg ? (end - beg + p.bn - 1) / p.bn : 0;
-    for (int d = 1; d < MAX_GROUPS; d *= 2) {
-      const int u = __shfl_up_sync(0xffffffffu, tiles, d);
-      if (lane >= d) tiles += u;
-    }
+    auto tiles_of = [&](int bn) {              // token tiles of groups 0..lane
+      int t = end > beg ? (end - beg + bn - 1) / bn : 0;
+      for (int d = 1; d < MAX_GROUPS; d *= 2) {
+        const int u = __shfl_up_sync(0xffffffffu, t, d);
+        if (lane >= d) t += u;
+      }
+      return t;
+    };
+    int tiles = tiles_of(p.bn[0]);
+    const int pick = p.bn[1] != p.bn[0] && __shfl_sync(0xffffffffu, tiles, p.G - 1) * p.n_ft > int(gridDim.x);
+    if (pick) tiles = tiles_of(p.bn[1]);
     if (lane < p.G) {
       ctl.beg[lane] = beg;
       ctl.end[lane] = end;
       ctl.first[lane + 1] = tiles;
     }
-    if (lane == 0) ctl.first[0] = 0;
+    if (lane == 0) {
+      ctl.first[0] = 0;
+      ctl.pick = pick;
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
+  const bool alt = __any_sync(0xffffffffu, ctl.pick);      // a vote: uniform registers, which MMAs and copies are issued from
+  const int bn = alt ? p.bn[1] : p.bn[0], S = alt ? p.chunks[1] : p.chunks[0], n_ch = p.K / (BK * CK);
+  const uint32_t kb_bytes = uint32_t(bn) * BK * 2, b_bytes = kb_bytes * CK;
+  const uint32_t b_base = base + uint32_t(S) * (CK * A_BYTES);
+  const CUtensorMap* tmap_x = alt ? &maps.x[1] : &maps.x[0];
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     Items it;
-    bool more = it.first(p, ctl);
+    bool more = it.first(p, ctl, bn);
     if (p.settled) {
       pdl_wait();
       pdl_trigger();
@@ -138,14 +157,14 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
     int s = 0;
     uint32_t ph = 1u;
     bool ok = true;
-    for (; ok && more; more = it.next(p, ctl)) {
+    for (; ok && more; more = it.next(p, ctl, bn)) {
 #pragma unroll 1
       for (int c = 0; c < n_ch; ++c) {
         const uint32_t full = smem_u32(&ctl.full[s]);
         if (!mbar_wait(smem_u32(&ctl.empty[s]), ph, abort_flag, p.status, JB200_STATUS_GEMM_PRODUCER)) { ok = false; break; }
         if (elect_one()) {
           mbar_arrive_expect_tx(full, b_bytes);
-          tma_load_3d(b_base + uint32_t(s) * b_bytes, &tmap_x, 0, it.tok0, c * CK, full);
+          tma_load_3d(b_base + uint32_t(s) * b_bytes, tmap_x, 0, it.tok0, c * CK, full);
         }
         __syncwarp();
         if (++s == S) { s = 0; ph ^= 1u; }
@@ -154,18 +173,18 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     Items it;
-    bool more = it.first(p, ctl);
+    bool more = it.first(p, ctl, bn);
     if (p.settled) {
       pdl_wait();
       pdl_trigger();
     }
-    const uint32_t idesc = umma_idesc_bf16(BM, p.bn);
+    const uint32_t idesc = umma_idesc_bf16(BM, bn);
     const uint64_t adesc0 = umma_desc_k_sw128(base), bdesc0 = umma_desc_k_sw128(b_base);
     uint64_t ad = adesc0, bd = bdesc0;
     int s = 0;
     uint32_t ph = 0u, tile = 0u;
     bool ok = true;
-    for (; ok && more; more = it.next(p, ctl), ++tile) {
+    for (; ok && more; more = it.next(p, ctl, bn), ++tile) {
       if (!mbar_wait(smem_u32(&ctl.acc_empty), (tile & 1u) ^ 1u, abort_flag, p.status, JB200_STATUS_GEMM_MMA)) break;
       tc_fence_after_sync();
 #pragma unroll 1
@@ -241,7 +260,7 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
     };
     const int fresh = S < n_ch ? S : n_ch;           // chunks that go into unused slots
     Items it;
-    bool more = it.first(p, ctl);
+    bool more = it.first(p, ctl, bn);
     if (more) {
       weights_of(it);
       start_codes();
@@ -254,7 +273,7 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
     }
     const int q4 = warp & 3;                         // TMEM lane quadrant of this warp
     uint32_t tile = 0u;
-    for (; ok && more; more = it.next(p, ctl), ++tile) {
+    for (; ok && more; more = it.next(p, ctl, bn), ++tile) {
       if (tile > 0) {
         c = 0;
         weights_of(it);
@@ -262,7 +281,7 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
       }
       decode_to(n_ch, false);
       if (!ok) break;
-      const int n = min(p.bn, it.end - it.tok0), f0 = it.ft * BM + q4 * 32;
+      const int n = min(bn, it.end - it.tok0), f0 = it.ft * BM + q4 * 32;
       if (!mbar_wait(smem_u32(&ctl.acc_full), tile & 1u, abort_flag, p.status, JB200_STATUS_GEMM_EPILOGUE)) break;
       tc_fence_after_sync();
       __syncwarp();
@@ -324,35 +343,42 @@ mid_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MidParams p) {
 }  // namespace
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, bool settled,
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int bn_max, bool settled,
                     cudaStream_t stream) {
-  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn <= 256 && bn % 16 == 0 &&
+  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn % 16 == 0 &&
+                 bn_max >= bn && bn_max <= 256 && bn_max % 16 == 0 &&
                  G >= 1 && G <= MAX_GROUPS,
              "mid_gemm: bad shape (M=%d, N=%d, K=%d, bn=%d)", M, N, K, bn);
   MidParams p;
   p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
-  p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / BM; p.alpha_rows = alpha_rows; p.bn = bn; p.epilogue = epilogue;
+  p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / BM; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
   p.settled = settled ? 1 : 0;
-  p.tmem_cols = bn <= 32 ? 32u : bn <= 64 ? 64u : bn <= 128 ? 128u : 256u;
+  p.tmem_cols = bn_max <= 32 ? 32u : bn_max <= 64 ? 64u : bn_max <= 128 ? 128u : 256u;
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
-  const int n_kb = K / BK, kb_bytes = A_BYTES + bn * BK * 2;
-  int S = (224 * 1024) / (CK * kb_bytes);
-  if (S > MAX_CHUNKS) S = MAX_CHUNKS;
-  if (S > n_kb / CK) S = n_kb / CK;
-  p.chunks = S;
-  CUtensorMap tmap;                            // [K-block][token][64]: one copy takes the same rows of CK K-blocks
+  const int n_kb = K / BK;
+  Maps maps;                                   // [K-block][token][64]: one copy takes the same rows of CK K-blocks
   const cuuint64_t gdim[3] = {cuuint64_t(BK), cuuint64_t(M), cuuint64_t(n_kb)};
   const cuuint64_t gstride[2] = {cuuint64_t(K) * 2, cuuint64_t(BK) * 2};
-  const cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(bn), cuuint32_t(CK)};
-  const int rc = encode_tiled(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, x_bf16, gdim, gstride, box, CU_TENSOR_MAP_SWIZZLE_128B,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "mid_gemm");
-  if (rc != JB200_OK) return rc;
+  size_t smem = 0;
+  for (int i = 0; i < 2; ++i) {
+    p.bn[i] = i ? bn_max : bn;
+    const int chunk = CK * (A_BYTES + p.bn[i] * BK * 2);
+    int S = (224 * 1024) / chunk;
+    if (S > MAX_CHUNKS) S = MAX_CHUNKS;
+    if (S > n_kb / CK) S = n_kb / CK;
+    p.chunks[i] = S;
+    smem = std::max(smem, size_t(S) * chunk + 1024);
+    const cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(p.bn[i]), cuuint32_t(CK)};
+    const int rc = encode_tiled(&maps.x[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, x_bf16, gdim, gstride, box,
+                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "mid_gemm");
+    if (rc != JB200_OK) return rc;
+  }
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
-  const long tiles = seg ? (M + bn - 1) / bn + G - 1 : long(G) * ((M + bn - 1) / bn), items = tiles * (N / BM);   // at most
+  const long tiles = seg ? (M + bn - 1) / bn + G - 1 : long(G) * ((M + bn - 1) / bn), items = tiles * p.n_ft;   // at most
   JB_MAX_SMEM(mid_gemm_kernel, 225 * 1024);
-  launch_dep(mid_gemm_kernel, dim3(unsigned(items < sms ? items : sms)), THREADS, size_t(S) * CK * kb_bytes + 1024, stream, tmap, p);
+  launch_dep(mid_gemm_kernel, dim3(unsigned(items < sms ? items : sms)), THREADS, smem, stream, maps, p);
   JB_LAUNCH_CHECK("mid_gemm_kernel");
   return JB200_OK;
 }
