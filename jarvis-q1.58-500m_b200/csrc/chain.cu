@@ -50,9 +50,9 @@ struct Workspace {
 
 // Which form of the ternary product a call of so many tokens runs (their results are the same bits): up to 16 tokens
 // mma.sync straight from the codes (24 layers of single-token steps 0.62 against 0.86 ms at 1 sequence, equal at 16), up to
-// MID_TOKENS the tcgen05 form that is built for latency (256 tokens 1.90 against 2.12 ms, 512 2.46 against 2.57, 777 2.91
-// against 2.86), beyond that the persistent pipeline.
-constexpr int SMALL_TOKENS = 16, MID_TOKENS = 640;
+// MID_TOKENS the tcgen05 form that is built for latency (512 tokens 2.15 against 2.54 ms, 1024 2.65 against 2.75, 1280 equal,
+// 1500 3.13 against 3.08), beyond that the persistent pipeline.
+constexpr int SMALL_TOKENS = 16, MID_TOKENS = 1280;
 // Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
 // tokens) that leaves a launch of so many rows in each group one wave.
 inline int mid_tile(int rows, int groups, int n_ft, int sms) {

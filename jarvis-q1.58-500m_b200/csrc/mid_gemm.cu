@@ -37,14 +37,14 @@ struct MidParams {
   const int32_t* scatter;
   void* out;
   int M, N, K, G, n_ft, alpha_rows, epilogue;
-  int bn[2], chunks[2];        // token tile and ring: the first one where its items are one wave, else the second
+  int bn[3], chunks[3];        // token tiles and their rings: the first whose items are one wave, else the last
   int settled;                 // weights and segments were complete before the kernel ahead of this one started
   uint32_t tmem_cols;
   unsigned int* status;
 };
 
 struct Maps {
-  CUtensorMap x[2];            // one box per token tile
+  CUtensorMap x[3];            // one box per token tile
 };
 
 struct Ctl {
@@ -123,9 +123,11 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
       }
       return t;
     };
-    int tiles = tiles_of(p.bn[0]);
-    const int pick = p.bn[1] != p.bn[0] && __shfl_sync(0xffffffffu, tiles, p.G - 1) * p.n_ft > int(gridDim.x);
-    if (pick) tiles = tiles_of(p.bn[1]);
+    int pick = 0, tiles = tiles_of(p.bn[0]);
+    while (pick < 2 && p.bn[2] != p.bn[0] && __shfl_sync(0xffffffffu, tiles, p.G - 1) * p.n_ft > int(gridDim.x)) {
+      ++pick;
+      tiles = tiles_of(pick == 1 ? p.bn[1] : p.bn[2]);
+    }
     if (lane < p.G) {
       ctl.beg[lane] = beg;
       ctl.end[lane] = end;
@@ -141,11 +143,14 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   tc_fence_after_sync();
   const uint32_t tmem = ctl.tmem_base;
   volatile uint32_t* abort_flag = &ctl.abort_flag;
-  const bool alt = __any_sync(0xffffffffu, ctl.pick);      // a vote: uniform registers, which MMAs and copies are issued from
-  const int bn = alt ? p.bn[1] : p.bn[0], S = alt ? p.chunks[1] : p.chunks[0], n_ch = p.K / (BK * CK);
+  // votes: their results are in uniform registers, which copies and MMAs are issued from (a value read from shared memory
+  // there cost 1.8 us a launch)
+  const bool t1 = __any_sync(0xffffffffu, ctl.pick == 1), t2 = __any_sync(0xffffffffu, ctl.pick == 2);
+  const int bn = t2 ? p.bn[2] : t1 ? p.bn[1] : p.bn[0], n_ch = p.K / (BK * CK);
+  const int S = t2 ? p.chunks[2] : t1 ? p.chunks[1] : p.chunks[0];
   const uint32_t kb_bytes = uint32_t(bn) * BK * 2, b_bytes = kb_bytes * CK;
   const uint32_t b_base = base + uint32_t(S) * (CK * A_BYTES);
-  const CUtensorMap* tmap_x = alt ? &maps.x[1] : &maps.x[0];
+  const CUtensorMap* tmap_x = t2 ? &maps.x[2] : t1 ? &maps.x[1] : &maps.x[0];
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     Items it;
@@ -361,8 +366,8 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   const cuuint64_t gdim[3] = {cuuint64_t(BK), cuuint64_t(M), cuuint64_t(n_kb)};
   const cuuint64_t gstride[2] = {cuuint64_t(K) * 2, cuuint64_t(BK) * 2};
   size_t smem = 0;
-  for (int i = 0; i < 2; ++i) {
-    p.bn[i] = i ? bn_max : bn;
+  for (int i = 0; i < 3; ++i) {
+    p.bn[i] = i == 0 ? bn : i == 1 ? (bn + bn_max) / 32 * 16 : bn_max;
     const int chunk = CK * (A_BYTES + p.bn[i] * BK * 2);
     int S = (224 * 1024) / chunk;
     if (S > MAX_CHUNKS) S = MAX_CHUNKS;

@@ -88,9 +88,9 @@ def test_cross_entropy_matches_torch(rows, V, ld):
 
 @pytest.mark.parametrize("B,T", [(1, 1), (4, 1), (5, 1), (8, 1), (9, 1), (16, 1), (17, 1), (33, 1), (64, 1), (65, 1), (128, 1),
                                  (129, 1), (1, 2), (3, 3), (1, 16), (2, 20), (1, 64), (1, 65), (2, 64), (1, 128), (1, 129),
-                                 (1, 640), (1, 641)])
+                                 (1, 640), (1, 641), (1, 1280), (1, 1281)])
 def test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T):
-    """d_model 1024: the kernels for few tokens (GEMM forms up to 16, up to 640 and beyond, router up to 64, row cluster up to
+    """d_model 1024: the kernels for few tokens (GEMM forms up to 16, up to 1280 and beyond, router up to 64, row cluster up to
     128) against the kernel-by-kernel path; mixed routing, carried state, one expert without tokens at the smallest sizes."""
     from jarvis_b200 import chain
     torch.manual_seed(7)
@@ -113,4 +113,24 @@ def test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T):
     for got, ref in zip((counts, offsets, scatter, gather, gate_idx), want):
         assert torch.equal(got, ref)                                          # dispatch order: bit-exact
     assert int(torch.bincount(idx.flatten(), minlength=4).sum()) == 2 * B * T
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("skew", [0.5, 4.0])
+@pytest.mark.parametrize("T", [17, 64, 129, 256, 640, 1280])
+def test_chain_with_uneven_experts(T, skew):
+    """Tokens that lean one way go to the same experts: token tiles beyond an even share, groups without rows."""
+    from jarvis_b200 import chain
+    torch.manual_seed(7)
+    blk = jm.ternary_init_(jm.JarvisBlock(1024, 16, max_seq_len=2048)).cuda().eval()
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, 1024, generator=gen, device="cuda") + skew * torch.randn(1, 1024, generator=gen, device="cuda")
+    norm = (torch.ones(1024, device="cuda"), 1e-6)
+    xa, xb = x.clone(), x.clone()
+    acc, hist = torch.zeros(6, dtype=torch.float64, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    blk.forward_rows(xa, 1, T, None, 0, None, scratch=(acc, hist, torch.zeros(3, device="cuda")))
+    chain.run(chain.table_of(blk, [blk]), xb, 1, T, start_pos=0, final_norm=norm)
+    assert rel(xb, xa) < TOL
+    counts = torch.bincount(blk.moe.last_routing[0].flatten(), minlength=4)
+    assert int(counts.max()) > T * (5 if skew < 1 else 8) // 10, counts
     assert _lib.device_status() == 0
