@@ -24,6 +24,8 @@
 // travel by TMA (cp.async.bulk.tensor) through a ring of shared-memory stages - loads complete on mbarriers
 // (bounded waits), results are written into the tile in place and leave by a TMA store - so the bytes in flight
 // no longer depend on how many registers a thread can spare for outstanding loads.
+#include <type_traits>
+
 #include "common.cuh"
 #include "gemm_shared.cuh"
 #include "moe_finalize.cuh"
@@ -53,14 +55,25 @@ struct LsfParams {
   int n_pre_tiles;         // tiles in the non-final segments = (nseg - 1) * seg_len / tile
   float* seg_end;          // [B][n_pre_tiles][D] end value of each of those tiles from a zero carry
   float* seg_prod;         // [B][n_pre_tiles][D] product of its decays (tensor mode)
+};
+
+// What a chain's kernels get.  Kernels that no chain runs take LsfParams alone: with the accumulators among their
+// parameters per-element decays compiled to 182 registers instead of 255, fewer loads in flight and 287 us at 32 x 2048
+// instead of 273 (8 x 8192 in segments 80 us instead of 66).
+struct LsfChainParams : LsfParams {
   LsfStats st;             // st.stats != null: act_var comes from the MoE layer's accumulators
 };
+template <bool STATS>
+using LsfArgs = std::conditional_t<STATS, LsfChainParams, LsfParams>;
 
 // The scalar decay of a call (model semantics).  With st.stats the variance of the MoE output is derived here, as
 // moe_finalize_kernel would have, instead of in a launch of its own between the combine and the scan.
-__device__ __forceinline__ float lsf_decay(const LsfParams& p) {
+template <typename Args>
+__device__ __forceinline__ float lsf_decay(const Args& p) {
   if (p.alpha_s) return __ldg(p.alpha_s);
-  const float var = p.st.stats ? moe_act_var(p.st.stats, p.st.n_elems) : __ldg(p.act_var);
+  float var;
+  if constexpr (std::is_same_v<Args, LsfChainParams>) var = p.st.stats ? moe_act_var(p.st.stats, p.st.n_elems) : __ldg(p.act_var);
+  else var = __ldg(p.act_var);
   return lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), var);
 }
 // One thread of the whole grid leaves the MoE layer's scalars.
@@ -90,8 +103,8 @@ __device__ __forceinline__ void st2<__nv_bfloat16>(__nv_bfloat16* p, float a, fl
   *reinterpret_cast<uint32_t*>(p) = pack_bf16x2(a, b);
 }
 
-template <bool TENSOR_ALPHA, typename TM, typename TOut, int TPW, bool ENDS_ONLY>
-__global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_kernel(const LsfParams p) {
+template <bool TENSOR_ALPHA, typename TM, typename TOut, int TPW, bool ENDS_ONLY, bool STATS>
+__global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_kernel(const LsfArgs<STATS> p) {
   pdl_wait();
   pdl_trigger();
   __shared__ float2 s_end[2][LSF_WARPS][32];   // end value of each warp's run
@@ -106,9 +119,8 @@ __global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_ke
   TOut* out = reinterpret_cast<TOut*>(p.out);
 
   float alpha = 0.f, pw[TPW];  // scalar mode: pw[i] = alpha^(i+1)
-  if (!TENSOR_ALPHA) {
+  if constexpr (!TENSOR_ALPHA) {
     alpha = lsf_decay(p);
-    if (!ENDS_ONLY) lsf_leave_scalars(p.st);
     float a = alpha;
 #pragma unroll
     for (int i = 0; i < TPW; ++i) { pw[i] = a; a *= alpha; }
@@ -225,7 +237,7 @@ __global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_ke
 
 // Short sequences (decode steps): one thread per channel pair walks the few tokens itself.
 template <bool TENSOR_ALPHA, typename TM, typename TOut>
-__global__ void __launch_bounds__(256) lsf_short_kernel(const LsfParams p) {
+__global__ void __launch_bounds__(256) lsf_short_kernel(const LsfArgs<!TENSOR_ALPHA> p) {
   pdl_wait();
   pdl_trigger();
   const size_t pair = size_t(blockIdx.x) * 256 + threadIdx.x;
@@ -236,7 +248,7 @@ __global__ void __launch_bounds__(256) lsf_short_kernel(const LsfParams p) {
   const TM* at = reinterpret_cast<const TM*>(p.alpha_t);
   TOut* out = reinterpret_cast<TOut*>(p.out);
   float alpha = 0.f;
-  if (!TENSOR_ALPHA) {
+  if constexpr (!TENSOR_ALPHA) {
     alpha = lsf_decay(p);
     lsf_leave_scalars(p.st);
   }
@@ -335,7 +347,7 @@ constexpr int LSF_TPW = 16;                       // tokens per warp per tile
 constexpr int LSF_TILE = LSF_WARPS * LSF_TPW;     // 128 tokens
 
 template <bool TA, typename TM, typename TOut>
-int launch_t(const LsfParams& p, cudaStream_t stream) {
+int launch_t(const LsfChainParams& p, cudaStream_t stream) {
   if (p.T <= 8) {
     const size_t pairs = size_t(p.B) * (p.D / 2);
     launch_dep(lsf_short_kernel<TA, TM, TOut>, unsigned((pairs + 255) / 256), 256, 0, stream, p);
@@ -344,11 +356,11 @@ int launch_t(const LsfParams& p, cudaStream_t stream) {
   }
   if (p.nseg > 1) {
     dim3 grid_a((p.D + LSF_CH - 1) / LSF_CH, p.B, p.n_pre_tiles);
-    launch_dep(lsf_scan_kernel<TA, TM, TOut, LSF_TPW, true>, grid_a, LSF_THREADS, 0, stream, p);
+    launch_dep(lsf_scan_kernel<TA, TM, TOut, LSF_TPW, true, false>, grid_a, LSF_THREADS, 0, stream, p);
     JB_LAUNCH_CHECK("lsf_scan_kernel<ends>");
   }
   dim3 grid((p.D + LSF_CH - 1) / LSF_CH, p.B, p.nseg);
-  launch_dep(lsf_scan_kernel<TA, TM, TOut, LSF_TPW, false>, grid, LSF_THREADS, 0, stream, p);
+  launch_dep(lsf_scan_kernel<TA, TM, TOut, LSF_TPW, false, false>, grid, LSF_THREADS, 0, stream, p);
   JB_LAUNCH_CHECK("lsf_scan_kernel");
   return JB200_OK;
 }
@@ -376,7 +388,7 @@ struct LsfTma {
 
 template <bool FUSED>
 __global__ void __launch_bounds__(LSF_THREADS, FUSED ? 2 : 4)
-lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_io, const LsfParams p,
+lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_io, const LsfArgs<FUSED> p,
                const int n_stages, unsigned int* status) {
   pdl_wait();
   pdl_trigger();
@@ -401,7 +413,7 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
   const int n_tiles = (t_end - t_begin + LT_TOK - 1) / LT_TOK;
 
   const float alpha = lsf_decay(p);
-  lsf_leave_scalars(p.st);
+  if constexpr (FUSED) lsf_leave_scalars(p.st);
   float pw[TPW];   // alpha^(i+1)
   {
     float a = alpha;
@@ -505,6 +517,104 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
   if (threadIdx.x == 0) bulk_wait_group<0>();   // every store has landed before the CTA gives up its shared memory
 }
 
+// Fused form for sequences of 2 to 8 tiles where a CTA per (sequence, 64 channels) leaves the chip idle: those CTAs work
+// through their tiles one after another, ~2 us each (3 x 777 tokens: 15.4 us on 48 CTAs for 8 us worth of bytes), although only
+// the carry is sequential.  Here a cluster takes the tiles of a sequence side by side: every CTA scans its runs from zero,
+// sends their ends to the CTAs of the later tiles, and after one cluster barrier each works out its own carry along all
+// runs before it.  The chain of roundings is lsf_tma_kernel's, so are the results.  In a chain the residual tile and the
+// membrane are fetched before the grid dependency is waited for (`ahead`: the kernel before this one made only m).
+constexpr int LC_MAX_TILES = 8;
+constexpr size_t LC_END_BYTES = LSF_WARPS * 32 * sizeof(float2);      // run ends of one tile
+inline size_t lc_smem_bytes(int tiles) { return 128 + LT_M_BYTES + LT_R_BYTES + size_t(tiles) * LC_END_BYTES; }
+
+__global__ void __launch_bounds__(LSF_THREADS, 3)
+lsf_cluster_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_io, const LsfChainParams p,
+                   const bool ahead, unsigned int* status) {
+  constexpr int TPW = LT_TOK / LSF_WARPS;
+  extern __shared__ uint8_t lsf_smem_raw[];
+  __shared__ uint64_t bar_m, bar_r;
+  __shared__ uint32_t abort_flag;
+  const uint32_t raw_addr = smem_u32(lsf_smem_raw);
+  uint8_t* m_tile = lsf_smem_raw + (((raw_addr + 127u) & ~127u) - raw_addr);
+  uint8_t* r_tile = m_tile + LT_M_BYTES;
+  float2 (*ends)[LSF_WARPS][32] = reinterpret_cast<float2 (*)[LSF_WARPS][32]>(r_tile + LT_R_BYTES);   // [tile][run][lane]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x, n_tiles = gridDim.x, b = blockIdx.z;       // cluster: the tiles of one sequence
+  const int ch0 = blockIdx.y * LSF_CH, ch = ch0 + lane * 2;
+  const bool ch_ok = ch < p.D;
+  cluster_arrive();
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&bar_m), 1);
+    mbar_init(smem_u32(&bar_r), 1);
+    abort_flag = 0;
+    fence_mbar_init();
+    mbar_arrive_expect_tx(smem_u32(&bar_m), LT_M_BYTES);
+    mbar_arrive_expect_tx(smem_u32(&bar_r), LT_R_BYTES);
+    if (ahead) tma_load_3d(smem_u32(r_tile), &tm_io, ch0, tile * LT_TOK, b, smem_u32(&bar_r));
+    tma_prefetch_desc(&tm_m);
+  }
+  float2 c = make_float2(0.f, 0.f);
+  if (ahead && p.h0 && ch_ok) c = *reinterpret_cast<const float2*>(p.h0 + size_t(b) * p.D + ch);
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    tma_load_3d(smem_u32(m_tile), &tm_m, ch0, tile * LT_TOK, b, smem_u32(&bar_m));
+    if (!ahead) tma_load_3d(smem_u32(r_tile), &tm_io, ch0, tile * LT_TOK, b, smem_u32(&bar_r));
+  }
+  if (!ahead && p.h0 && ch_ok) c = *reinterpret_cast<const float2*>(p.h0 + size_t(b) * p.D + ch);
+  const float alpha = lsf_decay(p);
+  const float one_m = 1.0f - alpha;
+  float a_run = alpha;                           // alpha^TPW
+#pragma unroll
+  for (int j = 1; j < TPW; ++j) a_run *= alpha;
+
+  bool ok = mbar_wait(smem_u32(&bar_m), 0u, &abort_flag, status, JB200_STATUS_LSF_LOAD);
+  const int tl0 = warp * TPW;
+  float2 loc[TPW], h = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int j = 0; j < TPW; ++j) {
+    const uint32_t w = *reinterpret_cast<const uint32_t*>(m_tile + size_t(tl0 + j) * (LSF_CH * 2) + lane * 4);
+    h.x = alpha * h.x + one_m * bf16_lo(w);
+    h.y = alpha * h.y + one_m * bf16_hi(w);
+    loc[j] = h;
+  }
+  __syncwarp();
+  cluster_wait();                                // the other CTAs have started: their shared memory may be written
+  ends[tile][warp][lane] = h;
+  for (int t = tile + 1; t < n_tiles; ++t) cluster_st_64(cluster_map(smem_u32(&ends[tile][warp][lane]), uint32_t(t)), h);
+  __syncwarp();
+  cluster_arrive();
+  lsf_leave_scalars(p.st);
+  __syncwarp();
+  cluster_wait();
+#pragma unroll 8
+  for (int q = 0; q < tile * LSF_WARPS + warp; ++q) {
+    const float2 e = (&ends[0][0][0])[q * 32 + lane];
+    c.x = a_run * c.x + e.x;
+    c.y = a_run * c.y + e.y;
+  }
+  ok = mbar_wait(smem_u32(&bar_r), 0u, &abort_flag, status, JB200_STATUS_LSF_LOAD) && ok;
+  const int t0 = tile * LT_TOK + tl0;
+  float a = alpha;
+#pragma unroll
+  for (int j = 0; j < TPW; ++j, a *= alpha) {
+    const float hx = loc[j].x + a * c.x, hy = loc[j].y + a * c.y;
+    float2* r = reinterpret_cast<float2*>(r_tile + size_t(tl0 + j) * (LSF_CH * 4) + lane * 8);
+    const float2 old = *r;
+    *r = make_float2(old.x + hx, old.y + hy);
+    if (t0 + j == p.T - 1 && p.h_last && ch_ok && ok)
+      *reinterpret_cast<float2*>(p.h_last + size_t(b) * p.D + ch) = make_float2(hx, hy);
+  }
+  fence_proxy_async_smem();
+  if (__syncthreads_or(!ok)) return;
+  if (threadIdx.x == 0) {
+    tma_store_3d(&tm_io, ch0, tile * LT_TOK, b, smem_u32(r_tile));
+    bulk_commit_group();
+    bulk_wait_group<0>();
+  }
+}
+
 int make_lsf_map(CUtensorMap* tm, const void* ptr, CUtensorMapDataType dt, int elem, int B, int T, int D) {
   const cuuint64_t gdim[3] = {cuuint64_t(D), cuuint64_t(T), cuuint64_t(B)};
   const cuuint64_t gstride[2] = {cuuint64_t(D) * elem, cuuint64_t(T) * D * elem};
@@ -514,7 +624,7 @@ int make_lsf_map(CUtensorMap* tm, const void* ptr, CUtensorMapDataType dt, int e
 }
 
 template <bool FUSED>
-int launch_tma(LsfParams p, cudaStream_t stream) {
+int launch_tma(LsfChainParams p, cudaStream_t stream) {
   using Cfg = LsfTma<FUSED>;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
@@ -536,9 +646,19 @@ int launch_tma(LsfParams p, cudaStream_t stream) {
   if (rc != JB200_OK) return rc;
   unsigned int* status = device_status_ptr();
   if (!status) return JB200_ERR_CUDA;
+  // all tiles at once where a CTA per sequence and channel tile would leave SMs empty (beyond, deep rings overlap as well:
+  // 8 x 300 tokens 3.28 against 3.25 ms for 24 layers)
+  const int n_tiles = (p.T + LT_TOK - 1) / LT_TOK;
+  if (FUSED && p.nseg == 1 && n_tiles >= 2 && n_tiles <= LC_MAX_TILES && 2 * ctas < sms) {
+    JB_MAX_SMEM(lsf_cluster_kernel, lc_smem_bytes(LC_MAX_TILES));
+    launch_dep_cluster(lsf_cluster_kernel, dim3(n_tiles, (p.D + LSF_CH - 1) / LSF_CH, p.B), LSF_THREADS, lc_smem_bytes(n_tiles),
+                       n_tiles, stream, tm_m, tm_io, p, p.st.stats != nullptr, status);
+    JB_LAUNCH_CHECK("lsf_cluster_kernel");
+    return JB200_OK;
+  }
   if (p.nseg > 1) {
     dim3 grid_a((p.D + LSF_CH - 1) / LSF_CH, p.B, p.n_pre_tiles);
-    launch_dep(lsf_scan_kernel<false, __nv_bfloat16, __nv_bfloat16, LSF_TPW, true>, grid_a, LSF_THREADS, 0, stream, p);
+    launch_dep(lsf_scan_kernel<false, __nv_bfloat16, __nv_bfloat16, LSF_TPW, true, FUSED>, grid_a, LSF_THREADS, 0, stream, p);
     JB_LAUNCH_CHECK("lsf_scan_kernel<ends>");
   }
   dim3 grid((p.D + LSF_CH - 1) / LSF_CH, p.B, p.nseg);
@@ -590,7 +710,7 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
   JB_REQUIRE(!resid || (reinterpret_cast<uintptr_t>(resid) & a8) == 0, "lsf_scan: residual pointer misaligned");
   JB_REQUIRE((!h0 || (reinterpret_cast<uintptr_t>(h0) & a8) == 0) && (!h_last || (reinterpret_cast<uintptr_t>(h_last) & a8) == 0),
              "lsf_scan: state pointer misaligned");
-  LsfParams p = {};
+  LsfChainParams p = {};
   p.m = m; p.alpha_t = alpha_tensor; p.alpha_s = alpha_scalar; p.act_var = act_var; p.var_scale = var_scale;
   p.alpha_min = alpha_min; p.alpha_max = alpha_max; p.h0 = h0; p.resid = resid; p.out = out; p.h_last = h_last;
   p.B = B; p.T = T; p.D = D;
@@ -616,6 +736,7 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
     if (resid && !out && aligned16(resid)) return launch_tma<true>(p, stream);
     if (out && !resid && out_dtype == 1 && aligned16(out)) return launch_tma<false>(p, stream);
   }
+  JB_REQUIRE(!st || (!ta && T <= 8), "lsf_scan: the decay comes from the accumulators in the fused form alone");
   if (!ta) {
     if (m_dtype == 1 && out_dtype == 1) return launch_t<false, bf, bf>(p, stream);
     if (m_dtype == 1 && out_dtype == 0) return launch_t<false, bf, float>(p, stream);

@@ -134,3 +134,22 @@ def test_chain_with_uneven_experts(T, skew):
     counts = torch.bincount(blk.moe.last_routing[0].flatten(), minlength=4)
     assert int(counts.max()) > T * (5 if skew < 1 else 8) // 10, counts
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T,D", [(1, 129, 1024), (1, 256, 64), (3, 777, 1024), (2, 1023, 200), (9, 300, 1024), (10, 300, 1024)])
+def test_residual_scan_with_its_tiles_side_by_side(B, T, D):
+    """The fused scan of sequences of two to eight tiles against the recurrence in f64; the membrane is updated in place."""
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    m = torch.randn(B, T, D, generator=gen, device="cuda").bfloat16()
+    h0 = torch.randn(B, D, generator=gen, device="cuda")
+    x = torch.randn(B, T, D, generator=gen, device="cuda")
+    alpha, h, want = torch.tensor([0.97], device="cuda"), h0.double(), x.double()
+    a = float(alpha)
+    for t in range(T):
+        h = a * h + (1.0 - a) * m[:, t].double()
+        want[:, t] += h
+    got, last = x.clone(), h0.clone()
+    ops.lsf_scan(m, alpha_scalar=alpha, h0=last, resid=got, want_out=False, last_out=last)
+    # every step rounds values below 5 three times (2^-24 of them), and errors fade by alpha: 3 * 5 * 2^-24 / 0.03 = 3e-5
+    assert float((got.double() - want).abs().max()) < 3e-5 and float((last.double() - h).abs().max()) < 3e-5
+    assert _lib.device_status() == 0
