@@ -276,6 +276,12 @@ int jb200_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const f
                    const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,
                    float* resid, void* out, int out_dtype, float* h_last, void* scratch, int B, int T, int D,
                    void* stream);
+/* The same with the last state stored as f32 (last_dtype 0) or rounded to bf16 (1; scalar decays only): no
+ * conversion after it. */
+int jb200_lsf_scan_cast(const void* m, int m_dtype, const void* alpha_tensor, const float* alpha_scalar,
+                        const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,
+                        float* resid, void* out, int out_dtype, void* h_last, int last_dtype, void* scratch, int B, int T,
+                        int D, void* stream);
 
 /* Tail of a block for single-token steps (T = 1), three of the calls above in one launch with their results bit
  * for bit: jb200_moe_finalize (scalars from the accumulators; SparseMoELayer.forward, jarvis_model.py:244-250),

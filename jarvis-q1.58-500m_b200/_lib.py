@@ -71,6 +71,7 @@ PROTOTYPES = {
     "jb200_moe_scatter_combine": (_I, [_P, _P, _P, _I, _I, _I, _P, _I, _P, _P]),
     "jb200_moe_finalize": (_I, [_P, _P, _P, _I, C.c_longlong, C.c_longlong, _F, _P, _P]),
     "jb200_lsf_scan": (_I, [_P, _I, _P, _P, _P, _P, _F, _F, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P]),
+    "jb200_lsf_scan_cast": (_I, [_P, _I, _P, _P, _P, _P, _F, _F, _P, _P, _P, _I, _P, _I, _P, _I, _I, _I, _P]),
     "jb200_lsf_scan_scratch_bytes": (_Z, [_I, _I, _I]),
     "jb200_lsf_step_norm": (_I, [_P, _P, _P, _P, _I, C.c_longlong, C.c_longlong, _F, _P, _P, _F, _F, _P, _P, _P, _P, _F, _P,
                                  _I, _I, _P]),

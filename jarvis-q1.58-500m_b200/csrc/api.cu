@@ -404,7 +404,15 @@ int jb200_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const f
                    float* resid, void* out, int out_dtype, float* h_last, void* scratch, int B, int T, int D,
                    void* stream) {
   return launch_lsf_scan(m, m_dtype, alpha_tensor, alpha_scalar, act_var, var_scale, alpha_min, alpha_max, h0, resid,
-                         out, out_dtype, h_last, scratch, B, T, D, static_cast<cudaStream_t>(stream));
+                         out, out_dtype, h_last, 0, scratch, B, T, D, static_cast<cudaStream_t>(stream));
+}
+
+int jb200_lsf_scan_cast(const void* m, int m_dtype, const void* alpha_tensor, const float* alpha_scalar,
+                        const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,
+                        float* resid, void* out, int out_dtype, void* h_last, int last_dtype, void* scratch, int B, int T,
+                        int D, void* stream) {
+  return launch_lsf_scan(m, m_dtype, alpha_tensor, alpha_scalar, act_var, var_scale, alpha_min, alpha_max, h0, resid,
+                         out, out_dtype, h_last, last_dtype, scratch, B, T, D, static_cast<cudaStream_t>(stream));
 }
 
 size_t jb200_lsf_scan_scratch_bytes(int B, int T, int D) { return lsf_scan_scratch_bytes(B, T, D); }

@@ -213,7 +213,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     } else {
       void* lsf_scratch = (h_in && h_in == h_out) || ws.lsf == ws.meta ? nullptr : w + ws.lsf;
       JB_TRY(launch_lsf_scan(out, 1, nullptr, nullptr, nullptr, p.var_scale, p.alpha_min, p.alpha_max, h_in, x, nullptr, 0,
-                             h_out, lsf_scratch, B, T, C, st, &stats));
+                             h_out, 0, lsf_scratch, B, T, C, st, &stats));
       if (w_next) JB_TRY(launch_rmsnorm(x, 0, w_next, eps_next, xn_next, 1, N, C, st));
     }
   }

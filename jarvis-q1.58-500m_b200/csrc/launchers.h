@@ -81,7 +81,7 @@ struct LsfStats {
 };
 int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const float* alpha_scalar,
                     const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,
-                    float* resid, void* out, int out_dtype, float* h_last, void* scratch, int B, int T, int D,
+                    float* resid, void* out, int out_dtype, void* h_last, int last_dtype, void* scratch, int B, int T, int D,
                     cudaStream_t stream, const LsfStats* st = nullptr);
 size_t lsf_scan_scratch_bytes(int B, int T, int D);
 int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* var_scale, float alpha_min, float alpha_max,

@@ -57,14 +57,23 @@ struct LsfParams {
   float* seg_prod;         // [B][n_pre_tiles][D] product of its decays (tensor mode)
 };
 
-// What a chain's kernels get.  Kernels that no chain runs take LsfParams alone: with the accumulators among their
-// parameters per-element decays compiled to 182 registers instead of 255, fewer loads in flight and 287 us at 32 x 2048
-// instead of 273 (8 x 8192 in segments 80 us instead of 66).
-struct LsfChainParams : LsfParams {
+// Kernels get no more than they use: what these two add, among the parameters of a kernel that does not read it, changed
+// its schedule for the worse (per-element decays 32 x 2048: 268 us without, 281 to 304 with; the ends of 8 x 8192: 66, 81).
+struct LsfScalarParams : LsfParams {      // one decay per call
+  __nv_bfloat16* last16;   // [B][D] or null: the last state in bf16 (h_last is null then)
+};
+struct LsfChainParams : LsfScalarParams {
   LsfStats st;             // st.stats != null: act_var comes from the MoE layer's accumulators
 };
-template <bool STATS>
-using LsfArgs = std::conditional_t<STATS, LsfChainParams, LsfParams>;
+template <bool SCALAR, bool STATS>
+using LsfArgs = std::conditional_t<STATS, LsfChainParams, std::conditional_t<SCALAR, LsfScalarParams, LsfParams>>;
+
+template <typename Args>
+__device__ __forceinline__ void store_last(const Args& p, size_t at, float2 h) {
+  if (p.h_last) *reinterpret_cast<float2*>(p.h_last + at) = h;
+  if constexpr (std::is_base_of_v<LsfScalarParams, Args>)
+    if (p.last16) *reinterpret_cast<uint32_t*>(p.last16 + at) = pack_bf16x2(h.x, h.y);
+}
 
 // The scalar decay of a call (model semantics).  With st.stats the variance of the MoE output is derived here, as
 // moe_finalize_kernel would have, instead of in a launch of its own between the combine and the scan.
@@ -104,7 +113,7 @@ __device__ __forceinline__ void st2<__nv_bfloat16>(__nv_bfloat16* p, float a, fl
 }
 
 template <bool TENSOR_ALPHA, typename TM, typename TOut, int TPW, bool ENDS_ONLY, bool STATS>
-__global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_kernel(const LsfArgs<STATS> p) {
+__global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_kernel(const LsfArgs<!TENSOR_ALPHA && !ENDS_ONLY, STATS> p) {
   pdl_wait();
   pdl_trigger();
   __shared__ float2 s_end[2][LSF_WARPS][32];   // end value of each warp's run
@@ -224,7 +233,7 @@ __global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_ke
         const size_t o = seq_base + size_t(t) * p.D;
         if (out) st2<TOut>(out + o, hx, hy);
         if (p.resid) *reinterpret_cast<float2*>(p.resid + o) = make_float2(rold[i].x + hx, rold[i].y + hy);
-        if (t == p.T - 1 && p.h_last) *reinterpret_cast<float2*>(p.h_last + size_t(b) * p.D + ch) = make_float2(hx, hy);
+        if (t == p.T - 1) store_last(p, size_t(b) * p.D + ch, make_float2(hx, hy));
       }
     }
   }
@@ -237,7 +246,7 @@ __global__ void __launch_bounds__(LSF_THREADS, TENSOR_ALPHA ? 1 : 2) lsf_scan_ke
 
 // Short sequences (decode steps): one thread per channel pair walks the few tokens itself.
 template <bool TENSOR_ALPHA, typename TM, typename TOut>
-__global__ void __launch_bounds__(256) lsf_short_kernel(const LsfArgs<!TENSOR_ALPHA> p) {
+__global__ void __launch_bounds__(256) lsf_short_kernel(const LsfArgs<false, !TENSOR_ALPHA> p) {
   pdl_wait();
   pdl_trigger();
   const size_t pair = size_t(blockIdx.x) * 256 + threadIdx.x;
@@ -267,7 +276,7 @@ __global__ void __launch_bounds__(256) lsf_short_kernel(const LsfArgs<!TENSOR_AL
       *r = make_float2(rv.x + h.x, rv.y + h.y);
     }
   }
-  if (p.h_last) *reinterpret_cast<float2*>(p.h_last + size_t(b) * p.D + ch) = h;
+  store_last(p, size_t(b) * p.D + ch, h);
 }
 
 // Single-token tail of a block (decode steps), three launches in one: the MoE layer's scalars from its accumulated
@@ -375,10 +384,13 @@ constexpr int LT_TOK = LSF_WARPS * 16;       // 128 tokens per tile (= LSF_TILE:
 constexpr int LT_M_BYTES = LT_TOK * LSF_CH * 2;    // 16 KiB
 constexpr int LT_R_BYTES = LT_TOK * LSF_CH * 4;    // 32 KiB
 
-template <bool FUSED>
+// CH channels per CTA.  64: a warp takes a run of 16 tokens; 32: two runs, one per half warp, so a tile takes four warps.
+template <bool FUSED, int CH>
 struct LsfTma {
-  static constexpr int STAGE_BYTES = LT_M_BYTES + (FUSED ? LT_R_BYTES : 0);
-  static constexpr size_t CTL_BYTES = 128 + 2 * LSF_WARPS * 32 * sizeof(float2);   // barriers + flag, run ends
+  static constexpr int RPW = LSF_CH / CH, THREADS = LSF_THREADS / RPW;
+  static constexpr int M_BYTES = LT_M_BYTES / RPW;
+  static constexpr int STAGE_BYTES = (LT_M_BYTES + (FUSED ? LT_R_BYTES : 0)) / RPW;
+  static constexpr size_t CTL_BYTES = 128 + 2 * LSF_WARPS * (CH / 2) * sizeof(float2);   // barriers + flag, run ends
   static constexpr size_t smem_bytes(int stages) { return size_t(stages) * STAGE_BYTES + CTL_BYTES + 128 /* alignment slack */; }
   // Stages: enough CTAs to put two (fused) or three (plain) on every SM -> a short ring each; a grid that leaves
   // SMs with one CTA -> that CTA gets a ring of four stages (and sequences are not cut into segments).
@@ -386,13 +398,13 @@ struct LsfTma {
   static constexpr int STAGES_ALONE = 4;
 };
 
-template <bool FUSED>
-__global__ void __launch_bounds__(LSF_THREADS, FUSED ? 2 : 4)
-lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_io, const LsfArgs<FUSED> p,
+template <bool FUSED, int CH>
+__global__ void __launch_bounds__(LsfTma<FUSED, CH>::THREADS, (FUSED ? 2 : 4) * LsfTma<FUSED, CH>::RPW)
+lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_io, const LsfArgs<true, FUSED> p,
                const int n_stages, unsigned int* status) {
   pdl_wait();
   pdl_trigger();
-  using Cfg = LsfTma<FUSED>;
+  using Cfg = LsfTma<FUSED, CH>;
   constexpr int TPW = LT_TOK / LSF_WARPS;    // 16 (sixteen warps of 8 tokens were measured: slower)
   extern __shared__ uint8_t lsf_smem_raw[];
   const uint32_t raw_addr = smem_u32(lsf_smem_raw);
@@ -401,11 +413,11 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
   uint8_t* ctl = tiles + size_t(n_stages) * Cfg::STAGE_BYTES;
   uint64_t* full = reinterpret_cast<uint64_t*>(ctl);                       // [STAGES]
   uint32_t* abort_flag = reinterpret_cast<uint32_t*>(ctl + 64);
-  float2 (*s_end)[LSF_WARPS][32] = reinterpret_cast<float2 (*)[LSF_WARPS][32]>(ctl + 128);   // [2][8][32]
+  float2 (*s_end)[LSF_WARPS][CH / 2] = reinterpret_cast<float2 (*)[LSF_WARPS][CH / 2]>(ctl + 128);   // [2][8][channel pairs]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int run = threadIdx.x / (CH / 2), lane = threadIdx.x % (CH / 2);   // this thread's run of a tile and channel pair
   const int b = blockIdx.y, seg = blockIdx.z;
-  const int ch0 = blockIdx.x * LSF_CH;
+  const int ch0 = blockIdx.x * CH;
   const int ch = ch0 + lane * 2;
   const bool ch_ok = ch < p.D;
   const int t_begin = seg * p.seg_len;
@@ -439,7 +451,7 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
     const uint32_t dst = smem_u32(tiles + size_t(s) * Cfg::STAGE_BYTES);
     mbar_arrive_expect_tx(bar, Cfg::STAGE_BYTES);
     tma_load_3d(dst, &tm_m, ch0, t_begin + i * LT_TOK, b, bar);
-    if (FUSED) tma_load_3d(dst + LT_M_BYTES, &tm_io, ch0, t_begin + i * LT_TOK, b, bar);
+    if (FUSED) tma_load_3d(dst + Cfg::M_BYTES, &tm_io, ch0, t_begin + i * LT_TOK, b, bar);
   };
   if (threadIdx.x == 0) {
     for (int s = 0; s < n_stages; ++s) mbar_init(smem_u32(&full[s]), 1);
@@ -456,28 +468,28 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
     const int s = i % n_stages;
     const int buf = i & 1;
     uint8_t* m_tile = tiles + size_t(s) * Cfg::STAGE_BYTES;
-    uint8_t* r_tile = m_tile + LT_M_BYTES;
+    uint8_t* r_tile = m_tile + Cfg::M_BYTES;
     if (!mbar_wait(smem_u32(&full[s]), uint32_t(i / n_stages) & 1u, abort_flag, status, JB200_STATUS_LSF_LOAD)) ok = false;
-    const int tl0 = warp * TPW;                          // first token of this warp's run inside the tile
+    const int tl0 = run * TPW;                           // first token of this run inside the tile
     const int t0 = t_begin + i * LT_TOK + tl0;
     float2 loc[TPW];
     float2 h = make_float2(0.f, 0.f);
     if (ok) {
 #pragma unroll
       for (int j = 0; j < TPW; ++j) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(m_tile + size_t(tl0 + j) * (LSF_CH * 2) + lane * 4);
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(m_tile + size_t(tl0 + j) * (CH * 2) + lane * 4);
         h.x = alpha * h.x + (1.0f - alpha) * bf16_lo(w);
         h.y = alpha * h.y + (1.0f - alpha) * bf16_hi(w);
         loc[j] = h;
       }
     }
-    s_end[buf][warp][lane] = h;
+    s_end[buf][run][lane] = h;
     if (__syncthreads_or(!ok)) { ok = false; break; }
-    // carry into this warp's run, and the carry out of the whole tile (the recurrence is an affine map)
+    // carry into this run, and the carry out of the whole tile (the recurrence is an affine map)
     float2 c = carry, cn = carry;
 #pragma unroll
     for (int w = 0; w < LSF_WARPS; ++w) {
-      if (w == warp) cn = c;
+      if (w == run) cn = c;
       const float2 e = s_end[buf][w][lane];
       c.x = pw[TPW - 1] * c.x + e.x;
       c.y = pw[TPW - 1] * c.y + e.y;
@@ -487,11 +499,11 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
     for (int j = 0; j < TPW; ++j) {
       const float hx = loc[j].x + pw[j] * cn.x, hy = loc[j].y + pw[j] * cn.y;
       if (FUSED) {
-        float2* r = reinterpret_cast<float2*>(r_tile + size_t(tl0 + j) * (LSF_CH * 4) + lane * 8);
+        float2* r = reinterpret_cast<float2*>(r_tile + size_t(tl0 + j) * (CH * 4) + lane * 8);
         const float2 old = *r;
         *r = make_float2(old.x + hx, old.y + hy);
       } else {
-        *reinterpret_cast<uint32_t*>(m_tile + size_t(tl0 + j) * (LSF_CH * 2) + lane * 4) = pack_bf16x2(hx, hy);
+        *reinterpret_cast<uint32_t*>(m_tile + size_t(tl0 + j) * (CH * 2) + lane * 4) = pack_bf16x2(hx, hy);
       }
       if (t0 + j == p.T - 1 && p.h_last && ch_ok)
         *reinterpret_cast<float2*>(p.h_last + size_t(b) * p.D + ch) = make_float2(hx, hy);
@@ -512,6 +524,13 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
         bulk_wait_group_read<0>();   // the store has read the stage: it may be filled again
         issue(i + n_stages);
       }
+    }
+  }
+  if constexpr (!FUSED) {          // the last row of the output is the last state in bf16 (stored in the loop it cost a spill)
+    if (ok && p.last16 && t_end == p.T && run == 0 && ch_ok) {
+      const uint8_t* tile = tiles + size_t((n_tiles - 1) % n_stages) * Cfg::STAGE_BYTES;
+      *reinterpret_cast<uint32_t*>(p.last16 + size_t(b) * p.D + ch) =
+          *reinterpret_cast<const uint32_t*>(tile + size_t((p.T - 1 - t_begin) % LT_TOK) * (CH * 2) + lane * 4);
     }
   }
   if (threadIdx.x == 0) bulk_wait_group<0>();   // every store has landed before the CTA gives up its shared memory
@@ -603,8 +622,8 @@ lsf_cluster_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_consta
     float2* r = reinterpret_cast<float2*>(r_tile + size_t(tl0 + j) * (LSF_CH * 4) + lane * 8);
     const float2 old = *r;
     *r = make_float2(old.x + hx, old.y + hy);
-    if (t0 + j == p.T - 1 && p.h_last && ch_ok && ok)
-      *reinterpret_cast<float2*>(p.h_last + size_t(b) * p.D + ch) = make_float2(hx, hy);
+    if (t0 + j == p.T - 1 && ch_ok && ok)
+      store_last(p, size_t(b) * p.D + ch, make_float2(hx, hy));
   }
   fence_proxy_async_smem();
   if (__syncthreads_or(!ok)) return;
@@ -615,17 +634,17 @@ lsf_cluster_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_consta
   }
 }
 
-int make_lsf_map(CUtensorMap* tm, const void* ptr, CUtensorMapDataType dt, int elem, int B, int T, int D) {
+int make_lsf_map(CUtensorMap* tm, const void* ptr, CUtensorMapDataType dt, int elem, int B, int T, int D, int channels = LSF_CH) {
   const cuuint64_t gdim[3] = {cuuint64_t(D), cuuint64_t(T), cuuint64_t(B)};
   const cuuint64_t gstride[2] = {cuuint64_t(D) * elem, cuuint64_t(T) * D * elem};
-  const cuuint32_t box[3] = {cuuint32_t(LSF_CH), cuuint32_t(LT_TOK), 1};
+  const cuuint32_t box[3] = {cuuint32_t(channels), cuuint32_t(LT_TOK), 1};
   return encode_tiled(tm, dt, 3, ptr, gdim, gstride, box, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                       "lsf_scan");
 }
 
 template <bool FUSED>
 int launch_tma(LsfChainParams p, cudaStream_t stream) {
-  using Cfg = LsfTma<FUSED>;
+  using Cfg = LsfTma<FUSED, LSF_CH>;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
   const long ctas = long((p.D + LSF_CH - 1) / LSF_CH) * p.B;
@@ -646,6 +665,22 @@ int launch_tma(LsfChainParams p, cudaStream_t stream) {
   if (rc != JB200_OK) return rc;
   unsigned int* status = device_status_ptr();
   if (!status) return JB200_ERR_CUDA;
+  if constexpr (!FUSED) {
+    // Between two and four CTAs of 64 channels per SM some SMs hold one CTA more than others and finish last (32 x 2048:
+    // 3.46 on average, 4 on most); tiles of half the channels halve that step.
+    const long half = long((p.D + LSF_CH / 2 - 1) / (LSF_CH / 2)) * p.B, per_sm = (ctas + sms - 1) / sms;
+    if (ctas > 2L * sms && ctas <= 4L * sms && (half + sms - 1) / sms < 2 * per_sm) {
+      using Half = LsfTma<false, LSF_CH / 2>;
+      if ((rc = make_lsf_map(&tm_m, p.m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.B, p.T, p.D, LSF_CH / 2)) != JB200_OK) return rc;
+      if ((rc = make_lsf_map(&tm_io, p.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.B, p.T, p.D, LSF_CH / 2)) != JB200_OK) return rc;
+      auto kernel = lsf_tma_kernel<false, LSF_CH / 2>;
+      JB_MAX_SMEM(kernel, Half::smem_bytes(Half::STAGES_SHARED));
+      launch_dep(kernel, dim3((p.D + LSF_CH / 2 - 1) / (LSF_CH / 2), p.B, 1), Half::THREADS, Half::smem_bytes(Half::STAGES_SHARED), stream,
+                 tm_m, tm_io, p, Half::STAGES_SHARED, status);
+      JB_LAUNCH_CHECK("lsf_tma_kernel<half>");
+      return JB200_OK;
+    }
+  }
   // all tiles at once where a CTA per sequence and channel tile would leave SMs empty (beyond, deep rings overlap as well:
   // 8 x 300 tokens 3.28 against 3.25 ms for 24 layers)
   const int n_tiles = (p.T + LT_TOK - 1) / LT_TOK;
@@ -662,8 +697,9 @@ int launch_tma(LsfChainParams p, cudaStream_t stream) {
     JB_LAUNCH_CHECK("lsf_scan_kernel<ends>");
   }
   dim3 grid((p.D + LSF_CH - 1) / LSF_CH, p.B, p.nseg);
-  JB_MAX_SMEM(lsf_tma_kernel<FUSED>, Cfg::smem_bytes(Cfg::STAGES_ALONE));
-  launch_dep(lsf_tma_kernel<FUSED>, grid, LSF_THREADS, Cfg::smem_bytes(stages), stream, tm_m, tm_io, p, stages, status);
+  auto kernel = lsf_tma_kernel<FUSED, LSF_CH>;
+  JB_MAX_SMEM(kernel, Cfg::smem_bytes(Cfg::STAGES_ALONE));
+  launch_dep(kernel, grid, LSF_THREADS, Cfg::smem_bytes(stages), stream, tm_m, tm_io, p, stages, status);
   JB_LAUNCH_CHECK("lsf_tma_kernel");
   return JB200_OK;
 }
@@ -693,12 +729,12 @@ size_t lsf_scan_scratch_bytes(int B, int T, int D) {
 
 int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const float* alpha_scalar,
                     const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,
-                    float* resid, void* out, int out_dtype, float* h_last, void* scratch, int B, int T, int D,
+                    float* resid, void* out, int out_dtype, void* h_last, int last_dtype, void* scratch, int B, int T, int D,
                     cudaStream_t stream, const LsfStats* st) {
   JB_REQUIRE(B >= 0 && T >= 0 && D > 0, "lsf_scan: bad shape (%d, %d, %d)", B, T, D);
   JB_REQUIRE(D % 2 == 0, "lsf_scan: channel count (%d) must be even", D);
   JB_REQUIRE(B <= 65535, "lsf_scan: batch (%d) exceeds 65535", B);
-  JB_REQUIRE((m_dtype == 0 || m_dtype == 1) && (out_dtype == 0 || out_dtype == 1), "lsf_scan: dtype must be 0 (f32) or 1 (bf16)");
+  JB_REQUIRE((m_dtype == 0 || m_dtype == 1) && (out_dtype == 0 || out_dtype == 1) && (last_dtype == 0 || last_dtype == 1), "lsf_scan: dtype must be 0 (f32) or 1 (bf16)");
   if (B == 0 || T == 0) return JB200_OK;
   JB_REQUIRE(m != nullptr, "lsf_scan: null input");
   JB_REQUIRE(alpha_tensor || alpha_scalar || ((act_var || st) && var_scale), "lsf_scan: no decay given");
@@ -712,7 +748,9 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
              "lsf_scan: state pointer misaligned");
   LsfChainParams p = {};
   p.m = m; p.alpha_t = alpha_tensor; p.alpha_s = alpha_scalar; p.act_var = act_var; p.var_scale = var_scale;
-  p.alpha_min = alpha_min; p.alpha_max = alpha_max; p.h0 = h0; p.resid = resid; p.out = out; p.h_last = h_last;
+  p.alpha_min = alpha_min; p.alpha_max = alpha_max; p.h0 = h0; p.resid = resid; p.out = out;
+  p.h_last = last_dtype ? nullptr : static_cast<float*>(h_last);
+  p.last16 = last_dtype ? static_cast<__nv_bfloat16*>(h_last) : nullptr;
   p.B = B; p.T = T; p.D = D;
   p.seg_len = (T + LSF_TILE - 1) / LSF_TILE * LSF_TILE;
   p.nseg = 1;
@@ -730,10 +768,11 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
   }
   JB_REQUIRE(p.nseg <= 65535 && p.n_pre_tiles <= 65535, "lsf_scan: too many segments");
   const bool ta = alpha_tensor != nullptr;
+  JB_REQUIRE(!ta || last_dtype == 0, "lsf_scan: per-element decays leave an f32 state");
   using bf = __nv_bfloat16;
   // the forms the model and the scan sweep run: tiles by TMA (3-D maps need 16-byte aligned rows)
   if (!ta && m_dtype == 1 && T > 8 && D % 8 == 0 && aligned16(m) && B * long(T) * D < (1L << 40)) {
-    if (resid && !out && aligned16(resid)) return launch_tma<true>(p, stream);
+    if (resid && !out && last_dtype == 0 && aligned16(resid)) return launch_tma<true>(p, stream);
     if (out && !resid && out_dtype == 1 && aligned16(out)) return launch_tma<false>(p, stream);
   }
   JB_REQUIRE(!st || (!ta && T <= 8), "lsf_scan: the decay comes from the accumulators in the fused form alone");

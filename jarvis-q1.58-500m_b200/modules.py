@@ -367,13 +367,14 @@ class LiquidStateFusion(nn.Module):
         self.var_scale = nn.Parameter(torch.tensor(1.0))
 
     def forward(self, x, act_var, h_prev=None):
-        act_var = torch.as_tensor(act_var, dtype=torch.float32, device=x.device).reshape(1)
+        if not (torch.is_tensor(act_var) and act_var.dtype is torch.float32 and act_var.device == x.device and act_var.numel() == 1):
+            act_var = torch.as_tensor(act_var, dtype=torch.float32, device=x.device).reshape(1)
         h0 = None if h_prev is None else h_prev.to(torch.float32).contiguous()
         m = x.contiguous()
         if m.dtype not in (torch.float32, torch.bfloat16):
             m = m.float()
         out, last = ops.lsf_scan(m, act_var=act_var, var_scale=_f32(self.var_scale, scalar=True),
-                                 alpha_min=self.alpha_min, alpha_max=self.alpha_max, h0=h0)
+                                 alpha_min=self.alpha_min, alpha_max=self.alpha_max, h0=h0, last_dtype=m.dtype)
         return out.to(x.dtype), last.to(x.dtype)
 
 
