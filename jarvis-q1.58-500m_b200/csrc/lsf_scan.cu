@@ -666,10 +666,10 @@ int launch_tma(LsfChainParams p, cudaStream_t stream) {
   unsigned int* status = device_status_ptr();
   if (!status) return JB200_ERR_CUDA;
   if constexpr (!FUSED) {
-    // Between two and four CTAs of 64 channels per SM some SMs hold one CTA more than others and finish last (32 x 2048:
-    // 3.46 on average, 4 on most); tiles of half the channels halve that step.
-    const long half = long((p.D + LSF_CH / 2 - 1) / (LSF_CH / 2)) * p.B, per_sm = (ctas + sms - 1) / sms;
-    if (ctas > 2L * sms && ctas <= 4L * sms && (half + sms - 1) / sms < 2 * per_sm) {
+    // Well beyond three CTAs of 64 channels per SM some SMs hold a fourth and finish last (32 x 2048: 3.46 on average); tiles
+    // of half the channels even that out, though they cost 3 % of themselves (30 x 2048 54.7 against 58.9 us, 32 x 2048 57.4
+    // against 60.5, but 28 x 2048 52.5 against 51.0 and 24 x 2048 47.2 against 44.5).
+    if (ctas > 3L * sms + sms / 8 && ctas <= 4L * sms) {
       using Half = LsfTma<false, LSF_CH / 2>;
       if ((rc = make_lsf_map(&tm_m, p.m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.B, p.T, p.D, LSF_CH / 2)) != JB200_OK) return rc;
       if ((rc = make_lsf_map(&tm_io, p.out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.B, p.T, p.D, LSF_CH / 2)) != JB200_OK) return rc;
