@@ -419,8 +419,11 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // 1 the first part of a cut one (leaves its end state in handoff), 2 the second part (starts from it).
   int h = blockIdx.x, b = blockIdx.y, seg = blockIdx.z, piece = 0;
   int ck_begin = seg * p.seg_chunks, ck_end = min(n_chunks, ck_begin + p.seg_chunks);
-  auto piece_of = [&](int t) {
-    const int U = p.B * p.H;
+  if (p.n_split > 0) {
+    // a ticket instead of the block index: whoever holds a second part started after every first part was taken
+    if (tid == 0) sm->ticket = atomicAdd(p.ctrl, 1);
+    __syncthreads();
+    const int t = sm->ticket, U = p.B * p.H;
     seg = 0;
     int unit = t;                                     // = b * H + h
     if (t < p.n_split) { piece = 1; ck_begin = 0; ck_end = p.split_chunk; }
@@ -428,28 +431,6 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     else { unit = t - U; piece = 2; ck_begin = p.split_chunk; ck_end = n_chunks; }
     b = unit / p.H;
     h = unit - b * p.H;
-  };
-  auto load_qk = [&](int lc, int s) {                 // the producer thread alone
-    const int r = b * T + (ck_begin + lc) * CH;
-    mbar_arrive_expect_tx(smem_u32(&sm->full_qk[s]), 2 * TILE_BYTES);
-    tma_load_2d(smem_u32(sm->q[s]), &tm_q, h * D, r, smem_u32(&sm->full_qk[s]));
-    tma_load_2d(smem_u32(sm->k[s]), &tm_k, h * D, r, smem_u32(&sm->full_qk[s]));
-  };
-  auto load_v = [&](int lc, int s) {
-    mbar_arrive_expect_tx(smem_u32(&sm->full_v[s]), TILE_BYTES);
-    tma_load_2d(smem_u32(sm->v[s]), &tm_v, h * D, b * T + (ck_begin + lc) * CH, smem_u32(&sm->full_v[s]));
-  };
-  if (tid == 0) {
-    // a ticket instead of the block index: whoever holds a second part started after every first part was taken
-    if (p.n_split > 0) piece_of(sm->ticket = atomicAdd(p.ctrl, 1));
-    for (int lc = 0; lc < NST && lc < ck_end - ck_begin; ++lc) {   // under way while the tables below are made
-      load_qk(lc, lc);
-      load_v(lc, lc);
-    }
-  }
-  if (p.n_split > 0) {
-    __syncthreads();
-    piece_of(sm->ticket);
   }
   const int n_loc = ck_end - ck_begin;
   const int row0 = b * T;
@@ -472,16 +453,20 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if (lane == 0) {
       JB_T_DECL
       int s = 0;
-      uint32_t prev = 0u;                       // parity of the PREVIOUS use of the stage
-      for (int lc = NST; lc < n_loc; ++lc) {
+      uint32_t prev = 1u;                       // parity of the PREVIOUS use of the stage
+      for (int lc = 0; lc < n_loc; ++lc) {
+        const int r = row0 + (ck_begin + lc) * CH;
         JB_T_MARK(0)
-        if (!mbar_wait(smem_u32(&sm->empty_qk[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+        if (lc >= NST && !mbar_wait(smem_u32(&sm->empty_qk[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
         JB_T_MARK(1)
-        load_qk(lc, s);
+        mbar_arrive_expect_tx(smem_u32(&sm->full_qk[s]), 2 * TILE_BYTES);
+        tma_load_2d(smem_u32(sm->q[s]), &tm_q, h * D, r, smem_u32(&sm->full_qk[s]));
+        tma_load_2d(smem_u32(sm->k[s]), &tm_k, h * D, r, smem_u32(&sm->full_qk[s]));
         JB_T_MARK(0)
-        if (!mbar_wait(smem_u32(&sm->empty_v[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+        if (lc >= NST && !mbar_wait(smem_u32(&sm->empty_v[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
         JB_T_MARK(2)
-        load_v(lc, s);
+        mbar_arrive_expect_tx(smem_u32(&sm->full_v[s]), TILE_BYTES);
+        tma_load_2d(smem_u32(sm->v[s]), &tm_v, h * D, r, smem_u32(&sm->full_v[s]));
         if (++s == NST) { s = 0; prev ^= 1u; }
       }
       JB_T_MARK(0)
