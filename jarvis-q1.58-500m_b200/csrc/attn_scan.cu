@@ -413,8 +413,12 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tmem_alloc(smem_u32(&sm->tmem_base), PIPE_TMEM_COLS);
     tmem_relinquish();
   }
-  pdl_wait();        // everything above overlapped the kernel before this one; global memory is read from here on
-  pdl_trigger();
+  // The decay tables come from a weight, so they too are made while the kernel before this one runs, unless the head is not
+  // known before the ticket is.
+  if (p.n_split > 0) {
+    pdl_wait();
+    pdl_trigger();
+  }
   // Which chunks of which sequence-head this CTA scans.  piece: 0 a whole sequence-head or a pre-passed segment,
   // 1 the first part of a cut one (leaves its end state in handoff), 2 the second part (starts from it).
   int h = blockIdx.x, b = blockIdx.y, seg = blockIdx.z, piece = 0;
@@ -447,6 +451,10 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_after_sync();
   const uint32_t tm = sm->tmem_base;
   volatile uint32_t* abort_flag = &sm->abort_flag;
+  if (p.n_split == 0) {
+    pdl_wait();
+    pdl_trigger();
+  }
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------

@@ -206,10 +206,10 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
                          w_next ? xn_next : nullptr, B, T, C, st));
       continue;
     }
-    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st));
+    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st, true));
     if (T == 1) {
       JB_TRY(launch_lsf_step_norm(out, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
-                                  w_next ? xn_next : nullptr, B, C, st));
+                                  w_next ? xn_next : nullptr, B, C, st, true));
     } else {
       void* lsf_scratch = (h_in && h_in == h_out) || ws.lsf == ws.meta ? nullptr : w + ws.lsf;
       JB_TRY(launch_lsf_scan(out, 1, nullptr, nullptr, nullptr, p.var_scale, p.alpha_min, p.alpha_max, h_in, x, nullptr, 0,

@@ -359,6 +359,14 @@ inline void launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   (void)cudaLaunchKernelEx(&cfg, kernel, KArgs(static_cast<Args&&>(args))...);   // errors: cudaGetLastError in JB_LAUNCH_CHECK
 }
 
+// Reads n floats into this SM's L1 (a word of every 128-byte line), for use after the grid dependency.
+__device__ __forceinline__ void touch_floats(const float* p, int n) {
+  for (int i = int(threadIdx.x) * 32; i < n; i += int(blockDim.x) * 32) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p + i));
+  }
+}
+
 // Same for a grid of thread-block clusters (grid.x a multiple of `cluster`).
 template <typename... KArgs, typename... Args>
 inline void launch_dep_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t stream,

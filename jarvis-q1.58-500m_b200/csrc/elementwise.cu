@@ -41,6 +41,7 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* p, const fl
 template <typename TIn, typename TOut, int MAXV>
 __global__ void __launch_bounds__(ROW_THREADS) rmsnorm_kernel(const TIn* __restrict__ x, const float* __restrict__ w,
                                                               float eps, TOut* __restrict__ y, int n_rows, int C) {
+  touch_floats(w, C);                      // a weight: not written by a kernel that may still be running
   pdl_wait();
   pdl_trigger();
   const int row = blockIdx.x * (ROW_THREADS / 32) + (threadIdx.x >> 5);

@@ -61,7 +61,7 @@ int launch_moe_metadata_static(const int64_t* topk_idx, int n_tokens, int K, int
 int launch_dispatch_gather(const void* x_bf16, const int* gather_map, int M, int n_tokens, int C, void* dispatched,
                            cudaStream_t stream);
 int launch_scatter_combine(const void* y_bf16, const float* gates, const int* scatter_map, int n_tokens, int K, int C,
-                           void* out, int out_dtype, double* stats, cudaStream_t stream);
+                           void* out, int out_dtype, double* stats, cudaStream_t stream, bool ahead = false);
 int launch_moe_finalize(const double* stats, const double* probs_sum, const int* top1_hist, int E, long long n_tokens,
                         long long n_elems, float balance_alpha, float* scalars, cudaStream_t stream);
 
@@ -86,7 +86,7 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
 size_t lsf_scan_scratch_bytes(int B, int T, int D);
 int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* var_scale, float alpha_min, float alpha_max,
                          const float* h_in, float* h_out, float* x, const float* w_norm, float eps, void* xn_bf16, int B,
-                         int C, cudaStream_t stream);
+                         int C, cudaStream_t stream, bool ahead = false);
 
 // settled (T == 1): s_in and pos0 were complete before the kernel ahead of this one on the stream began.
 int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, const float* gamma,

@@ -86,12 +86,13 @@ __device__ __forceinline__ float lsf_decay(const Args& p) {
   return lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), var);
 }
 // One thread of the whole grid leaves the MoE layer's scalars.
+__device__ __forceinline__ void moe_leave_scalars(const LsfStats& st) {
+  moe_finalize_scalars(st.stats, st.probs_sum, st.top1_hist, st.E, st.n_tokens, st.n_elems, st.balance_alpha, st.scalars);
+  if (st.reflect)
+    *st.reflect = reflect_penalty(st.lam, st.tau, __ldg(st.mu), moe_act_mean(st.stats, st.n_elems), moe_act_var(st.stats, st.n_elems));
+}
 __device__ __forceinline__ void lsf_leave_scalars(const LsfStats& st) {
-  if (st.stats && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) {
-    moe_finalize_scalars(st.stats, st.probs_sum, st.top1_hist, st.E, st.n_tokens, st.n_elems, st.balance_alpha, st.scalars);
-    if (st.reflect)
-      *st.reflect = reflect_penalty(st.lam, st.tau, __ldg(st.mu), moe_act_mean(st.stats, st.n_elems), moe_act_var(st.stats, st.n_elems));
-  }
+  if (st.stats && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) moe_leave_scalars(st);
 }
 
 template <typename T>
@@ -296,16 +297,41 @@ struct LsfStepParams {
   float eps;
   __nv_bfloat16* xn;           // [B][C] out (with w_norm)
   int B, C;
+  bool ahead;
 };
 
+// The scalars are left by a CTA of their own.  What the kernel before this one did not make (`ahead`: it made m and the
+// statistics) is fetched before the grid dependency is waited for.
 __global__ void __launch_bounds__(256) lsf_step_norm_kernel(const LsfStepParams p) {
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const bool scalars = blockIdx.x == gridDim.x - 1, on = !scalars && row < p.B;
+  const size_t base = size_t(row) * p.C;
+  float4 hq[4][2], xq[4][2];
+  auto fetch = [&] {
+    if (!on) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = (i * 32 + lane) * 8;
+      if (c < p.C) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          hq[i][q] = p.h_in ? *reinterpret_cast<const float4*>(p.h_in + base + c + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+          xq[i][q] = *reinterpret_cast<const float4*>(p.x + base + c + 4 * q);
+        }
+      }
+    }
+  };
+  if (p.ahead) fetch();
+  __syncwarp();
   pdl_wait();
   pdl_trigger();
-  lsf_leave_scalars(p.st);
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= p.B) return;
+  if (!p.ahead) fetch();
+  if (scalars) {
+    if (threadIdx.x == 0) moe_leave_scalars(p.st);
+    return;
+  }
+  if (!on) return;
   const float alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), moe_act_var(p.st.stats, p.st.n_elems));
-  const size_t base = size_t(row) * p.C;
   float v[4][8];
   float ss = 0.f;
 #pragma unroll
@@ -315,16 +341,8 @@ __global__ void __launch_bounds__(256) lsf_step_norm_kernel(const LsfStepParams 
       const uint4 mw = __ldg(reinterpret_cast<const uint4*>(p.m + base + c));
       const float mv[8] = {bf16_lo(mw.x), bf16_hi(mw.x), bf16_lo(mw.y), bf16_hi(mw.y),
                            bf16_lo(mw.z), bf16_hi(mw.z), bf16_lo(mw.w), bf16_hi(mw.w)};
-      float h[8];
-      if (p.h_in) {
-        const float4 a = *reinterpret_cast<const float4*>(p.h_in + base + c), b = *reinterpret_cast<const float4*>(p.h_in + base + c + 4);
-        h[0] = a.x; h[1] = a.y; h[2] = a.z; h[3] = a.w; h[4] = b.x; h[5] = b.y; h[6] = b.z; h[7] = b.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) h[j] = 0.f;
-      }
-      const float4 xa = *reinterpret_cast<const float4*>(p.x + base + c), xb = *reinterpret_cast<const float4*>(p.x + base + c + 4);
-      const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+      float h[8] = {hq[i][0].x, hq[i][0].y, hq[i][0].z, hq[i][0].w, hq[i][1].x, hq[i][1].y, hq[i][1].z, hq[i][1].w};
+      const float xv[8] = {xq[i][0].x, xq[i][0].y, xq[i][0].z, xq[i][0].w, xq[i][1].x, xq[i][1].y, xq[i][1].z, xq[i][1].w};
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         h[j] = lsf_step(alpha, h[j], mv[j]);
@@ -402,8 +420,6 @@ template <bool FUSED, int CH>
 __global__ void __launch_bounds__(LsfTma<FUSED, CH>::THREADS, (FUSED ? 2 : 4) * LsfTma<FUSED, CH>::RPW)
 lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_io, const LsfArgs<true, FUSED> p,
                const int n_stages, unsigned int* status) {
-  pdl_wait();
-  pdl_trigger();
   using Cfg = LsfTma<FUSED, CH>;
   constexpr int TPW = LT_TOK / LSF_WARPS;    // 16 (sixteen warps of 8 tokens were measured: slower)
   extern __shared__ uint8_t lsf_smem_raw[];
@@ -424,6 +440,32 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
   const int t_end = min(p.T, t_begin + p.seg_len);
   const int n_tiles = (t_end - t_begin + LT_TOK - 1) / LT_TOK;
 
+  // in a chain the kernel before this one made m and the statistics alone: residual tiles are fetched ahead of it
+  bool ahead = false;
+  if constexpr (FUSED) ahead = p.st.stats != nullptr;
+  auto issue = [&](int i, bool residual, bool input) {      // thread 0 only
+    const int s = i % n_stages;
+    const uint32_t bar = smem_u32(&full[s]);
+    const uint32_t dst = smem_u32(tiles + size_t(s) * Cfg::STAGE_BYTES);
+    if (residual) mbar_arrive_expect_tx(bar, Cfg::STAGE_BYTES);
+    if (FUSED && residual) tma_load_3d(dst + Cfg::M_BYTES, &tm_io, ch0, t_begin + i * LT_TOK, b, bar);
+    if (input) tma_load_3d(dst, &tm_m, ch0, t_begin + i * LT_TOK, b, bar);
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < n_stages; ++s) mbar_init(smem_u32(&full[s]), 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tm_m);
+    tma_prefetch_desc(&tm_io);
+    if (ahead)
+      for (int i = 0; i < n_stages && i < n_tiles; ++i) issue(i, true, false);
+  }
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+  if (threadIdx.x == 0)
+    for (int i = 0; i < n_stages && i < n_tiles; ++i) issue(i, !ahead, true);
+  __syncwarp();
   const float alpha = lsf_decay(p);
   if constexpr (FUSED) lsf_leave_scalars(p.st);
   float pw[TPW];   // alpha^(i+1)
@@ -445,22 +487,6 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
     }
   }
 
-  auto issue = [&](int i) {      // thread 0 only
-    const int s = i % n_stages;
-    const uint32_t bar = smem_u32(&full[s]);
-    const uint32_t dst = smem_u32(tiles + size_t(s) * Cfg::STAGE_BYTES);
-    mbar_arrive_expect_tx(bar, Cfg::STAGE_BYTES);
-    tma_load_3d(dst, &tm_m, ch0, t_begin + i * LT_TOK, b, bar);
-    if (FUSED) tma_load_3d(dst + Cfg::M_BYTES, &tm_io, ch0, t_begin + i * LT_TOK, b, bar);
-  };
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < n_stages; ++s) mbar_init(smem_u32(&full[s]), 1);
-    *abort_flag = 0;
-    fence_mbar_init();
-    tma_prefetch_desc(&tm_m);
-    tma_prefetch_desc(&tm_io);
-    for (int i = 0; i < n_stages && i < n_tiles; ++i) issue(i);
-  }
   __syncthreads();
 
   bool ok = true;
@@ -518,11 +544,11 @@ lsf_tma_kernel(const __grid_constant__ CUtensorMap tm_m, const __grid_constant__
         // it, so that this thread does not sit out the latency of the store it has just issued
         if (i >= 1 && i - 1 + n_stages < n_tiles) {
           bulk_wait_group_read<1>();
-          issue(i - 1 + n_stages);
+          issue(i - 1 + n_stages, true, true);
         }
       } else if (i + n_stages < n_tiles) {
         bulk_wait_group_read<0>();   // the store has read the stage: it may be filled again
-        issue(i + n_stages);
+        issue(i + n_stages, true, true);
       }
     }
   }
@@ -790,7 +816,7 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
 
 int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* var_scale, float alpha_min, float alpha_max,
                          const float* h_in, float* h_out, float* x, const float* w_norm, float eps, void* xn_bf16, int B,
-                         int C, cudaStream_t stream) {
+                         int C, cudaStream_t stream, bool ahead) {
   JB_REQUIRE(B >= 0 && C > 0, "lsf_step_norm: bad shape (%d, %d)", B, C);
   JB_REQUIRE(C % 8 == 0 && C <= 1024, "lsf_step_norm: d_model (%d) must be a multiple of 8 and at most 1024", C);
   JB_REQUIRE(st.E >= 0 && st.E <= 64 && st.n_tokens > 0 && st.n_elems > 0, "lsf_step_norm: bad counts");
@@ -807,7 +833,8 @@ int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* va
   p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;
   p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
   p.B = B; p.C = C;
-  launch_dep(lsf_step_norm_kernel, (B + 7) / 8, 256, 0, stream, p);
+  p.ahead = ahead;
+  launch_dep(lsf_step_norm_kernel, (B + 7) / 8 + 1, 256, 0, stream, p);
   JB_LAUNCH_CHECK("lsf_step_norm_kernel");
   return JB200_OK;
 }
