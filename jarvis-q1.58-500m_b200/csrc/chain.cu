@@ -157,7 +157,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     else if (mid)
       JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv));
     else
-      JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st));
+      JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st, nullptr, true));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
     void* attn_scratch = (T > 1 && !(s_in && s_in == s_out)) ? w + ws.attn : nullptr;
     if (attn_scratch && ws.attn == ws.lsf) attn_scratch = nullptr;            // no scratch wanted at this shape
@@ -168,7 +168,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     else if (mid)
       JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x));
     else
-      JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st));
+      JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st, nullptr, true));
 
     // moe(norm2(x))
     if (N <= ROUTE_SMALL_MAX) {
@@ -186,14 +186,14 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       if (mid)
         JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid));
       else
-        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st));
+        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, N, true, st));
     else if (mid)
       JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y));
     else
-      JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st));
+      JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st, nullptr, true));
 
     // combine, x += lsf(moe), and the norm of what follows
     const float* w_next = last ? f->w_final : layers[l + 1].w_norm1;

@@ -114,6 +114,7 @@ struct GemmParams {
   int bn;                    // token tile
   int epilogue;
   int w_layout;              // 0 canonical weight_packing.py layout, 1 prepared layout
+  int settled;               // weights and segments were complete before the kernel ahead of this one started
   unsigned int* status;
   // JB200_EPI_RESID_F32: 8 staging tiles of [32 tokens][32 features] f32 in shared memory (one per epilogue warp),
   // from which the tile is ADDED to the residual stream by a TMA reduction; 0 = plain read-modify-write from registers

@@ -24,7 +24,7 @@ struct GemmRope {
 };
 int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packed, const float* alpha,
                         int alpha_rows, int N, int G, const int32_t* seg_offsets, int epilogue, void* out,
-                        int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope = nullptr);
+                        int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope = nullptr, bool settled = false);
 // The same product for a few tokens (small_gemm.cu), bit for bit.  idx / scatter ([M][2]): all M rows go through every group's
 // matrix and row n is stored at scatter[2n + k] where idx[2n + k] is the group; else seg as above.  tokens: about how many
 // rows a call holds (chooses the tile).  settled: weights and seg were complete before the kernel ahead of this one on the

@@ -233,8 +233,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     pair_tmem_relinquish();
   }
   __syncwarp();
-  pdl_wait();
-  pdl_trigger();
+  // In a chain (`settled`) only the activations are the work of the kernel before this one: the warp that loads them waits
+  // for it, while codes are loaded and decoded into every stage there is.  All else follows from its loads.
+  if (!p.settled) {
+    pdl_wait();
+    pdl_trigger();
+  }
   if (threadIdx.x == 0) {
     if (p.seg_offsets) {
       for (int g = 0; g <= p.G; ++g) ctl->seg[g] = min(max(p.seg_offsets[g], 0), p.M);
@@ -257,6 +261,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer: this CTA's tokens (and, dense, its weight rows) ----------------
+    if (p.settled) {
+      pdl_wait();
+      pdl_trigger();
+    }
     int s = 0;
     uint32_t ph = 1u;
     bool ok = true;
