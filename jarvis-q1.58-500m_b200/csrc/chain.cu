@@ -50,9 +50,9 @@ struct Workspace {
 
 // Which form of the ternary product a call of so many tokens runs (their results are the same bits): up to 16 tokens
 // mma.sync straight from the codes (24 layers of single-token steps 0.62 against 0.86 ms at 1 sequence, equal at 16), up to
-// MID_TOKENS the tcgen05 form that is built for latency (512 tokens 2.15 against 2.54 ms, 1024 2.65 against 2.75, 1280 equal,
-// 1500 3.13 against 3.08), beyond that the persistent pipeline.
-constexpr int SMALL_TOKENS = 16, MID_TOKENS = 1280;
+// MID_TOKENS the tcgen05 form that is built for latency (640 tokens 1.96 against 2.08 ms, 900 2.20 against 2.29, 1000 equal,
+// 1152 2.81 against 2.74), beyond that the persistent pipeline.
+constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
 // tokens) that leaves a launch of so many rows in each group one wave.
 inline int mid_tile(int rows, int groups, int n_ft, int sms) {
