@@ -53,6 +53,8 @@ struct Workspace {
 // MID_TOKENS the tcgen05 form that is built for latency (640 tokens 1.96 against 2.08 ms, 900 2.20 against 2.29, 1000 equal,
 // 1152 2.81 against 2.74), beyond that the persistent pipeline.
 constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
+// Up to here the first expert GEMM takes all rows for every expert and stores the routed ones: more MMAs, no dispatch.
+constexpr int ALL_ROWS_TOKENS = 64;
 // Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
 // tokens) that leaves a launch of so many rows in each group one wave.
 inline int mid_tile(int rows, int groups, int n_ft, int sms) {
@@ -174,14 +176,17 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (N <= ROUTE_SMALL_MAX) {
       JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, ticket, counts, offs,
                                 scatter, gather, gate_idx, st));
+    } else {
+      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st));
+      JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
+    }
+    if (N <= ALL_ROWS_TOKENS) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
       if (small)
         JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, N, true, st));
       else
         JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid));
     } else {
-      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st));
-      JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
       JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
         JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid));

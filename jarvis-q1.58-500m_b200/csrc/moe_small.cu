@@ -53,7 +53,10 @@ struct RouteParams {
 
 // One warp per token and CTA: with all weights of the lane's channels in registers before the residual row arrives, the
 // chain is load - sum - norm - dot - sums - softmax.
-template <int E>
+// ROUNDS: 32 assignments each that the last warp sorts, all loaded at once (one by one they were 300 cycles each, twice).
+// Up to 256 tokens it beats the persistent router and the metadata kernel (24 single-token layers: 128 sequences 1485 -> 1454 us,
+// 256 1809 -> 1791; 64, from the loads alone, 1122 -> 1104).
+template <int E, int ROUNDS>
 __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
   __shared__ int h_acc[E];
   const int lane = threadIdx.x, tok = blockIdx.x;
@@ -134,11 +137,14 @@ __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
   const int M = 2 * p.N;
   const long long* ids = reinterpret_cast<const long long*>(p.idx);
   int n_of = 0;                                  // lane e < E: assignments of expert e
-  for (int m0 = 0; m0 < M; m0 += 32) {
-    const int e = m0 + lane < M ? int(__ldcg(ids + m0 + lane)) : -1;
+  int ex[ROUNDS];
+#pragma unroll
+  for (int i = 0; i < ROUNDS; ++i) ex[i] = i * 32 + lane < M ? int(__ldcg(ids + i * 32 + lane)) : -1;
+#pragma unroll
+  for (int i = 0; i < ROUNDS; ++i) {
 #pragma unroll
     for (int q = 0; q < E; ++q) {
-      const unsigned b = __ballot_sync(0xffffffffu, e == q);
+      const unsigned b = __ballot_sync(0xffffffffu, ex[i] == q);
       if (lane == q) n_of += __popc(b);
     }
   }
@@ -154,9 +160,9 @@ __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
     p.offsets[lane] = at;
     if (lane == E - 1) p.offsets[E] = incl;
   }
-  for (int m0 = 0; m0 < M; m0 += 32) {
-    const int m = m0 + lane;
-    const int e = m < M ? int(__ldcg(ids + m)) : -1;
+#pragma unroll
+  for (int i = 0; i < ROUNDS; ++i) {
+    const int m = i * 32 + lane, e = ex[i];
     int slot = 0;
 #pragma unroll
     for (int q = 0; q < E; ++q) {
@@ -561,8 +567,14 @@ int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_
   p.idx = idx; p.gates = gates; p.probs_sum = probs_sum; p.hist = hist; p.ticket = ticket;
   p.counts = counts; p.offsets = offsets; p.scatter = scatter; p.gather = gather; p.gate_idx = gate_idx;
   p.eps = eps; p.N = N; p.C = C;
-  if (E == 4) launch_dep(route_small_kernel<4>, N, 32, 0, stream, p);
-  else launch_dep(route_small_kernel<8>, N, 32, 0, stream, p);
+  static_assert(ROUTE_SMALL_MAX == 256, "sixteen rounds of sixteen tokens");
+  if (N <= 64) {
+    if (E == 4) launch_dep(route_small_kernel<4, 4>, N, 32, 0, stream, p);
+    else launch_dep(route_small_kernel<8, 4>, N, 32, 0, stream, p);
+  } else {
+    if (E == 4) launch_dep(route_small_kernel<4, 16>, N, 32, 0, stream, p);
+    else launch_dep(route_small_kernel<8, 16>, N, 32, 0, stream, p);
+  }
   JB_LAUNCH_CHECK("route_small_kernel");
   return JB200_OK;
 }
