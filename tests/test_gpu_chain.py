@@ -169,3 +169,19 @@ def test_attention_at_the_line_between_whole_sequences_and_segments(B, T, cut):
     # cut: the state enters a segment through gamma^(chunk length) and one more f32 sum; outputs are bf16 (2^-9)
     assert rel(o1.float(), o2.float()) < 2.0 ** -9 and rel(s1, s2) < 1e-5
     assert torch.equal(s1, s2) is not cut
+
+
+@pytest.mark.parametrize("E", [1, 4, 16])
+@pytest.mark.parametrize("N", [1, 17, 511, 512, 513, 1000, 1024, 1025])
+def test_dispatch_metadata_around_the_one_cta_form(N, E):
+    """One round, two rounds, three kernels; expected maps from a stable sort on the host."""
+    idx = torch.randint(0, E, (N, 2), generator=torch.Generator().manual_seed(N))
+    idx[N // 2:] = E - 1                                                       # uneven
+    flat = idx.flatten()
+    order = torch.argsort(flat, stable=True)
+    counts = torch.bincount(flat, minlength=E)
+    slots = torch.empty(2 * N, dtype=torch.long)
+    slots[order] = torch.arange(2 * N)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+    for got, want in zip(ops.moe_metadata(idx.cuda(), E), (counts, offsets, slots, order // 2, order % 2)):
+        assert torch.equal(got.cpu().flatten().long(), want)
