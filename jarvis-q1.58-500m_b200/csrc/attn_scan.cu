@@ -1199,13 +1199,6 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   p.nseg = 1;
   p.seg_state = reinterpret_cast<float*>(scratch);
   if (scratch) pick_segments(B, T, H, sms, &p.seg_chunks, &p.nseg);   // without scratch: one segment per sequence
-  // A chunk takes 1.9 us; cutting costs the pass over the segments ahead: 3.5 us and 3.7 us per chunk of a segment in all
-  // (per layer of a forward; 4 chunks whole 3.3 us less than in two segments, 4 x 600 tokens 4.3 us less, 8 chunks in four
-  // segments 4.3 us less than whole).
-  if (o && 20 * ((T + CH - 1) / CH) < 38 * p.seg_chunks + 36) {
-    p.seg_chunks = (T + CH - 1) / CH;
-    p.nseg = 1;
-  }
   JB_REQUIRE(p.nseg <= 65535, "attn_scan: too many segments");
   JB_REQUIRE(!scratch || aligned16(scratch), "attn_scan: scratch pointer must be 16-byte aligned");
   p.n_pieces = o ? p.nseg - 1 : p.nseg;

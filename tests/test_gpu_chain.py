@@ -155,22 +155,6 @@ def test_residual_scan_with_its_tiles_side_by_side(B, T, D):
     assert _lib.device_status() == 0
 
 
-@pytest.mark.parametrize("B,T,cut", [(4, 600, False), (3, 896, False), (3, 897, True), (1, 897, True), (4, 1024, False)])
-def test_attention_at_the_line_between_whole_sequences_and_segments(B, T, cut):
-    """Few sequences of few chunks are scanned whole although SMs stay empty; the bits tell which way a call went."""
-    gen = torch.Generator(device="cuda").manual_seed(T)
-    qkv = torch.randn(B * T, 3072, generator=gen, device="cuda").bfloat16()
-    S = torch.randn(B, 16, 64, 64, generator=gen, device="cuda")
-    gamma = torch.rand(16, generator=gen, device="cuda") * 0.099 + 0.9
-    cos, sin = jm.RotaryEmbedding(64, T).half_tables(T, qkv.device)
-    args = (qkv[:, :1024], qkv[:, 1024:2048], qkv[:, 2048:], gamma, cos, sin, B, T, 16)
-    o1, s1 = ops.attn_scan(*args, state_in=S, want_state=True)
-    o2, s2 = ops.attn_scan(*args, state_in=S, want_state=True, segmented=False)
-    # cut: the state enters a segment through gamma^(chunk length) and one more f32 sum; outputs are bf16 (2^-9)
-    assert rel(o1.float(), o2.float()) < 2.0 ** -9 and rel(s1, s2) < 1e-5
-    assert torch.equal(s1, s2) is not cut
-
-
 @pytest.mark.parametrize("E", [1, 4, 16])
 @pytest.mark.parametrize("N", [1, 17, 511, 512, 513, 1000, 1024, 1025])
 def test_dispatch_metadata_around_the_one_cta_form(N, E):
