@@ -54,17 +54,20 @@ namespace {
 
 constexpr int BM = 128;         // out-feature rows per tile  (UMMA M)
 constexpr int BK = 64;          // k elements per stage (= one 128-byte swizzle row of bf16)
-constexpr int STAGES = 4;
+constexpr int MAX_STAGES = 8;
 constexpr int BN_MAX = 256;     // token columns per tile (UMMA N), runtime 32..256
 constexpr int A_STAGE_BYTES = BM * BK * 2;       // 16 KiB
-constexpr int B_STAGE_BYTES = BN_MAX * BK * 2;   // 32 KiB
+// Ring of four stages with room for 256 tokens each, or of eight for at most 64 tokens: dense weights for few tokens are a
+// stream from HBM, and four weight tiles in flight per SM do not cover its latency (lm_head, 1 to 64 rows: 23.4-24.6 us with
+// four, 21.7-23.2 with eight; 16 us of bytes, in three rounds of tiles where 2.65 are needed).
+constexpr int b_stage_bytes(int stages) { return (stages == 8 ? 64 : BN_MAX) * BK * 2; }
 constexpr int NUM_THREADS = 576;
 constexpr int DEC_WARP0 = 2, EPI_WARP0 = 10;
 constexpr int TMEM_COLS = 512;
 
 struct SmemCtl {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
@@ -74,7 +77,8 @@ struct SmemCtl {
 
 constexpr size_t CTL_BYTES = ((sizeof(SmemCtl) + 127) / 128) * 128;
 constexpr int RESID_STAGE_BYTES = 32 * 32 * 4;                   // one [32 tokens][32 features] f32 tile per epilogue warp
-constexpr size_t SMEM_BYTES = 1024 /*alignment slack*/ + size_t(STAGES) * (A_STAGE_BYTES + B_STAGE_BYTES) + CTL_BYTES;
+constexpr size_t SMEM_BYTES = 1024 /*alignment slack*/ + size_t(4) * (A_STAGE_BYTES + b_stage_bytes(4)) + CTL_BYTES;
+static_assert(8 * (A_STAGE_BYTES + b_stage_bytes(8)) == 4 * (A_STAGE_BYTES + b_stage_bytes(4)), "the rings take the same room");
 constexpr size_t SMEM_BYTES_RESID = SMEM_BYTES + 8 * RESID_STAGE_BYTES;
 
 struct TileCoord {
@@ -103,9 +107,11 @@ __device__ __forceinline__ bool tile_coord(const SmemCtl* ctl, int t, int n_ft, 
   return false;
 }
 
+template <int STAGES>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 ternary_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                     const __grid_constant__ CUtensorMap tmap_out, const GemmParams p) {
+  constexpr int B_STAGE_BYTES = b_stage_bytes(STAGES);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -370,9 +376,11 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
   if (!p.status) return JB200_ERR_CUDA;
 
   // More than 512 rows: the CTA-pair kernel (24 layers of 700 / 2048 / 16384 tokens 2.54 / 3.32 / 14.0 ms against 2.63 / 3.68 /
-  // 15.7 here).  What is left to this one are small calls, in-features that are no multiple of 256, the q/k RoPE epilogue
+  // 15.7 here).  Dense weights: from 65 rows on, since the tiles of 64 tokens that a small call is cut into here read all of them
+  // once each (lm_head, 128 rows 25.7 against 36.7 us, 256 27.5 against 62, 512 46.8 against 113; 64 rows 24.1 against 22.8).
+  // What is left to this one are small calls, in-features that are no multiple of 256, the q/k RoPE epilogue
   // and callers that ask for a token tile.
-  if (bn_override == 0 && K % 256 == 0 && M > 512 && !rope) return launch_pair_gemm(p, x_bf16, sms, stream);
+  if (bn_override == 0 && K % 256 == 0 && M > (w_layout == 2 ? 64 : 512) && !rope) return launch_pair_gemm(p, x_bf16, sms, stream);
 
   CUtensorMap tmap;
   const cuuint64_t gdim[2] = {cuuint64_t(K), cuuint64_t(M)};
@@ -404,10 +412,12 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
     p.resid_stage_smem = 1;
   }
   const size_t smem_bytes = p.resid_stage_smem ? SMEM_BYTES_RESID : SMEM_BYTES;
-  JB_MAX_SMEM(ternary_gemm_kernel, SMEM_BYTES_RESID);
+  auto kernel = w_layout == 2 && bn <= 64 ? ternary_gemm_kernel<8> : ternary_gemm_kernel<4>;
+  JB_MAX_SMEM(ternary_gemm_kernel<4>, SMEM_BYTES_RESID);
+  JB_MAX_SMEM(ternary_gemm_kernel<8>, SMEM_BYTES_RESID);
   const long max_tiles = long((M + bn - 1) / bn + (G - 1)) * n_ft;
   const int grid = int(max_tiles < sms ? max_tiles : sms);
-  launch_dep(ternary_gemm_kernel, grid, NUM_THREADS, smem_bytes, stream, tmap, tmap_w, tmap_out, p);
+  launch_dep(kernel, grid, NUM_THREADS, smem_bytes, stream, tmap, tmap_w, tmap_out, p);
   JB_LAUNCH_CHECK("ternary_gemm_kernel");
   return JB200_OK;
 }

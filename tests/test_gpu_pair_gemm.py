@@ -1,4 +1,4 @@
-"""The CTA-pair GEMM (calls of more than 512 rows) at the sizes where it can go wrong: ragged token tiles and segments, empty
+"""The CTA-pair GEMM (calls of more than 512 rows, dense weights from 65 rows on) at the sizes where it can go wrong: ragged token tiles and segments, empty
 segments, out-features that are odd multiples of 128, cut tiles of the last wave, one to many K-chunks.  Small-integer
 activations make every product and sum exact, so the comparison with a plain f32 matmul is exact; the GELU form is compared
 with the one-CTA kernel bit for bit."""
@@ -51,7 +51,8 @@ def test_grouped_forms_are_exact(M, N, K, cuts):
     assert _lib.device_status() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(513, 128, 256), (1111, 640, 1024), (3000, 50304, 256)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (33, 640, 1024), (64, 50304, 1024), (65, 128, 256), (100, 640, 1024),
+                                   (256, 50304, 1024), (257, 384, 512), (513, 128, 256), (1111, 640, 1024), (3000, 50304, 256)])
 def test_dense_weights_are_exact(M, N, K):
     gen = torch.Generator(device="cuda").manual_seed(N)
     x = torch.randint(-3, 4, (M, K), generator=gen, device="cuda").bfloat16()
