@@ -6,6 +6,7 @@ runs in C++ and Python pays for one call, a handful of allocations and the check
 from __future__ import annotations
 
 import ctypes as C
+import math
 import operator
 import weakref
 from typing import List, Optional
@@ -138,18 +139,40 @@ def table_of(owner, blocks) -> Optional[LayerTable]:
     return tab if tab.local() else None
 
 
-def _f32_list(ts: Optional[List[Optional[torch.Tensor]]]):
-    if ts is None:
-        return None
-    return [t if t is None or (t.dtype is torch.float32 and t.is_contiguous()) else t.float().contiguous() for t in ts]
+def _carried(ts, n: int, shape, dev, what: str, exact: bool = True, must_alias=None) -> List[Optional[torch.Tensor]]:
+    """The carried states of n layers as contiguous f32 tensors (or None), checked: the native call reads and writes through
+    their addresses.  exact: the shape itself and not just its number of elements.  must_alias(t): the caller's own tensor is
+    to be updated, so one that would have to be converted is refused."""
+    ts = list(ts)
+    if len(ts) < n:
+        raise RuntimeError(f"forward: {what} has {len(ts)} entries for {n} layers")
+    numel, out = math.prod(shape), []
+    for t in ts[:n]:
+        if t is not None:
+            if t.device != dev:
+                raise RuntimeError(f"forward: {what} on {t.device}, expected {dev} (this path has no CPU fallback)")
+            if t.shape != shape if exact else t.numel() != numel:
+                raise RuntimeError(f"forward: {what} of shape {tuple(t.shape)}, expected {shape}")
+            if t.dtype is not torch.float32 or not t.is_contiguous():
+                if must_alias is not None and must_alias(t):
+                    raise RuntimeError(f"forward: {what} updated in place must be contiguous f32, got {t.dtype} {tuple(t.stride())}")
+                t = t.float().contiguous()
+        out.append(t)
+    return out
 
 
 def _pointers(n, ts):
     return (C.c_void_p * n)(*[None if t is None else t.data_ptr() for t in ts])
 
 
-def _rows_of(n, base, stride):
-    return (C.c_void_p * n)(*range(base, base + n * stride, stride))
+def _results(n, given, inplace, shape, dev):
+    """Where the states after the call go, one tensor per layer: the given ones (in place), new ones where there are none."""
+    kept = given if inplace and given is not None else [None] * n
+    missing = sum(t is None for t in kept)
+    if not missing:
+        return kept
+    new = iter(torch.empty((missing, *shape), dtype=torch.float32, device=dev).unbind(0))
+    return [next(new) if t is None else t for t in kept]
 
 
 class Result:
@@ -161,10 +184,18 @@ class Result:
 def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0, max_position=None, h_in=None, s_in=None,
         want_state=False, inplace=False, final_norm=None) -> Result:
     """One jb200_forward_layers call on the current stream.  x: f32 (B*T, C), updated in place (written from `ids` and the
-    embedding `table` when given).  h_in / s_in: lists with one f32 tensor or None per layer, or None."""
+    embedding `table` when given).  h_in / s_in: lists with one tensor or None per layer, or None; inplace: layer by layer, the
+    states that are given are updated."""
     n, dev = tab.n, tab.device
-    if not (x.is_cuda and x.dtype is torch.float32 and x.is_contiguous()):
-        raise RuntimeError("forward: expected a contiguous f32 CUDA residual stream (this path has no CPU fallback)")
+    if not (x.device == dev and x.dtype is torch.float32 and x.is_contiguous() and x.shape == (B * T, tab.C)):
+        raise RuntimeError(f"forward: expected a contiguous f32 residual stream ({B * T}, {tab.C}) on {dev} (this path has no CPU fallback)")
+    step = ids is not None and T == 1         # a model's single-token step
+    if h_in is not None:
+        # the tail of a single-token step leaves a new membrane where it cannot update the one it was given
+        alias = (lambda t: t.dtype is torch.float32 or not step) if inplace else None
+        h_in = _carried(h_in, n, (B, tab.C), dev, "the membrane", exact=step, must_alias=alias)
+    if s_in is not None:
+        s_in = _carried(s_in, n, (B, tab.H, 64, 64), dev, "the attention state")
     ws_bytes, routing_bytes, _ = tab.sizes(B, T)
     head = (n * tab.acc_bytes + 255) // 256 * 256
     work = torch.empty(head + ws_bytes, dtype=torch.uint8, device=dev)
@@ -178,8 +209,8 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
         f.ids, f.table, f.vocab = ids.data_ptr(), table.data_ptr(), table.shape[0]
     f.x = x.data_ptr()
     if torch.is_tensor(start_pos):
-        if not (start_pos.is_cuda and start_pos.dtype is torch.int32 and start_pos.is_contiguous() and start_pos.numel() == B):
-            raise RuntimeError("forward: per-sequence positions must be a contiguous int32 CUDA tensor with one entry per sequence")
+        if not (start_pos.device == dev and start_pos.dtype is torch.int32 and start_pos.is_contiguous() and start_pos.numel() >= B):
+            raise RuntimeError(f"forward: per-sequence positions must be a contiguous int32 tensor on {dev} with one entry per sequence")
         # without the caller's bound the table is sized from the positions themselves (a host read)
         end = (max_position if max_position is not None else int(start_pos.max())) + T
         f.pos0 = start_pos.data_ptr()
@@ -188,26 +219,19 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
         end = f.pos0_scalar + T
     cos, sin = tab.rotary.half_tables(end, dev)
     f.cos_tab, f.sin_tab, f.n_pos = cos.data_ptr(), sin.data_ptr(), cos.shape[0]
-    h_in, s_in = _f32_list(h_in), _f32_list(s_in)
     if h_in is not None:
         h_ptrs = _pointers(n, h_in)
         f.h_in = C.addressof(h_ptrs)
     if s_in is not None:
         s_ptrs = _pointers(n, s_in)
         f.s_in = C.addressof(s_ptrs)
-    if inplace and h_in is not None and None not in h_in:
-        res.h, ho_ptrs = h_in, h_ptrs
-    else:
-        h_all = torch.empty((n, B, tab.C), dtype=torch.float32, device=dev)
-        res.h, ho_ptrs = list(h_all.unbind(0)), _rows_of(n, h_all.data_ptr(), B * tab.C * 4)
+    res.h = _results(n, h_in, inplace, (B, tab.C), dev)
+    ho_ptrs = _pointers(n, res.h)
     f.h_out = C.addressof(ho_ptrs)
     res.S = None
-    if inplace and s_in is not None and None not in s_in:
-        res.S, so_ptrs = s_in, s_ptrs
-        f.s_out = C.addressof(so_ptrs)
-    elif want_state:
-        s_all = torch.empty((n, B, tab.H, 64, 64), dtype=torch.float32, device=dev)
-        res.S, so_ptrs = list(s_all.unbind(0)), _rows_of(n, s_all.data_ptr(), B * tab.H * 64 * 64 * 4)
+    if want_state or (inplace and s_in is not None):
+        res.S = _results(n, s_in, inplace, (B, tab.H, 64, 64), dev)
+        so_ptrs = _pointers(n, res.S)
         f.s_out = C.addressof(so_ptrs)
     base = work.data_ptr()
     f.accumulators, f.workspace = base, base + head

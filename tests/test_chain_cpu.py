@@ -1,0 +1,34 @@
+"""Host side of the native forward call (chain.py) without a GPU: what it refuses before anything is launched."""
+import pytest
+import torch
+
+from jarvis_b200 import chain
+
+CPU = torch.device("cpu")
+
+
+def test_carried_states_are_checked_before_their_addresses_are_taken():
+    good = [torch.zeros(3, 128), None, torch.zeros(3, 128, dtype=torch.bfloat16)]
+    out = chain._carried(good, 3, (3, 128), CPU, "h")
+    assert out[0] is good[0] and out[1] is None and out[2].dtype is torch.float32
+    assert len(chain._carried(good + [None], 3, (3, 128), CPU, "h")) == 3          # more entries than layers: the first ones count
+    with pytest.raises(RuntimeError, match="2 entries for 3 layers"):
+        chain._carried(good[:2], 3, (3, 128), CPU, "h")
+    for exact, shape in ((True, (2, 128)), (False, (2, 128)), (True, (3, 1, 128)), (False, (4, 128))):
+        with pytest.raises(RuntimeError, match="of shape"):
+            chain._carried([torch.zeros(shape)], 1, (3, 128), CPU, "h", exact=exact)
+    chain._carried([torch.zeros(3, 1, 128)], 1, (3, 128), CPU, "h", exact=False)
+    with pytest.raises(RuntimeError, match="on meta, expected cpu"):
+        chain._carried([torch.zeros(3, 128, device="meta")], 1, (3, 128), CPU, "h")
+    with pytest.raises(RuntimeError, match="in place"):
+        chain._carried(good, 3, (3, 128), CPU, "h", must_alias=lambda t: True)
+    with pytest.raises(RuntimeError, match="in place"):
+        chain._carried([torch.zeros(128, 3).t()], 1, (3, 128), CPU, "h", must_alias=lambda t: t.dtype is torch.float32)
+
+
+def test_states_are_updated_in_place_layer_by_layer():
+    a, b = torch.zeros(3, 8), torch.zeros(3, 8)
+    got = chain._results(4, [a, None, b, None], True, (3, 8), CPU)
+    assert got[0] is a and got[2] is b and got[1].shape == got[3].shape == (3, 8) and got[1].data_ptr() != got[3].data_ptr()
+    assert all(g is not a and g is not b for g in chain._results(2, [a, b], False, (3, 8), CPU))
+    assert all(g is t for g, t in zip(chain._results(2, [a, b], True, (3, 8), CPU), (a, b)))

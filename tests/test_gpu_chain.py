@@ -169,3 +169,38 @@ def test_dispatch_metadata_around_the_one_cta_form(N, E):
     offsets = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
     for got, want in zip(ops.moe_metadata(idx.cuda(), E), (counts, offsets, slots, order // 2, order % 2)):
         assert torch.equal(got.cpu().flatten().long(), want)
+
+
+@pytest.mark.parametrize("T", [1, 5])
+def test_carried_state_that_does_not_fit_is_refused(T):
+    """Wrong batch, host memory, too few layers, a membrane that cannot be updated in place: an error before any launch."""
+    model = _model(2)
+    idx = torch.zeros((3, T), dtype=torch.int64, device="cuda")
+
+    def state(B=3, n=2, dev="cuda", dtype=torch.float32):
+        return {"h": [torch.zeros(B, 128, device=dev, dtype=dtype) for _ in range(n)],
+                "S": [torch.zeros(B, 2, 64, 64, device=dev) for _ in range(n)]}
+    model(idx)
+    launches = _lib.kernel_launches()
+    for bad in (state(B=2), state(n=1), state(dev="cpu"), {"h": state()["h"], "S": state(B=2)["S"]}):
+        for inplace in (False, True):
+            with pytest.raises((RuntimeError, IndexError)):
+                model.step(idx, 0, bad, max_position=16, inplace=inplace)
+    with pytest.raises(RuntimeError):
+        model.step(idx, torch.zeros(2, dtype=torch.int32, device="cuda"), state(), max_position=16)
+    strided = {"h": [torch.zeros(128, 3, device="cuda").t() for _ in range(2)], "S": state()["S"]}
+    with pytest.raises(RuntimeError):
+        model.step(idx, 0, strided, max_position=16, inplace=True)
+    if T > 1:
+        with pytest.raises(RuntimeError):
+            model.step(idx, 0, state(dtype=torch.bfloat16), max_position=16, inplace=True)
+    assert _lib.kernel_launches() == launches
+    model.step(idx, 0, strided, max_position=16)                   # converted where nothing has to alias
+    st = state()
+    st["S"][1] = st["h"][0] = None                                 # layers without a state get a new one, the others are updated
+    _, new = model.step(idx, 0, st, max_position=16, inplace=True)
+    assert new["S"][0] is st["S"][0] and new["h"][1] is st["h"][1] and float(st["S"][0].abs().sum()) > 0
+    assert new["S"][1] is not None and new["h"][0].shape == (3, 128)
+    with pytest.raises(RuntimeError):
+        model.blocks[0].forward_rows(torch.zeros(3 * T + 1, 128, device="cuda"), 3, T)
+    assert _lib.device_status() == 0
