@@ -20,15 +20,25 @@ _version = operator.attrgetter("_version")
 
 
 def supported(blocks) -> bool:
-    """Shapes jb200_forward_layers takes, all parameters on one CUDA device."""
+    """Shapes jb200_forward_layers takes: all parameters on one CUDA device and of the sizes the first block gives, since the
+    native call knows nothing but their addresses."""
     a = blocks[0].attn
     d_model = a.q_proj.weight.shape[1]
     hidden, E, dev = blocks[0].moe.w1[0].weight.shape[0], blocks[0].moe.num_experts, blocks[0].norm1.weight.device
     if d_model % 128 or d_model > 1024 or hidden % 128 or E not in (4, 8) or dev.type != "cuda":
         return False
-    return all(b.attn.n_heads == a.n_heads and b.attn.head_dim == 64 and b.attn.q_proj.weight.shape[1] == d_model and
-               b.moe.num_experts == E and b.moe.top_k == 2 and b.moe.w1[0].weight.shape[0] == hidden and
-               b.attn.rotary.base == a.rotary.base and all(p.device == dev for p in b.parameters()) for b in blocks)
+    return all(_fits(b, a, d_model, hidden, E) and all(p.device == dev for p in b.parameters()) for b in blocks)
+
+
+def _fits(b, a, d_model, hidden, E) -> bool:
+    at, moe = b.attn, b.moe
+    square, up, down = (d_model, d_model), (hidden, d_model), (d_model, hidden)
+    return (at.n_heads == a.n_heads and at.head_dim == 64 and at.n_heads * 64 == d_model and at.rotary.base == a.rotary.base and
+            at.gamma_raw.numel() == at.n_heads and moe.num_experts == E and moe.top_k == 2 and
+            len(moe.w1) == len(moe.w2) == E and moe.router.weight.shape == (E, d_model) and
+            b.norm1.weight.numel() == b.norm2.weight.numel() == d_model and b.liquid.var_scale.numel() == 1 and
+            all(m.weight.shape == square for m in (at.q_proj, at.k_proj, at.v_proj, at.out_proj)) and
+            all(m.weight.shape == up for m in moe.w1) and all(m.weight.shape == down for m in moe.w2))
 
 
 class LayerTable:
@@ -189,6 +199,9 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
     n, dev = tab.n, tab.device
     if not (x.device == dev and x.dtype is torch.float32 and x.is_contiguous() and x.shape == (B * T, tab.C)):
         raise RuntimeError(f"forward: expected a contiguous f32 residual stream ({B * T}, {tab.C}) on {dev} (this path has no CPU fallback)")
+    for name, t in (("embedding table", table), ("final norm", final_norm and final_norm[0])):
+        if t is not None and (t.device != dev or t.shape[-1] != tab.C):
+            raise RuntimeError(f"forward: the {name} ({t.device}, {tuple(t.shape)}) does not belong to {tab.C} channels on {dev}")
     step = ids is not None and T == 1         # a model's single-token step
     if h_in is not None:
         # the tail of a single-token step leaves a new membrane where it cannot update the one it was given

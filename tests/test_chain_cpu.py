@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from jarvis_b200 import chain
+from jarvis_b200 import chain, modules as jm
 
 CPU = torch.device("cpu")
 
@@ -32,3 +32,20 @@ def test_states_are_updated_in_place_layer_by_layer():
     assert got[0] is a and got[2] is b and got[1].shape == got[3].shape == (3, 8) and got[1].data_ptr() != got[3].data_ptr()
     assert all(g is not a and g is not b for g in chain._results(2, [a, b], False, (3, 8), CPU))
     assert all(g is t for g, t in zip(chain._results(2, [a, b], True, (3, 8), CPU), (a, b)))
+
+
+def test_a_table_is_made_for_weights_of_one_size():
+    """The native call knows no weight's size: a block with one that differs takes the kernel-by-kernel path, which checks."""
+    def block():
+        return jm.JarvisBlock(128, 2)
+
+    def fits(b):
+        return chain._fits(b, b.attn, 128, 256, 4)
+    assert fits(block())
+    narrow, wide, odd, short, few = block(), block(), block(), block(), block()
+    narrow.moe.w2[1] = jm.TernaryLinear(128, 128)
+    wide.moe.w1[3] = jm.TernaryLinear(128, 512)
+    odd.attn.k_proj = jm.TernaryLinear(256, 128)
+    short.norm2.weight = torch.nn.Parameter(torch.ones(64))
+    few.moe.w2 = few.moe.w2[:3]
+    assert not any(map(fits, (narrow, wide, odd, short, few)))

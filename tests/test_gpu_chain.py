@@ -204,3 +204,18 @@ def test_carried_state_that_does_not_fit_is_refused(T):
     with pytest.raises(RuntimeError):
         model.blocks[0].forward_rows(torch.zeros(3 * T + 1, 128, device="cuda"), 3, T)
     assert _lib.device_status() == 0
+
+
+def test_weights_left_on_the_host_are_refused():
+    model = _model(1)
+    idx = torch.zeros((2, 3), dtype=torch.int64, device="cuda")
+    model(idx)
+    for name in ("tok_emb", "final_norm"):
+        getattr(model, name).cpu()
+        with pytest.raises(RuntimeError):
+            model(idx)
+        getattr(model, name).cuda()
+    model.blocks[0].moe.w2 = torch.nn.ModuleList(jm.ternary_init_(jm.TernaryLinear(384, 128)).cuda() for _ in range(4))
+    with pytest.raises(RuntimeError):
+        model(idx)
+    assert _lib.device_status() == 0
