@@ -378,9 +378,11 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
   // More than 512 rows: the CTA-pair kernel (24 layers of 700 / 2048 / 16384 tokens 2.54 / 3.32 / 14.0 ms against 2.63 / 3.68 /
   // 15.7 here).  Dense weights: from 65 rows on, since the tiles of 64 tokens that a small call is cut into here read all of them
   // once each (lm_head, 128 rows 25.7 against 36.7 us, 256 27.5 against 62, 512 46.8 against 113; 64 rows 24.1 against 22.8).
-  // What is left to this one are small calls, in-features that are no multiple of 256, the q/k RoPE epilogue
-  // and callers that ask for a token tile.
-  if (bn_override == 0 && K % 256 == 0 && M > (w_layout == 2 ? 64 : 512) && !rope) return launch_pair_gemm(p, x_bf16, sms, stream);
+  // What is left to this one are small calls, in-features that are no multiple of 256, the q/k RoPE epilogue, callers that ask
+  // for a token tile, and outputs on 16-byte boundaries: the pair kernel stores 32 bytes at a time (a residual it adds to by
+  // reductions of 16).
+  const bool out_ok = epilogue == JB200_EPI_RESID_F32 || (reinterpret_cast<uintptr_t>(out) & 31u) == 0;
+  if (bn_override == 0 && K % 256 == 0 && M > (w_layout == 2 ? 64 : 512) && !rope && out_ok) return launch_pair_gemm(p, x_bf16, sms, stream);
 
   CUtensorMap tmap;
   const cuuint64_t gdim[2] = {cuuint64_t(K), cuuint64_t(M)};

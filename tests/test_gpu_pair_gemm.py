@@ -61,3 +61,32 @@ def test_dense_weights_are_exact(M, N, K):
     assert torch.equal(ops.dense_linear(x, w, out_dtype=torch.float32), want)
     assert torch.equal(ops.dense_linear(x, w), want.bfloat16())
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 128, 256), (513, 384, 256), (767, 1024, 1024)])
+def test_outputs_that_start_on_a_16_byte_boundary(M, N, K):
+    """The entry points take them; the CTA-pair kernel's stores need 32 bytes."""
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randint(-3, 4, (M, K), generator=gen, device="cuda").bfloat16()
+    w, packed = _weights(1, N, K, gen, True)
+    alpha = torch.tensor([0.25], device="cuda")
+    want = 0.25 * (x.float() @ w[0].t())
+    dense = 0.25 * w[0].bfloat16()
+
+    def out(dtype):
+        t = torch.zeros(M * N + 32, dtype=dtype, device="cuda")
+        at = 16 // t.element_size() if t.data_ptr() % 32 == 0 else 0
+        t = t[at:at + M * N].view(M, N)
+        assert t.data_ptr() % 32 == 16
+        return t
+    offs = torch.tensor([0, M], dtype=torch.int32, device="cuda")
+    f32, bf16 = torch.float32, torch.bfloat16
+    assert torch.equal(ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_F32, out=out(f32), prepared=True), want)
+    assert torch.equal(ops.ternary_linear(x, packed[0], alpha, out=out(bf16), prepared=True), want.bfloat16())
+    assert torch.equal(ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_RESID_F32, out=out(f32), prepared=True), want)
+    assert torch.equal(ops.ternary_linear_grouped(x, packed, alpha, offs, out=out(bf16), prepared=True), want.bfloat16())
+    assert torch.equal(ops.dense_linear(x, dense, out_dtype=f32, out=out(f32)), want)
+    assert torch.equal(ops.dense_linear(x, dense, out=out(bf16)), want.bfloat16())
+    gelu = ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_GELU_BF16, out=out(bf16), prepared=True)
+    assert torch.equal(gelu, ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_GELU_BF16, prepared=True))
+    assert _lib.device_status() == 0
