@@ -319,7 +319,8 @@ typedef struct jb200_layer {
 } jb200_layer;
 
 /* One call of jb200_forward_layers.  Pointer arrays live on the HOST and hold one device pointer per layer; an array
- * or an entry may be NULL (no state in / not wanted out).  s_out[l] may be s_in[l], h_out[l] may be h_in[l]. */
+ * or an entry may be NULL (no state in / not wanted out).  s_out[l] may be s_in[l], h_out[l] may be h_in[l].  Device pointers
+ * are 16-byte aligned unless a line says otherwise; an argument error leaves everything as it was. */
 typedef struct jb200_forward {
   int B, T, C, H, E, hidden;     /* top-2 experts; C % 128 == 0, C <= 1024, C == 64 H */
   const int64_t* ids;            /* [B*T] token ids, or NULL: x already holds the residual stream */
@@ -333,8 +334,8 @@ typedef struct jb200_forward {
   int pos0_scalar;
   const float* const* s_in;      /* f32 [B][H][64][64] */
   float* const* s_out;
-  const float* const* h_in;      /* f32 [B][C] */
-  float* const* h_out;           /* required */
+  const float* const* h_in;      /* f32 [B][C], 8-byte aligned */
+  float* const* h_out;           /* required, 8-byte aligned */
   void* accumulators;            /* n_layers * jb200_accumulator_bytes, 8-byte aligned: cleared and used by the call */
   float* scalars;                /* f32 [n_layers][3]: l_balance, act_mean, act_var of every layer */
   float* reflect;                /* f32 [n_layers]: lam * ((mu - act_mean)^2 + relu(act_var - tau)); or NULL */

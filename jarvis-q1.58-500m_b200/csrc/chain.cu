@@ -96,6 +96,25 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   JB_REQUIRE(f->x && f->cos_tab && f->sin_tab && f->h_out && f->accumulators && f->scalars && f->routing && f->workspace,
              "forward_layers: null pointer");
   JB_REQUIRE((f->w_final == nullptr) == (f->hidden_out == nullptr), "forward_layers: w_final and hidden_out come together");
+  JB_REQUIRE(!f->ids || (f->table && f->vocab > 0), "forward_layers: ids without an embedding table");
+  // Everything is looked at before the first launch: an error leaves x and the states as they were.
+  const uintptr_t a8 = 7u, a256 = 255u;
+  JB_REQUIRE(aligned16(f->x) && aligned16(f->cos_tab) && aligned16(f->sin_tab) && aligned16(f->routing) && aligned16(f->table) &&
+                 aligned16(f->w_final) && aligned16(f->hidden_out) && (reinterpret_cast<uintptr_t>(f->accumulators) & a8) == 0 &&
+                 (reinterpret_cast<uintptr_t>(f->workspace) & a256) == 0,
+             "forward_layers: pointers must be 16-byte aligned (accumulators 8, workspace 256)");
+  for (int l = 0; l < n_layers; ++l) {
+    const jb200_layer& p = layers[l];
+    JB_REQUIRE(p.w_norm1 && p.w_norm2 && p.w_router && p.gamma && p.var_scale && p.w_qkv && p.a_qkv && p.w_out && p.a_out &&
+                   p.w1 && p.a1 && p.w2 && p.a2 && f->h_out[l],
+               "forward_layers: a pointer of layer %d is missing", l);
+    JB_REQUIRE(aligned16(p.w_norm1) && aligned16(p.w_norm2) && aligned16(p.w_router) && aligned16(p.w_qkv) &&
+                   aligned16(p.w_out) && aligned16(p.w1) && aligned16(p.w2),
+               "forward_layers: weights must be 16-byte aligned (layer %d)", l);
+    const uintptr_t hs = reinterpret_cast<uintptr_t>(f->h_out[l]) | reinterpret_cast<uintptr_t>(f->h_in ? f->h_in[l] : nullptr);
+    JB_REQUIRE((hs & a8) == 0 && aligned16(f->s_in ? f->s_in[l] : nullptr) && aligned16(f->s_out ? f->s_out[l] : nullptr),
+               "forward_layers: attention states must be 16-byte aligned, membranes 8 (layer %d)", l);
+  }
   const int N = B * T;
   const Workspace ws(B, T, C, H, E, hidden);
   const Routing rl(N, E);
@@ -141,7 +160,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     float* s_out = f->s_out ? f->s_out[l] : nullptr;
     const float* h_in = f->h_in ? f->h_in[l] : nullptr;
     float* h_out = f->h_out[l];
-    JB_REQUIRE(h_out != nullptr, "forward_layers: h_out of layer %d missing", l);
+    const bool h16 = aligned16(h_in) && aligned16(h_out);      // the fused tails read 16 bytes at a time, the scan 8
     double* acc = reinterpret_cast<double*>(acc0 + l * acc_stride);            // sum, sum of squares, P_e
     int32_t* hist = reinterpret_cast<int32_t*>(acc + 2 + E);                   // top-1 counts
     int32_t* ticket = hist + E;
@@ -206,13 +225,13 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     void* xn_next = last ? f->hidden_out : static_cast<void*>(xn);
     const LsfStats stats = {acc, acc + 2, hist, E, N, (long long)N * C, p.balance_alpha, scalars,
                             p.mu, p.reflect_lam, p.reflect_tau, (f->reflect && p.mu) ? f->reflect + l : nullptr};
-    if (N <= tail_max_tokens(C, T)) {
+    if (h16 && N <= tail_max_tokens(C, T)) {
       JB_TRY(launch_tail(y, gates, scatter, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
                          w_next ? xn_next : nullptr, B, T, C, st));
       continue;
     }
     JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st, true));
-    if (T == 1) {
+    if (h16 && T == 1) {
       JB_TRY(launch_lsf_step_norm(out, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
                                   w_next ? xn_next : nullptr, B, C, st, true));
     } else {

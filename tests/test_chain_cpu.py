@@ -1,8 +1,10 @@
 """Host side of the native forward call (chain.py) without a GPU: what it refuses before anything is launched."""
+import ctypes as C
+
 import pytest
 import torch
 
-from jarvis_b200 import chain, modules as jm
+from jarvis_b200 import _lib, chain, modules as jm
 
 CPU = torch.device("cpu")
 
@@ -49,3 +51,39 @@ def test_a_table_is_made_for_weights_of_one_size():
     short.norm2.weight = torch.nn.Parameter(torch.ones(64))
     few.moe.w2 = few.moe.w2[:3]
     assert not any(map(fits, (narrow, wide, odd, short, few)))
+
+
+def _call(**over):
+    """An argument block with made-up addresses: for calls that end before anything is launched."""
+    lib, n = _lib.load(), 2
+    layers = (_lib.Layer * n)()
+    for d in layers:
+        for i, (name, kind) in enumerate(_lib.Layer._fields_):
+            if kind is C.c_void_p:
+                setattr(d, name, 0x10000 + 0x1000 * i)
+    f = _lib.Forward()
+    f.B, f.T, f.C, f.H, f.E, f.hidden = 2, 1, 128, 2, 4, 256
+    for i, name in enumerate(("x", "cos_tab", "sin_tab", "accumulators", "scalars", "routing", "workspace")):
+        setattr(f, name, 0x100000 + 0x1000 * i)
+    states = {k: (C.c_void_p * n)(*(0x200000 + 0x1000 * i for i in range(n))) for k in ("h_in", "h_out", "s_in", "s_out")}
+    for k, v in states.items():
+        setattr(f, k, C.addressof(v))
+    for k, v in over.items():
+        if k in states:
+            states[k][1] = v
+        elif hasattr(layers[1], k):
+            setattr(layers[1], k, v)
+        else:
+            setattr(f, k, v)
+    return lib.jb200_forward_layers(layers, n, C.byref(f), None), _lib.last_error()
+
+
+@pytest.mark.parametrize("over,text", [
+    (dict(x=0x100004), "16-byte aligned"), (dict(workspace=0x100080), "workspace 256"), (dict(routing=0x100008), "16-byte aligned"),
+    (dict(accumulators=0x100004), "accumulators 8"), (dict(w_router=0x10004), "layer 1"), (dict(w_norm2=0x10008), "layer 1"),
+    (dict(w1=0x10008), "layer 1"), (dict(w2=None), "layer 1 is missing"), (dict(h_out=None), "layer 1 is missing"),
+    (dict(h_in=0x200004), "membranes 8"), (dict(h_out=0x20000C), "membranes 8"), (dict(s_in=0x200008), "attention states"),
+    (dict(s_out=0x200004), "attention states"), (dict(ids=0x300000), "embedding table")])
+def test_forward_arguments_are_checked_before_the_first_launch(over, text):
+    rc, message = _call(**over)
+    assert rc == _lib.ERR_ARG and text in message

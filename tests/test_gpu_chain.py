@@ -219,3 +219,20 @@ def test_weights_left_on_the_host_are_refused():
     with pytest.raises(RuntimeError):
         model(idx)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T", [(3, 1), (130, 1), (2, 2), (2, 9), (1, 64), (1, 200), (2, 300)])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_membranes_on_an_8_byte_boundary(B, T, inplace):
+    """The LSF scan takes them; the fused tails, which read 16 bytes at a time, leave them to it.  Same bits."""
+    torch.manual_seed(3)
+    blk = jm.ternary_init_(jm.JarvisBlock(256, 4, max_seq_len=512)).cuda().eval()
+    gen = torch.Generator(device="cuda").manual_seed(B * 1000 + T)
+    x, h = torch.randn(B * T, 256, generator=gen, device="cuda"), torch.randn(B, 256, generator=gen, device="cuda")
+    odd = torch.empty(B * 256 + 2, device="cuda")[2:].view(B, 256).copy_(h)
+    assert odd.data_ptr() % 16 == 8
+    xa, xb, aligned = x.clone(), x.clone(), h.clone()
+    ha = blk.forward_rows(xa, B, T, aligned, inplace_state=inplace)[0]
+    hb = blk.forward_rows(xb, B, T, odd, inplace_state=inplace)[0]
+    assert torch.equal(xa, xb) and torch.equal(ha, hb) and (hb is odd) == inplace
+    assert _lib.device_status() == 0
