@@ -73,7 +73,7 @@ struct AttnParams {
   float* handoff;          // [n_split][64][64] f32
   int* ctrl;               // [1 + n_split], zeroed before the launch
   unsigned int* status;
-  int settled;             // single-token step: state and positions were complete before the kernel ahead of this one started
+  int settled;             // decays (single-token step: state and positions too) were complete before the kernel ahead of this one started
 };
 
 __device__ __forceinline__ uint32_t swz(int row, int chunk16) {  // byte offset inside a swizzled [rows][128 B] tile
@@ -413,9 +413,10 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tmem_alloc(smem_u32(&sm->tmem_base), PIPE_TMEM_COLS);
     tmem_relinquish();
   }
-  // The decay tables come from a weight, so they too are made while the kernel before this one runs, unless the head is not
-  // known before the ticket is.
-  if (p.n_split > 0) {
+  // `settled`: the decay tables too are made while the kernel before this one runs, unless the head is not known before the
+  // ticket is.
+  const bool tables_first = p.settled && p.n_split == 0;
+  if (!tables_first) {
     pdl_wait();
     pdl_trigger();
   }
@@ -451,7 +452,7 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_after_sync();
   const uint32_t tm = sm->tmem_base;
   volatile uint32_t* abort_flag = &sm->abort_flag;
-  if (p.n_split == 0) {
+  if (tables_first) {
     pdl_wait();
     pdl_trigger();
   }
@@ -1200,6 +1201,7 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   p.seg_state = reinterpret_cast<float*>(scratch);
   if (scratch) pick_segments(B, T, H, sms, &p.seg_chunks, &p.nseg);   // without scratch: one segment per sequence
   JB_REQUIRE(p.nseg <= 65535, "attn_scan: too many segments");
+  p.settled = settled || p.nseg > 1;      // the pass over the segments waited for whatever made gamma
   JB_REQUIRE(!scratch || aligned16(scratch), "attn_scan: scratch pointer must be 16-byte aligned");
   p.n_pieces = o ? p.nseg - 1 : p.nseg;
   p.n_split = 0; p.split_chunk = 0; p.handoff = nullptr; p.ctrl = nullptr;

@@ -196,7 +196,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, ticket, counts, offs,
                                 scatter, gather, gate_idx, st));
     } else {
-      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st));
+      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true));
       JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
     }
     if (N <= ALL_ROWS_TOKENS) {
@@ -238,7 +238,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       void* lsf_scratch = (h_in && h_in == h_out) || ws.lsf == ws.meta ? nullptr : w + ws.lsf;
       JB_TRY(launch_lsf_scan(out, 1, nullptr, nullptr, nullptr, p.var_scale, p.alpha_min, p.alpha_max, h_in, x, nullptr, 0,
                              h_out, 0, lsf_scratch, B, T, C, st, &stats));
-      if (w_next) JB_TRY(launch_rmsnorm(x, 0, w_next, eps_next, xn_next, 1, N, C, st));
+      if (w_next) JB_TRY(launch_rmsnorm(x, 0, w_next, eps_next, xn_next, 1, N, C, st, true));
     }
   }
   return JB200_OK;

@@ -40,8 +40,8 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* p, const fl
 // One warp per row; the row is kept in registers between the two passes when C <= 8*32*MAXV.
 template <typename TIn, typename TOut, int MAXV>
 __global__ void __launch_bounds__(ROW_THREADS) rmsnorm_kernel(const TIn* __restrict__ x, const float* __restrict__ w,
-                                                              float eps, TOut* __restrict__ y, int n_rows, int C) {
-  touch_floats(w, C);                      // a weight: not written by a kernel that may still be running
+                                                              float eps, TOut* __restrict__ y, int n_rows, int C, bool ahead) {
+  if (ahead) touch_floats(w, C);           // the weight was complete before the kernel ahead of this one started
   pdl_wait();
   pdl_trigger();
   const int row = blockIdx.x * (ROW_THREADS / 32) + (threadIdx.x >> 5);
@@ -91,14 +91,14 @@ __global__ void __launch_bounds__(ROW_THREADS) embedding_kernel(const int64_t* _
 }
 
 template <typename TIn, typename TOut>
-int launch_rmsnorm_t(const void* x, const float* w, float eps, void* y, int n_rows, int C, cudaStream_t stream) {
+int launch_rmsnorm_t(const void* x, const float* w, float eps, void* y, int n_rows, int C, bool ahead, cudaStream_t stream) {
   const int blocks = (n_rows + ROW_THREADS / 32 - 1) / (ROW_THREADS / 32);
   if (C <= 1024)
     launch_dep(rmsnorm_kernel<TIn, TOut, 4>, blocks, ROW_THREADS, 0, stream, reinterpret_cast<const TIn*>(x), w, eps,
-               reinterpret_cast<TOut*>(y), n_rows, C);
+               reinterpret_cast<TOut*>(y), n_rows, C, ahead);
   else
     launch_dep(rmsnorm_kernel<TIn, TOut, 16>, blocks, ROW_THREADS, 0, stream, reinterpret_cast<const TIn*>(x), w, eps,
-               reinterpret_cast<TOut*>(y), n_rows, C);
+               reinterpret_cast<TOut*>(y), n_rows, C, ahead);
   JB_LAUNCH_CHECK("rmsnorm_kernel");
   return JB200_OK;
 }
@@ -106,7 +106,7 @@ int launch_rmsnorm_t(const void* x, const float* w, float eps, void* y, int n_ro
 }  // namespace
 
 int launch_rmsnorm(const void* x, int x_dtype, const float* w, float eps, void* y, int y_dtype, int n_rows, int C,
-                   cudaStream_t stream) {
+                   cudaStream_t stream, bool ahead) {
   JB_REQUIRE(n_rows >= 0 && C > 0, "rmsnorm: bad shape (%d, %d)", n_rows, C);
   JB_REQUIRE(C % 8 == 0 && C <= 4096, "rmsnorm: row length (%d) must be a multiple of 8 and at most 4096", C);
   JB_REQUIRE((x_dtype == 0 || x_dtype == 1) && (y_dtype == 0 || y_dtype == 1), "rmsnorm: dtype must be 0 (f32) or 1 (bf16)");
@@ -114,10 +114,10 @@ int launch_rmsnorm(const void* x, int x_dtype, const float* w, float eps, void* 
   JB_REQUIRE(x && w && y, "rmsnorm: null pointer");
   JB_REQUIRE(aligned16(x) && aligned16(w) && aligned16(y), "rmsnorm: pointers must be 16-byte aligned");
   if (n_rows == 0) return JB200_OK;
-  if (x_dtype == 0 && y_dtype == 1) return launch_rmsnorm_t<float, __nv_bfloat16>(x, w, eps, y, n_rows, C, stream);
-  if (x_dtype == 0 && y_dtype == 0) return launch_rmsnorm_t<float, float>(x, w, eps, y, n_rows, C, stream);
-  if (x_dtype == 1 && y_dtype == 1) return launch_rmsnorm_t<__nv_bfloat16, __nv_bfloat16>(x, w, eps, y, n_rows, C, stream);
-  return launch_rmsnorm_t<__nv_bfloat16, float>(x, w, eps, y, n_rows, C, stream);
+  if (x_dtype == 0 && y_dtype == 1) return launch_rmsnorm_t<float, __nv_bfloat16>(x, w, eps, y, n_rows, C, ahead, stream);
+  if (x_dtype == 0 && y_dtype == 0) return launch_rmsnorm_t<float, float>(x, w, eps, y, n_rows, C, ahead, stream);
+  if (x_dtype == 1 && y_dtype == 1) return launch_rmsnorm_t<__nv_bfloat16, __nv_bfloat16>(x, w, eps, y, n_rows, C, ahead, stream);
+  return launch_rmsnorm_t<__nv_bfloat16, float>(x, w, eps, y, n_rows, C, ahead, stream);
 }
 
 int launch_embedding(const int64_t* idx, const float* table, int vocab, float* out, int n_rows, int C,

@@ -41,8 +41,10 @@ int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepa
 void decode16_host(uint32_t w, uint32_t* out8);
 void decode16_prepared_host(uint32_t w_canonical, uint32_t* out8);
 
+// ahead (here and below): the weights were complete before the kernel ahead of this one on the stream began, so they may be
+// fetched before it ends.  True within jb200_forward_layers; a caller of a single stage may have just written them.
 int launch_rmsnorm(const void* x, int x_dtype, const float* w, float eps, void* y, int y_dtype, int n_rows, int C,
-                   cudaStream_t stream);
+                   cudaStream_t stream, bool ahead = false);
 int launch_embedding(const int64_t* idx, const float* table, int vocab, float* out, int n_rows, int C,
                      cudaStream_t stream);
 
@@ -50,7 +52,7 @@ int launch_router_top2(const void* x_bf16, const float* w_router, int n_tokens, 
                        float* gates, float* probs_out, double* probs_sum, int* top1_hist, cudaStream_t stream);
 int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router,
                           int n_tokens, int C, int E, int64_t* topk_idx, float* gates, double* probs_sum,
-                          int* top1_hist, cudaStream_t stream);
+                          int* top1_hist, cudaStream_t stream, bool ahead = false);
 size_t moe_metadata_scratch_bytes(int n_tokens, int K, int E);
 int launch_moe_metadata(const int64_t* topk_idx, int n_tokens, int K, int E, int* expert_counts, int* expert_offsets,
                         int* scatter_map, int* gather_map, int* gate_idx_map, void* scratch, cudaStream_t stream);
@@ -88,7 +90,7 @@ int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* va
                          const float* h_in, float* h_out, float* x, const float* w_norm, float eps, void* xn_bf16, int B,
                          int C, cudaStream_t stream, bool ahead = false);
 
-// settled (T == 1): s_in and pos0 were complete before the kernel ahead of this one on the stream began.
+// settled: gamma and, at T == 1, s_in and pos0 were complete before the kernel ahead of this one on the stream began.
 int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, const float* gamma,
                      const float* cos_tab, const float* sin_tab, int n_pos, const int32_t* pos0, int pos0_scalar,
                      const float* s_in, void* o, int ld_o, float* s_out, void* scratch, int B, int T, int H,

@@ -89,17 +89,20 @@ __global__ void __launch_bounds__(ROUTER_THREADS, 2)
 rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_norm, float eps,
                       __nv_bfloat16* __restrict__ xn, const float* __restrict__ w_router, int n_tokens, int C,
                       int64_t* __restrict__ topk_idx, float* __restrict__ gates,
-                      double* __restrict__ probs_sum, int* __restrict__ top1_hist) {
+                      double* __restrict__ probs_sum, int* __restrict__ top1_hist, bool ahead) {
   extern __shared__ float w_s[];  // [E][C]
   __shared__ float p_acc[ROUTER_THREADS / 32][E];
   __shared__ int h_acc[E];
-  // weights are no kernel's output that could still be running (no kernel that lets its successor start early writes them)
-  for (int i = threadIdx.x; i < E * C; i += ROUTER_THREADS) w_s[(i / C) * C + router_w_index(i % C)] = __ldg(w_router + i);
+  auto stage = [&] {
+    for (int i = threadIdx.x; i < E * C; i += ROUTER_THREADS) w_s[(i / C) * C + router_w_index(i % C)] = __ldg(w_router + i);
+    touch_floats(w_norm, C);
+  };
   if (threadIdx.x < E) h_acc[threadIdx.x] = 0;
-  touch_floats(w_norm, C);
-  __syncthreads();
+  if (ahead) stage();
   pdl_wait();
   pdl_trigger();
+  if (!ahead) stage();
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float p_local[E];
 #pragma unroll
@@ -524,7 +527,7 @@ int launch_router_top2(const void* x_bf16, const float* w_router, int n_tokens, 
 
 int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router,
                           int n_tokens, int C, int E, int64_t* topk_idx, float* gates, double* probs_sum,
-                          int* top1_hist, cudaStream_t stream) {
+                          int* top1_hist, cudaStream_t stream, bool ahead) {
   JB_REQUIRE(n_tokens >= 0 && C > 0, "rmsnorm_router: bad shape");
   JB_REQUIRE(E == 4 || E == 8, "rmsnorm_router: num_experts (%d) must be 4 or 8", E);
   JB_REQUIRE(C % 8 == 0 && C <= 1024, "rmsnorm_router: d_model (%d) must be a multiple of 8 and at most 1024", C);
@@ -542,10 +545,10 @@ int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* 
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
   if (E == 4)
     launch_dep(rmsnorm_router_kernel<4>, blocks, ROUTER_THREADS, smem, stream, x, w_norm, eps, xn, w_router, n_tokens, C,
-               topk_idx, gates, probs_sum, top1_hist);
+               topk_idx, gates, probs_sum, top1_hist, ahead);
   else
     launch_dep(rmsnorm_router_kernel<8>, blocks, ROUTER_THREADS, smem, stream, x, w_norm, eps, xn, w_router, n_tokens, C,
-               topk_idx, gates, probs_sum, top1_hist);
+               topk_idx, gates, probs_sum, top1_hist, ahead);
   JB_LAUNCH_CHECK("rmsnorm_router_kernel");
   return JB200_OK;
 }

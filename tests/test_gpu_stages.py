@@ -644,3 +644,25 @@ def test_empty_inputs_are_accepted_everywhere():
     assert tuple(tok.shape) == (0, 1)
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
+
+
+def test_weights_written_by_the_kernel_right_before_a_call():
+    """A caller of a single stage may have just made its weights: nothing of them is read before that kernel has ended."""
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(64, 256, generator=gen, device="cuda")
+    qkv = torch.randn(200, 3 * 256, generator=gen, device="cuda").bfloat16()
+    cos, sin = rope_tabs(200)
+    w_norm, w_router, gamma = torch.ones(256, device="cuda"), torch.zeros(4, 256, device="cuda"), torch.full((4,), 0.5, device="cuda")
+    stages = [(w_norm, lambda: ops.rmsnorm(x, w_norm)), (w_router, lambda: ops.rmsnorm_router(x, w_norm, 1e-6, w_router)[2]),
+              (gamma, lambda: ops.attn_scan(qkv[:, :256], qkv[:, 256:512], qkv[:, 512:], gamma, cos, sin, 1, 200, 4)[0])]
+    new = [torch.rand(t.shape, generator=gen, device="cuda") * 0.5 + 0.4 for t, _ in stages]
+    for _ in range(20):
+        for t, stage in stages:
+            t.fill_(0.7)
+            stage()
+        got = []
+        for (t, stage), v in zip(stages, new):
+            t.copy_(v)
+            got.append(stage())
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, stage()) for a, (_, stage) in zip(got, stages))
