@@ -137,7 +137,7 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, uint32_t (&
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(alpha * __uint_as_float(v[j]));
   if (p.epilogue == JB200_EPI_RESID_F32) {
-    // grouped calls (their tiles end inside a matrix, where a tile reduction would not be clipped)
+    // calls with segments (their tiles end inside the matrix, where a tile reduction would not be clipped)
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
@@ -480,7 +480,7 @@ int launch_pair_gemm(const GemmParams& p, const void* x_bf16, int sms, cudaStrea
   const long tiles = (long((p.M + 2 * BM - 1) / (2 * BM)) + (p.G - 1)) * ((p.N + BN - 1) / BN) * 4;   // at most, with cut tiles
   const dim3 grid(2 * unsigned(tiles < pairs ? tiles : pairs));
   CUtensorMap tmap_out = tmap;
-  if (p.epilogue == JB200_EPI_RESID_F32 && p.G == 1) {
+  if (p.epilogue == JB200_EPI_RESID_F32 && !p.seg_offsets) {
     const cuuint64_t odim[2] = {cuuint64_t(p.N), cuuint64_t(p.M)};
     const cuuint64_t ostride[1] = {cuuint64_t(p.N) * 4};
     const cuuint32_t obox[2] = {32, 32};

@@ -400,11 +400,11 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
     if (rc != JB200_OK) return rc;
   }
 
-  // Residual epilogue of a single matrix: the tile is added to the f32 stream by TMA reductions (needs 16-byte
-  // aligned rows); grouped calls and odd strides keep the read-modify-write from registers.
+  // Residual epilogue of a single matrix over all rows: the tile is added to the f32 stream by TMA reductions (needs 16-byte
+  // aligned rows), which clip at the matrix; calls with segments, one alone too, keep the read-modify-write from registers.
   CUtensorMap tmap_out = tmap;
   p.resid_stage_smem = 0;
-  if (epilogue == JB200_EPI_RESID_F32 && G == 1 && N % 4 == 0 && aligned16(out)) {
+  if (epilogue == JB200_EPI_RESID_F32 && !seg_offsets && N % 4 == 0 && aligned16(out)) {
     const cuuint64_t odim[2] = {cuuint64_t(N), cuuint64_t(M)};
     const cuuint64_t ostride[1] = {cuuint64_t(N) * 4};
     const cuuint32_t obox[2] = {32, 32};

@@ -90,3 +90,18 @@ def test_outputs_that_start_on_a_16_byte_boundary(M, N, K):
     gelu = ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_GELU_BF16, out=out(bf16), prepared=True)
     assert torch.equal(gelu, ops.ternary_linear(x, packed[0], alpha, epilogue=ops.EPI_GELU_BF16, prepared=True))
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("M,cut", [(40, (0, 33)), (300, (5, 170)), (513, (0, 500)), (1500, (3, 1025))])
+def test_residual_of_one_segment_leaves_the_rows_around_it(M, cut):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randint(-3, 4, (M, 256), generator=gen, device="cuda").bfloat16()
+    w, packed = _weights(1, 384, 256, gen, True)
+    offs = torch.tensor(cut, dtype=torch.int32, device="cuda")
+    base = torch.randint(-8, 9, (M, 384), generator=gen, device="cuda").float()
+    want = base.clone()
+    want[cut[0]:cut[1]] += 0.5 * (x[cut[0]:cut[1]].float() @ w[0].t())
+    got = ops.ternary_linear_grouped(x, packed, torch.tensor([0.5], device="cuda"), offs, epilogue=ops.EPI_RESID_F32, out=base.clone(),
+                                     prepared=True)
+    assert torch.equal(got, want)
+    assert _lib.device_status() == 0
