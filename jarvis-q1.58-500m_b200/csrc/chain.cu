@@ -2,6 +2,8 @@
 // of the model's loop around it (:498-516), issued from C++ over one caller-owned workspace.  A forward is a few
 // hundred launches; issued one by one from Python they cost ~15 us each (5 ms for 24 layers), more than the GPU
 // needs for anything below a few thousand tokens, issued here ~2 us each.
+#include <algorithm>
+
 #include "common.cuh"
 #include "launchers.h"
 
@@ -124,7 +126,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   uint16_t *y = reinterpret_cast<uint16_t*>(w + ws.y), *out = reinterpret_cast<uint16_t*>(w + ws.out);
   uint16_t* disp = qkv;
   float* x = f->x;
-  const bool small = N <= SMALL_TOKENS;
+  const bool small = N <= SMALL_TOKENS && small_gemm_fits(N, std::max(C, hidden));   // beyond, the tcgen05 form streams K
   const bool mid = !small && N <= MID_TOKENS;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;

@@ -32,6 +32,9 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
 int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
                       int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
                       int tokens, bool settled, cudaStream_t stream);
+// It keeps whole rows of codes and activations in shared memory: in-features it can take at so many tokens (about 7200 up to 8
+// tokens, 4800 from 9 on).
+bool small_gemm_fits(int tokens, int K);
 // The same product again, latency form on tcgen05 (mid_gemm.cu) with token tiles of bn rows, or of bn_max rows
 // where the segments need more tiles of bn than there are SMs.  Arguments as launch_small_gemm.
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,

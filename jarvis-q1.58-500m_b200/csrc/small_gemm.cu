@@ -179,7 +179,16 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) small_gemm_kernel(const SmallG
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+constexpr size_t SMEM_MAX = 226 * 1024;
+inline int tile_tokens(int tokens) { return tokens <= 8 ? 8 : 16; }
+// All codes of a CTA's out-features and the token rows of a tile, each row padded by 16 bytes.
+inline size_t smem_need(int tokens, int K) {
+  return size_t(16 * ROW_WARPS) * (K / 4 + 16) + size_t(tile_tokens(tokens)) * (size_t(K) * 2 + 16);
+}
+
 }  // namespace
+
+bool small_gemm_fits(int tokens, int K) { return smem_need(tokens, K) <= SMEM_MAX; }
 
 int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
                       int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
@@ -190,15 +199,14 @@ int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepare
   p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
   p.M = M; p.N = N; p.K = K; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
   p.settled = settled ? 1 : 0;
-  const int tok = tokens <= 8 ? 8 : 16;
-  const size_t smem = size_t(16 * ROW_WARPS) * (K / 4 + 16) + size_t(tok) * (size_t(K) * 2 + 16);
-  JB_REQUIRE(smem <= 226 * 1024, "small_gemm: in_features (%d) too large", K);
+  const size_t smem = smem_need(tokens, K);
+  JB_REQUIRE(smem <= SMEM_MAX, "small_gemm: in_features (%d) too large", K);
   const dim3 grid(N / (16 * ROW_WARPS), G);
-  if (tok == 8) {
-    JB_MAX_SMEM(small_gemm_kernel<1>, 226 * 1024);
+  if (tile_tokens(tokens) == 8) {
+    JB_MAX_SMEM(small_gemm_kernel<1>, SMEM_MAX);
     launch_dep(small_gemm_kernel<1>, grid, 32 * ROW_WARPS, smem, stream, p);
   } else {
-    JB_MAX_SMEM(small_gemm_kernel<2>, 226 * 1024);
+    JB_MAX_SMEM(small_gemm_kernel<2>, SMEM_MAX);
     launch_dep(small_gemm_kernel<2>, grid, 32 * ROW_WARPS, smem, stream, p);
   }
   JB_LAUNCH_CHECK("small_gemm_kernel");

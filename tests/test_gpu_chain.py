@@ -236,3 +236,20 @@ def test_membranes_on_an_8_byte_boundary(B, T, inplace):
     hb = blk.forward_rows(xb, B, T, odd, inplace_state=inplace)[0]
     assert torch.equal(xa, xb) and torch.equal(ha, hb) and (hb is odd) == inplace
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T,mult", [(1, 1, 8), (8, 1, 7), (9, 1, 5), (2, 8, 5), (16, 1, 4)])
+def test_few_tokens_with_wide_experts(B, T, mult):
+    """Expert widths whose rows do not fit the shared memory of the kernel for a few tokens (from 4800 at 9 to 16 tokens, 7200
+    below), and the widest that does."""
+    torch.manual_seed(5)
+    blk = jm.JarvisBlock(1024, 16, max_seq_len=64)
+    blk.moe = jm.SparseMoELayer(1024, hidden_mult=mult)
+    blk = jm.ternary_init_(blk).cuda().eval()
+    x = torch.randn(B * T, 1024, generator=torch.Generator(device="cuda").manual_seed(B), device="cuda")
+    xa, xb = x.clone(), x.clone()
+    blk.forward_rows(xa, B, T, scratch=(torch.zeros(6, dtype=torch.float64, device="cuda"),
+                                        torch.zeros(4, dtype=torch.int32, device="cuda"), torch.zeros(3, device="cuda")))
+    blk.forward_rows(xb, B, T)
+    assert torch.equal(xa, xb)
+    assert _lib.device_status() == 0
