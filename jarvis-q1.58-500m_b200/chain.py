@@ -19,9 +19,32 @@ _data_ptr = torch.Tensor.data_ptr
 _version = operator.attrgetter("_version")
 
 
+# Methods of the stock classes that the native call stands for: class -> {name: function}, filled where the classes are.
+_STOCK = {}
+
+
+def stands_for(cls, *names):
+    _STOCK[cls] = {n: cls.__dict__[n] for n in names}
+
+
+def _roles(block):
+    """(module, stock class) of the parts of a block whose methods the native call stands for."""
+    from .modules import AssociativeLinearAttention, JarvisBlock, RotaryEmbedding, SparseMoELayer, TernaryLinear
+    at = block.attn
+    return ((block, JarvisBlock), (at, AssociativeLinearAttention), (block.moe, SparseMoELayer),
+            (getattr(at, "out_proj", None), TernaryLinear), (getattr(at, "rotary", None), RotaryEmbedding))
+
+
+def _stock(block) -> bool:
+    """Nothing of the block overrides what the native call stands for (a subclass that leaves those methods alone may)."""
+    return all(getattr(type(m), n, None) is fn and n not in m.__dict__ for m, cls in _roles(block) for n, fn in _STOCK[cls].items())
+
+
 def supported(blocks) -> bool:
-    """Shapes jb200_forward_layers takes: all parameters on one CUDA device and of the sizes the first block gives, since the
+    """Blocks without overrides, of the shapes jb200_forward_layers takes: all parameters on one CUDA device and of the sizes the first block gives, since the
     native call knows nothing but their addresses."""
+    if not all(map(_stock, blocks)):
+        return False
     a = blocks[0].attn
     d_model = a.q_proj.weight.shape[1]
     hidden, E, dev = blocks[0].moe.w1[0].weight.shape[0], blocks[0].moe.num_experts, blocks[0].norm1.weight.device
@@ -91,8 +114,11 @@ class LayerTable:
             for lst in (moe.w1, moe.w2):
                 mods += [(lst, str(i)) for i in range(len(lst))]
                 slots += [(m, "weight") for m in lst]
-            self._flags.append((at.__dict__, moe.__dict__))
+            self._flags.append((at.__dict__, moe.__dict__, b.reflect.__dict__))
             self._consts.append((b.norm1, b.norm2, moe, b.liquid, b.reflect))
+        held = [(m, n, fn) for b in blocks for m, cls in _roles(b) for n, fn in _STOCK[cls].items()]
+        self._dicts, self._names = [m.__dict__ for m, _, _ in held], [n for _, n, _ in held]     # instance overrides
+        self._methods = list({(type(m), n): fn for m, n, fn in held}.items())                    # and those of the classes
         self._slots = [(m._parameters, n) for m, n in slots]
         if self.has_reflect:
             self._slots += [(b.reflect._buffers, "mu_t") for b in blocks]
@@ -113,14 +139,19 @@ class LayerTable:
             return (all(map(operator.is_, now, self._params)) and list(map(_data_ptr, now)) == self._ptrs and
                     list(map(_version, now)) == self._versions and
                     all(map(operator.is_, [d[n] for d, n in self._mods], self._mod_objs)) and
+                    not any(map(operator.contains, self._dicts, self._names)) and
+                    all(getattr(t, n) is fn for (t, n), fn in self._methods) and
                     self._read_consts() == self._const_vals)
         except (KeyError, AttributeError):
             return False
 
     def local(self) -> bool:
-        """No hook that needs the per-kernel path: statistics or experts shared with other GPUs, fused prologue, training."""
-        for at, moe in self._flags:
+        """Nothing that needs the per-kernel path: statistics or experts shared with other GPUs, fused prologue, training, a
+        penalty that has to be called (its running mean moves in training, hooks see its call)."""
+        for at, moe, refl in self._flags:
             if moe["stats_group"] is not None or moe["_ep"] is not None or at["fuse_prologue"] or moe["training"]:
+                return False
+            if self.has_reflect and (refl["training"] or refl["_forward_hooks"] or refl["_forward_pre_hooks"] or "forward" in refl):
                 return False
         return True
 
@@ -144,7 +175,10 @@ def table_of(owner, blocks) -> Optional[LayerTable]:
     if tab is None or tab.n != len(blocks) or any(r() is not b for r, b in zip(tab.blocks, blocks)) or not tab.current():
         if not supported(blocks):
             return None
-        tab = LayerTable(blocks)
+        try:
+            tab = LayerTable(blocks)
+        except KeyError:             # a weight that is no plain parameter (parametrised, pruned): read it anew on every call
+            return None
         owner.__dict__["_layer_table"] = tab
     return tab if tab.local() else None
 
@@ -255,7 +289,7 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
         res.hidden = torch.empty((B * T, tab.C), dtype=torch.bfloat16, device=dev)
         f.w_final, f.eps_final, f.hidden_out = final_norm[0].data_ptr(), final_norm[1], res.hidden.data_ptr()
     _lib.check(_lib.load().jb200_forward_layers(tab.array, n, C.byref(f), ops._stream()), "jb200_forward_layers")
-    for i, (_, moe) in enumerate(tab._flags):
+    for i, (_, moe, _) in enumerate(tab._flags):
         moe["_routing"] = RoutingSource((routing, i, B * T, tab.E))      # the views are built when somebody looks at them
     return res
 

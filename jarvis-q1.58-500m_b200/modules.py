@@ -525,6 +525,13 @@ class JarvisBlock(nn.Module):
         return rows.view(B, T, C).to(x.dtype), h_last.to(x.dtype), sc[0], l_reflect
 
 
+chain.stands_for(JarvisBlock, "forward_rows", "step_rows")
+chain.stands_for(AssociativeLinearAttention, "scan_rows", "qkv_packed")
+chain.stands_for(SparseMoELayer, "run_rows", "packed")
+chain.stands_for(TernaryLinear, "packed")
+chain.stands_for(RotaryEmbedding, "half_tables")
+
+
 class Jarvis(nn.Module):
     """jarvis_engine/jarvis_model.py:444-546.  forward(idx, targets=None, persist_state=False) ->
     (logits, loss); reset_state(); get_backend_status(); param_count().  Logits are bf16
@@ -709,7 +716,9 @@ class Jarvis(nn.Module):
             aux = self.last_aux if torch.is_tensor(self.last_aux) else torch.stack(self.last_aux)
             reflect = self._reflect
             if reflect is None:
-                reflect = torch.stack([b.reflect(sc[1], sc[2]) for b, sc in zip(self.blocks, self.last_aux)])
+                # whatever a penalty of the caller's own returns: a tensor or a number
+                reflect = torch.stack([torch.as_tensor(b.reflect(sc[1], sc[2]), dtype=torch.float32, device=logits.device).reshape(())
+                                       for b, sc in zip(self.blocks, self.last_aux)])
             loss = ops.cross_entropy(logits, targets, aux, reflect)
         if self.logits_dtype != torch.bfloat16:
             logits = logits.to(self.logits_dtype)

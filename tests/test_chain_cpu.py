@@ -87,3 +87,25 @@ def _call(**over):
 def test_forward_arguments_are_checked_before_the_first_launch(over, text):
     rc, message = _call(**over)
     assert rc == _lib.ERR_ARG and text in message
+
+
+def test_overridden_methods_need_the_kernel_by_kernel_path(monkeypatch):
+    class Attn(jm.AssociativeLinearAttention):
+        def scan_rows(self, *a, **k):
+            return super().scan_rows(*a, **k)
+
+    class Harmless(jm.JarvisBlock):
+        def extra_repr(self):
+            return "named"
+
+    def block(cls=jm.JarvisBlock):
+        return cls(128, 2)
+    assert chain._stock(block()) and chain._stock(block(Harmless))
+    sub, inst, other, packed = block(), block(), block(), block()
+    sub.attn = Attn(128, 2)
+    inst.moe.run_rows = lambda *a, **k: None
+    other.attn = torch.nn.Identity()
+    packed.attn.out_proj.packed = lambda: None
+    assert not any(map(chain._stock, (sub, inst, other, packed)))
+    monkeypatch.setattr(jm.JarvisBlock, "step_rows", lambda *a, **k: None)
+    assert not chain._stock(block())

@@ -253,3 +253,48 @@ def test_few_tokens_with_wide_experts(B, T, mult):
     blk.forward_rows(xb, B, T)
     assert torch.equal(xa, xb)
     assert _lib.device_status() == 0
+
+
+def test_overrides_and_penalties_of_the_callers_own_are_honoured():
+    model = _model(2)
+    idx = torch.arange(24, device="cuda").view(1, 24)
+    base, loss = model(idx, targets=idx)
+    calls = []
+    moe, plain = model.blocks[1].moe, model.blocks[1].moe.run_rows
+    moe.run_rows = lambda *a, **k: (calls.append(1), plain(*a, **k))[1]           # after the table was made
+    assert torch.equal(model(idx)[0], base) and calls == [1]
+    model.blocks[1](torch.randn(1, 4, 128, device="cuda"))
+    assert calls == [1, 1]
+    del moe.run_rows
+    assert torch.equal(model(idx)[0], base) and calls == [1, 1]
+    model.step(idx)
+
+    class Attn(jm.AssociativeLinearAttention):
+        def scan_rows(self, *a, **k):
+            o, s = super().scan_rows(*a, **k)
+            return torch.zeros_like(o), s
+    stock, ours = model.blocks[0].attn, Attn(128, 2, max_seq_len=640).cuda().eval()
+    ours.load_state_dict(stock.state_dict())
+    model.blocks[0].attn = ours
+    assert not torch.equal(model(idx)[0], base) and not torch.equal(model.step(idx)[0], base)
+    model.blocks[0].attn = stock
+    assert torch.equal(model(idx)[0], base)
+
+    # the penalty: its running mean moves in training, hooks see the call, and it may return a number
+    refl = model.blocks[0].reflect
+    refl.train()
+    before = refl.mu_t.clone()
+    model(idx, targets=idx)
+    assert not torch.equal(refl.mu_t, before)
+    refl.eval().mu_t = before
+    seen = []
+    hook = refl.register_forward_hook(lambda m, args, out: seen.append(float(out)))
+    got = model(idx, targets=idx)[1]
+    hook.remove()
+    assert len(seen) == 1 and abs(float(got) - float(loss)) < 1e-5 * abs(float(loss))
+    zero = torch.nn.Module()
+    zero.forward = lambda mean, var: 0.25
+    model.blocks[0].reflect = zero
+    shifted = model(idx, targets=idx)[1]
+    assert abs(float(shifted) - (float(loss) - seen[0] + 0.25)) < 1e-5 * abs(float(shifted))
+    assert _lib.device_status() == 0
