@@ -103,6 +103,10 @@ class LayerTable:
             d.eps1, d.eps2, d.balance_alpha = b.norm1.eps, b.norm2.eps, moe.balance_alpha
             d.alpha_min, d.alpha_max = lq.alpha_min, lq.alpha_max
 
+    def __reduce__(self):
+        """Addresses mean nothing in a copy: a copied, saved or sent module makes its own table."""
+        return type(None), ()
+
     def _watch(self, blocks):
         slots, mods, self._flags, self._consts = [], [], [], []
         for b in blocks:

@@ -1,5 +1,7 @@
 """Host side of the native forward call (chain.py) without a GPU: what it refuses before anything is launched."""
+import copy
 import ctypes as C
+import pickle
 
 import pytest
 import torch
@@ -109,3 +111,13 @@ def test_overridden_methods_need_the_kernel_by_kernel_path(monkeypatch):
     assert not any(map(chain._stock, (sub, inst, other, packed)))
     monkeypatch.setattr(jm.JarvisBlock, "step_rows", lambda *a, **k: None)
     assert not chain._stock(block())
+
+
+def test_modules_that_hold_a_table_can_be_copied_and_pickled():
+    block = jm.JarvisBlock(128, 2)
+    tab = object.__new__(chain.LayerTable)
+    tab.array = (_lib.Layer * 1)()                 # ctypes structures with pointers cannot be pickled
+    block.__dict__["_layer_table"] = tab
+    for twin in (copy.deepcopy(block), pickle.loads(pickle.dumps(block))):
+        assert twin.__dict__["_layer_table"] is None and block.__dict__["_layer_table"] is tab
+        assert torch.equal(twin.attn.q_proj.weight, block.attn.q_proj.weight)

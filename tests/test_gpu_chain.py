@@ -1,5 +1,8 @@
 """jb200_forward_layers (whole layers in one native call) against the kernel-by-kernel path, and the loss kernel against
 torch, at the sizes where they can go wrong."""
+import copy
+import io
+
 import pytest
 import torch
 
@@ -298,3 +301,18 @@ def test_overrides_and_penalties_of_the_callers_own_are_honoured():
     shifted = model(idx, targets=idx)[1]
     assert abs(float(shifted) - (float(loss) - seen[0] + 0.25)) < 1e-5 * abs(float(shifted))
     assert _lib.device_status() == 0
+
+
+def test_a_model_that_has_run_can_be_copied_and_saved():
+    model = _model(2)
+    idx = torch.arange(24, device="cuda").view(1, 24)
+    want = model(idx)[0].clone()
+    model.blocks[0](torch.randn(1, 4, 128, device="cuda"))
+    buf = io.BytesIO()
+    torch.save(model, buf)
+    buf.seek(0)
+    for twin in (copy.deepcopy(model), torch.load(buf, weights_only=False)):
+        assert torch.equal(twin(idx)[0], want)
+        with torch.no_grad():
+            twin.blocks[0].attn.gamma_raw.neg_()
+        assert not torch.equal(twin(idx)[0], want) and torch.equal(model(idx)[0], want)
