@@ -90,9 +90,8 @@ class LayerTable:
             qkv, a_qkv = at.qkv_packed()
             out, a_out = at.out_proj.packed()
             (w1, a1), (w2, a2) = moe.packed()
-            gamma = torch.sigmoid(at.gamma_raw.detach().float())
             tensors = dict(w_norm1=_f32(b.norm1.weight), w_norm2=_f32(b.norm2.weight), w_router=_f32(moe.router.weight),
-                           gamma=gamma, var_scale=_f32(lq.var_scale, scalar=True), w_qkv=qkv, a_qkv=a_qkv, w_out=out,
+                           gamma=at.decays(), var_scale=_f32(lq.var_scale, scalar=True), w_qkv=qkv, a_qkv=a_qkv, w_out=out,
                            a_out=a_out, w1=w1, a1=a1, w2=w2, a2=a2)
             if self.has_reflect:
                 tensors["mu"] = _f32(b.reflect.mu_t, scalar=True)

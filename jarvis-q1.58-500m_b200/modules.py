@@ -184,6 +184,13 @@ class AssociativeLinearAttention(nn.Module):
             self._qkv_rope = (canon, ops.prepare_weights(rows))
         return self._qkv_rope[1], self._qkv.alpha
 
+    def decays(self):
+        """sigmoid(gamma_raw), kept until gamma_raw changes: a captured graph holds its address."""
+        gkey = (self.gamma_raw.data_ptr(), self.gamma_raw._version)
+        if self._gamma is None or self._gamma[0] != gkey:
+            self._gamma = (gkey, torch.sigmoid(self.gamma_raw.detach().float()))
+        return self._gamma[1]
+
     def scan_rows(self, xn_rows, B, T, start_pos=0, h_prev=None, want_state=False, inplace_state=False, cp=None):
         """xn_rows: bf16 (B*T, C) normalised input -> (o bf16 (B*T, C), state or None).
         cp: a parallel.ContextParallel when this rank holds one T-token slice of longer sequences
@@ -206,10 +213,7 @@ class AssociativeLinearAttention(nn.Module):
             packed, alpha = self.qkv_packed_interleaved()
             qkv = ops.qkv_linear_rope(xn_rows, packed, alpha, cos, sin, T, 2 * C, start_pos=start_pos, alpha_rows=C,
                                       prepared=True)
-        gkey = (self.gamma_raw.data_ptr(), self.gamma_raw._version)
-        if self._gamma is None or self._gamma[0] != gkey:
-            self._gamma = (gkey, torch.sigmoid(self.gamma_raw.detach().float()))
-        gamma = self._gamma[1]
+        gamma = self.decays()
         if h_prev is not None:
             h_prev = h_prev.to(torch.float32).contiguous()
         if cp is not None:

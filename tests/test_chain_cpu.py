@@ -121,3 +121,15 @@ def test_modules_that_hold_a_table_can_be_copied_and_pickled():
     for twin in (copy.deepcopy(block), pickle.loads(pickle.dumps(block))):
         assert twin.__dict__["_layer_table"] is None and block.__dict__["_layer_table"] is tab
         assert torch.equal(twin.attn.q_proj.weight, block.attn.q_proj.weight)
+
+
+def test_decays_are_kept_while_their_parameter_is():
+    """Captured graphs hold their address, so an edit of another parameter must not make new ones."""
+    at = jm.AssociativeLinearAttention(128, 2)
+    first = at.decays()
+    with torch.no_grad():
+        at.q_proj.weight.add_(1.0)
+    assert at.decays() is first and torch.equal(first, torch.sigmoid(at.gamma_raw))
+    with torch.no_grad():
+        at.gamma_raw.add_(1.0)
+    assert at.decays() is not first and torch.equal(at.decays(), torch.sigmoid(at.gamma_raw))

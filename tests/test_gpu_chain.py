@@ -316,3 +316,25 @@ def test_a_model_that_has_run_can_be_copied_and_saved():
         with torch.no_grad():
             twin.blocks[0].attn.gamma_raw.neg_()
         assert not torch.equal(twin(idx)[0], want) and torch.equal(model(idx)[0], want)
+
+
+def test_a_captured_step_outlives_the_layer_table():
+    """An in-place edit of a norm weight makes the next eager call build a new table; what the graph reads must stay."""
+    model = _model(2)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    idx = torch.randint(0, 320, (5, 1), generator=gen, device="cuda")
+    state = {"h": [torch.randn(5, 128, generator=gen, device="cuda") for _ in range(2)],
+             "S": [torch.randn(5, 2, 64, 64, generator=gen, device="cuda") for _ in range(2)]}
+    pos = torch.full((5,), 3, dtype=torch.int32, device="cuda")
+    session = jm.DecodeSession(model, state, pos, 640).capture()
+    gammas = [b.attn.decays() for b in model.blocks]
+    with torch.no_grad():
+        model.blocks[0].norm1.weight.mul_(1.5)
+    model(idx)
+    assert all(b.attn.decays() is g for b, g in zip(model.blocks, gammas))
+    junk = [torch.full((2,), 0.01, device="cuda") for _ in range(2000)]             # freed blocks of that size would be taken
+    session.load_state(state, pos)
+    got = session.step(idx).clone()
+    want, _ = model.step(idx, pos, state, max_position=640)
+    assert torch.equal(got, want) and len(junk) == 2000
+    assert _lib.device_status() == 0
