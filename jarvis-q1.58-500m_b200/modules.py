@@ -777,6 +777,17 @@ class Jarvis(nn.Module):
         return n, f"{n/1e6:.1f}M parameters"
 
 
+def _made_from_parameters(model: "Jarvis"):
+    """What a forward reads that is made from parameters and replaced when they change or a longer prompt comes (packed
+    weights, decays, angle tables): a captured graph holds the addresses, so its owner keeps these alive."""
+    held = [model._lm_head_bf16, model.__dict__.get("_layer_table")]
+    for b in model.blocks:
+        at, moe = b.attn, b.moe
+        caches = (at._qkv, at.out_proj._cache, moe._p1, moe._p2)
+        held += [(c.packed, c.alpha) for c in caches] + [at._gamma, at._qkv_rope, at.rotary._half]
+    return held
+
+
 class DecodeSession:
     """One-token-per-step decode of B concurrent sequences with the whole step captured in a CUDA
     graph (the pattern of the reference's runtime/cuda_graph_runner.py:47-70, applied to the real
@@ -810,6 +821,7 @@ class DecodeSession:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self.logits = self._one()
+        self._held = _made_from_parameters(self.model)
         return self
 
     def load_state(self, state: dict, positions: torch.Tensor):
@@ -854,6 +866,7 @@ class PrefillSession:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph), torch.no_grad():
             self.logits = self.model(self.idx)[0]
+        self._held = _made_from_parameters(self.model)
         return self
 
     def __call__(self, idx: torch.Tensor) -> torch.Tensor:

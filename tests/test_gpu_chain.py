@@ -338,3 +338,19 @@ def test_a_captured_step_outlives_the_layer_table():
     want, _ = model.step(idx, pos, state, max_position=640)
     assert torch.equal(got, want) and len(junk) == 2000
     assert _lib.device_status() == 0
+
+
+def test_a_captured_step_outlives_its_angle_tables():
+    """A longer prompt makes the model's angle tables anew; the graph goes on with those it was captured with."""
+    torch.manual_seed(12)
+    model = jm.ternary_init_(jm.Jarvis(vocab_size=320, d_model=128, n_layers=2, n_heads=2, max_seq_len=256)).cuda().eval()
+    idx = torch.arange(5, device="cuda").view(5, 1)
+    state = {"h": [torch.ones(5, 128, device="cuda") for _ in range(2)],
+             "S": [torch.ones(5, 2, 64, 64, device="cuda") for _ in range(2)]}
+    pos = torch.full((5,), 200, dtype=torch.int32, device="cuda")
+    want, _ = model.step(idx, pos, state, max_position=250)
+    session = jm.DecodeSession(model, state, pos, 250).capture()
+    model(torch.zeros((1, 700), dtype=torch.int64, device="cuda"))
+    junk = [torch.full((256, 32), 9.0, device="cuda") for _ in range(50)]
+    session.load_state(state, pos)
+    assert torch.equal(session.step(idx), want) and len(junk) == 50
