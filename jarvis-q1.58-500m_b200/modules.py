@@ -781,10 +781,10 @@ def _made_from_parameters(model: "Jarvis"):
     """What a forward reads that is made from parameters and replaced when they change or a longer prompt comes (packed
     weights, decays, angle tables): a captured graph holds the addresses, so its owner keeps these alive."""
     held = [model._lm_head_bf16, model.__dict__.get("_layer_table")]
-    for b in model.blocks:
-        at, moe = b.attn, b.moe
-        caches = (at._qkv, at.out_proj._cache, moe._p1, moe._p2)
-        held += [(c.packed, c.alpha) for c in caches] + [at._gamma, at._qkv_rope, at.rotary._half]
+    held += [getattr(p, "_jb_f32", None) for p in model.parameters()]
+    for m in model.modules():
+        held += [(c.packed, c.alpha) for c in vars(m).values() if isinstance(c, _PackCache)]
+        held += [vars(m).get(name) for name in ("_gamma", "_qkv_rope", "_half")]
     return held
 
 

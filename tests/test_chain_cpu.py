@@ -133,3 +133,13 @@ def test_decays_are_kept_while_their_parameter_is():
     with torch.no_grad():
         at.gamma_raw.add_(1.0)
     assert at.decays() is not first and torch.equal(at.decays(), torch.sigmoid(at.gamma_raw))
+
+
+def test_what_a_captured_session_keeps():
+    model = jm.Jarvis(vocab_size=32, d_model=128, n_layers=1, n_heads=2)
+    at = model.blocks[0].attn
+    at._qkv.packed, at._qkv.alpha = torch.zeros(3), torch.ones(3)
+    made = [at.decays(), at._qkv.packed, at.rotary.half_tables(8, CPU)[0], jm._f32(model.final_norm.weight)]
+    model.blocks[0].moe = torch.nn.Identity()                       # a part of the caller's own
+    flat = [t for entry in jm._made_from_parameters(model) if isinstance(entry, tuple) for t in entry]
+    assert all(any(t is m for t in flat) for m in made)
