@@ -563,8 +563,13 @@ class Jarvis(nn.Module):
         self.logits_dtype = torch.bfloat16
         self.use_chain = True      # False: every kernel by its own ops call (to put something between them)
         self._lm_head_bf16 = None
-        self.last_aux = None
+        self._aux = None           # what last_aux shows: f32 (layers, 3), or a list of its rows
         self._reflect = None
+
+    @property
+    def last_aux(self):
+        """Per layer f32 [l_balance, act_mean, act_var] of the most recent forward, a list; None before the first."""
+        return list(self._aux.unbind(0)) if torch.is_tensor(self._aux) else self._aux
 
     def get_backend_status(self):
         n = len(self.blocks)
@@ -634,7 +639,7 @@ class Jarvis(nn.Module):
             r = self._chain_rows(tab, idx, start_pos, h_in, s_in, self.carry_attention_state)
             self._h_states = r.h
             self._attn_states = r.S if r.S is not None else [None] * tab.n
-            self.last_aux, self._reflect = r.scalars, r.reflect
+            self._aux, self._reflect = r.scalars, r.reflect
             return r.hidden
         self._reflect = None
         x = ops.embedding(idx.contiguous(), _f32(self.tok_emb.weight)).view(B * T, self.d_model)
@@ -660,7 +665,7 @@ class Jarvis(nn.Module):
             aux.append(sc)
         self._h_states = new_h
         self._attn_states = new_s
-        self.last_aux = aux
+        self._aux = aux
         return ops.rmsnorm(x, _f32(self.final_norm.weight), self.final_norm.eps)
 
     @torch.no_grad()
@@ -717,12 +722,12 @@ class Jarvis(nn.Module):
         logits = self._logits(self.hidden_rows(idx, persist_state), B, T)
         loss = None
         if targets is not None:
-            aux = self.last_aux if torch.is_tensor(self.last_aux) else torch.stack(self.last_aux)
+            aux = self._aux if torch.is_tensor(self._aux) else torch.stack(self._aux)
             reflect = self._reflect
             if reflect is None:
                 # whatever a penalty of the caller's own returns: a tensor or a number
                 reflect = torch.stack([torch.as_tensor(b.reflect(sc[1], sc[2]), dtype=torch.float32, device=logits.device).reshape(())
-                                       for b, sc in zip(self.blocks, self.last_aux)])
+                                       for b, sc in zip(self.blocks, self._aux)])
             loss = ops.cross_entropy(logits, targets, aux, reflect)
         if self.logits_dtype != torch.bfloat16:
             logits = logits.to(self.logits_dtype)

@@ -143,3 +143,12 @@ def test_what_a_captured_session_keeps():
     model.blocks[0].moe = torch.nn.Identity()                       # a part of the caller's own
     flat = [t for entry in jm._made_from_parameters(model) if isinstance(entry, tuple) for t in entry]
     assert all(any(t is m for t in flat) for m in made)
+
+
+def test_last_aux_is_a_list_on_either_path():
+    model = jm.Jarvis(vocab_size=32, d_model=128, n_layers=2, n_heads=2)
+    assert model.last_aux is None
+    rows = torch.arange(6.0).view(2, 3)
+    for aux in (rows, list(rows.unbind(0))):
+        model._aux = aux
+        assert isinstance(model.last_aux, list) and torch.equal(torch.stack(model.last_aux), rows)

@@ -44,7 +44,7 @@ def test_chain_matches_the_kernel_by_kernel_path(B, T):
         first, loss = model(idx, targets=idx, persist_state=True)
         second, _ = model(idx, persist_state=True)
         assert model._token_pos == 2 * T
-        aux = model.last_aux if torch.is_tensor(model.last_aux) else torch.stack(model.last_aux)
+        aux = torch.stack(model.last_aux)                          # a list on either path
         got[chain] = [logits.float(), into.float(), torch.stack(new["h"]), torch.stack(new["S"]), torch.stack(same["S"]),
                       first.float(), second.float(), loss.reshape(1), aux]
         idxs = [b.moe.last_routing[0].clone() for b in model.blocks]
