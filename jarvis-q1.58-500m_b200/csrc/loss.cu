@@ -27,7 +27,12 @@ ce_rows_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int V, const in
 #pragma unroll
     for (int j = 1; j < 8; ++j) mx = fmaxf(mx, v[j]);
     if (mx > m) { s *= exp2f((m - mx) * LOG2E); m = mx; }
-    if (m == -INFINITY) return;
+    if (m == -INFINITY) {                  // no finite value yet: fmaxf passes NaN over, and -inf counts as nothing
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (v[j] != v[j]) s = v[j];
+      return;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) s += exp2f((v[j] - m) * LOG2E);
   };
@@ -47,7 +52,7 @@ ce_rows_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int V, const in
   }
   auto merge = [&](float m2, float s2) {
     const float mx = fmaxf(m, m2);
-    if (mx != -INFINITY) s = s * exp2f((m - mx) * LOG2E) + s2 * exp2f((m2 - mx) * LOG2E);
+    s = mx == -INFINITY ? s + s2 : s * exp2f((m - mx) * LOG2E) + s2 * exp2f((m2 - mx) * LOG2E);
     m = mx;
   };
 #pragma unroll

@@ -89,6 +89,28 @@ def test_cross_entropy_matches_torch(rows, V, ld):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("V", [1, 7, 4101, 50257])
+def test_cross_entropy_of_values_that_are_not_finite(V):
+    """A NaN anywhere makes the loss NaN, also where a thread has met nothing else yet; -inf logits count as nothing."""
+    gen = torch.Generator(device="cuda").manual_seed(V)
+    clean = (torch.randn(1, 2, (V + 7) // 8 * 8, generator=gen, device="cuda") * 5).bfloat16()
+    y = torch.full((1, 2), V - 1, device="cuda", dtype=torch.int64)
+    none = torch.zeros(1, 3, device="cuda"), torch.zeros(1, device="cuda")
+    nan, inf = float("nan"), float("inf")
+    for value, spans in ((nan, [(0, 1), (0, 8), (max(V - 8, 0), V), (0, V)]), (-inf, [(0, 8), (0, max(V - 1, 0)), (0, V)]), (inf, [(0, 1)])):
+        for a, b in spans:
+            buf = clean.clone()
+            buf[0, 1, a:min(b, V)] = value
+            logits = buf[..., :V]
+            got, want = float(ops.cross_entropy(logits, y, *none)), float(torch.nn.functional.cross_entropy(logits[0].double(), y[0]))
+            assert (got != got) == (want != want), (value, a, b, got, want)
+            assert want != want or got == want or abs(got - want) < 2e-5 * max(1.0, abs(want))
+    mixed = clean.clone()
+    mixed[0, 0, :8] = -inf
+    mixed[0, 0, 0] = nan                                            # NaN among -inf in one thread's first values
+    assert bool(torch.isnan(ops.cross_entropy(mixed[..., :V], y, *none)))
+
+
 @pytest.mark.parametrize("B,T", [(1, 1), (4, 1), (5, 1), (8, 1), (9, 1), (16, 1), (17, 1), (33, 1), (64, 1), (65, 1), (128, 1),
                                  (129, 1), (1, 2), (3, 3), (1, 16), (2, 20), (1, 64), (1, 65), (2, 64), (1, 128), (1, 129),
                                  (1, 256), (1, 257), (257, 1), (1, 640), (1, 960), (1, 961)])
