@@ -188,8 +188,6 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
 // ---------------------------------------------------------------------------------------------
 // dispatch metadata: stable counting sort of M = N*K assignments by expert id
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ int clamp_expert(long long e, int E) { return e < 0 ? 0 : (e >= E ? E - 1 : int(e)); }
-
 __global__ void __launch_bounds__(META_CHUNK)
 meta_hist_kernel(const int64_t* __restrict__ flat_idx, int M, int E, int* __restrict__ chunk_counts) {
   pdl_wait();

@@ -6,6 +6,9 @@ namespace jb {
 
 #if defined(__CUDACC__)
 
+// The expert an assignment is sorted under: router_finish leaves -1 where logits are NaN.
+__device__ __forceinline__ int clamp_expert(long long e, int E) { return e < 0 ? 0 : (e >= E ? E - 1 : int(e)); }
+
 // logits of one token (already warp-reduced, identical in every lane) -> softmax, top-2 with ties going
 // to the lower expert id, gates, and the per-warp accumulators of P and the top-1 histogram.
 template <int E>

@@ -376,3 +376,18 @@ def test_a_captured_step_outlives_its_angle_tables():
     junk = [torch.full((256, 32), 9.0, device="cuda") for _ in range(50)]
     session.load_state(state, pos)
     assert torch.equal(session.step(idx), want) and len(junk) == 50
+
+
+@pytest.mark.parametrize("N", [3, 64, 65, 200])
+def test_dispatch_maps_of_tokens_whose_router_is_nan(N):
+    """A token without finite logits has no second expert (-1); the maps still hold every assignment, as the general sort's do."""
+    torch.manual_seed(9)
+    blk = jm.ternary_init_(jm.JarvisBlock(256, 4, max_seq_len=256)).cuda().eval()
+    x = torch.randn(N, 256, device="cuda")
+    x[N // 2] = float("nan")
+    blk.forward_rows(x, 1, N)
+    idx, _, got = blk.moe.last_routing
+    assert int(idx.min()) == -1
+    for a, b in zip(got, ops.moe_metadata(idx.contiguous(), 4)):
+        assert torch.equal(a, b)
+    assert _lib.device_status() == 0
