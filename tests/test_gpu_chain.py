@@ -348,7 +348,7 @@ def test_a_captured_step_outlives_the_layer_table():
     state = {"h": [torch.randn(5, 128, generator=gen, device="cuda") for _ in range(2)],
              "S": [torch.randn(5, 2, 64, 64, generator=gen, device="cuda") for _ in range(2)]}
     pos = torch.full((5,), 3, dtype=torch.int32, device="cuda")
-    session = jm.DecodeSession(model, state, pos, 640).capture()
+    session = jm.DecodeSession(model, {k: [s.clone() for s in v] for k, v in state.items()}, pos, 640).capture()
     gammas = [b.attn.decays() for b in model.blocks]
     with torch.no_grad():
         model.blocks[0].norm1.weight.mul_(1.5)
@@ -371,7 +371,7 @@ def test_a_captured_step_outlives_its_angle_tables():
              "S": [torch.ones(5, 2, 64, 64, device="cuda") for _ in range(2)]}
     pos = torch.full((5,), 200, dtype=torch.int32, device="cuda")
     want, _ = model.step(idx, pos, state, max_position=250)
-    session = jm.DecodeSession(model, state, pos, 250).capture()
+    session = jm.DecodeSession(model, {k: [s.clone() for s in v] for k, v in state.items()}, pos, 250).capture()
     model(torch.zeros((1, 700), dtype=torch.int64, device="cuda"))
     junk = [torch.full((256, 32), 9.0, device="cuda") for _ in range(50)]
     session.load_state(state, pos)
