@@ -6,6 +6,7 @@ runs in C++ and Python pays for one call, a handful of allocations and the check
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import math
 import operator
 import weakref
@@ -120,8 +121,12 @@ class LayerTable:
             self._flags.append((at.__dict__, moe.__dict__, b.reflect.__dict__))
             self._consts.append((b.norm1, b.norm2, moe, b.liquid, b.reflect))
         held = [(m, n, fn) for b in blocks for m, cls in _roles(b) for n, fn in _STOCK[cls].items()]
-        self._dicts, self._names = [m.__dict__ for m, _, _ in held], [n for _, n, _ in held]     # instance overrides
-        self._methods = list({(type(m), n): fn for m, n, fn in held}.items())                    # and those of the classes
+        # instance overrides; not the blocks' own dictionaries, which may hold this table (`current` gets those to look at)
+        own = set(map(id, blocks))
+        self._dicts, self._names = zip(*((m.__dict__, n) for m, n, _ in held if id(m) not in own))
+        self._block_names = [n for m, n, _ in held if m is blocks[0]]
+        stock = {(type(m), n): fn for m, n, fn in held}                                           # and those of the classes
+        self._types, self._methods = list(zip(*stock)), list(stock.values())
         self._slots = [(m._parameters, n) for m, n in slots]
         if self.has_reflect:
             self._slots += [(b.reflect._buffers, "mu_t") for b in blocks]
@@ -136,14 +141,17 @@ class LayerTable:
         return [(a.eps, b.eps, m.balance_alpha, q.alpha_min, q.alpha_max, getattr(r, "lam", None), getattr(r, "tau_max", None))
                 for a, b, m, q, r in self._consts]
 
-    def current(self) -> bool:
+    def current(self, blocks) -> bool:
         try:
+            for n in self._block_names:
+                if any(map(operator.contains, map(vars, blocks), itertools.repeat(n))):
+                    return False
             now = [d[n] for d, n in self._slots]
             return (all(map(operator.is_, now, self._params)) and list(map(_data_ptr, now)) == self._ptrs and
                     list(map(_version, now)) == self._versions and
                     all(map(operator.is_, [d[n] for d, n in self._mods], self._mod_objs)) and
                     not any(map(operator.contains, self._dicts, self._names)) and
-                    all(getattr(t, n) is fn for (t, n), fn in self._methods) and
+                    list(map(getattr, *self._types)) == self._methods and
                     self._read_consts() == self._const_vals)
         except (KeyError, AttributeError):
             return False
@@ -175,7 +183,7 @@ class LayerTable:
 def table_of(owner, blocks) -> Optional[LayerTable]:
     """The (cached) table of `blocks`, kept on `owner`; None when they need the per-kernel path."""
     tab = owner.__dict__.get("_layer_table")
-    if tab is None or tab.n != len(blocks) or any(r() is not b for r, b in zip(tab.blocks, blocks)) or not tab.current():
+    if tab is None or tab.n != len(blocks) or any(r() is not b for r, b in zip(tab.blocks, blocks)) or not tab.current(blocks):
         if not supported(blocks):
             return None
         try:
@@ -193,12 +201,12 @@ def _carried(ts, n: int, shape, dev, what: str, exact: bool = True, must_alias=N
     ts = list(ts)
     if len(ts) < n:
         raise RuntimeError(f"forward: {what} has {len(ts)} entries for {n} layers")
-    numel, out = math.prod(shape), []
+    out = []
     for t in ts[:n]:
         if t is not None:
             if t.device != dev:
                 raise RuntimeError(f"forward: {what} on {t.device}, expected {dev} (this path has no CPU fallback)")
-            if t.shape != shape if exact else t.numel() != numel:
+            if t.shape != shape and (exact or t.numel() != math.prod(shape)):
                 raise RuntimeError(f"forward: {what} of shape {tuple(t.shape)}, expected {shape}")
             if t.dtype is not torch.float32 or not t.is_contiguous():
                 if must_alias is not None and must_alias(t):
@@ -236,9 +244,9 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
     n, dev = tab.n, tab.device
     if not (x.device == dev and x.dtype is torch.float32 and x.is_contiguous() and x.shape == (B * T, tab.C)):
         raise RuntimeError(f"forward: expected a contiguous f32 residual stream ({B * T}, {tab.C}) on {dev} (this path has no CPU fallback)")
-    for name, t in (("embedding table", table), ("final norm", final_norm and final_norm[0])):
+    for t in (table, final_norm[0]) if final_norm is not None else (table,):
         if t is not None and (t.device != dev or t.shape[-1] != tab.C):
-            raise RuntimeError(f"forward: the {name} ({t.device}, {tuple(t.shape)}) does not belong to {tab.C} channels on {dev}")
+            raise RuntimeError(f"forward: embedding table or final norm ({t.device}, {tuple(t.shape)}): expected {tab.C} channels on {dev}")
     step = ids is not None and T == 1         # a model's single-token step
     if h_in is not None:
         # the tail of a single-token step leaves a new membrane where it cannot update the one it was given

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
   int n_of = 0;                                  // lane e < E: assignments of expert e
   int ex[ROUNDS];
 #pragma unroll
-  for (int i = 0; i < ROUNDS; ++i) ex[i] = i * 32 + lane < M ? clamp_expert(__ldcg(ids + i * 32 + lane), E) : -1;
+  for (int i = 0; i < ROUNDS; ++i) ex[i] = i * 32 + lane < M ? max(int(__ldcg(ids + i * 32 + lane)), 0) : -1;   // -1 (NaN logits) goes to expert 0
 #pragma unroll
   for (int i = 0; i < ROUNDS; ++i) {
 #pragma unroll

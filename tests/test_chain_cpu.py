@@ -1,12 +1,15 @@
 """Host side of the native forward call (chain.py) without a GPU: what it refuses before anything is launched."""
 import copy
 import ctypes as C
+import gc
 import pickle
+import weakref
 
 import pytest
 import torch
+from torch.nn.utils import prune
 
-from jarvis_b200 import _lib, chain, modules as jm
+from jarvis_b200 import _lib, chain, modules as jm, ops
 
 CPU = torch.device("cpu")
 
@@ -152,3 +155,45 @@ def test_last_aux_is_a_list_on_either_path():
     for aux in (rows, list(rows.unbind(0))):
         model._aux = aux
         assert isinstance(model.last_aux, list) and torch.equal(torch.stack(model.last_aux), rows)
+
+
+@pytest.fixture
+def tables_on_cpu(monkeypatch):
+    """Layer tables without a GPU: the packing is made up, nothing is ever launched with them."""
+    monkeypatch.setattr(ops, "pack_ternary", lambda w, alpha=None: (torch.zeros(w.shape[0], w.shape[1] // 4, dtype=torch.uint8), torch.ones(1)))
+    monkeypatch.setattr(ops, "prepare_weights", lambda p: p.clone())
+    monkeypatch.setattr(chain, "supported", lambda blocks: all(map(chain._stock, blocks)))
+
+
+def test_a_dropped_block_goes_at_once(tables_on_cpu):
+    """Its own table must not keep it until the next collection: the memory of a replaced model is wanted right away."""
+    block = jm.JarvisBlock(128, 2).eval()
+    assert chain.table_of(block, [block]) is not None and block.__dict__["_layer_table"] is not None
+    gone = weakref.ref(block)
+    gc.disable()
+    try:
+        del block
+        assert gone() is None
+    finally:
+        gc.enable()
+
+
+def test_a_table_follows_overrides_and_replaced_parts(tables_on_cpu):
+    blocks = [jm.JarvisBlock(128, 2).eval() for _ in range(2)]
+    owner = torch.nn.Module()
+    tab = chain.table_of(owner, blocks)
+    assert chain.table_of(owner, blocks) is tab
+    for part, name in ((blocks[1], "forward_rows"), (blocks[0], "step_rows"), (blocks[1].attn, "scan_rows"), (blocks[0].moe, "packed"),
+                       (blocks[0].attn.rotary, "half_tables")):
+        setattr(part, name, lambda *a, **k: None)
+        assert chain.table_of(owner, blocks) is None
+        delattr(part, name)
+        assert chain.table_of(owner, blocks) is not None
+    with torch.no_grad():
+        blocks[0].norm1.weight.mul_(2.0)
+    assert chain.table_of(owner, blocks) is not tab
+    blocks[0].reflect.train()
+    assert chain.table_of(owner, blocks) is None
+    blocks[0].reflect.eval()
+    prune.identity(blocks[0].attn.q_proj, "weight")          # the weight is no parameter any more
+    assert chain.table_of(owner, blocks) is None
