@@ -169,11 +169,11 @@ def test_a_dropped_block_goes_at_once(tables_on_cpu):
     """Its own table must not keep it until the next collection: the memory of a replaced model is wanted right away."""
     block = jm.JarvisBlock(128, 2).eval()
     assert chain.table_of(block, [block]) is not None and block.__dict__["_layer_table"] is not None
-    gone = weakref.ref(block)
+    gone = [weakref.ref(t) for t in (block, block.attn, block.moe.w1[0].weight)]
     gc.disable()
     try:
         del block
-        assert gone() is None
+        assert all(ref() is None for ref in gone)
     finally:
         gc.enable()
 
