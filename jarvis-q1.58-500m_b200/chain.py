@@ -6,7 +6,6 @@ runs in C++ and Python pays for one call, a handful of allocations and the check
 from __future__ import annotations
 
 import ctypes as C
-import itertools
 import math
 import operator
 import weakref
@@ -127,12 +126,12 @@ class LayerTable:
         self._block_names = [n for m, n, _ in held if m is blocks[0]]
         stock = {(type(m), n): fn for m, n, fn in held}                                           # and those of the classes
         self._types, self._methods = list(zip(*stock)), list(stock.values())
-        self._slots = [(m._parameters, n) for m, n in slots]
+        slots = [(m._parameters, n) for m, n in slots]
         if self.has_reflect:
-            self._slots += [(b.reflect._buffers, "mu_t") for b in blocks]
-        self._mods = [(m._modules, n) for m, n in mods]
-        self._mod_objs = [d[n] for d, n in self._mods]
-        self._params = [d[n] for d, n in self._slots]
+            slots += [(b.reflect._buffers, "mu_t") for b in blocks]
+        self._slots, self._mods = list(zip(*slots)), list(zip(*((m._modules, n) for m, n in mods)))
+        self._mod_objs = list(map(operator.getitem, *self._mods))
+        self._params = list(map(operator.getitem, *self._slots))
         self._ptrs = list(map(_data_ptr, self._params))
         self._versions = list(map(_version, self._params))
         self._const_vals = self._read_consts()
@@ -143,14 +142,12 @@ class LayerTable:
 
     def current(self, blocks) -> bool:
         try:
-            for n in self._block_names:
-                if any(map(operator.contains, map(vars, blocks), itertools.repeat(n))):
-                    return False
-            now = [d[n] for d, n in self._slots]
+            now = list(map(operator.getitem, *self._slots))
             return (all(map(operator.is_, now, self._params)) and list(map(_data_ptr, now)) == self._ptrs and
                     list(map(_version, now)) == self._versions and
-                    all(map(operator.is_, [d[n] for d, n in self._mods], self._mod_objs)) and
+                    list(map(operator.getitem, *self._mods)) == self._mod_objs and      # modules compare by identity
                     not any(map(operator.contains, self._dicts, self._names)) and
+                    not any(n in b.__dict__ for n in self._block_names for b in blocks) and
                     list(map(getattr, *self._types)) == self._methods and
                     self._read_consts() == self._const_vals)
         except (KeyError, AttributeError):
@@ -223,9 +220,11 @@ def _pointers(n, ts):
 def _results(n, given, inplace, shape, dev):
     """Where the states after the call go, one tensor per layer: the given ones (in place), new ones where there are none."""
     kept = given if inplace and given is not None else [None] * n
-    missing = sum(t is None for t in kept)
+    missing = n if kept is not given else sum(t is None for t in kept)
     if not missing:
         return kept
+    if n == 1:
+        return [torch.empty(shape, dtype=torch.float32, device=dev)]
     new = iter(torch.empty((missing, *shape), dtype=torch.float32, device=dev).unbind(0))
     return [next(new) if t is None else t for t in kept]
 

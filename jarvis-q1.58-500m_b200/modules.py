@@ -522,11 +522,11 @@ class JarvisBlock(nn.Module):
         tab = chain.table_of(self, [self]) if x.is_cuda else None
         if tab is not None and tab.has_reflect:
             r = self._chain(tab, rows, B, T, h_prev, start_pos)
-            h_last, sc, l_reflect = r.h[0], r.scalars[0], r.reflect[0]
+            h_last, l_balance, l_reflect = r.h[0], r.scalars[0, 0], r.reflect[0]
         else:
             h_last, sc, _ = self.forward_rows(rows, B, T, h_prev, start_pos)
-            l_reflect = self.reflect(sc[1], sc[2])
-        return rows.view(B, T, C).to(x.dtype), h_last.to(x.dtype), sc[0], l_reflect
+            l_balance, l_reflect = sc[0], self.reflect(sc[1], sc[2])
+        return rows.view(B, T, C).to(x.dtype), h_last.to(x.dtype), l_balance, l_reflect
 
 
 chain.stands_for(JarvisBlock, "forward_rows", "step_rows")
