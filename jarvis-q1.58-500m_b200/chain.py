@@ -19,25 +19,25 @@ _data_ptr = torch.Tensor.data_ptr
 _version = operator.attrgetter("_version")
 
 
-# Methods of the stock classes that the native call stands for: class -> {name: function}, filled where the classes are.
+# Methods of the stock classes that the native call stands for, by the part a module plays in a block: {name: function}, filled
+# where the classes are.
 _STOCK = {}
 
 
-def stands_for(cls, *names):
-    _STOCK[cls] = {n: cls.__dict__[n] for n in names}
+def stands_for(part, cls, *names):
+    _STOCK[part] = {n: cls.__dict__[n] for n in names}
 
 
-def _roles(block):
-    """(module, stock class) of the parts of a block whose methods the native call stands for."""
-    from .modules import AssociativeLinearAttention, JarvisBlock, RotaryEmbedding, SparseMoELayer, TernaryLinear
+def _methods(block):
+    """(module, name, stock function) of every method of the block's parts that the native call stands for."""
     at = block.attn
-    return ((block, JarvisBlock), (at, AssociativeLinearAttention), (block.moe, SparseMoELayer),
-            (getattr(at, "out_proj", None), TernaryLinear), (getattr(at, "rotary", None), RotaryEmbedding))
+    parts = dict(block=block, attn=at, moe=block.moe, out_proj=getattr(at, "out_proj", None), rotary=getattr(at, "rotary", None))
+    return [(m, n, fn) for part, m in parts.items() for n, fn in _STOCK[part].items()]
 
 
 def _stock(block) -> bool:
     """Nothing of the block overrides what the native call stands for (a subclass that leaves those methods alone may)."""
-    return all(getattr(type(m), n, None) is fn and n not in m.__dict__ for m, cls in _roles(block) for n, fn in _STOCK[cls].items())
+    return all(getattr(type(m), n, None) is fn and n not in m.__dict__ for m, n, fn in _methods(block))
 
 
 def supported(blocks) -> bool:
@@ -119,7 +119,7 @@ class LayerTable:
                 slots += [(m, "weight") for m in lst]
             self._flags.append((at.__dict__, moe.__dict__, b.reflect.__dict__))
             self._consts.append((b.norm1, b.norm2, moe, b.liquid, b.reflect))
-        held = [(m, n, fn) for b in blocks for m, cls in _roles(b) for n, fn in _STOCK[cls].items()]
+        held = [h for b in blocks for h in _methods(b)]
         # instance overrides; not the blocks' own dictionaries, which may hold this table (`current` gets those to look at)
         own = set(map(id, blocks))
         self._dicts, self._names = zip(*((m.__dict__, n) for m, n, _ in held if id(m) not in own))

@@ -135,14 +135,14 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const int n_ft = n_out / 128;
     if (!seg) {                                // every group over all rows
       const int bn = mid_tile(M, G, n_ft, sms);
-      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn, true, st);
+      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn, st);
     }
     // Segments are known on the device alone: a tile for rows that are spread evenly, with an eighth to spare, and one for
     // whatever they are (M / bn_max tiles and one cut short in every other group).
     const int even = (M + G - 1) / G, bn = mid_tile(even + (even + 7) / 8, G, n_ft, sms);
     int bn_max = bn;
     while (bn_max < 256 && long(n_ft) * ((M + bn_max - 1) / bn_max + G - 1) > sms) bn_max += 16;
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn_max, true, st);
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn_max, st);
   };
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
@@ -176,7 +176,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
 
     // x += attn(norm1(x))
     if (small)
-      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, N, true, st));
+      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, N, st));
     else if (mid)
       JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv));
     else
@@ -187,7 +187,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     JB_TRY(launch_attn_scan(qkv, qkv + C, qkv + 2 * C, 3 * C, p.gamma, f->cos_tab, f->sin_tab, f->n_pos, f->pos0, f->pos0_scalar,
                             s_in, o, C, s_out, attn_scratch, B, T, H, 64, 0, st, true));
     if (small)
-      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, N, true, st));
+      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, N, st));
     else if (mid)
       JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x));
     else
@@ -204,7 +204,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (N <= ALL_ROWS_TOKENS) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
       if (small)
-        JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, N, true, st));
+        JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, N, st));
       else
         JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid));
     } else {
@@ -215,7 +215,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
         JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true));
     }
     if (small)
-      JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, N, true, st));
+      JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, N, st));
     else if (mid)
       JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y));
     else

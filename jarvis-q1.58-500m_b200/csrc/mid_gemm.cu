@@ -38,7 +38,6 @@ struct MidParams {
   void* out;
   int M, N, K, G, n_ft, alpha_rows, epilogue;
   int bn[3], chunks[3];        // token tiles and their rings: the first whose items are one wave, else the last
-  int settled;                 // weights and segments were complete before the kernel ahead of this one started
   uint32_t tmem_cols;
   unsigned int* status;
 };
@@ -104,10 +103,8 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     tmem_alloc(smem_u32(&ctl.tmem_base), p.tmem_cols);
     tmem_relinquish();
   }
-  if (!p.settled) {
-    pdl_wait();
-    pdl_trigger();
-  }
+  // Weights and segments were complete before the kernel ahead of this one started: every role waits for the grid dependency
+  // where it first needs the rows.
   if (warp == 1) {
     static_assert(MAX_GROUPS <= 32, "one lane per group");
     int beg = 0, end = 0;
@@ -155,10 +152,8 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     // ---------------- TMA producer ----------------
     Items it;
     bool more = it.first(p, ctl, bn);
-    if (p.settled) {
-      pdl_wait();
-      pdl_trigger();
-    }
+    pdl_wait();
+    pdl_trigger();
     int s = 0;
     uint32_t ph = 1u;
     bool ok = true;
@@ -179,10 +174,8 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     // ---------------- MMA issuer ----------------
     Items it;
     bool more = it.first(p, ctl, bn);
-    if (p.settled) {
-      pdl_wait();
-      pdl_trigger();
-    }
+    pdl_wait();
+    pdl_trigger();
     const uint32_t idesc = umma_idesc_bf16(BM, bn);
     const uint64_t adesc0 = umma_desc_k_sw128(base), bdesc0 = umma_desc_k_sw128(b_base);
     uint64_t ad = adesc0, bd = bdesc0;
@@ -272,10 +265,8 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
       decode_to(fresh, true);
     }
     __syncwarp();
-    if (p.settled) {
-      pdl_wait();
-      pdl_trigger();
-    }
+    pdl_wait();
+    pdl_trigger();
     const int q4 = warp & 3;                         // TMEM lane quadrant of this warp
     uint32_t tile = 0u;
     for (; ok && more; more = it.next(p, ctl, bn), ++tile) {
@@ -304,18 +295,14 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
         uint32_t v[32];
         tmem_ld_32x32(tmem + (uint32_t(q4 * 32) << 16) + uint32_t(c0), v);
         tmem_ld_wait();
-        if (p.epilogue == JB200_EPI_RESID_F32 || p.epilogue == JB200_EPI_F32) {
+        if (p.epilogue == JB200_EPI_RESID_F32) {
           // lane = feature: a warp instruction covers 128 bytes of one token's row
           float* o = reinterpret_cast<float*>(p.out) + f0 + lane;
-          const bool resid = p.epilogue == JB200_EPI_RESID_F32;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int rj = __shfl_sync(0xffffffffu, row, j);
             const float val = alpha * __uint_as_float(v[j]);
-            if (rj >= 0) {
-              if (resid) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + size_t(rj) * p.N), "f"(val) : "memory");
-              else o[size_t(rj) * p.N] = val;
-            }
+            if (rj >= 0) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + size_t(rj) * p.N), "f"(val) : "memory");
           }
         } else {
           const bool gelu = p.epilogue == JB200_EPI_GELU_BF16;
@@ -348,8 +335,9 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
 }  // namespace
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int bn_max, bool settled,
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int bn_max,
                     cudaStream_t stream) {
+  JB_REQUIRE(epilogue == JB200_EPI_BF16 || epilogue == JB200_EPI_GELU_BF16 || epilogue == JB200_EPI_RESID_F32, "mid_gemm: epilogue %d", epilogue);
   JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn % 16 == 0 &&
                  bn_max >= bn && bn_max <= 256 && bn_max % 16 == 0 &&
                  G >= 1 && G <= MAX_GROUPS,
@@ -357,7 +345,6 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   MidParams p;
   p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
   p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / BM; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
-  p.settled = settled ? 1 : 0;
   p.tmem_cols = bn_max <= 32 ? 32u : bn_max <= 64 ? 64u : bn_max <= 128 ? 128u : 256u;
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;

@@ -39,7 +39,6 @@ struct SmallGemmParams {
   const int32_t* scatter;      //   idx[2n + k] is the group ([M][2] both); or null: group g takes rows [seg[g], seg[g + 1])
   void* out;                   // [M][N], or [2M][N] with idx
   int M, N, K, alpha_rows, epilogue;
-  int settled;                 // weights and segments were written before the kernel ahead of this one started
 };
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -57,8 +56,6 @@ __device__ __forceinline__ void store_pair(const SmallGemmParams& p, size_t o, f
   if (p.epilogue == JB200_EPI_RESID_F32) {
     // one addition per element, done by the memory system: nothing waits for the old value
     asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(reinterpret_cast<float*>(p.out) + o), "f"(a), "f"(b) : "memory");
-  } else if (p.epilogue == JB200_EPI_F32) {
-    *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.out) + o) = make_float2(a, b);
   } else {
     if (p.epilogue == JB200_EPI_GELU_BF16) { a = gelu_erf(a); b = gelu_erf(b); }
     *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + o) = pack_bf16x2(a, b);
@@ -116,20 +113,17 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) small_gemm_kernel(const SmallG
     }
     cp_async_commit();
   };
+  // weights and segments were complete before the kernel ahead of this one started
   int beg = 0, end = p.M;
-  auto early = [&]() {
-    copy_rows(wgt, p.w + (size_t(grp) * p.N + f0) * size_t(p.K / 4), ROWS, p.K / 64);
-    if (p.seg) {
-      beg = min(max(__ldg(p.seg + grp), 0), p.M);
-      end = min(max(__ldg(p.seg + grp + 1), 0), p.M);
-    }
-  };
-  if (p.settled) early();
+  copy_rows(wgt, p.w + (size_t(grp) * p.N + f0) * size_t(p.K / 4), ROWS, p.K / 64);
+  if (p.seg) {
+    beg = min(max(__ldg(p.seg + grp), 0), p.M);
+    end = min(max(__ldg(p.seg + grp + 1), 0), p.M);
+  }
   const float alpha = 0.5f * __ldg(p.alpha + size_t(grp) * (p.N / p.alpha_rows) + f0 / p.alpha_rows);   // codes decode to +-2
   __syncwarp();
   pdl_wait();
   pdl_trigger();
-  if (!p.settled) early();
 
 #pragma unroll 1
   for (int tb = beg; tb < end; tb += TOK) {
@@ -192,13 +186,13 @@ bool small_gemm_fits(int tokens, int K) { return smem_need(tokens, K) <= SMEM_MA
 
 int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
                       int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
-                      int tokens, bool settled, cudaStream_t stream) {
+                      int tokens, cudaStream_t stream) {
+  JB_REQUIRE(epilogue == JB200_EPI_BF16 || epilogue == JB200_EPI_GELU_BF16 || epilogue == JB200_EPI_RESID_F32, "small_gemm: epilogue %d", epilogue);
   JB_REQUIRE(M >= 1 && K % 128 == 0 && N % 64 == 0 && alpha_rows % 64 == 0, "small_gemm: bad shape (M=%d, N=%d, K=%d)", M, N, K);
   SmallGemmParams p;
   p.x = reinterpret_cast<const __nv_bfloat16*>(x_bf16);
   p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
   p.M = M; p.N = N; p.K = K; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
-  p.settled = settled ? 1 : 0;
   const size_t smem = smem_need(tokens, K);
   JB_REQUIRE(smem <= SMEM_MAX, "small_gemm: in_features (%d) too large", K);
   const dim3 grid(N / (16 * ROW_WARPS), G);

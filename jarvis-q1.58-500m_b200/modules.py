@@ -529,11 +529,11 @@ class JarvisBlock(nn.Module):
         return rows.view(B, T, C).to(x.dtype), h_last.to(x.dtype), l_balance, l_reflect
 
 
-chain.stands_for(JarvisBlock, "forward_rows", "step_rows")
-chain.stands_for(AssociativeLinearAttention, "scan_rows", "qkv_packed")
-chain.stands_for(SparseMoELayer, "run_rows", "packed")
-chain.stands_for(TernaryLinear, "packed")
-chain.stands_for(RotaryEmbedding, "half_tables")
+chain.stands_for("block", JarvisBlock, "forward_rows", "step_rows")
+chain.stands_for("attn", AssociativeLinearAttention, "scan_rows", "qkv_packed")
+chain.stands_for("moe", SparseMoELayer, "run_rows", "packed")
+chain.stands_for("out_proj", TernaryLinear, "packed")
+chain.stands_for("rotary", RotaryEmbedding, "half_tables")
 
 
 class Jarvis(nn.Module):
