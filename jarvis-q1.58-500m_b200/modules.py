@@ -282,6 +282,10 @@ class SparseMoELayer(nn.Module):
         r = self._routing
         return chain.routing_views(r) if isinstance(r, chain.RoutingSource) else r
 
+    @last_routing.setter
+    def last_routing(self, value):
+        self._routing = value
+
     def packed(self):
         return (self._p1.get([m.weight for m in self.w1], stack=True),
                 self._p2.get([m.weight for m in self.w2], stack=True))
@@ -570,6 +574,10 @@ class Jarvis(nn.Module):
     def last_aux(self):
         """Per layer f32 [l_balance, act_mean, act_var] of the most recent forward, a list; None before the first."""
         return list(self._aux.unbind(0)) if torch.is_tensor(self._aux) else self._aux
+
+    @last_aux.setter
+    def last_aux(self, value):
+        self._aux, self._reflect = value, None
 
     def get_backend_status(self):
         n = len(self.blocks)

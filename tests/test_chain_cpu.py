@@ -155,6 +155,9 @@ def test_last_aux_is_a_list_on_either_path():
     for aux in (rows, list(rows.unbind(0))):
         model._aux = aux
         assert isinstance(model.last_aux, list) and torch.equal(torch.stack(model.last_aux), rows)
+    model._reflect = rows
+    model.last_aux = model.blocks[0].moe.last_routing = ["of an override"]
+    assert model._aux == model.blocks[0].moe._routing == ["of an override"] and model._reflect is None
 
 
 @pytest.fixture
