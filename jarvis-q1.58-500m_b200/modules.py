@@ -634,6 +634,7 @@ class Jarvis(nn.Module):
         if self.training:
             raise RuntimeError("Jarvis (sm_100a): inference only; call .eval() first")
         B, T = idx.shape
+        idx = ops._need(idx.contiguous(), torch.int64, "embedding.idx")      # before anything is carried on
         start_pos = self._token_pos if persist_state else 0
         if persist_state:
             self._token_pos += T * (self._cp.world if self._cp is not None else 1)
@@ -650,7 +651,7 @@ class Jarvis(nn.Module):
             self._aux, self._reflect = r.scalars, r.reflect
             return r.hidden
         self._reflect = None
-        x = ops.embedding(idx.contiguous(), _f32(self.tok_emb.weight)).view(B * T, self.d_model)
+        x = ops.embedding(idx, _f32(self.tok_emb.weight)).view(B * T, self.d_model)
         h_prevs = self._h_states if persist_state else [None] * len(self.blocks)
         s_prevs = self._attn_states if (persist_state and self.carry_attention_state) else [None] * len(self.blocks)
         new_h, new_s, aux = [], [], []

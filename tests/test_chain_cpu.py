@@ -200,3 +200,10 @@ def test_a_table_follows_overrides_and_replaced_parts(tables_on_cpu):
     blocks[0].reflect.eval()
     prune.identity(blocks[0].attn.q_proj, "weight")          # the weight is no parameter any more
     assert chain.table_of(owner, blocks) is None
+
+
+def test_refused_tokens_do_not_move_the_position():
+    model = jm.Jarvis(vocab_size=32, d_model=128, n_layers=1, n_heads=2).eval()
+    with pytest.raises(RuntimeError):
+        model(torch.zeros((1, 5), dtype=torch.int64), persist_state=True)
+    assert model._token_pos == 0
