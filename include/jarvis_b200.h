@@ -63,8 +63,9 @@ int jb200_abi_version(void);
 long long jb200_kernel_launches(int reset);
 
 /* The kernels of the forward chain are launched with programmatic stream serialisation: each starts while the
- * kernel before it on the stream is still running and waits (griddepcontrol.wait) before it touches memory, so
- * launch latency and set-up overlap the predecessor; captured into CUDA graphs as programmatic edges.  No
+ * kernel before it on the stream is still running and waits (griddepcontrol.wait) before it touches memory that that
+ * kernel may have written (a call of one stage: any memory), so launch latency and set-up overlap the predecessor;
+ * captured into CUDA graphs as programmatic edges.  No
  * reference counterpart (the reference launches each kernel fully serialised).  enable = 0 launches them fully
  * serialised again; returns the previous setting.  The environment variable JB200_DEPENDENT_LAUNCH=0 sets the
  * initial state. */

@@ -694,7 +694,8 @@ int launch_tma(LsfChainParams p, cudaStream_t stream) {
   if constexpr (!FUSED) {
     // Well beyond three CTAs of 64 channels per SM some SMs hold a fourth and finish last (32 x 2048: 3.46 on average); tiles
     // of half the channels even that out, though they cost 3 % of themselves (30 x 2048 54.7 against 58.9 us, 32 x 2048 57.4
-    // against 60.5, but 28 x 2048 52.5 against 51.0 and 24 x 2048 47.2 against 44.5).
+    // against 60.5, but 28 x 2048 52.5 against 51.0 and 24 x 2048 47.2 against 44.5).  Measured at T = 2048; the
+    // same unevenness beyond four CTAs per SM is left alone.
     if (ctas > 3L * sms + sms / 8 && ctas <= 4L * sms) {
       using Half = LsfTma<false, LSF_CH / 2>;
       if ((rc = make_lsf_map(&tm_m, p.m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.B, p.T, p.D, LSF_CH / 2)) != JB200_OK) return rc;

@@ -856,10 +856,10 @@ class DecodeSession:
 
 class PrefillSession:
     """A fixed-shape stateless forward (B x T token ids -> logits) captured in a CUDA graph, the pattern of the
-    reference's runtime/cuda_graph_runner.py:47-70 applied to the whole model.  The forward is ~340 launches; from
-    Python each costs tens of microseconds of host time, which is hidden behind a 14 ms step at B=8 x T=2048 but
-    not when the step is short (a small batch, or one batch split over several GPUs: the per-layer statistics
-    all-reduce of set_batch_split is captured with it).  A replay is one launch; programmatic dependent launch
+    reference's runtime/cuda_graph_runner.py:47-70 applied to the whole model.  A forward is 170 to 340 launches; in
+    one native call they cost about 0.6 ms of host time, kernel by kernel (one batch split over several GPUs: the per-layer
+    statistics all-reduce of set_batch_split is captured with it) several ms, which a step of 13 ms hides and a short one
+    does not.  A replay is one launch; programmatic dependent launch
     edges are kept inside the graph."""
 
     def __init__(self, model: "Jarvis", batch: int, seq_len: int, device=None):

@@ -13,8 +13,8 @@ from ._lib import ATTN_QK_PREPARED, EPI_BF16, EPI_F32, EPI_GELU_BF16, EPI_RESID_
 
 
 # torch's current stream of the current device as a raw cudaStream_t.  torch.cuda.current_stream() builds a Stream
-# object behind several Python-level checks (~7 us); with ~340 launches per forward that is a third of the
-# host time of a forward, so the two C accessors are used directly when this torch has them.
+# object behind several Python-level checks (~7 us), once per call: a third of the host time of a forward issued
+# kernel by kernel, so the two C accessors are used directly when this torch has them.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
