@@ -41,8 +41,8 @@ def _stock(block) -> bool:
 
 
 def supported(blocks) -> bool:
-    """Blocks without overrides, of the shapes jb200_forward_layers takes: all parameters on one CUDA device and of the sizes the first block gives, since the
-    native call knows nothing but their addresses."""
+    """Blocks without overrides, of the shapes jb200_forward_layers takes: all parameters on one CUDA device and of the sizes the
+    first block gives, since the native call knows nothing but their addresses."""
     if not all(map(_stock, blocks)):
         return False
     a = blocks[0].attn
