@@ -48,6 +48,7 @@ extern "C" {
 #define JB200_STATUS_ATTN_HANDOFF 0x23u   /* the second part of a cut sequence never saw the first part's state */
 #define JB200_STATUS_LSF_LOAD 0x31u
 #define JB200_STATUS_PEER_BARRIER 0x41u
+#define JB200_STATUS_STEP_CLUSTER 0x51u
 #define JB200_STATUS_SELFTEST_WAIT 0x7Fu
 
 /* ---- library ----------------------------------------------------------------------- */
@@ -359,6 +360,16 @@ size_t jb200_forward_workspace_bytes(int B, int T, int C, int H, int E, int hidd
  * points with their results; one call instead of ~14 per layer keeps the host (about 15 us per call from Python) out
  * of the way of short forwards. */
 int jb200_forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, void* stream);
+
+/* The same with every layer's weights at hand in a second layout as well (step_weights: HOST array of n_layers device pointers,
+ * entries and the array may be NULL): single-token steps of few sequences then run all layers in one launch, with the same results.
+ * jb200_step_weight_bytes: of one layer, 0 where the sizes have no such form; jb200_prepare_step_weights lays a layer out
+ * (again whenever one of its tensors changes), 16-byte aligned. */
+size_t jb200_step_weight_bytes(int C, int H, int E, int hidden);
+int jb200_step_max_sequences(void);      /* most sequences of such a step on the current device, 0: none */
+int jb200_prepare_step_weights(const jb200_layer* layer, int C, int H, int E, int hidden, void* out, void* stream);
+int jb200_forward_layers_prepared(const jb200_layer* layers, int n_layers, const jb200_forward* f, const void* const* step_weights,
+                                  void* stream);
 
 /* Training / evaluation loss from bf16 logits (jarvis_engine/jarvis_model.py:536-545): cross entropy averaged over the
  * rows whose target is not -100, plus the sums of n_aux entries of aux_a (stride stride_a) and aux_b (stride 1), e.g.

@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import operator
+import threading
 import weakref
 from typing import List, Optional
 
@@ -64,6 +65,9 @@ def _fits(b, a, d_model, hidden, E) -> bool:
             all(m.weight.shape == up for m in moe.w1) and all(m.weight.shape == down for m in moe.w2))
 
 
+_step_lock = threading.Lock()
+
+
 class LayerTable:
     """jb200_layer array of `blocks`, valid as long as every parameter it was built from is the same unmodified tensor in
     the same place (identity, storage and version are compared on every call: 16 tensors per layer, ~0.1 us each)."""
@@ -83,6 +87,7 @@ class LayerTable:
         self.array = (_lib.Layer * self.n)()
         self._keep = []
         self._sizes = {}
+        self._step = None
         self.has_reflect = all(type(b.reflect) is ReflectivePenalty for b in blocks)
         self._watch(blocks)
         for d, b in zip(self.array, blocks):
@@ -162,6 +167,26 @@ class LayerTable:
             if self.has_reflect and (refl["training"] or refl["_forward_hooks"] or refl["_forward_pre_hooks"] or "forward" in refl):
                 return False
         return True
+
+    def step_weights(self, B: int):
+        """The layers' weights as the one-launch step of B sequences reads them (host array of device pointers), laid out when first
+        wanted; None where there is no such step.  Not made inside a stream capture, which would only record the work."""
+        lib = _lib.load()
+        if B > lib.jb200_step_max_sequences():
+            return None
+        if self._step is None:
+            nbytes = lib.jb200_step_weight_bytes(self.C, self.H, self.E, self.hidden)
+            if not nbytes or torch.cuda.is_current_stream_capturing():
+                return None
+            with _step_lock:
+                if self._step is None:
+                    buf = torch.empty((self.n, nbytes), dtype=torch.uint8, device=self.device)
+                    for d, out in zip(self.array, buf):
+                        _lib.check(lib.jb200_prepare_step_weights(C.byref(d), self.C, self.H, self.E, self.hidden, out.data_ptr(),
+                                                                  ops._stream()), "jb200_prepare_step_weights")
+                    torch.cuda.current_stream(self.device).synchronize()      # any stream may be the next to read them
+                    self._step = buf, _pointers(self.n, buf)
+        return self._step[1]
 
     def sizes(self, B: int, T: int):
         key = (B, T)
@@ -298,7 +323,8 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
     if final_norm is not None:
         res.hidden = torch.empty((B * T, tab.C), dtype=torch.bfloat16, device=dev)
         f.w_final, f.eps_final, f.hidden_out = final_norm[0].data_ptr(), final_norm[1], res.hidden.data_ptr()
-    _lib.check(_lib.load().jb200_forward_layers(tab.array, n, C.byref(f), ops._stream()), "jb200_forward_layers")
+    step = tab.step_weights(B) if T == 1 else None
+    _lib.check(_lib.load().jb200_forward_layers_prepared(tab.array, n, C.byref(f), step, ops._stream()), "jb200_forward_layers")
     for i, (_, moe, _) in enumerate(tab._flags):
         moe["_routing"] = RoutingSource((routing, i, B * T, tab.E))      # the views are built when somebody looks at them
     return res

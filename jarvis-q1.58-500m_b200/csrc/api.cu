@@ -195,7 +195,7 @@ extern "C" {
 
 const char* jb200_last_error(void) { return g_err; }
 
-int jb200_abi_version(void) { return 12; }
+int jb200_abi_version(void) { return 13; }
 
 long long jb200_kernel_launches(int reset) {
   return reset ? g_launches.exchange(0) : g_launches.load();
@@ -435,7 +435,20 @@ size_t jb200_forward_workspace_bytes(int B, int T, int C, int H, int E, int hidd
 }
 
 int jb200_forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, void* stream) {
-  return forward_layers(layers, n_layers, f, static_cast<cudaStream_t>(stream));
+  return forward_layers(layers, n_layers, f, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+size_t jb200_step_weight_bytes(int C, int H, int E, int hidden) { return step_weight_bytes(C, H, E, hidden); }
+
+int jb200_step_max_sequences(void) { return step_max_sequences(); }
+
+int jb200_prepare_step_weights(const jb200_layer* layer, int C, int H, int E, int hidden, void* out, void* stream) {
+  return launch_step_weights(layer, C, H, E, hidden, out, static_cast<cudaStream_t>(stream));
+}
+
+int jb200_forward_layers_prepared(const jb200_layer* layers, int n_layers, const jb200_forward* f, const void* const* step_weights,
+                                  void* stream) {
+  return forward_layers(layers, n_layers, f, step_weights, static_cast<cudaStream_t>(stream));
 }
 
 int jb200_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,

@@ -35,6 +35,7 @@
 // Extra HBM traffic: k and v of the non-final segments are read twice (the second time mostly from L2).
 #include <type_traits>
 
+#include "attn_step.cuh"
 #include "common.cuh"
 #include "launchers.h"
 
@@ -112,17 +113,6 @@ __device__ __forceinline__ void st_global_256(void* p, const uint32_t* w) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                : "memory");
-}
-
-// ELU(x)+1 = max(x, 0) + exp(min(x, 0)) = (x + |x|)/2 + 2^((x - |x|) * log2(e)/2): two adds, one multiply, one
-// ex2.approx (flush-to-zero form: a single MUFU, rel. error 2^-22, far below the bf16 rounding of the result) and
-// one fused multiply-add, all on the FMA / MUFU pipes - no compare, no select.  For x > 0 the exponent is exactly
-// 0 and the result is x + 1 rounded once; for x <= 0 the first term is exactly 0.
-__device__ __forceinline__ float elu1(float x) {
-  const float ax = fabsf(x);
-  float e;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((x - ax) * 0.72134752044448170368f));
-  return fmaf(x + ax, 0.5f, e);
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -905,16 +895,6 @@ __global__ void __launch_bounds__(256) attn_fold_states_kernel(const AttnParams 
   }
 }
 
-// One element of the single-token state update, S' = gamma S + v k', with its roundings spelled out so that both
-// decode kernels below produce the same state bits.
-__device__ __forceinline__ float decode_update(float gamma, float s, float v, float k) {
-  return __fmaf_rn(gamma, s, __fmul_rn(v, k));
-}
-
-// RoPE of a pair (d, d + 32), roundings spelled out for the same reason.
-__device__ __forceinline__ float rope_lo(float a, float b, float c, float s) { return __fmaf_rn(a, c, -__fmul_rn(b, s)); }
-__device__ __forceinline__ float rope_hi(float a, float b, float c, float s) { return __fmaf_rn(b, c, __fmul_rn(a, s)); }
-
 // One-token step (decode): S <- gamma*S + v (x) k', o = S q' for every (sequence, head).  Pure state
 // streaming: 2 x 16 KiB of fp32 state per (sequence, head) against 384 B of q, k, v, so the kernel is a
 // coalesced read-modify-write of S with the feature map + RoPE of the single token done in shared memory.
@@ -922,7 +902,7 @@ __device__ __forceinline__ float rope_hi(float a, float b, float c, float s) { r
 __global__ void __launch_bounds__(256)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                    const __nv_bfloat16* __restrict__ v, int ld_qkv, const AttnParams p) {
-  __shared__ float sv[D], rq[D], rk[D];
+  __shared__ __align__(16) float sv[D], rq[D], rk[D];
   const int h = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
   // What the token does not decide first: the thread's 64 bytes of state, the position and its angles.  In a chain they
   // were written long before and are fetched while the projection still runs.
@@ -964,7 +944,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     const int c = c0 + 4 * i;
     st[i].x = decode_update(gamma, st[i].x, vr, rk[c]);      st[i].y = decode_update(gamma, st[i].y, vr, rk[c + 1]);
     st[i].z = decode_update(gamma, st[i].z, vr, rk[c + 2]);  st[i].w = decode_update(gamma, st[i].w, vr, rk[c + 3]);
-    acc += st[i].x * rq[c] + st[i].y * rq[c + 1] + st[i].z * rq[c + 2] + st[i].w * rq[c + 3];
+    acc += decode_dot4(st[i], *reinterpret_cast<const float4*>(rq + c));
   }
   if (p.s_out) {
 #pragma unroll
@@ -1062,7 +1042,7 @@ attn_decode_stream_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat
       st.x = decode_update(gamma, st.x, vr, kq.x);  st.y = decode_update(gamma, st.y, vr, kq.y);
       st.z = decode_update(gamma, st.z, vr, kq.z);  st.w = decode_update(gamma, st.w, vr, kq.w);
       *cell = st;
-      acc[j] = st.x * qq.x + st.y * qq.y + st.z * qq.z + st.w * qq.w;
+      acc[j] = decode_dot4(st, qq);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

@@ -73,7 +73,7 @@ inline int mid_tile(int rows, int groups, int n_ft, int sms) {
 
 }  // namespace
 
-size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(E + 1) * 4 + 7) / 8 * 8; }
+size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(E + 1) * 4 + 7) / 8 * 8 + step_exchange_bytes(); }
 
 size_t routing_layout(int N, int E, size_t* offsets) {
   const Routing r(N > 0 ? N : 0, E > 0 ? E : 0);
@@ -89,7 +89,7 @@ size_t forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden) {
   return Workspace(B, T, C, H, E, hidden).bytes;
 }
 
-int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, cudaStream_t st) {
+int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, const void* const* step_weights, cudaStream_t st) {
   JB_REQUIRE(layers && f && n_layers >= 1, "forward_layers: null pointer or no layers");
   const int B = f->B, T = f->T, C = f->C, H = f->H, E = f->E, hidden = f->hidden;
   JB_REQUIRE(B >= 1 && T >= 1 && size_t(B) * T < (size_t(1) << 30), "forward_layers: bad shape (B=%d, T=%d)", B, T);
@@ -116,6 +116,11 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const uintptr_t hs = reinterpret_cast<uintptr_t>(f->h_out[l]) | reinterpret_cast<uintptr_t>(f->h_in ? f->h_in[l] : nullptr);
     JB_REQUIRE((hs & a8) == 0 && aligned16(f->s_in ? f->s_in[l] : nullptr) && aligned16(f->s_out ? f->s_out[l] : nullptr),
                "forward_layers: attention states must be 16-byte aligned, membranes 8 (layer %d)", l);
+  }
+  if (T == 1 && step_weights) {
+    bool taken = false;
+    JB_TRY(launch_step_cluster(layers, n_layers, f, step_weights, st, &taken));
+    if (taken) return JB200_OK;
   }
   const int N = B * T;
   const Workspace ws(B, T, C, H, E, hidden);

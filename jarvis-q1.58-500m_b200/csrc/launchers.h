@@ -112,12 +112,20 @@ int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_
 int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const LsfStats& st, const float* var_scale,
                 float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x, const float* w_norm, float eps,
                 void* xn_bf16, int B, int T, int C, cudaStream_t stream);
+// A single-token step of all layers in one launch (step_cluster.cu).  weights[l]: launch_step_weights' layout of layer l
+// (step_weight_bytes, 0 where there is no such form).  taken: false where the call is not one of its kind and nothing was done.
+size_t step_weight_bytes(int C, int H, int E, int hidden);
+int step_max_sequences();
+size_t step_exchange_bytes();            // of a layer's accumulators, where the sums of several clusters meet
+int launch_step_weights(const jb200_layer* layer, int C, int H, int E, int hidden, void* out, cudaStream_t stream);
+int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_forward* f, const void* const* weights,
+                        cudaStream_t stream, bool* taken);
 int launch_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
                          const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, cudaStream_t stream);
 size_t accumulator_bytes(int E);
 size_t routing_layout(int N, int E, size_t* offsets);
 size_t forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden);
-int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, cudaStream_t stream);
+int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward* f, const void* const* step_weights, cudaStream_t stream);
 
 int launch_peer_barrier(const void* const* peer_flags, int world, int rank, cudaStream_t stream);
 int launch_ep_pull_gather(const void* const* peer_offs, const void* const* peer_gmap, const void* const* peer_xn,

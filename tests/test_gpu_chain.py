@@ -395,3 +395,57 @@ def test_dispatch_maps_of_tokens_whose_router_is_nan(N):
     for a, b in zip(got, ops.moe_metadata(idx.contiguous(), 4)):
         assert torch.equal(a, b)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B,layers,states,skew", [(1, 3, True, 0.0), (1, 2, False, 0.0), (2, 34, True, 0.0), (3, 3, True, 3.0), (3, 2, False, 0.0),
+                                                  (4, 3, True, 0.0), (7, 3, True, 3.0), (8, 3, True, 0.0), (13, 3, True, 3.0),
+                                                  (15, 3, True, 0.0), (29, 2, True, 0.0), (49, 3, True, 3.0), (56, 3, True, 0.0),
+                                                  (57, 2, True, 0.0), (5, 2, False, 0.0)])
+def test_one_launch_step_against_the_kernels_it_stands_for(B, layers, states, skew, monkeypatch):
+    """All layers of a single-token step in one launch, bit for bit: one and several clusters, one to eight sequences in each, no states,
+    more layers than a launch takes, experts nobody wants (skew: most tokens go to two), states updated in place over several
+    steps; beyond the last size the kernels themselves run on either side."""
+    from jarvis_b200 import chain
+    torch.manual_seed(B)
+    model = jm.ternary_init_(jm.Jarvis(vocab_size=320, d_model=1024, n_layers=layers, n_heads=16, max_seq_len=64)).cuda().eval()
+    with torch.no_grad():
+        for b in model.blocks:
+            b.moe.router.weight[:2] += skew * b.moe.router.weight[2:].abs().mean() * torch.sign(torch.randn(1024, device="cuda"))
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    state = {"h": [torch.randn(B, 1024, generator=gen, device="cuda") for _ in range(layers)],
+             "S": [torch.randn(B, 16, 64, 64, generator=gen, device="cuda") for _ in range(layers)]} if states else None
+    pos = torch.randint(0, 20, (B,), generator=gen, device="cuda", dtype=torch.int32)
+    idx = torch.randint(0, 320, (4, B, 1), generator=gen, device="cuda")
+    model.step(idx[0], pos, None, max_position=64)             # weights are packed
+    if state:
+        model.step(idx[0], pos, {k: [t.clone() for t in v] for k, v in state.items()}, max_position=64)
+    few = B <= min(56, _lib.load().jb200_step_max_sequences()) and (states or B < 4)
+    got = {}
+    for one_launch in (True, False):
+        if not one_launch:
+            monkeypatch.setattr(chain.LayerTable, "step_weights", lambda self, B: None)
+        st = state and {k: [t.clone() for t in v] for k, v in state.items()}
+        out, before = [], _lib.kernel_launches()
+        for t in range(4):
+            logits, st = model.step(idx[t], pos + t, st, max_position=64, inplace=st is not None)
+            out += [logits, torch.stack([b.moe.last_routing[0] for b in model.blocks]), torch.stack([b.moe.last_routing[1] for b in model.blocks])]
+            out += [torch.cat([m.flatten() for m in b.moe.last_routing[2]]) for b in model.blocks]
+        got[one_launch] = out + st["h"] + st["S"], _lib.kernel_launches() - before
+    assert all(torch.equal(a, b) for a, b in zip(got[True][0], got[False][0]))
+    assert got[True][1] < got[False][1] if few else got[True][1] <= got[False][1]
+    assert _lib.device_status() == 0
+
+
+def test_states_that_overlap_go_kernel_by_kernel():
+    """The one-launch step fetches states layers ahead: a state that another layer writes is left to the kernels, in their order."""
+    torch.manual_seed(3)
+    model = jm.ternary_init_(jm.Jarvis(vocab_size=320, d_model=1024, n_layers=2, n_heads=16, max_seq_len=64)).cuda().eval()
+    idx = torch.tensor([[5], [9]], device="cuda")
+    h, S = torch.randn(2, 1024, device="cuda"), torch.randn(2, 16, 64, 64, device="cuda")
+    apart, shared = [{"h": [h.clone()] * 2, "S": [S.clone()] * 2} for _ in range(2)]
+    model.use_chain = False
+    want, _ = model.step(idx, 0, apart, max_position=64, inplace=True)
+    model.use_chain = True
+    got, _ = model.step(idx, 0, shared, max_position=64, inplace=True)
+    assert torch.equal(got, want) and torch.equal(shared["S"][0], apart["S"][0]) and torch.equal(shared["h"][1], apart["h"][1])
+    assert _lib.device_status() == 0
