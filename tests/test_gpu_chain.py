@@ -416,10 +416,9 @@ def test_one_launch_step_against_the_kernels_it_stands_for(B, layers, states, sk
              "S": [torch.randn(B, 16, 64, 64, generator=gen, device="cuda") for _ in range(layers)]} if states else None
     pos = torch.randint(0, 20, (B,), generator=gen, device="cuda", dtype=torch.int32)
     idx = torch.randint(0, 320, (4, B, 1), generator=gen, device="cuda")
-    model.step(idx[0], pos, None, max_position=64)             # weights are packed
-    if state:
-        model.step(idx[0], pos, {k: [t.clone() for t in v] for k, v in state.items()}, max_position=64)
-    few = B <= min(56, _lib.load().jb200_step_max_sequences()) and (states or B < 4)
+    _, first = model.step(idx[0], pos, None, max_position=64)             # weights are packed, on the next call laid out
+    model.step(idx[0], pos, first, max_position=64)
+    few = B <= min(56, _lib.load().jb200_step_max_sequences())
     got = {}
     for one_launch in (True, False):
         if not one_launch:
