@@ -55,6 +55,12 @@ struct Workspace {
 // MID_TOKENS the tcgen05 form that is built for latency (640 tokens 1.96 against 2.08 ms, 900 2.20 against 2.29, 1000 equal,
 // 1152 2.81 against 2.74), beyond that the persistent pipeline.
 constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
+// The products of the attention have few out-features: the tcgen05 form runs them on 8 to 24 SMs.  mma.sync with the token tiles side
+// by side (8 rows each for prompts, 16 for steps) fills the chip, and its chain over K is shorter.  24 layers and head as a graph: prompts
+// of 37, 64, 100 tokens with the out-projection so 1052 -> 1035, 1110 -> 1096, 1322 -> 1287 us, 180 equal, 256 1402 -> 1447; with q|k|v
+// so 20 tokens 1015 -> 1008, 37 1052 -> 1047, 64 1110 -> 1122.  Steps of 64, 100, 128 sequences with q|k|v so 1094 -> 1070,
+// 1361 -> 1351, equal; their out-projection, behind the attention's stores, gets slower (64: 1094 -> 1114).
+constexpr int OUT_TILED_TOKENS = 128, QKV_TILED_PROMPT = 40, QKV_TILED_STEP = 100;
 // Up to here the first expert GEMM takes all rows for every expert and stores the routed ones: more MMAs, no dispatch.
 constexpr int ALL_ROWS_TOKENS = 64;
 // Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
@@ -131,7 +137,10 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   uint16_t *y = reinterpret_cast<uint16_t*>(w + ws.y), *out = reinterpret_cast<uint16_t*>(w + ws.out);
   uint16_t* disp = qkv;
   float* x = f->x;
-  const bool small = N <= SMALL_TOKENS && small_gemm_fits(N, std::max(C, hidden));   // beyond, the tcgen05 form streams K
+  const int small_tile = N <= 8 ? 8 : 16;
+  const bool small = N <= SMALL_TOKENS && small_gemm_fits(small_tile, std::max(C, hidden));   // beyond, the tcgen05 form streams K
+  const int out_tile = T > 1 && N <= OUT_TILED_TOKENS ? 8 : 0;
+  const int qkv_tile = T > 1 ? (N <= QKV_TILED_PROMPT ? 8 : 0) : (N <= QKV_TILED_STEP ? 16 : 0);
   const bool mid = !small && N <= MID_TOKENS;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
@@ -181,7 +190,9 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
 
     // x += attn(norm1(x))
     if (small)
-      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, N, st));
+      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, 1, st));
+    else if (qkv_tile)
+      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile, (N + qkv_tile - 1) / qkv_tile, st));
     else if (mid)
       JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv));
     else
@@ -192,7 +203,9 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     JB_TRY(launch_attn_scan(qkv, qkv + C, qkv + 2 * C, 3 * C, p.gamma, f->cos_tab, f->sin_tab, f->n_pos, f->pos0, f->pos0_scalar,
                             s_in, o, C, s_out, attn_scratch, B, T, H, 64, 0, st, true));
     if (small)
-      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, N, st));
+      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, 1, st));
+    else if (out_tile)
+      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile, (N + out_tile - 1) / out_tile, st));
     else if (mid)
       JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x));
     else
@@ -209,7 +222,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (N <= ALL_ROWS_TOKENS) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
       if (small)
-        JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, N, st));
+        JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, small_tile, 1, st));
       else
         JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid));
     } else {
@@ -220,7 +233,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
         JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true));
     }
     if (small)
-      JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, N, st));
+      JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, 1, st));
     else if (mid)
       JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y));
     else
