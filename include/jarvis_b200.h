@@ -248,6 +248,14 @@ int jb200_moe_metadata_static(const int64_t* topk_idx, int N, int K, int E, int3
 int jb200_moe_dispatch_gather(const void* x, const int32_t* gather_map, int M, int N, int C, void* dispatched,
                               void* stream);
 
+/* Both at once for top-2 assignments of up to 131,072 tokens, 4 or 8 experts, C <= 1024 (multiple of 8): the maps of
+ * jb200_moe_metadata and the rows of jb200_moe_dispatch_gather, in two launches and with every row read once.
+ * scratch: jb200_moe_dispatch_scratch_bytes, 16-byte aligned. */
+size_t jb200_moe_dispatch_scratch_bytes(int n_tokens, int E);
+int jb200_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int32_t* expert_counts,
+                       int32_t* expert_offsets, int32_t* scatter_map, int32_t* gather_map, int32_t* gate_idx_map, void* dispatched,
+                       void* scratch, void* stream);
+
 /* scatter_combine (sparse_model.cu:117-165): out[i] = sum_k gates[i][k] * y[scatter_map[i][k]] with f32
  * accumulation; y: bf16 [N*K][C]; out: f32 (0) or bf16 (1) [N][C].  stats: f64 [2] or NULL, ACCUMULATES
  * sum(out) and sum(out^2) of the unrounded values (for act_mean / act_var, jarvis_model.py:249-250). */

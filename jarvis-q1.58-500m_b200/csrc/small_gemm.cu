@@ -6,8 +6,9 @@
 // and the token rows - one contiguous block each - to shared memory with asynchronous 16-byte copies, all in flight at
 // once (one bulk copy per row measured 1-3 us slower); a warp then walks all of K for 16 out-features x 8 or 16 tokens.
 // The weights do not depend on the kernel before this one: in a chain they are requested before the grid dependency is
-// waited for.  Token tiles beyond the first can be given to CTAs of their own (grid z), which copy the codes again.  The first expert matrix takes every token for every expert and stores only the routed ones (fetching rows
-// through the gather map put one more memory latency and most of the instructions of a call in front of its first MMA).
+// waited for.  Token tiles beyond the first can be given to CTAs of their own (grid z), which copy the codes again.  The first
+// expert matrix takes every token for every expert and stores only the routed ones (fetching rows through the gather map put one
+// more memory latency and most of the instructions of a call in front of its first MMA).
 //
 // Results are those of ternary_gemm_kernel bit for bit: the f32 accumulator is one chain over K in steps of 16, and
 // mma.sync.m16n8k16 rounds a step as tcgen05.mma does (measured: no differing bit for K = 16..2048, normal and

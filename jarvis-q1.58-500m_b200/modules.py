@@ -322,8 +322,11 @@ class SparseMoELayer(nn.Module):
             idx, gates, _ = ops.router_top2(xn_rows, w_r, probs_sum=acc[2:], top1_hist=hist)
         # expert parallel: the gather map and the expert offsets are written where the other ranks read them
         meta_in_slab = ep is not None and N <= ep.ex.n_max
+        disp = None
         if meta_in_slab:
             meta = ops.moe_metadata(idx, E, gather_out=ep.ex.gmap[:N * self.top_k], offsets_out=ep.ex.offs[:E + 1])
+        elif ep is None and 256 < N <= ops.DISPATCH_MAX and C <= 1024:
+            meta, disp = ops.moe_dispatch(xn_rows, idx, E)
         else:
             meta = ops.moe_metadata(idx, E)
         counts, offsets, scatter, gather, gate_idx = meta
@@ -333,7 +336,8 @@ class SparseMoELayer(nn.Module):
                                 meta_in_slab=meta_in_slab, out_dtype=out_dtype, stats=acc[:2])
         else:
             (p1, a1), (p2, a2) = self.packed()
-            disp = ops.dispatch_gather(xn_rows, gather)
+            if disp is None:
+                disp = ops.dispatch_gather(xn_rows, gather)
             hid = ops.ternary_linear_grouped(disp, p1, a1, offsets, epilogue=ops.EPI_GELU_BF16, prepared=True)
             y = ops.ternary_linear_grouped(hid, p2, a2, offsets, epilogue=ops.EPI_BF16, prepared=True)
             out = ops.scatter_combine(y, gates, scatter, out_dtype=out_dtype, stats=acc[:2])

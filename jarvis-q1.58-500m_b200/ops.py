@@ -424,6 +424,27 @@ def dispatch_gather(x: torch.Tensor, gather_map: torch.Tensor) -> torch.Tensor:
     return out
 
 
+DISPATCH_MAX = 131072      # tokens of moe_dispatch
+
+
+def moe_dispatch(x: torch.Tensor, topk_idx: torch.Tensor, num_experts: int):
+    """moe_metadata and dispatch_gather of top-2 assignments at once: ((counts, offsets, scatter, gather, gate_idx), rows)."""
+    lib = _lib.load()
+    _need(x, torch.bfloat16, "moe_dispatch.x")
+    _need(topk_idx, torch.int64, "moe_dispatch.topk_idx")
+    N, C = x.shape
+    if topk_idx.shape != (N, 2):
+        raise RuntimeError(f"moe_dispatch: topk_idx of shape {tuple(topk_idx.shape)}, expected {(N, 2)}")
+    E, dev, i32 = num_experts, x.device, torch.int32
+    counts, offsets = torch.empty((E,), dtype=i32, device=dev), torch.empty((E + 1,), dtype=i32, device=dev)
+    scatter, gather, gate_idx = torch.empty((3, 2 * N), dtype=i32, device=dev).unbind(0)
+    out = torch.empty((2 * N, C), dtype=torch.bfloat16, device=dev)
+    scratch = torch.empty((lib.jb200_moe_dispatch_scratch_bytes(N, E) // 4,), dtype=i32, device=dev)
+    _lib.check(lib.jb200_moe_dispatch(_ptr(topk_idx), _ptr(x), N, C, E, _ptr(counts), _ptr(offsets), _ptr(scatter), _ptr(gather),
+                                      _ptr(gate_idx), _ptr(out), _ptr(scratch), _stream()), "jb200_moe_dispatch")
+    return (counts, offsets, scatter.view(N, 2), gather, gate_idx), out
+
+
 def scatter_combine(y: torch.Tensor, gates: torch.Tensor, scatter_map: torch.Tensor, *, out_dtype=torch.bfloat16,
                     stats: torch.Tensor | None = None) -> torch.Tensor:
     lib = _lib.load()

@@ -448,3 +448,21 @@ def test_states_that_overlap_go_kernel_by_kernel():
     got, _ = model.step(idx, 0, shared, max_position=64, inplace=True)
     assert torch.equal(got, want) and torch.equal(shared["S"][0], apart["S"][0]) and torch.equal(shared["h"][1], apart["h"][1])
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("E,C", [(4, 1024), (8, 136)])
+@pytest.mark.parametrize("N", [1, 63, 64, 65, 257, 4095, 4097, 70000])
+def test_dispatch_in_one_launch_against_metadata_and_gather(N, E, C):
+    """Chunk edges, one to a thousand chunks, an expert nobody takes, assignments without an expert."""
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    first = torch.randint(0, E - 1, (N,), generator=gen, device="cuda")
+    idx = torch.stack([first, (first + torch.randint(1, E - 1, (N,), generator=gen, device="cuda")) % (E - 1)], 1)
+    idx[N // 2, 1] = -1
+    idx[N // 3] = 0
+    x = torch.randn(N, C, generator=gen, device="cuda").bfloat16()
+    got, rows = ops.moe_dispatch(x, idx, E)
+    want = ops.moe_metadata(idx, E)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(rows, ops.dispatch_gather(x, want[3]))
+    with pytest.raises(RuntimeError):
+        ops.moe_dispatch(x, idx[:, :1].contiguous(), E)
+    assert _lib.device_status() == 0
