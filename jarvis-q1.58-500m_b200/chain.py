@@ -323,8 +323,9 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
     if final_norm is not None:
         res.hidden = torch.empty((B * T, tab.C), dtype=torch.bfloat16, device=dev)
         f.w_final, f.eps_final, f.hidden_out = final_norm[0].data_ptr(), final_norm[1], res.hidden.data_ptr()
-    # a lone token without any carried state is no decode loop: not worth a second layout of the weights
-    step = tab.step_weights(B) if T == 1 and (h_in is not None or s_in is not None) else None
+    # A lone token without any carried state is no decode loop: not worth a second layout of the weights.  From four sequences on the
+    # one-launch step takes an attention state and leaves one.
+    step = tab.step_weights(B) if T == 1 and (s_in is not None or (h_in is not None and B < 4)) else None
     _lib.check(_lib.load().jb200_forward_layers_prepared(tab.array, n, C.byref(f), step, ops._stream()), "jb200_forward_layers")
     for i, (_, moe, _) in enumerate(tab._flags):
         moe["_routing"] = RoutingSource((routing, i, B * T, tab.E))      # the views are built when somebody looks at them

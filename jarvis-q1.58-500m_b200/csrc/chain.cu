@@ -79,7 +79,7 @@ inline int mid_tile(int rows, int groups, int n_ft, int sms) {
 
 }  // namespace
 
-size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(E + 1) * 4 + 7) / 8 * 8 + step_exchange_bytes(); }
+size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(E + 1) * 4 + 7) / 8 * 8; }
 
 size_t routing_layout(int N, int E, size_t* offsets) {
   const Routing r(N > 0 ? N : 0, E > 0 ? E : 0);

@@ -1003,7 +1003,6 @@ int max_clusters() {
 
 size_t step_weight_bytes(int c, int h, int e, int hidden) { return c == C && h == CTAS && e == E && hidden == HID ? LAYER_BYTES : 0; }
 int step_max_sequences() { return max_clusters() * MAX_TOKENS; }
-size_t step_exchange_bytes() { return MAX_CLUSTERS * 32; }
 
 int launch_step_weights(const jb200_layer* y, int c, int h, int e, int hidden, void* out, cudaStream_t stream) {
   JB_REQUIRE(y && out && y->w_qkv && y->w_out && y->w1 && y->w2 && y->w_router && y->gamma && y->a_qkv && y->a_out && y->a1 && y->a2 && y->var_scale,
@@ -1046,10 +1045,12 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
   const Plan s = plan_of(tokens, full);
   size_t off[7];
   StepParams p = {};
+  // A layer's accumulators, and the words in which the sums of several clusters meet, lie in the workspace: the rest of it is not used here.
+  p.acc_stride = accumulator_bytes(E) + MAX_CLUSTERS * 32;
+  if (forward_workspace_bytes(N, 1, C, CTAS, E, HID) < n_layers * p.acc_stride) return JB200_OK;
   p.routing_stride = routing_layout(N, E, off);
   p.r_idx = uint32_t(off[0]); p.r_gates = uint32_t(off[1]); p.r_counts = uint32_t(off[2]); p.r_offsets = uint32_t(off[3]);
   p.r_scatter = uint32_t(off[4]); p.r_gather = uint32_t(off[5]); p.r_gate_idx = uint32_t(off[6]);
-  p.acc_stride = accumulator_bytes(E);
   p.o_p1 = s.o_p1; p.o_p2 = s.o_p2; p.o_sc = s.o_sc; p.o_rx = s.o_rx; p.o_xn = s.o_xn; p.o_rh = s.o_rh; p.o_qkv = s.o_qkv; p.o_ho = s.o_ho; p.o_ry = s.o_ry;
   p.o_cs = s.o_cs; p.o_scr = s.o_scr; p.o_ring = s.o_ring; p.units = s.units;
   p.x = f->x; p.cos_tab = f->cos_tab; p.sin_tab = f->sin_tab; p.pos0 = f->pos0; p.pos0_scalar = f->pos0_scalar; p.n_pos = f->n_pos;
@@ -1058,7 +1059,7 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
   p.units_inv = uint32_t(0xffffffffu / uint32_t(s.units)) + 1u;
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
-  if (n_cl > 1) JB_CUDA(cudaMemsetAsync(f->accumulators, 0, n_layers * p.acc_stride, stream));
+  if (n_cl > 1) JB_CUDA(cudaMemsetAsync(f->workspace, 0, n_layers * p.acc_stride, stream));
   for (int l0 = 0; l0 < n_layers; l0 += MAX_LAYERS) {
     const int n = n_layers - l0 < MAX_LAYERS ? n_layers - l0 : MAX_LAYERS;
     const bool end = l0 + n == n_layers;
@@ -1068,7 +1069,7 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
     p.w_final = end ? f->w_final : nullptr;
     p.eps_final = f->eps_final;
     p.hidden_out = reinterpret_cast<__nv_bfloat16*>(f->hidden_out);
-    p.acc = static_cast<uint8_t*>(f->accumulators) + l0 * p.acc_stride;
+    p.acc = static_cast<uint8_t*>(f->workspace) + l0 * p.acc_stride;
     p.routing = static_cast<uint8_t*>(f->routing) + l0 * p.routing_stride;
     p.scalars = f->scalars + size_t(l0) * 3;
     p.reflect = f->reflect ? f->reflect + l0 : nullptr;
