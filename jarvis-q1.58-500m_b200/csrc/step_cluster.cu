@@ -21,8 +21,7 @@
 // belongs to four CTAs, which exchange its hidden rows among themselves.
 // Measured (24 layers and the vocabulary head, replayed as a graph, kernel by kernel -> here): 1 sequence 621 -> 496 us, 2 675 -> 516,
 // 4 710 -> 511, 7 715 -> 515, 8 718 -> 641, 16 810 -> 663, 32 937 -> 751, 56 1049 -> 941.  With more tokens a cluster the form
-// loses: every cluster decodes all weights for itself, and shared memory runs out at eight (64 sequences in ten-token clusters
-// took 1015 us against 1092, with a ring too shallow for its warps).
+// loses: every cluster decodes all weights for itself, and shared memory holds eight.
 // Every value is rounded and every sum ordered as in the kernels this one stands for: results are theirs bit for bit.
 #include "attn_step.cuh"
 #include "common.cuh"
