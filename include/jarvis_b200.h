@@ -375,6 +375,9 @@ int jb200_forward_layers(const jb200_layer* layers, int n_layers, const jb200_fo
  * (again whenever one of its tensors changes), 16-byte aligned. */
 size_t jb200_step_weight_bytes(int C, int H, int E, int hidden);
 int jb200_step_max_sequences(void);      /* most sequences of such a step on the current device, 0: none */
+/* Thread-block clusters that such a step of B sequences runs in where `resident` of them fit the device; 0: kernel by kernel.
+ * carried: every layer is given an attention state and leaves one. */
+int jb200_step_clusters(int B, int resident, int carried);
 int jb200_prepare_step_weights(const jb200_layer* layer, int C, int H, int E, int hidden, void* out, void* stream);
 int jb200_forward_layers_prepared(const jb200_layer* layers, int n_layers, const jb200_forward* f, const void* const* step_weights,
                                   void* stream);

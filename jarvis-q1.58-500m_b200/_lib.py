@@ -84,6 +84,7 @@ PROTOTYPES = {
     "jb200_forward_layers": (_I, [_P, _I, C.POINTER(Forward), _P]),
     "jb200_step_weight_bytes": (_Z, [_I] * 4),
     "jb200_step_max_sequences": (_I, []),
+    "jb200_step_clusters": (_I, [_I, _I, _I]),
     "jb200_prepare_step_weights": (_I, [_P, _I, _I, _I, _I, _P, _P]),
     "jb200_forward_layers_prepared": (_I, [_P, _I, C.POINTER(Forward), _P, _P]),
     "jb200_peer_buffer_alloc": (_I, [_Z, _P, _P]),

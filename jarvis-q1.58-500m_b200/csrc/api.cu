@@ -451,6 +451,8 @@ size_t jb200_step_weight_bytes(int C, int H, int E, int hidden) { return step_we
 
 int jb200_step_max_sequences(void) { return step_max_sequences(); }
 
+int jb200_step_clusters(int B, int resident, int carried) { return step_clusters(B, resident, carried != 0); }
+
 int jb200_prepare_step_weights(const jb200_layer* layer, int C, int H, int E, int hidden, void* out, void* stream) {
   return launch_step_weights(layer, C, H, E, hidden, out, static_cast<cudaStream_t>(stream));
 }

@@ -121,6 +121,7 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
 // (step_weight_bytes, 0 where there is no such form).  taken: false where the call is not one of its kind and nothing was done.
 size_t step_weight_bytes(int C, int H, int E, int hidden);
 int step_max_sequences();
+int step_clusters(int N, int most, bool carried);
 int launch_step_weights(const jb200_layer* layer, int C, int H, int E, int hidden, void* out, cudaStream_t stream);
 int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_forward* f, const void* const* weights,
                         cudaStream_t stream, bool* taken);

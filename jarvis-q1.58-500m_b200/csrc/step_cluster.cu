@@ -967,6 +967,8 @@ Plan plan_of(int tokens, bool full) {
   return s;
 }
 
+bool stream_sums(int N) { return N * CTAS >= 64; }      // launch_attn_scan's choice
+
 // Clusters of sixteen that are resident at once on the current device (0: none); asked once per device.
 int max_clusters() {
   static std::atomic<int> known[64];
@@ -1003,6 +1005,21 @@ int max_clusters() {
 size_t step_weight_bytes(int c, int h, int e, int hidden) { return c == C && h == CTAS && e == E && hidden == HID ? LAYER_BYTES : 0; }
 int step_max_sequences() { return max_clusters() * MAX_TOKENS; }
 
+// Clusters that a step of N sequences runs in where `most` are resident at once; 0: kernel by kernel.  carried: every layer takes an
+// attention state and leaves one.
+//
+// A sequence per cluster while there are clusters (two sequences in one cluster 591 us, in two 516), then two in each (8 sequences in two,
+// three, four clusters 694, 657, 641 us), then as many as it takes.  From launch_attn_scan's limit on sums are attn_decode_stream_kernel's,
+// which knows no call without states; several sequences in a cluster exist with these sums alone, so two or three sequences
+// that do not get a cluster each (a device with room for one or two) are left to the kernels.
+int step_clusters(int N, int most, bool carried) {
+  if (most > MAX_CLUSTERS) most = MAX_CLUSTERS;
+  if (N < 1 || N > most * MAX_TOKENS || (stream_sums(N) && !carried)) return 0;
+  int n_cl = N <= most ? N : (N + 1) / 2;
+  if (n_cl > most) n_cl = most;
+  return n_cl < N && !stream_sums(N) ? 0 : n_cl;
+}
+
 int launch_step_weights(const jb200_layer* y, int c, int h, int e, int hidden, void* out, cudaStream_t stream) {
   JB_REQUIRE(y && out && y->w_qkv && y->w_out && y->w1 && y->w2 && y->w_router && y->gamma && y->a_qkv && y->a_out && y->a1 && y->a2 && y->var_scale,
              "step_weights: null pointer");
@@ -1020,13 +1037,13 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
   *taken = false;
   const int N = f->B;
   if (f->T != 1 || !weights || step_weight_bytes(f->C, f->H, f->E, f->hidden) == 0) return JB200_OK;
-  const int most = max_clusters();
-  if (N > most * MAX_TOKENS) return JB200_OK;
-  const bool stream_sums = N * CTAS >= 64;       // launch_attn_scan's choice
+  bool carried = true;
   for (int l = 0; l < n_layers; ++l) {
-    if (stream_sums && !(f->s_in && f->s_in[l] && f->s_out && f->s_out[l])) return JB200_OK;      // they take a state and leave one
+    carried = carried && f->s_in && f->s_in[l] && f->s_out && f->s_out[l];
     if (!weights[l] || !aligned16(weights[l]) || !aligned16(f->h_out[l]) || (f->h_in && !aligned16(f->h_in[l]))) return JB200_OK;
   }
+  const int n_cl = step_clusters(N, max_clusters(), carried);
+  if (n_cl == 0) return JB200_OK;
   // States and membranes are fetched layers ahead: what one layer writes must not be what another one reads, nor its own input
   // except in place.
   for (int l = 0; l < n_layers; ++l)
@@ -1035,10 +1052,6 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
       if (meet(f->h_in ? f->h_in[l] : nullptr, f->h_out[k], size_t(N) * C) ||
           meet(f->s_in ? f->s_in[l] : nullptr, f->s_out ? f->s_out[k] : nullptr, size_t(N) * C * D)) return JB200_OK;
     }
-  // A sequence per cluster while there are clusters (two sequences in one cluster 591 us, in two 516), then two in each (8 sequences in two,
-  // three, four clusters 694, 657, 641 us), then as many as it takes.
-  int n_cl = N <= most ? N : (N + 1) / 2;
-  if (n_cl > most) n_cl = most;
   const int tokens = (N + n_cl - 1) / n_cl;
   const bool full = tokens == 1;
   const Plan s = plan_of(tokens, full);
@@ -1096,8 +1109,8 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
       at[1].val.programmaticStreamSerializationAllowed = dependent_launch_enabled() ? 1 : 0;
     }
     const cudaError_t e = !full ? cudaLaunchKernelEx(&cfg, step_cluster_kernel<false, true>, p)
-                          : stream_sums ? cudaLaunchKernelEx(&cfg, step_cluster_kernel<true, true>, p)
-                                        : cudaLaunchKernelEx(&cfg, step_cluster_kernel<true, false>, p);
+                          : stream_sums(N) ? cudaLaunchKernelEx(&cfg, step_cluster_kernel<true, true>, p)
+                                           : cudaLaunchKernelEx(&cfg, step_cluster_kernel<true, false>, p);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       if (l0 == 0 && e == cudaErrorCooperativeLaunchTooLarge) return JB200_OK;      // fewer SMs than the device has: kernel by kernel

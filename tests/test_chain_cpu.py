@@ -207,3 +207,22 @@ def test_refused_tokens_do_not_move_the_position():
     with pytest.raises(RuntimeError):
         model(torch.zeros((1, 5), dtype=torch.int64), persist_state=True)
     assert model._token_pos == 0
+
+
+def test_which_single_token_steps_run_in_one_launch():
+    """Several sequences in a cluster only with the sums of four and more, and those only with states, however few clusters fit."""
+    lib = _lib.load()
+    for resident in range(10):
+        for B in range(0, 80):
+            for carried in (0, 1):
+                n = lib.jb200_step_clusters(B, resident, carried)
+                if n == 0:
+                    continue
+                assert 1 <= n <= min(resident, 8, B) and -(-B // n) <= 8
+                assert B >= 4 or n == B                  # the kernels sum two or three sequences another way
+                assert carried or B < 4
+    whole = [lib.jb200_step_clusters(B, 7, 1) for B in range(1, 60)]
+    assert whole == [1, 2, 3, 4, 5, 6, 7, 4, 5, 5, 6, 6] + [7] * 44 + [0] * 3
+    assert [lib.jb200_step_clusters(B, 7, 0) for B in range(1, 6)] == [1, 2, 3, 0, 0]
+    assert [lib.jb200_step_clusters(B, 1, 1) for B in (1, 2, 3, 4, 8, 9)] == [1, 0, 0, 1, 1, 0]
+    assert [lib.jb200_step_clusters(B, 2, c) for B in (2, 3) for c in (0, 1)] == [2, 2, 0, 0]
