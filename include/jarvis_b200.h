@@ -371,8 +371,9 @@ int jb200_forward_layers(const jb200_layer* layers, int n_layers, const jb200_fo
 
 /* The same with every layer's weights at hand in a second layout as well (step_weights: HOST array of n_layers device pointers,
  * entries and the array may be NULL): single-token steps of few sequences then run all layers in one launch, with the same results.
- * jb200_step_weight_bytes: of one layer, 0 where the sizes have no such form; jb200_prepare_step_weights lays a layer out
- * (again whenever one of its tensors changes), 16-byte aligned. */
+ * jb200_step_weight_bytes: of one layer, 0 where the sizes have no such form; jb200_prepare_step_weights lays a layer's packed
+ * matrices, their scales and gamma out (again whenever one of these changes; the step reads norms, router, var_scale and mu from
+ * the layer itself), 16-byte aligned. */
 size_t jb200_step_weight_bytes(int C, int H, int E, int hidden);
 int jb200_step_max_sequences(void);      /* most sequences of such a step on the current device, 0: none */
 /* Thread-block clusters that such a step of B sequences runs in where `resident` of them fit the device; 0: kernel by kernel.

@@ -36,21 +36,23 @@ namespace jb {
 namespace {
 
 constexpr int CTAS = 16, C = 1024, D = 64, E = 4, HID = 2048;      // cluster; d_model = 16 heads x 64, experts of 2048
-constexpr int WARPS = 16, THREADS = 32 * (WARPS + 1);              // sixteen that compute and the producer
+constexpr int WARPS = 16, THREADS = 32 * (WARPS + 2);              // sixteen that compute, the producer, the one of settle()
 constexpr int UNIT = 4096, MAX_UNITS = 48;
 constexpr int ROW_C = 2 * C + 16, ROW_H = 2 * HID + 16;            // bf16 rows that ldmatrix reads, padded against bank conflicts
 constexpr int MAX_TOKENS = 8;                                     // of a cluster
 constexpr int MAX_CLUSTERS = 8, MAX_LAYERS = 32;                   // layers of one launch
 constexpr int SCRATCH = 512;                                       // bytes per warp
 
-// A layer's weights: 16-row x 1024-in-feature tiles of q|k|v, out-projection, w1, w2 (two halves each), then router rows, scalars
-constexpr int T_OUT = 3 * C / 16, T_W1 = T_OUT + C / 16, T_W2 = T_W1 + E * HID / 16, T_ROUTER = T_W2 + 2 * E * C / 16;
-constexpr int SC_GAMMA = 0, SC_AQKV = 16, SC_AOUT = 19, SC_A1 = 20, SC_A2 = 24, SC_VAR = 28, SC_FLOATS = 32;
-constexpr size_t LAYER_BYTES = size_t(T_ROUTER + E) * UNIT + 256;
+// A layer's weights: 16-row x 1024-in-feature tiles of q|k|v, out-projection, w1, w2 (two halves each), then scalars.  Only what is
+// derived from parameters by quantising or by the decays' sigmoid; norms, router and var_scale are read where the caller has them, so
+// that a captured step follows an edit of those as the kernels do.
+constexpr int T_OUT = 3 * C / 16, T_W1 = T_OUT + C / 16, T_W2 = T_W1 + E * HID / 16, T_END = T_W2 + 2 * E * C / 16;
+constexpr int SC_GAMMA = 0, SC_AQKV = 16, SC_AOUT = 19, SC_A1 = 20, SC_A2 = 24, SC_FLOATS = 32;
+constexpr size_t LAYER_BYTES = size_t(T_END) * UNIT + 256;
 
 struct StepLayer {
   const uint8_t* tiles;
-  const float *w_norm1, *w_norm2, *s_in, *h_in, *mu;
+  const float *w_norm1, *w_norm2, *w_router, *var_scale, *s_in, *h_in, *mu;
   float *s_out, *h_out;
   float eps1, eps2, alpha_min, alpha_max, balance_alpha, lam, tau;
 };
@@ -77,13 +79,13 @@ struct StepParams {
 };
 
 struct Ctl {
-  uint64_t full[MAX_UNITS], empty[MAX_UNITS], p1_full, p1_empty, p2_full, p2_empty;
+  uint64_t full[MAX_UNITS], empty[MAX_UNITS], p1_full, p1_empty, p2_there, p2_full, p2_empty;
   uint64_t got_o, got_x, got_h, got_y;               // rows that have arrived
   double part[MAX_TOKENS][2];
   alignas(8) float gates2[MAX_TOKENS][2];
   alignas(8) uint32_t word[32];
   int expert[MAX_TOKENS][2];                         // two different ones
-  float alpha;
+  float alpha, var_scale[2];
   uint32_t abort_flag;
   int last;
   uint8_t list[WARPS][2 * MAX_TOKENS];
@@ -232,7 +234,7 @@ struct Step {
       if (elect_one()) {
         mbar_arrive_expect_tx(bar(ctl.p1_full), C * 4 + (lay ? SC_FLOATS * 4 : 0));
         bulk_load_1d(base + p.o_p1, w, C * 4, bar(ctl.p1_full));
-        if (lay) bulk_load_1d(base + p.o_sc + uint32_t(i & 1) * (SC_FLOATS * 4), p.layer[i].tiles + size_t(T_ROUTER + E) * UNIT, SC_FLOATS * 4, bar(ctl.p1_full));
+        if (lay) bulk_load_1d(base + p.o_sc + uint32_t(i & 1) * (SC_FLOATS * 4), p.layer[i].tiles + size_t(T_END) * UNIT, SC_FLOATS * 4, bar(ctl.p1_full));
       }
       __syncwarp();
     };
@@ -270,7 +272,7 @@ struct Step {
         const StepLayer& z = p.layer[l + 1];
         if (z.s_in && lane < NT) l2_prefetch(z.s_in + (size_t(n0 + lane) * CTAS + c) * (D * D), D * D * 4);
 #pragma unroll 1
-        for (int i = cluster * CTAS + c + p.n_clusters * CTAS * lane; i < T_ROUTER / 4; i += p.n_clusters * CTAS * 32)
+        for (int i = cluster * CTAS + c + p.n_clusters * CTAS * lane; i < T_END / 4; i += p.n_clusters * CTAS * 32)
           l2_prefetch(z.tiles + size_t(i) * (4 * UNIT), 4 * UNIT);
         __syncwarp();
       }
@@ -280,9 +282,9 @@ struct Step {
         if (kind == OUT) {
           ok = wait(ctl.p2_empty, uint32_t(l) ^ 1u);
           if (ok && elect_one()) {
-            mbar_arrive_expect_tx(bar(ctl.p2_full), C * 4 + E * UNIT);
-            bulk_load_1d(base + p.o_p2, y.w_norm2, C * 4, bar(ctl.p2_full));
-            bulk_load_1d(base + p.o_p2 + C * 4, w + size_t(T_ROUTER) * UNIT, E * UNIT, bar(ctl.p2_full));
+            mbar_arrive_expect_tx(bar(ctl.p2_there), C * 4 + E * UNIT);
+            bulk_load_1d(base + p.o_p2, y.w_norm2, C * 4, bar(ctl.p2_there));
+            bulk_load_1d(base + p.o_p2 + C * 4, y.w_router, E * UNIT, bar(ctl.p2_there));
           }
           __syncwarp();
         }
@@ -296,6 +298,31 @@ struct Step {
       for (int u = issued > p.units ? issued - p.units : 0; u < issued; ++u)
 #pragma unroll 1
         for (int i = 0; i < 2000 && !phase_done(bar(ctl.full[u % p.units]), uint32_t(u / p.units) & 1u); ++i) {}
+    }
+  }
+
+  // ---------------- what a layer reads from the parameters themselves, by a warp of its own ----------------
+  // The router's rows in the order in which route() reads them without bank conflicts: 16 bytes (group i, half, lane) hold channels
+  // (32 i + lane) 8 + 4 half; in their own order every read is a two-way conflict.  And var_scale.  By the producer, as copies of 16 bytes,
+  // this cost a step 1 % at one sequence and 5 % at 32; by warps that have no part in q, k, v the layer's code grew from 47 to 61 KB
+  // (592 us for 498).
+  __device__ __forceinline__ void settle() const {
+    const uint32_t router = base + p.o_p2 + C * 4, to = router + uint32_t(lane & 1) * 512u + uint32_t(lane >> 1) * 16u;
+#pragma unroll 1
+    for (int l = 0; l < p.n_layers; ++l) {
+      const float var_scale = *p.layer[l].var_scale;
+      if (!wait(ctl.p2_there, uint32_t(l))) return;
+#pragma unroll 4
+      for (uint32_t i = 0; i < E * UNIT; i += 1024) {        // a group's 1 KB stays where it is
+        const uint4 a = lds128(router + i + uint32_t(lane) * 16u), b = lds128(router + i + 512u + uint32_t(lane) * 16u);
+        __syncwarp();
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to + i), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w) : "memory");
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to + i + 256u), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the next layer's bulk copy comes after these stores
+      ctl.var_scale[l & 1] = var_scale;       // two: the next one may be here before decay() has run
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(ctl.p2_full));
     }
   }
   static __device__ __forceinline__ void l2_prefetch(const void* src, uint32_t bytes) {
@@ -566,7 +593,7 @@ struct Step {
   }
 
   // The decay of layer l from the sums over all tokens, by one warp; -> ctl.alpha
-  __device__ __forceinline__ void decay(int l, float var_scale) const {
+  __device__ __forceinline__ void decay(int l) const {
     const StepLayer& y = p.layer[l];
     double s[2] = {0.0, 0.0};
 #pragma unroll 1
@@ -605,7 +632,7 @@ struct Step {
     const double mean64 = div_by(s[0], p.n_elems, p.n_inv), var64 = div_by(s[1] - s[0] * mean64, p.n_elems - 1.0, p.n1_inv);
     const float mean = float(mean64), var = float(var64 > 0.0 ? var64 : 0.0);
     if (lane == 0) {
-      ctl.alpha = lsf_alpha_from_var(y.alpha_min, y.alpha_max, var_scale, var);
+      ctl.alpha = lsf_alpha_from_var(y.alpha_min, y.alpha_max, ctl.var_scale[l & 1], var);
       if (cluster == 0 && c == 0) {
         p.scalars[size_t(l) * 3 + 1] = mean;
         p.scalars[size_t(l) * 3 + 2] = var;
@@ -781,7 +808,7 @@ struct Step {
         }
         // One token's warp would need neither barrier; without any, the compiler threads the tail's branches into copies of its code.
         if (!FULL) bar_compute();
-        if (warp == (FULL ? 0 : WARPS - 1)) decay(l, sc[SC_VAR]);
+        if (warp == (FULL ? 0 : WARPS - 1)) decay(l);
         bar_compute();
       }
       // ---- LSF, residual, the norm that follows ----
@@ -869,6 +896,7 @@ __global__ void __launch_bounds__(THREADS, 1) step_cluster_kernel(const __grid_c
     }
     mbar_init(smem_u32(&ctl.p1_full), 1);
     mbar_init(smem_u32(&ctl.p1_empty), WARPS);
+    mbar_init(smem_u32(&ctl.p2_there), 1);
     mbar_init(smem_u32(&ctl.p2_full), 1);
     mbar_init(smem_u32(&ctl.p2_empty), WARPS);
     mbar_init(smem_u32(&ctl.got_o), 1);
@@ -886,6 +914,7 @@ __global__ void __launch_bounds__(THREADS, 1) step_cluster_kernel(const __grid_c
   const Step<FULL, STREAM> s{p, ctl, step_smem, smem_u32(step_smem), warp_index(), int(threadIdx.x & 31), int(cluster_rank()), cluster, n0,
                      FULL ? 1 : (cluster + 1) * p.N / p.n_clusters - n0, &ctl.abort_flag};
   if (s.warp == WARPS) s.produce();
+  else if (s.warp == WARPS + 1) s.settle();
   else s.compute();
   __syncwarp();
   cluster_arrive();
@@ -899,22 +928,17 @@ __global__ void __launch_bounds__(THREADS, 1) step_cluster_kernel(const __grid_c
 // (sign << 1) | nonzero, so that a shift and a mask give a bf16 pair of {0, +-2}.
 __global__ void __launch_bounds__(256)
 step_weights_kernel(const uint8_t* __restrict__ w_qkv, const uint8_t* __restrict__ w_out, const uint8_t* __restrict__ w1,
-                    const uint8_t* __restrict__ w2, const float* __restrict__ w_router, const float* __restrict__ gamma,
-                    const float* __restrict__ a_qkv, const float* __restrict__ a_out, const float* __restrict__ a1,
-                    const float* __restrict__ a2, const float* __restrict__ var_scale, uint8_t* __restrict__ out) {
+                    const uint8_t* __restrict__ w2, const float* __restrict__ gamma, const float* __restrict__ a_qkv,
+                    const float* __restrict__ a_out, const float* __restrict__ a1, const float* __restrict__ a2,
+                    uint8_t* __restrict__ out) {
   const int u = blockIdx.x, lane = threadIdx.x & 31, ch = threadIdx.x >> 5;
   uint4* dst = reinterpret_cast<uint4*>(out + size_t(u) * UNIT) + threadIdx.x;
-  if (u >= T_ROUTER + E) {
+  if (u >= T_END) {
     const int i = threadIdx.x;
     if (i >= SC_FLOATS) return;
     reinterpret_cast<float*>(out + size_t(u) * UNIT)[i] =
         i < SC_AQKV ? gamma[i] : i < SC_AOUT ? a_qkv[i - SC_AQKV] : i < SC_A1 ? a_out[0] : i < SC_A2 ? a1[i - SC_A1]
-        : i < SC_VAR ? a2[i - SC_A2] : i == SC_VAR ? var_scale[0] : 0.f;
-    return;
-  }
-  if (u >= T_ROUTER) {             // 16 bytes (i, half, lane): channels (32 i + lane) 8 + 4 half
-    const int i = ch >> 1, half = ch & 1;
-    *dst = *reinterpret_cast<const uint4*>(w_router + size_t(u - T_ROUTER) * C + (i * 32 + lane) * 8 + half * 4);
+        : i < SC_A2 + E ? a2[i - SC_A2] : 0.f;
     return;
   }
   const uint8_t* rows;
@@ -1021,13 +1045,13 @@ int step_clusters(int N, int most, bool carried) {
 }
 
 int launch_step_weights(const jb200_layer* y, int c, int h, int e, int hidden, void* out, cudaStream_t stream) {
-  JB_REQUIRE(y && out && y->w_qkv && y->w_out && y->w1 && y->w2 && y->w_router && y->gamma && y->a_qkv && y->a_out && y->a1 && y->a2 && y->var_scale,
+  JB_REQUIRE(y && out && y->w_qkv && y->w_out && y->w1 && y->w2 && y->gamma && y->a_qkv && y->a_out && y->a1 && y->a2,
              "step_weights: null pointer");
   JB_REQUIRE(step_weight_bytes(c, h, e, hidden) != 0, "step_weights: d_model %d / heads %d / experts %d x %d have no such form", c, h, e, hidden);
-  JB_REQUIRE(aligned16(out) && aligned16(y->w_router) && aligned16(y->w_qkv) && aligned16(y->w_out) && aligned16(y->w1) && aligned16(y->w2),
+  JB_REQUIRE(aligned16(out) && aligned16(y->w_qkv) && aligned16(y->w_out) && aligned16(y->w1) && aligned16(y->w2),
              "step_weights: pointers must be 16-byte aligned");
-  step_weights_kernel<<<T_ROUTER + E + 1, 256, 0, stream>>>(y->w_qkv, y->w_out, y->w1, y->w2, y->w_router, y->gamma, y->a_qkv, y->a_out, y->a1,
-                                                            y->a2, y->var_scale, static_cast<uint8_t*>(out));
+  step_weights_kernel<<<T_END + 1, 256, 0, stream>>>(y->w_qkv, y->w_out, y->w1, y->w2, y->gamma, y->a_qkv, y->a_out, y->a1, y->a2,
+                                                     static_cast<uint8_t*>(out));
   JB_LAUNCH_CHECK("step_weights_kernel");
   return JB200_OK;
 }
@@ -1089,7 +1113,7 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
       const jb200_layer& y = layers[l0 + i];
       StepLayer& d = p.layer[i];
       d.tiles = static_cast<const uint8_t*>(weights[l0 + i]);
-      d.w_norm1 = y.w_norm1; d.w_norm2 = y.w_norm2; d.mu = y.mu;
+      d.w_norm1 = y.w_norm1; d.w_norm2 = y.w_norm2; d.w_router = y.w_router; d.var_scale = y.var_scale; d.mu = y.mu;
       d.s_in = f->s_in ? f->s_in[l0 + i] : nullptr; d.s_out = f->s_out ? f->s_out[l0 + i] : nullptr;
       d.h_in = f->h_in ? f->h_in[l0 + i] : nullptr; d.h_out = f->h_out[l0 + i];
       d.eps1 = y.eps1; d.eps2 = y.eps2; d.alpha_min = y.alpha_min; d.alpha_max = y.alpha_max; d.balance_alpha = y.balance_alpha;

@@ -366,6 +366,32 @@ def test_a_captured_step_outlives_the_layer_table():
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("B", [1, 5, 13])
+def test_a_captured_step_follows_edits_in_place(B):
+    """Norms, router and var_scale are read from the parameters themselves, by the one-launch step as by the kernels."""
+    torch.manual_seed(12)
+    model = jm.ternary_init_(jm.Jarvis(vocab_size=320, d_model=1024, n_layers=2, n_heads=16, max_seq_len=64)).cuda().eval()
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    idx = torch.randint(0, 320, (B, 1), generator=gen, device="cuda")
+    state = {"h": [torch.randn(B, 1024, generator=gen, device="cuda") for _ in range(2)],
+             "S": [torch.randn(B, 16, 64, 64, generator=gen, device="cuda") for _ in range(2)]}
+    pos = torch.full((B,), 3, dtype=torch.int32, device="cuda")
+    session = jm.DecodeSession(model, {k: [s.clone() for s in v] for k, v in state.items()}, pos, 64).capture()
+    router, var_scale = model.blocks[0].moe.router.weight, model.blocks[1].liquid.var_scale
+    edits = [lambda: None, lambda: model.blocks[0].norm2.weight.mul_(1.5), lambda: router.copy_(router.flip(0)), lambda: var_scale.add_(2.0)]
+    seen = []
+    for edit in edits:
+        with torch.no_grad():
+            edit()
+        session.load_state(state, pos)
+        seen.append(session.step(idx).clone())
+        want, new = model.step(idx, pos, state, max_position=64)
+        assert torch.equal(seen[-1], want)
+        assert all(torch.equal(a, b) for a, b in zip(session.state["h"] + session.state["S"], new["h"] + new["S"]))
+    assert not any(torch.equal(a, b) for a, b in zip(seen, seen[1:]))
+    assert _lib.device_status() == 0
+
+
 def test_a_captured_step_outlives_its_angle_tables():
     """A longer prompt makes the model's angle tables anew; the graph goes on with those it was captured with."""
     torch.manual_seed(12)
