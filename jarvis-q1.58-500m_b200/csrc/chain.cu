@@ -61,7 +61,9 @@ constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // so 20 tokens 1015 -> 1008, 37 1052 -> 1047, 64 1110 -> 1122.  Steps of 64, 100, 128 sequences with q|k|v so 1094 -> 1070,
 // 1361 -> 1351, equal; their out-projection, behind the attention's stores, gets slower (64: 1094 -> 1114).
 constexpr int OUT_TILED_TOKENS = 128, QKV_TILED_PROMPT = 40, QKV_TILED_STEP = 100;
-// Up to here the first expert GEMM takes all rows for every expert and stores the routed ones: more MMAs, no dispatch.
+// Up to here the first expert GEMM takes all rows for every expert and stores the routed ones: more MMAs, no dispatch.  A token without
+// finite router logits is stored once, for expert 0, and its second hidden row holds whatever was there: combine and tail
+// take the first one's output for both assignments (stored twice by the GEMM, 64 sequences were 1.5 % slower).
 constexpr int ALL_ROWS_TOKENS = 64;
 // Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
 // tokens) that leaves a launch of so many rows in each group one wave.
@@ -246,11 +248,11 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const LsfStats stats = {acc, acc + 2, hist, E, N, (long long)N * C, p.balance_alpha, scalars,
                             p.mu, p.reflect_lam, p.reflect_tau, (f->reflect && p.mu) ? f->reflect + l : nullptr};
     if (h16 && N <= tail_max_tokens(C, T)) {
-      JB_TRY(launch_tail(y, gates, scatter, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
+      JB_TRY(launch_tail(y, gates, scatter, idx, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
                          w_next ? xn_next : nullptr, B, T, C, st));
       continue;
     }
-    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st, true));
+    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st, true, N <= ALL_ROWS_TOKENS ? idx : nullptr));
     if (h16 && T == 1) {
       JB_TRY(launch_lsf_step_norm(out, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
                                   w_next ? xn_next : nullptr, B, C, st, true));

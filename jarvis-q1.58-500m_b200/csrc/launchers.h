@@ -70,8 +70,10 @@ int launch_moe_metadata_static(const int64_t* topk_idx, int n_tokens, int K, int
                                cudaStream_t stream);
 int launch_dispatch_gather(const void* x_bf16, const int* gather_map, int M, int n_tokens, int C, void* dispatched,
                            cudaStream_t stream);
+// topk_idx (top-2 of a chain only, or null): a token whose second id is -1 takes its first row twice.
 int launch_scatter_combine(const void* y_bf16, const float* gates, const int* scatter_map, int n_tokens, int K, int C,
-                           void* out, int out_dtype, double* stats, cudaStream_t stream, bool ahead = false);
+                           void* out, int out_dtype, double* stats, cudaStream_t stream, bool ahead = false,
+                           const int64_t* topk_idx = nullptr);
 int launch_moe_finalize(const double* stats, const double* probs_sum, const int* top1_hist, int E, long long n_tokens,
                         long long n_elems, float balance_alpha, float* scalars, cudaStream_t stream);
 
@@ -114,9 +116,9 @@ int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const f
 int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router, int N, int C, int E,
                        int64_t* idx, float* gates, double* probs_sum, int* hist, int* ticket, int* counts, int* offsets,
                        int* scatter, int* gather, int* gate_idx, cudaStream_t stream);
-int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const LsfStats& st, const float* var_scale,
-                float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x, const float* w_norm, float eps,
-                void* xn_bf16, int B, int T, int C, cudaStream_t stream);
+int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const int64_t* idx, const LsfStats& st,
+                const float* var_scale, float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x,
+                const float* w_norm, float eps, void* xn_bf16, int B, int T, int C, cudaStream_t stream);
 // A single-token step of all layers in one launch (step_cluster.cu).  weights[l]: launch_step_weights' layout of layer l
 // (step_weight_bytes, 0 where there is no such form).  taken: false where the call is not one of its kind and nothing was done.
 size_t step_weight_bytes(int C, int H, int E, int hidden);

@@ -534,7 +534,8 @@ scatter_combine_kernel(const __nv_bfloat16* __restrict__ y, const float* __restr
 template <typename TOut>
 __global__ void __launch_bounds__(256)
 top2_combine_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ gates, const int* __restrict__ scatter_map,
-                    int n_tokens, int C, bool ahead, TOut* __restrict__ out, double* __restrict__ stats) {
+                    const int64_t* __restrict__ topk_idx, int n_tokens, int C, bool ahead, TOut* __restrict__ out,
+                    double* __restrict__ stats) {
   __shared__ float red[2][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tok = blockIdx.x * 8 + warp, M = 2 * n_tokens;
@@ -546,6 +547,7 @@ top2_combine_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict
     g = *(reinterpret_cast<const float2*>(gates) + tok);
     sl.x = sl.x < 0 ? 0 : (sl.x >= M ? M - 1 : sl.x);
     sl.y = sl.y < 0 ? 0 : (sl.y >= M ? M - 1 : sl.y);
+    if (topk_idx && topk_idx[2 * tok + 1] < 0) sl.y = sl.x;
   };
   if (ahead) route();
   __syncwarp();
@@ -788,7 +790,7 @@ int launch_dispatch_gather(const void* x_bf16, const int* gather_map, int M, int
 }
 
 int launch_scatter_combine(const void* y_bf16, const float* gates, const int* scatter_map, int n_tokens, int K, int C,
-                           void* out, int out_dtype, double* stats, cudaStream_t stream, bool ahead) {
+                           void* out, int out_dtype, double* stats, cudaStream_t stream, bool ahead, const int64_t* topk_idx) {
   JB_REQUIRE(n_tokens >= 0 && K >= 1 && K <= 8 && C > 0 && C % 8 == 0, "scatter_combine: bad shape");
   JB_REQUIRE(out_dtype == 0 || out_dtype == 1, "scatter_combine: out_dtype must be 0 (f32) or 1 (bf16)");
   if (n_tokens == 0) return JB200_OK;
@@ -799,10 +801,10 @@ int launch_scatter_combine(const void* y_bf16, const float* gates, const int* sc
   if (K == 2 && C <= 1024 && (reinterpret_cast<uintptr_t>(gates) & 7u) == 0 && (reinterpret_cast<uintptr_t>(scatter_map) & 7u) == 0) {
     const __nv_bfloat16* y = reinterpret_cast<const __nv_bfloat16*>(y_bf16);
     if (out_dtype == 1)
-      launch_dep(top2_combine_kernel<__nv_bfloat16>, blocks, 256, 0, stream, y, gates, scatter_map, n_tokens, C, ahead,
+      launch_dep(top2_combine_kernel<__nv_bfloat16>, blocks, 256, 0, stream, y, gates, scatter_map, topk_idx, n_tokens, C, ahead,
                  reinterpret_cast<__nv_bfloat16*>(out), stats);
     else
-      launch_dep(top2_combine_kernel<float>, blocks, 256, 0, stream, y, gates, scatter_map, n_tokens, C, ahead,
+      launch_dep(top2_combine_kernel<float>, blocks, 256, 0, stream, y, gates, scatter_map, topk_idx, n_tokens, C, ahead,
                  reinterpret_cast<float*>(out), stats);
     JB_LAUNCH_CHECK("top2_combine_kernel");
     return JB200_OK;

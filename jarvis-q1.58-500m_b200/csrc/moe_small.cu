@@ -126,6 +126,7 @@ struct TailParams {
   const __nv_bfloat16* y;      // [2N][C] expert outputs in dispatch order: the only input the kernel before this one made
   const float* gates;          // [N][2]
   const int* scatter;          // [N][2]
+  const int64_t* idx;          // [N][2]
   LsfStats st;                 // stats is not read: the sums are made here
   double inv_tokens;
   const float* var_scale;
@@ -141,6 +142,14 @@ struct TailParams {
 
 constexpr int MAX_CTAS = 8;
 constexpr int MAX_WARPS = TAIL_MAX / MAX_CTAS;         // tokens per CTA: one warp each
+
+// Slots of a token's two expert rows.  Without finite logits (idx -1) both are expert 0's, and a GEMM that takes all rows for every
+// expert has made the first of them alone.
+__device__ __forceinline__ int2 tail_slots(const TailParams& p, int n) {
+  int2 s = *reinterpret_cast<const int2*>(p.scatter + 2 * n);
+  if (p.idx[2 * n + 1] < 0) s.y = s.x;
+  return s;
+}
 
 // The combined row of one token: put(i, 8 values rounded to bf16) for every group; the sums of the unrounded ones over the warp.
 template <typename F>
@@ -228,7 +237,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailPar
   int2 sl = make_int2(0, 0);
   float2 g = make_float2(0.f, 0.f);
   if (on) {
-    sl = *reinterpret_cast<const int2*>(p.scatter + 2 * n);
+    sl = tail_slots(p, n);
     g = *reinterpret_cast<const float2*>(p.gates + 2 * n);
 #pragma unroll
     for (int i = 0; i < GROUPS; ++i) {
@@ -308,7 +317,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   int2 sl = make_int2(0, 0);
   float2 g = make_float2(0.f, 0.f);
   if (on) {
-    sl = *reinterpret_cast<const int2*>(p.scatter + 2 * own);
+    sl = tail_slots(p, own);
     g = *reinterpret_cast<const float2*>(p.gates + 2 * own);
   }
   for (int i = tid; i < B * SCAN_CH / 4; i += threads) {
@@ -503,13 +512,13 @@ int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_
   return JB200_OK;
 }
 
-int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const LsfStats& st, const float* var_scale,
-                float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x, const float* w_norm, float eps,
-                void* xn_bf16, int B, int T, int C, cudaStream_t stream) {
+int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const int64_t* idx, const LsfStats& st,
+                const float* var_scale, float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x,
+                const float* w_norm, float eps, void* xn_bf16, int B, int T, int C, cudaStream_t stream) {
   const int N = B * T;
   JB_REQUIRE(N >= 1 && N <= tail_max_tokens(C, T) && C % 128 == 0 && C <= 1024, "tail: bad shape (B=%d, T=%d, C=%d)", B, T, C);
   TailParams p;
-  p.y = reinterpret_cast<const __nv_bfloat16*>(y_bf16); p.gates = gates; p.scatter = scatter; p.st = st;
+  p.y = reinterpret_cast<const __nv_bfloat16*>(y_bf16); p.gates = gates; p.scatter = scatter; p.idx = idx; p.st = st;
   p.inv_tokens = 1.0 / double(st.n_tokens);
   p.var_scale = var_scale; p.alpha_min = alpha_min; p.alpha_max = alpha_max;
   p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;

@@ -85,6 +85,7 @@ struct Ctl {
   alignas(8) float gates2[MAX_TOKENS][2];
   alignas(8) uint32_t word[32];
   int expert[MAX_TOKENS][2];                         // two different ones
+  uint32_t second[MAX_TOKENS];                       // where the second assignment's row is, after the first one's
   float alpha, var_scale[2];
   uint32_t abort_flag;
   int last;
@@ -545,7 +546,10 @@ struct Step {
       const float gate = (lane ? p1 : p0) / (p0 + p1 + 1e-8f);
       const int id = lane ? i1 : i0;
       ctl.gates2[warp][lane] = gate;
-      ctl.expert[warp][lane] = lane && (i1 < 0 || i1 == i0) ? (i0 + 1) % E : id;      // NaN logits: any other one
+      // NaN logits: both assignments are expert i0's, as in the maps.  Two different ones run all the same, which the exchanges count on;
+      // the other one's row is not read.
+      ctl.expert[warp][lane] = id < 0 ? (i0 + 1) % E : id;
+      if (lane) ctl.second[warp] = id < 0 ? 0u : 2u * C;
       if (c == 0) {
         uint8_t* r = p.routing + l * p.routing_stride;
         const size_t at = size_t(n0 + warp) * 2 + lane;
@@ -566,10 +570,11 @@ struct Step {
     uint8_t* row = smem + p.o_ry + warp * (C * 4) + lane * 16;
     const float2 gate = *reinterpret_cast<const float2*>(ctl.gates2[warp]);
     const uint64_t ga = f32x2(gate.x, gate.x), gb = f32x2(gate.y, gate.y);
+    const uint8_t* row_b = row + ctl.second[warp];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll 1
     for (int i = 0; i < GROUPS; ++i) {
-      const uint4 a = *reinterpret_cast<const uint4*>(row + i * 512), b = *reinterpret_cast<const uint4*>(row + 2 * C + i * 512);
+      const uint4 a = *reinterpret_cast<const uint4*>(row + i * 512), b = *reinterpret_cast<const uint4*>(row_b + i * 512);
       auto one = [&](uint32_t wa, uint32_t wb) {
         float lo, hi;
         f32x2_split(fma_f32x2(gb, f32x2(bf16_lo(wb), bf16_hi(wb)), mul_f32x2(ga, f32x2(bf16_lo(wa), bf16_hi(wa)))), lo, hi);

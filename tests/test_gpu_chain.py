@@ -423,6 +423,36 @@ def test_dispatch_maps_of_tokens_whose_router_is_nan(N):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("B,T,C", [(1, 1, 1024), (3, 1, 1024), (8, 1, 1024), (13, 1, 1024), (56, 1, 1024), (64, 1, 1024), (1, 3, 1024),
+                                   (1, 16, 1024), (2, 20, 1024), (1, 64, 1024), (1, 65, 1024), (2, 150, 1024), (7, 1, 128), (2, 20, 128)])
+def test_both_assignments_of_a_token_whose_router_is_nan_run(B, T, C):
+    """Logits that overflow where everything else of the token is finite: its two assignments are expert 0's, as the maps say, in every
+    form, and the other tokens of the call do not notice."""
+    torch.manual_seed(9)
+    model = jm.ternary_init_(jm.Jarvis(vocab_size=320, d_model=C, n_layers=2, n_heads=C // 64, max_seq_len=512)).cuda().eval()
+    with torch.no_grad():
+        model.tok_emb.weight[:, 0] = 0.0                           # token 7 alone has a channel that overflows in the first router
+        model.tok_emb.weight[7, 0] = 5.0
+        model.blocks[0].attn.out_proj.weight[0] = 0.0
+        model.blocks[0].moe.router.weight[:, 0] = 3e38
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    idx = torch.randint(8, 320, (B, T), generator=gen, device="cuda")
+    idx.view(-1)[B * T // 2] = 7
+    state = {"h": [torch.randn(B, C, generator=gen, device="cuda") for _ in range(2)],
+             "S": [torch.randn(B, C // 64, 64, 64, generator=gen, device="cuda") for _ in range(2)]}
+    pos = torch.full((B,), 3, dtype=torch.int32, device="cuda")
+    got = []
+    for model.use_chain in (False, True, True):                    # twice: the one-launch step lays its weights out first
+        logits, st = model.step(idx, pos, state, max_position=512)
+        ids, _, maps = model.blocks[0].moe.last_routing
+        got.append([logits, torch.stack(st["h"]), torch.stack(st["S"]), ids, *maps])
+    assert got[0][3].view(-1, 2)[B * T // 2].tolist() == [0, -1] and int((got[0][3] < 0).sum()) == 1
+    assert all(bool(torch.isfinite(t).all()) for t in got[0][:3])
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("B,layers,states,skew", [(1, 3, True, 0.0), (1, 2, False, 0.0), (2, 34, True, 0.0), (3, 3, True, 3.0), (3, 2, False, 0.0),
                                                   (4, 3, True, 0.0), (7, 3, True, 3.0), (8, 3, True, 0.0), (13, 3, True, 3.0),
                                                   (15, 3, True, 0.0), (29, 2, True, 0.0), (49, 3, True, 3.0), (56, 3, True, 0.0),
