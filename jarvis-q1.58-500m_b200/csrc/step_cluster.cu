@@ -974,8 +974,8 @@ struct Plan {
   uint32_t o_p1, o_p2, o_sc, o_rx, o_ry, o_xn, o_rh, o_qkv, o_ho, o_cs, o_scr, o_ring;
   size_t smem;
 };
-Plan plan_of(int tokens, bool full) {
-  Plan s;
+constexpr Plan plan_of(int tokens, bool full) {
+  Plan s = {};
   uint32_t at = 0;
   auto take = [&](size_t n) { const uint32_t o = at; at += uint32_t((n + 127) / 128 * 128); return o; };
   s.o_p1 = take(C * 4);
@@ -995,6 +995,10 @@ Plan plan_of(int tokens, bool full) {
   s.smem = at + size_t(s.units) * UNIT;
   return s;
 }
+// unit_wait goes by parity, so the unit two turns before the awaited one must have been given back.  The producer works in order: what is a
+// ring before the warp's last unit has been.  The two are at most sixteen units apart (32 with a token per cluster, where a
+// warp may have no tile of a used expert; block barriers between them only help), hence rings of no fewer.
+static_assert(plan_of(MAX_TOKENS, false).units >= 16 && plan_of(1, true).units >= 32, "the ring is too short for waits by parity");
 
 bool stream_sums(int N) { return N * CTAS >= 64; }      // launch_attn_scan's choice
 
