@@ -170,7 +170,8 @@ class LayerTable:
 
     def step_weights(self, B: int):
         """The layers' weights as the one-launch step of B sequences reads them (host array of device pointers), laid out when first
-        wanted; None where there is no such step.  Not made inside a stream capture, which would only record the work."""
+        wanted; None where there is no such step, or no memory for them when that was.  Not made inside a stream capture, which would
+        only record the work."""
         lib = _lib.load()
         if B > lib.jb200_step_max_sequences():
             return None
@@ -180,7 +181,11 @@ class LayerTable:
                 return None
             with _step_lock:
                 if self._step is None:
-                    buf = torch.empty((self.n, nbytes), dtype=torch.uint8, device=self.device)
+                    try:
+                        buf = torch.empty((self.n, nbytes), dtype=torch.uint8, device=self.device)
+                    except torch.OutOfMemoryError:       # the kernels need none; not tried again, a failing allocation is slow
+                        self._step = None, None
+                        return None
                     for d, out in zip(self.array, buf):
                         _lib.check(lib.jb200_prepare_step_weights(C.byref(d), self.C, self.H, self.E, self.hidden, out.data_ptr(),
                                                                   ops._stream()), "jb200_prepare_step_weights")

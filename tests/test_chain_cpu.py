@@ -3,6 +3,7 @@ import copy
 import ctypes as C
 import gc
 import pickle
+import types
 import weakref
 
 import pytest
@@ -226,3 +227,44 @@ def test_which_single_token_steps_run_in_one_launch():
     assert [lib.jb200_step_clusters(B, 7, 0) for B in range(1, 6)] == [1, 2, 3, 0, 0]
     assert [lib.jb200_step_clusters(B, 1, 1) for B in (1, 2, 3, 4, 8, 9)] == [1, 0, 0, 1, 1, 0]
     assert [lib.jb200_step_clusters(B, 2, c) for B in (2, 3) for c in (0, 1)] == [2, 2, 0, 0]
+
+
+class _StepLibrary:
+    """The library with a one-launch step of layouts of 64 bytes; counts the layers that are laid out."""
+
+    def __init__(self, lib):
+        self._lib, self.laid = lib, 0
+
+    def __getattr__(self, name):
+        return getattr(self._lib, name)
+
+    def jb200_step_max_sequences(self):
+        return 56
+
+    def jb200_step_weight_bytes(self, *sizes):
+        return 64
+
+    def jb200_prepare_step_weights(self, *args):
+        self.laid += 1
+        return _lib.OK
+
+
+@pytest.fixture
+def step_library(tables_on_cpu, monkeypatch):
+    lib = _StepLibrary(_lib.load())
+    monkeypatch.setattr(_lib, "load", lambda: lib)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: types.SimpleNamespace(synchronize=lambda: None))
+    return lib
+
+
+def test_without_memory_for_a_second_layout_steps_go_kernel_by_kernel(step_library, monkeypatch):
+    blocks = [jm.JarvisBlock(128, 2).eval() for _ in range(2)]
+    tab, asked = chain.LayerTable(blocks), []
+
+    def empty(*a, **k):
+        asked.append(a)
+        raise torch.OutOfMemoryError("out of memory")
+    monkeypatch.setattr(chain.torch, "empty", empty)
+    assert tab.step_weights(1) is None and tab.step_weights(1) is None and len(asked) == 1
