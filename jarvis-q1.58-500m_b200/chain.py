@@ -66,13 +66,15 @@ def _fits(b, a, d_model, hidden, E) -> bool:
 
 
 _step_lock = threading.Lock()
+_LAID_OUT = ("w_qkv", "a_qkv", "w_out", "a_out", "w1", "a1", "w2", "a2", "gamma")      # what a layer's second layout is made of
 
 
 class LayerTable:
     """jb200_layer array of `blocks`, valid as long as every parameter it was built from is the same unmodified tensor in
     the same place (identity, storage and version are compared on every call: 16 tensors per layer, ~0.1 us each)."""
 
-    def __init__(self, blocks):
+    def __init__(self, blocks, before: Optional["LayerTable"] = None):
+        """before: the table that this one takes the place of; layers whose packed weights are still its keep their second layout."""
         from .modules import ReflectivePenalty, _f32
         blocks = list(blocks)
         # weak: a block may own its table, and a cycle would keep a dropped model's memory until the next collection
@@ -106,6 +108,10 @@ class LayerTable:
             self._keep.append(tensors)
             d.eps1, d.eps2, d.balance_alpha = b.norm1.eps, b.norm2.eps, moe.balance_alpha
             d.alpha_min, d.alpha_max = lq.alpha_min, lq.alpha_max
+        self._laid = [None] * self.n
+        if before is not None and before.device == self.device:
+            same = [all(a[k] is b[k] for k in _LAID_OUT) for a, b in zip(self._keep, before._keep)]
+            self._laid = [t if ok else None for t, ok in zip(before._laid, same)] + [None] * (self.n - len(same))
 
     def __reduce__(self):
         """Addresses mean nothing in a copy: a copied, saved or sent module makes its own table."""
@@ -181,17 +187,21 @@ class LayerTable:
                 return None
             with _step_lock:
                 if self._step is None:
+                    laid = list(self._laid)
+                    new = [i for i, t in enumerate(laid) if t is None]
                     try:
-                        buf = torch.empty((self.n, nbytes), dtype=torch.uint8, device=self.device)
+                        buf = torch.empty((len(new), nbytes), dtype=torch.uint8, device=self.device)
                     except torch.OutOfMemoryError:       # the kernels need none; not tried again, a failing allocation is slow
-                        self._step = None, None
+                        self._step = (None,)
                         return None
-                    for d, out in zip(self.array, buf):
-                        _lib.check(lib.jb200_prepare_step_weights(C.byref(d), self.C, self.H, self.E, self.hidden, out.data_ptr(),
-                                                                  ops._stream()), "jb200_prepare_step_weights")
-                    torch.cuda.current_stream(self.device).synchronize()      # any stream may be the next to read them
-                    self._step = buf, _pointers(self.n, buf)
-        return self._step[1]
+                    for i, out in zip(new, buf):
+                        _lib.check(lib.jb200_prepare_step_weights(C.byref(self.array[i]), self.C, self.H, self.E, self.hidden,
+                                                                  out.data_ptr(), ops._stream()), "jb200_prepare_step_weights")
+                        laid[i] = out
+                    if new:
+                        torch.cuda.current_stream(self.device).synchronize()      # any stream may be the next to read them
+                    self._laid, self._step = laid, (_pointers(self.n, laid),)
+        return self._step[0]
 
     def sizes(self, B: int, T: int):
         key = (B, T)
@@ -214,7 +224,7 @@ def table_of(owner, blocks) -> Optional[LayerTable]:
         if not supported(blocks):
             return None
         try:
-            tab = LayerTable(blocks)
+            tab = LayerTable(blocks, tab)
         except KeyError:             # a weight that is no plain parameter (parametrised, pruned): read it anew on every call
             return None
         owner.__dict__["_layer_table"] = tab

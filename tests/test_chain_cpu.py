@@ -268,3 +268,28 @@ def test_without_memory_for_a_second_layout_steps_go_kernel_by_kernel(step_libra
         raise torch.OutOfMemoryError("out of memory")
     monkeypatch.setattr(chain.torch, "empty", empty)
     assert tab.step_weights(1) is None and tab.step_weights(1) is None and len(asked) == 1
+
+
+def test_an_edited_layer_alone_is_laid_out_again(step_library):
+    blocks = [jm.JarvisBlock(128, 2).eval() for _ in range(3)]
+    owner = torch.nn.Module()
+
+    def layouts():
+        tab = chain.table_of(owner, blocks)
+        return list(tab.step_weights(1)), tab
+    first, tab = layouts()
+    assert step_library.laid == 3 and len(set(first)) == 3 and layouts()[1] is tab
+    with torch.no_grad():                    # read from the parameters themselves
+        for p in (blocks[0].norm1.weight, blocks[1].moe.router.weight, blocks[2].liquid.var_scale):
+            p.mul_(1.5)
+    second, other = layouts()
+    assert other is not tab and second == first and step_library.laid == 3
+    with torch.no_grad():
+        blocks[1].moe.w2[3].weight.mul_(1.5)
+        blocks[2].attn.gamma_raw.add_(1.0)
+    third, _ = layouts()
+    assert step_library.laid == 5 and third[0] == first[0] and third[1] != first[1] and third[2] != first[2]
+    held = [weakref.ref(tab), weakref.ref(other)]
+    del tab, other
+    gc.collect()
+    assert all(ref() is None for ref in held)            # a table does not keep the one before it
