@@ -248,8 +248,8 @@ int jb200_moe_metadata_static(const int64_t* topk_idx, int N, int K, int E, int3
 int jb200_moe_dispatch_gather(const void* x, const int32_t* gather_map, int M, int N, int C, void* dispatched,
                               void* stream);
 
-/* Both at once for top-2 assignments of up to 131,072 tokens, 4 or 8 experts, C <= 1024 (multiple of 8): the maps of
- * jb200_moe_metadata and the rows of jb200_moe_dispatch_gather, in two launches and with every row read once.
+/* Both in one call for top-2 assignments, 4 or 8 experts, C <= 1024 (multiple of 8): the maps of
+ * jb200_moe_metadata and the rows of jb200_moe_dispatch_gather; beyond a thousand tokens with every row read once.
  * scratch: jb200_moe_dispatch_scratch_bytes, 16-byte aligned. */
 size_t jb200_moe_dispatch_scratch_bytes(int n_tokens, int E);
 int jb200_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int32_t* expert_counts,

@@ -426,12 +426,12 @@ int jb200_lsf_step_norm(const void* m_bf16, const double* stats, const double* p
                               static_cast<cudaStream_t>(stream));
 }
 
-size_t jb200_moe_dispatch_scratch_bytes(int n_tokens, int E) { return n_tokens > 0 && E > 0 ? moe_dispatch_count_bytes(n_tokens, E) : 0; }
+size_t jb200_moe_dispatch_scratch_bytes(int n_tokens, int E) { return n_tokens > 0 && E > 0 ? moe_dispatch_scratch_bytes(n_tokens, E) : 0; }
 
 int jb200_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int32_t* expert_counts,
                        int32_t* expert_offsets, int32_t* scatter_map, int32_t* gather_map, int32_t* gate_idx_map, void* dispatched,
                        void* scratch, void* stream) {
-  return launch_moe_dispatch(topk_idx, x_bf16, n_tokens, C, E, static_cast<int*>(scratch), expert_counts, expert_offsets, scatter_map,
+  return launch_moe_dispatch(topk_idx, x_bf16, n_tokens, C, E, scratch, expert_counts, expert_offsets, scatter_map,
                              gather_map, gate_idx_map, dispatched, static_cast<cudaStream_t>(stream));
 }
 

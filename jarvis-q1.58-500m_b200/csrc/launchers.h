@@ -57,10 +57,9 @@ int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* 
                           int n_tokens, int C, int E, int64_t* topk_idx, float* gates, double* probs_sum,
                           int* top1_hist, cudaStream_t stream, bool ahead = false);
 size_t moe_metadata_scratch_bytes(int n_tokens, int K, int E);
-// Maps and rows of top-2 assignments at once.  chunk_counts: moe_dispatch_count_bytes of scratch.
-constexpr int DISPATCH_MAX = 131072;   // tokens: beyond, the counts that every CTA adds up are more than its rows
-size_t moe_dispatch_count_bytes(int n_tokens, int E);
-int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int* chunk_counts, int* expert_counts,
+// Maps and rows of top-2 assignments at once.  scratch: moe_dispatch_scratch_bytes.
+size_t moe_dispatch_scratch_bytes(int n_tokens, int E);
+int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, void* scratch, int* expert_counts,
                         int* expert_offsets, int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream);
 int launch_moe_metadata(const int64_t* topk_idx, int n_tokens, int K, int E, int* expert_counts, int* expert_offsets,
                         int* scatter_map, int* gather_map, int* gate_idx_map, void* scratch, cudaStream_t stream);

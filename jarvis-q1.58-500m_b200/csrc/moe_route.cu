@@ -359,17 +359,17 @@ dispatch_hist_kernel(const int64_t* __restrict__ topk_idx, int M, int* __restric
   if (threadIdx.x < E) chunk_counts[blockIdx.x * E + threadIdx.x] = h[threadIdx.x];
 }
 
-// One CTA per chunk of 32 tokens, or of 64 where that leaves few counts and CTAs enough.  Every CTA adds up the counts of the chunks
-// before its own (at most 32 KB from L2), ranks its assignments with ballots - the order of the kernels above - and copies its rows:
-// each is read once and stored at both of its slots.  For an MoE layer called by itself, in the place of histogram, scan, assignment
-// and gather: launches of ~3 us (and ~10 us of host time each) around a copy that read every row twice.  The layer alone: 260 tokens 128 -> 89 us,
-// 1000 129 -> 90, 8000 150.8 -> 148.5, 65,536 899 -> 880.  Inside the native call the separate kernels stay: there the products read the segments while the kernel ahead of them
-// still runs, which this one makes; with the segments left by the router instead, 300 tokens 1564 -> 1690 us and 8 x 2048 12.9 -> 13.3 ms.
+// One CTA per chunk of 32 tokens, or of 64 where that leaves few counts and CTAs enough.  Every CTA adds up the counts of all
+// chunks (E integers each, from L2), ranks its assignments with ballots - the order of the kernels above - and copies its rows:
+// each is read once and stored at both of its slots, where the gather reads every row twice.  For an MoE layer called by itself;
+// sizes and times at one_launch_dispatch.  Inside the native call the separate kernels stay: there the products read the
+// segments while the kernel ahead of them still runs, which this one makes; with the segments left by the router instead,
+// 300 tokens 1564 -> 1690 us and 8 x 2048 12.9 -> 13.3 ms.
 template <int E, int TOK>
 __global__ void __launch_bounds__(DISP_THREADS)
-dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __restrict__ x, const int* __restrict__ chunk_counts, int n_tokens, int C, int* __restrict__ expert_counts, int* __restrict__ expert_offsets,
-                int* __restrict__ scatter_map, int* __restrict__ gather_map, int* __restrict__ gate_idx_map,
-                __nv_bfloat16* __restrict__ dispatched) {
+dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __restrict__ x, const int* __restrict__ chunk_counts,
+                int n_tokens, int C, int* __restrict__ expert_counts, int* __restrict__ expert_offsets, int* __restrict__ scatter_map,
+                int* __restrict__ gather_map, int* __restrict__ gate_idx_map, __nv_bfloat16* __restrict__ dispatched) {
   constexpr int WARPS = DISP_THREADS / 32, RANK_WARPS = 2 * TOK / 32, PER_WARP = TOK / WARPS;
   __shared__ int red[WARPS][2 * E], in_warp[RANK_WARPS][E], slots[2 * TOK];
   pdl_wait();
@@ -680,29 +680,44 @@ size_t moe_metadata_scratch_bytes(int n_tokens, int K, int E) {
 }
 
 namespace {
+// Where the metadata are one CTA's work, metadata and gather are two launches as well, and shorter ones; beyond, they are four, which a
+// layer called by itself pays for on the host up to some 8000 tokens (4000 tokens 137 us, 133 with two).  Device time of metadata and
+// gather -> histogram and dispatch_kernel: 4 experts, 1024 channels: 300 tokens 3.8 -> 7.4 us, 1024 5.2 -> 7.5, 4096 8.2 -> 8.0, 8192
+// 11.3 -> 11.2, 16,384 18.4 -> 18.9, 32,768 43.7 -> 41.1, 65,536 88.5 -> 71.0, 131,072 170 -> 135, 262,144 333 -> 261, 524,288 659 -> 537.
+// 8 experts, 512 channels (twice the counts, half the rows): 16,384 12.4 -> 14.5, 32,768 equal, 131,072 102 -> 84, 262,144 206 -> 195, 524,288
+// 408 -> 494: every CTA adds up all counts.
+constexpr int DISPATCH_MAX = 262144;
+bool one_launch_dispatch(int n_tokens) { return 2 * n_tokens > META_SMALL_MAX && n_tokens <= DISPATCH_MAX; }
 int dispatch_tokens(int n_tokens) { return n_tokens <= 16384 ? 32 : 64; }      // per CTA: 8000 tokens fill the chip only with the smaller
+int dispatch_chunks(int n_tokens) { return (n_tokens + dispatch_tokens(n_tokens) - 1) / dispatch_tokens(n_tokens); }
 }  // namespace
 
-size_t moe_dispatch_count_bytes(int n_tokens, int E) {
-  const int t = dispatch_tokens(n_tokens);
-  return size_t((n_tokens + t - 1) / t) * E * sizeof(int);
+size_t moe_dispatch_scratch_bytes(int n_tokens, int E) {
+  return one_launch_dispatch(n_tokens) ? size_t(dispatch_chunks(n_tokens)) * E * sizeof(int) : moe_metadata_scratch_bytes(n_tokens, 2, E);
 }
 
-int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int* chunk_counts, int* expert_counts,
+int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, void* scratch, int* expert_counts,
                         int* expert_offsets, int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream) {
-  JB_REQUIRE(n_tokens >= 1 && n_tokens <= DISPATCH_MAX && (E == 4 || E == 8) && C >= 8 && C % 8 == 0 && C <= 1024,
+  JB_REQUIRE(n_tokens >= 1 && n_tokens < (1 << 30) && (E == 4 || E == 8) && C >= 8 && C % 8 == 0 && C <= 1024,
              "moe_dispatch: bad shape (N=%d, C=%d, E=%d)", n_tokens, C, E);
-  JB_REQUIRE(topk_idx && x_bf16 && chunk_counts && expert_counts && expert_offsets && scatter_map && gather_map && gate_idx_map && dispatched,
+  JB_REQUIRE(topk_idx && x_bf16 && scratch && expert_counts && expert_offsets && scatter_map && gather_map && gate_idx_map && dispatched,
              "moe_dispatch: null pointer");
-  JB_REQUIRE(aligned16(x_bf16) && aligned16(dispatched) && aligned16(chunk_counts), "moe_dispatch: pointers must be 16-byte aligned");
-  const int tok = dispatch_tokens(n_tokens), blocks = (n_tokens + tok - 1) / tok;
+  JB_REQUIRE(aligned16(x_bf16) && aligned16(dispatched) && aligned16(scratch), "moe_dispatch: pointers must be 16-byte aligned");
+  if (!one_launch_dispatch(n_tokens)) {
+    const int rc = launch_moe_metadata(topk_idx, n_tokens, 2, E, expert_counts, expert_offsets, scatter_map, gather_map, gate_idx_map,
+                                       scratch, stream);
+    return rc == JB200_OK ? launch_dispatch_gather(x_bf16, gather_map, 2 * n_tokens, n_tokens, C, dispatched, stream) : rc;
+  }
+  const int tok = dispatch_tokens(n_tokens), blocks = dispatch_chunks(n_tokens);
+  int* chunk_counts = static_cast<int*>(scratch);
   const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(x_bf16);
   __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(dispatched);
   auto hist = tok == 32 ? (E == 4 ? dispatch_hist_kernel<4, 32> : dispatch_hist_kernel<8, 32>)
                         : (E == 4 ? dispatch_hist_kernel<4, 64> : dispatch_hist_kernel<8, 64>);
   launch_dep(hist, blocks, 2 * tok, 0, stream, topk_idx, 2 * n_tokens, chunk_counts);
   JB_LAUNCH_CHECK("dispatch_hist_kernel");
-  auto kernel = tok == 32 ? (E == 4 ? dispatch_kernel<4, 32> : dispatch_kernel<8, 32>) : (E == 4 ? dispatch_kernel<4, 64> : dispatch_kernel<8, 64>);
+  auto kernel = tok == 32 ? (E == 4 ? dispatch_kernel<4, 32> : dispatch_kernel<8, 32>)
+                          : (E == 4 ? dispatch_kernel<4, 64> : dispatch_kernel<8, 64>);
   launch_dep(kernel, blocks, DISP_THREADS, 0, stream, topk_idx, x, chunk_counts, n_tokens, C, expert_counts, expert_offsets, scatter_map,
              gather_map, gate_idx_map, d);
   JB_LAUNCH_CHECK("dispatch_kernel");

@@ -325,7 +325,7 @@ class SparseMoELayer(nn.Module):
         disp = None
         if meta_in_slab:
             meta = ops.moe_metadata(idx, E, gather_out=ep.ex.gmap[:N * self.top_k], offsets_out=ep.ex.offs[:E + 1])
-        elif ep is None and 256 < N <= ops.DISPATCH_MAX and C <= 1024:
+        elif ep is None and N > 0 and C <= 1024:
             meta, disp = ops.moe_dispatch(xn_rows, idx, E)
         else:
             meta = ops.moe_metadata(idx, E)

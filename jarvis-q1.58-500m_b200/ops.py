@@ -424,11 +424,8 @@ def dispatch_gather(x: torch.Tensor, gather_map: torch.Tensor) -> torch.Tensor:
     return out
 
 
-DISPATCH_MAX = 131072      # tokens of moe_dispatch
-
-
 def moe_dispatch(x: torch.Tensor, topk_idx: torch.Tensor, num_experts: int):
-    """moe_metadata and dispatch_gather of top-2 assignments at once: ((counts, offsets, scatter, gather, gate_idx), rows)."""
+    """moe_metadata and dispatch_gather of top-2 assignments in one call: ((counts, offsets, scatter, gather, gate_idx), rows)."""
     lib = _lib.load()
     _need(x, torch.bfloat16, "moe_dispatch.x")
     _need(topk_idx, torch.int64, "moe_dispatch.topk_idx")

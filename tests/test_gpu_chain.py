@@ -522,3 +522,17 @@ def test_dispatch_in_one_launch_against_metadata_and_gather(N, E, C):
     with pytest.raises(RuntimeError):
         ops.moe_dispatch(x, idx[:, :1].contiguous(), E)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("E,C", [(4, 1024), (8, 136)])
+@pytest.mark.parametrize("N", [1024, 1025, 16384, 16385, 262144, 262145])
+def test_dispatch_around_the_sizes_of_its_one_launch_form(N, E, C):
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    first = torch.randint(0, E, (N,), generator=gen, device="cuda")
+    idx = torch.stack([first, (first + torch.randint(1, E, (N,), generator=gen, device="cuda")) % E], 1)
+    idx[N // 2, 1] = -1
+    x = torch.randn(N, C, generator=gen, device="cuda").bfloat16()
+    got, rows = ops.moe_dispatch(x, idx, E)
+    want = ops.moe_metadata(idx, E)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(rows, ops.dispatch_gather(x, want[3]))
+    assert _lib.device_status() == 0
