@@ -55,11 +55,13 @@ struct Workspace {
 // MID_TOKENS the tcgen05 form that is built for latency (640 tokens 1.96 against 2.08 ms, 900 2.20 against 2.29, 1000 equal,
 // 1152 2.81 against 2.74), beyond that the persistent pipeline.
 constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
-// The products of the attention have few out-features: the tcgen05 form runs them on 8 to 24 SMs.  mma.sync with the token tiles side
-// by side (8 rows each for prompts, 16 for steps) fills the chip, and its chain over K is shorter.  24 layers and head as a graph: prompts
-// of 37, 64, 100 tokens with the out-projection so 1052 -> 1035, 1110 -> 1096, 1322 -> 1287 us, 180 equal, 256 1402 -> 1447; with q|k|v
-// so 20 tokens 1015 -> 1008, 37 1052 -> 1047, 64 1110 -> 1122.  Steps of 64, 100, 128 sequences with q|k|v so 1094 -> 1070,
-// 1361 -> 1351, equal; their out-projection, behind the attention's stores, gets slower (64: 1094 -> 1114).
+// The products of the attention have few out-features: the tcgen05 form runs them on 8 to 24 SMs.  mma.sync with the token tiles
+// side by side (8 rows each for prompts, 16 for steps) fills the chip, and its chain over K is shorter.  24 layers and head as a
+// graph: prompts of 37, 64, 100 tokens with the out-projection so 1052 -> 1035, 1110 -> 1096, 1322 -> 1287 us, 180 equal, 256
+// 1402 -> 1447; on top of that with q|k|v so 17 tokens 995 -> 966, 24 1008 -> 977, 32 1024 -> 1010, 40 1038 -> 1020; 41 to
+// 64 between 1 % faster and 1.6 % slower, by the GPU (48: 1053 -> 1048 on one, 1046 -> 1054 on another); 80 1256 -> 1282, 128
+// 1375 -> 1430.  Steps of 64, 100, 128 sequences with q|k|v so 1094 -> 1070, 1361 -> 1351, equal; their out-projection, behind the
+// attention's stores, gets slower (64: 1094 -> 1114).
 constexpr int OUT_TILED_TOKENS = 128, QKV_TILED_PROMPT = 40, QKV_TILED_STEP = 100;
 // Up to here the first expert GEMM takes all rows for every expert and stores the routed ones: more MMAs, no dispatch.  A token without
 // finite router logits is stored once, for expert 0, and its second hidden row holds whatever was there: combine and tail

@@ -116,7 +116,7 @@ def test_cross_entropy_of_values_that_are_not_finite(V):
 
 @pytest.mark.parametrize("B,T", [(1, 1), (4, 1), (5, 1), (8, 1), (9, 1), (16, 1), (17, 1), (33, 1), (64, 1), (65, 1), (128, 1),
                                  (129, 1), (1, 2), (3, 3), (1, 16), (2, 20), (1, 64), (1, 65), (2, 64), (1, 128), (1, 129),
-                                 (1, 256), (1, 257), (257, 1), (1, 640), (1, 960), (1, 961)])
+                                 (1, 256), (1, 257), (257, 1), (1, 640), (1, 960), (1, 961), (1, 40), (1, 41)])
 def test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T):
     """d_model 1024: the kernels for few tokens (GEMM forms up to 16, up to 960 and beyond, router up to 256, row cluster up to
     128) against the kernel-by-kernel path; mixed routing, carried state, one expert without tokens at the smallest sizes."""
