@@ -196,7 +196,8 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, 1, st));
     else if (qkv_tile)
-      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile, (N + qkv_tile - 1) / qkv_tile, st));
+      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile,
+                              (N + qkv_tile - 1) / qkv_tile, st));
     else if (mid)
       JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv));
     else
@@ -209,7 +210,8 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, 1, st));
     else if (out_tile)
-      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile, (N + out_tile - 1) / out_tile, st));
+      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile,
+                              (N + out_tile - 1) / out_tile, st));
     else if (mid)
       JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x));
     else

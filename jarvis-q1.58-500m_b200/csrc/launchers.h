@@ -27,8 +27,8 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
                         int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope = nullptr, bool settled = false);
 // The same product for a few tokens (small_gemm.cu), bit for bit; bf16, GELU and residual epilogues.  idx / scatter ([M][2]):
 // all M rows go through every group's matrix and row n is stored at scatter[2n + k] where idx[2n + k] is the group; else seg
-// as above.  tile: rows a CTA takes at a time, 8 or 16; tiles: CTAs that share a segment's tiles.  Within a chain only: weights and seg were complete
-// before the kernel ahead of this one on the stream began, and are read while it runs.
+// as above.  tile: rows a CTA takes at a time, 8 or 16; tiles: CTAs that share a segment's tiles.  Within a chain only: weights
+// and seg were complete before the kernel ahead of this one on the stream began, and are read while it runs.
 int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
                       int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
                       int tile, int tiles, cudaStream_t stream);

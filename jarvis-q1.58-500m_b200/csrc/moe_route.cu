@@ -684,8 +684,8 @@ namespace {
 // layer called by itself pays for on the host up to some 8000 tokens (4000 tokens 137 us, 133 with two).  Device time of metadata and
 // gather -> histogram and dispatch_kernel: 4 experts, 1024 channels: 300 tokens 3.8 -> 7.4 us, 1024 5.2 -> 7.5, 4096 8.2 -> 8.0, 8192
 // 11.3 -> 11.2, 16,384 18.4 -> 18.9, 32,768 43.7 -> 41.1, 65,536 88.5 -> 71.0, 131,072 170 -> 135, 262,144 333 -> 261, 524,288 659 -> 537.
-// 8 experts, 512 channels (twice the counts, half the rows): 16,384 12.4 -> 14.5, 32,768 equal, 131,072 102 -> 84, 262,144 206 -> 195, 524,288
-// 408 -> 494: every CTA adds up all counts.
+// 8 experts, 512 channels (twice the counts, half the rows): 16,384 12.4 -> 14.5, 32,768 equal, 131,072 102 -> 84, 262,144
+// 206 -> 195, 524,288 408 -> 494: every CTA adds up all counts.
 constexpr int DISPATCH_MAX = 262144;
 bool one_launch_dispatch(int n_tokens) { return 2 * n_tokens > META_SMALL_MAX && n_tokens <= DISPATCH_MAX; }
 int dispatch_tokens(int n_tokens) { return n_tokens <= 16384 ? 32 : 64; }      // per CTA: 8000 tokens fill the chip only with the smaller

@@ -27,7 +27,8 @@ __device__ __forceinline__ uint4 norm8(const float (&v)[8], float r, float4 wa, 
 // of the unrounded values over the warp.
 struct Combined { float s1, s2; };
 template <typename F>
-__device__ __forceinline__ Combined combine_values(const uint4 (&ya)[GROUPS], const uint4 (&yb)[GROUPS], float2 g, int lane, int C, F&& put) {
+__device__ __forceinline__ Combined combine_values(const uint4 (&ya)[GROUPS], const uint4 (&yb)[GROUPS], float2 g, int lane, int C,
+                                                   F&& put) {
   float s1 = 0.f, s2 = 0.f;
 #pragma unroll
   for (int i = 0; i < GROUPS; ++i) {

@@ -17,12 +17,14 @@
 //     of eight steps (the prepared layout cost 16 wavefronts of shared memory per eight steps, this one 4);
 //   - sequences meet only in the variance that sets the LSF decay: with several clusters their sums travel as tagged
 //     words through global memory, one exchange a layer.  Those clusters wait for one another, so they are one cooperative launch.
-// With one token in a cluster (FULL) every CTA takes a sixteenth of every expert (few experts are used, each by one token); beyond, an expert
-// belongs to four CTAs, which exchange its hidden rows among themselves.
-// Measured (24 layers and the vocabulary head, replayed as a graph, kernel by kernel -> here): 1 sequence 621 -> 496 us, 2 675 -> 516,
-// 4 710 -> 511, 7 715 -> 515, 8 718 -> 641, 16 810 -> 663, 32 937 -> 751, 56 1049 -> 941.  With more tokens a cluster the form
+// With one token in a cluster (FULL) every CTA takes a sixteenth of every expert (few experts are used, each by one token);
+// beyond, an expert belongs to four CTAs, which exchange its hidden rows among themselves.
+// Measured (24 layers and the vocabulary head, replayed as a graph, kernel by kernel -> here): 1 sequence 621 -> 498 us, 2 675 -> 517,
+// 4 710 -> 504, 7 715 -> 511, 8 718 -> 631, 16 810 -> 655, 32 937 -> 751, 56 1049 -> 936.  With more tokens a cluster the form
 // loses: every cluster decodes all weights for itself, and shared memory holds eight.
-// Every value is rounded and every sum ordered as in the kernels this one stands for: results are theirs bit for bit.
+// Every value is rounded and every f32 sum ordered as in the kernels this one stands for.  The f64 sums over tokens behind mean and
+// variance, and those of the router's probabilities, are added in another order and rounded to f32 after that: the tests find the
+// results equal bit for bit, and a last bit of those scalars is what could differ.
 #include "attn_step.cuh"
 #include "common.cuh"
 #include "gemm_shared.cuh"
@@ -235,7 +237,9 @@ struct Step {
       if (elect_one()) {
         mbar_arrive_expect_tx(bar(ctl.p1_full), C * 4 + (lay ? SC_FLOATS * 4 : 0));
         bulk_load_1d(base + p.o_p1, w, C * 4, bar(ctl.p1_full));
-        if (lay) bulk_load_1d(base + p.o_sc + uint32_t(i & 1) * (SC_FLOATS * 4), p.layer[i].tiles + size_t(T_END) * UNIT, SC_FLOATS * 4, bar(ctl.p1_full));
+        if (lay)
+          bulk_load_1d(base + p.o_sc + uint32_t(i & 1) * (SC_FLOATS * 4), p.layer[i].tiles + size_t(T_END) * UNIT, SC_FLOATS * 4,
+                       bar(ctl.p1_full));
       }
       __syncwarp();
     };
@@ -279,7 +283,8 @@ struct Step {
       }
 #pragma unroll 1
       for (int i = 0; i < (l < 0 ? 0 : runs) && ok; ++i) {
-        const int kind = __shfl_sync(0xffffffffu, r_kind, i), off = __shfl_sync(0xffffffffu, r_off, i), n = __shfl_sync(0xffffffffu, r_n, i);
+        const int kind = __shfl_sync(0xffffffffu, r_kind, i), off = __shfl_sync(0xffffffffu, r_off, i);
+        const int n = __shfl_sync(0xffffffffu, r_n, i);
         if (kind == OUT) {
           ok = wait(ctl.p2_empty, uint32_t(l) ^ 1u);
           if (ok && elect_one()) {
@@ -289,7 +294,9 @@ struct Step {
           }
           __syncwarp();
         }
-        const uint8_t* src = kind == STATE ? reinterpret_cast<const uint8_t*>(y.s_in) : kind == MEMBRANE ? reinterpret_cast<const uint8_t*>(y.h_in) : w;
+        const uint8_t* src = kind == STATE      ? reinterpret_cast<const uint8_t*>(y.s_in)
+                             : kind == MEMBRANE ? reinterpret_cast<const uint8_t*>(y.h_in)
+                                                : w;
         if (src) units(src + size_t(off) * UNIT, kind == DOWN ? 2 * UNIT : UNIT, n);
       }
       norm1(l + 1);
@@ -444,7 +451,8 @@ struct Step {
     if ((!FULL || lane < 16) && !*abort_flag) {
       const int part = lane >> 4;
       const uint32_t to = base + p.o_rh + uint32_t(n) * ROW_C + uint32_t(c * D + row0) * 2u + uint32_t(part) * 16u;
-      st_async16(cluster_map(to, uint32_t(lane & 15)), cluster_map(bar(ctl.got_o), uint32_t(lane & 15)), lds128(scratch() + uint32_t(part) * 16u));
+      st_async16(cluster_map(to, uint32_t(lane & 15)), cluster_map(bar(ctl.got_o), uint32_t(lane & 15)),
+                 lds128(scratch() + uint32_t(part) * 16u));
     }
     __syncwarp();
   }
@@ -453,7 +461,8 @@ struct Step {
   // written only when all of them are past that layer's tail.
   __device__ __forceinline__ void membrane_out(int l) const {
     if (lane < 16)
-      reinterpret_cast<float4*>(p.layer[l].h_out + size_t(n0 + warp) * C + c * D)[lane] = reinterpret_cast<const float4*>(smem + p.o_ho + warp * (D * 4))[lane];
+      reinterpret_cast<float4*>(p.layer[l].h_out + size_t(n0 + warp) * C + c * D)[lane] =
+          reinterpret_cast<const float4*>(smem + p.o_ho + warp * (D * 4))[lane];
   }
 
   // ---- a token's row in shared memory, eight channels a lane in four groups (loops are left rolled: a quarter of the code) ----
@@ -497,7 +506,8 @@ struct Step {
       also(i, v);
     }
   }
-  __device__ __forceinline__ bool own(int i) const { return i == (c >> 2) && (lane >> 3) == (c & 3); }      // group i of this lane is in the CTA's 64 channels
+  // group i of this lane is in the CTA's 64 channels
+  __device__ __forceinline__ bool own(int i) const { return i == (c >> 2) && (lane >> 3) == (c & 3); }
 
   // norm2 and router of token `warp`: router_finish's values with an expert per lane
   __device__ __forceinline__ void route(int l) const {
@@ -514,7 +524,8 @@ struct Step {
     }
     float acc[E] = {};
     norm_row(ss, y.eps2, p.o_p2, [&](int i, const uint32_t (&v)[4]) {
-      const float xv[8] = {bf16_lo(v[0]), bf16_hi(v[0]), bf16_lo(v[1]), bf16_hi(v[1]), bf16_lo(v[2]), bf16_hi(v[2]), bf16_lo(v[3]), bf16_hi(v[3])};
+      const float xv[8] = {bf16_lo(v[0]), bf16_hi(v[0]), bf16_lo(v[1]), bf16_hi(v[1]),
+                           bf16_lo(v[2]), bf16_hi(v[2]), bf16_lo(v[3]), bf16_hi(v[3])};
 #pragma unroll
       for (int e = 0; e < E; ++e) {
         const float4* w = reinterpret_cast<const float4*>(smem + p.o_p2 + C * 4 + e * UNIT) + i * 64 + lane;
@@ -692,18 +703,17 @@ struct Step {
           mbar_arrive_expect_tx(bar(ctl.got_x), uint32_t(NT) * (C * 4));
           mbar_arrive_expect_tx(bar(ctl.got_y), uint32_t(NT) * (C * 4));
         }
-        // FULL: the states of this warp's rows travel while q, k, v are made
+        // FULL: the states of this warp's eight rows travel while q, k, v are made, in attn_decode_kernel's lanes (sixteen columns of
+        // a row) or attn_decode_stream_kernel's (four columns of every other row)
         float4 st[4];
-        auto fetch = [&](int j) {
-          // attn_decode_kernel's lanes: sixteen columns of a row; attn_decode_stream_kernel's: four columns of every other row
-          const size_t at = (size_t(n0 + (j >> 3)) * CTAS + c) * (D * D) + (j & 7) * (8 * D) + (STREAM ? 4 * lane : 16 * lane);
+        if (FULL) {
+          const size_t at = (size_t(n0) * CTAS + c) * (D * D) + (warp & 7) * (8 * D) + (STREAM ? 4 * lane : 16 * lane);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             st[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (y.s_in && j < 8 * NT) st[i] = *reinterpret_cast<const float4*>(y.s_in + at + (STREAM ? 2 * D : 4) * i);
+            if (y.s_in && warp < 8) st[i] = *reinterpret_cast<const float4*>(y.s_in + at + (STREAM ? 2 * D : 4) * i);
           }
-        };
-        if (FULL) fetch(warp);
+        }
         unsigned used = 0;
         int n_e = 0;
         // ---- the four products: q, k, v of head c; output projection; first and second expert matrix ----
@@ -713,10 +723,8 @@ struct Step {
             bar_compute();
             const float gamma = sc[SC_GAMMA + c];
 #pragma unroll 1
-            for (int j = warp; j < (FULL ? 8 : 4) * NT; j += WARPS) {
-              if (FULL && j >= WARPS) fetch(j);
-              attend(u0 + 12 + j, st, FULL ? j >> 3 : j >> 2, FULL ? (j & 7) * 8 : (j & 3) * 16, gamma, y.s_out);
-            }
+            for (int j = warp; j < (FULL ? 8 : 4 * NT); j += WARPS)
+              attend(u0 + 12 + j, st, FULL ? 0 : j >> 2, FULL ? j * 8 : (j & 3) * 16, gamma, y.s_out);
           } else if (ph == 2) {
             if (warp < NT) route(l);
             __syncwarp();
@@ -727,7 +735,8 @@ struct Step {
               if (warp == WARPS - 1 && lane == 0 && !*abort_flag) mbar_arrive_expect_tx(bar(ctl.got_h), uint32_t(NT) * (4 * HID));
             } else {
               n_e = tokens_of(c & 3);
-              if (n_e > 0 && warp == WARPS - 1 && lane == 0 && !*abort_flag) mbar_arrive_expect_tx(bar(ctl.got_h), uint32_t(n_e) * (2 * HID));
+              if (n_e > 0 && warp == WARPS - 1 && lane == 0 && !*abort_flag)
+                mbar_arrive_expect_tx(bar(ctl.got_h), uint32_t(n_e) * (2 * HID));
             }
           }
           const int jobs = ph < 2 ? (warp < (ph ? 4 : 12) ? 1 : 0) : FULL ? E : ph == 2 ? 2 : 1;
@@ -755,7 +764,8 @@ struct Step {
             const int halves = ph == 3 ? 2 : 1;
             float acc[4] = {};
             const int s = min(lane & 7, n - 1), row = !on ? 0 : ph < 2 ? s : ph == 2 ? list[s] >> 1 : FULL ? list[s] : s;
-            uint32_t xa = base + ((ph & 1) ? p.o_rh : p.o_xn) + uint32_t(row) * uint32_t(ph == 3 ? ROW_H : ROW_C) + uint32_t(lane >> 3) * 16u;
+            uint32_t xa = base + ((ph & 1) ? p.o_rh : p.o_xn) + uint32_t(row) * uint32_t(ph == 3 ? ROW_H : ROW_C) +
+                          uint32_t(lane >> 3) * 16u;
 #pragma unroll 1
             for (int h = 0; h < halves; ++h) {
               const int slot = unit_wait(u + 16 * h);
@@ -768,7 +778,8 @@ struct Step {
             }
             if (!on) continue;
             // ---- epilogue: a row of 16 features per token, then in pieces of 16 bytes to whoever needs it ----
-            const float alpha = 0.5f * sc[ph == 0 ? SC_AQKV + (warp >> 2) : ph == 1 ? SC_AOUT : ph == 2 ? SC_A1 + e : SC_A2 + e];      // codes decode to +-2
+            // codes decode to +-2
+            const float alpha = 0.5f * sc[ph == 0 ? SC_AQKV + (warp >> 2) : ph == 1 ? SC_AOUT : ph == 2 ? SC_A1 + e : SC_A2 + e];
             const int g = lane >> 2, t = lane & 3;
             const uint32_t rows = ph == 0 ? base + p.o_qkv + uint32_t(f0) * 2u : scratch();
             const uint32_t row_bytes = ph == 0 ? 3 * D * 2 : ph == 1 ? 64 : 32;
@@ -780,7 +791,8 @@ struct Step {
               const uint32_t at = rows + uint32_t(tok) * row_bytes;
               if (ph == 1) {
                 const float2 r = *reinterpret_cast<const float2*>(smem + p.o_rx + tok * (C * 4) + (c * D + f0 + 2 * g) * 4);
-                asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(at + uint32_t(g) * 8u), "f"(__fadd_rn(r.x, a)), "f"(__fadd_rn(r.y, b)) : "memory");
+                asm volatile("st.shared.v2.f32 [%0], {%1, %2};"
+                             ::"r"(at + uint32_t(g) * 8u), "f"(__fadd_rn(r.x, a)), "f"(__fadd_rn(r.y, b)) : "memory");
               } else {
                 if (ph == 2) { a = gelu_erf(a); b = gelu_erf(b); }
                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + uint32_t(g) * 4u), "r"(pack_bf16x2(a, b)) : "memory");
@@ -848,7 +860,8 @@ struct Step {
         if (follow) {
           wait(ctl.p1_full, par ^ 1u);
           norm_row(ss, last ? p.eps_final : p.layer[last ? 0 : l + 1].eps1, p.o_p1, [&](int i, const uint32_t (&v)[4]) {
-            if (last && own(i)) *reinterpret_cast<uint4*>(p.hidden_out + size_t(n0 + warp) * C + (i * 32 + lane) * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+            if (last && own(i))
+              *reinterpret_cast<uint4*>(p.hidden_out + size_t(n0 + warp) * C + (i * 32 + lane) * 8) = make_uint4(v[0], v[1], v[2], v[3]);
           });
         }
       }
@@ -956,7 +969,8 @@ step_weights_kernel(const uint8_t* __restrict__ w_qkv, const uint8_t* __restrict
   uint32_t v[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {    // row 2g + (i >> 1), steps 4 (i & 1) ..
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(rows + size_t(tile * 16 + 2 * g + (i >> 1)) * (K / 4)) + half * 64 + ch * 8 + 4 * (i & 1);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(rows + size_t(tile * 16 + 2 * g + (i >> 1)) * (K / 4)) + half * 64 + ch * 8 +
+                          4 * (i & 1);
     uint32_t o = 0;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
@@ -1009,7 +1023,8 @@ int max_clusters() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   int n = known[dev].load(std::memory_order_acquire);
   if (n == 0) {
-    for (const void* k : {reinterpret_cast<const void*>(step_cluster_kernel<true, false>), reinterpret_cast<const void*>(step_cluster_kernel<true, true>),
+    for (const void* k : {reinterpret_cast<const void*>(step_cluster_kernel<true, false>),
+                          reinterpret_cast<const void*>(step_cluster_kernel<true, true>),
                           reinterpret_cast<const void*>(step_cluster_kernel<false, true>)}) {
       if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
           cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(DYN_MAX)) != cudaSuccess) {
@@ -1056,7 +1071,8 @@ int step_clusters(int N, int most, bool carried) {
 int launch_step_weights(const jb200_layer* y, int c, int h, int e, int hidden, void* out, cudaStream_t stream) {
   JB_REQUIRE(y && out && y->w_qkv && y->w_out && y->w1 && y->w2 && y->gamma && y->a_qkv && y->a_out && y->a1 && y->a2,
              "step_weights: null pointer");
-  JB_REQUIRE(step_weight_bytes(c, h, e, hidden) != 0, "step_weights: d_model %d / heads %d / experts %d x %d have no such form", c, h, e, hidden);
+  JB_REQUIRE(step_weight_bytes(c, h, e, hidden) != 0, "step_weights: d_model %d / heads %d / experts %d x %d have no such form", c, h, e,
+             hidden);
   JB_REQUIRE(aligned16(out) && aligned16(y->w_qkv) && aligned16(y->w_out) && aligned16(y->w1) && aligned16(y->w2),
              "step_weights: pointers must be 16-byte aligned");
   step_weights_kernel<<<T_END + 1, 256, 0, stream>>>(y->w_qkv, y->w_out, y->w1, y->w2, y->gamma, y->a_qkv, y->a_out, y->a1, y->a2,
@@ -1090,14 +1106,15 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
   const Plan s = plan_of(tokens, full);
   size_t off[7];
   StepParams p = {};
-  // A layer's accumulators, and the words in which the sums of several clusters meet, lie in the workspace: the rest of it is not used here.
+  // A layer's accumulators, and the words in which the sums of several clusters meet, lie in the workspace: the rest of it is not
+  // used here.
   p.acc_stride = accumulator_bytes(E) + MAX_CLUSTERS * 32;
   if (forward_workspace_bytes(N, 1, C, CTAS, E, HID) < n_layers * p.acc_stride) return JB200_OK;
   p.routing_stride = routing_layout(N, E, off);
   p.r_idx = uint32_t(off[0]); p.r_gates = uint32_t(off[1]); p.r_counts = uint32_t(off[2]); p.r_offsets = uint32_t(off[3]);
   p.r_scatter = uint32_t(off[4]); p.r_gather = uint32_t(off[5]); p.r_gate_idx = uint32_t(off[6]);
-  p.o_p1 = s.o_p1; p.o_p2 = s.o_p2; p.o_sc = s.o_sc; p.o_rx = s.o_rx; p.o_xn = s.o_xn; p.o_rh = s.o_rh; p.o_qkv = s.o_qkv; p.o_ho = s.o_ho; p.o_ry = s.o_ry;
-  p.o_cs = s.o_cs; p.o_scr = s.o_scr; p.o_ring = s.o_ring; p.units = s.units;
+  p.o_p1 = s.o_p1; p.o_p2 = s.o_p2; p.o_sc = s.o_sc; p.o_rx = s.o_rx; p.o_xn = s.o_xn; p.o_rh = s.o_rh; p.o_qkv = s.o_qkv;
+  p.o_ho = s.o_ho; p.o_ry = s.o_ry; p.o_cs = s.o_cs; p.o_scr = s.o_scr; p.o_ring = s.o_ring; p.units = s.units;
   p.x = f->x; p.cos_tab = f->cos_tab; p.sin_tab = f->sin_tab; p.pos0 = f->pos0; p.pos0_scalar = f->pos0_scalar; p.n_pos = f->n_pos;
   p.N = N; p.n_clusters = n_cl; p.vocab = f->vocab;
   p.n_elems = double(N) * C; p.n_inv = 1.0 / p.n_elems; p.n1_inv = 1.0 / (p.n_elems - 1.0);
