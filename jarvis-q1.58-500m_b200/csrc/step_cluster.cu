@@ -209,7 +209,7 @@ struct Step {
 
   // ---------------- producer ----------------
   __device__ __forceinline__ void produce() const {
-    int slot = 0, issued = 0;
+    int slot = 0, issued = 0, norms = 0, routers = 0;
     uint32_t ph = 1u;
     bool ok = true;
     // `n` units from src, `stride` bytes apart
@@ -234,6 +234,7 @@ struct Step {
       if (!ok || !w) return;
       ok = wait(ctl.p1_empty, uint32_t(i) ^ 1u);
       if (!ok) return;
+      ++norms;
       if (elect_one()) {
         mbar_arrive_expect_tx(bar(ctl.p1_full), C * 4 + (lay ? SC_FLOATS * 4 : 0));
         bulk_load_1d(base + p.o_p1, w, C * 4, bar(ctl.p1_full));
@@ -287,6 +288,7 @@ struct Step {
         const int n = __shfl_sync(0xffffffffu, r_n, i);
         if (kind == OUT) {
           ok = wait(ctl.p2_empty, uint32_t(l) ^ 1u);
+          routers += ok ? 1 : 0;
           if (ok && elect_one()) {
             mbar_arrive_expect_tx(bar(ctl.p2_there), C * 4 + E * UNIT);
             bulk_load_1d(base + p.o_p2, y.w_norm2, C * 4, bar(ctl.p2_there));
@@ -302,10 +304,14 @@ struct Step {
       norm1(l + 1);
     }
     if (!ok) {           // given up: copies in flight land before this CTA's shared memory goes
+      auto landed = [&](const uint64_t& b, int n) {           // n phases of it, the last of which may be open
 #pragma unroll 1
-      for (int u = issued > p.units ? issued - p.units : 0; u < issued; ++u)
+        for (int i = 0; n > 0 && i < 2000 && !phase_done(bar(b), uint32_t(n - 1) & 1u); ++i) {}
+      };
+      landed(ctl.p1_full, norms);
+      landed(ctl.p2_there, routers);
 #pragma unroll 1
-        for (int i = 0; i < 2000 && !phase_done(bar(ctl.full[u % p.units]), uint32_t(u / p.units) & 1u); ++i) {}
+      for (int u = issued > p.units ? issued - p.units : 0; u < issued; ++u) landed(ctl.full[u % p.units], u / p.units + 1);
     }
   }
 
