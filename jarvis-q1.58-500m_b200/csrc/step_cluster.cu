@@ -19,8 +19,8 @@
 //     words through global memory, one exchange a layer.  Those clusters wait for one another, so they are one cooperative launch.
 // With one token in a cluster (FULL) every CTA takes a sixteenth of every expert (few experts are used, each by one token);
 // beyond, an expert belongs to four CTAs, which exchange its hidden rows among themselves.
-// Measured (24 layers and the vocabulary head, replayed as a graph, kernel by kernel -> here): 1 sequence 621 -> 498 us, 2 675 -> 517,
-// 4 710 -> 504, 7 715 -> 511, 8 718 -> 631, 16 810 -> 655, 32 937 -> 751, 56 1049 -> 936.  With more tokens a cluster the form
+// Measured (24 layers and the vocabulary head, replayed as a graph, kernel by kernel -> here): 1 sequence 621 -> 494 us, 2 675 -> 517,
+// 4 710 -> 504, 7 715 -> 511, 8 718 -> 630, 16 810 -> 655, 32 937 -> 751, 56 1049 -> 928.  With more tokens a cluster the form
 // loses: every cluster decodes all weights for itself, and shared memory holds eight.
 // Every value is rounded and every f32 sum ordered as in the kernels this one stands for.  The f64 sums over tokens behind mean and
 // variance, and those of the router's probabilities, are added in another order and rounded to f32 after that: the tests find the
