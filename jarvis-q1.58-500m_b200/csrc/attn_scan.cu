@@ -7,8 +7,8 @@
 //                                                                      kernel A3, associative_attention_cuda.cu:218-265)
 //
 // The reference's chunk-parallel path does the four chunk products as batched library GEMMs over materialised
-// per-chunk states (associative_attention.py:242-266).  Here one CTA per (sequence, head, segment) walks its part
-// of the sequence in 128-token chunks and issues the same four products as tcgen05.mma (bf16 operands from shared
+// per-chunk states (associative_attention.py:242-266).  Here a CTA walks (sequence, head, segment)s in 128-token
+// chunks and issues the same four products as tcgen05.mma (bf16 operands from shared
 // memory, fp32 accumulators in tensor memory); the state S never leaves the SM (fp32 master copy in registers,
 // bf16 copy in shared memory as an MMA operand), so HBM traffic is q, k, v in / o out (512 B per token-head)
 // plus one optional state load / store per (sequence, head).  Chunk length is free: the chunked form equals
@@ -16,17 +16,15 @@
 //
 // Per chunk of c <= 128 tokens (i, j: query / key token inside the chunk; g = gamma):
 //   TMA (128B-swizzled [128 tokens][64] boxes)                        ->  q, k, v tiles in shared memory
-//   all threads: feature map + RoPE in place on q and k;  kw[j] = k'[j] * g^(c-1-j)
-//   MMA  A:  scores = Q' K'^T       (M=128 i, N=128 j, K=64; both operands K-major)             -> TMEM [0,128)
-//            O2     = Q' S^T        (M=128 i, N=64 dv, K=64; S bf16 [dv][dk] is K-major)        -> TMEM [128,192)
+//   feature map + RoPE in place on q and k;  kw[j] = k'[j] * g^(c-1-j)
+//   MMA  A:  scores = Q' K'^T       (M=128 i, N=128 j, K=64; both operands K-major)
+//            O2     = Q' S^T        (M=128 i, N=64 dv, K=64; S bf16 [dv][dk] is K-major)
 //   MMA  S:  dS     = V^T Kw        (M=dv, N=dk, K=128 j; both operands are the [token][64] tiles read
-//                                    MN-major; M is padded to 128 by reading the 64 dv twice)    -> TMEM [192,256)
-//   all threads: P[i][j] = scores * g^(i-j) / 8 for j <= i, else 0      (TMEM -> registers -> bf16 tile in smem)
-//   MMA  B:  O1     = P V           (M=128 i, N=64 dv, K=128 j; V read MN-major from its raw tile) -> TMEM [0,64)
-//   all threads: S = g^c S + dS (registers; bf16 copy to smem);   o[i] = O1 + g^(i+1)/8 * O2  -> global
-// One thread issues the TMA loads and the MMAs; every wait (TMA arrival, MMA completion) is an mbarrier wait
-// bounded in time.  256 TMEM columns, 105 KiB of shared memory and <= 128 registers per thread let two CTAs
-// share an SM and cover each other's latencies.
+//                                    MN-major; M is padded to 128 by reading the 64 dv twice)
+//   P[i][j] = scores * g^(i-j) / 8 for j <= i, else 0                   (TMEM -> registers -> TMEM, bf16)
+//   MMA  B:  O1     = P V           (M=128 i, N=64 dv, K=128 j; V read MN-major from its raw tile)
+//   S = g^c S + dS (registers; bf16 copy to smem);   o[i] = O1 + g^(i+1)/8 * O2  -> global
+// Every wait (TMA arrival, MMA completion) is an mbarrier wait bounded in time.
 //
 // Sequence segments: when B*H alone cannot fill the GPU (prefill of a few long sequences), T is cut into
 // segments.  A first launch (STATE_ONLY) runs only the k/v half of the work for every non-final segment from a
@@ -65,14 +63,14 @@ struct AttnParams {
   float* seg_state;        // [B][H][n_pieces][64][64]: state contribution of each piece
   int n_pieces;            // pieces stored per (sequence, head): nseg - 1, or nseg in a state-only call
   int qk_prepared;         // q, k already hold phi(.) + RoPE with the head dim interleaved (d, d+32 adjacent)
-  int wide_store;          // output rows are 32-byte aligned: 256-bit stores
-  // Balanced launch (more sequence-heads than SMs, a partly filled last wave): the first n_split sequence-heads are
-  // cut in two at chunk split_chunk.  CTAs take tickets from ctrl[0]; tickets [0, n_split) are the first parts,
-  // [n_split, B*H) whole sequence-heads, [B*H, B*H + n_split) the second parts, which find the state after the
-  // first part in handoff[unit] once ctrl[1 + unit] has counted the eight consumer warps that wrote it.
-  int n_split, split_chunk;
-  float* handoff;          // [n_split][64][64] f32
-  int* ctrl;               // [1 + n_split], zeroed before the launch
+  int wide_tab;            // RoPE tables are 32-byte aligned: 256-bit loads
+  // Several sequence-heads per CTA (as many CTAs as SMs): with split, equal shares of all chunks, cut wherever they end.  CTAs
+  // take tickets from ctrl[0]; the CTA with ticket t leaves the state after its first part of a cut sequence-head in handoff[t],
+  // counts its state warps in ctrl[1 + t], and ticket t + 1 goes on from there.
+  int split;
+  int per_cta, spare;      // sequence-heads, or with split chunks, of every CTA; the first `spare` take one more
+  float* handoff;          // [CTAs][64][64] f32
+  int* ctrl;               // [1 + CTAs], zeroed before the launch
   unsigned int* status;
   int settled;             // decays (single-token step: state and positions too) were complete before the kernel ahead of this one started
 };
@@ -109,10 +107,16 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
       : "memory");
 }
 
-__device__ __forceinline__ void st_global_256(void* p, const uint32_t* w) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-               ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-               : "memory");
+// Eight angles of a row of a RoPE table: 32 bytes at a 32-byte step from the table's start, in one load where that is aligned.
+__device__ __forceinline__ void load_angles8(const float* src, bool wide, float (&a)[8]) {
+  if (wide) {
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7])
+        : "l"(src));
+  } else {
+    const float4 lo = __ldg(reinterpret_cast<const float4*>(src)), hi = __ldg(reinterpret_cast<const float4*>(src) + 1);
+    a[0] = lo.x; a[1] = lo.y; a[2] = lo.z; a[3] = lo.w; a[4] = hi.x; a[5] = hi.y; a[6] = hi.z; a[7] = hi.w;
+  }
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -306,54 +310,79 @@ attn_state_pass_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// The full pass as a warp-specialised pipeline: one CTA per SM, 576 threads, several chunks in flight.
-//   warp 0       TMA producer: q, k, v tiles of chunk c+2 as soon as the MMAs that read stage c%2 have retired
-//   warp 1       MMA issuer (one thread), per chunk c in this order:
-//                  S(c)  dS = V^T Kw                 -> TMEM DS        (needs the prologue of c, v of c)
-//                  A2(c) O2 = Q' S^T                  -> TMEM O2[c%2]   (needs the state after chunk c-1 in smem)
-//                  B(c)  O1 = P V                     -> TMEM SC[c%2] columns 0-63 (needs P of c)
-//                  A1(c+1) scores = Q' K'^T of the NEXT chunk -> TMEM SC[(c+1)%2]
-//                so the scores of chunk c+1 are computed while the consumers finish chunk c
-//   warps 2-9    prologue: feature map + RoPE in place on q and k of a stage, kw = k' * gamma^(c-1-j)
-//   warps 10-17  consumers (two per TMEM lane quarter): decay mask scores -> P, state update, output rows
-// Double-buffered: q/k/kw/v stages, score and O2 accumulators, the bf16 state copy.  Single: P (its reader,
-// MMA B, has retired before the next mask step starts, because the output rows of a chunk wait for it).
+// The full pass as a warp-specialised pipeline: one CTA per SM, 24 warps, several chunks in flight.
+//   warp 0       TMA producer: q, k, v tiles of a chunk as soon as the MMAs that read its stage have retired
+//   warp 1       MMA issuer, per chunk c:  A1(c) scores = Q' K'^T -> TMEM SC[c%2];  S(c) dS = V^T Kw -> TMEM DS[c%2];
+//                A2(c) O2 = Q' S^T -> TMEM O2[c%2] (needs the state before chunk c in smem)
+//   warp 2       MMA issuer, B(c): O1 = P V -> TMEM SC[c%2] columns 0-63 (needs P of c), on its own so that it never
+//                waits behind the next chunk's prologue
+//   warp 3       idle (registers are handed out to groups of four warps)
+//   warps 4-11   prologue: feature map + RoPE in place on q and k of a stage, kw = k' * gamma^(c-1-j)
+//   warps 12-15  state: S = gamma^c S + dS in registers, its bf16 copy in smem; decay tables of the heads to come
+//   warps 16-19, 20-23  consumers of the even and of the odd chunks: decay mask scores -> P, output rows (by TMA through the v
+//                tile of the chunk, which P V was the last to read)
+// What bounds it now: the prologue, 3700 of the ~4100 cycles of a chunk (two warps per scheduler; sixteen warps, or more registers,
+// were 3 to 8 % slower, its two rows unrolled 20 %: the roles' loops share the instruction caches, at 67 KB of code a chunk took 5000
+// cycles when all SMs ran and 3700 on one alone).  With one group of consumers (eight warps, half the columns each) for every
+// chunk the period was the serial chain scores -> mask -> P V -> output rows, 5500 cycles.  Two groups of four warps overlap the chains of
+// two chunks, the state has warps of its own, one lane of a warp arrives on a barrier (256 arrivals took 300-400 cycles, four a chunk), a
+// CTA walks several sequence-heads without draining (filling and draining took ~12 us each), output rows go by TMA (stored
+// directly they took 512 of 3000 wavefronts of a chunk), angles come 32 bytes a load.  B x T of 16 heads, before -> after: 32 x 2048 158 -> 125 us,
+// 32 x 512 55.5 -> 43, 8 x 2048 43.1 -> 36.6, 32 x 64 24.3 -> 15.5, 1 x 16384 in segments 77 -> 71, 1 x 37 and 1 x 128 5.9 -> 6.2 and
+// 6.4 -> 6.8 (the chain of a lone chunk).
+// P (bf16 pairs, 64 columns) overlays score columns 64-127: a warp owns its lanes, and walks the 16-key blocks downwards, so
+// what it overwrites it has read.
 // ------------------------------------------------------------------------------------------------------------
-// Per-role cycle counters of one CTA (block 0,0,0), compiled in with -DJB_ATTN_TIMING only: every role adds the
+// Per-role cycle counters of one CTA (block 0), compiled in with -DJB_ATTN_TIMING only: every role adds the
 // cycles it spends in each of its waits and work phases; a harness reads g_attn_timing after the launch.
 #ifdef JB_ATTN_TIMING
-__device__ long long g_attn_timing[18 * 8];
+__device__ long long g_attn_timing[24 * 8];
 #define JB_T_DECL long long t_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}; long long t_last = clock64();
 #define JB_T_MARK(k) { const long long t_now = clock64(); t_acc[k] += t_now - t_last; t_last = t_now; }
-#define JB_T_FLUSH(w) if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0) { for (int kk = 0; kk < 8; ++kk) g_attn_timing[(w) * 8 + kk] = t_acc[kk]; }
+#define JB_T_FLUSH(w) if (blockIdx.x == 0 && lane == 0) { for (int kk = 0; kk < 8; ++kk) g_attn_timing[(w) * 8 + kk] = t_acc[kk]; }
 #else
 #define JB_T_DECL
 #define JB_T_MARK(k)
 #define JB_T_FLUSH(w)
 #endif
 
-constexpr int PIPE_THREADS = 576;
-constexpr int PRO_WARP0 = 2, CON_WARP0 = 10;
+constexpr int PRO_WARP0 = 4, STATE_WARP0 = 12, CON_WARP0 = 16, PIPE_THREADS = 24 * 32;
+constexpr int PRO_WARPS = 8, STATE_WARPS = 4, CON_WARPS = 4;  // consumers: of each group
+// Registers a thread: the CTA is launched with 80 for each of its six groups of four warps; the issuers give up what the
+// others take.
+constexpr int LAUNCH_REGS = 80, ISSUE_REGS = 48, PRO_REGS = 88, STATE_REGS = 80, CON_REGS = 88;
+static_assert(ISSUE_REGS + 2 * PRO_REGS + STATE_REGS + 2 * CON_REGS <= 6 * LAUNCH_REGS, "no more registers than the CTA was launched with");
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 constexpr int NST = 3;                                       // stages of the q / k / kw / v tiles
 constexpr uint32_t PIPE_TMEM_COLS = 512;
-constexpr uint32_t PT_SC = 0, PT_O2 = 256, PT_DS = 384, PT_P = 448;   // SC[2] x 128, O2[2] x 64, DS x 64, P x 64
+constexpr uint32_t PT_SC = 0, PT_O2 = 256, PT_DS = 384;      // SC[2] x 128, O2[2] x 64, DS[2] x 64
+constexpr uint32_t PT_P = 64;                                // P inside SC
+
+// Powers of a head's decay.  NTAB: the state warps fill the tables of the sequence-head after next while the consumers
+// may still be two chunks, so at most two sequence-heads, behind.
+struct DecayTab {
+  float pwm[2 * CH];           // pwm[x + CH] = gamma^x / 8 for x >= 0, 0 for x < 0: the decay mask by (i - j)
+  float pw[CH + 4];            // gamma^n, n <= CH
+};
+constexpr int NTAB = 6;
 
 struct PipeSmem {
   uint8_t q[NST][TILE_BYTES];
   uint8_t k[NST][TILE_BYTES];
   uint8_t kw[NST][TILE_BYTES];
   uint8_t v[NST][TILE_BYTES];
-  uint8_t s[2][S_BYTES];       // bf16 state copy, [n & 1] = state after n chunks of this CTA
-  float pwm[2 * CH];           // pwm[x + CH] = gamma^x / 8 for x >= 0, 0 for x < 0: the decay mask by (i - j)
-  float pw[CH + 1];            // gamma^n
+  uint8_t s[2][S_BYTES];       // bf16 state copy, [c & 1] = state before chunk c of this CTA
+  DecayTab tab[NTAB];
   uint64_t full_qk[NST], full_v[NST], empty_qk[NST], empty_v[NST], pro_done[NST];
-  uint64_t bar_sc[2], bar_b[2], o_done[2];
-  uint64_t bar_s, s_done, p_done;
+  uint64_t bar_sc[2], bar_s[2], bar_o2[2], bar_b[2], s_done[2], p_done[2], o_done[2];
+  uint64_t tab_full[NTAB];
   uint32_t tmem_base;
   uint32_t abort_flag;
   int ticket;
 };
 constexpr size_t PIPE_SMEM_BYTES = sizeof(PipeSmem) + 1024;
+static_assert(PIPE_SMEM_BYTES <= 227 * 1024, "shared memory of a CTA");
 
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -364,15 +393,75 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
+// The sequence-heads of a CTA, and of those that are not whole the chunks.  One segment of one sequence-head where sequences
+// are cut into segments; else a share of all chunks in order of (sequence, head, chunk): from chunk c0 of unit u0 to before
+// chunk c1 of unit u1.  The first part of the last unit is scanned first and the second part of the first unit last: a second
+// part needs the state that the CTA before this one leaves behind its first item.
+struct Item {
+  int unit, begin, end;
+  int piece;                   // 0 a whole sequence-head or a segment, 1 a first part (leaves its end state in handoff), 2 a second part
+};
+struct Share {
+  int u0, c0, u1, c1, begin, end, n_items, n_chunks;
+  __device__ __forceinline__ Share(const AttnParams& p, int cta, int n_chunks_) : n_chunks(n_chunks_) {
+    begin = 0;
+    end = n_chunks;
+    c0 = c1 = 0;
+    const int U = p.B * p.H;
+    if (p.nseg > 1) {
+      const int seg = cta / U;
+      u0 = cta - seg * U;
+      u1 = u0 + 1;
+      begin = seg * p.seg_chunks;
+      end = min(n_chunks, begin + p.seg_chunks);
+    } else {
+      const int a = cta * p.per_cta + min(cta, p.spare), e = a + p.per_cta + (cta < p.spare);
+      u0 = a;
+      u1 = e;
+      if (p.split) {
+        u0 = a / n_chunks;
+        c0 = a - u0 * n_chunks;
+        u1 = e / n_chunks;
+        c1 = e - u1 * n_chunks;
+      }
+    }
+    n_items = u1 - u0 + (c1 > 0);
+  }
+  __device__ __forceinline__ int chunks() const { return (u1 - u0) * (end - begin) - c0 + c1; }
+  __device__ __forceinline__ Item at(int k) const {
+    const int first = c1 > 0, whole = c0 > 0;
+    if (k < first) return {u1, 0, c1, 1};
+    if (whole && k == n_items - 1) return {u0, c0, n_chunks, 2};
+    return {u0 + whole + k - first, begin, end, 0};
+  }
+};
+
+__device__ __forceinline__ void fill_tab(DecayTab& t, float log_g, int tid, int threads) {
+  for (int n = tid; n <= CH; n += threads) t.pw[n] = expf(log_g * float(n));
+  for (int n = tid; n < 2 * CH; n += threads) {
+    // gamma^(i-j) / sqrt(D): the 1/8 of the query feature map is a power of two, so applying it to the scores
+    // (and to the cross-chunk factor) instead of to every element of q gives the same bits
+    const int x = n - CH;
+    t.pwm[n] = x >= 0 ? 0.125f * expf(log_g * float(x)) : 0.f;
+  }
+}
+
+template <bool PREPARED>
 __global__ void __launch_bounds__(PIPE_THREADS, 1)
 attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                      const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   PipeSmem* sm = reinterpret_cast<PipeSmem*>(smem_raw + (base - raw_addr));
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int T = p.T;
   const int n_chunks = (T + CH - 1) / CH;
 
@@ -381,22 +470,25 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       mbar_init(smem_u32(&sm->full_qk[s]), 1);
       mbar_init(smem_u32(&sm->full_v[s]), 1);
       mbar_init(smem_u32(&sm->empty_qk[s]), 1);
-      mbar_init(smem_u32(&sm->empty_v[s]), 1);
-      mbar_init(smem_u32(&sm->pro_done[s]), 256);
+      mbar_init(smem_u32(&sm->empty_v[s]), CON_WARPS);
+      mbar_init(smem_u32(&sm->pro_done[s]), PRO_WARPS);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(&sm->bar_sc[s]), 1);
+      mbar_init(smem_u32(&sm->bar_s[s]), 1);
+      mbar_init(smem_u32(&sm->bar_o2[s]), 1);
       mbar_init(smem_u32(&sm->bar_b[s]), 1);
-      mbar_init(smem_u32(&sm->o_done[s]), 256);
+      mbar_init(smem_u32(&sm->s_done[s]), STATE_WARPS);
+      mbar_init(smem_u32(&sm->p_done[s]), CON_WARPS);
+      mbar_init(smem_u32(&sm->o_done[s]), CON_WARPS);
     }
-    mbar_init(smem_u32(&sm->bar_s), 1);
-    mbar_init(smem_u32(&sm->s_done), 256);
-    mbar_init(smem_u32(&sm->p_done), 256);
+    for (int s = 0; s < NTAB; ++s) mbar_init(smem_u32(&sm->tab_full[s]), STATE_WARPS);
     sm->abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
+    tma_prefetch_desc(&tm_o);
   }
   if (warp == 0) {
     __syncwarp();                 // tcgen05.alloc is warp-collective: lane 0 rejoins from the barrier set-up first
@@ -405,38 +497,20 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
   // `settled`: the decay tables too are made while the kernel before this one runs, unless the head is not known before the
   // ticket is.
-  const bool tables_first = p.settled && p.n_split == 0;
+  const bool tables_first = p.settled && !p.split;
   if (!tables_first) {
     pdl_wait();
     pdl_trigger();
   }
-  // Which chunks of which sequence-head this CTA scans.  piece: 0 a whole sequence-head or a pre-passed segment,
-  // 1 the first part of a cut one (leaves its end state in handoff), 2 the second part (starts from it).
-  int h = blockIdx.x, b = blockIdx.y, seg = blockIdx.z, piece = 0;
-  int ck_begin = seg * p.seg_chunks, ck_end = min(n_chunks, ck_begin + p.seg_chunks);
-  if (p.n_split > 0) {
-    // a ticket instead of the block index: whoever holds a second part started after every first part was taken
+  int cta = blockIdx.x;
+  if (p.split) {
+    // a ticket instead of the block index: whoever holds a second part started after the first part was taken
     if (tid == 0) sm->ticket = atomicAdd(p.ctrl, 1);
     __syncthreads();
-    const int t = sm->ticket, U = p.B * p.H;
-    seg = 0;
-    int unit = t;                                     // = b * H + h
-    if (t < p.n_split) { piece = 1; ck_begin = 0; ck_end = p.split_chunk; }
-    else if (t < U) { ck_begin = 0; ck_end = n_chunks; }
-    else { unit = t - U; piece = 2; ck_begin = p.split_chunk; ck_end = n_chunks; }
-    b = unit / p.H;
-    h = unit - b * p.H;
+    cta = sm->ticket;
   }
-  const int n_loc = ck_end - ck_begin;
-  const int row0 = b * T;
-  const float log_g = logf(__ldg(p.gamma + h));
-  for (int n = tid; n <= CH; n += PIPE_THREADS) sm->pw[n] = expf(log_g * float(n));
-  for (int n = tid; n < 2 * CH; n += PIPE_THREADS) {
-    // gamma^(i-j) / sqrt(D): the 1/8 of the query feature map is a power of two, so applying it to the scores
-    // (and to the cross-chunk factor) instead of to every element of q gives the same bits
-    const int x = n - CH;
-    sm->pwm[n] = x >= 0 ? 0.125f * expf(log_g * float(x)) : 0.f;
-  }
+  const Share share(p, cta, n_chunks);
+  fill_tab(sm->tab[0], logf(__ldg(p.gamma + share.at(0).unit % p.H)), tid, PIPE_THREADS);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -447,126 +521,137 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     pdl_trigger();
   }
 
+  // Chunks are counted over all items (g): stages, accumulators and barrier phases follow that count.
+  if (warp < PRO_WARP0) {
+    regs_dec<ISSUE_REGS>();
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      JB_T_DECL
-      int s = 0;
-      uint32_t prev = 1u;                       // parity of the PREVIOUS use of the stage
-      for (int lc = 0; lc < n_loc; ++lc) {
-        const int r = row0 + (ck_begin + lc) * CH;
+    JB_T_DECL
+    int s = 0, g = 0;
+    uint32_t prev = 1u;                         // parity of the PREVIOUS use of the stage
+    bool ok = true;
+    for (int k = 0; ok && k < share.n_items; ++k) {
+      const Item it = share.at(k);
+      const int b = it.unit / p.H, col = (it.unit - b * p.H) * D;
+      for (int ck = it.begin; ck < it.end; ++ck, ++g) {
+        const int r = b * T + ck * CH;
         JB_T_MARK(0)
-        if (lc >= NST && !mbar_wait(smem_u32(&sm->empty_qk[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+        if (g >= NST && !mbar_wait(smem_u32(&sm->empty_qk[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
         JB_T_MARK(1)
-        mbar_arrive_expect_tx(smem_u32(&sm->full_qk[s]), 2 * TILE_BYTES);
-        tma_load_2d(smem_u32(sm->q[s]), &tm_q, h * D, r, smem_u32(&sm->full_qk[s]));
-        tma_load_2d(smem_u32(sm->k[s]), &tm_k, h * D, r, smem_u32(&sm->full_qk[s]));
+        if (elect_one()) {
+          mbar_arrive_expect_tx(smem_u32(&sm->full_qk[s]), 2 * TILE_BYTES);
+          tma_load_2d(smem_u32(sm->k[s]), &tm_k, col, r, smem_u32(&sm->full_qk[s]));
+          tma_load_2d(smem_u32(sm->q[s]), &tm_q, col, r, smem_u32(&sm->full_qk[s]));
+        }
+        __syncwarp();
         JB_T_MARK(0)
-        if (lc >= NST && !mbar_wait(smem_u32(&sm->empty_v[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+        if (g >= NST && !mbar_wait(smem_u32(&sm->empty_v[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
         JB_T_MARK(2)
-        mbar_arrive_expect_tx(smem_u32(&sm->full_v[s]), TILE_BYTES);
-        tma_load_2d(smem_u32(sm->v[s]), &tm_v, h * D, r, smem_u32(&sm->full_v[s]));
+        if (elect_one()) {
+          mbar_arrive_expect_tx(smem_u32(&sm->full_v[s]), TILE_BYTES);
+          tma_load_2d(smem_u32(sm->v[s]), &tm_v, col, r, smem_u32(&sm->full_v[s]));
+        }
+        __syncwarp();
         if (++s == NST) { s = 0; prev ^= 1u; }
       }
-      JB_T_MARK(0)
-      JB_T_FLUSH(0)
     }
+    JB_T_MARK(0)
+    JB_T_FLUSH(0)
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t id_sc = umma_idesc(128, 128, 0, 0), id_o2 = umma_idesc(128, 64, 0, 0);
-      constexpr uint32_t id_ds = umma_idesc(128, 64, 1, 1), id_o1 = umma_idesc(128, 64, 0, 1);
-      // Operand descriptors of stage 0; stage s is +s*TILE_BYTES (+1024 in the address field).  A K-step of 16
-      // elements is +32 bytes (+2) inside a K-major row, +2048 bytes (+128: two 8-row groups) in the MN-major
-      // [token][64] tiles.
-      constexpr uint64_t STG = TILE_BYTES >> 4;
-      const uint64_t d_q0 = umma_desc(smem_u32(sm->q[0]), 16, 1024), d_k0 = umma_desc(smem_u32(sm->k[0]), 16, 1024);
-      const uint64_t d_kw0 = umma_desc(smem_u32(sm->kw[0]), 1024, 1024);
-      const uint64_t d_va0 = umma_desc(smem_u32(sm->v[0]), 0, 1024);      // as the M operand of dS: the 64 dv read twice
-      const uint64_t d_vb0 = umma_desc(smem_u32(sm->v[0]), 1024, 1024);   // as the N operand of P V
-      const uint64_t d_s0 = umma_desc(smem_u32(sm->s[0]), 16, 1024);
-      auto issue_scores = [&](int stage, int buf) {
-        const uint64_t dq = d_q0 + uint64_t(stage) * STG, dk = d_k0 + uint64_t(stage) * STG;
+    // ---------------- MMA issuer: scores, dS, O2 ----------------
+    constexpr uint32_t id_sc = umma_idesc(128, 128, 0, 0), id_o2 = umma_idesc(128, 64, 0, 0), id_ds = umma_idesc(128, 64, 1, 1);
+    // Operand descriptors of stage 0; stage s is +s*TILE_BYTES (+1024 in the address field).  A K-step of 16
+    // elements is +32 bytes (+2) inside a K-major row, +2048 bytes (+128: two 8-row groups) in the MN-major
+    // [token][64] tiles.
+    constexpr uint64_t STG = TILE_BYTES >> 4;
+    const uint64_t d_q0 = umma_desc(smem_u32(sm->q[0]), 16, 1024), d_k0 = umma_desc(smem_u32(sm->k[0]), 16, 1024);
+    const uint64_t d_kw0 = umma_desc(smem_u32(sm->kw[0]), 1024, 1024);
+    const uint64_t d_v0 = umma_desc(smem_u32(sm->v[0]), 0, 1024);       // as the M operand of dS: the 64 dv read twice
+    const uint64_t d_s0 = umma_desc(smem_u32(sm->s[0]), 16, 1024);
+    const int n_tot = share.chunks();
+    JB_T_DECL
+    int s = 0;                                   // stage of chunk g
+    uint32_t sp = 0u;                            // parity of this use of the stage
+    for (int g = 0; g < n_tot; ++g) {
+      const int buf = g & 1;                     // accumulators and the state copy alternate
+      const uint32_t u = uint32_t(g >> 1) & 1u;
+      const uint64_t dq = d_q0 + uint64_t(s) * STG, dk = d_k0 + uint64_t(s) * STG, dkw = d_kw0 + uint64_t(s) * STG;
+      const uint64_t dv = d_v0 + uint64_t(s) * STG, ds = d_s0 + uint64_t(buf) * (S_BYTES >> 4);
+      JB_T_MARK(0)
+      if (!mbar_wait(smem_u32(&sm->pro_done[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+      JB_T_MARK(1)
+      // the output rows of chunk g - 2 have left SC[buf] and O2[buf]
+      if (g >= 2 && !mbar_wait(smem_u32(&sm->o_done[buf]), u ^ 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+      JB_T_MARK(2)
+      tc_fence_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           umma_bf16_ss(tm + PT_SC + 128 * buf, dq + uint64_t(ks * 2), dk + uint64_t(ks * 2), id_sc, ks != 0);
         umma_commit(smem_u32(&sm->bar_sc[buf]));
-      };
-      JB_T_DECL
-      bool ok = n_loc > 0 && mbar_wait(smem_u32(&sm->pro_done[0]), 0u, abort_flag, p.status, JB200_STATUS_ATTN_MMA);
-      JB_T_MARK(4)
-      if (ok) {
-        tc_fence_after_sync();
-        issue_scores(0, 0);
       }
-      int s = 0;                                 // stage of chunk lc
-      uint32_t sp = 0u;                          // parity of this use of the stage
-      for (int lc = 0; ok && lc < n_loc; ++lc) {
-        const int buf = lc & 1;                  // accumulator buffers SC / O2 and the state copy alternate
-        const uint32_t u = uint32_t(lc >> 1) & 1u;
-        const int s1 = s + 1 == NST ? 0 : s + 1; // stage and parity of chunk lc + 1
-        const uint32_t sp1 = s + 1 == NST ? sp ^ 1u : sp;
-        const uint64_t dq = d_q0 + uint64_t(s) * STG, dkw = d_kw0 + uint64_t(s) * STG;
-        const uint64_t dva = d_va0 + uint64_t(s) * STG, dvb = d_vb0 + uint64_t(s) * STG;
-        const uint64_t ds = d_s0 + uint64_t(buf) * (S_BYTES >> 4);
-        // S(lc): needs v of the chunk, and the consumers to be done with the previous dS (completion #lc of s_done,
-        // which also says that s[lc & 1] holds the state after lc chunks)
-        JB_T_MARK(0)
-        if (!mbar_wait(smem_u32(&sm->full_v[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
-        JB_T_MARK(1)
-        if (!mbar_wait(smem_u32(&sm->s_done), uint32_t(lc) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-        JB_T_MARK(2)
-        tc_fence_after_sync();
+      __syncwarp();
+      JB_T_MARK(0)
+      if (!mbar_wait(smem_u32(&sm->full_v[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+      JB_T_MARK(3)
+      // DS[buf] was read before the state before chunk g - 1 was published, which A2(g - 1) waited for
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(tm + PT_DS, dva + uint64_t(ks * 128), dkw + uint64_t(ks * 128), id_ds, ks != 0);
-        umma_commit(smem_u32(&sm->bar_s));
-        // A2(lc): O2 = Q' S^T.  O2[buf] was read by the output rows of chunk lc - 2, which the scores of this chunk
-        // (issued into SC[buf] earlier) already waited for.
+          umma_bf16_ss(tm + PT_DS + 64 * buf, dv + uint64_t(ks * 128), dkw + uint64_t(ks * 128), id_ds, ks != 0);
+        umma_commit(smem_u32(&sm->bar_s[buf]));
+      }
+      __syncwarp();
+      JB_T_MARK(0)
+      if (!mbar_wait(smem_u32(&sm->s_done[buf]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+      JB_T_MARK(4)
+      tc_fence_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           umma_bf16_ss(tm + PT_O2 + 64 * buf, dq + uint64_t(ks * 2), ds + uint64_t(ks * 2), id_o2, ks != 0);
-        umma_commit(smem_u32(&sm->empty_qk[s]));       // q, k, kw of this stage: every MMA that reads them is issued
-        // A1(lc + 1): scores of the next chunk into the other accumulator, ahead of B(lc) when the next chunk's
-        // prologue is already done (then the consumers find them ready when they finish this chunk)
-        bool scores_issued = lc + 1 >= n_loc;
-        if (!scores_issued && mbar_try_wait(smem_u32(&sm->pro_done[s1]), sp1) &&
-            (lc + 1 < 2 || mbar_try_wait(smem_u32(&sm->o_done[buf ^ 1]), (uint32_t((lc + 1) >> 1) - 1u) & 1u))) {
-          tc_fence_after_sync();
-          issue_scores(s1, buf ^ 1);
-          scores_issued = true;
-        }
-        // B(lc): O1 = P V into the score columns the mask step has fully read; P (bf16 pairs) is read from TMEM
-        JB_T_MARK(0)
-        if (!mbar_wait(smem_u32(&sm->p_done), uint32_t(lc) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-        JB_T_MARK(3)
-        tc_fence_after_sync();
+        umma_commit(smem_u32(&sm->bar_o2[buf]));
+        umma_commit(smem_u32(&sm->empty_qk[s]));       // q, k, kw of this stage, and v but for B(g)
+      }
+      __syncwarp();
+      if (++s == NST) { s = 0; sp ^= 1u; }
+    }
+    JB_T_MARK(0)
+    JB_T_FLUSH(1)
+  } else if (warp == 2) {
+    // ---------------- MMA issuer: O1 = P V into the score columns the mask has read; P is read from TMEM ----------------
+    constexpr uint32_t id_o1 = umma_idesc(128, 64, 0, 1);
+    const uint64_t d_v0 = umma_desc(smem_u32(sm->v[0]), 1024, 1024);    // as the N operand
+    const int n_tot = share.chunks();
+    JB_T_DECL
+    int s = 0;
+    uint32_t sp = 0u;
+    for (int g = 0; g < n_tot; ++g) {
+      const int buf = g & 1;
+      const uint64_t dv = d_v0 + uint64_t(s) * (TILE_BYTES >> 4);
+      JB_T_MARK(0)
+      if (!mbar_wait(smem_u32(&sm->full_v[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+      if (!mbar_wait(smem_u32(&sm->p_done[buf]), uint32_t(g >> 1) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+      if (n_tot == 1 && !mbar_wait(smem_u32(&sm->p_done[1]), 0u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+      JB_T_MARK(1)
+      tc_fence_after_sync();
+      const uint32_t tm_p = tm + PT_SC + PT_P + (n_tot == 1 ? 128 : 128 * buf);
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ts(tm + PT_SC + 128 * buf, tm + PT_P + ks * 8, dvb + uint64_t(ks * 128), id_o1, ks != 0);
+          umma_bf16_ts(tm + PT_SC + 128 * buf, tm_p + ks * 8, dv + uint64_t(ks * 128), id_o1, ks != 0);
         umma_commit(smem_u32(&sm->bar_b[buf]));
-        umma_commit(smem_u32(&sm->empty_v[s]));
-        if (!scores_issued) {
-          JB_T_MARK(0)
-          if (!mbar_wait(smem_u32(&sm->pro_done[s1]), sp1, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-          JB_T_MARK(4)
-          if (lc + 1 >= 2 && !mbar_wait(smem_u32(&sm->o_done[buf ^ 1]), (uint32_t((lc + 1) >> 1) - 1u) & 1u, abort_flag,
-                                        p.status, JB200_STATUS_ATTN_MMA)) break;
-          JB_T_MARK(5)
-          tc_fence_after_sync();
-          issue_scores(s1, buf ^ 1);
-        }
-        (void)u;
-        s = s1;
-        sp = sp1;
       }
-      JB_T_MARK(0)
-      JB_T_FLUSH(1)
+      __syncwarp();
+      if (++s == NST) { s = 0; sp ^= 1u; }
     }
-  } else if (warp < CON_WARP0) {
+    JB_T_MARK(0)
+    JB_T_FLUSH(2)
+  }
+  } else if (warp < STATE_WARP0) {
+    regs_inc<PRO_REGS>();
     // ---------------- prologue warps ----------------
     const int ptid = tid - PRO_WARP0 * 32;
-    const int pos_base = p.pos0 ? p.pos0[b] : p.pos0_scalar;
     // 128 rows x 4 column groups of 8 rotary pairs = 512 items per chunk, two per thread: (row r, group cg) and
     // (row r + 64, group cg).  Eight consecutive lanes take 4 groups of two rows that are 4 apart, so that their
     // 16-byte accesses to the swizzled tiles fall into different banks.
@@ -578,289 +663,401 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // away (angle addition in f32: error ~1e-7 against the 4e-3 of the bf16 result).  Every chunk starts from
     // the table again, so results do not depend on how a sequence is cut into segments or calls.
     float cs[8], sn[8], c64[8], s64[8];
-    auto load_angles = [&](int ck) {
-      int pos = pos_base + ck * CH + r_lo;
+    auto load_angles = [&](int unit, int ck) {
+      int pos = (p.pos0 ? p.pos0[unit / p.H] : p.pos0_scalar) + ck * CH + r_lo;
       pos = pos < 0 ? 0 : (pos >= p.n_pos ? p.n_pos - 1 : pos);
-      const float4* cp = reinterpret_cast<const float4*>(p.cos_tab + size_t(pos) * 32 + cg * 8);
-      const float4* sp = reinterpret_cast<const float4*>(p.sin_tab + size_t(pos) * 32 + cg * 8);
-      const float4 a0 = __ldg(cp), a1 = __ldg(cp + 1), b0 = __ldg(sp), b1 = __ldg(sp + 1);
-      cs[0] = a0.x; cs[1] = a0.y; cs[2] = a0.z; cs[3] = a0.w; cs[4] = a1.x; cs[5] = a1.y; cs[6] = a1.z; cs[7] = a1.w;
-      sn[0] = b0.x; sn[1] = b0.y; sn[2] = b0.z; sn[3] = b0.w; sn[4] = b1.x; sn[5] = b1.y; sn[6] = b1.z; sn[7] = b1.w;
+      load_angles8(p.cos_tab + size_t(pos) * 32 + cg * 8, p.wide_tab, cs);
+      load_angles8(p.sin_tab + size_t(pos) * 32 + cg * 8, p.wide_tab, sn);
     };
     {
       const int stp = 64 < p.n_pos ? 64 : p.n_pos - 1;     // tables shorter than 65 rows: rows >= 64 are past the end anyway
-      const float4* cq = reinterpret_cast<const float4*>(p.cos_tab + size_t(stp) * 32 + cg * 8);
-      const float4* sq = reinterpret_cast<const float4*>(p.sin_tab + size_t(stp) * 32 + cg * 8);
-      const float4 d0 = __ldg(cq), d1 = __ldg(cq + 1), e0 = __ldg(sq), e1 = __ldg(sq + 1);
-      c64[0] = d0.x; c64[1] = d0.y; c64[2] = d0.z; c64[3] = d0.w; c64[4] = d1.x; c64[5] = d1.y; c64[6] = d1.z; c64[7] = d1.w;
-      s64[0] = e0.x; s64[1] = e0.y; s64[2] = e0.z; s64[3] = e0.w; s64[4] = e1.x; s64[5] = e1.y; s64[6] = e1.z; s64[7] = e1.w;
-      load_angles(ck_begin);
+      load_angles8(p.cos_tab + size_t(stp) * 32 + cg * 8, p.wide_tab, c64);
+      load_angles8(p.sin_tab + size_t(stp) * 32 + cg * 8, p.wide_tab, s64);
     }
     JB_T_DECL
     int s = 0;
     uint32_t sp = 0u;
-    for (int lc = 0; lc < n_loc; ++lc) {
-      const int ck = ck_begin + lc;
-      const int c_len = min(CH, T - ck * CH);
-      uint8_t* q_p = sm->q[s];
-      uint8_t* k_p = sm->k[s];
-      uint8_t* kw_p = sm->kw[s];
+    bool ok = true;
+    for (int k = 0; ok && k < share.n_items; ++k) {
+      const Item itm = share.at(k);
+      const float* pw = sm->tab[k % NTAB].pw;
+      if (k == 0 && !PREPARED) load_angles(itm.unit, itm.begin);
       JB_T_MARK(0)
-      if (!mbar_wait(smem_u32(&sm->full_qk[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
-      JB_T_MARK(1)
+      if (k > 0 && !mbar_wait(smem_u32(&sm->tab_full[k % NTAB]), uint32_t(k / NTAB) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+      JB_T_MARK(4)
+      for (int ck = itm.begin; ck < itm.end; ++ck) {
+        const int c_len = min(CH, T - ck * CH);
+        uint8_t* q_p = sm->q[s];
+        uint8_t* k_p = sm->k[s];
+        uint8_t* kw_p = sm->kw[s];
+        JB_T_MARK(0)
+        if (!mbar_wait(smem_u32(&sm->full_qk[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
+        JB_T_MARK(1)
+#pragma unroll 1
+        for (int it = 0; it < 2; ++it) {
+          const int r = r_lo + 64 * it;
+          const float w = r < c_len ? pw[c_len - 1 - r] : 0.f;   // rows past the end contribute nothing
+          if (PREPARED) {
+            // q', k' came out of the projection's epilogue: only the decay-weighted copy of k is made here
+            const uint4 lo = *reinterpret_cast<const uint4*>(k_p + swz(r, cg));
+            const uint4 hi = *reinterpret_cast<const uint4*>(k_p + swz(r, cg + 4));
+            *reinterpret_cast<uint4*>(kw_p + swz(r, cg)) =
+                make_uint4(pack_bf16x2(bf16_lo(lo.x) * w, bf16_hi(lo.x) * w), pack_bf16x2(bf16_lo(lo.y) * w, bf16_hi(lo.y) * w),
+                           pack_bf16x2(bf16_lo(lo.z) * w, bf16_hi(lo.z) * w), pack_bf16x2(bf16_lo(lo.w) * w, bf16_hi(lo.w) * w));
+            *reinterpret_cast<uint4*>(kw_p + swz(r, cg + 4)) =
+                make_uint4(pack_bf16x2(bf16_lo(hi.x) * w, bf16_hi(hi.x) * w), pack_bf16x2(bf16_lo(hi.y) * w, bf16_hi(hi.y) * w),
+                           pack_bf16x2(bf16_lo(hi.z) * w, bf16_hi(hi.z) * w), pack_bf16x2(bf16_lo(hi.w) * w, bf16_hi(hi.w) * w));
+            continue;
+          }
+          // all four 16-byte pieces of the row pair first, so that their latencies overlap
+          uint4* ql_p = reinterpret_cast<uint4*>(q_p + swz(r, cg));
+          uint4* qh_p = reinterpret_cast<uint4*>(q_p + swz(r, cg + 4));
+          uint4* kl_p = reinterpret_cast<uint4*>(k_p + swz(r, cg));
+          uint4* kh_p = reinterpret_cast<uint4*>(k_p + swz(r, cg + 4));
+          const uint4 ql = *ql_p, qh = *qh_p, kl = *kl_p, kh = *kh_p;
 #pragma unroll
-      for (int it = 0; it < 2; ++it) {
-        const int r = r_lo + 64 * it;
-        const float w = r < c_len ? sm->pw[c_len - 1 - r] : 0.f;   // rows past the end contribute nothing
-        if (p.qk_prepared) {
-          // q', k' came out of the projection's epilogue: only the decay-weighted copy of k is made here
-          const uint4 lo = *reinterpret_cast<const uint4*>(k_p + swz(r, cg));
-          const uint4 hi = *reinterpret_cast<const uint4*>(k_p + swz(r, cg + 4));
-          *reinterpret_cast<uint4*>(kw_p + swz(r, cg)) =
-              make_uint4(pack_bf16x2(bf16_lo(lo.x) * w, bf16_hi(lo.x) * w), pack_bf16x2(bf16_lo(lo.y) * w, bf16_hi(lo.y) * w),
-                         pack_bf16x2(bf16_lo(lo.z) * w, bf16_hi(lo.z) * w), pack_bf16x2(bf16_lo(lo.w) * w, bf16_hi(lo.w) * w));
-          *reinterpret_cast<uint4*>(kw_p + swz(r, cg + 4)) =
-              make_uint4(pack_bf16x2(bf16_lo(hi.x) * w, bf16_hi(hi.x) * w), pack_bf16x2(bf16_lo(hi.y) * w, bf16_hi(hi.y) * w),
-                         pack_bf16x2(bf16_lo(hi.z) * w, bf16_hi(hi.z) * w), pack_bf16x2(bf16_lo(hi.w) * w, bf16_hi(hi.w) * w));
-          continue;
-        }
-        // all four 16-byte pieces of the row pair first, so that their latencies overlap
-        uint4* ql_p = reinterpret_cast<uint4*>(q_p + swz(r, cg));
-        uint4* qh_p = reinterpret_cast<uint4*>(q_p + swz(r, cg + 4));
-        uint4* kl_p = reinterpret_cast<uint4*>(k_p + swz(r, cg));
-        uint4* kh_p = reinterpret_cast<uint4*>(k_p + swz(r, cg + 4));
-        const uint4 ql = *ql_p, qh = *qh_p, kl = *kl_p, kh = *kh_p;
+          for (int which = 0; which < 2; ++which) {  // 0: q, 1: k
+            const uint4 lo = which == 0 ? ql : kl, hi = which == 0 ? qh : kh;
+            const uint32_t lw[4] = {lo.x, lo.y, lo.z, lo.w}, hw[4] = {hi.x, hi.y, hi.z, hi.w};
+            uint32_t ol[4], oh[4], wl[4], wh[4];
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {  // 0: q, 1: k
-          const uint4 lo = which == 0 ? ql : kl, hi = which == 0 ? qh : kh;
-          const uint32_t lw[4] = {lo.x, lo.y, lo.z, lo.w}, hw[4] = {hi.x, hi.y, hi.z, hi.w};
-          uint32_t ol[4], oh[4], wl[4], wh[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float a0 = elu1(bf16_lo(lw[j])), a1 = elu1(bf16_hi(lw[j]));   // d
-            const float b0 = elu1(bf16_lo(hw[j])), b1 = elu1(bf16_hi(hw[j]));   // d + 32
-            // x*cos + rotate_half(x)*sin:  out[d] = x[d]cos - x[d+32]sin,  out[d+32] = x[d+32]cos + x[d]sin
-            const float l0 = a0 * cs[2 * j] - b0 * sn[2 * j], l1 = a1 * cs[2 * j + 1] - b1 * sn[2 * j + 1];
-            const float h0 = b0 * cs[2 * j] + a0 * sn[2 * j], h1 = b1 * cs[2 * j + 1] + a1 * sn[2 * j + 1];
-            ol[j] = pack_bf16x2(l0, l1);
-            oh[j] = pack_bf16x2(h0, h1);
+            for (int j = 0; j < 4; ++j) {
+              const float a0 = elu1(bf16_lo(lw[j])), a1 = elu1(bf16_hi(lw[j]));   // d
+              const float b0 = elu1(bf16_lo(hw[j])), b1 = elu1(bf16_hi(hw[j]));   // d + 32
+              // x*cos + rotate_half(x)*sin:  out[d] = x[d]cos - x[d+32]sin,  out[d+32] = x[d+32]cos + x[d]sin
+              const float l0 = a0 * cs[2 * j] - b0 * sn[2 * j], l1 = a1 * cs[2 * j + 1] - b1 * sn[2 * j + 1];
+              const float h0 = b0 * cs[2 * j] + a0 * sn[2 * j], h1 = b1 * cs[2 * j + 1] + a1 * sn[2 * j + 1];
+              ol[j] = pack_bf16x2(l0, l1);
+              oh[j] = pack_bf16x2(h0, h1);
+              if (which == 1) {
+                wl[j] = pack_bf16x2(l0 * w, l1 * w);
+                wh[j] = pack_bf16x2(h0 * w, h1 * w);
+              }
+            }
+            *(which == 0 ? ql_p : kl_p) = make_uint4(ol[0], ol[1], ol[2], ol[3]);
+            *(which == 0 ? qh_p : kh_p) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
             if (which == 1) {
-              wl[j] = pack_bf16x2(l0 * w, l1 * w);
-              wh[j] = pack_bf16x2(h0 * w, h1 * w);
+              *reinterpret_cast<uint4*>(kw_p + swz(r, cg)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+              *reinterpret_cast<uint4*>(kw_p + swz(r, cg + 4)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
             }
           }
-          *(which == 0 ? ql_p : kl_p) = make_uint4(ol[0], ol[1], ol[2], ol[3]);
-          *(which == 0 ? qh_p : kh_p) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
-          if (which == 1) {
-            *reinterpret_cast<uint4*>(kw_p + swz(r, cg)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-            *reinterpret_cast<uint4*>(kw_p + swz(r, cg + 4)) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+          if (it == 0) {             // advance the angles by 64 positions: to the thread's second row
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float cn = cs[e] * c64[e] - sn[e] * s64[e];
+              sn[e] = sn[e] * c64[e] + cs[e] * s64[e];
+              cs[e] = cn;
+            }
           }
         }
-        if (it == 0) {             // advance the angles by 64 positions: to the thread's second row
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float cn = cs[e] * c64[e] - sn[e] * s64[e];
-            sn[e] = sn[e] * c64[e] + cs[e] * s64[e];
-            cs[e] = cn;
+        if (!PREPARED) {
+          if (ck + 1 < itm.end) {
+            load_angles(itm.unit, ck + 1);
+          } else if (k + 1 < share.n_items) {
+            const Item nx = share.at(k + 1);
+            load_angles(nx.unit, nx.begin);
           }
+        }
+        JB_T_MARK(2)
+        fence_proxy_async_smem();                          // generic-proxy writes -> visible to the tensor core
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm->pro_done[s]));
+        JB_T_MARK(3)
+        if (++s == NST) { s = 0; sp ^= 1u; }
+      }
+    }
+    JB_T_FLUSH(warp)
+  } else if (warp < CON_WARP0) {
+    // ---------------- state ----------------
+    
+    // f32 state: row dv = 32*(qd&1) + lane, columns dk = 32*half .. +31 (the accumulator of MMA S holds the 64 dv rows
+    // twice, lanes 0-63 and 64-127, so every warp finds its share in its own lane quarter)
+    const int qd = warp & 3, half = qd >> 1, s_row = 32 * (qd & 1) + lane;
+    const int stid = tid - STATE_WARP0 * 32;
+    const uint32_t tm_ds = tm + (uint32_t(32 * qd) << 16) + PT_DS + 32 * half;
+    float S[32];
+    auto add4 = [&](const float* src, float f, bool coherent) {        // S = f * S + src, 16 bytes at a time
+#pragma unroll
+      for (int e4 = 0; e4 < 8; ++e4) {
+        const float4 v4 = coherent ? __ldcg(reinterpret_cast<const float4*>(src) + e4) : __ldg(reinterpret_cast<const float4*>(src) + e4);
+        S[4 * e4 + 0] = f * S[4 * e4 + 0] + v4.x; S[4 * e4 + 1] = f * S[4 * e4 + 1] + v4.y;
+        S[4 * e4 + 2] = f * S[4 * e4 + 2] + v4.z; S[4 * e4 + 3] = f * S[4 * e4 + 3] + v4.w;
+      }
+    };
+    auto publish_state = [&](int buf) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        *reinterpret_cast<uint4*>(sm->s[buf] + swz(s_row, 4 * half + c)) =
+            make_uint4(pack_bf16x2(S[8 * c], S[8 * c + 1]), pack_bf16x2(S[8 * c + 2], S[8 * c + 3]),
+                       pack_bf16x2(S[8 * c + 4], S[8 * c + 5]), pack_bf16x2(S[8 * c + 6], S[8 * c + 7]));
+      }
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm->s_done[buf]));
+    };
+    JB_T_DECL
+    bool ok = true;
+    int g = 0;
+    for (int k = 0; ok && k < share.n_items; ++k) {
+      const Item it = share.at(k);
+      const int h = it.unit % p.H;
+      const size_t bh = size_t(it.unit);
+      const float* pw = sm->tab[k % NTAB].pw;
+#pragma unroll
+      for (int e = 0; e < 32; ++e) S[e] = 0.f;
+      if (it.piece == 2) {
+        // second part of a cut sequence-head: the state after the first part, written by the state warps of the CTA that
+        // scanned it (in this kernel's own element order).  Bounded wait on their count.
+        if (lane == 0) {
+          int* flag = p.ctrl + cta;                      // 1 + (the ticket before this one)
+          const unsigned long long t0 = globaltimer_ns();
+          int seen;
+          for (;;) {
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
+            if (seen >= STATE_WARPS || *abort_flag) break;
+            if (globaltimer_ns() - t0 > JB_WAIT_LIMIT_NS) {
+              *abort_flag = 1u;
+              atomicCAS(p.status, 0u, JB200_STATUS_ATTN_HANDOFF);
+              break;
+            }
+            __nanosleep(200);
+          }
+        }
+        __syncwarp();
+        __threadfence();
+        add4(p.handoff + size_t(cta - 1) * D * D + s_row * D + 32 * half, 0.f, true);
+      } else {
+        if (p.s_in) {
+          const float* sp = p.s_in + bh * D * D + s_row * D;
+          if (PREPARED) {      // prepared q/k: the dk axis is interleaved
+#pragma unroll
+            for (int e = 0; e < 32; ++e) S[e] = __ldg(sp + (16 * half + (e >> 1)) + 32 * (e & 1));
+          } else {
+            add4(sp + 32 * half, 0.f, false);
+          }
+        }
+        if (it.begin > 0) {   // state entering this segment: fold the earlier segments' contributions, oldest first
+          const float gL = expf(logf(__ldg(p.gamma + h)) * float(p.seg_chunks * CH));
+          const float* dp = p.seg_state + bh * p.n_pieces * D * D + s_row * D + 32 * half;
+          for (int s2 = it.begin / p.seg_chunks; s2 > 0; --s2, dp += D * D) add4(dp, gL, false);
         }
       }
-      if (!p.qk_prepared && lc + 1 < n_loc) load_angles(ck + 1);
-      JB_T_MARK(2)
-      fence_proxy_async_smem();                          // generic-proxy writes -> visible to the tensor core
-      mbar_arrive(smem_u32(&sm->pro_done[s]));
-      JB_T_MARK(3)
-      if (++s == NST) { s = 0; sp ^= 1u; }
+      JB_T_MARK(0)
+      publish_state(g & 1);
+      // decay tables, two sequence-heads ahead (the first one's are there)
+      for (int n = k == 0 ? 0 : k + 2; n <= k + 2 && n < share.n_items; ++n) {
+        if (n > 0) fill_tab(sm->tab[n % NTAB], logf(__ldg(p.gamma + share.at(n).unit % p.H)), stid, 32 * STATE_WARPS);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm->tab_full[n % NTAB]));
+      }
+      if (k > 0 && !mbar_wait(smem_u32(&sm->tab_full[k % NTAB]), uint32_t(k / NTAB) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
+      JB_T_MARK(1)
+      for (int ck = it.begin; ck < it.end; ++ck, ++g) {
+        const float gc = pw[min(CH, T - ck * CH)];
+        JB_T_MARK(0)
+        if (!mbar_wait(smem_u32(&sm->bar_s[g & 1]), uint32_t(g >> 1) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
+        JB_T_MARK(2)
+        tc_fence_after_sync();
+        __syncwarp();               // tcgen05.ld / st are warp-collective: rejoin after the per-thread wait
+        uint32_t r[32];
+        tmem_ld_32x32(tm_ds + 64 * (g & 1), r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 32; ++e) S[e] = gc * S[e] + __uint_as_float(r[e]);
+        if (ck + 1 < it.end) publish_state((g + 1) & 1);
+        JB_T_MARK(3)
+      }
+      if (!ok) break;
+      if (it.piece == 1) {
+        // first part of a cut sequence-head: its end state for the CTA that takes the second part
+        float* hp = p.handoff + size_t(cta) * D * D + s_row * D + 32 * half;
+#pragma unroll
+        for (int e4 = 0; e4 < 8; ++e4)
+          __stcg(reinterpret_cast<float4*>(hp) + e4, make_float4(S[4 * e4], S[4 * e4 + 1], S[4 * e4 + 2], S[4 * e4 + 3]));
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) atomicAdd(p.ctrl + 1 + cta, 1);
+      } else if (p.s_out && it.end == n_chunks) {
+        float* sp = p.s_out + bh * D * D + s_row * D;
+        if (PREPARED) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sp[(16 * half + (e >> 1)) + 32 * (e & 1)] = S[e];
+        } else {
+#pragma unroll
+          for (int e4 = 0; e4 < 8; ++e4)
+            *reinterpret_cast<float4*>(sp + 32 * half + 4 * e4) = make_float4(S[4 * e4], S[4 * e4 + 1], S[4 * e4 + 2], S[4 * e4 + 3]);
+        }
+      }
     }
     JB_T_FLUSH(warp)
   } else {
     // ---------------- consumers ----------------
+    regs_inc<CON_REGS>();
     const int qd = warp & 3;                             // TMEM lane quarter of this warp
-    const int hf = (warp - CON_WARP0) >> 2;              // which half of the columns it takes
-    const uint32_t tm_lane = tm + (uint32_t(32 * qd) << 16);
+    const int grp = (warp - CON_WARP0) / CON_WARPS;      // takes the chunks with this parity
     const int i = 32 * qd + lane;                        // query row = TMEM lane
-    // fp32 state: row dv = 32*(qd&1) + lane, columns dk = 16*cg .. 16*cg+15 (the accumulator of MMA S holds the
-    // 64 dv rows twice, lanes 0-63 and 64-127, so every consumer warp finds its share in its own lane quarter)
-    const int s_row = 32 * (qd & 1) + lane;
-    const int s_cg = 2 * (qd >> 1) + hf;
-    const size_t bh = size_t(b) * p.H + h;
-    // P lives in TMEM as bf16 pairs: lane = query row, column c = keys 2c, 2c+1.  32-key blocks above the diagonal
-    // of this warp's rows are never written by the mask step: zero them once.
-    {
-      uint32_t z[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) z[e] = 0u;
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const int jb = 2 * hf + jj;
-        if (jb > qd) tmem_st_32x16(tm_lane + PT_P + 16 * jb, z);
-      }
-      tmem_st_wait();
-    }
-    float S[16];
-    if (piece == 2) {
-      // second part of a cut sequence-head: the state after the first part, written by the eight consumer warps of
-      // the CTA that scanned it (in this kernel's own element order).  Bounded wait on their count.
-      int* flag = p.ctrl + 1 + bh;
-      if (lane == 0) {
-        const unsigned long long t0 = globaltimer_ns();
-        int seen;
-        for (;;) {
-          asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
-          if (seen >= 8 || *abort_flag) break;
-          if (globaltimer_ns() - t0 > JB_WAIT_LIMIT_NS) {
-            *abort_flag = 1u;
-            atomicCAS(p.status, 0u, JB200_STATUS_ATTN_HANDOFF);
-            break;
-          }
-          __nanosleep(200);
-        }
-      }
-      __syncwarp();
-      __threadfence();
-      const float* hp = p.handoff + bh * D * D + s_row * D + 16 * s_cg;
-#pragma unroll
-      for (int e4 = 0; e4 < 4; ++e4) {
-        const float4 v4 = __ldcg(reinterpret_cast<const float4*>(hp) + e4);
-        S[4 * e4] = v4.x; S[4 * e4 + 1] = v4.y; S[4 * e4 + 2] = v4.z; S[4 * e4 + 3] = v4.w;
-      }
-    } else {
-      const float* sin_p = p.s_in ? p.s_in + bh * D * D + s_row * D : nullptr;
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        const int c = 16 * s_cg + e;
-        const int d = p.qk_prepared ? (c >> 1) + 32 * (c & 1) : c;   // prepared q/k: the dk axis is interleaved
-        S[e] = sin_p ? __ldg(sin_p + d) : 0.f;
-      }
-      if (seg > 0) {   // state entering this segment: fold the earlier segments' contributions, oldest first
-        const float gL = expf(log_g * float(p.seg_chunks * CH));
-        const float* dp = p.seg_state + bh * p.n_pieces * D * D + s_row * D + 16 * s_cg;
-        for (int s2 = 0; s2 < seg; ++s2, dp += D * D) {
-#pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {
-            const float4 v4 = __ldg(reinterpret_cast<const float4*>(dp) + e4);
-            S[4 * e4 + 0] = gL * S[4 * e4 + 0] + v4.x; S[4 * e4 + 1] = gL * S[4 * e4 + 1] + v4.y;
-            S[4 * e4 + 2] = gL * S[4 * e4 + 2] + v4.z; S[4 * e4 + 3] = gL * S[4 * e4 + 3] + v4.w;
-          }
-        }
-      }
-    }
-    auto publish_state = [&](int buf) {
-      uint32_t w[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) w[e] = pack_bf16x2(S[2 * e], S[2 * e + 1]);
-      *reinterpret_cast<uint4*>(sm->s[buf] + swz(s_row, 2 * s_cg)) = make_uint4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<uint4*>(sm->s[buf] + swz(s_row, 2 * s_cg + 1)) = make_uint4(w[4], w[5], w[6], w[7]);
-      fence_proxy_async_smem();
-      tc_fence_before_sync();
-      mbar_arrive(smem_u32(&sm->s_done));
-    };
-    publish_state(0);
+    const uint32_t tm_sc = tm + (uint32_t(32 * qd) << 16) + PT_SC + 128 * grp;
+    const uint32_t tm_o2 = tm + (uint32_t(32 * qd) << 16) + PT_O2 + 64 * grp;
+    uint32_t u = 0u;                                     // phase of the group's barriers
     bool ok = true;
+    int g = 0, s = 0, pending = -1;                      // stage of chunk g; the one whose v tile this warp's rows are leaving through
+    auto release = [&](int stage) {
+      if (lane == 0) {
+        bulk_wait_group_read<0>();
+        mbar_arrive(smem_u32(&sm->empty_v[stage]));
+      }
+      __syncwarp();
+    };
     JB_T_DECL
-    for (int lc = 0; lc < n_loc; ++lc) {
-      const int buf = lc & 1;
-      const uint32_t u = uint32_t(lc >> 1) & 1u;
-      const int ck = ck_begin + lc;
-      const int c_len = min(CH, T - ck * CH);
-      // ---- decay mask: scores -> P ----
-      JB_T_MARK(0)
-      if (!mbar_wait(smem_u32(&sm->bar_sc[buf]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
-      JB_T_MARK(1)
-      tc_fence_after_sync();
-      __syncwarp();               // tcgen05.ld / st are warp-collective: rejoin after the per-thread wait
+    if (share.chunks() == 1) {
+      // A lone chunk: both groups work on it, the upper and the lower key blocks of a row (P goes to the other accumulator, since
+      // what one group writes the other may not have read), then half of the output columns each, stored directly (one
+      // sequence of 37 and 128 tokens 6.9 -> 6.2 and 7.2 -> 6.8 us).
+      const Item it = share.at(0);
+      const int b = it.unit / p.H, col = (it.unit - b * p.H) * D + 32 * grp;
+      const DecayTab& tab = sm->tab[0];
+      const uint32_t tm_lane = tm + (uint32_t(32 * qd) << 16);
+      if (mbar_wait(smem_u32(&sm->bar_sc[0]), 0u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) {
+        tc_fence_after_sync();
+        __syncwarp();
+        uint32_t r[16], w[8];
+#pragma unroll 1
+        for (int n = 0; n <= qd; ++n) {
+          const int jb = n + (grp ? qd + 1 : 0);             // 16-key block
+          tmem_ld_32x16(tm_lane + PT_SC + 16 * jb, r);
+          tmem_ld_wait();
+          const float* f = tab.pwm + (i - 16 * jb + CH);
 #pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const int jb = 2 * hf + jj;                      // 32-key block
-        if (jb > qd) continue;                           // above the diagonal for all rows of this warp: stays zero
-        uint32_t r[32];
-        tmem_ld_32x32(tm_lane + PT_SC + 128 * buf + 32 * jb, r);
-        tmem_ld_wait();
-        const float* f = sm->pwm + (i - 32 * jb + CH);   // f[-c]: factor of key 32*jb + c
-        uint32_t w[16];
+          for (int c2 = 0; c2 < 8; ++c2) w[c2] = pack_bf16x2(__uint_as_float(r[2 * c2]) * f[-2 * c2], __uint_as_float(r[2 * c2 + 1]) * f[-2 * c2 - 1]);
+          tmem_st_32x8(tm_lane + PT_SC + 128 + PT_P + 8 * jb, w);
+        }
 #pragma unroll
-        for (int c2 = 0; c2 < 16; ++c2)
-          w[c2] = pack_bf16x2(__uint_as_float(r[2 * c2]) * f[-2 * c2], __uint_as_float(r[2 * c2 + 1]) * f[-2 * c2 - 1]);
-        tmem_st_32x16(tm_lane + PT_P + 16 * jb, w);
-      }
-      tmem_st_wait();
-      JB_T_MARK(2)
-      tc_fence_before_sync();
-      mbar_arrive(smem_u32(&sm->p_done));
-      JB_T_MARK(3)
-      // ---- state update: S = gamma^c S + dS ----
-      if (!mbar_wait(smem_u32(&sm->bar_s), uint32_t(lc) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
-      JB_T_MARK(4)
-      tc_fence_after_sync();
-      __syncwarp();
-      {
-        uint32_t r[16];
-        tmem_ld_32x16(tm_lane + PT_DS + 16 * s_cg, r);
-        tmem_ld_wait();
-        const float gc = sm->pw[c_len];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) S[e] = gc * S[e] + __uint_as_float(r[e]);
-      }
-      publish_state((lc + 1) & 1);
-      JB_T_MARK(5)
-      // ---- output rows: o[i] = O1 + gamma^(i+1)/8 * O2 ----
-      if (!mbar_wait(smem_u32(&sm->bar_b[buf]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
-      JB_T_MARK(6)
-      tc_fence_after_sync();
-      __syncwarp();
-      {
-        uint32_t a[32], c2[32];
-        tmem_ld_32x32(tm_lane + PT_SC + 128 * buf + 32 * hf, a);
-        tmem_ld_32x32(tm_lane + PT_O2 + 64 * buf + 32 * hf, c2);
-        tmem_ld_wait();
+        for (int e = 0; e < 8; ++e) w[e] = 0u;
+        for (int jb = 2 * qd + 2 + grp; jb < 8; jb += 2) tmem_st_32x8(tm_lane + PT_SC + 128 + PT_P + 8 * jb, w);   // above the diagonal
+        tmem_st_wait();
         tc_fence_before_sync();
-        mbar_arrive(smem_u32(&sm->o_done[buf]));         // both accumulators are in registers now
-        const float g = 0.125f * sm->pw[i + 1];
-        uint32_t w[16];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm->p_done[grp]));
+      }
+      const float gi = 0.125f * tab.pw[i + 1];
+      const int t = it.begin * CH + i;
+      __nv_bfloat16* op = p.o + size_t(b * T + t) * p.ld_o + col;
+      if (mbar_wait(smem_u32(&sm->bar_o2[0]), 0u, abort_flag, p.status, JB200_STATUS_ATTN_MMA) &&
+          mbar_wait(smem_u32(&sm->bar_b[0]), 0u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) {
+        tc_fence_after_sync();
+        __syncwarp();
+        uint32_t a[32], c2[32];
+        tmem_ld_32x32(tm_lane + PT_SC + 32 * grp, a);
+        tmem_ld_32x32(tm_lane + PT_O2 + 32 * grp, c2);
+        tmem_ld_wait();
+        if (t < T) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e)
-          w[e] = pack_bf16x2(fmaf(g, __uint_as_float(c2[2 * e]), __uint_as_float(a[2 * e])),
-                             fmaf(g, __uint_as_float(c2[2 * e + 1]), __uint_as_float(a[2 * e + 1])));
-        if (i < c_len) {
-          __nv_bfloat16* op = p.o + size_t(row0 + ck * CH + i) * p.ld_o + h * D + 32 * hf;
-          if (p.wide_store) {
-            st_global_256(op, w);
-            st_global_256(op + 16, w + 8);
-          } else {
+          for (int c = 0; c < 4; ++c) {
+            uint32_t w[4];
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4)
-              *reinterpret_cast<uint4*>(op + 8 * q4) = make_uint4(w[4 * q4], w[4 * q4 + 1], w[4 * q4 + 2], w[4 * q4 + 3]);
+            for (int e = 0; e < 4; ++e)
+              w[e] = pack_bf16x2(fmaf(gi, __uint_as_float(c2[8 * c + 2 * e]), __uint_as_float(a[8 * c + 2 * e])),
+                                 fmaf(gi, __uint_as_float(c2[8 * c + 2 * e + 1]), __uint_as_float(a[8 * c + 2 * e + 1])));
+            *reinterpret_cast<uint4*>(op + 8 * c) = make_uint4(w[0], w[1], w[2], w[3]);
           }
         }
-      }
-      JB_T_MARK(7)
-    }
-    JB_T_FLUSH(warp)
-    if (piece == 1) {
-      // first part of a cut sequence-head: its end state for the CTA that takes the second part
-      if (ok) {
-        float* hp = p.handoff + bh * D * D + s_row * D + 16 * s_cg;
-#pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4)
-          __stcg(reinterpret_cast<float4*>(hp) + e4, make_float4(S[4 * e4], S[4 * e4 + 1], S[4 * e4 + 2], S[4 * e4 + 3]));
-        __threadfence();
         __syncwarp();
-        if (lane == 0) atomicAdd(p.ctrl + 1 + bh, 1);
       }
-    } else if (ok && p.s_out && seg == p.nseg - 1) {
-      float* sp = p.s_out + bh * D * D + s_row * D;
-      if (p.qk_prepared) {
+      ok = false;                                          // nothing left for the loop
+    }
+    for (int k = 0; ok && k < share.n_items; ++k) {
+      const Item it = share.at(k);
+      const int b = it.unit / p.H, col = (it.unit - b * p.H) * D;
+      const DecayTab& tab = sm->tab[k % NTAB];
+      for (int ck = it.begin; ck < it.end; ++ck, ++g, s = s + 1 == NST ? 0 : s + 1) {
+        if ((g & 1) != grp) continue;
+        if (pending >= 0) release(pending);
+        // ---- decay mask: scores -> P (lane = query row, column c = keys 2c, 2c+1) ----
+        JB_T_MARK(0)
+        if (k > 0 && !mbar_wait(smem_u32(&sm->tab_full[k % NTAB]), uint32_t(k / NTAB) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
+        if (!mbar_wait(smem_u32(&sm->bar_sc[grp]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
+        JB_T_MARK(1)
+        tc_fence_after_sync();
+        __syncwarp();
+        {
+          uint32_t r[2][16];
+          tmem_ld_32x16(tm_sc + 32 * qd + 16, r[0]);
+          {
+            uint32_t z[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int c = 16 * s_cg + e;
-          sp[(c >> 1) + 32 * (c & 1)] = S[e];
+            for (int e = 0; e < 16; ++e) z[e] = 0u;
+#pragma unroll
+            for (int jb = 1; jb < 4; ++jb)
+              if (jb > qd) tmem_st_32x16(tm_sc + PT_P + 16 * jb, z);     // above the diagonal for all rows of this warp
+          }
+          const float* f = tab.pwm + (i - 32 * qd - 16 + CH);   // f[-c]: factor of key 16*jb + c
+#pragma unroll 1
+          for (int jb = 2 * qd + 1; jb > 0; jb -= 2) {         // 16-key blocks jb and jb - 1
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+              tmem_ld_wait();
+              if (n == 0) tmem_ld_32x16(tm_sc + 16 * (jb - 1), r[1]);
+              else if (jb > 1) tmem_ld_32x16(tm_sc + 16 * (jb - 2), r[0]);
+              uint32_t w[8];
+#pragma unroll
+              for (int c2 = 0; c2 < 8; ++c2)
+                w[c2] = pack_bf16x2(__uint_as_float(r[n][2 * c2]) * f[16 * n - 2 * c2], __uint_as_float(r[n][2 * c2 + 1]) * f[16 * n - 2 * c2 - 1]);
+              tmem_st_32x8(tm_sc + PT_P + 8 * (jb - n), w);
+            }
+            f += 32;
+          }
+          tmem_st_wait();
         }
-      } else {
+        JB_T_MARK(2)
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm->p_done[grp]));
+        JB_T_MARK(3)
+        // ---- output rows: o[i] = O1 + gamma^(i+1)/8 * O2 ----
+        const float gi = 0.125f * tab.pw[i + 1];
+        if (!mbar_wait(smem_u32(&sm->bar_o2[grp]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
+        JB_T_MARK(4)
+        if (!mbar_wait(smem_u32(&sm->bar_b[grp]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
+        JB_T_MARK(5)
+        u ^= 1u;
+        tc_fence_after_sync();
+        __syncwarp();
+        uint8_t* o_p = sm->v[s];                           // P V has read the chunk's v tile: the rows leave through it
+#pragma unroll 1
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t a[32], c2[32];
+          tmem_ld_32x32(tm_sc + 32 * hf, a);
+          tmem_ld_32x32(tm_o2 + 32 * hf, c2);
+          tmem_ld_wait();
+          if (hf == 1) {                                   // both accumulators are in registers now
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sm->o_done[grp]));
+          }
 #pragma unroll
-        for (int e4 = 0; e4 < 4; ++e4)
-          *reinterpret_cast<float4*>(sp + 16 * s_cg + 4 * e4) = make_float4(S[4 * e4], S[4 * e4 + 1], S[4 * e4 + 2], S[4 * e4 + 3]);
+          for (int c = 0; c < 4; ++c) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              w[e] = pack_bf16x2(fmaf(gi, __uint_as_float(c2[8 * c + 2 * e]), __uint_as_float(a[8 * c + 2 * e])),
+                                 fmaf(gi, __uint_as_float(c2[8 * c + 2 * e + 1]), __uint_as_float(a[8 * c + 2 * e + 1])));
+            *reinterpret_cast<uint4*>(o_p + swz(i, 4 * hf + c)) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (32 * qd < T - ck * CH) tma_store_3d(&tm_o, col, ck * CH + 32 * qd, b, smem_u32(o_p) + 32 * 128 * qd);
+          bulk_commit_group();
+        }
+        pending = s;
+        JB_T_MARK(6)
       }
     }
+    if (lane == 0) bulk_wait_group<0>();
+    __syncwarp();
+    JB_T_FLUSH(warp)
   }
 
   tc_fence_before_sync();
@@ -1077,6 +1274,10 @@ int make_map(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld) {
 
 }  // namespace
 
+// From so many chunks on a cut is worth the ticket, the hand-off and the clearing of their words (16 x 512, four chunks: 26.4 us
+// before and now; eight: 32 x 1024 in equal shares 3.5 sequence-heads per SM instead of four).
+static constexpr int SPLIT_CHUNKS = 4;
+
 // Segments: the pipeline kernel runs one CTA per SM, so sequences are cut only when B*H leaves SMs idle;
 // each segment is at least two chunks long.
 static void pick_segments(int B, int T, int H, int sms, int* seg_chunks, int* nseg) {
@@ -1089,16 +1290,12 @@ static void pick_segments(int B, int T, int H, int sms, int* seg_chunks, int* ns
   *nseg = (n_chunks + sc - 1) / sc;
 }
 
-// Balanced launch: with more sequence-heads than SMs and a last wave that is at most half full, that many
-// sequence-heads are cut in two; the first parts run first, the second parts last, and the makespan drops by half
-// a sequence (B=32 x 16 heads on 148 SMs: 64 -> 56 chunk times).  A sequence's chunks are serial, so nothing is to be
-// gained when every SM holds at most one sequence-head.
-static int pick_split(int B, int T, int H, int sms) {
+// More sequence-heads than SMs: as many CTAs as SMs walk them, and where they do not come out even, shares are cut inside a
+// sequence-head.
+static bool pick_split(int B, int T, int H, int sms) {
   const long U = long(B) * H;
-  const int n_chunks = (T + CH - 1) / CH;
-  if (U <= sms || n_chunks < 8) return 0;      // short sequences: the ticket and the hand-off cost more than they save
-  const int R = int(U % sms);
-  return (R > 0 && 2 * R <= sms) ? R : 0;
+  const long n_chunks = (T + CH - 1) / CH;
+  return U > sms && U % sms != 0 && n_chunks >= SPLIT_CHUNKS && U * n_chunks < (1l << 31);
 }
 
 size_t attn_scan_scratch_bytes(int B, int T, int H) {
@@ -1108,8 +1305,7 @@ size_t attn_scan_scratch_bytes(int B, int T, int H) {
   int sc, ns;
   pick_segments(B, T, H, sms, &sc, &ns);
   const size_t seg_bytes = size_t(B) * H * size_t(ns) * D * D * sizeof(float);   // ns - 1 pieces for a full call, ns for a state-only one
-  const int n_split = pick_split(B, T, H, sms);
-  const size_t split_bytes = n_split ? size_t(n_split) * D * D * sizeof(float) + (size_t(n_split) + 1) * sizeof(int) : 0;
+  const size_t split_bytes = pick_split(B, T, H, sms) ? size_t(sms) * D * D * sizeof(float) + (size_t(sms) + 1) * sizeof(int) : 0;
   return seg_bytes > split_bytes ? seg_bytes : split_bytes;
 }
 
@@ -1141,7 +1337,7 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
     dp.gamma = gamma; dp.cos_tab = cos_tab; dp.sin_tab = sin_tab; dp.pos0 = pos0; dp.pos0_scalar = pos0_scalar;
     dp.n_pos = n_pos; dp.s_in = s_in; dp.s_out = s_out; dp.o = reinterpret_cast<__nv_bfloat16*>(o); dp.ld_o = ld_o;
     dp.B = B; dp.T = 1; dp.H = H; dp.seg_chunks = 1; dp.nseg = 1; dp.seg_state = nullptr; dp.n_pieces = 0; dp.qk_prepared = 0;
-    dp.wide_store = 0; dp.settled = settled ? 1 : 0; dp.status = device_status_ptr();
+    dp.wide_tab = 0; dp.settled = settled ? 1 : 0; dp.status = device_status_ptr();
     if (!dp.status) return JB200_ERR_CUDA;
     if (s_in && s_out && B * H >= 64) {
       // the state streams through shared memory as bulk copies: two CTAs per SM walk the (sequence, head) pairs
@@ -1170,7 +1366,7 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   p.n_pos = n_pos; p.s_in = s_in; p.s_out = s_out; p.o = reinterpret_cast<__nv_bfloat16*>(o); p.ld_o = ld_o;
   p.B = B; p.T = T; p.H = H;
   p.qk_prepared = (flags & JB200_ATTN_QK_PREPARED) ? 1 : 0;
-  p.wide_store = (o && (reinterpret_cast<uintptr_t>(o) & 31u) == 0 && ld_o % 16 == 0) ? 1 : 0;
+  p.wide_tab = ((reinterpret_cast<uintptr_t>(cos_tab) | reinterpret_cast<uintptr_t>(sin_tab)) & 31u) == 0 ? 1 : 0;
   p.n_pieces = 0;
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
@@ -1184,7 +1380,7 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   p.settled = settled || p.nseg > 1;      // the pass over the segments waited for whatever made gamma
   JB_REQUIRE(!scratch || aligned16(scratch), "attn_scan: scratch pointer must be 16-byte aligned");
   p.n_pieces = o ? p.nseg - 1 : p.nseg;
-  p.n_split = 0; p.split_chunk = 0; p.handoff = nullptr; p.ctrl = nullptr;
+  p.split = 0; p.handoff = nullptr; p.ctrl = nullptr;
   if (!o) {
     // state only: the k/v pass over every piece, then the fold
     JB_MAX_SMEM(attn_state_pass_kernel, STATE_SMEM_BYTES);
@@ -1194,23 +1390,34 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
     JB_LAUNCH_CHECK("attn_fold_states_kernel");
     return JB200_OK;
   }
-  JB_MAX_SMEM(attn_scan_pipe_kernel, PIPE_SMEM_BYTES);
+  if (p.qk_prepared) JB_MAX_SMEM(attn_scan_pipe_kernel<true>, PIPE_SMEM_BYTES);
+  else JB_MAX_SMEM(attn_scan_pipe_kernel<false>, PIPE_SMEM_BYTES);
   if (p.nseg > 1) {
     JB_MAX_SMEM(attn_state_pass_kernel, STATE_SMEM_BYTES);
     launch_dep(attn_state_pass_kernel, dim3(H, B, p.nseg - 1), STATE_THREADS, STATE_SMEM_BYTES, stream, tk, tv, p);
     JB_LAUNCH_CHECK("attn_state_pass_kernel");
   }
-  if (scratch && p.nseg == 1 && (p.n_split = pick_split(B, T, H, sms)) > 0) {
-    p.split_chunk = ((T + CH - 1) / CH) / 2;
+  // output rows leave 32 at a time, clipped at the end of their sequence
+  CUtensorMap to;
+  const cuuint64_t odim[3] = {cuuint64_t(H) * D, cuuint64_t(T), cuuint64_t(B)};
+  const cuuint64_t ostride[2] = {cuuint64_t(ld_o) * 2, cuuint64_t(T) * ld_o * 2};
+  const cuuint32_t obox[3] = {cuuint32_t(D), 32, 1};
+  if ((rc = encode_tiled(&to, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, o, odim, ostride, obox, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "attn_scan")) != JB200_OK)
+    return rc;
+  const long units = long(B) * H * p.nseg;
+  const unsigned grid = unsigned(p.nseg > 1 || units < sms ? units : sms);
+  if (scratch && p.nseg == 1 && pick_split(B, T, H, sms)) {
+    p.split = 1;
     p.handoff = reinterpret_cast<float*>(scratch);
-    p.ctrl = reinterpret_cast<int*>(p.handoff + size_t(p.n_split) * D * D);
-    JB_CUDA(cudaMemsetAsync(p.ctrl, 0, (size_t(p.n_split) + 1) * sizeof(int), stream));
-    launch_dep(attn_scan_pipe_kernel, dim3(unsigned(long(B) * H + p.n_split)), PIPE_THREADS, PIPE_SMEM_BYTES, stream, tq, tk,
-               tv, p);
-    JB_LAUNCH_CHECK("attn_scan_pipe_kernel");
-    return JB200_OK;
+    p.ctrl = reinterpret_cast<int*>(p.handoff + size_t(grid) * D * D);
+    JB_CUDA(cudaMemsetAsync(p.ctrl, 0, (size_t(grid) + 1) * sizeof(int), stream));
   }
-  launch_dep(attn_scan_pipe_kernel, dim3(H, B, p.nseg), PIPE_THREADS, PIPE_SMEM_BYTES, stream, tq, tk, tv, p);
+  const long total = p.split ? long(B) * H * p.seg_chunks : long(B) * H;
+  p.per_cta = int(total / grid);
+  p.spare = int(total % grid);
+  launch_dep(p.qk_prepared ? attn_scan_pipe_kernel<true> : attn_scan_pipe_kernel<false>, dim3(grid), PIPE_THREADS, PIPE_SMEM_BYTES, stream, tq,
+             tk, tv, to, p);
   JB_LAUNCH_CHECK("attn_scan_pipe_kernel");
   return JB200_OK;
 }
@@ -1218,7 +1425,7 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
 #ifdef JB_ATTN_TIMING
 // Timing builds only: copies the per-role cycle counters of the last pipeline launch to the host.
 extern "C" int jb200_debug_attn_timing(long long* out) {
-  return cudaMemcpyFromSymbol(out, g_attn_timing, sizeof(long long) * 18 * 8) == cudaSuccess ? 0 : 1;
+  return cudaMemcpyFromSymbol(out, g_attn_timing, sizeof(long long) * 24 * 8) == cudaSuccess ? 0 : 1;
 }
 #endif
 

@@ -112,6 +112,30 @@ def test_attn_scan_balanced_launch_cuts_sequences_in_two(B, H, T):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("B,H,T", [(10, 16, 100), (10, 16, 128), (150, 1, 130), (19, 8, 257), (37, 4, 384), (300, 1, 300), (33, 16, 512),
+                                   (12, 16, 700), (149, 1, 513)])
+def test_attn_scan_walks_several_sequence_heads(B, H, T):
+    """As many sequence-heads as SMs, a few more or several times as many, of one to six chunks: shares cut inside a sequence-head (four
+    chunks on), whole ones, last chunks of every kind.  Every sequence has the bits that it has alone, one CTA per head."""
+    g = torch.Generator(device="cuda").manual_seed(B + T)
+    C = H * 64
+    qkv = torch.randn(B * T, 3 * C, generator=g, device="cuda").bfloat16()
+    gamma = torch.rand(H, generator=g, device="cuda") * 0.2 + 0.799
+    S0 = torch.randn(B, H, 64, 64, generator=g, device="cuda")
+    pos = torch.randint(0, 200, (B,), generator=g, device="cuda", dtype=torch.int32)
+    cos, sin = rope_tabs(T + 200)
+    big = torch.full((B * T + 1, C), 7.0, dtype=torch.bfloat16, device="cuda")
+    _, S = ops.attn_scan(qkv[:, :C], qkv[:, C:2 * C], qkv[:, 2 * C:], gamma, cos, sin, B, T, H, start_pos=pos, state_in=S0, want_state=True,
+                         out=big[:B * T])
+    assert bool((big[B * T] == 7.0).all())                  # nothing is stored past the last sequence's rows
+    for b in sorted({0, 1, B // 2, B - 2, B - 1}):
+        r = qkv[b * T:(b + 1) * T]
+        o1, S1 = ops.attn_scan(r[:, :C], r[:, C:2 * C], r[:, 2 * C:], gamma, cos, sin, 1, T, H, start_pos=pos[b:b + 1].contiguous(),
+                               state_in=S0[b:b + 1].contiguous(), want_state=True, segmented=False)
+        assert torch.equal(big[b * T:(b + 1) * T], o1) and torch.equal(S[b:b + 1], S1), b
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("B,H", [(3, 2), (40, 4), (301, 16)])
 def test_attn_single_token_steps_with_carried_state(B, H):
     """T = 1 with a carried state and ragged positions: a handful of (sequence, head) pairs take the per-pair
