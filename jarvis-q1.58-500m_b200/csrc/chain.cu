@@ -52,27 +52,36 @@ struct Workspace {
 
 // Which form of the ternary product a call of so many tokens runs (their results are the same bits): up to 16 tokens
 // mma.sync straight from the codes (24 layers of single-token steps 0.62 against 0.86 ms at 1 sequence, equal at 16), up to
-// MID_TOKENS the tcgen05 form that is built for latency (640 tokens 1.96 against 2.08 ms, 900 2.20 against 2.29, 1000 equal,
-// 1152 2.81 against 2.74), beyond that the persistent pipeline.
+// MID_TOKENS the tcgen05 form that is built for latency (37 tokens 916 -> 880 us against mma.sync with its token tiles side by side
+// for the attention's products, 64 sequences 1004 -> 957; 640 tokens 1.96 against 2.08 ms with the persistent pipeline, 900 2.20
+// against 2.29, 1000 equal, 1152 2.81 against 2.74), beyond that the persistent pipeline.
 constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
-// The products of the attention have few out-features: the tcgen05 form runs them on 8 to 24 SMs.  mma.sync with the token tiles
-// side by side (8 rows each for prompts, 16 for steps) fills the chip, and its chain over K is shorter.  24 layers and head as a
-// graph: prompts of 37, 64, 100 tokens with the out-projection so 1052 -> 1035, 1110 -> 1096, 1322 -> 1287 us, 180 equal, 256
-// 1402 -> 1447; on top of that with q|k|v so 17 tokens 995 -> 966, 24 1008 -> 977, 32 1024 -> 1010, 40 1038 -> 1020; 41 to
-// 64 between 1 % faster and 1.6 % slower, by the GPU (48: 1053 -> 1048 on one, 1046 -> 1054 on another); 80 1256 -> 1282, 128
-// 1375 -> 1430.  Steps of 64, 100, 128 sequences with q|k|v so 1094 -> 1070, 1361 -> 1351, equal; their out-projection, behind the
-// attention's stores, gets slower (64: 1094 -> 1114).
-constexpr int OUT_TILED_TOKENS = 128, QKV_TILED_PROMPT = 40, QKV_TILED_STEP = 100;
 // Up to here the first expert GEMM takes all rows for every expert and stores the routed ones: more MMAs, no dispatch.  A token without
 // finite router logits is stored once, for expert 0, and its second hidden row holds whatever was there: combine and tail
-// take the first one's output for both assignments (stored twice by the GEMM, 64 sequences were 1.5 % slower).
-constexpr int ALL_ROWS_TOKENS = 64;
-// Token tile of the latency form: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
-// tokens) that leaves a launch of so many rows in each group one wave.
-inline int mid_tile(int rows, int groups, int n_ft, int sms) {
+// take the first one's output for both assignments (stored twice by the GEMM, 64 sequences were 1.5 % slower).  24 layers and head as a graph
+// with the dispatch -> without: 80 tokens 1141 -> 1060 us, 128 1188 -> 1133, 5 x 30 1227 -> 1200, 180 1310 -> 1298, steps of 128 sequences
+// 1360 -> 1326, 192 equal, 256 tokens 1375 -> 1423.
+constexpr int ALL_ROWS_TOKENS = 160;
+// Tiles of the latency form.  Tokens: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
+// tokens) that leaves a launch of so many rows in each group on `room` SMs.
+inline int mid_tile(int rows, int groups, int n_ft, int room) {
   int bn = rows <= 64 ? (rows + 15) / 16 * 16 : 64;
-  while (bn < 256 && long(n_ft) * groups * ((rows + bn - 1) / bn) > sms) bn += 16;
+  while (bn < 256 && long(n_ft) * groups * ((rows + bn - 1) / bn) > room) bn += 16;
   return bn;
+}
+// Out-features: 64 or 128 a tile.  The time of a tile goes with both its sides, but SMs that a launch takes are not there for the
+// next one to begin on (barriers, codes fetched and decoded): 64 where they are at most `most`.  24 layers and head as a graph with 64
+// for one product alone: q|k|v of 64 tokens (48 SMs) 1000 -> 979 us, of 128 sequences (96) 1441 -> 1400, of 256 (144) 1745 -> 1776;
+// out-projection of 64 sequences 1083 -> 1052, of 400 tokens (112 SMs; the router behind it needs little of an SM) 1661 -> 1633, of 700
+// (144) 1885 -> 1919; second expert matrix of 37 tokens (64 SMs) 949 -> 916, of 128 sequences (128) 1441 -> 1451; first
+// expert matrix of 37 tokens (128 SMs) 949 -> 1013.
+constexpr int QKV_MOST = 100, OUT_MOST = 120, EXPERT_MOST = 74;
+struct MidTile {
+  int bm, bn;
+};
+inline MidTile mid_tiles(int rows, int groups, int n_out, int room, int most) {
+  const int b64 = mid_tile(rows, groups, n_out / 64, room), b128 = mid_tile(rows, groups, n_out / 128, room);
+  return long(n_out / 64) * groups * ((rows + b64 - 1) / b64) <= most && 64 + b64 < 128 + b128 ? MidTile{64, b64} : MidTile{128, b128};
 }
 
 #define JB_TRY(call)                    \
@@ -143,24 +152,22 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   float* x = f->x;
   const int small_tile = N <= 8 ? 8 : 16;
   const bool small = N <= SMALL_TOKENS && small_gemm_fits(small_tile, std::max(C, hidden));   // beyond, the tcgen05 form streams K
-  const int out_tile = T > 1 && N <= OUT_TILED_TOKENS ? 8 : 0;
-  const int qkv_tile = T > 1 ? (N <= QKV_TILED_PROMPT ? 8 : 0) : (N <= QKV_TILED_STEP ? 16 : 0);
   const bool mid = !small && N <= MID_TOKENS;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
   auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
-                      const int32_t* seg, const int64_t* ids, const int32_t* sc, int epi, void* dst) {
-    const int n_ft = n_out / 128;
+                      const int32_t* seg, const int64_t* ids, const int32_t* sc, int epi, void* dst, int most) {
     if (!seg) {                                // every group over all rows
-      const int bn = mid_tile(M, G, n_ft, sms);
-      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn, st);
+      const MidTile t = mid_tiles(M, G, n_out, G > 1 ? most : sms, most);
+      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, t.bm, t.bn, t.bn, st);
     }
     // Segments are known on the device alone: a tile for rows that are spread evenly, with an eighth to spare, and one for
     // whatever they are (M / bn_max tiles and one cut short in every other group).
-    const int even = (M + G - 1) / G, bn = mid_tile(even + (even + 7) / 8, G, n_ft, sms);
-    int bn_max = bn;
-    while (bn_max < 256 && long(n_ft) * ((M + bn_max - 1) / bn_max + G - 1) > sms) bn_max += 16;
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, bn, bn_max, st);
+    const int even = (M + G - 1) / G;
+    const MidTile t = mid_tiles(even + (even + 7) / 8, G, n_out, sms, most);
+    int bn_max = t.bn;
+    while (bn_max < 256 && long(n_out / t.bm) * ((M + bn_max - 1) / bn_max + G - 1) > sms) bn_max += 16;
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, t.bm, t.bn, bn_max, st);
   };
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
@@ -194,12 +201,9 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
 
     // x += attn(norm1(x))
     if (small)
-      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, 1, st));
-    else if (qkv_tile)
-      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile,
-                              (N + qkv_tile - 1) / qkv_tile, st));
+      JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv));
+      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, QKV_MOST));
     else
       JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st, nullptr, true));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
@@ -208,12 +212,9 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     JB_TRY(launch_attn_scan(qkv, qkv + C, qkv + 2 * C, 3 * C, p.gamma, f->cos_tab, f->sin_tab, f->n_pos, f->pos0, f->pos0_scalar,
                             s_in, o, C, s_out, attn_scratch, B, T, H, 64, 0, st, true));
     if (small)
-      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, 1, st));
-    else if (out_tile)
-      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile,
-                              (N + out_tile - 1) / out_tile, st));
+      JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x));
+      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, OUT_MOST));
     else
       JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st, nullptr, true));
 
@@ -228,20 +229,20 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (N <= ALL_ROWS_TOKENS) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
       if (small)
-        JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, small_tile, 1, st));
+        JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, small_tile, st));
       else
-        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid));
+        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
     } else {
       JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
-        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid));
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
       else
         JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true));
     }
     if (small)
-      JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, 1, st));
+      JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y));
+      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, EXPERT_MOST));
     else
       JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st, nullptr, true));
 

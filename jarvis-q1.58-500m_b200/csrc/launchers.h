@@ -27,19 +27,19 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
                         int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope = nullptr, bool settled = false);
 // The same product for a few tokens (small_gemm.cu), bit for bit; bf16, GELU and residual epilogues.  idx / scatter ([M][2]):
 // all M rows go through every group's matrix and row n is stored at scatter[2n + k] where idx[2n + k] is the group; else seg
-// as above.  tile: rows a CTA takes at a time, 8 or 16; tiles: CTAs that share a segment's tiles.  Within a chain only: weights
+// as above.  tile: rows a CTA takes at a time, 8 or 16.  Within a chain only: weights
 // and seg were complete before the kernel ahead of this one on the stream began, and are read while it runs.
 int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
                       int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
-                      int tile, int tiles, cudaStream_t stream);
+                      int tile, cudaStream_t stream);
 // It keeps whole rows of codes and activations in shared memory: in-features it can take with such tiles (about 7200 with 8
 // rows, 4800 with 16).
 bool small_gemm_fits(int tile, int K);
-// The same product again, latency form on tcgen05 (mid_gemm.cu) with token tiles of bn rows, or of bn_max rows
+// The same product again, latency form on tcgen05 (mid_gemm.cu) with tiles of bm (64 or 128) out-features and bn rows, or of bn_max rows
 // where the segments need more tiles of bn than there are SMs.  Arguments as launch_small_gemm.
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int bn_max,
-                    cudaStream_t stream);
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bm, int bn,
+                    int bn_max, cudaStream_t stream);
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);
 void decode16_prepared_host(uint32_t w_canonical, uint32_t* out8);

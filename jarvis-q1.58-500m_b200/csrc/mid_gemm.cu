@@ -24,9 +24,9 @@ namespace jb {
 
 namespace {
 
-constexpr int BM = 128, BK = 64, A_BYTES = BM * BK * 2;
+constexpr int BK = 64;
 constexpr int CK = 2;                          // K-blocks per chunk (four: 1-3 % slower, the ring gets too coarse)
-constexpr int MAX_CHUNKS = 6, DEC_WARP0 = 2, THREADS = 320;
+constexpr int MAX_CHUNKS = 8, DEC_WARP0 = 2, THREADS = 320;
 constexpr int SLOTS = 4;                       // chunks whose codes are in registers
 
 struct MidParams {
@@ -78,8 +78,25 @@ struct Items {
   }
 };
 
+// Accumulator of a tile of 64 out-features: 16 in each quarter of the lanes.  32 columns of the lower 16 lanes; thread (g, c) of
+// 8 x 4 receives of rows g (v[4j], v[4j + 1]) and g + 8 (v[4j + 2], v[4j + 3]) the columns 8j + 2c and 8j + 2c + 1.
+__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+// BM: out-features of a tile.  128 is the MMA's full rate; but up to ~100 tokens a step is bound by the shared memory that its
+// operands are read from (BM + bn rows of 32 bytes, 128 bytes a cycle, and the same again for the decoded weights and
+// the copied rows), so tiles of 64, on twice as many SMs, take less time each: half the codes to fetch and decode, half the epilogue.
+template <int BM>
 __global__ void __launch_bounds__(THREADS, 1)
 mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
+  constexpr int A_BYTES = BM * BK * 2;
   extern __shared__ uint8_t smem_raw[];
   __shared__ Ctl ctl;
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -208,27 +225,39 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     }
   } else {
     // ---------------- decoders, then epilogue ----------------
-    const int par = (warp - DEC_WARP0) >> 2;                       // this thread decodes K-block par of every chunk,
-    const int r = ((warp - DEC_WARP0) & 3) * 32 + lane;             // weight row r of the tile
+    // This thread decodes, of K-block `par` of every chunk, row r of the tile: all 64 codes with 128 rows, half `hh` of them with 64.
+    // Rows g and g + 8 of 16 are out-features 2g and 2g + 1 there, so that the epilogue's threads end up with neighbours.
+    constexpr int WORDS = BM / 32;                                 // words of 16 codes
+    const int par = (warp - DEC_WARP0) >> 2, idx = ((warp - DEC_WARP0) & 3) * 32 + lane;
+    const int r = idx % BM, hh = idx / BM;
+    const int feat = BM == 128 ? r : (r & ~15) + 2 * (r & 7) + ((r >> 3) & 1);
     const uint8_t* wrow = nullptr;
     float alpha = 0.f;
     auto weights_of = [&](const Items& it) {
-      wrow = p.w + (size_t(it.grp) * p.N + size_t(it.ft) * BM + r) * (size_t(p.K) / 4) + par * 16;
+      wrow = p.w + (size_t(it.grp) * p.N + size_t(it.ft) * BM + feat) * (size_t(p.K) / 4) + par * 16 + hh * 8;
       alpha = 0.5f * __ldg(p.alpha + size_t(it.grp) * (p.N / p.alpha_rows) + (it.ft * BM) / p.alpha_rows);   // codes decode to +-2
     };
     const uint32_t swz = uint32_t(r & 7);
-    uint4 code[SLOTS];
+    struct Codes { uint32_t w[WORDS]; };
+    Codes code[SLOTS];
     auto load_codes = [&](int u, int c) {
-      code[u] = c < n_ch ? __ldg(reinterpret_cast<const uint4*>(wrow + size_t(c * CK) * 16)) : make_uint4(0u, 0u, 0u, 0u);
+      const uint8_t* src = wrow + size_t(c * CK) * 16;
+      if constexpr (WORDS == 4) {
+        const uint4 v = c < n_ch ? __ldg(reinterpret_cast<const uint4*>(src)) : make_uint4(0u, 0u, 0u, 0u);
+        code[u].w[0] = v.x; code[u].w[1] = v.y; code[u].w[2] = v.z; code[u].w[3] = v.w;
+      } else {
+        const uint2 v = c < n_ch ? __ldg(reinterpret_cast<const uint2*>(src)) : make_uint2(0u, 0u);
+        code[u].w[0] = v.x; code[u].w[1] = v.y;
+      }
     };
-    auto put = [&](const uint4& cw, uint8_t* arow) {       // 64 codes -> one swizzled 128-byte row
-      const uint32_t words[4] = {cw.x, cw.y, cw.z, cw.w};
+    auto put = [&](const Codes& cw, uint8_t* arow) {       // codes -> (its half of) a swizzled 128-byte row
 #pragma unroll
-      for (int wi = 0; wi < 4; ++wi) {
+      for (int wi = 0; wi < WORDS; ++wi) {
         uint32_t v[8];
-        decode16_prepared(words[wi], v);
-        *reinterpret_cast<uint4*>(arow + ((uint32_t(2 * wi) ^ swz) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<uint4*>(arow + ((uint32_t(2 * wi + 1) ^ swz) << 4)) = make_uint4(v[4], v[5], v[6], v[7]);
+        decode16_prepared(cw.w[wi], v);
+        const uint32_t piece = uint32_t(2 * (wi + WORDS * hh));
+        *reinterpret_cast<uint4*>(arow + ((piece ^ swz) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<uint4*>(arow + (((piece + 1) ^ swz) << 4)) = make_uint4(v[4], v[5], v[6], v[7]);
       }
     };
     // Chunk c of a tile goes to ring slot and phase of the running count over all tiles; code[c % SLOTS] is its codes.
@@ -277,7 +306,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
       }
       decode_to(n_ch, false);
       if (!ok) break;
-      const int n = min(bn, it.end - it.tok0), f0 = it.ft * BM + q4 * 32;
+      const int n = min(bn, it.end - it.tok0), f0 = it.ft * BM + q4 * (BM / 4);
       if (!mbar_wait(smem_u32(&ctl.acc_full), tile & 1u, abort_flag, p.status, JB200_STATUS_GEMM_EPILOGUE)) break;
       tc_fence_after_sync();
       __syncwarp();
@@ -292,30 +321,50 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
           if (row >= 2 * p.M) row = -1;
         }
         __syncwarp();
-        uint32_t v[32];
-        tmem_ld_32x32(tmem + (uint32_t(q4 * 32) << 16) + uint32_t(c0), v);
-        tmem_ld_wait();
-        if (p.epilogue == JB200_EPI_RESID_F32) {
-          // lane = feature: a warp instruction covers 128 bytes of one token's row
-          float* o = reinterpret_cast<float*>(p.out) + f0 + lane;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int rj = __shfl_sync(0xffffffffu, row, j);
-            const float val = alpha * __uint_as_float(v[j]);
-            if (rj >= 0) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + size_t(rj) * p.N), "f"(val) : "memory");
+        if constexpr (BM == 128) {
+          uint32_t v[32];
+          tmem_ld_32x32(tmem + (uint32_t(q4 * 32) << 16) + uint32_t(c0), v);
+          tmem_ld_wait();
+          if (p.epilogue == JB200_EPI_RESID_F32) {
+            // lane = feature: a warp instruction covers 128 bytes of one token's row
+            float* o = reinterpret_cast<float*>(p.out) + f0 + lane;
+  #pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int rj = __shfl_sync(0xffffffffu, row, j);
+              const float val = alpha * __uint_as_float(v[j]);
+              if (rj >= 0) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + size_t(rj) * p.N), "f"(val) : "memory");
+            }
+          } else {
+            const bool gelu = p.epilogue == JB200_EPI_GELU_BF16;
+            const int odd = lane & 1;
+            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + f0 + (lane & ~1);
+  #pragma unroll
+            for (int jj = 0; jj < 16; ++jj) {
+              float a = alpha * __uint_as_float(v[2 * jj]), b = alpha * __uint_as_float(v[2 * jj + 1]);
+              if (gelu) { a = gelu_erf(a); b = gelu_erf(b); }
+              const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+              const uint32_t w2 = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);   // features (f & ~1, f | 1)
+              const int rj = __shfl_sync(0xffffffffu, row, 2 * jj + odd);            // token 2jj (even lanes) / 2jj + 1 (odd)
+              if (rj >= 0) *reinterpret_cast<uint32_t*>(o + size_t(rj) * p.N) = w2;
+            }
           }
         } else {
-          const bool gelu = p.epilogue == JB200_EPI_GELU_BF16;
-          const int odd = lane & 1;
-          __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + f0 + (lane & ~1);
+          const int feat = f0 + (lane >> 2) * 2, c = lane & 3;
+          uint32_t v[16];
+          tmem_ld_16x256b_x4(tmem + (uint32_t(q4 * 32) << 16) + uint32_t(c0), v);
+          tmem_ld_wait();
 #pragma unroll
-          for (int jj = 0; jj < 16; ++jj) {
-            float a = alpha * __uint_as_float(v[2 * jj]), b = alpha * __uint_as_float(v[2 * jj + 1]);
-            if (gelu) { a = gelu_erf(a); b = gelu_erf(b); }
-            const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-            const uint32_t w2 = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);   // features (f & ~1, f | 1)
-            const int rj = __shfl_sync(0xffffffffu, row, 2 * jj + odd);            // token 2jj (even lanes) / 2jj + 1 (odd)
-            if (rj >= 0) *reinterpret_cast<uint32_t*>(o + size_t(rj) * p.N) = w2;
+          for (int j = 0; j < 8; ++j) {                    // token 8 (j / 2) + 2c + j % 2
+            const int rj = __shfl_sync(0xffffffffu, row, 8 * (j >> 1) + 2 * c + (j & 1));
+            float a = alpha * __uint_as_float(v[4 * (j >> 1) + (j & 1)]), b = alpha * __uint_as_float(v[4 * (j >> 1) + 2 + (j & 1)]);
+            if (p.epilogue == JB200_EPI_RESID_F32) {
+              if (rj >= 0)
+                asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(reinterpret_cast<float*>(p.out) + size_t(rj) * p.N + feat),
+                             "f"(a), "f"(b) : "memory");
+            } else {
+              if (p.epilogue == JB200_EPI_GELU_BF16) { a = gelu_erf(a); b = gelu_erf(b); }
+              if (rj >= 0) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.out) + size_t(rj) * p.N + feat) = pack_bf16x2(a, b);
+            }
           }
         }
       }
@@ -335,16 +384,16 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
 }  // namespace
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bn, int bn_max,
-                    cudaStream_t stream) {
+                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bm, int bn,
+                    int bn_max, cudaStream_t stream) {
   JB_REQUIRE(epilogue == JB200_EPI_BF16 || epilogue == JB200_EPI_GELU_BF16 || epilogue == JB200_EPI_RESID_F32, "mid_gemm: epilogue %d", epilogue);
-  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn % 16 == 0 &&
+  JB_REQUIRE(M >= 1 && (bm == 64 || bm == 128) && N % bm == 0 && K % (BK * CK) == 0 && alpha_rows % bm == 0 && bn >= 16 && bn % 16 == 0 &&
                  bn_max >= bn && bn_max <= 256 && bn_max % 16 == 0 &&
                  G >= 1 && G <= MAX_GROUPS,
              "mid_gemm: bad shape (M=%d, N=%d, K=%d, bn=%d)", M, N, K, bn);
   MidParams p;
   p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
-  p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / BM; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
+  p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / bm; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
   p.tmem_cols = bn_max <= 32 ? 32u : bn_max <= 64 ? 64u : bn_max <= 128 ? 128u : 256u;
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
@@ -355,7 +404,7 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   size_t smem = 0;
   for (int i = 0; i < 3; ++i) {
     p.bn[i] = i == 0 ? bn : i == 1 ? (bn + bn_max) / 32 * 16 : bn_max;
-    const int chunk = CK * (A_BYTES + p.bn[i] * BK * 2);
+    const int chunk = CK * (bm * BK * 2 + p.bn[i] * BK * 2);
     int S = (224 * 1024) / chunk;
     if (S > MAX_CHUNKS) S = MAX_CHUNKS;
     if (S > n_kb / CK) S = n_kb / CK;
@@ -369,8 +418,14 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
   const long tiles = seg ? (M + bn - 1) / bn + G - 1 : long(G) * ((M + bn - 1) / bn), items = tiles * p.n_ft;   // at most
-  JB_MAX_SMEM(mid_gemm_kernel, 225 * 1024);
-  launch_dep(mid_gemm_kernel, dim3(unsigned(items < sms ? items : sms)), THREADS, smem, stream, maps, p);
+  const dim3 grid(unsigned(items < sms ? items : sms));
+  if (bm == 64) {
+    JB_MAX_SMEM(mid_gemm_kernel<64>, 225 * 1024);
+    launch_dep(mid_gemm_kernel<64>, grid, THREADS, smem, stream, maps, p);
+  } else {
+    JB_MAX_SMEM(mid_gemm_kernel<128>, 225 * 1024);
+    launch_dep(mid_gemm_kernel<128>, grid, THREADS, smem, stream, maps, p);
+  }
   JB_LAUNCH_CHECK("mid_gemm_kernel");
   return JB200_OK;
 }

@@ -6,7 +6,7 @@
 // and the token rows - one contiguous block each - to shared memory with asynchronous 16-byte copies, all in flight at
 // once (one bulk copy per row measured 1-3 us slower); a warp then walks all of K for 16 out-features x 8 or 16 tokens.
 // The weights do not depend on the kernel before this one: in a chain they are requested before the grid dependency is
-// waited for.  Token tiles beyond the first can be given to CTAs of their own (grid z), which copy the codes again.  The first
+// waited for.  The first
 // expert matrix takes every token for every expert and stores only the routed ones (fetching rows through the gather map put one
 // more memory latency and most of the instructions of a call in front of its first MMA).
 //
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) small_gemm_kernel(const SmallG
   pdl_trigger();
 
 #pragma unroll 1
-  for (int tb = beg + int(blockIdx.z) * TOK; tb < end; tb += int(gridDim.z) * TOK) {
+  for (int tb = beg; tb < end; tb += TOK) {
     const int n = min(TOK, end - tb);
     copy_rows(act, p.x + size_t(tb) * p.K, n, p.K / 8);
     int dst[TT][2];                              // output rows of this lane's tokens, -1: not stored
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) small_gemm_kernel(const SmallG
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         if (dst[i][h] >= 0) store_pair(p, size_t(dst[i][h]) * p.N + feat, alpha * acc[i][h], alpha * acc[i][2 + h]);
-    if (tb + int(gridDim.z) * TOK < end) __syncthreads();         // this pass has used its rows
+    if (tb + TOK < end) __syncthreads();         // this pass has used its rows
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
@@ -184,7 +184,7 @@ bool small_gemm_fits(int tile, int K) { return smem_need(tile, K) <= SMEM_MAX; }
 
 int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N,
                       int G, const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out,
-                      int tile, int tiles, cudaStream_t stream) {
+                      int tile, cudaStream_t stream) {
   JB_REQUIRE(epilogue == JB200_EPI_BF16 || epilogue == JB200_EPI_GELU_BF16 || epilogue == JB200_EPI_RESID_F32, "small_gemm: epilogue %d", epilogue);
   JB_REQUIRE(M >= 1 && K % 128 == 0 && N % 64 == 0 && alpha_rows % 64 == 0, "small_gemm: bad shape (M=%d, N=%d, K=%d)", M, N, K);
   SmallGemmParams p;
@@ -192,9 +192,9 @@ int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepare
   p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
   p.M = M; p.N = N; p.K = K; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
   const size_t smem = smem_need(tile, K);
-  JB_REQUIRE((tile == 8 || tile == 16) && tiles >= 1 && tiles <= 65535, "small_gemm: %d tiles of %d tokens", tiles, tile);
+  JB_REQUIRE(tile == 8 || tile == 16, "small_gemm: tiles of %d tokens", tile);
   JB_REQUIRE(smem <= SMEM_MAX, "small_gemm: in_features (%d) too large", K);
-  const dim3 grid(N / (16 * ROW_WARPS), G, tiles);
+  const dim3 grid(N / (16 * ROW_WARPS), G);
   if (tile == 8) {
     JB_MAX_SMEM(small_gemm_kernel<1>, SMEM_MAX);
     launch_dep(small_gemm_kernel<1>, grid, 32 * ROW_WARPS, smem, stream, p);

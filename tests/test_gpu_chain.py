@@ -145,6 +145,12 @@ def test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("B,T", [(1, 48), (1, 80), (1, 100), (100, 1), (160, 1), (161, 1), (192, 1), (300, 1), (1, 160), (1, 161), (1, 448), (1, 449)])
+def test_chain_around_the_edges_of_its_gemm_tiles(B, T):
+    """Products in tiles of 64 and of 128 out-features, one and several token tiles, all rows for every expert and dispatched ones."""
+    test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T)
+
+
 @pytest.mark.parametrize("skew", [0.5, 4.0])
 @pytest.mark.parametrize("T", [17, 64, 129, 256, 640, 960])
 def test_chain_with_uneven_experts(T, skew):
