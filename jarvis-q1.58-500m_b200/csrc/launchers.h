@@ -108,7 +108,7 @@ size_t attn_scan_scratch_bytes(int B, int T, int H);
 
 // Few tokens (moe_small.cu).
 constexpr int ROUTE_SMALL_MAX = 256;   // tokens
-constexpr int TAIL_MAX = 128;          // tokens: a warp each in the eight CTAs of a cluster
+constexpr int TAIL_MAX = 256;          // tokens: a warp each in the CTAs of a cluster
 int tail_max_tokens(int C, int T);     // tokens launch_tail takes at this width
 int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const float* w_norm, float eps, float* x, void* xn_bf16,
                       int n_rows, int C, void* zero, size_t zero_bytes, cudaStream_t stream);

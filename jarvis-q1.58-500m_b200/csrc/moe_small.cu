@@ -11,6 +11,8 @@
 // waited for.  Every value is rounded and every sum ordered as in the kernels these stand for (rmsnorm_router_kernel,
 // meta_small_kernel, scatter_combine_kernel, lsf_step_norm_kernel, lsf_tma_kernel, lsf_short_kernel, rmsnorm_kernel): the
 // results are theirs bit for bit, so that a token's experts do not depend on how many others share its call.
+#include <algorithm>
+
 #include "common.cuh"
 #include "moe_finalize.cuh"
 #include "moe_router.cuh"
@@ -140,7 +142,7 @@ struct TailParams {
   int B, T, N, C;
 };
 
-constexpr int MAX_CTAS = 8;
+constexpr int MAX_CTAS = 16;                           // non-portable cluster size: asked for before use (tail_fits)
 constexpr int MAX_WARPS = TAIL_MAX / MAX_CTAS;         // tokens per CTA: one warp each
 
 // Slots of a token's two expert rows.  Without finite logits (idx -1) both are expert 0's, and a GEMM that takes all rows for every
@@ -182,7 +184,7 @@ __device__ __forceinline__ float tail_decay(const TailParams& p, Combined c, flo
   if (warp == 0) {
     double a = lane < n_warps ? part[lane][0] : 0.0, b = lane < n_warps ? part[lane][1] : 0.0;
 #pragma unroll
-    for (int o = MAX_WARPS / 2; o > 0; o >>= 1) {
+    for (int o = 16; o > 0; o >>= 1) {
       a += __shfl_xor_sync(0xffffffffu, a, o);
       b += __shfl_xor_sync(0xffffffffu, b, o);
     }
@@ -295,24 +297,32 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailPar
 }
 
 // Several tokens per sequence.  Rows are combined and normalised by the CTA that owns the token (token n: CTA n % n_cta, a
-// warp each), the scan runs where all tokens of a channel are (CTA k: channels [128 k, 128 k + 128)); the rows change
-// hands through distributed shared memory.  ms [N][128] bf16: combined rows of the CTA's channels; hs: their membranes; xr [N / n_cta][C] f32:
-// updated residual rows of the CTA's tokens.
-constexpr int SCAN_CH = 128, RUN = 16;         // channels per CTA; tokens per run (lsf_tma_kernel's warp runs)
+// warp each), the scan runs where all tokens of a channel are (CTA k: channels [64 k, 64 k + 64)); the rows change
+// hands through distributed shared memory.  ms [N][64] bf16: combined rows of the CTA's channels; hs [B][64]: their membranes; xr
+// [N / n_cta][C] f32: updated residual rows of the CTA's tokens; ends [B * runs][64]: what a run of tokens leaves from a zero carry.
+// Bound by latency: copies, three exchanges and one chain over a run.  Sixteen CTAs of 64 channels move half the rows per SM that eight
+// of 128 did, a run's end is worked out once, by its own warp, and residual rows are fetched while the kernel ahead runs (with eight, carries
+// recomputed by every later run and rows fetched behind the exchange 24 layers and head took 1034, 1067, 1370 us at 37, 64, 128 tokens;
+// so 963, 973, 1199).
+constexpr int SCAN_CH = 64, RUN = 16;          // channels per CTA, two per lane; tokens per run (lsf_tma_kernel's warp runs)
 
 __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailParams p, const int n_cta) {
   extern __shared__ __align__(16) uint8_t tail_smem[];
   __shared__ double s_part[MAX_WARPS][2], s_all[MAX_CTAS][2];
   __shared__ float s_alpha;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, threads = blockDim.x;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, n_warps = blockDim.x >> 5;
   const int N = p.N, B = p.B, T = p.T, C = p.C;
-  const int rank = n_cta > 1 ? int(cluster_rank()) : 0;
-  uint8_t* ms = tail_smem;                                                     // [N][256 bytes]
-  float* hs = reinterpret_cast<float*>(tail_smem + size_t(N) * SCAN_CH * 2);   // [B][128]: h_out may be h_in
-  float* xr = hs + size_t(B) * SCAN_CH;                                        // [ceil(N / n_cta)][C]
+  const int rank = int(cluster_rank());
+  // runs of 16 tokens from a zero carry, the carries along the runs, then every token's value, with the roundings of
+  // lsf_tma_kernel (T > 8) or lsf_short_kernel
+  const int n_runs = T > 8 ? (T + RUN - 1) / RUN : 1, run_len = T > 8 ? RUN : T, items = B * n_runs;
+  uint8_t* ms = tail_smem;                                                     // [N][128 bytes]
+  float* hs = reinterpret_cast<float*>(tail_smem + size_t(N) * SCAN_CH * 2);   // h_out may be h_in
+  float* xr = hs + size_t(B) * SCAN_CH;
+  float* ends = xr + size_t((N + n_cta - 1) / n_cta) * C;
   const int own = rank + warp * n_cta;                                         // this warp's token
   const bool on = own < N;
-  if (n_cta > 1) cluster_arrive();
+  cluster_arrive();
   const float var_scale = __ldg(p.var_scale);
   int2 sl = make_int2(0, 0);
   float2 g = make_float2(0.f, 0.f);
@@ -320,13 +330,23 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
     sl = tail_slots(p, own);
     g = *reinterpret_cast<const float2*>(p.gates + 2 * own);
   }
-  for (int i = tid; i < B * SCAN_CH / 4; i += threads) {
+  const size_t ch = size_t(rank) * SCAN_CH + lane * 2;
+  float2 xv[RUN];                // the run's residual values, all in flight together
+  auto load_x = [&](int b, int run) {
+#pragma unroll
+    for (int j = 0; j < RUN; ++j) {
+      const int t = run * RUN + j;
+      if (j < run_len && t < T) xv[j] = *reinterpret_cast<const float2*>(p.x + size_t(b * T + t) * C + ch);
+    }
+  };
+  if (warp < items) load_x(warp / n_runs, warp % n_runs);
+  for (int i = tid; i < B * SCAN_CH / 4; i += blockDim.x) {
     const int b = i / (SCAN_CH / 4), q = i % (SCAN_CH / 4);
     reinterpret_cast<float4*>(hs)[i] =
         p.h_in ? *(reinterpret_cast<const float4*>(p.h_in + size_t(b) * C + rank * SCAN_CH) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   float l_bal = 0.f;
-  if (rank == 0 && tid == threads - 1)
+  if (rank == 0 && tid == int(blockDim.x) - 1)
     l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.inv_tokens, p.st.balance_alpha);
   __syncwarp();
   pdl_wait();
@@ -340,19 +360,12 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
 #pragma unroll
       for (int i = 0; i < GROUPS; ++i) {
         const int c = (i * 32 + lane) * 8;
-        if (c < C) {
-          const uint32_t dst = smem_u32(ms) + uint32_t(own) * (SCAN_CH * 2) + uint32_t(c % SCAN_CH) * 2u;
-          cluster_st_128(n_cta > 1 ? cluster_map(dst, uint32_t(c / SCAN_CH)) : dst, m[i]);
-        }
+        if (c < C) cluster_st_128(cluster_map(smem_u32(ms) + uint32_t(own) * (SCAN_CH * 2) + uint32_t(c % SCAN_CH) * 2u, uint32_t(c / SCAN_CH)), m[i]);
       }
     }
   });
-  if (rank == 0 && tid == threads - 1) p.st.scalars[0] = l_bal;
+  if (rank == 0 && tid == int(blockDim.x) - 1) p.st.scalars[0] = l_bal;
 
-  // ---- scan of the CTA's channels, two per thread: runs of 16 tokens from a zero carry, the carries along the runs,
-  // then every token's value, with the roundings of lsf_tma_kernel (T > 8) or lsf_short_kernel ----
-  const int pairs = SCAN_CH / 2, col = tid % pairs, slot = tid / pairs, slots = threads / pairs;
-  const int n_runs = T > 8 ? (T + RUN - 1) / RUN : 1, run_len = T > 8 ? RUN : T;
   const float one_m = 1.0f - alpha;
   float pw[RUN];
   {
@@ -360,30 +373,32 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
 #pragma unroll
     for (int i = 0; i < RUN; ++i) { pw[i] = a; a *= alpha; }
   }
-  auto m_at = [&](int n) { return *reinterpret_cast<const uint32_t*>(ms + size_t(n) * (SCAN_CH * 2) + col * 4); };
+  auto m_at = [&](int n) { return *reinterpret_cast<const uint32_t*>(ms + size_t(n) * (SCAN_CH * 2) + lane * 4); };
+  if (n_runs > 1) {
 #pragma unroll 1
-  for (int w = slot; w < B * n_runs; w += slots) {           // (sequence, run)
-    const int b = w / n_runs, run = w - b * n_runs;
-    const size_t ch = size_t(rank) * SCAN_CH + col * 2;
-    float2 h = *reinterpret_cast<const float2*>(hs + b * SCAN_CH + col * 2);
-    float2 xv[RUN];              // the run's residual values, all in flight together
-#pragma unroll
-    for (int j = 0; j < RUN; ++j) {
-      const int t = run * RUN + j;
-      if (j < run_len && t < T) xv[j] = *reinterpret_cast<const float2*>(p.x + size_t(b * T + t) * C + ch);
-    }
-    // the carry into this run: the ends of the runs before it, each scanned from zero (at most seven)
-#pragma unroll 1
-    for (int q = 0; q < run; ++q) {
+    for (int w = warp; w < items; w += n_warps) {
+      const int b = w / n_runs, run = w - b * n_runs;
+      if (run == n_runs - 1) continue;                       // nobody's carry
       float2 e = make_float2(0.f, 0.f);
-#pragma unroll 4
+#pragma unroll
       for (int j = 0; j < RUN; ++j) {
-        const uint32_t v = m_at(b * T + q * RUN + j);
-        e.x = alpha * e.x + one_m * bf16_lo(v);
-        e.y = alpha * e.y + one_m * bf16_hi(v);
+        const uint32_t v = m_at(b * T + run * RUN + j);
+        e.x = __fmaf_rn(alpha, e.x, __fmul_rn(one_m, bf16_lo(v)));
+        e.y = __fmaf_rn(alpha, e.y, __fmul_rn(one_m, bf16_hi(v)));
       }
-      h.x = pw[RUN - 1] * h.x + e.x;
-      h.y = pw[RUN - 1] * h.y + e.y;
+      *reinterpret_cast<float2*>(ends + w * SCAN_CH + lane * 2) = e;
+    }
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int w = warp; w < items; w += n_warps) {              // (sequence, run)
+    const int b = w / n_runs, run = w - b * n_runs;
+    if (w != warp) load_x(b, run);
+    float2 h = *reinterpret_cast<const float2*>(hs + b * SCAN_CH + lane * 2);
+    for (int q = 0; q < run; ++q) {                          // the carry into this run
+      const float2 e = *reinterpret_cast<const float2*>(ends + (b * n_runs + q) * SCAN_CH + lane * 2);
+      h.x = __fmaf_rn(pw[RUN - 1], h.x, e.x);
+      h.y = __fmaf_rn(pw[RUN - 1], h.y, e.y);
     }
     float2 loc = make_float2(0.f, 0.f);
     float2 hv = h;
@@ -394,10 +409,10 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
         const int n = b * T + t;
         const uint32_t v = m_at(n);
         if (T > 8) {
-          loc.x = alpha * loc.x + one_m * bf16_lo(v);
-          loc.y = alpha * loc.y + one_m * bf16_hi(v);
-          hv.x = loc.x + pw[j] * h.x;
-          hv.y = loc.y + pw[j] * h.y;
+          loc.x = __fmaf_rn(alpha, loc.x, __fmul_rn(one_m, bf16_lo(v)));
+          loc.y = __fmaf_rn(alpha, loc.y, __fmul_rn(one_m, bf16_hi(v)));
+          hv.x = __fmaf_rn(pw[j], h.x, loc.x);
+          hv.y = __fmaf_rn(pw[j], h.y, loc.y);
         } else {
           hv.x = lsf_step(alpha, hv.x, bf16_lo(v));
           hv.y = lsf_step(alpha, hv.y, bf16_hi(v));
@@ -405,13 +420,25 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
         xv[j].x = xv[j].x + hv.x;
         xv[j].y = xv[j].y + hv.y;
         *reinterpret_cast<float2*>(p.x + size_t(n) * C + ch) = xv[j];
-        const uint32_t dst = smem_u32(xr) + (uint32_t(n / n_cta) * uint32_t(C) + uint32_t(ch)) * 4u;
-        cluster_st_64(n_cta > 1 ? cluster_map(dst, uint32_t(n % n_cta)) : dst, xv[j]);
+        cluster_st_64(cluster_map(smem_u32(xr) + (uint32_t(n / n_cta) * uint32_t(C) + uint32_t(ch)) * 4u, uint32_t(n % n_cta)), xv[j]);
         if (t == T - 1) *reinterpret_cast<float2*>(p.h_out + size_t(b) * C + ch) = hv;
       }
     }
   }
-  if (n_cta > 1) { __syncwarp(); cluster_arrive(); cluster_wait(); } else __syncthreads();
+  float4 wn[GROUPS][2];
+  if (p.w_norm) {
+#pragma unroll
+    for (int i = 0; i < GROUPS; ++i) {
+      const int c = (i * 32 + lane) * 8;
+      if (c < C) {
+        wn[i][0] = __ldg(reinterpret_cast<const float4*>(p.w_norm + c));
+        wn[i][1] = __ldg(reinterpret_cast<const float4*>(p.w_norm + c) + 1);
+      }
+    }
+  }
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
   if (!p.w_norm || !on) return;
 
   // ---- the norm of the warp's token ----
@@ -431,10 +458,41 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
 #pragma unroll
   for (int i = 0; i < GROUPS; ++i) {
     const int c = (i * 32 + lane) * 8;
-    if (c < C)
-      *reinterpret_cast<uint4*>(p.xn + size_t(own) * C + c) =
-          norm8(v[i], r, __ldg(reinterpret_cast<const float4*>(p.w_norm + c)), __ldg(reinterpret_cast<const float4*>(p.w_norm + c) + 1));
+    if (c < C) *reinterpret_cast<uint4*>(p.xn + size_t(own) * C + c) = norm8(v[i], r, wn[i][0], wn[i][1]);
   }
+}
+
+// [N][64] bf16, [B][64] f32, [rows][C] f32, [items][64] f32; B and items are at most N / 2 and N / 16 + B.
+inline size_t tail_smem_bytes(int N, int B, int rows, int C, int items) {
+  return size_t(N) * SCAN_CH * 2 + (size_t(B) * SCAN_CH + size_t(rows) * C + size_t(items) * SCAN_CH) * sizeof(float);
+}
+constexpr size_t TAIL_SMEM = 200 * 1024;
+
+// Whether clusters of sixteen CTAs can run here, with the shared memory of the largest call; also sets the kernels up for them.
+bool tail_fits() {
+  constexpr int MAX_DEVICES = 64;
+  static std::atomic<int> known[MAX_DEVICES];            // 0 not asked yet, 1 yes, -1 no
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return false;
+  int k = known[dev].load(std::memory_order_acquire);
+  if (k == 0) {
+    int n = 0;
+    const void* scan = reinterpret_cast<const void*>(tail_scan_kernel);
+    const void* step = reinterpret_cast<const void*>(tail_step_kernel);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = MAX_CTAS; cfg.blockDim = 32 * MAX_WARPS; cfg.dynamicSmemBytes = TAIL_SMEM; cfg.attrs = at; cfg.numAttrs = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = MAX_CTAS; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    const bool ok = cudaFuncSetAttribute(scan, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaFuncSetAttribute(step, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_SMEM)) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, tail_scan_kernel, &cfg) == cudaSuccess && n >= 1;
+    if (!ok) (void)cudaGetLastError();
+    k = ok ? 1 : -1;
+    known[dev].store(k, std::memory_order_release);
+  }
+  return k > 0;
 }
 
 // Embedding rows into the f32 residual stream (jarvis_model.py:498) and, while they are in registers, norm1 of the first
@@ -526,7 +584,7 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
   p.B = B; p.T = T; p.N = N; p.C = C;
   if (T == 1) {
     // a lone CTA while its SM can take the rows (4 KB in, 10 KB out each), else eight
-    const int n_cta = N <= 4 ? 1 : MAX_CTAS;
+    const int n_cta = N <= 4 ? 1 : 8;
     const int warps = (N + n_cta - 1) / n_cta;
     if (n_cta == 1) launch_dep(tail_step_kernel, 1, 32 * warps, 0, stream, p, 1);
     else launch_dep_cluster(tail_step_kernel, n_cta, 32 * warps, 0, n_cta, stream, p, n_cta);
@@ -534,14 +592,19 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
     return JB200_OK;
   }
   const int n_cta = C / SCAN_CH, rows = (N + n_cta - 1) / n_cta;
-  const size_t smem = size_t(N) * SCAN_CH * 2 + (size_t(B) * SCAN_CH + size_t(rows) * C) * sizeof(float);
-  JB_MAX_SMEM(tail_scan_kernel, size_t(TAIL_MAX) * SCAN_CH * 2 + (size_t(TAIL_MAX / 2) * SCAN_CH + size_t(MAX_WARPS) * 1024) * sizeof(float));
-  if (n_cta == 1) launch_dep(tail_scan_kernel, 1, 32 * MAX_WARPS, smem, stream, p, 1);
-  else launch_dep_cluster(tail_scan_kernel, n_cta, 32 * MAX_WARPS, smem, n_cta, stream, p, n_cta);
+  const int items = B * (T > 8 ? (T + RUN - 1) / RUN : 1), warps = std::max(rows, std::min(items, MAX_WARPS));
+  const size_t smem = tail_smem_bytes(N, B, rows, C, items);
+  JB_MAX_SMEM(tail_scan_kernel, TAIL_SMEM);
+  launch_dep_cluster(tail_scan_kernel, n_cta, 32 * warps, smem, n_cta, stream, p, n_cta);
   JB_LAUNCH_CHECK("tail_scan_kernel");
   return JB200_OK;
 }
 
-int tail_max_tokens(int C, int T) { return T == 1 ? TAIL_MAX : MAX_WARPS * (C / SCAN_CH); }
+int tail_max_tokens(int C, int T) {
+  // steps: sixteen CTAs for 129 to 256 of them lose against combine and lsf_step_norm (150 1431 -> 1479 us a step, 256 1747 -> 1843);
+  // prompts against combine, scan and norm: 129 tokens 1291 -> 1244 us, 180 1337 -> 1307, 4 x 60 1323 -> 1340, 256 1381 -> 1402
+  if (T == 1) return 8 * MAX_WARPS;
+  return C / SCAN_CH <= 8 || tail_fits() ? 12 * (C / SCAN_CH) : 0;
+}
 
 }  // namespace jb

@@ -151,6 +151,12 @@ def test_chain_around_the_edges_of_its_gemm_tiles(B, T):
     test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T)
 
 
+@pytest.mark.parametrize("B,T", [(1, 192), (1, 193), (2, 96), (64, 3), (21, 9), (11, 17), (10, 19), (5, 33), (24, 8)])
+def test_chain_around_the_edges_of_its_tail_cluster(B, T):
+    """Runs of up to 8, 16 and more tokens, more of them than warps, tokens for every warp of a CTA and for few."""
+    test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T)
+
+
 @pytest.mark.parametrize("skew", [0.5, 4.0])
 @pytest.mark.parametrize("T", [17, 64, 129, 256, 640, 960])
 def test_chain_with_uneven_experts(T, skew):
