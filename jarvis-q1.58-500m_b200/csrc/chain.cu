@@ -61,7 +61,7 @@ constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // take the first one's output for both assignments (stored twice by the GEMM, 64 sequences were 1.5 % slower).  24 layers and head as a graph
 // with the dispatch -> without: 80 tokens 1141 -> 1060 us, 128 1188 -> 1133, 5 x 30 1227 -> 1200, 180 1310 -> 1298, steps of 128 sequences
 // 1360 -> 1326, 192 equal, 256 tokens 1375 -> 1423.
-constexpr int ALL_ROWS_TOKENS = 160;
+constexpr int ALL_ROWS_TOKENS = MID_ROUTE_TOKENS, LATE_MAPS_TOKENS = 64;
 // Tiles of the latency form.  Tokens: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
 // tokens) that leaves a launch of so many rows in each group on `room` SMs.
 inline int mid_tile(int rows, int groups, int n_ft, int room) {
@@ -156,10 +156,10 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
   auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
-                      const int32_t* seg, const int64_t* ids, const int32_t* sc, int epi, void* dst, int most) {
-    if (!seg) {                                // every group over all rows
+                      const int32_t* seg, const MidRoutes* routes, int epi, void* dst, int most) {
+    if (!seg && !(routes && routes->segments)) {                                // every group over all rows
       const MidTile t = mid_tiles(M, G, n_out, G > 1 ? most : sms, most);
-      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, t.bm, t.bn, t.bn, st);
+      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bm, t.bn, t.bn, st);
     }
     // Segments are known on the device alone: a tile for rows that are spread evenly, with an eighth to spare, and one for
     // whatever they are (M / bn_max tiles and one cut short in every other group).
@@ -167,7 +167,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const MidTile t = mid_tiles(even + (even + 7) / 8, G, n_out, sms, most);
     int bn_max = t.bn;
     while (bn_max < 256 && long(n_out / t.bm) * ((M + bn_max - 1) / bn_max + G - 1) > sms) bn_max += 16;
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, ids, sc, epi, dst, t.bm, t.bn, bn_max, st);
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bm, t.bn, bn_max, st);
   };
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
@@ -203,7 +203,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, QKV_MOST));
+      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, JB200_EPI_BF16, qkv, QKV_MOST));
     else
       JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st, nullptr, true));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
@@ -214,14 +214,20 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, OUT_MOST));
+      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, JB200_EPI_RESID_F32, x, OUT_MOST));
     else
       JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st, nullptr, true));
 
-    // moe(norm2(x))
+    // moe(norm2(x)).  late_maps: the first expert GEMM makes the dispatch maps in a warp of its own, beside its MMAs; in the router
+    // they are behind a fence, a ticket and a second reading of the ids.  24 layers and head as a graph so 80 tokens 1061 -> 1005 us, 128
+    // 1139 -> 1098, 5 x 30 1199 -> 1157, steps of 100 sequences 1187 -> 1158; 37 tokens 877 -> 888, 64 939 -> 942: the sort is short there,
+    // and the epilogue waits for its slots.
+    const bool late_maps = mid && N > LATE_MAPS_TOKENS && N <= ALL_ROWS_TOKENS;
+    const MidRoutes store = {idx, !late_maps, false, counts, offs, scatter, gather, gate_idx};
+    const MidRoutes rows_of = {idx, false, true, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (N <= ROUTE_SMALL_MAX) {
       JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, ticket, counts, offs,
-                                scatter, gather, gate_idx, st));
+                                late_maps ? nullptr : scatter, gather, gate_idx, st));
     } else {
       JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true));
       JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
@@ -231,18 +237,18 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       if (small)
         JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, small_tile, st));
       else
-        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
+        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, &store, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
     } else {
       JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
-        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, nullptr, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
       else
         JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, EXPERT_MOST));
+      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, late_maps ? nullptr : offs, late_maps ? &rows_of : nullptr, JB200_EPI_BF16, y, EXPERT_MOST));
     else
       JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st, nullptr, true));
 

@@ -35,10 +35,19 @@ int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepare
 // It keeps whole rows of codes and activations in shared memory: in-features it can take with such tiles (about 7200 with 8
 // rows, 4800 with 16).
 bool small_gemm_fits(int tile, int K);
-// The same product again, latency form on tcgen05 (mid_gemm.cu) with tiles of bm (64 or 128) out-features and bn rows, or of bn_max rows
-// where the segments need more tiles of bn than there are SMs.  Arguments as launch_small_gemm.
+// The same product again, latency form on tcgen05 (mid_gemm.cu) with tiles of bm (64 or 128) out-features and bn rows,
+// or of bn_max rows where the segments need more tiles of bn than there are SMs.  Arguments as launch_small_gemm, but for routes
+// (top-2 assignments).  Every group takes all M rows and the routed ones are stored at their slots: `given` by scatter, or, for at
+// most MID_ROUTE_TOKENS tokens, in dispatch order, and the maps are left in scatter and the others.  With segments (no maps) the M rows
+// are the assignments in that order.
+constexpr int MID_ROUTE_TOKENS = 160;
+struct MidRoutes {
+  const int64_t* ids;          // [tokens][2]
+  bool given, segments;
+  int *counts, *offsets, *scatter, *gather, *gate_idx;
+};
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bm, int bn,
+                    const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bm, int bn,
                     int bn_max, cudaStream_t stream);
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);
@@ -112,6 +121,7 @@ constexpr int TAIL_MAX = 256;          // tokens: a warp each in the CTAs of a c
 int tail_max_tokens(int C, int T);     // tokens launch_tail takes at this width
 int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const float* w_norm, float eps, float* x, void* xn_bf16,
                       int n_rows, int C, void* zero, size_t zero_bytes, cudaStream_t stream);
+// scatter null: the assignments alone, no maps.
 int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router, int N, int C, int E,
                        int64_t* idx, float* gates, double* probs_sum, int* hist, int* ticket, int* counts, int* offsets,
                        int* scatter, int* gather, int* gate_idx, cudaStream_t stream);

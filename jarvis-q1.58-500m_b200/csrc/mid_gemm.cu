@@ -19,6 +19,7 @@
 #include "common.cuh"
 #include "gemm_shared.cuh"
 #include "launchers.h"
+#include "row_math.cuh"
 
 namespace jb {
 
@@ -26,15 +27,14 @@ namespace {
 
 constexpr int BK = 64;
 constexpr int CK = 2;                          // K-blocks per chunk (four: 1-3 % slower, the ring gets too coarse)
-constexpr int MAX_CHUNKS = 8, DEC_WARP0 = 2, THREADS = 320;
+constexpr int MAX_CHUNKS = 8, DEC_WARP0 = 2, THREADS = 320, MAP_WARP = 10;
 constexpr int SLOTS = 4;                       // chunks whose codes are in registers
 
 struct MidParams {
   const uint8_t* w;            // prepared [G][N][K/4]
   const float* alpha;          // [G][N / alpha_rows]
-  const int32_t* seg;          // device [G+1] or null (every group takes rows [0, M))
-  const int64_t* idx;          // [M][2]: row n of group g goes to out row scatter[2n + k] where idx[2n + k] == g; null: row n
-  const int32_t* scatter;
+  const int32_t* seg;          // device [G+1] or null (every group takes rows [0, M), or the segments are counted from routes)
+  MidRoutes routes;
   void* out;
   int M, N, K, G, n_ft, alpha_rows, epilogue;
   int bn[3], chunks[3];        // token tiles and their rings: the first whose items are one wave, else the last
@@ -93,8 +93,16 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)
 // BM: out-features of a tile.  128 is the MMA's full rate; but up to ~100 tokens a step is bound by the shared memory that its
 // operands are read from (BM + bn rows of 32 bytes, 128 bytes a cycle, and the same again for the decoded weights and
 // the copied rows), so tiles of 64, on twice as many SMs, take less time each: half the codes to fetch and decode, half the epilogue.
-template <int BM>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int E>
+__device__ __forceinline__ void sort_some(const long long* ids, int N, int lane, const MidRoutes& r) {
+  if (N <= 64) sort_routes<E, 4>(ids, N, lane, r.counts, r.offsets, r.scatter, r.gather, r.gate_idx);
+  else sort_routes<E, 2 * MID_ROUTE_TOKENS / 32>(ids, N, lane, r.counts, r.offsets, r.scatter, r.gather, r.gate_idx);
+}
+
+// ROUTE: 0 rows or segments as given, 1 rows stored in dispatch order and the maps left by a warp of their own, 2 segments counted from
+// the ids, 3 rows stored at the slots of the maps (kernels of their own: the code of the others costs a plain call 1 %).
+template <int BM, int ROUTE>
+__global__ void __launch_bounds__(ROUTE == 1 ? THREADS + 32 : THREADS, ROUTE == 1 || ROUTE == 2 ? 2 : 1)
 mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   constexpr int A_BYTES = BM * BK * 2;
   extern __shared__ uint8_t smem_raw[];
@@ -128,6 +136,24 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     if (lane < p.G) {
       beg = p.seg ? min(max(__ldg(p.seg + lane), 0), p.M) : 0;
       end = p.seg ? min(max(__ldg(p.seg + lane + 1), 0), p.M) : p.M;
+    }
+    if constexpr (ROUTE == 2) {                // the kernel ahead makes the offsets; the ids are older
+      constexpr int ROUNDS = 2 * MID_ROUTE_TOKENS / 32;
+      int ex[ROUNDS], n_of = 0;
+#pragma unroll
+      for (int i = 0; i < ROUNDS; ++i) ex[i] = i * 32 + lane < p.M ? max(int(p.routes.ids[i * 32 + lane]), 0) : -1;
+      for (int q = 0; q < p.G; ++q) {
+        int n = 0;
+#pragma unroll
+        for (int i = 0; i < ROUNDS; ++i) n += __popc(__ballot_sync(0xffffffffu, ex[i] == q));
+        if (lane == q) n_of = n;
+      }
+      end = n_of;
+      for (int d = 1; d < MAX_GROUPS; d *= 2) {
+        const int u = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += u;
+      }
+      beg = end - n_of;
     }
     auto tiles_of = [&](int bn) {              // token tiles of groups 0..lane
       int t = end > beg ? (end - beg + bn - 1) / bn : 0;
@@ -223,6 +249,15 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
         if (++s == S) { s = 0; ph ^= 1u; ad = adesc0; bd = bdesc0; }
       }
     }
+  } else if (ROUTE == 1 && warp == MAP_WARP) {
+    // ---------------- dispatch maps, beside everything else ----------------
+    pdl_wait();
+    pdl_trigger();
+    if (blockIdx.x == 0) {
+      const long long* ids = reinterpret_cast<const long long*>(p.routes.ids);
+      if (p.G == 4) sort_some<4>(ids, p.M, lane, p.routes);
+      else sort_some<8>(ids, p.M, lane, p.routes);
+    }
   } else {
     // ---------------- decoders, then epilogue ----------------
     // This thread decodes, of K-block `par` of every chunk, row r of the tile: all 64 codes with 128 rows, half `hh` of them with 64.
@@ -307,6 +342,28 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
       decode_to(n_ch, false);
       if (!ok) break;
       const int n = min(bn, it.end - it.tok0), f0 = it.ft * BM + q4 * (BM / 4);
+      // The slots of the group's rows in dispatch order, while the last MMAs run: those of all lower groups come first, then rank
+      // by token (a token has at most one assignment of a group; without finite logits both are group 0's, and the first is stored).
+      constexpr int BLOCKS = MID_ROUTE_TOKENS / 32;
+      unsigned first[BLOCKS], second[BLOCKS];          // tokens whose first / second assignment is the group's
+      int slot0 = 0;
+      if constexpr (ROUTE == 1) {
+        int a[BLOCKS], b[BLOCKS];
+#pragma unroll
+        for (int k = 0; k < BLOCKS; ++k) {
+          const int t = 32 * k + lane;
+          const longlong2 e = t < p.M ? *reinterpret_cast<const longlong2*>(p.routes.ids + 2 * t) : make_longlong2(MAX_GROUPS, MAX_GROUPS);
+          a[k] = max(int(e.x), 0);
+          b[k] = max(int(e.y), 0);
+        }
+#pragma unroll
+        for (int k = 0; k < BLOCKS; ++k) {
+          if (32 * k >= p.M) { first[k] = second[k] = 0u; continue; }
+          first[k] = __ballot_sync(0xffffffffu, a[k] == it.grp);
+          second[k] = __ballot_sync(0xffffffffu, b[k] == it.grp);
+          slot0 += __popc(__ballot_sync(0xffffffffu, a[k] < it.grp)) + __popc(__ballot_sync(0xffffffffu, b[k] < it.grp));
+        }
+      }
       if (!mbar_wait(smem_u32(&ctl.acc_full), tile & 1u, abort_flag, p.status, JB200_STATUS_GEMM_EPILOGUE)) break;
       tc_fence_after_sync();
       __syncwarp();
@@ -314,11 +371,24 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
       for (int c0 = par * 32; c0 < n; c0 += 64) {
         // output row of token c0 + lane; -1: not stored
         int row = c0 + lane < n ? it.tok0 + c0 + lane : -1;
-        if (p.idx && row >= 0) {
-          const longlong2 e = *reinterpret_cast<const longlong2*>(p.idx + 2 * row);
-          const int2 sc = *reinterpret_cast<const int2*>(p.scatter + 2 * row);
+        if (ROUTE == 3 && row >= 0) {
+          const longlong2 e = *reinterpret_cast<const longlong2*>(p.routes.ids + 2 * row);
+          const int2 sc = *reinterpret_cast<const int2*>(p.routes.scatter + 2 * row);
           row = e.x == it.grp ? sc.x : (e.y == it.grp ? sc.y : -1);
           if (row >= 2 * p.M) row = -1;
+        }
+        if constexpr (ROUTE == 1) {
+          const int t = it.tok0 + c0 + lane;
+          int slot = slot0;
+          bool mine = false;
+#pragma unroll
+          for (int k = 0; k < BLOCKS; ++k) {
+            const int d = t - 32 * k;
+            const unsigned before = d <= 0 ? 0u : d >= 32 ? 0xffffffffu : (1u << d) - 1u;
+            slot += __popc(first[k] & before) + __popc(second[k] & before);
+            if (d >= 0 && d < 32) mine = ((first[k] | second[k]) >> d) & 1u;
+          }
+          row = row >= 0 && mine && slot < 2 * p.M ? slot : -1;
         }
         __syncwarp();
         if constexpr (BM == 128) {
@@ -328,7 +398,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
           if (p.epilogue == JB200_EPI_RESID_F32) {
             // lane = feature: a warp instruction covers 128 bytes of one token's row
             float* o = reinterpret_cast<float*>(p.out) + f0 + lane;
-  #pragma unroll
+#pragma unroll
             for (int j = 0; j < 32; ++j) {
               const int rj = __shfl_sync(0xffffffffu, row, j);
               const float val = alpha * __uint_as_float(v[j]);
@@ -338,7 +408,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
             const bool gelu = p.epilogue == JB200_EPI_GELU_BF16;
             const int odd = lane & 1;
             __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + f0 + (lane & ~1);
-  #pragma unroll
+#pragma unroll
             for (int jj = 0; jj < 16; ++jj) {
               float a = alpha * __uint_as_float(v[2 * jj]), b = alpha * __uint_as_float(v[2 * jj + 1]);
               if (gelu) { a = gelu_erf(a); b = gelu_erf(b); }
@@ -384,7 +454,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
 }  // namespace
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const int64_t* idx, const int32_t* scatter, int epilogue, void* out, int bm, int bn,
+                    const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bm, int bn,
                     int bn_max, cudaStream_t stream) {
   JB_REQUIRE(epilogue == JB200_EPI_BF16 || epilogue == JB200_EPI_GELU_BF16 || epilogue == JB200_EPI_RESID_F32, "mid_gemm: epilogue %d", epilogue);
   JB_REQUIRE(M >= 1 && (bm == 64 || bm == 128) && N % bm == 0 && K % (BK * CK) == 0 && alpha_rows % bm == 0 && bn >= 16 && bn % 16 == 0 &&
@@ -392,8 +462,11 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
                  G >= 1 && G <= MAX_GROUPS,
              "mid_gemm: bad shape (M=%d, N=%d, K=%d, bn=%d)", M, N, K, bn);
   MidParams p;
-  p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.idx = idx; p.scatter = scatter; p.out = out;
+  p.w = w_prepared; p.alpha = alpha; p.seg = seg; p.routes = routes ? *routes : MidRoutes{}; p.out = out;
   p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / bm; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
+  const bool cut = seg || p.routes.segments, given = routes && routes->given;
+  JB_REQUIRE(!routes || given || (!seg && (G == 4 || G == 8) && M <= (cut ? 2 : 1) * MID_ROUTE_TOKENS && (p.routes.scatter == nullptr) == cut),
+             "mid_gemm: %d rows by %d groups cannot be routed here", M, G);
   p.tmem_cols = bn_max <= 32 ? 32u : bn_max <= 64 ? 64u : bn_max <= 128 ? 128u : 256u;
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
@@ -417,15 +490,27 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   }
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
-  const long tiles = seg ? (M + bn - 1) / bn + G - 1 : long(G) * ((M + bn - 1) / bn), items = tiles * p.n_ft;   // at most
+  const long tiles = cut ? (M + bn - 1) / bn + G - 1 : long(G) * ((M + bn - 1) / bn), items = tiles * p.n_ft;   // at most
   const dim3 grid(unsigned(items < sms ? items : sms));
-  if (bm == 64) {
-    JB_MAX_SMEM(mid_gemm_kernel<64>, 225 * 1024);
-    launch_dep(mid_gemm_kernel<64>, grid, THREADS, smem, stream, maps, p);
-  } else {
-    JB_MAX_SMEM(mid_gemm_kernel<128>, 225 * 1024);
-    launch_dep(mid_gemm_kernel<128>, grid, THREADS, smem, stream, maps, p);
-  }
+  const int route = !routes ? 0 : given ? 3 : cut ? 2 : 1;
+  auto launch = [&](auto kernel, std::atomic<unsigned long long>* set_up) {
+    const int rc = set_max_smem(reinterpret_cast<const void*>(kernel), 225 * 1024, set_up);
+    if (rc == JB200_OK) launch_dep(kernel, grid, route == 1 ? THREADS + 32 : THREADS, smem, stream, maps, p);
+    return rc;
+  };
+  static std::atomic<unsigned long long> set_up[8];
+  int rc;
+  if (bm == 64)
+    rc = route == 0   ? launch(mid_gemm_kernel<64, 0>, set_up)
+         : route == 1 ? launch(mid_gemm_kernel<64, 1>, set_up + 1)
+         : route == 2 ? launch(mid_gemm_kernel<64, 2>, set_up + 2)
+                      : launch(mid_gemm_kernel<64, 3>, set_up + 3);
+  else
+    rc = route == 0   ? launch(mid_gemm_kernel<128, 0>, set_up + 4)
+         : route == 1 ? launch(mid_gemm_kernel<128, 1>, set_up + 5)
+         : route == 2 ? launch(mid_gemm_kernel<128, 2>, set_up + 6)
+                      : launch(mid_gemm_kernel<128, 3>, set_up + 7);
+  if (rc != JB200_OK) return rc;
   JB_LAUNCH_CHECK("mid_gemm_kernel");
   return JB200_OK;
 }

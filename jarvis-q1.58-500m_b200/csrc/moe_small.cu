@@ -33,7 +33,7 @@ struct RouteParams {
   double* probs_sum;           // [E] accumulated
   int* hist;                   // [E] accumulated
   int* ticket;                 // zero on entry
-  int *counts, *offsets, *scatter, *gather, *gate_idx;
+  int *counts, *offsets, *scatter, *gather, *gate_idx;   // scatter null: no maps
   float eps;
   int N, C;
 };
@@ -115,8 +115,10 @@ __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
       atomicAdd(p.probs_sum + e, double(pr[e]));
       if (h_acc[e]) atomicAdd(p.hist + e, 1);
     }
-    __threadfence();
-    last = atomicAdd(p.ticket, 1) == p.N - 1;
+    if (p.scatter) {
+      __threadfence();
+      last = atomicAdd(p.ticket, 1) == p.N - 1;
+    }
   }
   if (!__shfl_sync(0xffffffffu, last, 0)) return;
   __threadfence();
