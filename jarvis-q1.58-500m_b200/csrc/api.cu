@@ -474,5 +474,8 @@ int jb200_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepar
 
 void jb200_host_decode16(uint32_t word, uint32_t* out8) { decode16_host(word, out8); }
 void jb200_host_decode16_prepared(uint32_t word, uint32_t* out8) { decode16_prepared_host(word, out8); }
+int jb200_host_expert_tiles(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out6) {
+  return expert_tiles_host(tokens, second, C, E, hidden, sms, out6);
+}
 
 }  // extern "C"

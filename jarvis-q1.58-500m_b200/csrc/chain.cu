@@ -60,13 +60,19 @@ constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // finite router logits is stored once, for expert 0, and its second hidden row holds whatever was there: combine and tail
 // take the first one's output for both assignments (stored twice by the GEMM, 64 sequences were 1.5 % slower).  24 layers and head as a graph
 // with the dispatch -> without: 80 tokens 1141 -> 1060 us, 128 1188 -> 1133, 5 x 30 1227 -> 1200, 180 1310 -> 1298, steps of 128 sequences
-// 1360 -> 1326, 192 equal, 256 tokens 1375 -> 1423.
+// 1360 -> 1326, 192 equal, 256 tokens 1375 -> 1423.  The same line for eight experts and for wide ones, though their MMAs are four times
+// the routed ones (d_model 1024, us a layer, 65, 100 and 160 tokens): 8 x 2048 48.8 -> 44.7, 52.5 -> 48.1, 58.0 -> 55.3; 4 x 4096 51.1 -> 47.9, 53.5 -> 50.4,
+// 61.4 -> 58.5; 8 x 4096 61.2 -> 60.9, 67.1 -> 65.6, 76.8 -> 73.6; steps of 160 sequences 67.2 -> 65.5, 67.3 -> 65.4, 86.5 -> 80.2.
 constexpr int ALL_ROWS_TOKENS = MID_ROUTE_TOKENS, LATE_MAPS_TOKENS = 64;
 // Tiles of the latency form.  Tokens: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
-// tokens) that leaves a launch of so many rows in each group on `room` SMs.
+// tokens) that leaves a launch of so many rows in each group on `room` SMs; where even one tile for all rows does not, that one.  (A
+// larger one would be MMAs, copies and shared memory for rows that are not there: 256 rows where the first expert matrix has more than
+// EXPERT_MOST tiles, us a layer at d_model 1024, 17, 37 and 128 tokens: 8 x 2048 49.4 -> 42.6, 50.5 -> 43.8, 51.4 -> 49.6; 4 x 4096 51.1 -> 44.0,
+// 52.0 -> 45.3, 55.1 -> 53.6; 8 x 4096 74.6 -> 55.4, 74.7 -> 59.5, 70.8 -> 67.7.)
 inline int mid_tile(int rows, int groups, int n_ft, int room) {
-  int bn = rows <= 64 ? (rows + 15) / 16 * 16 : 64;
-  while (bn < 256 && long(n_ft) * groups * ((rows + bn - 1) / bn) > room) bn += 16;
+  const int all = rows < 256 ? (rows + 15) / 16 * 16 : 256;
+  int bn = all < 64 ? all : 64;
+  while (bn < all && long(n_ft) * groups * ((rows + bn - 1) / bn) > room) bn += 16;
   return bn;
 }
 // Out-features: 64 or 128 a tile.  The time of a tile goes with both its sides, but SMs that a launch takes are not there for the
@@ -77,11 +83,28 @@ inline int mid_tile(int rows, int groups, int n_ft, int room) {
 // expert matrix of 37 tokens (128 SMs) 949 -> 1013.
 constexpr int QKV_MOST = 100, OUT_MOST = 120, EXPERT_MOST = 74;
 struct MidTile {
-  int bm, bn;
+  int bm, bn, bn_max;
 };
 inline MidTile mid_tiles(int rows, int groups, int n_out, int room, int most) {
   const int b64 = mid_tile(rows, groups, n_out / 64, room), b128 = mid_tile(rows, groups, n_out / 128, room);
-  return long(n_out / 64) * groups * ((rows + b64 - 1) / b64) <= most && 64 + b64 < 128 + b128 ? MidTile{64, b64} : MidTile{128, b128};
+  const bool narrow = long(n_out / 64) * groups * ((rows + b64 - 1) / b64) <= most && 64 + b64 < 128 + b128;
+  return narrow ? MidTile{64, b64, b64} : MidTile{128, b128, b128};
+}
+// Tiles of a launch: every group takes all M rows, or (cut) M rows are cut into segments that are known on the device alone: a
+// tile for rows that are spread evenly, with an eighth to spare, and one for whatever they are (M / bn_max tiles and one cut short in
+// every other group), up to one for all of them.
+inline MidTile mid_plan(int M, int groups, int n_out, bool cut, int most, int sms) {
+  if (!cut) return mid_tiles(M, groups, n_out, groups > 1 ? most : sms, most);
+  const int even = (M + groups - 1) / groups;
+  MidTile t = mid_tiles(even + (even + 7) / 8, groups, n_out, sms, most);
+  while (t.bn_max < 256 && t.bn_max < M && long(n_out / t.bm) * ((M + t.bn_max - 1) / t.bn_max + groups - 1) > sms) t.bn_max += 16;
+  return t;
+}
+
+// The first expert matrix takes every token's row, or the assignments in segments; the second one always segments.
+inline MidTile expert_plan(int tokens, bool second, int C, int E, int hidden, int sms) {
+  const bool cut = second || tokens > ALL_ROWS_TOKENS;
+  return mid_plan(cut ? 2 * tokens : tokens, E, second ? C : hidden, cut, EXPERT_MOST, sms);
 }
 
 #define JB_TRY(call)                    \
@@ -91,6 +114,16 @@ inline MidTile mid_tiles(int rows, int groups, int n_out, int room, int most) {
   } while (0)
 
 }  // namespace
+
+int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out) {
+  if (tokens < 1 || tokens > MID_TOKENS || C < 128 || E < 1 || hidden < 128 || sms < 1 || !out) return 0;
+  const MidTile t = expert_plan(tokens, second != 0, C, E, hidden, sms);
+  const int K = second ? hidden : C;
+  out[0] = !second && tokens <= ALL_ROWS_TOKENS;
+  out[1] = t.bm; out[2] = t.bn; out[3] = t.bn_max;
+  out[4] = mid_gemm_chunks(t.bm, t.bn, K); out[5] = mid_gemm_chunks(t.bm, t.bn_max, K);
+  return 1;
+}
 
 size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(E + 1) * 4 + 7) / 8 * 8; }
 
@@ -152,23 +185,15 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   float* x = f->x;
   const int small_tile = N <= 8 ? 8 : 16;
   const bool small = N <= SMALL_TOKENS && small_gemm_fits(small_tile, std::max(C, hidden));   // beyond, the tcgen05 form streams K
-  const bool mid = !small && N <= MID_TOKENS;
+  const bool mid = !small && N <= MID_TOKENS, all_rows = N <= ALL_ROWS_TOKENS;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
   auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
-                      const int32_t* seg, const MidRoutes* routes, int epi, void* dst, int most) {
-    if (!seg && !(routes && routes->segments)) {                                // every group over all rows
-      const MidTile t = mid_tiles(M, G, n_out, G > 1 ? most : sms, most);
-      return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bm, t.bn, t.bn, st);
-    }
-    // Segments are known on the device alone: a tile for rows that are spread evenly, with an eighth to spare, and one for
-    // whatever they are (M / bn_max tiles and one cut short in every other group).
-    const int even = (M + G - 1) / G;
-    const MidTile t = mid_tiles(even + (even + 7) / 8, G, n_out, sms, most);
-    int bn_max = t.bn;
-    while (bn_max < 256 && long(n_out / t.bm) * ((M + bn_max - 1) / bn_max + G - 1) > sms) bn_max += 16;
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bm, t.bn, bn_max, st);
+                      const int32_t* seg, const MidRoutes* routes, int epi, void* dst, const MidTile& t) {
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bm, t.bn, t.bn_max, st);
   };
+  const MidTile qkv_tile = mid_plan(N, 1, 3 * C, false, QKV_MOST, sms), out_tile = mid_plan(N, 1, C, false, OUT_MOST, sms);
+  const MidTile w1_tile = expert_plan(N, false, C, E, hidden, sms), w2_tile = expert_plan(N, true, C, E, hidden, sms);
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
   uint8_t* acc0 = static_cast<uint8_t*>(f->accumulators);
@@ -203,7 +228,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, JB200_EPI_BF16, qkv, QKV_MOST));
+      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile));
     else
       JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st, nullptr, true));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
@@ -214,7 +239,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, JB200_EPI_RESID_F32, x, OUT_MOST));
+      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile));
     else
       JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st, nullptr, true));
 
@@ -222,7 +247,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     // they are behind a fence, a ticket and a second reading of the ids.  24 layers and head as a graph so 80 tokens 1061 -> 1005 us, 128
     // 1139 -> 1098, 5 x 30 1199 -> 1157, steps of 100 sequences 1187 -> 1158; 37 tokens 877 -> 888, 64 939 -> 942: the sort is short there,
     // and the epilogue waits for its slots.
-    const bool late_maps = mid && N > LATE_MAPS_TOKENS && N <= ALL_ROWS_TOKENS;
+    const bool late_maps = mid && all_rows && N > LATE_MAPS_TOKENS;
     const MidRoutes store = {idx, !late_maps, false, counts, offs, scatter, gather, gate_idx};
     const MidRoutes rows_of = {idx, false, true, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (N <= ROUTE_SMALL_MAX) {
@@ -232,23 +257,23 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true));
       JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
     }
-    if (N <= ALL_ROWS_TOKENS) {
+    if (all_rows) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
       if (small)
         JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, small_tile, st));
       else
-        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, &store, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
+        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, &store, JB200_EPI_GELU_BF16, hid, w1_tile));
     } else {
       JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
-        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, JB200_EPI_GELU_BF16, hid, EXPERT_MOST));
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, JB200_EPI_GELU_BF16, hid, w1_tile));
       else
         JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, late_maps ? nullptr : offs, late_maps ? &rows_of : nullptr, JB200_EPI_BF16, y, EXPERT_MOST));
+      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, late_maps ? nullptr : offs, late_maps ? &rows_of : nullptr, JB200_EPI_BF16, y, w2_tile));
     else
       JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st, nullptr, true));
 
@@ -263,7 +288,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
                          w_next ? xn_next : nullptr, B, T, C, st));
       continue;
     }
-    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st, true, N <= ALL_ROWS_TOKENS ? idx : nullptr));
+    JB_TRY(launch_scatter_combine(y, gates, scatter, N, 2, C, out, 1, acc, st, true, all_rows ? idx : nullptr));
     if (h16 && T == 1) {
       JB_TRY(launch_lsf_step_norm(out, stats, p.var_scale, p.alpha_min, p.alpha_max, h_in, h_out, x, w_next, eps_next,
                                   w_next ? xn_next : nullptr, B, C, st, true));

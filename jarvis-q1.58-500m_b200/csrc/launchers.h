@@ -49,6 +49,7 @@ struct MidRoutes {
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
                     const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bm, int bn,
                     int bn_max, cudaStream_t stream);
+int mid_gemm_chunks(int bm, int bn, int K);   // chunks of its ring with such tiles
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);
 void decode16_prepared_host(uint32_t w_canonical, uint32_t* out8);
@@ -138,6 +139,7 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
                         cudaStream_t stream, bool* taken);
 int launch_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
                          const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, cudaStream_t stream);
+int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out);
 size_t accumulator_bytes(int E);
 size_t routing_layout(int N, int E, size_t* offsets);
 size_t forward_workspace_bytes(int B, int T, int C, int H, int E, int hidden);

@@ -451,7 +451,11 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   }
 }
 
+inline int chunk_bytes(int bm, int bn) { return CK * (bm + bn) * BK * 2; }
+
 }  // namespace
+
+int mid_gemm_chunks(int bm, int bn, int K) { return std::min({(224 * 1024) / chunk_bytes(bm, bn), MAX_CHUNKS, K / (BK * CK)}); }
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
                     const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bm, int bn,
@@ -477,12 +481,8 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   size_t smem = 0;
   for (int i = 0; i < 3; ++i) {
     p.bn[i] = i == 0 ? bn : i == 1 ? (bn + bn_max) / 32 * 16 : bn_max;
-    const int chunk = CK * (bm * BK * 2 + p.bn[i] * BK * 2);
-    int S = (224 * 1024) / chunk;
-    if (S > MAX_CHUNKS) S = MAX_CHUNKS;
-    if (S > n_kb / CK) S = n_kb / CK;
-    p.chunks[i] = S;
-    smem = std::max(smem, size_t(S) * chunk + 1024);
+    p.chunks[i] = mid_gemm_chunks(bm, p.bn[i], K);
+    smem = std::max(smem, size_t(p.chunks[i]) * chunk_bytes(bm, p.bn[i]) + 1024);
     const cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(p.bn[i]), cuuint32_t(CK)};
     const int rc = encode_tiled(&maps.x[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, x_bf16, gdim, gstride, box,
                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "mid_gemm");

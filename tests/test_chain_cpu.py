@@ -293,3 +293,26 @@ def test_an_edited_layer_alone_is_laid_out_again(step_library):
     del tab, other
     gc.collect()
     assert all(ref() is None for ref in held)            # a table does not keep the one before it
+
+
+@pytest.mark.parametrize("E", [4, 8])
+@pytest.mark.parametrize("hidden", [1024, 2048, 4096])
+def test_expert_tiles_are_no_larger_than_their_rows(E, hidden):
+    """However many tiles the experts need, a token tile ends with the rows there are: the smallest that leaves the launch on half of the
+    SMs (all rows for every expert) or on all of them, else one for all rows."""
+    lib, out = _lib.load(), (C.c_int32 * 6)()
+    up = lambda n: (n + 15) // 16 * 16
+    for tokens in range(1, 961):
+        assert lib.jb200_host_expert_tiles(tokens, 0, 1024, E, hidden, 148, out) == 1
+        all_rows, bm, bn, bn_max, ring, ring_max = out
+        rows = tokens if all_rows else -(-2 * tokens // E)
+        assert all_rows == (tokens <= 160) and bn <= bn_max <= min(256, up(2 * tokens)) and ring >= ring_max >= 2
+        if all_rows:
+            tiles = lambda n: hidden // bm * E * -(-tokens // n)
+            assert bn == bn_max <= up(tokens) and ring == min(8, 224 * 1024 // (256 * (bm + bn)))
+            assert tiles(bn) <= 74 or bn == up(tokens)
+            assert bn <= 64 or tiles(bn - 16) > 74
+        else:
+            assert bn <= up(rows + -(-rows // 8))
+        assert lib.jb200_host_expert_tiles(tokens, 1, 1024, E, hidden, 148, out) == 1 and out[2] <= out[3] <= min(256, up(2 * tokens))
+    assert lib.jb200_host_expert_tiles(961, 0, 1024, E, hidden, 148, out) == 0

@@ -548,3 +548,36 @@ def test_dispatch_around_the_sizes_of_its_one_launch_form(N, E, C):
     want = ops.moe_metadata(idx, E)
     assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(rows, ops.dispatch_gather(x, want[3]))
     assert _lib.device_status() == 0
+
+
+def _chain_against_kernels(C, E, mult, B, T):
+    """One block with E experts of mult * C features, carried states: chain and kernel by kernel, rows, states, routes and maps."""
+    from jarvis_b200 import chain
+    torch.manual_seed(7)
+    blk = jm.JarvisBlock(C, C // 64, num_experts=E, max_seq_len=256)
+    blk.moe = jm.SparseMoELayer(C, num_experts=E, hidden_mult=mult)
+    blk = jm.ternary_init_(blk).cuda().eval()
+    gen = torch.Generator(device="cuda").manual_seed(B * 1000 + T)
+    x, h = torch.randn(B * T, C, generator=gen, device="cuda"), torch.randn(B, C, generator=gen, device="cuda")
+    S = torch.randn(B, C // 64, 64, 64, generator=gen, device="cuda")
+    norm = (torch.rand(C, generator=gen, device="cuda") + 0.5, 1e-6)
+    xa, xb = x.clone(), x.clone()
+    acc, hist = torch.zeros(2 + E, dtype=torch.float64, device="cuda"), torch.zeros(E, dtype=torch.int32, device="cuda")
+    ha, sa, Sa = blk.forward_rows(xa, B, T, h, 5, S, want_attn_state=True, scratch=(acc, hist, torch.zeros(3, device="cuda")))
+    idx_a, gates_a, _ = blk.moe.last_routing
+    r = chain.run(chain.table_of(blk, [blk]), xb, B, T, start_pos=5, h_in=[h], s_in=[S], want_state=True, final_norm=norm)
+    idx, gates, maps = blk.moe.last_routing
+    assert torch.equal(idx, idx_a) and torch.equal(gates, gates_a)
+    assert all(torch.equal(a, b) for a, b in zip(maps, ops.moe_metadata(idx.contiguous(), E)))
+    assert torch.equal(xb, xa) and torch.equal(r.h[0], ha) and torch.equal(r.S[0], Sa)
+    assert torch.equal(r.hidden, ops.rmsnorm(xb, *norm))
+    assert torch.equal(r.scalars[0][1:], sa[1:]) and rel(r.scalars[0][:1], sa[:1]) <= 2 * ULP
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("E,mult,B,T", [(8, 2, 1, 17), (8, 2, 1, 37), (8, 2, 64, 1), (8, 2, 1, 65), (8, 2, 100, 1), (8, 2, 3, 30), (8, 2, 1, 160),
+                                        (8, 2, 1, 161), (8, 1, 1, 129), (4, 4, 1, 37), (4, 4, 1, 100), (4, 4, 1, 161), (8, 4, 1, 20), (8, 4, 1, 160),
+                                        (8, 4, 1, 300), (4, 5, 1, 12)])
+def test_chain_with_eight_experts_and_with_wide_ones(E, mult, B, T):
+    """All rows for every expert and dispatched ones, maps by the router and by the first expert matrix, more tiles than SMs."""
+    _chain_against_kernels(1024, E, mult, B, T)
