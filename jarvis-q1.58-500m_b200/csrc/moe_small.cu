@@ -470,29 +470,29 @@ inline size_t tail_smem_bytes(int N, int B, int rows, int C, int items) {
 }
 constexpr size_t TAIL_SMEM = 200 * 1024;
 
-// Whether clusters of sixteen CTAs can run here, with the shared memory of the largest call; also sets the kernels up for them.
-bool tail_fits() {
-  constexpr int MAX_DEVICES = 64;
-  static std::atomic<int> known[MAX_DEVICES];            // 0 not asked yet, 1 yes, -1 no
+// Whether clusters of n_cta CTAs can run here, with the shared memory of the largest call; also sets the kernel up for them.  Eight is the
+// portable limit; each size beyond it is asked for by itself, since a launch that is refused would come in the middle of a forward.
+bool tail_fits(int n_cta) {
+  constexpr int MAX_DEVICES = 64, PORTABLE = 8;
+  static std::atomic<int> known[MAX_DEVICES][MAX_CTAS + 1];            // 0 not asked yet, 1 yes, -1 no
+  if (n_cta <= PORTABLE) return true;
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return false;
-  int k = known[dev].load(std::memory_order_acquire);
+  if (n_cta > MAX_CTAS || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return false;
+  int k = known[dev][n_cta].load(std::memory_order_acquire);
   if (k == 0) {
     int n = 0;
     const void* scan = reinterpret_cast<const void*>(tail_scan_kernel);
-    const void* step = reinterpret_cast<const void*>(tail_step_kernel);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
-    cfg.gridDim = MAX_CTAS; cfg.blockDim = 32 * MAX_WARPS; cfg.dynamicSmemBytes = TAIL_SMEM; cfg.attrs = at; cfg.numAttrs = 1;
+    cfg.gridDim = n_cta; cfg.blockDim = 32 * MAX_WARPS; cfg.dynamicSmemBytes = TAIL_SMEM; cfg.attrs = at; cfg.numAttrs = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = MAX_CTAS; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.x = unsigned(n_cta); at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     const bool ok = cudaFuncSetAttribute(scan, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                    cudaFuncSetAttribute(step, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                     cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_SMEM)) == cudaSuccess &&
                     cudaOccupancyMaxActiveClusters(&n, tail_scan_kernel, &cfg) == cudaSuccess && n >= 1;
     if (!ok) (void)cudaGetLastError();
     k = ok ? 1 : -1;
-    known[dev].store(k, std::memory_order_release);
+    known[dev][n_cta].store(k, std::memory_order_release);
   }
   return k > 0;
 }
@@ -606,7 +606,7 @@ int tail_max_tokens(int C, int T) {
   // steps: sixteen CTAs for 129 to 256 of them lose against combine and lsf_step_norm (150 1431 -> 1479 us a step, 256 1747 -> 1843);
   // prompts against combine, scan and norm: 129 tokens 1291 -> 1244 us, 180 1337 -> 1307, 4 x 60 1323 -> 1340, 256 1381 -> 1402
   if (T == 1) return 8 * MAX_WARPS;
-  return C / SCAN_CH <= 8 || tail_fits() ? 12 * (C / SCAN_CH) : 0;
+  return tail_fits(C / SCAN_CH) ? 12 * (C / SCAN_CH) : 0;
 }
 
 }  // namespace jb

@@ -581,3 +581,10 @@ def _chain_against_kernels(C, E, mult, B, T):
 def test_chain_with_eight_experts_and_with_wide_ones(E, mult, B, T):
     """All rows for every expert and dispatched ones, maps by the router and by the first expert matrix, more tiles than SMs."""
     _chain_against_kernels(1024, E, mult, B, T)
+
+
+@pytest.mark.parametrize("C", [384, 512, 640, 768, 896])
+@pytest.mark.parametrize("B,T", [(1, 20), (1, 72), (7, 10), (9, 8), (1, 120), (2, 96)])
+def test_chain_at_other_widths(C, B, T):
+    """The tail in clusters of C / 64 CTAs, up to twelve tokens for each of them, and beyond that in kernels of its own."""
+    _chain_against_kernels(C, 4, 2, B, T)
