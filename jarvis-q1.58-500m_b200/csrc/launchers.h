@@ -118,8 +118,7 @@ size_t attn_scan_scratch_bytes(int B, int T, int H);
 
 // Few tokens (moe_small.cu).
 constexpr int ROUTE_SMALL_MAX = 256;   // tokens
-constexpr int TAIL_MAX = 256;          // tokens: a warp each in the CTAs of a cluster
-int tail_max_tokens(int C, int T);     // tokens launch_tail takes at this width
+int tail_max_tokens(int C, int T);     // most tokens that launch_tail takes: 128 of single-token steps, 12 for every 64 channels of prompts
 int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const float* w_norm, float eps, float* x, void* xn_bf16,
                       int n_rows, int C, void* zero, size_t zero_bytes, cudaStream_t stream);
 // scatter null: the assignments alone, no maps.

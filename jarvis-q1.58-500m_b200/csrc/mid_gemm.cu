@@ -93,16 +93,12 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)
 // BM: out-features of a tile.  128 is the MMA's full rate; but up to ~100 tokens a step is bound by the shared memory that its
 // operands are read from (BM + bn rows of 32 bytes, 128 bytes a cycle, and the same again for the decoded weights and
 // the copied rows), so tiles of 64, on twice as many SMs, take less time each: half the codes to fetch and decode, half the epilogue.
-template <int E>
-__device__ __forceinline__ void sort_some(const long long* ids, int N, int lane, const MidRoutes& r) {
-  if (N <= 64) sort_routes<E, 4>(ids, N, lane, r.counts, r.offsets, r.scatter, r.gather, r.gate_idx);
-  else sort_routes<E, 2 * MID_ROUTE_TOKENS / 32>(ids, N, lane, r.counts, r.offsets, r.scatter, r.gather, r.gate_idx);
-}
-
 // ROUTE: 0 rows or segments as given, 1 rows stored in dispatch order and the maps left by a warp of their own, 2 segments counted from
 // the ids, 3 rows stored at the slots of the maps (kernels of their own: the code of the others costs a plain call 1 %).
+// One CTA per SM, since its ring fills the shared memory: routes 1 and 2 kept to registers for two took 0.5 to 1.4 % of a layer more (65 to 160
+// tokens: prompts of 100 40.9 -> 41.2 us, steps of 100 46.8 -> 47.5).
 template <int BM, int ROUTE>
-__global__ void __launch_bounds__(ROUTE == 1 ? THREADS + 32 : THREADS, ROUTE == 1 || ROUTE == 2 ? 2 : 1)
+__global__ void __launch_bounds__(ROUTE == 1 ? THREADS + 32 : THREADS, 1)
 mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   constexpr int A_BYTES = BM * BK * 2;
   extern __shared__ uint8_t smem_raw[];
@@ -255,8 +251,10 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     pdl_trigger();
     if (blockIdx.x == 0) {
       const long long* ids = reinterpret_cast<const long long*>(p.routes.ids);
-      if (p.G == 4) sort_some<4>(ids, p.M, lane, p.routes);
-      else sort_some<8>(ids, p.M, lane, p.routes);
+      const MidRoutes& r = p.routes;
+      constexpr int ROUNDS = 2 * MID_ROUTE_TOKENS / 32;
+      if (p.G == 4) sort_routes<4, ROUNDS>(ids, p.M, lane, r.counts, r.offsets, r.scatter, r.gather, r.gate_idx);
+      else sort_routes<8, ROUNDS>(ids, p.M, lane, r.counts, r.offsets, r.scatter, r.gather, r.gate_idx);
     }
   } else {
     // ---------------- decoders, then epilogue ----------------

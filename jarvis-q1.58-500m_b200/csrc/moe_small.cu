@@ -145,7 +145,7 @@ struct TailParams {
 };
 
 constexpr int MAX_CTAS = 16;                           // non-portable cluster size: asked for before use (tail_fits)
-constexpr int MAX_WARPS = TAIL_MAX / MAX_CTAS;         // tokens per CTA: one warp each
+constexpr int MAX_WARPS = 16;                          // of a CTA; a warp takes one token (tail_max_tokens: how many come)
 
 // Slots of a token's two expert rows.  Without finite logits (idx -1) both are expert 0's, and a GEMM that takes all rows for every
 // expert has made the first of them alone.
