@@ -119,7 +119,8 @@ def test_cross_entropy_of_values_that_are_not_finite(V):
                                  (1, 256), (1, 257), (257, 1), (1, 640), (1, 960), (1, 961), (1, 40), (1, 41)])
 def test_chain_at_full_width_around_the_edges_of_its_small_kernels(B, T):
     """d_model 1024: the kernels for few tokens (GEMM forms up to 16, up to 960 and beyond, router up to 256, row cluster up to
-    128) against the kernel-by-kernel path; mixed routing, carried state, one expert without tokens at the smallest sizes."""
+    128 steps or 192 tokens of prompts) against the kernel-by-kernel path; mixed routing, carried state, one expert without tokens
+    at the smallest sizes."""
     from jarvis_b200 import chain
     torch.manual_seed(7)
     blk = jm.ternary_init_(jm.JarvisBlock(1024, 16, max_seq_len=1024)).cuda().eval()
@@ -588,3 +589,9 @@ def test_chain_with_eight_experts_and_with_wide_ones(E, mult, B, T):
 def test_chain_at_other_widths(C, B, T):
     """The tail in clusters of C / 64 CTAs, up to twelve tokens for each of them, and beyond that in kernels of its own."""
     _chain_against_kernels(C, 4, 2, B, T)
+
+
+@pytest.mark.parametrize("B,T,C", [(160, 1, 1024), (100, 1, 1024), (1, 100, 1024), (1, 160, 1024), (1, 20, 128)])
+def test_a_token_whose_router_is_nan_where_the_first_expert_matrix_makes_the_maps(B, T, C):
+    """65 to 160 tokens: its row is stored once and combine, or the tail cluster, takes it twice; and the smallest tail cluster."""
+    test_both_assignments_of_a_token_whose_router_is_nan_run(B, T, C)

@@ -136,6 +136,28 @@ def test_attn_scan_walks_several_sequence_heads(B, H, T):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("B,H,T,cut", [(10, 16, 300, False), (33, 16, 128, False), (12, 16, 700, True), (19, 8, 513, True)])
+def test_prepared_attn_scan_walks_several_sequence_heads(B, H, T, cut):
+    """The same with q and k as the projection's epilogue leaves them (columns interleaved): three chunks and fewer in whole
+    sequence-heads, from four on in shares that are cut, whose state changes hands in that order and is stored in the natural one."""
+    g = torch.Generator(device="cuda").manual_seed(B + T)
+    C = H * 64
+    qkv = torch.randn(B * T, 3 * C, generator=g, device="cuda").bfloat16()
+    gamma = torch.rand(H, generator=g, device="cuda") * 0.2 + 0.799
+    S0 = torch.randn(B, H, 64, 64, generator=g, device="cuda")
+    cos, sin = rope_tabs(T)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148:
+        assert B * H > sms and (B * H % sms != 0 and T > 3 * 128) == cut
+    o, S = ops.attn_scan(qkv[:, :C], qkv[:, C:2 * C], qkv[:, 2 * C:], gamma, cos, sin, B, T, H, state_in=S0, want_state=True, qk_prepared=True)
+    for b in sorted({0, 1, B // 2, B - 2, B - 1}):
+        r = qkv[b * T:(b + 1) * T]
+        o1, S1 = ops.attn_scan(r[:, :C], r[:, C:2 * C], r[:, 2 * C:], gamma, cos, sin, 1, T, H, state_in=S0[b:b + 1].contiguous(),
+                               want_state=True, segmented=False, qk_prepared=True)
+        assert torch.equal(o[b * T:(b + 1) * T], o1) and torch.equal(S[b:b + 1], S1), b
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("B,H", [(3, 2), (40, 4), (301, 16)])
 def test_attn_single_token_steps_with_carried_state(B, H):
     """T = 1 with a carried state and ragged positions: a handful of (sequence, head) pairs take the per-pair
