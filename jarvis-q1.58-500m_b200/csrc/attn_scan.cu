@@ -333,19 +333,6 @@ attn_state_pass_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 // P (bf16 pairs, 64 columns) overlays score columns 64-127: a warp owns its lanes, and walks the 16-key blocks downwards, so
 // what it overwrites it has read.
 // ------------------------------------------------------------------------------------------------------------
-// Per-role cycle counters of one CTA (block 0), compiled in with -DJB_ATTN_TIMING only: every role adds the
-// cycles it spends in each of its waits and work phases; a harness reads g_attn_timing after the launch.
-#ifdef JB_ATTN_TIMING
-__device__ long long g_attn_timing[24 * 8];
-#define JB_T_DECL long long t_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}; long long t_last = clock64();
-#define JB_T_MARK(k) { const long long t_now = clock64(); t_acc[k] += t_now - t_last; t_last = t_now; }
-#define JB_T_FLUSH(w) if (blockIdx.x == 0 && lane == 0) { for (int kk = 0; kk < 8; ++kk) g_attn_timing[(w) * 8 + kk] = t_acc[kk]; }
-#else
-#define JB_T_DECL
-#define JB_T_MARK(k)
-#define JB_T_FLUSH(w)
-#endif
-
 constexpr int PRO_WARP0 = 4, STATE_WARP0 = 12, CON_WARP0 = 16, PIPE_THREADS = 24 * 32;
 constexpr int PRO_WARPS = 8, STATE_WARPS = 4, CON_WARPS = 4;  // consumers: of each group
 // Registers a thread: the CTA is launched with 80 for each of its six groups of four warps; the issuers give up what the
@@ -524,130 +511,108 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // Chunks are counted over all items (g): stages, accumulators and barrier phases follow that count.
   if (warp < PRO_WARP0) {
     regs_dec<ISSUE_REGS>();
-  if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    JB_T_DECL
-    int s = 0, g = 0;
-    uint32_t prev = 1u;                         // parity of the PREVIOUS use of the stage
-    bool ok = true;
-    for (int k = 0; ok && k < share.n_items; ++k) {
-      const Item it = share.at(k);
-      const int b = it.unit / p.H, col = (it.unit - b * p.H) * D;
-      for (int ck = it.begin; ck < it.end; ++ck, ++g) {
-        const int r = b * T + ck * CH;
-        JB_T_MARK(0)
-        if (g >= NST && !mbar_wait(smem_u32(&sm->empty_qk[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
-        JB_T_MARK(1)
+    if (warp == 0) {
+      // ---------------- TMA producer ----------------
+      int s = 0, g = 0;
+      uint32_t prev = 1u;                         // parity of the PREVIOUS use of the stage
+      bool ok = true;
+      for (int k = 0; ok && k < share.n_items; ++k) {
+        const Item it = share.at(k);
+        const int b = it.unit / p.H, col = (it.unit - b * p.H) * D;
+        for (int ck = it.begin; ck < it.end; ++ck, ++g) {
+          const int r = b * T + ck * CH;
+          if (g >= NST && !mbar_wait(smem_u32(&sm->empty_qk[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
+          if (elect_one()) {
+            mbar_arrive_expect_tx(smem_u32(&sm->full_qk[s]), 2 * TILE_BYTES);
+            tma_load_2d(smem_u32(sm->k[s]), &tm_k, col, r, smem_u32(&sm->full_qk[s]));
+            tma_load_2d(smem_u32(sm->q[s]), &tm_q, col, r, smem_u32(&sm->full_qk[s]));
+          }
+          __syncwarp();
+          if (g >= NST && !mbar_wait(smem_u32(&sm->empty_v[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
+          if (elect_one()) {
+            mbar_arrive_expect_tx(smem_u32(&sm->full_v[s]), TILE_BYTES);
+            tma_load_2d(smem_u32(sm->v[s]), &tm_v, col, r, smem_u32(&sm->full_v[s]));
+          }
+          __syncwarp();
+          if (++s == NST) { s = 0; prev ^= 1u; }
+        }
+      }
+    } else if (warp == 1) {
+      // ---------------- MMA issuer: scores, dS, O2 ----------------
+      constexpr uint32_t id_sc = umma_idesc(128, 128, 0, 0), id_o2 = umma_idesc(128, 64, 0, 0), id_ds = umma_idesc(128, 64, 1, 1);
+      // Operand descriptors of stage 0; stage s is +s*TILE_BYTES (+1024 in the address field).  A K-step of 16
+      // elements is +32 bytes (+2) inside a K-major row, +2048 bytes (+128: two 8-row groups) in the MN-major
+      // [token][64] tiles.
+      constexpr uint64_t STG = TILE_BYTES >> 4;
+      const uint64_t d_q0 = umma_desc(smem_u32(sm->q[0]), 16, 1024), d_k0 = umma_desc(smem_u32(sm->k[0]), 16, 1024);
+      const uint64_t d_kw0 = umma_desc(smem_u32(sm->kw[0]), 1024, 1024);
+      const uint64_t d_v0 = umma_desc(smem_u32(sm->v[0]), 0, 1024);       // as the M operand of dS: the 64 dv read twice
+      const uint64_t d_s0 = umma_desc(smem_u32(sm->s[0]), 16, 1024);
+      const int n_tot = share.chunks();
+      int s = 0;                                   // stage of chunk g
+      uint32_t sp = 0u;                            // parity of this use of the stage
+      for (int g = 0; g < n_tot; ++g) {
+        const int buf = g & 1;                     // accumulators and the state copy alternate
+        const uint32_t u = uint32_t(g >> 1) & 1u;
+        const uint64_t dq = d_q0 + uint64_t(s) * STG, dk = d_k0 + uint64_t(s) * STG, dkw = d_kw0 + uint64_t(s) * STG;
+        const uint64_t dv = d_v0 + uint64_t(s) * STG, ds = d_s0 + uint64_t(buf) * (S_BYTES >> 4);
+        if (!mbar_wait(smem_u32(&sm->pro_done[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+        // the output rows of chunk g - 2 have left SC[buf] and O2[buf]
+        if (g >= 2 && !mbar_wait(smem_u32(&sm->o_done[buf]), u ^ 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+        tc_fence_after_sync();
         if (elect_one()) {
-          mbar_arrive_expect_tx(smem_u32(&sm->full_qk[s]), 2 * TILE_BYTES);
-          tma_load_2d(smem_u32(sm->k[s]), &tm_k, col, r, smem_u32(&sm->full_qk[s]));
-          tma_load_2d(smem_u32(sm->q[s]), &tm_q, col, r, smem_u32(&sm->full_qk[s]));
+  #pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16_ss(tm + PT_SC + 128 * buf, dq + uint64_t(ks * 2), dk + uint64_t(ks * 2), id_sc, ks != 0);
+          umma_commit(smem_u32(&sm->bar_sc[buf]));
         }
         __syncwarp();
-        JB_T_MARK(0)
-        if (g >= NST && !mbar_wait(smem_u32(&sm->empty_v[s]), prev, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
-        JB_T_MARK(2)
+        if (!mbar_wait(smem_u32(&sm->full_v[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+        // DS[buf] was read before the state before chunk g - 1 was published, which A2(g - 1) waited for
         if (elect_one()) {
-          mbar_arrive_expect_tx(smem_u32(&sm->full_v[s]), TILE_BYTES);
-          tma_load_2d(smem_u32(sm->v[s]), &tm_v, col, r, smem_u32(&sm->full_v[s]));
+  #pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16_ss(tm + PT_DS + 64 * buf, dv + uint64_t(ks * 128), dkw + uint64_t(ks * 128), id_ds, ks != 0);
+          umma_commit(smem_u32(&sm->bar_s[buf]));
         }
         __syncwarp();
-        if (++s == NST) { s = 0; prev ^= 1u; }
+        if (!mbar_wait(smem_u32(&sm->s_done[buf]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+  #pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16_ss(tm + PT_O2 + 64 * buf, dq + uint64_t(ks * 2), ds + uint64_t(ks * 2), id_o2, ks != 0);
+          umma_commit(smem_u32(&sm->bar_o2[buf]));
+          umma_commit(smem_u32(&sm->empty_qk[s]));       // q, k, kw of this stage, and v but for B(g)
+        }
+        __syncwarp();
+        if (++s == NST) { s = 0; sp ^= 1u; }
+      }
+    } else if (warp == 2) {
+      // ---------------- MMA issuer: O1 = P V into the score columns the mask has read; P is read from TMEM ----------------
+      constexpr uint32_t id_o1 = umma_idesc(128, 64, 0, 1);
+      const uint64_t d_v0 = umma_desc(smem_u32(sm->v[0]), 1024, 1024);    // as the N operand
+      const int n_tot = share.chunks();
+      int s = 0;
+      uint32_t sp = 0u;
+      for (int g = 0; g < n_tot; ++g) {
+        const int buf = g & 1;
+        const uint64_t dv = d_v0 + uint64_t(s) * (TILE_BYTES >> 4);
+        if (!mbar_wait(smem_u32(&sm->full_v[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
+        if (!mbar_wait(smem_u32(&sm->p_done[buf]), uint32_t(g >> 1) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+        if (n_tot == 1 && !mbar_wait(smem_u32(&sm->p_done[1]), 0u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
+        tc_fence_after_sync();
+        const uint32_t tm_p = tm + PT_SC + PT_P + (n_tot == 1 ? 128 : 128 * buf);
+        if (elect_one()) {
+  #pragma unroll
+          for (int ks = 0; ks < 8; ++ks)
+            umma_bf16_ts(tm + PT_SC + 128 * buf, tm_p + ks * 8, dv + uint64_t(ks * 128), id_o1, ks != 0);
+          umma_commit(smem_u32(&sm->bar_b[buf]));
+        }
+        __syncwarp();
+        if (++s == NST) { s = 0; sp ^= 1u; }
       }
     }
-    JB_T_MARK(0)
-    JB_T_FLUSH(0)
-  } else if (warp == 1) {
-    // ---------------- MMA issuer: scores, dS, O2 ----------------
-    constexpr uint32_t id_sc = umma_idesc(128, 128, 0, 0), id_o2 = umma_idesc(128, 64, 0, 0), id_ds = umma_idesc(128, 64, 1, 1);
-    // Operand descriptors of stage 0; stage s is +s*TILE_BYTES (+1024 in the address field).  A K-step of 16
-    // elements is +32 bytes (+2) inside a K-major row, +2048 bytes (+128: two 8-row groups) in the MN-major
-    // [token][64] tiles.
-    constexpr uint64_t STG = TILE_BYTES >> 4;
-    const uint64_t d_q0 = umma_desc(smem_u32(sm->q[0]), 16, 1024), d_k0 = umma_desc(smem_u32(sm->k[0]), 16, 1024);
-    const uint64_t d_kw0 = umma_desc(smem_u32(sm->kw[0]), 1024, 1024);
-    const uint64_t d_v0 = umma_desc(smem_u32(sm->v[0]), 0, 1024);       // as the M operand of dS: the 64 dv read twice
-    const uint64_t d_s0 = umma_desc(smem_u32(sm->s[0]), 16, 1024);
-    const int n_tot = share.chunks();
-    JB_T_DECL
-    int s = 0;                                   // stage of chunk g
-    uint32_t sp = 0u;                            // parity of this use of the stage
-    for (int g = 0; g < n_tot; ++g) {
-      const int buf = g & 1;                     // accumulators and the state copy alternate
-      const uint32_t u = uint32_t(g >> 1) & 1u;
-      const uint64_t dq = d_q0 + uint64_t(s) * STG, dk = d_k0 + uint64_t(s) * STG, dkw = d_kw0 + uint64_t(s) * STG;
-      const uint64_t dv = d_v0 + uint64_t(s) * STG, ds = d_s0 + uint64_t(buf) * (S_BYTES >> 4);
-      JB_T_MARK(0)
-      if (!mbar_wait(smem_u32(&sm->pro_done[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-      JB_T_MARK(1)
-      // the output rows of chunk g - 2 have left SC[buf] and O2[buf]
-      if (g >= 2 && !mbar_wait(smem_u32(&sm->o_done[buf]), u ^ 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-      JB_T_MARK(2)
-      tc_fence_after_sync();
-      if (elect_one()) {
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_bf16_ss(tm + PT_SC + 128 * buf, dq + uint64_t(ks * 2), dk + uint64_t(ks * 2), id_sc, ks != 0);
-        umma_commit(smem_u32(&sm->bar_sc[buf]));
-      }
-      __syncwarp();
-      JB_T_MARK(0)
-      if (!mbar_wait(smem_u32(&sm->full_v[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
-      JB_T_MARK(3)
-      // DS[buf] was read before the state before chunk g - 1 was published, which A2(g - 1) waited for
-      if (elect_one()) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(tm + PT_DS + 64 * buf, dv + uint64_t(ks * 128), dkw + uint64_t(ks * 128), id_ds, ks != 0);
-        umma_commit(smem_u32(&sm->bar_s[buf]));
-      }
-      __syncwarp();
-      JB_T_MARK(0)
-      if (!mbar_wait(smem_u32(&sm->s_done[buf]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-      JB_T_MARK(4)
-      tc_fence_after_sync();
-      if (elect_one()) {
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma_bf16_ss(tm + PT_O2 + 64 * buf, dq + uint64_t(ks * 2), ds + uint64_t(ks * 2), id_o2, ks != 0);
-        umma_commit(smem_u32(&sm->bar_o2[buf]));
-        umma_commit(smem_u32(&sm->empty_qk[s]));       // q, k, kw of this stage, and v but for B(g)
-      }
-      __syncwarp();
-      if (++s == NST) { s = 0; sp ^= 1u; }
-    }
-    JB_T_MARK(0)
-    JB_T_FLUSH(1)
-  } else if (warp == 2) {
-    // ---------------- MMA issuer: O1 = P V into the score columns the mask has read; P is read from TMEM ----------------
-    constexpr uint32_t id_o1 = umma_idesc(128, 64, 0, 1);
-    const uint64_t d_v0 = umma_desc(smem_u32(sm->v[0]), 1024, 1024);    // as the N operand
-    const int n_tot = share.chunks();
-    JB_T_DECL
-    int s = 0;
-    uint32_t sp = 0u;
-    for (int g = 0; g < n_tot; ++g) {
-      const int buf = g & 1;
-      const uint64_t dv = d_v0 + uint64_t(s) * (TILE_BYTES >> 4);
-      JB_T_MARK(0)
-      if (!mbar_wait(smem_u32(&sm->full_v[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
-      if (!mbar_wait(smem_u32(&sm->p_done[buf]), uint32_t(g >> 1) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-      if (n_tot == 1 && !mbar_wait(smem_u32(&sm->p_done[1]), 0u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) break;
-      JB_T_MARK(1)
-      tc_fence_after_sync();
-      const uint32_t tm_p = tm + PT_SC + PT_P + (n_tot == 1 ? 128 : 128 * buf);
-      if (elect_one()) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ts(tm + PT_SC + 128 * buf, tm_p + ks * 8, dv + uint64_t(ks * 128), id_o1, ks != 0);
-        umma_commit(smem_u32(&sm->bar_b[buf]));
-      }
-      __syncwarp();
-      if (++s == NST) { s = 0; sp ^= 1u; }
-    }
-    JB_T_MARK(0)
-    JB_T_FLUSH(2)
-  }
   } else if (warp < STATE_WARP0) {
     regs_inc<PRO_REGS>();
     // ---------------- prologue warps ----------------
@@ -674,7 +639,6 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       load_angles8(p.cos_tab + size_t(stp) * 32 + cg * 8, p.wide_tab, c64);
       load_angles8(p.sin_tab + size_t(stp) * 32 + cg * 8, p.wide_tab, s64);
     }
-    JB_T_DECL
     int s = 0;
     uint32_t sp = 0u;
     bool ok = true;
@@ -682,17 +646,13 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const Item itm = share.at(k);
       const float* pw = sm->tab[k % NTAB].pw;
       if (k == 0 && !PREPARED) load_angles(itm.unit, itm.begin);
-      JB_T_MARK(0)
       if (k > 0 && !mbar_wait(smem_u32(&sm->tab_full[k % NTAB]), uint32_t(k / NTAB) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) break;
-      JB_T_MARK(4)
       for (int ck = itm.begin; ck < itm.end; ++ck) {
         const int c_len = min(CH, T - ck * CH);
         uint8_t* q_p = sm->q[s];
         uint8_t* k_p = sm->k[s];
         uint8_t* kw_p = sm->kw[s];
-        JB_T_MARK(0)
         if (!mbar_wait(smem_u32(&sm->full_qk[s]), sp, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
-        JB_T_MARK(1)
 #pragma unroll 1
         for (int it = 0; it < 2; ++it) {
           const int r = r_lo + 64 * it;
@@ -758,18 +718,14 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             load_angles(nx.unit, nx.begin);
           }
         }
-        JB_T_MARK(2)
         fence_proxy_async_smem();                          // generic-proxy writes -> visible to the tensor core
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm->pro_done[s]));
-        JB_T_MARK(3)
         if (++s == NST) { s = 0; sp ^= 1u; }
       }
     }
-    JB_T_FLUSH(warp)
   } else if (warp < CON_WARP0) {
     // ---------------- state ----------------
-    
     // f32 state: row dv = 32*(qd&1) + lane, columns dk = 32*half .. +31 (the accumulator of MMA S holds the 64 dv rows
     // twice, lanes 0-63 and 64-127, so every warp finds its share in its own lane quarter)
     const int qd = warp & 3, half = qd >> 1, s_row = 32 * (qd & 1) + lane;
@@ -796,7 +752,6 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm->s_done[buf]));
     };
-    JB_T_DECL
     bool ok = true;
     int g = 0;
     for (int k = 0; ok && k < share.n_items; ++k) {
@@ -843,7 +798,6 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           for (int s2 = it.begin / p.seg_chunks; s2 > 0; --s2, dp += D * D) add4(dp, gL, false);
         }
       }
-      JB_T_MARK(0)
       publish_state(g & 1);
       // decay tables, two sequence-heads ahead (the first one's are there)
       for (int n = k == 0 ? 0 : k + 2; n <= k + 2 && n < share.n_items; ++n) {
@@ -852,12 +806,9 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if (lane == 0) mbar_arrive(smem_u32(&sm->tab_full[n % NTAB]));
       }
       if (k > 0 && !mbar_wait(smem_u32(&sm->tab_full[k % NTAB]), uint32_t(k / NTAB) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
-      JB_T_MARK(1)
       for (int ck = it.begin; ck < it.end; ++ck, ++g) {
         const float gc = pw[min(CH, T - ck * CH)];
-        JB_T_MARK(0)
         if (!mbar_wait(smem_u32(&sm->bar_s[g & 1]), uint32_t(g >> 1) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
-        JB_T_MARK(2)
         tc_fence_after_sync();
         __syncwarp();               // tcgen05.ld / st are warp-collective: rejoin after the per-thread wait
         uint32_t r[32];
@@ -866,7 +817,6 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
         for (int e = 0; e < 32; ++e) S[e] = gc * S[e] + __uint_as_float(r[e]);
         if (ck + 1 < it.end) publish_state((g + 1) & 1);
-        JB_T_MARK(3)
       }
       if (!ok) break;
       if (it.piece == 1) {
@@ -890,7 +840,6 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
       }
     }
-    JB_T_FLUSH(warp)
   } else {
     // ---------------- consumers ----------------
     regs_inc<CON_REGS>();
@@ -909,7 +858,6 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       }
       __syncwarp();
     };
-    JB_T_DECL
     if (share.chunks() == 1) {
       // A lone chunk: both groups work on it, the upper and the lower key blocks of a row (P goes to the other accumulator, since
       // what one group writes the other may not have read), then half of the output columns each, stored directly (one
@@ -974,10 +922,8 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if ((g & 1) != grp) continue;
         if (pending >= 0) release(pending);
         // ---- decay mask: scores -> P (lane = query row, column c = keys 2c, 2c+1) ----
-        JB_T_MARK(0)
         if (k > 0 && !mbar_wait(smem_u32(&sm->tab_full[k % NTAB]), uint32_t(k / NTAB) & 1u, abort_flag, p.status, JB200_STATUS_ATTN_LOAD)) { ok = false; break; }
         if (!mbar_wait(smem_u32(&sm->bar_sc[grp]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
-        JB_T_MARK(1)
         tc_fence_after_sync();
         __syncwarp();
         {
@@ -1009,17 +955,13 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           }
           tmem_st_wait();
         }
-        JB_T_MARK(2)
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm->p_done[grp]));
-        JB_T_MARK(3)
         // ---- output rows: o[i] = O1 + gamma^(i+1)/8 * O2 ----
         const float gi = 0.125f * tab.pw[i + 1];
         if (!mbar_wait(smem_u32(&sm->bar_o2[grp]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
-        JB_T_MARK(4)
         if (!mbar_wait(smem_u32(&sm->bar_b[grp]), u, abort_flag, p.status, JB200_STATUS_ATTN_MMA)) { ok = false; break; }
-        JB_T_MARK(5)
         u ^= 1u;
         tc_fence_after_sync();
         __syncwarp();
@@ -1052,12 +994,10 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           bulk_commit_group();
         }
         pending = s;
-        JB_T_MARK(6)
       }
     }
     if (lane == 0) bulk_wait_group<0>();
     __syncwarp();
-    JB_T_FLUSH(warp)
   }
 
   tc_fence_before_sync();
@@ -1421,12 +1361,5 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   JB_LAUNCH_CHECK("attn_scan_pipe_kernel");
   return JB200_OK;
 }
-
-#ifdef JB_ATTN_TIMING
-// Timing builds only: copies the per-role cycle counters of the last pipeline launch to the host.
-extern "C" int jb200_debug_attn_timing(long long* out) {
-  return cudaMemcpyFromSymbol(out, g_attn_timing, sizeof(long long) * 24 * 8) == cudaSuccess ? 0 : 1;
-}
-#endif
 
 }  // namespace jb
