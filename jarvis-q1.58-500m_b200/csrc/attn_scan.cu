@@ -329,7 +329,8 @@ attn_state_pass_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 // CTA walks several sequence-heads without draining (filling and draining took ~12 us each), output rows go by TMA (stored
 // directly they took 512 of 3000 wavefronts of a chunk), angles come 32 bytes a load.  B x T of 16 heads, before -> after: 32 x 2048 158 -> 125 us,
 // 32 x 512 55.5 -> 43, 8 x 2048 43.1 -> 36.6, 32 x 64 24.3 -> 15.5, 1 x 16384 in segments 77 -> 71, 1 x 37 and 1 x 128 5.9 -> 6.2 and
-// 6.4 -> 6.8 (the chain of a lone chunk).
+// 6.4 -> 6.8 (the chain of a lone chunk); up to nine sequences of one or two chunks 0.2 to 0.5 us more, with a carried state 1.1 to 1.7 less
+// (1 x 37 7.9 -> 6.7, 9 x 200 11.0 -> 9.7).
 // P (bf16 pairs, 64 columns) overlays score columns 64-127: a warp owns its lanes, and walks the 16-key blocks downwards, so
 // what it overwrites it has read.
 // ------------------------------------------------------------------------------------------------------------

@@ -60,9 +60,9 @@ constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // finite router logits is stored once, for expert 0, and its second hidden row holds whatever was there: combine and tail
 // take the first one's output for both assignments (stored twice by the GEMM, 64 sequences were 1.5 % slower).  24 layers and head as a graph
 // with the dispatch -> without: 80 tokens 1141 -> 1060 us, 128 1188 -> 1133, 5 x 30 1227 -> 1200, 180 1310 -> 1298, steps of 128 sequences
-// 1360 -> 1326, 192 equal, 256 tokens 1375 -> 1423.  The same line for eight experts and for wide ones, though their MMAs are four times
-// the routed ones (d_model 1024, us a layer, 65, 100 and 160 tokens): 8 x 2048 48.8 -> 44.7, 52.5 -> 48.1, 58.0 -> 55.3; 4 x 4096 51.1 -> 47.9, 53.5 -> 50.4,
-// 61.4 -> 58.5; 8 x 4096 61.2 -> 60.9, 67.1 -> 65.6, 76.8 -> 73.6; steps of 160 sequences 67.2 -> 65.5, 67.3 -> 65.4, 86.5 -> 80.2.
+// 1360 -> 1326, 192 equal, 256 tokens 1375 -> 1423.  The same line for eight experts, though their MMAs are four times the routed ones, and
+// for wide ones (d_model 1024, us a layer, 65, 100 and 160 tokens): 8 x 2048 48.8 -> 44.7, 52.5 -> 48.1, 58.0 -> 55.3; 4 x 4096 51.1 -> 47.9,
+// 53.5 -> 50.4, 61.4 -> 58.5; 8 x 4096 61.2 -> 60.9, 67.1 -> 65.6, 76.8 -> 73.6; steps of 160 sequences 67.2 -> 65.5, 67.3 -> 65.4, 86.5 -> 80.2.
 constexpr int ALL_ROWS_TOKENS = MID_ROUTE_TOKENS, LATE_MAPS_TOKENS = 64;
 // Tiles of the latency form.  Tokens: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
 // tokens) that leaves a launch of so many rows in each group on `room` SMs; where even one tile for all rows does not, that one.  (A

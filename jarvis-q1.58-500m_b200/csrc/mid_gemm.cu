@@ -95,8 +95,8 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)
 // the copied rows), so tiles of 64, on twice as many SMs, take less time each: half the codes to fetch and decode, half the epilogue.
 // ROUTE: 0 rows or segments as given, 1 rows stored in dispatch order and the maps left by a warp of their own, 2 segments counted from
 // the ids, 3 rows stored at the slots of the maps (kernels of their own: the code of the others costs a plain call 1 %).
-// One CTA per SM, since its ring fills the shared memory: routes 1 and 2 kept to registers for two took 0.5 to 1.4 % of a layer more (65 to 160
-// tokens: prompts of 100 40.9 -> 41.2 us, steps of 100 46.8 -> 47.5).
+// One CTA per SM, since its ring fills the shared memory: with routes 1 and 2 kept to the registers of two, 24 layers and head took 967 us where
+// they take 957 at 72 tokens, 1037 and 1032 at 100, as long from 128 on, and steps of 100 and 160 sequences 1144 and 1133, 1349 and 1340.
 template <int BM, int ROUTE>
 __global__ void __launch_bounds__(ROUTE == 1 ? THREADS + 32 : THREADS, 1)
 mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
