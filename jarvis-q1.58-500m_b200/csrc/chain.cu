@@ -52,9 +52,8 @@ struct Workspace {
 
 // Which form of the ternary product a call of so many tokens runs (their results are the same bits): up to 16 tokens
 // mma.sync straight from the codes (24 layers of single-token steps 0.62 against 0.86 ms at 1 sequence, equal at 16), up to
-// MID_TOKENS the tcgen05 form that is built for latency (37 tokens 916 -> 880 us against mma.sync with its token tiles side by side
-// for the attention's products, 64 sequences 1004 -> 957; 640 tokens 1.96 against 2.08 ms with the persistent pipeline, 900 2.20
-// against 2.29, 1000 equal, 1152 2.81 against 2.74), beyond that the persistent pipeline.
+// MID_TOKENS the tcgen05 form that is built for latency, beyond that the persistent pipeline (when the line was drawn: 640 tokens 1.96
+// against 2.08 ms with the pipeline, 900 2.20 against 2.29, 1000 equal, 1152 2.81 against 2.74).
 constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // Up to here the first expert GEMM takes all rows for every expert and stores the routed ones: more MMAs, no dispatch.  A token without
 // finite router logits is stored once, for expert 0, and its second hidden row holds whatever was there: combine and tail
@@ -64,47 +63,52 @@ constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // for wide ones (d_model 1024, us a layer, 65, 100 and 160 tokens): 8 x 2048 48.8 -> 44.7, 52.5 -> 48.1, 58.0 -> 55.3; 4 x 4096 51.1 -> 47.9,
 // 53.5 -> 50.4, 61.4 -> 58.5; 8 x 4096 61.2 -> 60.9, 67.1 -> 65.6, 76.8 -> 73.6; steps of 160 sequences 67.2 -> 65.5, 67.3 -> 65.4, 86.5 -> 80.2.
 constexpr int ALL_ROWS_TOKENS = MID_ROUTE_TOKENS, LATE_MAPS_TOKENS = 64;
-// Tiles of the latency form.  Tokens: the smallest multiple of 16 from 64 on (decoding weights takes as long as the MMAs of 64
-// tokens) that leaves a launch of so many rows in each group on `room` SMs; where even one tile for all rows does not, that one.  (A
-// larger one would be MMAs, copies and shared memory for rows that are not there: 256 rows where the first expert matrix has more than
+// Tiles of the latency form.  Tokens: the smallest multiple of 16 from r.least on that leaves a launch of so many rows in each group on
+// r.most SMs; with tiles of 64 it may take `room` SMs, and from there on the tile grows until it does; where even one tile for all rows
+// does not, that one.  (A larger one would be MMAs, copies and shared memory for rows that are not there: 256 rows where the first expert matrix has more than
 // EXPERT_MOST tiles, us a layer at d_model 1024, 17, 37 and 128 tokens: 8 x 2048 49.4 -> 42.6, 50.5 -> 43.8, 51.4 -> 49.6; 4 x 4096 51.1 -> 44.0,
 // 52.0 -> 45.3, 55.1 -> 53.6; 8 x 4096 74.6 -> 55.4, 74.7 -> 59.5, 70.8 -> 67.7.)
-inline int mid_tile(int rows, int groups, int n_ft, int room) {
-  const int all = rows < 256 ? (rows + 15) / 16 * 16 : 256;
-  int bn = all < 64 ? all : 64;
-  while (bn < all && long(n_ft) * groups * ((rows + bn - 1) / bn) > room) bn += 16;
+struct MidRule {
+  int least, most;
+};
+inline int mid_tile(int rows, int groups, int n_ft, MidRule r, int room) {
+  const int all = rows < 256 ? (rows + 15) / 16 * 16 : 256, usual = all < 64 ? all : 64;
+  auto ctas = [&](int bn) { return long(n_ft) * groups * ((rows + bn - 1) / bn); };
+  for (int bn = r.least; bn < usual; bn += 16)
+    if (ctas(bn) <= r.most) return bn;
+  int bn = usual;
+  while (bn < all && ctas(bn) > room) bn += 16;
   return bn;
 }
-// Out-features: 64 or 128 a tile.  The time of a tile goes with both its sides, but SMs that a launch takes are not there for the
-// next one to begin on (barriers, codes fetched and decoded): 64 where they are at most `most`.  24 layers and head as a graph with 64
-// for one product alone: q|k|v of 64 tokens (48 SMs) 1000 -> 979 us, of 128 sequences (96) 1441 -> 1400, of 256 (144) 1745 -> 1776;
-// out-projection of 64 sequences 1083 -> 1052, of 400 tokens (112 SMs; the router behind it needs little of an SM) 1661 -> 1633, of 700
-// (144) 1885 -> 1919; second expert matrix of 37 tokens (64 SMs) 949 -> 916, of 128 sequences (128) 1441 -> 1451; first
-// expert matrix of 37 tokens (128 SMs) 949 -> 1013.
-constexpr int QKV_MOST = 100, OUT_MOST = 120, EXPERT_MOST = 74;
+// Small tiles shorten chain and epilogue, but SMs that a launch takes are not there for the next one to begin on (barriers, codes
+// fetched and decoded).  24 layers and head as a graph, tiles from 64 on -> these: 37 tokens 821 -> 780 us, 64 864 -> 836, 80 883 -> 850, 128 967 -> 902,
+// 160 1049 -> 997, 256 1193 -> 1179, steps of 64, 128, 192 sequences 899 -> 875, 1166 -> 1120, 1342 -> 1328.  With other lines: q|k|v up to
+// 124 SMs steps of 192 1341; out-projection up to 130 SMs 512 tokens 1522 -> 1551, from 32 tokens on 128 898 -> 927; second expert matrix up to
+// 112 SMs 80 and 160 tokens 850 -> 868 and 997 -> 1016, the first one from 32 on up to 130 SMs 37 tokens 786 -> 816.
+constexpr MidRule QKV_TILES = {16, 74}, OUT_TILES = {16, 100}, W1_TILES = {64, 0}, W2_TILES = {16, 74};
+constexpr int EXPERT_MOST = 74;
 struct MidTile {
-  int bm, bn, bn_max;
+  int bn, bn_max;
 };
-inline MidTile mid_tiles(int rows, int groups, int n_out, int room, int most) {
-  const int b64 = mid_tile(rows, groups, n_out / 64, room), b128 = mid_tile(rows, groups, n_out / 128, room);
-  const bool narrow = long(n_out / 64) * groups * ((rows + b64 - 1) / b64) <= most && 64 + b64 < 128 + b128;
-  return narrow ? MidTile{64, b64, b64} : MidTile{128, b128, b128};
-}
 // Tiles of a launch: every group takes all M rows, or (cut) M rows are cut into segments that are known on the device alone: a
 // tile for rows that are spread evenly, with an eighth to spare, and one for whatever they are (M / bn_max tiles and one cut short in
 // every other group), up to one for all of them.
-inline MidTile mid_plan(int M, int groups, int n_out, bool cut, int most, int sms) {
-  if (!cut) return mid_tiles(M, groups, n_out, groups > 1 ? most : sms, most);
-  const int even = (M + groups - 1) / groups;
-  MidTile t = mid_tiles(even + (even + 7) / 8, groups, n_out, sms, most);
-  while (t.bn_max < 256 && t.bn_max < M && long(n_out / t.bm) * ((M + t.bn_max - 1) / t.bn_max + groups - 1) > sms) t.bn_max += 16;
+inline MidTile mid_plan(int M, int groups, int n_out, bool cut, MidRule r, int sms) {
+  const int n_ft = n_out / MID_FEATURES, even = (M + groups - 1) / groups;
+  if (!cut) {
+    const int bn = mid_tile(M, groups, n_ft, r, groups > 1 ? EXPERT_MOST : sms);
+    return {bn, bn};
+  }
+  MidTile t;
+  t.bn = t.bn_max = mid_tile(even + (even + 7) / 8, groups, n_ft, r, sms);
+  while (t.bn_max < 256 && t.bn_max < M && long(n_ft) * ((M + t.bn_max - 1) / t.bn_max + groups - 1) > sms) t.bn_max += 16;
   return t;
 }
 
 // The first expert matrix takes every token's row, or the assignments in segments; the second one always segments.
 inline MidTile expert_plan(int tokens, bool second, int C, int E, int hidden, int sms) {
   const bool cut = second || tokens > ALL_ROWS_TOKENS;
-  return mid_plan(cut ? 2 * tokens : tokens, E, second ? C : hidden, cut, EXPERT_MOST, sms);
+  return mid_plan(cut ? 2 * tokens : tokens, E, second ? C : hidden, cut, second ? W2_TILES : W1_TILES, sms);
 }
 
 #define JB_TRY(call)                    \
@@ -120,8 +124,8 @@ int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms,
   const MidTile t = expert_plan(tokens, second != 0, C, E, hidden, sms);
   const int K = second ? hidden : C;
   out[0] = !second && tokens <= ALL_ROWS_TOKENS;
-  out[1] = t.bm; out[2] = t.bn; out[3] = t.bn_max;
-  out[4] = mid_gemm_chunks(t.bm, t.bn, K); out[5] = mid_gemm_chunks(t.bm, t.bn_max, K);
+  out[1] = MID_FEATURES; out[2] = t.bn; out[3] = t.bn_max;
+  out[4] = mid_gemm_least_chunks(t.bn, K); out[5] = mid_gemm_least_chunks(t.bn_max, K);
   return 1;
 }
 
@@ -190,9 +194,9 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   if (sms <= 0) return JB200_ERR_CUDA;
   auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
                       const int32_t* seg, const MidRoutes* routes, int epi, void* dst, const MidTile& t) {
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bm, t.bn, t.bn_max, st);
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bn, t.bn_max, st);
   };
-  const MidTile qkv_tile = mid_plan(N, 1, 3 * C, false, QKV_MOST, sms), out_tile = mid_plan(N, 1, C, false, OUT_MOST, sms);
+  const MidTile qkv_tile = mid_plan(N, 1, 3 * C, false, QKV_TILES, sms), out_tile = mid_plan(N, 1, C, false, OUT_TILES, sms);
   const MidTile w1_tile = expert_plan(N, false, C, E, hidden, sms), w2_tile = expert_plan(N, true, C, E, hidden, sms);
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves

@@ -35,8 +35,8 @@ int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepare
 // It keeps whole rows of codes and activations in shared memory: in-features it can take with such tiles (about 7200 with 8
 // rows, 4800 with 16).
 bool small_gemm_fits(int tile, int K);
-// The same product again, latency form on tcgen05 (mid_gemm.cu) with tiles of bm (64 or 128) out-features and bn rows,
-// or of bn_max rows where the segments need more tiles of bn than there are SMs.  Arguments as launch_small_gemm, but for routes
+// The same product again, latency form on tcgen05 (mid_gemm.cu) with tiles of bn rows, or of bn_max rows where the segments
+// need more tiles of bn than there are SMs.  Arguments as launch_small_gemm, but for routes
 // (top-2 assignments).  Every group takes all M rows and the routed ones are stored at their slots: `given` by scatter, or, for at
 // most MID_ROUTE_TOKENS tokens, in dispatch order, and the maps are left in scatter and the others.  With segments (no maps) the M rows
 // are the assignments in that order.
@@ -47,9 +47,10 @@ struct MidRoutes {
   int *counts, *offsets, *scatter, *gather, *gate_idx;
 };
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bm, int bn,
-                    int bn_max, cudaStream_t stream);
-int mid_gemm_chunks(int bm, int bn, int K);   // chunks of its ring with such tiles
+                    const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
+                    cudaStream_t stream);
+constexpr int MID_FEATURES = 128;              // out-features of its tiles
+int mid_gemm_least_chunks(int bn, int K);      // what its ring holds at least with token tiles of bn
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);
 void decode16_prepared_host(uint32_t w_canonical, uint32_t* out8);

@@ -595,3 +595,11 @@ def test_chain_at_other_widths(C, B, T):
 def test_a_token_whose_router_is_nan_where_the_first_expert_matrix_makes_the_maps(B, T, C):
     """65 to 160 tokens: its row is stored once and combine, or the tail cluster, takes it twice; and the smallest tail cluster."""
     test_both_assignments_of_a_token_whose_router_is_nan_run(B, T, C)
+
+
+@pytest.mark.parametrize("C,E,mult,B,T", [(128, 4, 1, 1, 18), (128, 8, 2, 1, 200), (640, 4, 1, 1, 47), (384, 4, 3, 1, 500), (1024, 4, 4, 1, 33),
+                                          (1024, 4, 8, 1, 170), (1024, 8, 4, 1, 900), (896, 4, 5, 2, 480)])
+def test_chain_where_codes_and_weights_outgrow_their_rings(C, E, mult, B, T):
+    """The latency GEMM with one chunk and part of a box of codes (128 in-features), odd numbers of chunks, more boxes than its ring
+    has, and several tiles a CTA, whose chunks begin anywhere in the rings."""
+    _chain_against_kernels(C, E, mult, B, T)
