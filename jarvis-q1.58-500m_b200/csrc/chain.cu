@@ -105,6 +105,12 @@ inline MidTile mid_plan(int M, int groups, int n_out, bool cut, MidRule r, int s
   return t;
 }
 
+// Beyond MID_TOKENS the attention's products stay with the latency form while they are one wave of its largest tiles: a pair's 256 x 256
+// tiles leave half of the SMs idle there, and its first tile is stored 10 us after the dependency.  24 layers and head with pairs ->
+// out-projection in tiles of up to 256 rows: 1000 tokens 2178 -> 2101 us, 1800 2622 -> 2534, 3 x 777 3063 -> 2943, 4000 4140 -> 4047, 4600
+// 4425 -> 4383; q|k|v as well: 1000 2101 -> 2054, 1300 2618 -> 2562, 1536 2553 -> 2526.
+inline bool mid_wave(int N, int n_out, int sms) { return long(n_out / MID_FEATURES) * ((N + 255) / 256) <= sms; }
+
 // The first expert matrix takes every token's row, or the assignments in segments; the second one always segments.
 inline MidTile expert_plan(int tokens, bool second, int C, int E, int hidden, int sms) {
   const bool cut = second || tokens > ALL_ROWS_TOKENS;
@@ -197,6 +203,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bn, t.bn_max, st);
   };
   const MidTile qkv_tile = mid_plan(N, 1, 3 * C, false, QKV_TILES, sms), out_tile = mid_plan(N, 1, C, false, OUT_TILES, sms);
+  const bool mid_qkv = mid || (!small && mid_wave(N, 3 * C, sms)), mid_out = mid || (!small && mid_wave(N, C, sms));
   const MidTile w1_tile = expert_plan(N, false, C, E, hidden, sms), w2_tile = expert_plan(N, true, C, E, hidden, sms);
 
   // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
@@ -231,7 +238,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     // x += attn(norm1(x))
     if (small)
       JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, st));
-    else if (mid)
+    else if (mid_qkv)
       JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile));
     else
       JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st, nullptr, true));
@@ -242,7 +249,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
                             s_in, o, C, s_out, attn_scratch, B, T, H, 64, 0, st, true));
     if (small)
       JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, st));
-    else if (mid)
+    else if (mid_out)
       JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile));
     else
       JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st, nullptr, true));

@@ -603,3 +603,9 @@ def test_chain_where_codes_and_weights_outgrow_their_rings(C, E, mult, B, T):
     """The latency GEMM with one chunk and part of a box of codes (128 in-features), odd numbers of chunks, more boxes than its ring
     has, and several tiles a CTA, whose chunks begin anywhere in the rings."""
     _chain_against_kernels(C, E, mult, B, T)
+
+
+@pytest.mark.parametrize("B,T", [(1, 961), (1, 1536), (1, 1537), (2, 2304), (1, 4609)])
+def test_chain_where_the_attention_products_leave_the_latency_form(B, T):
+    """One wave of tiles of 256 rows: q|k|v up to 1536 tokens, the out-projection up to 4608 (148 SMs)."""
+    _chain_against_kernels(1024, 4, 2, B, T)
