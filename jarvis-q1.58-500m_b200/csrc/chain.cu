@@ -62,7 +62,7 @@ constexpr int SMALL_TOKENS = 16, MID_TOKENS = 960;
 // 1360 -> 1326, 192 equal, 256 tokens 1375 -> 1423.  The same line for eight experts, though their MMAs are four times the routed ones, and
 // for wide ones (d_model 1024, us a layer, 65, 100 and 160 tokens): 8 x 2048 48.8 -> 44.7, 52.5 -> 48.1, 58.0 -> 55.3; 4 x 4096 51.1 -> 47.9,
 // 53.5 -> 50.4, 61.4 -> 58.5; 8 x 4096 61.2 -> 60.9, 67.1 -> 65.6, 76.8 -> 73.6; steps of 160 sequences 67.2 -> 65.5, 67.3 -> 65.4, 86.5 -> 80.2.
-constexpr int ALL_ROWS_TOKENS = MID_ROUTE_TOKENS, LATE_MAPS_TOKENS = 64;
+constexpr int ALL_ROWS_TOKENS = MID_ROUTE_TOKENS;
 // Tiles of the latency form.  Tokens: the smallest multiple of 16 from r.least on that leaves a launch of so many rows in each group on
 // r.most SMs; with tiles of 64 it may take `room` SMs, and from there on the tile grows until it does; where even one tile for all rows
 // does not, that one.  (A larger one would be MMAs, copies and shared memory for rows that are not there: 256 rows where the first expert matrix has more than
@@ -256,11 +256,11 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
 
     // moe(norm2(x)).  late_maps: the first expert GEMM makes the dispatch maps in a warp of its own, beside its MMAs; in the router
     // they are behind a fence, a ticket and a second reading of the ids.  24 layers and head as a graph so 80 tokens 1061 -> 1005 us, 128
-    // 1139 -> 1098, 5 x 30 1199 -> 1157, steps of 100 sequences 1187 -> 1158; 37 tokens 877 -> 888, 64 939 -> 942: the sort is short there,
-    // and the epilogue waits for its slots.
-    const bool late_maps = mid && all_rows && N > LATE_MAPS_TOKENS;
-    const MidRoutes store = {idx, !late_maps, false, counts, offs, scatter, gather, gate_idx};
-    const MidRoutes rows_of = {idx, false, true, nullptr, nullptr, nullptr, nullptr, nullptr};
+    // 1139 -> 1098, 5 x 30 1199 -> 1157, steps of 100 sequences 1187 -> 1158; since its epilogue has its rows before the last MMA also
+    // 17, 37, 64 tokens 766 -> 759, 780 -> 774, 836 -> 816 and steps of 57 840 -> 835.
+    const bool late_maps = mid && all_rows;
+    const MidRoutes store = {idx, false, counts, offs, scatter, gather, gate_idx};
+    const MidRoutes rows_of = {idx, true, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (N <= ROUTE_SMALL_MAX) {
       JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, ticket, counts, offs,
                                 late_maps ? nullptr : scatter, gather, gate_idx, st));

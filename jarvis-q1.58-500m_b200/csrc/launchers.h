@@ -37,13 +37,13 @@ int launch_small_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepare
 bool small_gemm_fits(int tile, int K);
 // The same product again, latency form on tcgen05 (mid_gemm.cu) with tiles of bn rows, or of bn_max rows where the segments
 // need more tiles of bn than there are SMs.  Arguments as launch_small_gemm, but for routes
-// (top-2 assignments).  Every group takes all M rows and the routed ones are stored at their slots: `given` by scatter, or, for at
-// most MID_ROUTE_TOKENS tokens, in dispatch order, and the maps are left in scatter and the others.  With segments (no maps) the M rows
+// (top-2 assignments of at most MID_ROUTE_TOKENS tokens).  Every group takes all M rows, the routed ones are stored in dispatch order, and
+// the maps are left in scatter and the others.  With segments (no maps) the M rows
 // are the assignments in that order.
 constexpr int MID_ROUTE_TOKENS = 160;
 struct MidRoutes {
   const int64_t* ids;          // [tokens][2]
-  bool given, segments;
+  bool segments;
   int *counts, *offsets, *scatter, *gather, *gate_idx;
 };
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,

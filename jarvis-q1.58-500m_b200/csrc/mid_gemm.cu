@@ -108,13 +108,13 @@ __device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)
 __host__ __device__ constexpr int acc_cols(int bn) { return (bn + 63) / 64 * 64; }      // the ring of weights begins there
 
 // ROUTE: 0 rows or segments as given, 1 rows stored in dispatch order and the maps left by a warp of their own, 2 segments counted from
-// the ids, 3 rows stored at the slots of the maps (kernels of their own: the code of the others costs a plain call 1 %).
+// the ids (kernels of their own: the code of the others costs a plain call 1 %).
 template <int ROUTE>
 __global__ void __launch_bounds__(ROUTE == 1 ? THREADS + 32 : THREADS, 1)
 mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Ctl ctl;
-  __shared__ int s_rows[ROUTE == 1 || ROUTE == 3 ? 8 : 1][MID_ROUTE_TOKENS / 2];     // an epilogue warp's output rows
+  __shared__ int s_rows[ROUTE == 1 ? 8 : 1][MID_ROUTE_TOKENS / 2];     // an epilogue warp's output rows
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -390,41 +390,21 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
       }
       // Of 32 tokens, 16 are this warp's (those of its K-block's parity): lane % 16 holds the output row of one of them, -1 for none.
       const int t0 = 16 * par + (lane & 15);
-      if constexpr (ROUTE == 1 || ROUTE == 3) {
+      if constexpr (ROUTE == 1) {
         int* rows = s_rows[warp - DEC_WARP0];
-        if constexpr (ROUTE == 3) {
-          longlong2 e[BLOCKS];
-          int2 sc[BLOCKS];
-#pragma unroll
-          for (int k = 0; k < BLOCKS; ++k) {
-            const int t = it.tok0 + 32 * k + t0;
-            e[k] = make_longlong2(-1, -1);
-            if (32 * k + t0 < n) {
-              e[k] = *reinterpret_cast<const longlong2*>(p.routes.ids + 2 * t);
-              sc[k] = *reinterpret_cast<const int2*>(p.routes.scatter + 2 * t);
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < BLOCKS; ++k) {
-            int row = 32 * k + t0 >= n ? -1 : e[k].x == it.grp ? sc[k].x : e[k].y == it.grp ? sc[k].y : -1;
-            if (row >= 2 * p.M) row = -1;
-            if (lane < 16) rows[16 * k + lane] = row;
-          }
-        } else {
 #pragma unroll 1
-          for (int b = 0; 32 * b < n; ++b) {
-            const int t = it.tok0 + 32 * b + t0;
-            int slot = slot0;
-            bool mine = false;
+        for (int b = 0; 32 * b < n; ++b) {
+          const int t = it.tok0 + 32 * b + t0;
+          int slot = slot0;
+          bool mine = false;
 #pragma unroll
-            for (int k = 0; k < BLOCKS; ++k) {
-              const int d = t - 32 * k;
-              const unsigned before = d <= 0 ? 0u : d >= 32 ? 0xffffffffu : (1u << d) - 1u;
-              slot += __popc(first[k] & before) + __popc(second[k] & before);
-              if (d >= 0 && d < 32) mine = ((first[k] | second[k]) >> d) & 1u;
-            }
-            if (lane < 16) rows[16 * b + lane] = 32 * b + t0 < n && mine && slot < 2 * p.M ? slot : -1;
+          for (int k = 0; k < BLOCKS; ++k) {
+            const int d = t - 32 * k;
+            const unsigned before = d <= 0 ? 0u : d >= 32 ? 0xffffffffu : (1u << d) - 1u;
+            slot += __popc(first[k] & before) + __popc(second[k] & before);
+            if (d >= 0 && d < 32) mine = ((first[k] | second[k]) >> d) & 1u;
           }
+          if (lane < 16) rows[16 * b + lane] = 32 * b + t0 < n && mine && slot < 2 * p.M ? slot : -1;
         }
         __syncwarp();
       }
@@ -444,7 +424,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
         for (int q = 0; q < 4; ++q) {                              // token 8 (q / 2) + 2 (lane % 4) + q % 2 of the 16
           const int t = 8 * (q >> 1) + 2 * (lane & 3) + (q & 1);
           int row = 32 * b + 16 * par + t < n ? it.tok0 + 32 * b + 16 * par + t : -1;
-          if constexpr (ROUTE == 1 || ROUTE == 3) row = s_rows[warp - DEC_WARP0][16 * b + t];
+          if constexpr (ROUTE == 1) row = s_rows[warp - DEC_WARP0][16 * b + t];
           const int k = 4 * (q >> 1) + (q & 1);
           uint64_t y0 = mul_f32x2(f32x2(__uint_as_float(v[0][k]), __uint_as_float(v[0][k + 2])), f32x2(alpha, alpha));
           uint64_t y1 = mul_f32x2(f32x2(__uint_as_float(v[1][k]), __uint_as_float(v[1][k + 2])), f32x2(alpha, alpha));
@@ -512,8 +492,8 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   MidParams p;
   p.alpha = alpha; p.seg = seg; p.routes = routes ? *routes : MidRoutes{}; p.out = out;
   p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / BM; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
-  const bool cut = seg || p.routes.segments, given = routes && routes->given;
-  JB_REQUIRE(!routes || given || (!seg && (G == 4 || G == 8) && M <= (cut ? 2 : 1) * MID_ROUTE_TOKENS && (p.routes.scatter == nullptr) == cut),
+  const bool cut = seg || p.routes.segments;
+  JB_REQUIRE(!routes || (!seg && (G == 4 || G == 8) && M <= (cut ? 2 : 1) * MID_ROUTE_TOKENS && (p.routes.scatter == nullptr) == cut),
              "mid_gemm: %d rows by %d groups cannot be routed here", M, G);
   p.boxes = code_boxes(K);
   p.status = device_status_ptr();
@@ -541,17 +521,16 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   if (sms <= 0) return JB200_ERR_CUDA;
   const long tiles = cut ? (M + bn - 1) / bn + G - 1 : long(G) * ((M + bn - 1) / bn), items = tiles * p.n_ft;   // at most
   const dim3 grid(unsigned(items < sms ? items : sms));
-  const int route = !routes ? 0 : given ? 3 : cut ? 2 : 1;
+  const int route = !routes ? 0 : cut ? 2 : 1;
   auto launch = [&](auto kernel, std::atomic<unsigned long long>* set_up) {
     const int rc = set_max_smem(reinterpret_cast<const void*>(kernel), RING_SMEM + 1024, set_up);
     if (rc == JB200_OK) launch_dep(kernel, grid, route == 1 ? THREADS + 32 : THREADS, smem, stream, maps, p);
     return rc;
   };
-  static std::atomic<unsigned long long> set_up[4];
+  static std::atomic<unsigned long long> set_up[3];
   const int rc = route == 0   ? launch(mid_gemm_kernel<0>, set_up)
                  : route == 1 ? launch(mid_gemm_kernel<1>, set_up + 1)
-                 : route == 2 ? launch(mid_gemm_kernel<2>, set_up + 2)
-                              : launch(mid_gemm_kernel<3>, set_up + 3);
+                              : launch(mid_gemm_kernel<2>, set_up + 2);
   if (rc != JB200_OK) return rc;
   JB_LAUNCH_CHECK("mid_gemm_kernel");
   return JB200_OK;
