@@ -6,6 +6,13 @@ namespace jb {
 
 #if defined(__CUDACC__)
 
+// x / n to the last bit, given n's reciprocal rounded to nearest: one correction of the quotient by its remainder (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).
+__device__ __forceinline__ double div_by(double x, double n, double inv) {
+  const double q = x * inv;
+  return fabs(q) < __longlong_as_double(0x7ff0000000000000ll) ? fma(fma(-q, n, x), inv, q) : q;
+}
+
 // torch.var (unbiased) of the layer output from its sum and sum of squares; a single element gives NaN as torch does.
 __device__ __forceinline__ float moe_act_mean(const double* stats, long long n_elems) {
   return float(stats[0] / double(n_elems));
@@ -14,6 +21,12 @@ __device__ __forceinline__ float moe_act_var(const double* stats, long long n_el
   const double mean = stats[0] / double(n_elems);
   const double var = (stats[1] - stats[0] * mean) / double(n_elems - 1);
   return n_elems > 1 ? float(var > 0.0 ? var : 0.0) : __int_as_float(0x7fc00000);
+}
+
+// The same two with n's and (n - 1)'s reciprocals at hand, n > 1 (a division is 0.2 us where every nanosecond is waited for).
+__device__ __forceinline__ float2 moe_act_mean_var(double s1, double s2, double n, double inv_n, double inv_n1) {
+  const double mean = div_by(s1, n, inv_n), var = div_by(s2 - s1 * mean, n - 1.0, inv_n1);
+  return make_float2(float(mean), float(var > 0.0 ? var : 0.0));
 }
 
 // scalars[0] = l_balance, [1] = act_mean, [2] = act_var, all f32; one thread.

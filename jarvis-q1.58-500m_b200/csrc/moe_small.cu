@@ -132,7 +132,7 @@ struct TailParams {
   const int* scatter;          // [N][2]
   const int64_t* idx;          // [N][2]
   LsfStats st;                 // stats is not read: the sums are made here
-  double inv_tokens;
+  double inv_tokens, n_elems, inv_n, inv_n1;
   const float* var_scale;
   float alpha_min, alpha_max;
   const float* h_in;           // [B][C] or null
@@ -185,11 +185,12 @@ __device__ __forceinline__ float tail_decay(const TailParams& p, Combined c, flo
   __syncthreads();
   if (warp == 0) {
     double a = lane < n_warps ? part[lane][0] : 0.0, b = lane < n_warps ? part[lane][1] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = n_warps > 8 ? 8 : n_warps > 4 ? 4 : n_warps > 2 ? 2 : n_warps >> 1; o > 0; o >>= 1) {        // lanes from n_warps on are zeros
       a += __shfl_xor_sync(0xffffffffu, a, o);
       b += __shfl_xor_sync(0xffffffffu, b, o);
     }
+    a = __shfl_sync(0xffffffffu, a, 0);
+    b = __shfl_sync(0xffffffffu, b, 0);
     if (n_cta > 1) {
       if (lane < 2 * n_cta)
         cluster_st_f64(cluster_map(smem_u32(&all[rank][lane & 1]), uint32_t(lane >> 1)), (lane & 1) ? b : a);
@@ -208,18 +209,17 @@ __device__ __forceinline__ float tail_decay(const TailParams& p, Combined c, flo
     double s[2];
     s[0] = lane < n_cta ? all[lane][0] : 0.0;
     s[1] = lane < n_cta ? all[lane][1] : 0.0;
-#pragma unroll
-    for (int o = MAX_CTAS / 2; o > 0; o >>= 1) {
+    for (int o = n_cta > 8 ? 8 : 4; o > 0; o >>= 1) {
       s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
       s[1] += __shfl_xor_sync(0xffffffffu, s[1], o);
     }
     if (lane == 0) {
-      const float mean = moe_act_mean(s, p.st.n_elems), var = moe_act_var(s, p.st.n_elems);
-      *s_alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, var);
+      const float2 mv = moe_act_mean_var(s[0], s[1], p.n_elems, p.inv_n, p.inv_n1);
+      *s_alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, mv.y);
       if (rank == 0) {
-        p.st.scalars[1] = mean;
-        p.st.scalars[2] = var;
-        if (p.st.reflect) *p.st.reflect = reflect_penalty(p.st.lam, p.st.tau, __ldg(p.st.mu), mean, var);
+        p.st.scalars[1] = mv.x;
+        p.st.scalars[2] = mv.y;
+        if (p.st.reflect) *p.st.reflect = reflect_penalty(p.st.lam, p.st.tau, __ldg(p.st.mu), mv.x, mv.y);
       }
     }
   }
@@ -300,12 +300,13 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailPar
 
 // Several tokens per sequence.  Rows are combined and normalised by the CTA that owns the token (token n: CTA n % n_cta, a
 // warp each), the scan runs where all tokens of a channel are (CTA k: channels [64 k, 64 k + 64)); the rows change
-// hands through distributed shared memory.  ms [N][64] bf16: combined rows of the CTA's channels; hs [B][64]: their membranes; xr
-// [N / n_cta][C] f32: updated residual rows of the CTA's tokens; ends [B * runs][64]: what a run of tokens leaves from a zero carry.
-// Bound by latency: copies, three exchanges and one chain over a run.  Sixteen CTAs of 64 channels move half the rows per SM that eight
-// of 128 did, a run's end is worked out once, by its own warp, and residual rows are fetched while the kernel ahead runs (with eight, carries
-// recomputed by every later run and rows fetched behind the exchange 24 layers and head took 1034, 1067, 1370 us at 37, 64, 128 tokens;
-// so 963, 973, 1199).
+// hands through distributed shared memory.  ms [N][64] bf16: combined rows of the CTA's channels; xs [N][64] f32: their residual rows,
+// copied while the kernel ahead runs; hs [B][64]: their membranes; xr [N / n_cta][C] f32: updated residual rows of the CTA's tokens; ends
+// [B * runs][64]: what a run of tokens leaves from a zero carry.
+// Bound by latency: copies, three exchanges and one chain over a run; a run is worked on by up to four warps, each going along the
+// chain but storing four tokens of sixteen.  A launch fetches
+// its code anew (34 KB; unrolled over a run, with one for either kind of sequence, 63): the scan took 2.8 us of the 7.2 at 37 tokens, the f64
+// divisions 1.0.  24 layers and head 17, 37, 64, 128, 160 tokens 761 -> 713, 775 -> 746, 814 -> 784, 902 -> 891, 1006 -> 996 us.
 constexpr int SCAN_CH = 64, RUN = 16;          // channels per CTA, two per lane; tokens per run (lsf_tma_kernel's warp runs)
 
 __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailParams p, const int n_cta) {
@@ -318,8 +319,10 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   // runs of 16 tokens from a zero carry, the carries along the runs, then every token's value, with the roundings of
   // lsf_tma_kernel (T > 8) or lsf_short_kernel
   const int n_runs = T > 8 ? (T + RUN - 1) / RUN : 1, run_len = T > 8 ? RUN : T, items = B * n_runs;
+  const int split = T <= 8 ? 1 : 4 * items <= n_warps ? 4 : 2 * items <= n_warps ? 2 : 1;        // warps of a run
   uint8_t* ms = tail_smem;                                                     // [N][128 bytes]
-  float* hs = reinterpret_cast<float*>(tail_smem + size_t(N) * SCAN_CH * 2);   // h_out may be h_in
+  float* xs = reinterpret_cast<float*>(tail_smem + size_t(N) * SCAN_CH * 2);
+  float* hs = xs + size_t(N) * SCAN_CH;                                        // h_out may be h_in
   float* xr = hs + size_t(B) * SCAN_CH;
   float* ends = xr + size_t((N + n_cta - 1) / n_cta) * C;
   const int own = rank + warp * n_cta;                                         // this warp's token
@@ -333,15 +336,8 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
     g = *reinterpret_cast<const float2*>(p.gates + 2 * own);
   }
   const size_t ch = size_t(rank) * SCAN_CH + lane * 2;
-  float2 xv[RUN];                // the run's residual values, all in flight together
-  auto load_x = [&](int b, int run) {
-#pragma unroll
-    for (int j = 0; j < RUN; ++j) {
-      const int t = run * RUN + j;
-      if (j < run_len && t < T) xv[j] = *reinterpret_cast<const float2*>(p.x + size_t(b * T + t) * C + ch);
-    }
-  };
-  if (warp < items) load_x(warp / n_runs, warp % n_runs);
+  for (int i = tid; i < N * (SCAN_CH / 4); i += blockDim.x)
+    copy_async_16(smem_u32(xs) + uint32_t(i) * 16u, p.x + size_t(i / (SCAN_CH / 4)) * C + rank * SCAN_CH + i % (SCAN_CH / 4) * 4);
   for (int i = tid; i < B * SCAN_CH / 4; i += blockDim.x) {
     const int b = i / (SCAN_CH / 4), q = i % (SCAN_CH / 4);
     reinterpret_cast<float4*>(hs)[i] =
@@ -369,61 +365,74 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   if (rank == 0 && tid == int(blockDim.x) - 1) p.st.scalars[0] = l_bal;
 
   const float one_m = 1.0f - alpha;
-  float pw[RUN];
-  {
-    float a = alpha;
+  float whole = alpha;                                       // alpha to the power of a run's length
 #pragma unroll
-    for (int i = 0; i < RUN; ++i) { pw[i] = a; a *= alpha; }
-  }
+  for (int i = 1; i < RUN; ++i) whole *= alpha;
   auto m_at = [&](int n) { return *reinterpret_cast<const uint32_t*>(ms + size_t(n) * (SCAN_CH * 2) + lane * 4); };
+  auto along = [&](float2& v, uint32_t m) {                  // one token further
+    v.x = __fmaf_rn(alpha, v.x, __fmul_rn(one_m, bf16_lo(m)));
+    v.y = __fmaf_rn(alpha, v.y, __fmul_rn(one_m, bf16_hi(m)));
+  };
   if (n_runs > 1) {
 #pragma unroll 1
     for (int w = warp; w < items; w += n_warps) {
       const int b = w / n_runs, run = w - b * n_runs;
       if (run == n_runs - 1) continue;                       // nobody's carry
       float2 e = make_float2(0.f, 0.f);
+      uint32_t m[RUN];
 #pragma unroll
-      for (int j = 0; j < RUN; ++j) {
-        const uint32_t v = m_at(b * T + run * RUN + j);
-        e.x = __fmaf_rn(alpha, e.x, __fmul_rn(one_m, bf16_lo(v)));
-        e.y = __fmaf_rn(alpha, e.y, __fmul_rn(one_m, bf16_hi(v)));
-      }
+      for (int j = 0; j < RUN; ++j) m[j] = m_at(b * T + run * RUN + j);
+#pragma unroll
+      for (int j = 0; j < RUN; ++j) along(e, m[j]);
       *reinterpret_cast<float2*>(ends + w * SCAN_CH + lane * 2) = e;
     }
-    __syncthreads();
   }
+  copy_async_wait();
+  __syncthreads();
 #pragma unroll 1
-  for (int w = warp; w < items; w += n_warps) {              // (sequence, run)
-    const int b = w / n_runs, run = w - b * n_runs;
-    if (w != warp) load_x(b, run);
+  for (int w = warp; w < items * split; w += n_warps) {      // (sequence, run, part of it)
+    const int item = w / split, part = w - item * split, b = item / n_runs, run = item - b * n_runs;
+    if (part * (RUN / split) >= T - run * RUN) continue;
     float2 h = *reinterpret_cast<const float2*>(hs + b * SCAN_CH + lane * 2);
     for (int q = 0; q < run; ++q) {                          // the carry into this run
       const float2 e = *reinterpret_cast<const float2*>(ends + (b * n_runs + q) * SCAN_CH + lane * 2);
-      h.x = __fmaf_rn(pw[RUN - 1], h.x, e.x);
-      h.y = __fmaf_rn(pw[RUN - 1], h.y, e.y);
+      h.x = __fmaf_rn(whole, h.x, e.x);
+      h.y = __fmaf_rn(whole, h.y, e.y);
     }
-    float2 loc = make_float2(0.f, 0.f);
-    float2 hv = h;
+    const int left = T - run * RUN, first = b * T + run * RUN, last = min(min(run_len, left), (part + 1) * (RUN / split));
+    float2 loc = make_float2(0.f, 0.f), hv = h;
+    float pw = alpha;                                        // alpha to the power of the tokens since the carry
+#pragma unroll 1
+    for (int j0 = 0; j0 < last; j0 += 4) {
+      uint32_t m[4];
+      float2 x[4];
 #pragma unroll
-    for (int j = 0; j < RUN; ++j) {
-      const int t = run * RUN + j;
-      if (j < run_len && t < T) {
-        const int n = b * T + t;
-        const uint32_t v = m_at(n);
+      for (int k = 0; k < 4; ++k) {
+        const int n = min(first + j0 + k, N - 1);
+        m[k] = m_at(n);
+        x[k] = *reinterpret_cast<const float2*>(xs + size_t(n) * SCAN_CH + lane * 2);
+      }
+      const bool mine = j0 >= part * (RUN / split);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
         if (T > 8) {
-          loc.x = __fmaf_rn(alpha, loc.x, __fmul_rn(one_m, bf16_lo(v)));
-          loc.y = __fmaf_rn(alpha, loc.y, __fmul_rn(one_m, bf16_hi(v)));
-          hv.x = __fmaf_rn(pw[j], h.x, loc.x);
-          hv.y = __fmaf_rn(pw[j], h.y, loc.y);
+          along(loc, m[k]);
+          hv.x = __fmaf_rn(pw, h.x, loc.x);
+          hv.y = __fmaf_rn(pw, h.y, loc.y);
+          pw *= alpha;
         } else {
-          hv.x = lsf_step(alpha, hv.x, bf16_lo(v));
-          hv.y = lsf_step(alpha, hv.y, bf16_hi(v));
+          const float2 was = hv;
+          hv.x = lsf_step(alpha, was.x, bf16_lo(m[k]));
+          hv.y = lsf_step(alpha, was.y, bf16_hi(m[k]));
         }
-        xv[j].x = xv[j].x + hv.x;
-        xv[j].y = xv[j].y + hv.y;
-        *reinterpret_cast<float2*>(p.x + size_t(n) * C + ch) = xv[j];
-        cluster_st_64(cluster_map(smem_u32(xr) + (uint32_t(n / n_cta) * uint32_t(C) + uint32_t(ch)) * 4u, uint32_t(n % n_cta)), xv[j]);
-        if (t == T - 1) *reinterpret_cast<float2*>(p.h_out + size_t(b) * C + ch) = hv;
+        if (mine && j0 + k < last) {
+          const int n = first + j0 + k;
+          x[k].x = x[k].x + hv.x;
+          x[k].y = x[k].y + hv.y;
+          *reinterpret_cast<float2*>(p.x + size_t(n) * C + ch) = x[k];
+          cluster_st_64(cluster_map(smem_u32(xr) + (uint32_t(n / n_cta) * uint32_t(C) + uint32_t(ch)) * 4u, uint32_t(n % n_cta)), x[k]);
+          if (run * RUN + j0 + k == T - 1) *reinterpret_cast<float2*>(p.h_out + size_t(b) * C + ch) = hv;
+        }
       }
     }
   }
@@ -464,9 +473,9 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   }
 }
 
-// [N][64] bf16, [B][64] f32, [rows][C] f32, [items][64] f32; B and items are at most N / 2 and N / 16 + B.
+// [N][64] bf16 and f32, [B][64] f32, [rows][C] f32, [items][64] f32; B and items are at most N / 2 and N / 16 + B.
 inline size_t tail_smem_bytes(int N, int B, int rows, int C, int items) {
-  return size_t(N) * SCAN_CH * 2 + (size_t(B) * SCAN_CH + size_t(rows) * C + size_t(items) * SCAN_CH) * sizeof(float);
+  return size_t(N) * SCAN_CH * 6 + (size_t(B) * SCAN_CH + size_t(rows) * C + size_t(items) * SCAN_CH) * sizeof(float);
 }
 constexpr size_t TAIL_SMEM = 200 * 1024;
 
@@ -487,7 +496,8 @@ bool tail_fits(int n_cta) {
     cfg.gridDim = n_cta; cfg.blockDim = 32 * MAX_WARPS; cfg.dynamicSmemBytes = TAIL_SMEM; cfg.attrs = at; cfg.numAttrs = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = unsigned(n_cta); at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    const bool ok = cudaFuncSetAttribute(scan, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+    const bool ok = cudaFuncSetAttribute(reinterpret_cast<const void*>(tail_step_kernel), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaFuncSetAttribute(scan, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                     cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TAIL_SMEM)) == cudaSuccess &&
                     cudaOccupancyMaxActiveClusters(&n, tail_scan_kernel, &cfg) == cudaSuccess && n >= 1;
     if (!ok) (void)cudaGetLastError();
@@ -580,13 +590,15 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
   TailParams p;
   p.y = reinterpret_cast<const __nv_bfloat16*>(y_bf16); p.gates = gates; p.scatter = scatter; p.idx = idx; p.st = st;
   p.inv_tokens = 1.0 / double(st.n_tokens);
+  p.n_elems = double(st.n_elems); p.inv_n = 1.0 / p.n_elems; p.inv_n1 = 1.0 / (p.n_elems - 1.0);
   p.var_scale = var_scale; p.alpha_min = alpha_min; p.alpha_max = alpha_max;
   p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;
   p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
   p.B = B; p.T = T; p.N = N; p.C = C;
   if (T == 1) {
-    // a lone CTA while its SM can take the rows (4 KB in, 10 KB out each), else eight
-    const int n_cta = N <= 4 ? 1 : 8;
+    // a lone CTA while its SM can take the rows (4 KB in, 10 KB out each), else sixteen (steps of 64 and 128 sequences, 24 layers
+    // and head, in eight 876 and 1127 us, so 848 and 1065), or eight where a cluster cannot have more
+    const int n_cta = N <= 4 ? 1 : tail_fits(MAX_CTAS) ? MAX_CTAS : 8;
     const int warps = (N + n_cta - 1) / n_cta;
     if (n_cta == 1) launch_dep(tail_step_kernel, 1, 32 * warps, 0, stream, p, 1);
     else launch_dep_cluster(tail_step_kernel, n_cta, 32 * warps, 0, n_cta, stream, p, n_cta);
@@ -594,7 +606,7 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
     return JB200_OK;
   }
   const int n_cta = C / SCAN_CH, rows = (N + n_cta - 1) / n_cta;
-  const int items = B * (T > 8 ? (T + RUN - 1) / RUN : 1), warps = std::max(rows, std::min(items, MAX_WARPS));
+  const int items = B * (T > 8 ? (T + RUN - 1) / RUN : 1), warps = std::max(rows, std::min(T > 8 ? 4 * items : items, MAX_WARPS));
   const size_t smem = tail_smem_bytes(N, B, rows, C, items);
   JB_MAX_SMEM(tail_scan_kernel, TAIL_SMEM);
   launch_dep_cluster(tail_scan_kernel, n_cta, 32 * warps, smem, n_cta, stream, p, n_cta);
@@ -603,8 +615,8 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
 }
 
 int tail_max_tokens(int C, int T) {
-  // steps: sixteen CTAs for 129 to 256 of them lose against combine and lsf_step_norm (150 1431 -> 1479 us a step, 256 1747 -> 1843);
-  // prompts against combine, scan and norm: 129 tokens 1291 -> 1244 us, 180 1337 -> 1307, 4 x 60 1323 -> 1340, 256 1381 -> 1402
+  // steps: 129 to 256 of them, nine to sixteen a CTA, lose against combine and lsf_step_norm (140 1095 -> 1109 us a step, 192 1334 -> 1376,
+  // 256 1527 -> 1605); prompts against combine, scan and norm beyond 192 tokens (200 1158 -> 1139, 4 x 60 1118 -> 1136, 256 1186 -> 1203)
   if (T == 1) return 8 * MAX_WARPS;
   return tail_fits(C / SCAN_CH) ? 12 * (C / SCAN_CH) : 0;
 }

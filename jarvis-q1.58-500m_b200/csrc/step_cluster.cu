@@ -149,13 +149,6 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volati
   return phase_done(bar, parity) || wait_long(bar, parity, abort_flag, status);
 }
 
-// x / n to the last bit, given n's reciprocal rounded to nearest: one correction of the quotient by its remainder (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).
-__device__ __forceinline__ double div_by(double x, double n, double inv) {
-  const double q = x * inv;
-  return fabs(q) < __longlong_as_double(0x7ff0000000000000ll) ? fma(fma(-q, n, x), inv, q) : q;
-}
-
 // 16 out-features x 8 tokens x 1024 in-features: `a` is this lane's place in a weight unit, xa its ldmatrix row.  Activations are
 // fetched a double step ahead, weights eight steps: 26 cycles a step with four warps on the SM, 38, 53, 68 with 8, 12, 16 (the MMAs
 // alone 23, 25, 29, 39; the rest is the codes' shifts and masks).  Called in one place: see Step.
