@@ -135,7 +135,7 @@ int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms,
   return 1;
 }
 
-size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(E + 1) * 4 + 7) / 8 * 8; }
+size_t accumulator_bytes(int E) { return (size_t(2 + E) * 8 + size_t(2 * E + 1) * 4 + 7) / 8 * 8; }
 
 size_t routing_layout(int N, int E, size_t* offsets) {
   const Routing r(N > 0 ? N : 0, E > 0 ? E : 0);
@@ -199,8 +199,8 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
   auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
-                      const int32_t* seg, const MidRoutes* routes, int epi, void* dst, const MidTile& t) {
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, routes, epi, dst, t.bn, t.bn_max, st);
+                      const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epi, void* dst, const MidTile& t) {
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, counts, routes, epi, dst, t.bn, t.bn_max, st);
   };
   const MidTile qkv_tile = mid_plan(N, 1, 3 * C, false, QKV_TILES, sms), out_tile = mid_plan(N, 1, C, false, OUT_TILES, sms);
   const bool mid_qkv = mid || (!small && mid_wave(N, 3 * C, sms)), mid_out = mid || (!small && mid_wave(N, C, sms));
@@ -226,7 +226,8 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const bool h16 = aligned16(h_in) && aligned16(h_out);      // the fused tails read 16 bytes at a time, the scan 8
     double* acc = reinterpret_cast<double*>(acc0 + l * acc_stride);            // sum, sum of squares, P_e
     int32_t* hist = reinterpret_cast<int32_t*>(acc + 2 + E);                   // top-1 counts
-    int32_t* ticket = hist + E;
+    int32_t* load = hist + E;                                                  // assignments
+    int32_t* ticket = load + E;
     float* scalars = f->scalars + size_t(l) * 3;
     uint8_t* r = static_cast<uint8_t*>(f->routing) + size_t(l) * rl.bytes;
     int64_t* idx = reinterpret_cast<int64_t*>(r + rl.idx);
@@ -239,7 +240,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, st));
     else if (mid_qkv)
-      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile));
+      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile));
     else
       JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st, nullptr, true));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
@@ -250,7 +251,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, st));
     else if (mid_out)
-      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile));
+      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile));
     else
       JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st, nullptr, true));
 
@@ -261,30 +262,32 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const bool late_maps = mid && all_rows;
     const MidRoutes store = {idx, false, counts, offs, scatter, gather, gate_idx};
     const MidRoutes rows_of = {idx, true, nullptr, nullptr, nullptr, nullptr, nullptr};
+    const bool from_ids = !all_rows && N <= DISPATCH_IDS_MAX;       // maps and rows in one launch
     if (N <= ROUTE_SMALL_MAX) {
-      JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, ticket, counts, offs,
-                                late_maps ? nullptr : scatter, gather, gate_idx, st));
+      JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, from_ids ? load : nullptr, ticket,
+                                counts, offs, all_rows && !late_maps ? scatter : nullptr, gather, gate_idx, st));
     } else {
-      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true));
-      JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
+      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true, from_ids ? load : nullptr));
+      if (!from_ids) JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
     }
     if (all_rows) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
       if (small)
         JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, small_tile, st));
       else
-        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, &store, JB200_EPI_GELU_BF16, hid, w1_tile));
+        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, nullptr, &store, JB200_EPI_GELU_BF16, hid, w1_tile));
     } else {
-      JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
+      if (from_ids) JB_TRY(launch_dispatch_ids(idx, xn, N, C, E, counts, offs, scatter, gather, gate_idx, disp, st));
+      else JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
-        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, nullptr, JB200_EPI_GELU_BF16, hid, w1_tile));
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, nullptr, load, nullptr, JB200_EPI_GELU_BF16, hid, w1_tile));
       else
-        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true));
+        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true, from_ids ? load : nullptr));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, late_maps ? nullptr : offs, late_maps ? &rows_of : nullptr, JB200_EPI_BF16, y, w2_tile));
+      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, late_maps ? nullptr : offs, nullptr, late_maps ? &rows_of : nullptr, JB200_EPI_BF16, y, w2_tile));
     else
       JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st, nullptr, true));
 

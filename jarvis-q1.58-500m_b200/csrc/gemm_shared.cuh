@@ -108,6 +108,7 @@ struct GemmParams {
   const uint8_t* w_packed;   // [G][N][K/4]
   const float* alpha;        // [G][N / alpha_rows]
   const int32_t* seg_offsets;  // device [G+1] or nullptr (single segment [0, M))
+  const int32_t* seg_counts;   // settled: device [G], the segments' lengths, where the kernel ahead makes seg_offsets; or nullptr
   void* out;                 // bf16 [M][N] or f32 [M][N]
   int M, N, K, G;
   int alpha_rows;            // out-feature rows sharing one alpha (N for per-tensor)

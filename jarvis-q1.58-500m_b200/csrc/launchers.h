@@ -24,7 +24,8 @@ struct GemmRope {
 };
 int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packed, const float* alpha,
                         int alpha_rows, int N, int G, const int32_t* seg_offsets, int epilogue, void* out,
-                        int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope = nullptr, bool settled = false);
+                        int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope = nullptr, bool settled = false,
+                        const int32_t* seg_counts = nullptr);
 // The same product for a few tokens (small_gemm.cu), bit for bit; bf16, GELU and residual epilogues.  idx / scatter ([M][2]):
 // all M rows go through every group's matrix and row n is stored at scatter[2n + k] where idx[2n + k] is the group; else seg
 // as above.  tile: rows a CTA takes at a time, 8 or 16.  Within a chain only: weights
@@ -47,7 +48,7 @@ struct MidRoutes {
   int *counts, *offsets, *scatter, *gather, *gate_idx;
 };
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
+                    const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
                     cudaStream_t stream);
 constexpr int MID_FEATURES = 128;              // out-features of its tiles
 int mid_gemm_least_chunks(int bn, int K);      // what its ring holds at least with token tiles of bn
@@ -66,12 +67,16 @@ int launch_router_top2(const void* x_bf16, const float* w_router, int n_tokens, 
                        float* gates, float* probs_out, double* probs_sum, int* top1_hist, cudaStream_t stream);
 int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router,
                           int n_tokens, int C, int E, int64_t* topk_idx, float* gates, double* probs_sum,
-                          int* top1_hist, cudaStream_t stream, bool ahead = false);
+                          int* top1_hist, cudaStream_t stream, bool ahead = false, int* load = nullptr);
 size_t moe_metadata_scratch_bytes(int n_tokens, int K, int E);
 // Maps and rows of top-2 assignments at once.  scratch: moe_dispatch_scratch_bytes.
 size_t moe_dispatch_scratch_bytes(int n_tokens, int E);
 int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, void* scratch, int* expert_counts,
                         int* expert_offsets, int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream);
+// The same in one launch, inside a chain, without counts made before: up to where sixteen tokens a CTA are one wave.
+constexpr int DISPATCH_IDS_MAX = 2368;
+int launch_dispatch_ids(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int* expert_counts, int* expert_offsets,
+                        int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream);
 int launch_moe_metadata(const int64_t* topk_idx, int n_tokens, int K, int E, int* expert_counts, int* expert_offsets,
                         int* scatter_map, int* gather_map, int* gate_idx_map, void* scratch, cudaStream_t stream);
 int moe_metadata_static_max_assignments();
@@ -118,13 +123,13 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
 size_t attn_scan_scratch_bytes(int B, int T, int H);
 
 // Few tokens (moe_small.cu).
-constexpr int ROUTE_SMALL_MAX = 256;   // tokens
+constexpr int ROUTE_SMALL_MAX = 512, ROUTE_SORT_MAX = 16;   // tokens; tokens with maps
 int tail_max_tokens(int C, int T);     // most tokens that launch_tail takes: 128 of single-token steps, 12 for every 64 channels of prompts
 int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const float* w_norm, float eps, float* x, void* xn_bf16,
                       int n_rows, int C, void* zero, size_t zero_bytes, cudaStream_t stream);
-// scatter null: the assignments alone, no maps.
+// scatter null: the assignments alone, no maps.  load: how many of them every expert has, or null.
 int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router, int N, int C, int E,
-                       int64_t* idx, float* gates, double* probs_sum, int* hist, int* ticket, int* counts, int* offsets,
+                       int64_t* idx, float* gates, double* probs_sum, int* hist, int* load, int* ticket, int* counts, int* offsets,
                        int* scatter, int* gather, int* gate_idx, cudaStream_t stream);
 int launch_tail(const void* y_bf16, const float* gates, const int* scatter, const int64_t* idx, const LsfStats& st,
                 const float* var_scale, float alpha_min, float alpha_max, const float* h_in, float* h_out, float* x,

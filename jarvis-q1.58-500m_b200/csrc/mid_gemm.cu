@@ -42,7 +42,8 @@ constexpr uint32_t TMEM_COLS = 512, KB_COLS = BK / 2;                       // a
 
 struct MidParams {
   const float* alpha;          // [G][N / alpha_rows]
-  const int32_t* seg;          // device [G+1] or null (every group takes rows [0, M), or the segments are counted from routes)
+  const int32_t* seg;          // device [G+1] or null (every group takes rows [0, M), or the segments are given by counts or routes)
+  const int32_t* counts;       // device [G] or null: their lengths, where the kernel ahead makes the offsets
   MidRoutes routes;
   void* out;
   int M, N, K, G, n_ft, alpha_rows, epilogue;
@@ -149,23 +150,29 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
       beg = p.seg ? min(max(__ldg(p.seg + lane), 0), p.M) : 0;
       end = p.seg ? min(max(__ldg(p.seg + lane + 1), 0), p.M) : p.M;
     }
-    if constexpr (ROUTE == 2) {                // the kernel ahead makes the offsets; the ids are older
-      constexpr int ROUNDS = 2 * MID_ROUTE_TOKENS / 32;
-      int ex[ROUNDS], n_of = 0;
+    if (ROUTE == 2 || p.counts) {              // the kernel ahead makes the offsets; ids and counts are older
+      int n_of = 0;
+      if constexpr (ROUTE == 2) {
+        constexpr int ROUNDS = 2 * MID_ROUTE_TOKENS / 32;
+        int ex[ROUNDS];
 #pragma unroll
-      for (int i = 0; i < ROUNDS; ++i) ex[i] = i * 32 + lane < p.M ? max(int(p.routes.ids[i * 32 + lane]), 0) : -1;
-      for (int q = 0; q < p.G; ++q) {
-        int n = 0;
+        for (int i = 0; i < ROUNDS; ++i) ex[i] = i * 32 + lane < p.M ? max(int(p.routes.ids[i * 32 + lane]), 0) : -1;
+        for (int q = 0; q < p.G; ++q) {
+          int n = 0;
 #pragma unroll
-        for (int i = 0; i < ROUNDS; ++i) n += __popc(__ballot_sync(0xffffffffu, ex[i] == q));
-        if (lane == q) n_of = n;
+          for (int i = 0; i < ROUNDS; ++i) n += __popc(__ballot_sync(0xffffffffu, ex[i] == q));
+          if (lane == q) n_of = n;
+        }
+      } else if (lane < p.G) {
+        n_of = max(__ldg(p.counts + lane), 0);
       }
       end = n_of;
       for (int d = 1; d < MAX_GROUPS; d *= 2) {
         const int u = __shfl_up_sync(0xffffffffu, end, d);
         if (lane >= d) end += u;
       }
-      beg = end - n_of;
+      beg = min(end - n_of, p.M);
+      end = min(end, p.M);
     }
     auto tiles_of = [&](int bn) {              // token tiles of groups 0..lane
       int t = end > beg ? (end - beg + bn - 1) / bn : 0;
@@ -482,7 +489,7 @@ int mid_gemm_least_chunks(int bn, int K) {
 }
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
-                    const int32_t* seg, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
+                    const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
                     cudaStream_t stream) {
   JB_REQUIRE(epilogue == JB200_EPI_BF16 || epilogue == JB200_EPI_GELU_BF16 || epilogue == JB200_EPI_RESID_F32, "mid_gemm: epilogue %d", epilogue);
   JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn % 16 == 0 &&
@@ -490,9 +497,9 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
                  G >= 1 && G <= MAX_GROUPS,
              "mid_gemm: bad shape (M=%d, N=%d, K=%d, bn=%d)", M, N, K, bn);
   MidParams p;
-  p.alpha = alpha; p.seg = seg; p.routes = routes ? *routes : MidRoutes{}; p.out = out;
+  p.alpha = alpha; p.seg = seg; p.counts = counts; p.routes = routes ? *routes : MidRoutes{}; p.out = out;
   p.M = M; p.N = N; p.K = K; p.G = G; p.n_ft = N / BM; p.alpha_rows = alpha_rows; p.epilogue = epilogue;
-  const bool cut = seg || p.routes.segments;
+  const bool cut = seg || counts || p.routes.segments;
   JB_REQUIRE(!routes || (!seg && (G == 4 || G == 8) && M <= (cut ? 2 : 1) * MID_ROUTE_TOKENS && (p.routes.scatter == nullptr) == cut),
              "mid_gemm: %d rows by %d groups cannot be routed here", M, G);
   p.boxes = code_boxes(K);

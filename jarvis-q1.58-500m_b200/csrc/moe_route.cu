@@ -85,20 +85,20 @@ router_top2_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
 // is rounded to bf16 and stored for the expert GEMMs, and the SAME rounded values feed the router
 // logits in the same summation order as router_top2_kernel, so routing is bit-identical to running
 // the two kernels separately while the row is read from HBM once.
-template <int E>
+template <int E, int PER>
 __global__ void __launch_bounds__(ROUTER_THREADS, 2)
 rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_norm, float eps,
                       __nv_bfloat16* __restrict__ xn, const float* __restrict__ w_router, int n_tokens, int C,
                       int64_t* __restrict__ topk_idx, float* __restrict__ gates,
-                      double* __restrict__ probs_sum, int* __restrict__ top1_hist, bool ahead) {
+                      double* __restrict__ probs_sum, int* __restrict__ top1_hist, int* __restrict__ load, bool ahead) {
   extern __shared__ float w_s[];  // [E][C]
   __shared__ float p_acc[ROUTER_THREADS / 32][E];
-  __shared__ int h_acc[E];
+  __shared__ int h_acc[E], l_acc[E];
   auto stage = [&] {
     for (int i = threadIdx.x; i < E * C; i += ROUTER_THREADS) w_s[(i / C) * C + router_w_index(i % C)] = __ldg(w_router + i);
     touch_floats(w_norm, C);
   };
-  if (threadIdx.x < E) h_acc[threadIdx.x] = 0;
+  if (threadIdx.x < E) h_acc[threadIdx.x] = l_acc[threadIdx.x] = 0;
   if (ahead) stage();
   pdl_wait();
   pdl_trigger();
@@ -108,70 +108,72 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
   float p_local[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) p_local[e] = 0.f;
-  // A warp takes TWO tokens per pass: their loads are in flight together, the two dependency chains interleave,
+  // A warp takes PER tokens per pass: with two, their loads are in flight together, the two dependency chains interleave,
   // and the router weights read from shared memory serve both.  The CTAs are persistent (two per SM) and stride
-  // over the token pairs, so the router matrix is staged once per CTA.
-  const int n_pairs = (n_tokens + 1) >> 1;
-  for (int pair = blockIdx.x * (ROUTER_THREADS / 32) + warp; pair < n_pairs; pair += gridDim.x * (ROUTER_THREADS / 32)) {
-    const int tok = 2 * pair;
-    const bool two = tok + 1 < n_tokens;
-    const float* xr0 = x + size_t(tok) * C;
-    const float* xr1 = x + size_t(two ? tok + 1 : tok) * C;     // a lone last token is processed twice, stored once
-    float v[2][4][8];
-    float ss0 = 0.f, ss1 = 0.f;
+  // over the tokens, so the router matrix is staged once per CTA.  Where one token a warp is a single pass, it is over sooner (24
+  // layers and head, 600, 900, 1300 tokens 1667 -> 1637, 1848 -> 1803, 2511 -> 2480 us).
+  const int n_items = (n_tokens + PER - 1) / PER;
+  for (int item = blockIdx.x * (ROUTER_THREADS / 32) + warp; item < n_items; item += gridDim.x * (ROUTER_THREADS / 32)) {
+    const int tok = PER * item;
+    float v[PER][4][8], ss[PER], r[PER], acc[PER][E];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = (i * 32 + lane) * 8;
-      if (c < C) {
-        const float4 a0 = __ldg(reinterpret_cast<const float4*>(xr0 + c)), b0 = __ldg(reinterpret_cast<const float4*>(xr0 + c) + 1);
-        const float4 a1 = __ldg(reinterpret_cast<const float4*>(xr1 + c)), b1 = __ldg(reinterpret_cast<const float4*>(xr1 + c) + 1);
-        v[0][i][0] = a0.x; v[0][i][1] = a0.y; v[0][i][2] = a0.z; v[0][i][3] = a0.w;
-        v[0][i][4] = b0.x; v[0][i][5] = b0.y; v[0][i][6] = b0.z; v[0][i][7] = b0.w;
-        v[1][i][0] = a1.x; v[1][i][1] = a1.y; v[1][i][2] = a1.z; v[1][i][3] = a1.w;
-        v[1][i][4] = b1.x; v[1][i][5] = b1.y; v[1][i][6] = b1.z; v[1][i][7] = b1.w;
+    for (int k = 0; k < PER; ++k) {
+      const float* xr = x + size_t(min(tok + k, n_tokens - 1)) * C;     // a lone last token is processed twice, stored once
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = (i * 32 + lane) * 8;
+        if (c < C) {
+          const float4 a = __ldg(reinterpret_cast<const float4*>(xr + c)), b = __ldg(reinterpret_cast<const float4*>(xr + c) + 1);
+          v[k][i][0] = a.x; v[k][i][1] = a.y; v[k][i][2] = a.z; v[k][i][3] = a.w;
+          v[k][i][4] = b.x; v[k][i][5] = b.y; v[k][i][6] = b.z; v[k][i][7] = b.w;
+        }
       }
     }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) ss[k] = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if ((i * 32 + lane) * 8 < C) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { ss0 = __fmaf_rn(v[0][i][j], v[0][i][j], ss0); ss1 = __fmaf_rn(v[1][i][j], v[1][i][j], ss1); }
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int k = 0; k < PER; ++k) ss[k] = __fmaf_rn(v[k][i][j], v[k][i][j], ss[k]);
       }
     }
-    ss0 = warp_sum(ss0);
-    ss1 = warp_sum(ss1);
-    const float r0 = rsqrtf(ss0 / float(C) + eps), r1 = rsqrtf(ss1 / float(C) + eps);
-    float acc0[E], acc1[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) { acc0[e] = 0.f; acc1[e] = 0.f; }
+    for (int k = 0; k < PER; ++k) {
+      ss[k] = warp_sum(ss[k]);
+      r[k] = rsqrtf(ss[k] / float(C) + eps);
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[k][e] = 0.f;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int c = (i * 32 + lane) * 8;
       if (c < C) {
         const float4 wa = __ldg(reinterpret_cast<const float4*>(w_norm + c));
         const float4 wb = __ldg(reinterpret_cast<const float4*>(w_norm + c) + 1);
-        const uint4 pk0 = make_uint4(pack_bf16x2(v[0][i][0] * r0 * wa.x, v[0][i][1] * r0 * wa.y),
-                                     pack_bf16x2(v[0][i][2] * r0 * wa.z, v[0][i][3] * r0 * wa.w),
-                                     pack_bf16x2(v[0][i][4] * r0 * wb.x, v[0][i][5] * r0 * wb.y),
-                                     pack_bf16x2(v[0][i][6] * r0 * wb.z, v[0][i][7] * r0 * wb.w));
-        const uint4 pk1 = make_uint4(pack_bf16x2(v[1][i][0] * r1 * wa.x, v[1][i][1] * r1 * wa.y),
-                                     pack_bf16x2(v[1][i][2] * r1 * wa.z, v[1][i][3] * r1 * wa.w),
-                                     pack_bf16x2(v[1][i][4] * r1 * wb.x, v[1][i][5] * r1 * wb.y),
-                                     pack_bf16x2(v[1][i][6] * r1 * wb.z, v[1][i][7] * r1 * wb.w));
-        *reinterpret_cast<uint4*>(xn + size_t(tok) * C + c) = pk0;
-        if (two) *reinterpret_cast<uint4*>(xn + size_t(tok + 1) * C + c) = pk1;
-        const float xv0[8] = {bf16_lo(pk0.x), bf16_hi(pk0.x), bf16_lo(pk0.y), bf16_hi(pk0.y),
-                              bf16_lo(pk0.z), bf16_hi(pk0.z), bf16_lo(pk0.w), bf16_hi(pk0.w)};
-        const float xv1[8] = {bf16_lo(pk1.x), bf16_hi(pk1.x), bf16_lo(pk1.y), bf16_hi(pk1.y),
-                              bf16_lo(pk1.z), bf16_hi(pk1.z), bf16_lo(pk1.w), bf16_hi(pk1.w)};
-        router_dot8<E>(xv0, w_s, C, c, acc0);     // the same shared-memory words: the compiler loads them once
-        router_dot8<E>(xv1, w_s, C, c, acc1);
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const uint4 pk = make_uint4(pack_bf16x2(v[k][i][0] * r[k] * wa.x, v[k][i][1] * r[k] * wa.y),
+                                      pack_bf16x2(v[k][i][2] * r[k] * wa.z, v[k][i][3] * r[k] * wa.w),
+                                      pack_bf16x2(v[k][i][4] * r[k] * wb.x, v[k][i][5] * r[k] * wb.y),
+                                      pack_bf16x2(v[k][i][6] * r[k] * wb.z, v[k][i][7] * r[k] * wb.w));
+          if (k == 0 || tok + k < n_tokens) *reinterpret_cast<uint4*>(xn + size_t(tok + k) * C + c) = pk;
+          const float xv[8] = {bf16_lo(pk.x), bf16_hi(pk.x), bf16_lo(pk.y), bf16_hi(pk.y),
+                               bf16_lo(pk.z), bf16_hi(pk.z), bf16_lo(pk.w), bf16_hi(pk.w)};
+          router_dot8<E>(xv, w_s, C, c, acc[k]);     // the same shared-memory words for every token: the compiler loads them once
+        }
       }
     }
 #pragma unroll
-    for (int e = 0; e < E; ++e) { acc0[e] = warp_sum(acc0[e]); acc1[e] = warp_sum(acc1[e]); }
-    router_finish<E>(acc0, lane, tok, topk_idx, gates, nullptr, h_acc, p_local);
-    if (two) router_finish<E>(acc1, lane, tok + 1, topk_idx, gates, nullptr, h_acc, p_local);
+    for (int k = 0; k < PER; ++k) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[k][e] = warp_sum(acc[k][e]);
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+      if (k == 0 || tok + k < n_tokens) router_finish<E>(acc[k], lane, tok + k, topk_idx, gates, nullptr, h_acc, p_local, load ? l_acc : nullptr);
   }
   if (lane == 0) {
 #pragma unroll
@@ -183,6 +185,7 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
     for (int w = 0; w < ROUTER_THREADS / 32; ++w) s += p_acc[w][threadIdx.x];
     if (probs_sum) atomicAdd(&probs_sum[threadIdx.x], double(s));
     if (top1_hist && h_acc[threadIdx.x]) atomicAdd(&top1_hist[threadIdx.x], h_acc[threadIdx.x]);
+    if (load && l_acc[threadIdx.x]) atomicAdd(&load[threadIdx.x], l_acc[threadIdx.x]);
   }
 }
 
@@ -362,15 +365,18 @@ dispatch_hist_kernel(const int64_t* __restrict__ topk_idx, int M, int* __restric
 // One CTA per chunk of 32 tokens, or of 64 where that leaves few counts and CTAs enough.  Every CTA adds up the counts of all
 // chunks (E integers each, from L2), ranks its assignments with ballots - the order of the kernels above - and copies its rows:
 // each is read once and stored at both of its slots, where the gather reads every row twice.  For an MoE layer called by itself;
-// sizes and times at one_launch_dispatch.  Inside the native call the separate kernels stay: there the products read the
-// segments while the kernel ahead of them still runs, which this one makes; with the segments left by the router instead,
-// 300 tokens 1564 -> 1690 us and 8 x 2048 12.9 -> 13.3 ms.
-template <int E, int TOK>
+// sizes and times at one_launch_dispatch.
+// IDS, inside the native call: the counts are taken from the ids themselves, by every CTA, and the first expert matrix reads the segments
+// off the router's counts while this kernel runs.  Latency: ids and rows travel together, then one exchange over the CTA.  24 layers and
+// head against metadata (256 tokens: by the router's last warp, 3.6 of its 7 us) and gather: 180 tokens 1104 -> 1064 us, 256 1180 -> 1130,
+// 512 1525 -> 1506, 1300 2563 -> 2512, 3 x 777 2929 -> 2907, steps of 256 sequences 1528 -> 1484; every CTA reads all ids: 3000
+// 3442 -> 3448, 4096 4042 -> 4197, so the line is where CTAs of sixteen tokens are one wave.
+template <int E, int TOK, bool IDS>
 __global__ void __launch_bounds__(DISP_THREADS)
 dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __restrict__ x, const int* __restrict__ chunk_counts,
                 int n_tokens, int C, int* __restrict__ expert_counts, int* __restrict__ expert_offsets, int* __restrict__ scatter_map,
                 int* __restrict__ gather_map, int* __restrict__ gate_idx_map, __nv_bfloat16* __restrict__ dispatched) {
-  constexpr int WARPS = DISP_THREADS / 32, RANK_WARPS = 2 * TOK / 32, PER_WARP = TOK / WARPS;
+  constexpr int WARPS = DISP_THREADS / 32, RANK_WARPS = (2 * TOK + 31) / 32, PER_WARP = TOK / WARPS, ROWS = PER_WARP < 2 ? 1 : 2;
   __shared__ int red[WARPS][2 * E], in_warp[RANK_WARPS][E], slots[2 * TOK];
   pdl_wait();
   pdl_trigger();
@@ -378,10 +384,10 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
   const int tok0 = int(blockIdx.x) * TOK, M = 2 * n_tokens, m = 2 * tok0 + tid;
   // the warp's first two rows and its assignments travel while the counts are added up
   const int first = tok0 + warp * PER_WARP;
-  uint4 row[2][4];
+  uint4 row[ROWS][4];
   auto load_rows = [&](int t) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < ROWS; ++k)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int c = (i * 32 + lane) * 8;
@@ -393,15 +399,31 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
   int total[E], before[E];
 #pragma unroll
   for (int q = 0; q < E; ++q) total[q] = before[q] = 0;
-  for (int c = tid; c < int(gridDim.x); c += DISP_THREADS) {
+  if constexpr (IDS) {
+    unsigned long long all = 0, ahead = 0;               // a byte per expert: at most 2 * DISPATCH_IDS_MAX / DISP_THREADS
+#pragma unroll 4
+    for (int t = tid; t < n_tokens; t += DISP_THREADS) {
+      const longlong2 id = __ldcg(reinterpret_cast<const longlong2*>(topk_idx) + t);
+      const unsigned long long two = (1ull << (8 * clamp_expert(id.x, E))) + (1ull << (8 * clamp_expert(id.y, E)));
+      all += two;
+      ahead += t < tok0 ? two : 0ull;
+    }
 #pragma unroll
-    for (int q4 = 0; q4 < E / 4; ++q4) {
-      const int4 v = __ldcg(reinterpret_cast<const int4*>(chunk_counts + size_t(c) * E) + q4);
-      const int w[4] = {v.x, v.y, v.z, v.w};
+    for (int q = 0; q < E; ++q) {
+      total[q] = int(all >> (8 * q)) & 0xff;
+      before[q] = int(ahead >> (8 * q)) & 0xff;
+    }
+  } else {
+    for (int c = tid; c < int(gridDim.x); c += DISP_THREADS) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        total[4 * q4 + q] += w[q];
-        before[4 * q4 + q] += c < int(blockIdx.x) ? w[q] : 0;
+      for (int q4 = 0; q4 < E / 4; ++q4) {
+        const int4 v = __ldcg(reinterpret_cast<const int4*>(chunk_counts + size_t(c) * E) + q4);
+        const int w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          total[4 * q4 + q] += w[q];
+          before[4 * q4 + q] += c < int(blockIdx.x) ? w[q] : 0;
+        }
       }
     }
   }
@@ -442,9 +464,9 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
     if (tid < E) expert_counts[tid] = own;
   }
   __syncthreads();
-  for (int t = 0; t < PER_WARP; t += 2) {
+  for (int t = 0; t < PER_WARP; t += ROWS) {
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < ROWS; ++k) {
       if (first + t + k >= n_tokens) continue;
       const int at = 2 * (warp * PER_WARP + t + k);
 #pragma unroll
@@ -457,7 +479,7 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
         }
       }
     }
-    if (t + 2 < PER_WARP) load_rows(t + 2);
+    if (t + ROWS < PER_WARP) load_rows(t + ROWS);
   }
 }
 
@@ -647,7 +669,7 @@ int launch_router_top2(const void* x_bf16, const float* w_router, int n_tokens, 
 
 int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router,
                           int n_tokens, int C, int E, int64_t* topk_idx, float* gates, double* probs_sum,
-                          int* top1_hist, cudaStream_t stream, bool ahead) {
+                          int* top1_hist, cudaStream_t stream, bool ahead, int* load) {
   JB_REQUIRE(n_tokens >= 0 && C > 0, "rmsnorm_router: bad shape");
   JB_REQUIRE(E == 4 || E == 8, "rmsnorm_router: num_experts (%d) must be 4 or 8", E);
   JB_REQUIRE(C % 8 == 0 && C <= 1024, "rmsnorm_router: d_model (%d) must be a multiple of 8 and at most 1024", C);
@@ -656,19 +678,17 @@ int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* 
   JB_REQUIRE(aligned16(x) && aligned16(w_norm) && aligned16(xn_bf16) && aligned16(w_router),
              "rmsnorm_router: pointers must be 16-byte aligned");
   if (n_tokens == 0) return JB200_OK;
-  // persistent CTAs, two per SM, striding over the token pairs (one pair per warp and pass)
+  // persistent CTAs, two per SM, striding over the tokens: two per warp and pass, or one where that leaves a single pass
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
-  const int pair_blocks = ((n_tokens + 1) / 2 + ROUTER_THREADS / 32 - 1) / (ROUTER_THREADS / 32);
-  const int blocks = pair_blocks < 2 * sms ? pair_blocks : 2 * sms;
+  const int warps = ROUTER_THREADS / 32, per = n_tokens <= 2 * sms * warps ? 1 : 2;
+  const int blocks = std::min((n_tokens + per * warps - 1) / (per * warps), 2 * sms);
   const size_t smem = size_t(E) * C * sizeof(float);
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
-  if (E == 4)
-    launch_dep(rmsnorm_router_kernel<4>, blocks, ROUTER_THREADS, smem, stream, x, w_norm, eps, xn, w_router, n_tokens, C,
-               topk_idx, gates, probs_sum, top1_hist, ahead);
-  else
-    launch_dep(rmsnorm_router_kernel<8>, blocks, ROUTER_THREADS, smem, stream, x, w_norm, eps, xn, w_router, n_tokens, C,
-               topk_idx, gates, probs_sum, top1_hist, ahead);
+  auto kernel = per == 1 ? (E == 4 ? rmsnorm_router_kernel<4, 1> : rmsnorm_router_kernel<8, 1>)
+                         : (E == 4 ? rmsnorm_router_kernel<4, 2> : rmsnorm_router_kernel<8, 2>);
+  launch_dep(kernel, blocks, ROUTER_THREADS, smem, stream, x, w_norm, eps, xn, w_router, n_tokens, C, topk_idx, gates, probs_sum, top1_hist,
+             load, ahead);
   JB_LAUNCH_CHECK("rmsnorm_router_kernel");
   return JB200_OK;
 }
@@ -716,10 +736,29 @@ int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_token
                         : (E == 4 ? dispatch_hist_kernel<4, 64> : dispatch_hist_kernel<8, 64>);
   launch_dep(hist, blocks, 2 * tok, 0, stream, topk_idx, 2 * n_tokens, chunk_counts);
   JB_LAUNCH_CHECK("dispatch_hist_kernel");
-  auto kernel = tok == 32 ? (E == 4 ? dispatch_kernel<4, 32> : dispatch_kernel<8, 32>)
-                          : (E == 4 ? dispatch_kernel<4, 64> : dispatch_kernel<8, 64>);
+  auto kernel = tok == 32 ? (E == 4 ? dispatch_kernel<4, 32, false> : dispatch_kernel<8, 32, false>)
+                          : (E == 4 ? dispatch_kernel<4, 64, false> : dispatch_kernel<8, 64, false>);
   launch_dep(kernel, blocks, DISP_THREADS, 0, stream, topk_idx, x, chunk_counts, n_tokens, C, expert_counts, expert_offsets, scatter_map,
              gather_map, gate_idx_map, d);
+  JB_LAUNCH_CHECK("dispatch_kernel");
+  return JB200_OK;
+}
+
+int launch_dispatch_ids(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int* expert_counts, int* expert_offsets,
+                        int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream) {
+  JB_REQUIRE(n_tokens >= 1 && n_tokens <= DISPATCH_IDS_MAX && (E == 4 || E == 8) && C >= 8 && C % 8 == 0 && C <= 1024,
+             "dispatch_ids: bad shape (N=%d, C=%d, E=%d)", n_tokens, C, E);
+  JB_REQUIRE(topk_idx && x_bf16 && expert_counts && expert_offsets && scatter_map && gather_map && gate_idx_map && dispatched,
+             "dispatch_ids: null pointer");
+  JB_REQUIRE(aligned16(topk_idx) && aligned16(x_bf16) && aligned16(dispatched), "dispatch_ids: pointers must be 16-byte aligned");
+  static_assert(DISPATCH_IDS_MAX / DISP_THREADS * 2 < 256, "a byte per expert and thread");
+  const int tok = n_tokens <= 8 * 148 ? 8 : n_tokens <= 16 * 148 ? 16 : 32;        // a wave of CTAs, as small as they go
+  auto kernel = tok == 8    ? (E == 4 ? dispatch_kernel<4, 8, true> : dispatch_kernel<8, 8, true>)
+                : tok == 16 ? (E == 4 ? dispatch_kernel<4, 16, true> : dispatch_kernel<8, 16, true>)
+                            : (E == 4 ? dispatch_kernel<4, 32, true> : dispatch_kernel<8, 32, true>);
+  launch_dep(kernel, (n_tokens + tok - 1) / tok, DISP_THREADS, 0, stream, topk_idx, reinterpret_cast<const __nv_bfloat16*>(x_bf16),
+             static_cast<const int*>(nullptr), n_tokens, C, expert_counts, expert_offsets, scatter_map, gather_map, gate_idx_map,
+             reinterpret_cast<__nv_bfloat16*>(dispatched));
   JB_LAUNCH_CHECK("dispatch_kernel");
   return JB200_OK;
 }

@@ -13,7 +13,8 @@ __device__ __forceinline__ int clamp_expert(long long e, int E) { return e < 0 ?
 // to the lower expert id, gates, and the per-warp accumulators of P and the top-1 histogram.
 template <int E>
 __device__ __forceinline__ void router_finish(const float (&acc)[E], int lane, int tok, int64_t* topk_idx,
-                                              float* gates, float* probs_out, int* h_acc, float (&p_local)[E]) {
+                                              float* gates, float* probs_out, int* h_acc, float (&p_local)[E],
+                                              int* load_acc = nullptr) {
   float mx = acc[0];
 #pragma unroll
   for (int e = 1; e < E; ++e) mx = fmaxf(mx, acc[e]);
@@ -40,6 +41,10 @@ __device__ __forceinline__ void router_finish(const float (&acc)[E], int lane, i
       for (int e = 0; e < E; ++e) probs_out[size_t(tok) * E + e] = p[e];
     }
     atomicAdd(&h_acc[i0], 1);
+    if (load_acc) {                // assignments, first and second ones, as clamp_expert sorts them
+      atomicAdd(&load_acc[i0], 1);
+      atomicAdd(&load_acc[i1 < 0 ? 0 : i1], 1);
+    }
 #pragma unroll
     for (int e = 0; e < E; ++e) p_local[e] += p[e];
   }

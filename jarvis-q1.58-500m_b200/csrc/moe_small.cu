@@ -1,8 +1,8 @@
 // The glue of a block for few tokens (decode steps of small batches, short prompts), where every launch is latency: two
 // kernels in the place of five.
 //
-//   route_small_kernel  norm2 + top-2 router (jarvis_model.py:25-26, :218-224), a warp per token; the warp that finishes
-//                       last also makes the dispatch maps (sparse_model.cu:23-90)
+//   route_small_kernel  norm2 + top-2 router (jarvis_model.py:25-26, :218-224), a warp per token; up to sixteen tokens
+//                       the warp that finishes last also makes the dispatch maps (sparse_model.cu:23-90)
 //   tail_step_kernel, tail_scan_kernel  combine of the expert rows, MoE statistics, LSF scan, residual add and the RMSNorm
 //                       that follows (sparse_model.cu:117-165, jarvis_model.py:244-250, :281-314, :430-436) in one
 //                       thread-block cluster: the decay of the scan depends on the variance of ALL combined rows, and
@@ -32,6 +32,7 @@ struct RouteParams {
   float* gates;                // [N][2]
   double* probs_sum;           // [E] accumulated
   int* hist;                   // [E] accumulated
+  int* load;                   // [E] accumulated: assignments, first and second ones; null: not wanted
   int* ticket;                 // zero on entry
   int *counts, *offsets, *scatter, *gather, *gate_idx;   // scatter null: no maps
   float eps;
@@ -40,10 +41,10 @@ struct RouteParams {
 
 // One warp per token and CTA: with all weights of the lane's channels in registers before the residual row arrives, the
 // chain is load - sum - norm - dot - sums - softmax.
-// ROUNDS: 32 assignments each that the last warp sorts, all loaded at once (one by one they were 300 cycles each, twice).
-// Up to 256 tokens it beats the persistent router and the metadata kernel (24 single-token layers: 128 sequences 1485 -> 1454 us,
-// 256 1809 -> 1791; 64, from the loads alone, 1122 -> 1104).
-template <int E, int ROUNDS>
+// SORT: up to sixteen tokens the warp that finishes last makes the maps; beyond, the sort is 20 to 60 KB of code and up to 3.6 us, and
+// the kernels behind work their rows out from the ids.  Up to 512 tokens it beats the persistent router (300 tokens 1274 -> 1230 us
+// a forward, 400 1426 -> 1405, 512 1508 -> 1501, 700 1648 -> 1672: every warp reads all weights).
+template <int E, bool SORT>
 __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
   __shared__ int h_acc[E];
   const int lane = threadIdx.x, tok = blockIdx.x;
@@ -107,10 +108,10 @@ __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
   float pr[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) pr[e] = 0.f;
-  router_finish<E>(acc, lane, tok, p.idx, p.gates, nullptr, h_acc, pr);       // pr: the probabilities, in lane 0
+  router_finish<E>(acc, lane, tok, p.idx, p.gates, nullptr, h_acc, pr, p.load);       // pr: the probabilities, in lane 0
   int last = 0;
   if (lane == 0) {
-    if (p.scatter) {                             // before the sums: the fence would wait for them too (256 tokens 1366 -> 1358 us a forward)
+    if (SORT && p.scatter) {                     // before the sums: the fence would wait for them too (256 tokens 1366 -> 1358 us a forward)
       __threadfence();
       last = atomicAdd(p.ticket, 1) == p.N - 1;
     }
@@ -120,9 +121,9 @@ __global__ void __launch_bounds__(32) route_small_kernel(const RouteParams p) {
       if (h_acc[e]) atomicAdd(p.hist + e, 1);
     }
   }
-  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  if (!SORT || !__shfl_sync(0xffffffffu, last, 0)) return;
   __threadfence();
-  sort_routes<E, ROUNDS>(reinterpret_cast<const long long*>(p.idx), p.N, lane, p.counts, p.offsets, p.scatter, p.gather, p.gate_idx);
+  sort_routes<E, 1>(reinterpret_cast<const long long*>(p.idx), p.N, lane, p.counts, p.offsets, p.scatter, p.gather, p.gate_idx);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -562,22 +563,19 @@ int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const f
 }
 
 int launch_route_small(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router, int N, int C, int E,
-                       int64_t* idx, float* gates, double* probs_sum, int* hist, int* ticket, int* counts, int* offsets,
+                       int64_t* idx, float* gates, double* probs_sum, int* hist, int* load, int* ticket, int* counts, int* offsets,
                        int* scatter, int* gather, int* gate_idx, cudaStream_t stream) {
   JB_REQUIRE(N >= 1 && N <= ROUTE_SMALL_MAX && C % 8 == 0 && C <= 1024 && (E == 4 || E == 8), "route_small: bad shape (N=%d, C=%d, E=%d)", N, C, E);
   RouteParams p;
   p.x = x; p.w_norm = w_norm; p.w_router = w_router; p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
-  p.idx = idx; p.gates = gates; p.probs_sum = probs_sum; p.hist = hist; p.ticket = ticket;
+  p.idx = idx; p.gates = gates; p.probs_sum = probs_sum; p.hist = hist; p.load = load; p.ticket = ticket;
   p.counts = counts; p.offsets = offsets; p.scatter = scatter; p.gather = gather; p.gate_idx = gate_idx;
   p.eps = eps; p.N = N; p.C = C;
-  static_assert(ROUTE_SMALL_MAX == 256, "sixteen rounds of sixteen tokens");
-  if (N <= 64) {
-    if (E == 4) launch_dep(route_small_kernel<4, 4>, N, 32, 0, stream, p);
-    else launch_dep(route_small_kernel<8, 4>, N, 32, 0, stream, p);
-  } else {
-    if (E == 4) launch_dep(route_small_kernel<4, 16>, N, 32, 0, stream, p);
-    else launch_dep(route_small_kernel<8, 16>, N, 32, 0, stream, p);
-  }
+  JB_REQUIRE(!scatter || N <= ROUTE_SORT_MAX, "route_small: no maps of %d tokens", N);
+  static_assert(ROUTE_SORT_MAX == 16, "one round of the sort");
+  auto kernel = scatter ? (E == 4 ? route_small_kernel<4, true> : route_small_kernel<8, true>)
+                        : (E == 4 ? route_small_kernel<4, false> : route_small_kernel<8, false>);
+  launch_dep(kernel, N, 32, 0, stream, p);
   JB_LAUNCH_CHECK("route_small_kernel");
   return JB200_OK;
 }

@@ -240,7 +240,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     pdl_trigger();
   }
   if (threadIdx.x == 0) {
-    if (p.seg_offsets) {
+    if (p.seg_counts) {
+      int at = 0;
+      for (int g = 0; g < p.G; ++g) {
+        ctl->seg[g] = at;
+        at = min(at + max(p.seg_counts[g], 0), p.M);
+      }
+      ctl->seg[p.G] = at;
+    } else if (p.seg_offsets) {
       for (int g = 0; g <= p.G; ++g) ctl->seg[g] = min(max(p.seg_offsets[g], 0), p.M);
     } else {
       ctl->seg[0] = 0;

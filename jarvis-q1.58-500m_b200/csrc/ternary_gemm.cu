@@ -323,7 +323,8 @@ int pick_bn(int M, int G, int n_ft, int sms) {
 
 int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packed, const float* alpha,
                         int alpha_rows, int N, int G, const int32_t* seg_offsets, int epilogue, void* out,
-                        int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope, bool settled) {
+                        int bn_override, int w_layout, cudaStream_t stream, const GemmRope* rope, bool settled,
+                        const int32_t* seg_counts) {
   JB_REQUIRE(M >= 0 && N > 0 && K > 0, "ternary_linear: bad sizes M=%d N=%d K=%d", M, N, K);
   JB_REQUIRE(N % BM == 0, "ternary_linear: out_features (%d) must be a multiple of %d", N, BM);
   JB_REQUIRE(K % BK == 0, "ternary_linear: in_features (%d) must be a multiple of %d", K, BK);
@@ -358,6 +359,7 @@ int launch_ternary_gemm(const void* x_bf16, int M, int K, const uint8_t* w_packe
   p.w_packed = w_packed;
   p.alpha = alpha;
   p.seg_offsets = seg_offsets;
+  p.seg_counts = settled ? seg_counts : nullptr;
   p.out = out;
   p.M = M; p.N = N; p.K = K; p.G = G;
   p.alpha_rows = alpha_rows;

@@ -605,6 +605,13 @@ def test_chain_where_codes_and_weights_outgrow_their_rings(C, E, mult, B, T):
     _chain_against_kernels(C, E, mult, B, T)
 
 
+@pytest.mark.parametrize("C,E,N", [(1024, 4, 161), (1024, 8, 257), (1024, 4, 512), (1024, 8, 513), (1024, 4, 1184), (128, 8, 1185), (1024, 4, 2368),
+                                   (128, 4, 2369)])
+def test_chain_where_maps_and_rows_come_from_the_ids(C, E, N):
+    """161 to 2368 tokens: eight or sixteen tokens a CTA, around the lines of the routers and of the form with maps made before."""
+    _chain_against_kernels(C, E, 2, 1, N)
+
+
 @pytest.mark.parametrize("B,T", [(1, 961), (1, 1536), (1, 1537), (2, 2304), (1, 4609)])
 def test_chain_where_the_attention_products_leave_the_latency_form(B, T):
     """One wave of tiles of 256 rows: q|k|v up to 1536 tokens, the out-projection up to 4608 (148 SMs)."""
