@@ -105,6 +105,14 @@ struct LsfStats {
   const float* mu;           // with reflect: the layer's reflective penalty is left there
   float lam, tau;
   float* reflect;            // [1] out or null
+  // the counts as doubles with their reciprocals, for the quotients on the device: filled by the launch functions
+  double n_tok, inv_tok, n_el, inv_el, inv_el1;
+  LsfStats counted() const {
+    LsfStats s = *this;
+    s.n_tok = double(n_tokens); s.inv_tok = 1.0 / s.n_tok;
+    s.n_el = double(n_elems); s.inv_el = 1.0 / s.n_el; s.inv_el1 = 1.0 / (s.n_el - 1.0);
+    return s;
+  }
 };
 int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const float* alpha_scalar,
                     const float* act_var, const float* var_scale, float alpha_min, float alpha_max, const float* h0,

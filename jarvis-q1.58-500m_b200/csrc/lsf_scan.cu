@@ -75,21 +75,33 @@ __device__ __forceinline__ void store_last(const Args& p, size_t at, float2 h) {
     if (p.last16) *reinterpret_cast<uint32_t*>(p.last16 + at) = pack_bf16x2(h.x, h.y);
 }
 
+__device__ __forceinline__ float2 stats_mean_var(const LsfStats& st) {
+  return moe_act_mean_var(st.stats[0], st.stats[1], st.n_el, st.inv_el, st.inv_el1);
+}
+
 // The scalar decay of a call (model semantics).  With st.stats the variance of the MoE output is derived here, as
 // moe_finalize_kernel would have, instead of in a launch of its own between the combine and the scan.
 template <typename Args>
 __device__ __forceinline__ float lsf_decay(const Args& p) {
   if (p.alpha_s) return __ldg(p.alpha_s);
   float var;
-  if constexpr (std::is_same_v<Args, LsfChainParams>) var = p.st.stats ? moe_act_var(p.st.stats, p.st.n_elems) : __ldg(p.act_var);
+  if constexpr (std::is_same_v<Args, LsfChainParams>) var = p.st.stats ? stats_mean_var(p.st).y : __ldg(p.act_var);
   else var = __ldg(p.act_var);
   return lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), var);
 }
-// One thread of the whole grid leaves the MoE layer's scalars.
+// One thread of the whole grid leaves the MoE layer's scalars: moe_finalize_scalars, quotients from reciprocals (its CTA's others wait for
+// it: with divisions here and in the decay 24 layers and head of 256, 512 and 900 tokens took 1137, 1504 and 1829 us, so 1103, 1472 and 1803).
 __device__ __forceinline__ void moe_leave_scalars(const LsfStats& st) {
-  moe_finalize_scalars(st.stats, st.probs_sum, st.top1_hist, st.E, st.n_tokens, st.n_elems, st.balance_alpha, st.scalars);
-  if (st.reflect)
-    *st.reflect = reflect_penalty(st.lam, st.tau, __ldg(st.mu), moe_act_mean(st.stats, st.n_elems), moe_act_var(st.stats, st.n_elems));
+  const float2 mv = stats_mean_var(st);
+  if (st.probs_sum && st.top1_hist) {
+    double acc = 0.0;
+#pragma unroll 1
+    for (int e = 0; e < st.E; ++e) acc += div_by(double(st.top1_hist[e]), st.n_tok, st.inv_tok) * div_by(st.probs_sum[e], st.n_tok, st.inv_tok);
+    st.scalars[0] = float(double(st.balance_alpha) * double(st.E) * acc);
+  }
+  st.scalars[1] = mv.x;
+  st.scalars[2] = mv.y;
+  if (st.reflect) *st.reflect = reflect_penalty(st.lam, st.tau, __ldg(st.mu), mv.x, mv.y);
 }
 __device__ __forceinline__ void lsf_leave_scalars(const LsfStats& st) {
   if (st.stats && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) moe_leave_scalars(st);
@@ -331,7 +343,7 @@ __global__ void __launch_bounds__(256) lsf_step_norm_kernel(const LsfStepParams 
     return;
   }
   if (!on) return;
-  const float alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), moe_act_var(p.st.stats, p.st.n_elems));
+  const float alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, __ldg(p.var_scale), stats_mean_var(p.st).y);
   float v[4][8];
   float ss = 0.f;
 #pragma unroll
@@ -783,7 +795,7 @@ int launch_lsf_scan(const void* m, int m_dtype, const void* alpha_tensor, const 
   p.nseg = 1;
   p.n_pre_tiles = 0;
   p.seg_end = p.seg_prod = nullptr;
-  if (st) p.st = *st;
+  if (st) p.st = st->counted();
   if (scratch) {
     JB_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & a8) == 0, "lsf_scan: scratch pointer misaligned");
     const int sms = sm_count();
@@ -829,7 +841,7 @@ int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* va
              "lsf_step_norm: pointers must be 16-byte aligned");
   LsfStepParams p;
   p.m = reinterpret_cast<const __nv_bfloat16*>(m_bf16);
-  p.st = st;
+  p.st = st.counted();
   p.var_scale = var_scale; p.alpha_min = alpha_min; p.alpha_max = alpha_max;
   p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;
   p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);

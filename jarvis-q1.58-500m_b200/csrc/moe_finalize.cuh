@@ -23,10 +23,10 @@ __device__ __forceinline__ float moe_act_var(const double* stats, long long n_el
   return n_elems > 1 ? float(var > 0.0 ? var : 0.0) : __int_as_float(0x7fc00000);
 }
 
-// The same two with n's and (n - 1)'s reciprocals at hand, n > 1 (a division is 0.2 us where every nanosecond is waited for).
+// The same two with n's and (n - 1)'s reciprocals at hand (a division is 0.2 us where every nanosecond is waited for).
 __device__ __forceinline__ float2 moe_act_mean_var(double s1, double s2, double n, double inv_n, double inv_n1) {
   const double mean = div_by(s1, n, inv_n), var = div_by(s2 - s1 * mean, n - 1.0, inv_n1);
-  return make_float2(float(mean), float(var > 0.0 ? var : 0.0));
+  return make_float2(float(mean), n > 1.0 ? float(var > 0.0 ? var : 0.0) : __int_as_float(0x7fc00000));
 }
 
 // scalars[0] = l_balance, [1] = act_mean, [2] = act_var, all f32; one thread.

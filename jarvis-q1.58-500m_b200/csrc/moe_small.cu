@@ -133,7 +133,6 @@ struct TailParams {
   const int* scatter;          // [N][2]
   const int64_t* idx;          // [N][2]
   LsfStats st;                 // stats is not read: the sums are made here
-  double inv_tokens, n_elems, inv_n, inv_n1;
   const float* var_scale;
   float alpha_min, alpha_max;
   const float* h_in;           // [B][C] or null
@@ -215,7 +214,7 @@ __device__ __forceinline__ float tail_decay(const TailParams& p, Combined c, flo
       s[1] += __shfl_xor_sync(0xffffffffu, s[1], o);
     }
     if (lane == 0) {
-      const float2 mv = moe_act_mean_var(s[0], s[1], p.n_elems, p.inv_n, p.inv_n1);
+      const float2 mv = moe_act_mean_var(s[0], s[1], p.st.n_el, p.st.inv_el, p.st.inv_el1);
       *s_alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, mv.y);
       if (rank == 0) {
         p.st.scalars[1] = mv.x;
@@ -260,7 +259,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailPar
   }
   float l_bal = 0.f;
   if (rank == 0 && tid == int(blockDim.x) - 1)
-    l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.inv_tokens, p.st.balance_alpha);
+    l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.st.inv_tok, p.st.balance_alpha);
   __syncwarp();
   pdl_wait();
   pdl_trigger();
@@ -346,7 +345,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   }
   float l_bal = 0.f;
   if (rank == 0 && tid == int(blockDim.x) - 1)
-    l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.inv_tokens, p.st.balance_alpha);
+    l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.st.inv_tok, p.st.balance_alpha);
   __syncwarp();
   pdl_wait();
   pdl_trigger();
@@ -586,9 +585,7 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
   const int N = B * T;
   JB_REQUIRE(N >= 1 && N <= tail_max_tokens(C, T) && C % 128 == 0 && C <= 1024, "tail: bad shape (B=%d, T=%d, C=%d)", B, T, C);
   TailParams p;
-  p.y = reinterpret_cast<const __nv_bfloat16*>(y_bf16); p.gates = gates; p.scatter = scatter; p.idx = idx; p.st = st;
-  p.inv_tokens = 1.0 / double(st.n_tokens);
-  p.n_elems = double(st.n_elems); p.inv_n = 1.0 / p.n_elems; p.inv_n1 = 1.0 / (p.n_elems - 1.0);
+  p.y = reinterpret_cast<const __nv_bfloat16*>(y_bf16); p.gates = gates; p.scatter = scatter; p.idx = idx; p.st = st.counted();
   p.var_scale = var_scale; p.alpha_min = alpha_min; p.alpha_max = alpha_max;
   p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;
   p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
