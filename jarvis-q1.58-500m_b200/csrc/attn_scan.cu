@@ -72,7 +72,7 @@ struct AttnParams {
   float* handoff;          // [CTAs][64][64] f32
   int* ctrl;               // [1 + CTAs], zeroed before the launch
   unsigned int* status;
-  int settled;             // decays (single-token step: state and positions too) were complete before the kernel ahead of this one started
+  int settled;             // decays, angles and positions (single-token step: the state too) were complete before the kernel ahead of this one started
 };
 
 __device__ __forceinline__ uint32_t swz(int row, int chunk16) {  // byte offset inside a swizzled [rows][128 B] tile
@@ -173,17 +173,22 @@ attn_state_pass_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     tmem_alloc(smem_u32(&sm->tmem_base), STATE_TMEM_COLS);
     tmem_relinquish();
   }
-  pdl_wait();        // everything above overlapped the kernel before this one; global memory is read from here on
-  pdl_trigger();
-  const int pos_base = p.pos0 ? p.pos0[b] : p.pos0_scalar;
-  const float log_g = logf(__ldg(p.gamma + h));
-  for (int n = tid; n <= CH; n += STATE_THREADS) sm->pw[n] = expf(log_g * float(n));
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tm = sm->tmem_base;
-  const uint32_t tm_lane = tm + (uint32_t(32 * qd) << 16);
-
+  // What the kernel before this one did not make (`settled`) is read while it runs, and the first tiles are asked for as soon as
+  // they are there (behind the decay table they came 1.3 us later).
+  const int cg = tid & 3;
+  float c64[8], s64[8];
+  int pos_base = 0;
+  auto tables = [&] {
+    pos_base = p.pos0 ? p.pos0[b] : p.pos0_scalar;
+    const float log_g = logf(__ldg(p.gamma + h));
+    for (int n = tid; n <= CH; n += STATE_THREADS) sm->pw[n] = expf(log_g * float(n));
+    const int stp = 64 < p.n_pos ? 64 : p.n_pos - 1;
+    const float4* cq = reinterpret_cast<const float4*>(p.cos_tab + size_t(stp) * 32 + cg * 8);
+    const float4* sq = reinterpret_cast<const float4*>(p.sin_tab + size_t(stp) * 32 + cg * 8);
+    const float4 d0 = __ldg(cq), d1 = __ldg(cq + 1), e0 = __ldg(sq), e1 = __ldg(sq + 1);
+    c64[0] = d0.x; c64[1] = d0.y; c64[2] = d0.z; c64[3] = d0.w; c64[4] = d1.x; c64[5] = d1.y; c64[6] = d1.z; c64[7] = d1.w;
+    s64[0] = e0.x; s64[1] = e0.y; s64[2] = e0.z; s64[3] = e0.w; s64[4] = e1.x; s64[5] = e1.y; s64[6] = e1.z; s64[7] = e1.w;
+  };
   auto issue = [&](int ck) {      // thread 0 only
     const int st = (ck - ck_begin) & 1;
     const uint32_t bar = smem_u32(&sm->full[st]);
@@ -191,9 +196,19 @@ attn_state_pass_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     tma_load_2d(smem_u32(sm->k[st]), &tm_k, h * D, row0 + ck * CH, bar);
     tma_load_2d(smem_u32(sm->v[st]), &tm_v, h * D, row0 + ck * CH, bar);
   };
+  if (p.settled) tables();
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
   if (tid == 0) {
     for (int ck = ck_begin; ck < ck_begin + 2 && ck < ck_end; ++ck) issue(ck);
   }
+  if (!p.settled) tables();
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tm = sm->tmem_base;
+  const uint32_t tm_lane = tm + (uint32_t(32 * qd) << 16);
 
   // the thread's share of the state: row dv = 32*(qd&1) + lane, columns 16*cg .. 16*cg+15 (see the pipeline kernel)
   const int s_row = 32 * (qd & 1) + lane;
@@ -202,17 +217,7 @@ attn_state_pass_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
 #pragma unroll
   for (int e = 0; e < 16; ++e) S[e] = 0.f;
 
-  const int cg = tid & 3;
   const int r_lo = (tid >> 5) * 8 + ((tid >> 2) & 1) * 4 + ((tid >> 3) & 3);
-  float c64[8], s64[8];
-  {
-    const int stp = 64 < p.n_pos ? 64 : p.n_pos - 1;
-    const float4* cq = reinterpret_cast<const float4*>(p.cos_tab + size_t(stp) * 32 + cg * 8);
-    const float4* sq = reinterpret_cast<const float4*>(p.sin_tab + size_t(stp) * 32 + cg * 8);
-    const float4 d0 = __ldg(cq), d1 = __ldg(cq + 1), e0 = __ldg(sq), e1 = __ldg(sq + 1);
-    c64[0] = d0.x; c64[1] = d0.y; c64[2] = d0.z; c64[3] = d0.w; c64[4] = d1.x; c64[5] = d1.y; c64[6] = d1.z; c64[7] = d1.w;
-    s64[0] = e0.x; s64[1] = e0.y; s64[2] = e0.z; s64[3] = e0.w; s64[4] = e1.x; s64[5] = e1.y; s64[6] = e1.z; s64[7] = e1.w;
-  }
 
   bool ok = true;
   for (int ck = ck_begin; ck < ck_end; ++ck) {
@@ -504,16 +509,18 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_after_sync();
   const uint32_t tm = sm->tmem_base;
   volatile uint32_t* abort_flag = &sm->abort_flag;
-  if (tables_first) {
-    pdl_wait();
-    pdl_trigger();
-  }
+  // Then the roles that read what it made (tiles; states of segments) wait for it; angles are on their way before, and rows leave
+  // behind the tiles they come from.
 
   // Chunks are counted over all items (g): stages, accumulators and barrier phases follow that count.
   if (warp < PRO_WARP0) {
     regs_dec<ISSUE_REGS>();
     if (warp == 0) {
       // ---------------- TMA producer ----------------
+      if (tables_first) {
+        pdl_wait();
+        pdl_trigger();
+      }
       int s = 0, g = 0;
       uint32_t prev = 1u;                         // parity of the PREVIOUS use of the stage
       bool ok = true;
@@ -729,6 +736,7 @@ attn_scan_pipe_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // ---------------- state ----------------
     // f32 state: row dv = 32*(qd&1) + lane, columns dk = 32*half .. +31 (the accumulator of MMA S holds the 64 dv rows
     // twice, lanes 0-63 and 64-127, so every warp finds its share in its own lane quarter)
+    if (tables_first) pdl_wait();
     const int qd = warp & 3, half = qd >> 1, s_row = 32 * (qd & 1) + lane;
     const int stid = tid - STATE_WARP0 * 32;
     const uint32_t tm_ds = tm + (uint32_t(32 * qd) << 16) + PT_DS + 32 * half;
@@ -1325,7 +1333,9 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   if (!o) {
     // state only: the k/v pass over every piece, then the fold
     JB_MAX_SMEM(attn_state_pass_kernel, STATE_SMEM_BYTES);
-    launch_dep(attn_state_pass_kernel, dim3(H, B, p.nseg), STATE_THREADS, STATE_SMEM_BYTES, stream, tk, tv, p);
+    AttnParams ps = p;
+    ps.settled = settled ? 1 : 0;
+    launch_dep(attn_state_pass_kernel, dim3(H, B, p.nseg), STATE_THREADS, STATE_SMEM_BYTES, stream, tk, tv, ps);
     JB_LAUNCH_CHECK("attn_state_pass_kernel");
     launch_dep(attn_fold_states_kernel, dim3(H, B), 256, 0, stream, p);
     JB_LAUNCH_CHECK("attn_fold_states_kernel");
@@ -1335,7 +1345,9 @@ int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, co
   else JB_MAX_SMEM(attn_scan_pipe_kernel<false>, PIPE_SMEM_BYTES);
   if (p.nseg > 1) {
     JB_MAX_SMEM(attn_state_pass_kernel, STATE_SMEM_BYTES);
-    launch_dep(attn_state_pass_kernel, dim3(H, B, p.nseg - 1), STATE_THREADS, STATE_SMEM_BYTES, stream, tk, tv, p);
+    AttnParams ps = p;
+    ps.settled = settled ? 1 : 0;
+    launch_dep(attn_state_pass_kernel, dim3(H, B, p.nseg - 1), STATE_THREADS, STATE_SMEM_BYTES, stream, tk, tv, ps);
     JB_LAUNCH_CHECK("attn_state_pass_kernel");
   }
   // output rows leave 32 at a time, clipped at the end of their sequence

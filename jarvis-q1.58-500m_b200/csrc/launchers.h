@@ -123,7 +123,7 @@ int launch_lsf_step_norm(const void* m_bf16, const LsfStats& st, const float* va
                          const float* h_in, float* h_out, float* x, const float* w_norm, float eps, void* xn_bf16, int B,
                          int C, cudaStream_t stream, bool ahead = false);
 
-// settled: gamma and, at T == 1, s_in and pos0 were complete before the kernel ahead of this one on the stream began.
+// settled: gamma, angle tables, pos0 and, at T == 1, s_in were complete before the kernel ahead of this one on the stream began.
 int launch_attn_scan(const void* q, const void* k, const void* v, int ld_qkv, const float* gamma,
                      const float* cos_tab, const float* sin_tab, int n_pos, const int32_t* pos0, int pos0_scalar,
                      const float* s_in, void* o, int ld_o, float* s_out, void* scratch, int B, int T, int H,
