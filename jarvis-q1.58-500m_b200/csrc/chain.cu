@@ -45,7 +45,7 @@ struct Workspace {
     out = o;
     attn = take(T > 1 ? attn_scan_scratch_bytes(B, T, H) : 0);
     lsf = take(T > 1 ? lsf_scan_scratch_bytes(B, T, C) : 0);
-    meta = take(moe_metadata_scratch_bytes(int(N), 2, E));
+    meta = take(std::max(moe_metadata_scratch_bytes(int(N), 2, E), (N + 7) / 8 * sizeof(unsigned long long)));
     bytes = p;
   }
 };
@@ -262,13 +262,17 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     const bool late_maps = mid && all_rows;
     const MidRoutes store = {idx, false, counts, offs, scatter, gather, gate_idx};
     const MidRoutes rows_of = {idx, true, nullptr, nullptr, nullptr, nullptr, nullptr};
-    const bool from_ids = !all_rows && N <= DISPATCH_IDS_MAX;       // maps and rows in one launch
+    // maps and rows in one launch: from the ids, or where the router is a single pass of eight tokens a CTA from the counts it leaves
+    const bool one_launch = !all_rows && N <= std::min(DISPATCH_EIGHTS_MAX, 16 * sms);
+    static_assert(ROUTE_SMALL_MAX <= DISPATCH_IDS_MAX, "the router without counts");
+    unsigned long long* counts8 = one_launch && N > ROUTE_SMALL_MAX ? reinterpret_cast<unsigned long long*>(w + ws.meta) : nullptr;
     if (N <= ROUTE_SMALL_MAX) {
-      JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, from_ids ? load : nullptr, ticket,
+      JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, one_launch ? load : nullptr, ticket,
                                 counts, offs, all_rows && !late_maps ? scatter : nullptr, gather, gate_idx, st));
     } else {
-      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true, from_ids ? load : nullptr));
-      if (!from_ids) JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
+      JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true,
+                                   one_launch ? load : nullptr, counts8));
+      if (!one_launch) JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
     }
     if (all_rows) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
@@ -277,12 +281,12 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       else
         JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, nullptr, &store, JB200_EPI_GELU_BF16, hid, w1_tile));
     } else {
-      if (from_ids) JB_TRY(launch_dispatch_ids(idx, xn, N, C, E, counts, offs, scatter, gather, gate_idx, disp, st));
+      if (one_launch) JB_TRY(launch_dispatch_chain(idx, counts8, xn, N, C, E, counts, offs, scatter, gather, gate_idx, disp, st));
       else JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
         JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, nullptr, load, nullptr, JB200_EPI_GELU_BF16, hid, w1_tile));
       else
-        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true, from_ids ? load : nullptr));
+        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true, one_launch ? load : nullptr));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, st));

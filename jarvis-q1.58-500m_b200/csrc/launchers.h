@@ -67,16 +67,19 @@ int launch_router_top2(const void* x_bf16, const float* w_router, int n_tokens, 
                        float* gates, float* probs_out, double* probs_sum, int* top1_hist, cudaStream_t stream);
 int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router,
                           int n_tokens, int C, int E, int64_t* topk_idx, float* gates, double* probs_sum,
-                          int* top1_hist, cudaStream_t stream, bool ahead = false, int* load = nullptr);
+                          int* top1_hist, cudaStream_t stream, bool ahead = false, int* load = nullptr,
+                          unsigned long long* counts8 = nullptr);
 size_t moe_metadata_scratch_bytes(int n_tokens, int K, int E);
 // Maps and rows of top-2 assignments at once.  scratch: moe_dispatch_scratch_bytes.
 size_t moe_dispatch_scratch_bytes(int n_tokens, int E);
 int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, void* scratch, int* expert_counts,
                         int* expert_offsets, int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream);
-// The same in one launch, inside a chain, without counts made before: up to where sixteen tokens a CTA are one wave.
-constexpr int DISPATCH_IDS_MAX = 2368;
-int launch_dispatch_ids(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int* expert_counts, int* expert_offsets,
-                        int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream);
+// The same in one launch, inside a chain.  counts8: what launch_rmsnorm_router left, the assignments of every eight tokens, a byte per
+// expert; null: counted from the ids.
+constexpr int DISPATCH_IDS_MAX = 512, DISPATCH_EIGHTS_MAX = 2368;
+int launch_dispatch_chain(const int64_t* topk_idx, const unsigned long long* counts8, const void* x_bf16, int n_tokens, int C, int E,
+                          int* expert_counts, int* expert_offsets, int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched,
+                          cudaStream_t stream);
 int launch_moe_metadata(const int64_t* topk_idx, int n_tokens, int K, int E, int* expert_counts, int* expert_offsets,
                         int* scatter_map, int* gather_map, int* gate_idx_map, void* scratch, cudaStream_t stream);
 int moe_metadata_static_max_assignments();

@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(ROUTER_THREADS, 2)
 rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_norm, float eps,
                       __nv_bfloat16* __restrict__ xn, const float* __restrict__ w_router, int n_tokens, int C,
                       int64_t* __restrict__ topk_idx, float* __restrict__ gates,
-                      double* __restrict__ probs_sum, int* __restrict__ top1_hist, int* __restrict__ load, bool ahead) {
+                      double* __restrict__ probs_sum, int* __restrict__ top1_hist, int* __restrict__ load,
+                      unsigned long long* __restrict__ counts8, bool ahead) {
   extern __shared__ float w_s[];  // [E][C]
   __shared__ float p_acc[ROUTER_THREADS / 32][E];
   __shared__ int h_acc[E], l_acc[E];
@@ -186,6 +187,12 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
     if (probs_sum) atomicAdd(&probs_sum[threadIdx.x], double(s));
     if (top1_hist && h_acc[threadIdx.x]) atomicAdd(&top1_hist[threadIdx.x], h_acc[threadIdx.x]);
     if (load && l_acc[threadIdx.x]) atomicAdd(&load[threadIdx.x], l_acc[threadIdx.x]);
+  }
+  if (PER == 1 && counts8 && threadIdx.x == 32) {          // single pass: the CTA's eight tokens, a byte per expert
+    unsigned long long c = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) c |= (unsigned long long)(l_acc[e]) << (8 * e);
+    counts8[blockIdx.x] = c;
   }
 }
 
@@ -366,21 +373,26 @@ dispatch_hist_kernel(const int64_t* __restrict__ topk_idx, int M, int* __restric
 // chunks (E integers each, from L2), ranks its assignments with ballots - the order of the kernels above - and copies its rows:
 // each is read once and stored at both of its slots, where the gather reads every row twice.  For an MoE layer called by itself;
 // sizes and times at one_launch_dispatch.
-// IDS, inside the native call: the counts are taken from the ids themselves, by every CTA, and the first expert matrix reads the segments
-// off the router's counts while this kernel runs.  Latency: ids and rows travel together, then one exchange over the CTA.  24 layers and
-// head against metadata (256 tokens: by the router's last warp, 3.6 of its 7 us) and gather: 180 tokens 1104 -> 1064 us, 256 1180 -> 1130,
-// 512 1525 -> 1506, 1300 2563 -> 2512, 3 x 777 2929 -> 2907, steps of 256 sequences 1528 -> 1484; every CTA reads all ids: 3000
-// 3442 -> 3448, 4096 4042 -> 4197, so the line is where CTAs of sixteen tokens are one wave.
-template <int E, int TOK, bool IDS>
+// Inside the native call the counts are taken from the ids themselves (IDS, up to 512 tokens) or from what the router left for every
+// eight tokens (EIGHTS), by every CTA, and the first expert matrix reads the segments off the router's counts while this kernel runs.
+// Latency: ids or counts and rows travel together, then one exchange over the CTA.  24 layers and head against metadata (256 tokens:
+// by the router's last warp, 3.6 of its 7 us) and gather: 180 tokens 1104 -> 1064 us, 256 1180 -> 1130, steps of 256 sequences 1528 ->
+// 1484, all from the ids; then with sums per expert by shared-memory additions instead of a table that every thread adds up, and from the
+// router's counts beyond 512: 256 1084 -> 1054, 512 1440 -> 1413, 900 1741 -> 1686, 1300 2436 -> 2381, 3 x 777 2861 -> 2804 (2929 with
+// metadata and gather).  Up to 2368 tokens the router is one pass of eight tokens a CTA; from 3000 on, from the ids, it was no faster.
+enum DispatchCounts { CHUNKS, IDS, EIGHTS };
+template <int E, int TOK, DispatchCounts FROM>
 __global__ void __launch_bounds__(DISP_THREADS)
-dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __restrict__ x, const int* __restrict__ chunk_counts,
+dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __restrict__ x, const void* __restrict__ counted,
                 int n_tokens, int C, int* __restrict__ expert_counts, int* __restrict__ expert_offsets, int* __restrict__ scatter_map,
                 int* __restrict__ gather_map, int* __restrict__ gate_idx_map, __nv_bfloat16* __restrict__ dispatched) {
   constexpr int WARPS = DISP_THREADS / 32, RANK_WARPS = (2 * TOK + 31) / 32, PER_WARP = TOK / WARPS, ROWS = PER_WARP < 2 ? 1 : 2;
-  __shared__ int red[WARPS][2 * E], in_warp[RANK_WARPS][E], slots[2 * TOK];
+  __shared__ int all_of[E], ahead_of[E], in_warp[RANK_WARPS][E], slots[2 * TOK];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid < E) all_of[tid] = ahead_of[tid] = 0;
+  __syncthreads();
   pdl_wait();
   pdl_trigger();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tok0 = int(blockIdx.x) * TOK, M = 2 * n_tokens, m = 2 * tok0 + tid;
   // the warp's first two rows and its assignments travel while the counts are added up
   const int first = tok0 + warp * PER_WARP;
@@ -399,14 +411,23 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
   int total[E], before[E];
 #pragma unroll
   for (int q = 0; q < E; ++q) total[q] = before[q] = 0;
-  if constexpr (IDS) {
-    unsigned long long all = 0, ahead = 0;               // a byte per expert: at most 2 * DISPATCH_IDS_MAX / DISP_THREADS
-#pragma unroll 4
-    for (int t = tid; t < n_tokens; t += DISP_THREADS) {
-      const longlong2 id = __ldcg(reinterpret_cast<const longlong2*>(topk_idx) + t);
-      const unsigned long long two = (1ull << (8 * clamp_expert(id.x, E))) + (1ull << (8 * clamp_expert(id.y, E)));
-      all += two;
-      ahead += t < tok0 ? two : 0ull;
+  if constexpr (FROM != CHUNKS) {
+    unsigned long long all = 0, ahead = 0;               // a byte per expert and thread
+    if constexpr (FROM == IDS) {
+#pragma unroll 2
+      for (int t = tid; t < n_tokens; t += DISP_THREADS) {
+        const longlong2 id = __ldcg(reinterpret_cast<const longlong2*>(topk_idx) + t);
+        const unsigned long long two = (1ull << (8 * clamp_expert(id.x, E))) + (1ull << (8 * clamp_expert(id.y, E)));
+        all += two;
+        ahead += t < tok0 ? two : 0ull;
+      }
+    } else {
+#pragma unroll 2
+      for (int c = tid; 8 * c < n_tokens; c += DISP_THREADS) {
+        const unsigned long long v = __ldcg(static_cast<const unsigned long long*>(counted) + c);
+        all += v;
+        ahead += 8 * c < tok0 ? v : 0ull;
+      }
     }
 #pragma unroll
     for (int q = 0; q < E; ++q) {
@@ -417,7 +438,7 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
     for (int c = tid; c < int(gridDim.x); c += DISP_THREADS) {
 #pragma unroll
       for (int q4 = 0; q4 < E / 4; ++q4) {
-        const int4 v = __ldcg(reinterpret_cast<const int4*>(chunk_counts + size_t(c) * E) + q4);
+        const int4 v = __ldcg(reinterpret_cast<const int4*>(static_cast<const int*>(counted) + size_t(c) * E) + q4);
         const int w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -427,10 +448,15 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
       }
     }
   }
+  int mine = 0, before_mine = 0;                           // lane e: the warp's sums of expert e
 #pragma unroll
   for (int q = 0; q < E; ++q) {
     const int a = __reduce_add_sync(0xffffffffu, total[q]), b = __reduce_add_sync(0xffffffffu, before[q]);
-    if (lane == 0) { red[warp][q] = a; red[warp][E + q] = b; }
+    if (lane == q) { mine = a; before_mine = b; }
+  }
+  if (lane < E) {
+    atomicAdd(&all_of[lane], mine);
+    atomicAdd(&ahead_of[lane], before_mine);
   }
   int rank = 0;
   if (warp < RANK_WARPS) {
@@ -443,11 +469,8 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
   }
   __syncthreads();
   if (e >= 0) {
-    int slot = rank;
-    for (int w = 0; w < WARPS; ++w) {
-      slot += red[w][E + e];
-      for (int q = 0; q < e; ++q) slot += red[w][q];
-    }
+    int slot = rank + ahead_of[e];
+    for (int q = 0; q < e; ++q) slot += all_of[q];
     for (int w = 0; w < warp; ++w) slot += in_warp[w][e];
     scatter_map[m] = slot;
     gather_map[slot] = m >> 1;
@@ -455,13 +478,10 @@ dispatch_kernel(const int64_t* __restrict__ topk_idx, const __nv_bfloat16* __res
     slots[tid] = slot;
   }
   if (blockIdx.x == 0 && tid <= E) {
-    int off = 0, own = 0;
-    for (int w = 0; w < WARPS; ++w) {
-      for (int q = 0; q < tid; ++q) off += red[w][q];
-      if (tid < E) own += red[w][tid];
-    }
+    int off = 0;
+    for (int q = 0; q < tid; ++q) off += all_of[q];
     expert_offsets[tid] = off;
-    if (tid < E) expert_counts[tid] = own;
+    if (tid < E) expert_counts[tid] = all_of[tid];
   }
   __syncthreads();
   for (int t = 0; t < PER_WARP; t += ROWS) {
@@ -669,7 +689,8 @@ int launch_router_top2(const void* x_bf16, const float* w_router, int n_tokens, 
 
 int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* xn_bf16, const float* w_router,
                           int n_tokens, int C, int E, int64_t* topk_idx, float* gates, double* probs_sum,
-                          int* top1_hist, cudaStream_t stream, bool ahead, int* load) {
+                          int* top1_hist, cudaStream_t stream, bool ahead, int* load,
+                          unsigned long long* counts8) {
   JB_REQUIRE(n_tokens >= 0 && C > 0, "rmsnorm_router: bad shape");
   JB_REQUIRE(E == 4 || E == 8, "rmsnorm_router: num_experts (%d) must be 4 or 8", E);
   JB_REQUIRE(C % 8 == 0 && C <= 1024, "rmsnorm_router: d_model (%d) must be a multiple of 8 and at most 1024", C);
@@ -683,12 +704,13 @@ int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* 
   if (sms <= 0) return JB200_ERR_CUDA;
   const int warps = ROUTER_THREADS / 32, per = n_tokens <= 2 * sms * warps ? 1 : 2;
   const int blocks = std::min((n_tokens + per * warps - 1) / (per * warps), 2 * sms);
+  JB_REQUIRE(!counts8 || (per == 1 && load), "rmsnorm_router: counts of eight tokens need a single pass");
   const size_t smem = size_t(E) * C * sizeof(float);
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
   auto kernel = per == 1 ? (E == 4 ? rmsnorm_router_kernel<4, 1> : rmsnorm_router_kernel<8, 1>)
                          : (E == 4 ? rmsnorm_router_kernel<4, 2> : rmsnorm_router_kernel<8, 2>);
   launch_dep(kernel, blocks, ROUTER_THREADS, smem, stream, x, w_norm, eps, xn, w_router, n_tokens, C, topk_idx, gates, probs_sum, top1_hist,
-             load, ahead);
+             load, counts8, ahead);
   JB_LAUNCH_CHECK("rmsnorm_router_kernel");
   return JB200_OK;
 }
@@ -736,28 +758,32 @@ int launch_moe_dispatch(const int64_t* topk_idx, const void* x_bf16, int n_token
                         : (E == 4 ? dispatch_hist_kernel<4, 64> : dispatch_hist_kernel<8, 64>);
   launch_dep(hist, blocks, 2 * tok, 0, stream, topk_idx, 2 * n_tokens, chunk_counts);
   JB_LAUNCH_CHECK("dispatch_hist_kernel");
-  auto kernel = tok == 32 ? (E == 4 ? dispatch_kernel<4, 32, false> : dispatch_kernel<8, 32, false>)
-                          : (E == 4 ? dispatch_kernel<4, 64, false> : dispatch_kernel<8, 64, false>);
+  auto kernel = tok == 32 ? (E == 4 ? dispatch_kernel<4, 32, CHUNKS> : dispatch_kernel<8, 32, CHUNKS>)
+                          : (E == 4 ? dispatch_kernel<4, 64, CHUNKS> : dispatch_kernel<8, 64, CHUNKS>);
   launch_dep(kernel, blocks, DISP_THREADS, 0, stream, topk_idx, x, chunk_counts, n_tokens, C, expert_counts, expert_offsets, scatter_map,
              gather_map, gate_idx_map, d);
   JB_LAUNCH_CHECK("dispatch_kernel");
   return JB200_OK;
 }
 
-int launch_dispatch_ids(const int64_t* topk_idx, const void* x_bf16, int n_tokens, int C, int E, int* expert_counts, int* expert_offsets,
-                        int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched, cudaStream_t stream) {
-  JB_REQUIRE(n_tokens >= 1 && n_tokens <= DISPATCH_IDS_MAX && (E == 4 || E == 8) && C >= 8 && C % 8 == 0 && C <= 1024,
-             "dispatch_ids: bad shape (N=%d, C=%d, E=%d)", n_tokens, C, E);
+int launch_dispatch_chain(const int64_t* topk_idx, const unsigned long long* counts8, const void* x_bf16, int n_tokens, int C, int E,
+                          int* expert_counts, int* expert_offsets, int* scatter_map, int* gather_map, int* gate_idx_map, void* dispatched,
+                          cudaStream_t stream) {
+  JB_REQUIRE(n_tokens >= 1 && n_tokens <= (counts8 ? DISPATCH_EIGHTS_MAX : DISPATCH_IDS_MAX) && (E == 4 || E == 8) && C >= 8 && C % 8 == 0 &&
+                 C <= 1024,
+             "dispatch_chain: bad shape (N=%d, C=%d, E=%d)", n_tokens, C, E);
   JB_REQUIRE(topk_idx && x_bf16 && expert_counts && expert_offsets && scatter_map && gather_map && gate_idx_map && dispatched,
-             "dispatch_ids: null pointer");
-  JB_REQUIRE(aligned16(topk_idx) && aligned16(x_bf16) && aligned16(dispatched), "dispatch_ids: pointers must be 16-byte aligned");
-  static_assert(DISPATCH_IDS_MAX / DISP_THREADS * 2 < 256, "a byte per expert and thread");
-  const int tok = n_tokens <= 8 * 148 ? 8 : n_tokens <= 16 * 148 ? 16 : 32;        // a wave of CTAs, as small as they go
-  auto kernel = tok == 8    ? (E == 4 ? dispatch_kernel<4, 8, true> : dispatch_kernel<8, 8, true>)
-                : tok == 16 ? (E == 4 ? dispatch_kernel<4, 16, true> : dispatch_kernel<8, 16, true>)
-                            : (E == 4 ? dispatch_kernel<4, 32, true> : dispatch_kernel<8, 32, true>);
+             "dispatch_chain: null pointer");
+  JB_REQUIRE(aligned16(topk_idx) && aligned16(x_bf16) && aligned16(dispatched), "dispatch_chain: pointers must be 16-byte aligned");
+  static_assert(DISPATCH_IDS_MAX / DISP_THREADS * 2 < 256 && (DISPATCH_EIGHTS_MAX / 8 + DISP_THREADS - 1) / DISP_THREADS * 16 < 256,
+                "a byte per expert and thread");
+  const bool few = n_tokens <= 8 * 148;                    // a wave of CTAs, as small as they go
+  auto kernel = counts8 ? (few ? (E == 4 ? dispatch_kernel<4, 8, EIGHTS> : dispatch_kernel<8, 8, EIGHTS>)
+                               : (E == 4 ? dispatch_kernel<4, 16, EIGHTS> : dispatch_kernel<8, 16, EIGHTS>))
+                        : (E == 4 ? dispatch_kernel<4, 8, IDS> : dispatch_kernel<8, 8, IDS>);
+  const int tok = few || !counts8 ? 8 : 16;
   launch_dep(kernel, (n_tokens + tok - 1) / tok, DISP_THREADS, 0, stream, topk_idx, reinterpret_cast<const __nv_bfloat16*>(x_bf16),
-             static_cast<const int*>(nullptr), n_tokens, C, expert_counts, expert_offsets, scatter_map, gather_map, gate_idx_map,
+             static_cast<const void*>(counts8), n_tokens, C, expert_counts, expert_offsets, scatter_map, gather_map, gate_idx_map,
              reinterpret_cast<__nv_bfloat16*>(dispatched));
   JB_LAUNCH_CHECK("dispatch_kernel");
   return JB200_OK;
