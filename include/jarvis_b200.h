@@ -464,7 +464,7 @@ void jb200_host_decode16(uint32_t word, uint32_t* out8);
 void jb200_host_decode16_prepared(uint32_t word, uint32_t* out8);
 /* Tiles that jb200_forward_layers gives the first or second expert matrix where it runs in the tcgen05 form for few tokens, on a device
  * with `sms` multiprocessors: out6 = whether every expert takes all tokens, out-features of a tile, rows of a token tile for experts
- * that are used evenly and at most, and the chunks that either one's ring holds at least.  Runs on the CPU; used by the unit tests.  0: no such call. */
+ * that are used evenly and at most, and the chunks (of two K-blocks) that either one's ring holds at least.  Runs on the CPU; used by the unit tests.  0: no such call. */
 int jb200_host_expert_tiles(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out6);
 
 #ifdef __cplusplus

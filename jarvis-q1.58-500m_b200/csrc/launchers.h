@@ -49,9 +49,10 @@ struct MidRoutes {
 };
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
                     const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
-                    cudaStream_t stream);
+                    bool coarse, cudaStream_t stream);
 constexpr int MID_FEATURES = 128;              // out-features of its tiles
-int mid_gemm_least_chunks(int bn, int K);      // what its ring holds at least with token tiles of bn
+bool mid_gemm_coarse_fits(int bn, int K);      // `coarse`, chunks of four K-blocks in place of two: where its ring still holds three
+int mid_gemm_least_chunks(int bn, int K);      // what its ring holds at least with token tiles of bn, in chunks of two K-blocks
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);
 void decode16_prepared_host(uint32_t w_canonical, uint32_t* out8);

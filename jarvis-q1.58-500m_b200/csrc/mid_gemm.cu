@@ -9,16 +9,18 @@
 //     stage there is before the grid dependency is waited for;
 //   - the weights are the MMA's A operand in TENSOR memory: a K = 16 step of N tokens takes 10 + N / 2 cycles, where 128 rows read from
 //     shared memory cost 43 + N / 2 and 64 rows 27 + N / 2 (48 tokens: 34 against 67 and 51).  What the accumulator leaves of the
-//     512 columns holds seven chunks, so of K = 1024 nearly all is decoded ahead, when no MMA is in the way of the stores;
+//     512 columns holds twelve to fourteen K-blocks, so of K = 1024 nearly all is decoded ahead, when no MMA is in the way of the stores;
 //   - K-blocks travel in chunks of CK: one TMA copy, one barrier wait and one commit per chunk (~290, ~85 and ~45 cycles,
-//     none of which hides behind MMAs: issuing them takes as long as they do), with as many chunks in flight as fit;
+//     none of which hides behind MMAs: issuing them takes as long as they do), with as many chunks in flight as fit: four K-blocks a
+//     chunk where three of them do, else two (24 layers and head with two -> four: 17, 37, 64, 128, 256 tokens 677 -> 654, 697 -> 675,
+//     745 -> 712, 866 -> 841, 1062 -> 1030 us; with a ring of two or one 900 tokens 1694 -> 1784; counted at run time +1.5 %);
 //   - codes come by TMA, all at once up to K = 2048, in rows of 128 bytes;
 //   - the eight decoder warps become the epilogue; the residual is added by reductions, nothing waits for old values.  Weight
 //     rows are dealt to lanes so that a thread finds four neighbouring out-features of a token: 8- and 16-byte stores, no shuffles.
 // With weights in shared memory, in tiles of 64 or 128 out-features, and codes in registers 24 layers and head as a graph took 881 us at
 // 37 tokens (now 779), 1096 at 128 (904), 1360 at 256 (1181), 2068 at 900 (1849), steps of 64 and 256 sequences 958 (878) and 1699 (1533).
-// What is left: the first copy's way (0.5 us after the dependency), 0.17-0.2 us a chunk, epilogue and the end of the grid (0.6 and
-// 0.6-0.9 us), and where the kernel ahead is short, decoding (0.28 us a chunk).  Not kept: sixteen decoder warps (180 to 512 tokens 2-3 %
+// What is left: the first copy's way (0.5 us after the dependency), 0.17-0.2 us for two K-blocks, epilogue and the end of the grid (0.6 and
+// 0.6-0.9 us), and where the kernel ahead is short, decoding (0.14 us a K-block).  Not kept: sixteen decoder warps (180 to 512 tokens 2-3 %
 // slower: their registers are not free while the kernel ahead runs), one look at all barriers in place of a wait each, commits left out, a pass
 // through MMA loop and epilogue before the dependency (each +1-3 %), a box of codes stored in one go (+2 %).
 // Accumulation is the same chain of K = 16 steps as in ternary_gemm_kernel: results are its bit for bit.
@@ -34,10 +36,9 @@ namespace jb {
 namespace {
 
 constexpr int BM = 128, BK = 64;               // out-features of a tile, K of a block
-constexpr int CK = 2;                          // K-blocks per chunk (four: 1-3 % slower, the ring gets too coarse)
+constexpr int CK_MOST = 4;                     // K-blocks per chunk: four, or two where the ring would be too coarse
 constexpr int MAX_CHUNKS = 8, DEC_WARP0 = 2, CODE_WARP = 10, MAP_WARP = 11, THREADS = 32 * (CODE_WARP + 1);
 constexpr int BOX_KB = 8, BOX_BYTES = BM * BOX_KB * 16, MAX_BOXES = 4;      // codes of eight K-blocks a copy, 128 bytes a row
-constexpr int BOX_CHUNKS = BOX_KB / CK;
 constexpr uint32_t TMEM_COLS = 512, KB_COLS = BK / 2;                       // a K-block of weights: a bf16 pair per column
 
 struct MidParams {
@@ -110,7 +111,7 @@ __host__ __device__ constexpr int acc_cols(int bn) { return (bn + 63) / 64 * 64;
 
 // ROUTE: 0 rows or segments as given, 1 rows stored in dispatch order and the maps left by a warp of their own, 2 segments counted from
 // the ids (kernels of their own: the code of the others costs a plain call 1 %).
-template <int ROUTE>
+template <int ROUTE, int CK>
 __global__ void __launch_bounds__(ROUTE == 1 ? THREADS + 32 : THREADS, 1)
 mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -207,7 +208,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   const bool t1 = __any_sync(0xffffffffu, ctl.pick == 1), t2 = __any_sync(0xffffffffu, ctl.pick == 2);
   const int bn = t2 ? p.bn[2] : t1 ? p.bn[1] : p.bn[0], n_ch = p.K / (BK * CK);
   const int S = t2 ? p.chunks[2] : t1 ? p.chunks[1] : p.chunks[0];
-  const uint32_t kb_bytes = uint32_t(bn) * BK * 2, b_bytes = kb_bytes * CK;
+  const uint32_t kb_bytes = uint32_t(bn) * BK * 2, b_bytes = kb_bytes * uint32_t(CK);
   const uint32_t b_base = base + uint32_t(p.boxes) * BOX_BYTES, a_tmem = tmem + uint32_t(acc_cols(bn));
   const CUtensorMap* tmap_x = t2 ? &maps.x[2] : t1 ? &maps.x[1] : &maps.x[0];
   auto item = [&](Items& it, int i) {
@@ -313,7 +314,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     }
   } else {
     // ---------------- decoders, then epilogue ----------------
-    // This thread decodes, of K-block `par` of every chunk, the 64 codes of the out-feature that its lane of tensor memory holds.
+    // This thread decodes, of every other K-block from `par` on, the 64 codes of the out-feature that its lane of tensor memory holds.
     // Lanes g, g + 8, g + 16 and g + 24 of a warp's 32 are four neighbours, so that a thread of the epilogue has them together; which
     // of the four is turned by g / 2, for eight lanes' codes in eight different bank groups.
     const int par = (warp - DEC_WARP0) >> 2, q4 = warp & 3;                          // q4: the lanes this warp can reach
@@ -323,28 +324,33 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
     int c = 0, s = 0, box = 0;
     uint32_t ph = 1u, box_ph = 0u;
     bool ok = true;
+    constexpr int BOX_CHUNKS = BOX_KB / CK;
     auto decode_to = [&](int limit, bool fresh) {
 #pragma unroll 1
       for (; c < limit; ++c) {
-        if ((c & (BOX_CHUNKS - 1)) == 0 && !wait_for(smem_u32(&ctl.code_full[box]), box_ph, abort_flag, p.status, JB200_STATUS_GEMM_DECODE)) { ok = false; return; }
-        uint32_t w[4], v[32];
-        const uint32_t piece = uint32_t((c & (BOX_CHUNKS - 1)) * CK + par) ^ uint32_t(r & 7);       // 128-byte swizzle: no bank conflicts
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(code_row + uint32_t(box) * BOX_BYTES + (piece << 4)) : "memory");
-#pragma unroll
-        for (int i = 0; i < 4; ++i) decode16_prepared(w[i], v + 8 * i);
+        const int in_box = c & (BOX_CHUNKS - 1);
+        if (in_box == 0 && !wait_for(smem_u32(&ctl.code_full[box]), box_ph, abort_flag, p.status, JB200_STATUS_GEMM_DECODE)) { ok = false; return; }
         if (!fresh) {
           if (!wait_for(smem_u32(&ctl.empty[s]), ph, abort_flag, p.status, JB200_STATUS_GEMM_DECODE)) { ok = false; return; }
           tc_fence_after_sync();
           __syncwarp();
         }
-        tmem_st_32x32(a_lane + uint32_t(s) * (CK * KB_COLS), v);
+#pragma unroll 1
+        for (int h = 0; h < CK; h += 2) {
+          uint32_t w[4], v[32];
+          const uint32_t piece = uint32_t(in_box * CK + h + par) ^ uint32_t(r & 7);       // 128-byte swizzle: no bank conflicts
+          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(code_row + uint32_t(box) * BOX_BYTES + (piece << 4)) : "memory");
+#pragma unroll
+          for (int i = 0; i < 4; ++i) decode16_prepared(w[i], v + 8 * i);
+          tmem_st_32x32(a_lane + uint32_t(s * CK + h) * KB_COLS, v);
+        }
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctl.full[s]));
         if (++s == S) { s = 0; ph ^= 1u; }
-        if ((c & (BOX_CHUNKS - 1)) == BOX_CHUNKS - 1 || c + 1 == n_ch) {          // the box has been read
+        if (in_box == BOX_CHUNKS - 1 || c + 1 == n_ch) {          // the box has been read
           if (lane == 0) mbar_arrive(smem_u32(&ctl.code_empty[box]));
           if (++box == p.boxes) { box = 0; box_ph ^= 1u; }
         }
@@ -472,29 +478,31 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
   }
 }
 
-constexpr int RING_SMEM = 222 * 1024;
-inline int chunk_bytes(int bn) { return CK * bn * BK * 2; }
+constexpr int RING_SMEM = 222 * 1024, RING_LEAST = 3;
+inline int chunk_bytes(int bn, int ck) { return ck * bn * BK * 2; }
 inline int code_boxes(int K) { return std::min((K + BOX_KB * BK - 1) / (BOX_KB * BK), MAX_BOXES); }
 // Chunks in flight: weights in what the accumulator leaves of tensor memory, rows in what the codes leave of shared memory.
-inline int ring_chunks(int bn, int K) {
-  return std::min({(int(TMEM_COLS) - acc_cols(bn)) / int(CK * KB_COLS), (RING_SMEM - code_boxes(K) * BOX_BYTES) / chunk_bytes(bn),
-                   MAX_CHUNKS, K / (BK * CK)});
+inline int ring_chunks(int bn, int ck, int K) {
+  return std::min({(int(TMEM_COLS) - acc_cols(bn)) / int(ck * KB_COLS), (RING_SMEM - code_boxes(K) * BOX_BYTES) / chunk_bytes(bn, ck),
+                   MAX_CHUNKS, K / (BK * ck)});
 }
 constexpr size_t LEAST_SMEM = 116 * 1024;      // two CTAs of an SM would only wait for each other's tensor memory
 
 }  // namespace
 
+bool mid_gemm_coarse_fits(int bn, int K) { return K % (BK * CK_MOST) == 0 && ring_chunks(bn, CK_MOST, K) >= RING_LEAST; }
+
 int mid_gemm_least_chunks(int bn, int K) {
-  return std::min({(224 * 1024) / (chunk_bytes(BM) + chunk_bytes(bn)), MAX_CHUNKS, K / (BK * CK)});
+  return std::min({(224 * 1024) / (chunk_bytes(MID_FEATURES, 2) + chunk_bytes(bn, 2)), MAX_CHUNKS, K / (BK * 2)});
 }
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
                     const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
-                    cudaStream_t stream) {
+                    bool coarse, cudaStream_t stream) {
   JB_REQUIRE(epilogue == JB200_EPI_BF16 || epilogue == JB200_EPI_GELU_BF16 || epilogue == JB200_EPI_RESID_F32, "mid_gemm: epilogue %d", epilogue);
-  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * CK) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn % 16 == 0 &&
+  JB_REQUIRE(M >= 1 && N % BM == 0 && K % (BK * 2) == 0 && alpha_rows % BM == 0 && bn >= 16 && bn % 16 == 0 &&
                  bn_max >= bn && bn_max <= 256 && bn_max % 16 == 0 &&
-                 G >= 1 && G <= MAX_GROUPS,
+                 G >= 1 && G <= MAX_GROUPS && (!coarse || mid_gemm_coarse_fits(bn_max, K)),
              "mid_gemm: bad shape (M=%d, N=%d, K=%d, bn=%d)", M, N, K, bn);
   MidParams p;
   p.alpha = alpha; p.seg = seg; p.counts = counts; p.routes = routes ? *routes : MidRoutes{}; p.out = out;
@@ -505,16 +513,16 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   p.boxes = code_boxes(K);
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
-  const int n_kb = K / BK;
-  Maps maps;                                   // [K-block][token][64]: one copy takes the same rows of CK K-blocks
+  const int n_kb = K / BK, ck = coarse ? CK_MOST : 2;
+  Maps maps;                                   // [K-block][token][64]: one copy takes the same rows of ck K-blocks
   const cuuint64_t gdim[3] = {cuuint64_t(BK), cuuint64_t(M), cuuint64_t(n_kb)};
   const cuuint64_t gstride[2] = {cuuint64_t(K) * 2, cuuint64_t(BK) * 2};
   size_t smem = LEAST_SMEM;
   for (int i = 0; i < 3; ++i) {
     p.bn[i] = i == 0 ? bn : i == 1 ? (bn + bn_max) / 32 * 16 : bn_max;
-    p.chunks[i] = ring_chunks(p.bn[i], K);
-    smem = std::max(smem, size_t(p.boxes) * BOX_BYTES + size_t(p.chunks[i]) * chunk_bytes(p.bn[i]) + 1024);
-    const cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(p.bn[i]), cuuint32_t(CK)};
+    p.chunks[i] = ring_chunks(p.bn[i], ck, K);
+    smem = std::max(smem, size_t(p.boxes) * BOX_BYTES + size_t(p.chunks[i]) * chunk_bytes(p.bn[i], ck) + 1024);
+    const cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(p.bn[i]), cuuint32_t(ck)};
     const int rc = encode_tiled(&maps.x[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, x_bf16, gdim, gstride, box,
                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "mid_gemm");
     if (rc != JB200_OK) return rc;
@@ -534,10 +542,11 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
     if (rc == JB200_OK) launch_dep(kernel, grid, route == 1 ? THREADS + 32 : THREADS, smem, stream, maps, p);
     return rc;
   };
-  static std::atomic<unsigned long long> set_up[3];
-  const int rc = route == 0   ? launch(mid_gemm_kernel<0>, set_up)
-                 : route == 1 ? launch(mid_gemm_kernel<1>, set_up + 1)
-                              : launch(mid_gemm_kernel<2>, set_up + 2);
+  static std::atomic<unsigned long long> set_up[6];
+  auto pick = [&](auto two, auto four, std::atomic<unsigned long long>* done) { return ck == 2 ? launch(two, done) : launch(four, done + 1); };
+  const int rc = route == 0   ? pick(mid_gemm_kernel<0, 2>, mid_gemm_kernel<0, 4>, set_up)
+                 : route == 1 ? pick(mid_gemm_kernel<1, 2>, mid_gemm_kernel<1, 4>, set_up + 2)
+                              : pick(mid_gemm_kernel<2, 2>, mid_gemm_kernel<2, 4>, set_up + 4);
   if (rc != JB200_OK) return rc;
   JB_LAUNCH_CHECK("mid_gemm_kernel");
   return JB200_OK;
