@@ -366,14 +366,6 @@ inline void launch_dep(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
   (void)cudaLaunchKernelEx(&cfg, kernel, KArgs(static_cast<Args&&>(args))...);   // errors: cudaGetLastError in JB_LAUNCH_CHECK
 }
 
-// Reads n floats into this SM's L1 (a word of every 128-byte line), for use after the grid dependency.
-__device__ __forceinline__ void touch_floats(const float* p, int n) {
-  for (int i = int(threadIdx.x) * 32; i < n; i += int(blockDim.x) * 32) {
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p + i));
-  }
-}
-
 // Same for a grid of thread-block clusters (grid.x a multiple of `cluster`).
 template <typename... KArgs, typename... Args>
 inline void launch_dep_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t stream,
@@ -408,14 +400,13 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t smem_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
   return a;
 }
-__device__ __forceinline__ void cluster_st_f64(uint32_t addr, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+// 16 bytes into another CTA, counted by an mbarrier there.
+__device__ __forceinline__ void st_async16(uint32_t addr, uint32_t bar, uint4 v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
+               ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void cluster_st_64(uint32_t addr, float2 v) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
-}
-__device__ __forceinline__ void cluster_st_128(uint32_t addr, uint4 v) {
-  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
 #endif  // __CUDACC__

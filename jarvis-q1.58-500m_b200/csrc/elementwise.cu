@@ -38,15 +38,22 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* p, const fl
 }
 
 // One warp per row; the row is kept in registers between the two passes when C <= 8*32*MAXV.
-template <typename TIn, typename TOut, int MAXV>
+// AHEAD: the weight was complete before the kernel ahead of this one started, and is in registers when the rows come.  (Read into L1 in
+// time it was gone behind the grid dependency.)
+template <typename TIn, typename TOut, int MAXV, bool AHEAD>
 __global__ void __launch_bounds__(ROW_THREADS) rmsnorm_kernel(const TIn* __restrict__ x, const float* __restrict__ w,
-                                                              float eps, TOut* __restrict__ y, int n_rows, int C, bool ahead) {
-  if (ahead) touch_floats(w, C);           // the weight was complete before the kernel ahead of this one started
+                                                              float eps, TOut* __restrict__ y, int n_rows, int C) {
+  const int row = blockIdx.x * (ROW_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  float wk[AHEAD ? MAXV : 1][8];
+  if constexpr (AHEAD) {
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i)
+      if ((i * 32 + lane) * 8 < C) load8<float>(w + (i * 32 + lane) * 8, wk[i]);
+  }
+  __syncwarp();
   pdl_wait();
   pdl_trigger();
-  const int row = blockIdx.x * (ROW_THREADS / 32) + (threadIdx.x >> 5);
   if (row >= n_rows) return;
-  const int lane = threadIdx.x & 31;
   const TIn* xr = x + size_t(row) * C;
   TOut* yr = y + size_t(row) * C;
   float v[MAXV][8];
@@ -67,9 +74,9 @@ __global__ void __launch_bounds__(ROW_THREADS) rmsnorm_kernel(const TIn* __restr
     const int c = (i * 32 + lane) * 8;
     if (c < C) {
       float wv[8], o[8];
-      load8<float>(w + c, wv);
+      if (!AHEAD) load8<float>(w + c, wv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = v[i][j] * r * wv[j];
+      for (int j = 0; j < 8; ++j) o[j] = v[i][j] * r * (AHEAD ? wk[AHEAD ? i : 0][j] : wv[j]);
       store8<TOut>(yr + c, o);
     }
   }
@@ -93,12 +100,10 @@ __global__ void __launch_bounds__(ROW_THREADS) embedding_kernel(const int64_t* _
 template <typename TIn, typename TOut>
 int launch_rmsnorm_t(const void* x, const float* w, float eps, void* y, int n_rows, int C, bool ahead, cudaStream_t stream) {
   const int blocks = (n_rows + ROW_THREADS / 32 - 1) / (ROW_THREADS / 32);
-  if (C <= 1024)
-    launch_dep(rmsnorm_kernel<TIn, TOut, 4>, blocks, ROW_THREADS, 0, stream, reinterpret_cast<const TIn*>(x), w, eps,
-               reinterpret_cast<TOut*>(y), n_rows, C, ahead);
-  else
-    launch_dep(rmsnorm_kernel<TIn, TOut, 16>, blocks, ROW_THREADS, 0, stream, reinterpret_cast<const TIn*>(x), w, eps,
-               reinterpret_cast<TOut*>(y), n_rows, C, ahead);
+  // (beyond a wave of CTAs the registers are better spent on more of them)
+  auto kernel = C > 1024 ? rmsnorm_kernel<TIn, TOut, 16, false>
+                         : ahead && n_rows <= 4096 ? rmsnorm_kernel<TIn, TOut, 4, true> : rmsnorm_kernel<TIn, TOut, 4, false>;
+  launch_dep(kernel, blocks, ROW_THREADS, 0, stream, reinterpret_cast<const TIn*>(x), w, eps, reinterpret_cast<TOut*>(y), n_rows, C);
   JB_LAUNCH_CHECK("rmsnorm_kernel");
   return JB200_OK;
 }

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(256) lsf_step_norm_kernel(const LsfStepParams 
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const bool scalars = blockIdx.x == gridDim.x - 1, on = !scalars && row < p.B;
   const size_t base = size_t(row) * p.C;
-  float4 hq[4][2], xq[4][2];
+  float4 hq[4][2], xq[4][2], wq[4][2];
   auto fetch = [&] {
     if (!on) return;
 #pragma unroll
@@ -329,6 +329,7 @@ __global__ void __launch_bounds__(256) lsf_step_norm_kernel(const LsfStepParams 
         for (int q = 0; q < 2; ++q) {
           hq[i][q] = p.h_in ? *reinterpret_cast<const float4*>(p.h_in + base + c + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
           xq[i][q] = *reinterpret_cast<const float4*>(p.x + base + c + 4 * q);
+          if (p.w_norm) wq[i][q] = __ldg(reinterpret_cast<const float4*>(p.w_norm + c) + q);
         }
       }
     }
@@ -374,7 +375,7 @@ __global__ void __launch_bounds__(256) lsf_step_norm_kernel(const LsfStepParams 
   for (int i = 0; i < 4; ++i) {
     const int c = (i * 32 + lane) * 8;
     if (c < p.C) {
-      const float4 wa = __ldg(reinterpret_cast<const float4*>(p.w_norm + c)), wb = __ldg(reinterpret_cast<const float4*>(p.w_norm + c + 4));
+      const float4 wa = wq[i][0], wb = wq[i][1];
       *reinterpret_cast<uint4*>(p.xn + base + c) =
           make_uint4(pack_bf16x2(v[i][0] * r * wa.x, v[i][1] * r * wa.y), pack_bf16x2(v[i][2] * r * wa.z, v[i][3] * r * wa.w),
                      pack_bf16x2(v[i][4] * r * wb.x, v[i][5] * r * wb.y), pack_bf16x2(v[i][6] * r * wb.z, v[i][7] * r * wb.w));

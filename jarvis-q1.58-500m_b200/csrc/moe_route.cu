@@ -92,12 +92,12 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
                       int64_t* __restrict__ topk_idx, float* __restrict__ gates,
                       double* __restrict__ probs_sum, int* __restrict__ top1_hist, int* __restrict__ load,
                       unsigned long long* __restrict__ counts8, bool ahead) {
-  extern __shared__ float w_s[];  // [E][C]
+  extern __shared__ float w_s[];  // [E][C], [C]
   __shared__ float p_acc[ROUTER_THREADS / 32][E];
   __shared__ int h_acc[E], l_acc[E];
   auto stage = [&] {
     for (int i = threadIdx.x; i < E * C; i += ROUTER_THREADS) w_s[(i / C) * C + router_w_index(i % C)] = __ldg(w_router + i);
-    touch_floats(w_norm, C);
+    for (int i = threadIdx.x; i < C; i += ROUTER_THREADS) w_s[E * C + i] = __ldg(w_norm + i);
   };
   if (threadIdx.x < E) h_acc[threadIdx.x] = l_acc[threadIdx.x] = 0;
   if (ahead) stage();
@@ -152,8 +152,7 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
     for (int i = 0; i < 4; ++i) {
       const int c = (i * 32 + lane) * 8;
       if (c < C) {
-        const float4 wa = __ldg(reinterpret_cast<const float4*>(w_norm + c));
-        const float4 wb = __ldg(reinterpret_cast<const float4*>(w_norm + c) + 1);
+        const float4 wa = *reinterpret_cast<const float4*>(w_s + E * C + c), wb = *reinterpret_cast<const float4*>(w_s + E * C + c + 4);
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
           const uint4 pk = make_uint4(pack_bf16x2(v[k][i][0] * r[k] * wa.x, v[k][i][1] * r[k] * wa.y),
@@ -705,7 +704,7 @@ int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* 
   const int warps = ROUTER_THREADS / 32, per = n_tokens <= 2 * sms * warps ? 1 : 2;
   const int blocks = std::min((n_tokens + per * warps - 1) / (per * warps), 2 * sms);
   JB_REQUIRE(!counts8 || (per == 1 && load), "rmsnorm_router: counts of eight tokens need a single pass");
-  const size_t smem = size_t(E) * C * sizeof(float);
+  const size_t smem = size_t(E + 1) * C * sizeof(float);      // the router's rows and the norm's
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
   auto kernel = per == 1 ? (E == 4 ? rmsnorm_router_kernel<4, 1> : rmsnorm_router_kernel<8, 1>)
                          : (E == 4 ? rmsnorm_router_kernel<4, 2> : rmsnorm_router_kernel<8, 2>);

@@ -146,6 +146,7 @@ struct TailParams {
   float eps;
   __nv_bfloat16* xn;           // [N][C]
   int B, T, N, C;
+  unsigned int* status;
 };
 
 constexpr int MAX_CTAS = 16;                           // non-portable cluster size: asked for before use (tail_fits)
@@ -176,70 +177,91 @@ __device__ __forceinline__ Combined combine_row(const TailParams& p, int a, int 
   return combine_values(ya, yb, g, lane, p.C, put);
 }
 
-// Sums of the CTA's tokens (one per warp) -> every CTA of the cluster -> the decay of the call, the same bits everywhere.
-// Called by all threads after one cluster_arrive(); whatever `push` writes to other CTAs is visible to them when this
-// returns.
+// Exchange of the sums: 16 bytes from every CTA, and whatever rows come with them, counted by an mbarrier of the receiver (a cluster
+// barrier waits for all stores of all its threads as well: 0.6 us against 0.3).
+struct TailShared {
+  alignas(16) double part[MAX_WARPS][2], all[MAX_CTAS][2];
+  uint64_t bar;
+  uint32_t abort_flag;
+};
+struct Decay {
+  float alpha, mean, var;
+};
+__device__ __noinline__ void tail_wait_long(uint32_t bar, volatile uint32_t* abort_flag, unsigned int* status) {
+  (void)mbar_wait(bar, 0u, abort_flag, status, JB200_STATUS_LSF_LOAD);
+}
+// Ahead of everything else; the CTAs of a cluster have all done it behind the cluster_wait() of tail_decay.
+__device__ __forceinline__ void tail_begin(TailShared& s, int n_cta, uint32_t row_bytes) {
+  if (n_cta == 1) return;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&s.bar), 1);
+    s.abort_flag = 0;
+    fence_mbar_init();
+    mbar_arrive_expect_tx(smem_u32(&s.bar), uint32_t(n_cta) * 16u + row_bytes);
+  }
+  __syncwarp();
+  cluster_arrive();
+}
+
+// Sums of the CTA's tokens (one per warp) -> every CTA of the cluster -> the decay of the call, the same bits in every warp.
+// Called by all threads; what `push` sends to other CTAs on their `bar` is there when this returns.
 template <typename F>
-__device__ __forceinline__ float tail_decay(const TailParams& p, Combined c, float var_scale, double (*part)[2], double (*all)[2],
-                                            float* s_alpha, int rank, int n_cta, F&& push) {
+__device__ __forceinline__ Decay tail_decay(const TailParams& p, Combined c, float var_scale, TailShared& s, int rank, int n_cta, F&& push) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
-  if (lane == 0) { part[warp][0] = double(c.s1); part[warp][1] = double(c.s2); }
+  if (lane == 0) { s.part[warp][0] = double(c.s1); s.part[warp][1] = double(c.s2); }
   if (n_cta > 1) cluster_wait();               // the other CTAs have started: their shared memory may be written
   push();
   __syncthreads();
   if (warp == 0) {
-    double a = lane < n_warps ? part[lane][0] : 0.0, b = lane < n_warps ? part[lane][1] : 0.0;
+    double a = lane < n_warps ? s.part[lane][0] : 0.0, b = lane < n_warps ? s.part[lane][1] : 0.0;
     for (int o = n_warps > 8 ? 8 : n_warps > 4 ? 4 : n_warps > 2 ? 2 : n_warps >> 1; o > 0; o >>= 1) {        // lanes from n_warps on are zeros
       a += __shfl_xor_sync(0xffffffffu, a, o);
       b += __shfl_xor_sync(0xffffffffu, b, o);
     }
     a = __shfl_sync(0xffffffffu, a, 0);
     b = __shfl_sync(0xffffffffu, b, 0);
-    if (n_cta > 1) {
-      if (lane < 2 * n_cta)
-        cluster_st_f64(cluster_map(smem_u32(&all[rank][lane & 1]), uint32_t(lane >> 1)), (lane & 1) ? b : a);
-    } else if (lane == 0) {
-      all[0][0] = a;
-      all[0][1] = b;
+    if (n_cta == 1) {
+      if (lane == 0) { s.all[0][0] = a; s.all[0][1] = b; }
+    } else if (lane < n_cta) {
+      st_async16(cluster_map(smem_u32(&s.all[rank][0]), uint32_t(lane)), cluster_map(smem_u32(&s.bar), uint32_t(lane)),
+                 make_uint4(uint32_t(__double2loint(a)), uint32_t(__double2hiint(a)), uint32_t(__double2loint(b)), uint32_t(__double2hiint(b))));
     }
   }
-  if (n_cta > 1) {
-    __syncwarp();
-    cluster_arrive();
-    cluster_wait();
+  if (n_cta == 1) __syncthreads();
+  else if (!mbar_try_wait(smem_u32(&s.bar), 0u)) tail_wait_long(smem_u32(&s.bar), &s.abort_flag, p.status);
+  __syncwarp();
+  double sum = lane < n_cta ? s.all[lane][0] : 0.0, sq = lane < n_cta ? s.all[lane][1] : 0.0;
+  for (int o = n_cta > 8 ? 8 : 4; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    sq += __shfl_xor_sync(0xffffffffu, sq, o);
   }
-  if (warp == 0) {
-    __syncwarp();
-    double s[2];
-    s[0] = lane < n_cta ? all[lane][0] : 0.0;
-    s[1] = lane < n_cta ? all[lane][1] : 0.0;
-    for (int o = n_cta > 8 ? 8 : 4; o > 0; o >>= 1) {
-      s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-      s[1] += __shfl_xor_sync(0xffffffffu, s[1], o);
-    }
-    if (lane == 0) {
-      const float2 mv = moe_act_mean_var(s[0], s[1], p.st.n_el, p.st.inv_el, p.st.inv_el1);
-      *s_alpha = lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, mv.y);
-      if (rank == 0) {
-        p.st.scalars[1] = mv.x;
-        p.st.scalars[2] = mv.y;
-        if (p.st.reflect) *p.st.reflect = reflect_penalty(p.st.lam, p.st.tau, __ldg(p.st.mu), mv.x, mv.y);
-      }
-    }
-  }
-  __syncthreads();
-  return *s_alpha;
+  const float2 mv = moe_act_mean_var(__shfl_sync(0xffffffffu, sum, 0), __shfl_sync(0xffffffffu, sq, 0), p.st.n_el, p.st.inv_el, p.st.inv_el1);
+  return {lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, mv.y), mv.x, mv.y};
+}
+// The norm's weight, on its way while the kernel ahead runs (what a thread has read into L1 by then is gone behind the grid dependency: read
+// from global memory at the end, the weight took 1.9 us).
+__device__ __forceinline__ void copy_norm(const TailParams& p, float* s_norm) {
+  if (!p.w_norm) return;
+  for (int i = threadIdx.x; i < p.C / 4; i += blockDim.x) copy_async_16(smem_u32(s_norm + 4 * i), p.w_norm + 4 * i);
+}
+// The layer's scalars, by one thread of the cluster that has little else to do.
+__device__ __forceinline__ void tail_scalars(const TailParams& p, float l_bal, float mu, Decay d) {
+  p.st.scalars[0] = l_bal;
+  p.st.scalars[1] = d.mean;
+  p.st.scalars[2] = d.var;
+  if (p.st.reflect) *p.st.reflect = reflect_penalty(p.st.lam, p.st.tau, mu, d.mean, d.var);
 }
 
 // One token per sequence (decode): a warp per token, its row in registers throughout.
 __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailParams p, const int n_cta) {
-  __shared__ double s_part[MAX_WARPS][2], s_all[MAX_CTAS][2];
-  __shared__ float s_alpha;
+  __shared__ TailShared sh;
+  __shared__ __align__(16) float s_norm[GROUPS * 256];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = n_cta > 1 ? int(cluster_rank()) : 0;
   const int n = rank + warp * n_cta;
   const bool on = n < p.N;
-  if (n_cta > 1) cluster_arrive();
+  tail_begin(sh, n_cta, 0u);
+  copy_norm(p, s_norm);
   const float var_scale = __ldg(p.var_scale);
   float x[GROUPS][8], h[GROUPS][8];
   int2 sl = make_int2(0, 0);
@@ -261,18 +283,22 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailPar
       }
     }
   }
-  float l_bal = 0.f;
-  if (rank == 0 && tid == int(blockDim.x) - 1)
+  float l_bal = 0.f, mu = 0.f;
+  if (rank == 0 && tid == int(blockDim.x) - 1) {
     l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.st.inv_tok, p.st.balance_alpha);
+    if (p.st.reflect) mu = __ldg(p.st.mu);
+  }
   __syncwarp();
   pdl_wait();
   pdl_trigger();
 
+  copy_async_wait();             // visible to all behind the first barrier of tail_decay
   uint4 m[GROUPS];
   Combined c = {0.f, 0.f};
   if (on) c = combine_row(p, sl.x, sl.y, g, lane, [&](int i, uint4 v) { m[i] = v; });
-  const float alpha = tail_decay(p, c, var_scale, s_part, s_all, &s_alpha, rank, n_cta, [] {});
-  if (rank == 0 && tid == int(blockDim.x) - 1) p.st.scalars[0] = l_bal;
+  const Decay d = tail_decay(p, c, var_scale, sh, rank, n_cta, [] {});
+  const float alpha = d.alpha;
+  if (rank == 0 && tid == int(blockDim.x) - 1) tail_scalars(p, l_bal, mu, d);
   if (!on) return;
   float ss = 0.f;
 #pragma unroll
@@ -298,7 +324,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailPar
     const int ch = (i * 32 + lane) * 8;
     if (ch < p.C)
       *reinterpret_cast<uint4*>(p.xn + size_t(n) * p.C + ch) =
-          norm8(x[i], r, __ldg(reinterpret_cast<const float4*>(p.w_norm + ch)), __ldg(reinterpret_cast<const float4*>(p.w_norm + ch) + 1));
+          norm8(x[i], r, *reinterpret_cast<const float4*>(s_norm + ch), *reinterpret_cast<const float4*>(s_norm + ch + 4));
   }
 }
 
@@ -315,8 +341,8 @@ constexpr int SCAN_CH = 64, RUN = 16;          // channels per CTA, two per lane
 
 __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailParams p, const int n_cta) {
   extern __shared__ __align__(16) uint8_t tail_smem[];
-  __shared__ double s_part[MAX_WARPS][2], s_all[MAX_CTAS][2];
-  __shared__ float s_alpha;
+  __shared__ TailShared sh;
+  __shared__ __align__(16) float s_norm[GROUPS * 256];
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, n_warps = blockDim.x >> 5;
   const int N = p.N, B = p.B, T = p.T, C = p.C;
   const int rank = int(cluster_rank());
@@ -331,7 +357,8 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   float* ends = xr + size_t((N + n_cta - 1) / n_cta) * C;
   const int own = rank + warp * n_cta;                                         // this warp's token
   const bool on = own < N;
-  cluster_arrive();
+  tail_begin(sh, n_cta, uint32_t(N) * (SCAN_CH * 2));
+  copy_norm(p, s_norm);
   const float var_scale = __ldg(p.var_scale);
   int2 sl = make_int2(0, 0);
   float2 g = make_float2(0.f, 0.f);
@@ -347,9 +374,11 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
     reinterpret_cast<float4*>(hs)[i] =
         p.h_in ? *(reinterpret_cast<const float4*>(p.h_in + size_t(b) * C + rank * SCAN_CH) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  float l_bal = 0.f;
-  if (rank == 0 && tid == int(blockDim.x) - 1)
+  float l_bal = 0.f, mu = 0.f;
+  if (rank == 0 && tid == int(blockDim.x) - 1) {
     l_bal = moe_l_balance(p.st.probs_sum, p.st.top1_hist, p.st.E, p.st.inv_tok, p.st.balance_alpha);
+    if (p.st.reflect) mu = __ldg(p.st.mu);
+  }
   __syncwarp();
   pdl_wait();
   pdl_trigger();
@@ -357,18 +386,19 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   uint4 m[GROUPS];
   Combined cm = {0.f, 0.f};
   if (on) cm = combine_row(p, sl.x, sl.y, g, lane, [&](int i, uint4 v) { m[i] = v; });
-  const float alpha = tail_decay(p, cm, var_scale, s_part, s_all, &s_alpha, rank, n_cta, [&] {
+  const Decay d = tail_decay(p, cm, var_scale, sh, rank, n_cta, [&] {
     if (on) {
 #pragma unroll
       for (int i = 0; i < GROUPS; ++i) {
         const int c = (i * 32 + lane) * 8;
-        if (c < C) cluster_st_128(cluster_map(smem_u32(ms) + uint32_t(own) * (SCAN_CH * 2) + uint32_t(c % SCAN_CH) * 2u, uint32_t(c / SCAN_CH)), m[i]);
+        const uint32_t to = uint32_t(c / SCAN_CH);
+        if (c < C) st_async16(cluster_map(smem_u32(ms) + uint32_t(own) * (SCAN_CH * 2) + uint32_t(c % SCAN_CH) * 2u, to), cluster_map(smem_u32(&sh.bar), to), m[i]);
       }
     }
   });
-  if (rank == 0 && tid == int(blockDim.x) - 1) p.st.scalars[0] = l_bal;
+  if (rank == 0 && tid == int(blockDim.x) - 1) tail_scalars(p, l_bal, mu, d);
 
-  const float one_m = 1.0f - alpha;
+  const float alpha = d.alpha, one_m = 1.0f - alpha;
   float whole = alpha;                                       // alpha to the power of a run's length
 #pragma unroll
   for (int i = 1; i < RUN; ++i) whole *= alpha;
@@ -440,17 +470,6 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
       }
     }
   }
-  float4 wn[GROUPS][2];
-  if (p.w_norm) {
-#pragma unroll
-    for (int i = 0; i < GROUPS; ++i) {
-      const int c = (i * 32 + lane) * 8;
-      if (c < C) {
-        wn[i][0] = __ldg(reinterpret_cast<const float4*>(p.w_norm + c));
-        wn[i][1] = __ldg(reinterpret_cast<const float4*>(p.w_norm + c) + 1);
-      }
-    }
-  }
   __syncwarp();
   cluster_arrive();
   cluster_wait();
@@ -473,7 +492,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
 #pragma unroll
   for (int i = 0; i < GROUPS; ++i) {
     const int c = (i * 32 + lane) * 8;
-    if (c < C) *reinterpret_cast<uint4*>(p.xn + size_t(own) * C + c) = norm8(v[i], r, wn[i][0], wn[i][1]);
+    if (c < C) *reinterpret_cast<uint4*>(p.xn + size_t(own) * C + c) = norm8(v[i], r, *reinterpret_cast<const float4*>(s_norm + c), *reinterpret_cast<const float4*>(s_norm + c + 4));
   }
 }
 
@@ -594,6 +613,8 @@ int launch_tail(const void* y_bf16, const float* gates, const int* scatter, cons
   p.h_in = h_in; p.h_out = h_out; p.x = x; p.w_norm = w_norm; p.eps = eps;
   p.xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
   p.B = B; p.T = T; p.N = N; p.C = C;
+  p.status = device_status_ptr();
+  if (!p.status) return JB200_ERR_CUDA;
   if (T == 1) {
     // a lone CTA while its SM can take the rows (4 KB in, 10 KB out each), else sixteen (steps of 64 and 128 sequences, 24 layers
     // and head, in eight 876 and 1127 us, so 848 and 1065), or eight where a cluster cannot have more
