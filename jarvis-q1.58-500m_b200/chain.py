@@ -271,8 +271,17 @@ def _results(n, given, inplace, shape, dev):
 
 class Result:
     """What a call leaves: h / S (lists, one tensor per layer; S None when not wanted), scalars f32 (n, 3), reflect f32 (n,)
-    and hidden (normalised rows after the last layer, bf16)."""
-    __slots__ = ("h", "S", "scalars", "reflect", "hidden")
+    and hidden (normalised rows after the last layer, bf16).  scalars and reflect are views of aux (3 n, then n values), made when
+    somebody looks: a view is a microsecond of a block's call."""
+    __slots__ = ("h", "S", "aux", "has_reflect", "hidden")
+
+    @property
+    def scalars(self):
+        return self.aux[:self.aux.numel() // 4 * 3].view(-1, 3)
+
+    @property
+    def reflect(self):
+        return self.aux[self.aux.numel() // 4 * 3:] if self.has_reflect else None
 
 
 def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0, max_position=None, h_in=None, s_in=None,
@@ -298,8 +307,8 @@ def run(tab: LayerTable, x, B: int, T: int, *, ids=None, table=None, start_pos=0
     work = torch.empty(head + ws_bytes, dtype=torch.uint8, device=dev)
     routing = torch.empty(n * routing_bytes, dtype=torch.uint8, device=dev)
     res = Result()
-    aux = torch.empty(4 * n, dtype=torch.float32, device=dev)
-    res.scalars, res.reflect = aux[:3 * n].view(n, 3), aux[3 * n:] if tab.has_reflect else None
+    aux = res.aux = torch.empty(4 * n, dtype=torch.float32, device=dev)
+    res.has_reflect = tab.has_reflect
     f = _lib.Forward()
     f.B, f.T, f.C, f.H, f.E, f.hidden = B, T, tab.C, tab.H, tab.E, tab.hidden
     if ids is not None:

@@ -81,7 +81,7 @@ struct MapEntry {
   MapKey key;
   CUtensorMap map;
 };
-constexpr int MAP_CACHE = 64;
+constexpr int MAP_CACHE = 256;      // a forward of 24 layers uses some 110, 96 of them for its weights
 thread_local MapEntry g_maps[MAP_CACHE];   // zero keys match nothing: rank is never 0
 }  // namespace
 

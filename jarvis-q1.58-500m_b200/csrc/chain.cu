@@ -212,15 +212,10 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
                            all_rows && G > 1 ? (epi == JB200_EPI_GELU_BF16 ? w1_coarse : w2_coarse) : coarse, st);
   };
 
-  // the accumulators and the router's work counters are one block: cleared by the embedding kernel, or by themselves
+  // the accumulators and the router's work counters are one block: cleared by the first kernel
   uint8_t* acc0 = static_cast<uint8_t*>(f->accumulators);
   const size_t acc_stride = accumulator_bytes(E);
-  if (f->ids) {
-    JB_TRY(launch_embed_norm(f->ids, f->table, f->vocab, layers[0].w_norm1, layers[0].eps1, x, xn, N, C, acc0, n_layers * acc_stride, st));
-  } else {
-    JB_CUDA(cudaMemsetAsync(acc0, 0, n_layers * acc_stride, st));
-    JB_TRY(launch_rmsnorm(x, 0, layers[0].w_norm1, layers[0].eps1, xn, 1, N, C, st));
-  }
+  JB_TRY(launch_embed_norm(f->ids, f->table, f->vocab, layers[0].w_norm1, layers[0].eps1, x, xn, N, C, acc0, n_layers * acc_stride, st));
 
   for (int l = 0; l < n_layers; ++l) {
     const jb200_layer& p = layers[l];

@@ -522,6 +522,10 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
     p.bn[i] = i == 0 ? bn : i == 1 ? (bn + bn_max) / 32 * 16 : bn_max;
     p.chunks[i] = ring_chunks(p.bn[i], ck, K);
     smem = std::max(smem, size_t(p.boxes) * BOX_BYTES + size_t(p.chunks[i]) * chunk_bytes(p.bn[i], ck) + 1024);
+    if (i > 0 && p.bn[i] == p.bn[i - 1]) {
+      maps.x[i] = maps.x[i - 1];
+      continue;
+    }
     const cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(p.bn[i]), cuuint32_t(ck)};
     const int rc = encode_tiled(&maps.x[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, x_bf16, gdim, gstride, box,
                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, "mid_gemm");

@@ -531,7 +531,8 @@ bool tail_fits(int n_cta) {
 }
 
 // Embedding rows into the f32 residual stream (jarvis_model.py:498) and, while they are in registers, norm1 of the first
-// block; clears the chain's accumulators on the way.  One warp per token, C <= 1024.
+// block; clears the chain's accumulators on the way.  One warp per token, C <= 1024.  Without ids the rows are there already.
+template <bool IDS>
 __global__ void __launch_bounds__(256)
 embed_norm_kernel(const int64_t* __restrict__ ids, const float* __restrict__ table, int vocab, const float* __restrict__ w_norm,
                   float eps, float* __restrict__ x, __nv_bfloat16* __restrict__ xn, int n_rows, int C, uint32_t* __restrict__ zero,
@@ -542,9 +543,12 @@ embed_norm_kernel(const int64_t* __restrict__ ids, const float* __restrict__ tab
   for (int i = gtid; i < n_zero; i += gridDim.x * 256) zero[i] = 0u;
   const int row = gtid >> 5, lane = threadIdx.x & 31;
   if (row >= n_rows) return;
-  long long id = ids[row];
-  id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);            // clamp instead of faulting on a bad id
-  const float* src = table + size_t(id) * C;
+  const float* src = x + size_t(row) * C;
+  if constexpr (IDS) {
+    long long id = ids[row];
+    id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);          // clamp instead of faulting on a bad id
+    src = table + size_t(id) * C;
+  }
   float v[GROUPS][8], ss = 0.f;
 #pragma unroll
   for (int i = 0; i < GROUPS; ++i) {
@@ -555,7 +559,7 @@ embed_norm_kernel(const int64_t* __restrict__ ids, const float* __restrict__ tab
   for (int i = 0; i < GROUPS; ++i) {
     const int c = (i * 32 + lane) * 8;
     if (c < C) {
-      store8(x + size_t(row) * C + c, v[i]);
+      if (IDS) store8(x + size_t(row) * C + c, v[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) ss = __fmaf_rn(v[i][j], v[i][j], ss);
     }
@@ -575,10 +579,10 @@ embed_norm_kernel(const int64_t* __restrict__ ids, const float* __restrict__ tab
 
 int launch_embed_norm(const int64_t* ids, const float* table, int vocab, const float* w_norm, float eps, float* x, void* xn_bf16,
                       int n_rows, int C, void* zero, size_t zero_bytes, cudaStream_t stream) {
-  JB_REQUIRE(ids && table && w_norm && x && xn_bf16 && vocab > 0 && n_rows > 0, "embed_norm: null pointer or empty");
+  JB_REQUIRE((!ids || (table && vocab > 0)) && w_norm && x && xn_bf16 && n_rows > 0, "embed_norm: null pointer or empty");
   JB_REQUIRE(C % 8 == 0 && C <= 1024 && zero_bytes % 4 == 0, "embed_norm: row length %d", C);
   JB_REQUIRE(aligned16(table) && aligned16(x) && aligned16(xn_bf16) && aligned16(w_norm), "embed_norm: pointers must be 16-byte aligned");
-  launch_dep(embed_norm_kernel, (n_rows + 7) / 8, 256, 0, stream, ids, table, vocab, w_norm, eps, x,
+  launch_dep(ids ? embed_norm_kernel<true> : embed_norm_kernel<false>, (n_rows + 7) / 8, 256, 0, stream, ids, table, vocab, w_norm, eps, x,
              reinterpret_cast<__nv_bfloat16*>(xn_bf16), n_rows, C, reinterpret_cast<uint32_t*>(zero), int(zero_bytes / 4));
   JB_LAUNCH_CHECK("embed_norm_kernel");
   return JB200_OK;

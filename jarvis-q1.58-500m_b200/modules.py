@@ -530,7 +530,7 @@ class JarvisBlock(nn.Module):
         tab = chain.table_of(self, [self]) if x.is_cuda else None
         if tab is not None and tab.has_reflect:
             r = self._chain(tab, rows, B, T, h_prev, start_pos)
-            h_last, l_balance, l_reflect = r.h[0], r.scalars[0, 0], r.reflect[0]
+            h_last, l_balance, l_reflect = r.h[0], r.aux[0], r.aux[3]
         else:
             h_last, sc, _ = self.forward_rows(rows, B, T, h_prev, start_pos)
             l_balance, l_reflect = sc[0], self.reflect(sc[1], sc[2])
