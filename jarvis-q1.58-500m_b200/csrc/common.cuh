@@ -344,9 +344,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 // kernel produces) overlap the kernel before it.  The wait returns when the preceding kernel has completed and its
 // writes are visible; the trigger sits after the wait, so a kernel only ever overlaps its immediate predecessor,
 // which itself has passed its own wait: everything older has completed.  Both are no-ops in a kernel launched
-// without the attribute.  One kernel triggers before its wait (route_small_kernel without the sort), where its successor reads ahead
-// nothing that this one or the one before it makes.  Tried elsewhere it gives nothing or takes: successors that come early hold
-// registers and shared memory that the running kernels' next CTAs want (combine 300 tokens +2 %; norm and scans even).
+// without the attribute.  Two short kernels trigger before their wait (the router without the sort and a
+// chain's norm), where the successor reads ahead nothing that they or the kernel before them make; that one triggers behind its wait,
+// so whatever is older is complete.  Tried elsewhere it takes: successors that come early hold registers and shared memory that the
+// running kernels' next CTAs want (combine 300 tokens +2 %; scans even).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
