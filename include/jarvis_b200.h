@@ -466,6 +466,11 @@ void jb200_host_decode16_prepared(uint32_t word, uint32_t* out8);
  * with `sms` multiprocessors: out6 = whether every expert takes all tokens, out-features of a tile, rows of a token tile for experts
  * that are used evenly and at most, and the chunks (of two K-blocks) that either one's ring holds at least.  Runs on the CPU; used by the unit tests.  0: no such call. */
 int jb200_host_expert_tiles(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out6);
+/* How jb200_forward_layers dispatches so many tokens on a device with `sms` multiprocessors: out2 = what makes the maps (0 the router, 1 the
+ * first expert matrix, 2 the dispatch from the ids, 3 the dispatch from the router's counts of every eight tokens, 4 metadata kernels), and
+ * whether the router leaves the experts' assignments, which the first expert matrix then takes as its segments in place of the maps' offsets.
+ * Runs on the CPU; used by the unit tests.  0: no such call. */
+int jb200_host_dispatch_plan(int tokens, int C, int hidden, int sms, int32_t* out2);
 
 #ifdef __cplusplus
 }

@@ -117,6 +117,23 @@ inline MidTile expert_plan(int tokens, bool second, int C, int E, int hidden, in
   return mid_plan(cut ? 2 * tokens : tokens, E, second ? C : hidden, cut, second ? W2_TILES : W1_TILES, sms);
 }
 
+// What makes the dispatch maps of a call (counts, offsets, slots), and whether the router also leaves the assignments of every expert
+// (`load`), from which the first expert matrix takes its segments while maps and rows are made; without them it takes the maps' offsets.  Up
+// to ALL_ROWS_TOKENS there is no dispatch.  Beyond, maps and rows in one launch: from the ids on any device, or, where the router is a single
+// pass of eight tokens a CTA, two CTAs an SM, from the counts that it leaves.  Times of the forms: dispatch_kernel.
+struct Dispatch {
+  enum Maker { ROUTER, EXPERT_GEMM, FROM_IDS, FROM_EIGHTS, METADATA } maps;
+  bool load;
+};
+inline bool small_form(int N, int C, int hidden) { return N <= SMALL_TOKENS && small_gemm_fits(N <= 8 ? 8 : 16, std::max(C, hidden)); }
+inline Dispatch dispatch_plan(int N, bool small, int sms) {
+  static_assert(ROUTE_SMALL_MAX <= DISPATCH_IDS_MAX, "the router of few tokens leaves no counts of eight");
+  if (N <= ALL_ROWS_TOKENS) return {small ? Dispatch::ROUTER : Dispatch::EXPERT_GEMM, false};
+  if (N <= ROUTE_SMALL_MAX) return {Dispatch::FROM_IDS, true};
+  if (N <= std::min(DISPATCH_EIGHTS_MAX, 16 * sms)) return {Dispatch::FROM_EIGHTS, true};
+  return {Dispatch::METADATA, false};
+}
+
 #define JB_TRY(call)                    \
   do {                                  \
     const int rc__ = (call);            \
@@ -132,6 +149,13 @@ int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms,
   out[0] = !second && tokens <= ALL_ROWS_TOKENS;
   out[1] = MID_FEATURES; out[2] = t.bn; out[3] = t.bn_max;
   out[4] = mid_gemm_least_chunks(t.bn, K); out[5] = mid_gemm_least_chunks(t.bn_max, K);
+  return 1;
+}
+
+int dispatch_plan_host(int tokens, int C, int hidden, int sms, int32_t* out) {
+  if (tokens < 1 || C < 128 || hidden < 128 || sms < 1 || !out) return 0;
+  const Dispatch d = dispatch_plan(tokens, small_form(tokens, C, hidden), sms);
+  out[0] = d.maps; out[1] = d.load;
   return 1;
 }
 
@@ -194,10 +218,11 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   uint16_t* disp = qkv;
   float* x = f->x;
   const int small_tile = N <= 8 ? 8 : 16;
-  const bool small = N <= SMALL_TOKENS && small_gemm_fits(small_tile, std::max(C, hidden));   // beyond, the tcgen05 form streams K
+  const bool small = small_form(N, C, hidden);                  // beyond, the tcgen05 form streams K
   const bool mid = !small && N <= MID_TOKENS, all_rows = N <= ALL_ROWS_TOKENS;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
+  const Dispatch by = dispatch_plan(N, small, sms);
   const MidTile qkv_tile = mid_plan(N, 1, 3 * C, false, QKV_TILES, sms), out_tile = mid_plan(N, 1, C, false, OUT_TILES, sms);
   const bool mid_qkv = mid || (!small && mid_wave(N, 3 * C, sms)), mid_out = mid || (!small && mid_wave(N, C, sms));
   const MidTile w1_tile = expert_plan(N, false, C, E, hidden, sms), w2_tile = expert_plan(N, true, C, E, hidden, sms);
@@ -260,21 +285,20 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     // they are behind a fence, a ticket and a second reading of the ids.  24 layers and head as a graph so 80 tokens 1061 -> 1005 us, 128
     // 1139 -> 1098, 5 x 30 1199 -> 1157, steps of 100 sequences 1187 -> 1158; since its epilogue has its rows before the last MMA also
     // 17, 37, 64 tokens 766 -> 759, 780 -> 774, 836 -> 816 and steps of 57 840 -> 835.
-    const bool late_maps = mid && all_rows;
+    const bool late_maps = by.maps == Dispatch::EXPERT_GEMM;
     const MidRoutes store = {idx, false, counts, offs, scatter, gather, gate_idx};
     const MidRoutes rows_of = {idx, true, nullptr, nullptr, nullptr, nullptr, nullptr};
-    // maps and rows in one launch: from the ids, or where the router is a single pass of eight tokens a CTA from the counts it leaves
-    const bool one_launch = !all_rows && N <= std::min(DISPATCH_EIGHTS_MAX, 16 * sms);
-    static_assert(ROUTE_SMALL_MAX <= DISPATCH_IDS_MAX, "the router without counts");
-    unsigned long long* counts8 = one_launch && N > ROUTE_SMALL_MAX ? reinterpret_cast<unsigned long long*>(w + ws.meta) : nullptr;
+    int32_t* router_load = by.load ? load : nullptr;
+    unsigned long long* counts8 = by.maps == Dispatch::FROM_EIGHTS ? reinterpret_cast<unsigned long long*>(w + ws.meta) : nullptr;
     if (N <= ROUTE_SMALL_MAX) {
-      JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, one_launch ? load : nullptr, ticket,
-                                counts, offs, all_rows && !late_maps ? scatter : nullptr, gather, gate_idx, st));
+      JB_TRY(launch_route_small(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, router_load, ticket,
+                                counts, offs, by.maps == Dispatch::ROUTER ? scatter : nullptr, gather, gate_idx, st));
     } else {
       JB_TRY(launch_rmsnorm_router(x, p.w_norm2, p.eps2, xn, p.w_router, N, C, E, idx, gates, acc + 2, hist, st, true,
-                                   one_launch ? load : nullptr, counts8));
-      if (!one_launch) JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
+                                   router_load, counts8));
     }
+    if (by.maps == Dispatch::METADATA)
+      JB_TRY(launch_moe_metadata(idx, N, 2, E, counts, offs, scatter, gather, gate_idx, w + ws.meta, st));
     if (all_rows) {
       // every expert takes all rows where they are and stores the routed ones: no dispatch
       if (small)
@@ -282,12 +306,12 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       else
         JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, nullptr, &store, JB200_EPI_GELU_BF16, hid, w1_tile));
     } else {
-      if (one_launch) JB_TRY(launch_dispatch_chain(idx, counts8, xn, N, C, E, counts, offs, scatter, gather, gate_idx, disp, st));
+      if (by.maps != Dispatch::METADATA) JB_TRY(launch_dispatch_chain(idx, counts8, xn, N, C, E, counts, offs, scatter, gather, gate_idx, disp, st));
       else JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
-        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, nullptr, load, nullptr, JB200_EPI_GELU_BF16, hid, w1_tile));
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, by.load ? nullptr : offs, router_load, nullptr, JB200_EPI_GELU_BF16, hid, w1_tile));
       else
-        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true, one_launch ? load : nullptr));
+        JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true, router_load));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, st));

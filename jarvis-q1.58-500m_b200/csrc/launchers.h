@@ -156,6 +156,7 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
                         cudaStream_t stream, bool* taken);
 int launch_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
                          const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, cudaStream_t stream);
+int dispatch_plan_host(int tokens, int C, int hidden, int sms, int32_t* out);
 int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out);
 size_t accumulator_bytes(int E);
 size_t routing_layout(int N, int E, size_t* offsets);

@@ -316,3 +316,21 @@ def test_expert_tiles_are_no_larger_than_their_rows(E, hidden):
             assert bn <= up(rows + -(-rows // 8))
         assert lib.jb200_host_expert_tiles(tokens, 1, 1024, E, hidden, 148, out) == 1 and out[2] <= out[3] <= min(256, up(2 * tokens))
     assert lib.jb200_host_expert_tiles(961, 0, 1024, E, hidden, 148, out) == 0
+
+
+@pytest.mark.parametrize("sms", [8, 37, 59, 60, 132, 148, 160])
+def test_whoever_reads_maps_and_counts_finds_them_made_on_a_device_of_any_size(sms):
+    """161 to 512 tokens count the ids whatever the device; counts of every eight tokens need a router of a single pass (two CTAs of eight
+    tokens an SM); and the first expert matrix takes its segments from counts only where the router leaves them."""
+    lib, out = _lib.load(), (C.c_int32 * 2)()
+    ROUTER, EXPERT_GEMM, FROM_IDS, FROM_EIGHTS, METADATA = range(5)
+    for tokens in range(1, 3001):
+        for hidden in (2048, 8192):
+            assert lib.jb200_host_dispatch_plan(tokens, 1024, hidden, sms, out) == 1
+            maps, load = out
+            if tokens <= 160:
+                want = ROUTER if tokens <= (16 if hidden == 2048 else 0) else EXPERT_GEMM
+            else:
+                want = FROM_IDS if tokens <= 512 else FROM_EIGHTS if tokens <= min(16 * sms, 2368) else METADATA
+            assert maps == want and load == (maps in (FROM_IDS, FROM_EIGHTS)), (tokens, hidden)
+    assert lib.jb200_host_dispatch_plan(0, 1024, 2048, sms, out) == 0
