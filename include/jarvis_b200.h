@@ -464,8 +464,11 @@ void jb200_host_decode16(uint32_t word, uint32_t* out8);
 void jb200_host_decode16_prepared(uint32_t word, uint32_t* out8);
 /* Tiles that jb200_forward_layers gives the first or second expert matrix where it runs in the tcgen05 form for few tokens, on a device
  * with `sms` multiprocessors: out6 = whether every expert takes all tokens, out-features of a tile, rows of a token tile for experts
- * that are used evenly and at most, and the chunks (of two K-blocks) that either one's ring holds at least.  Runs on the CPU; used by the unit tests.  0: no such call. */
+ * that are used evenly and at most, and the chunks in either one's ring.  Runs on the CPU; used by the unit tests.  0: no such call. */
 int jb200_host_expert_tiles(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out6);
+/* That form's ring with token tiles of bn rows (a multiple of 16 up to 256) and K in-features, in chunks of two K-blocks or (coarse) four: out4 =
+ * chunks in flight, K-blocks of one, tensor-memory columns and bytes of shared memory that the CTA then uses.  As above.  0: no such ring. */
+int jb200_host_mid_ring(int bn, int K, int coarse, int32_t* out4);
 /* How jb200_forward_layers dispatches so many tokens on a device with `sms` multiprocessors: out2 = what makes the maps (0 the router, 1 the
  * first expert matrix, 2 the dispatch from the ids, 3 the dispatch from the router's counts of every eight tokens, 4 metadata kernels), and
  * whether the router leaves the experts' assignments, which the first expert matrix then takes as its segments in place of the maps' offsets.

@@ -97,6 +97,7 @@ PROTOTYPES = {
     "jb200_sample": (_I, [_P, _I, _I, _I, _I, _F, _I, _F, _P, _P, _P, _P]),
     "jb200_host_decode16": (None, [C.c_uint32, C.POINTER(C.c_uint32)]),
     "jb200_host_expert_tiles": (_I, [_I] * 6 + [C.POINTER(C.c_int32)]),
+    "jb200_host_mid_ring": (_I, [_I] * 3 + [C.POINTER(C.c_int32)]),
     "jb200_host_dispatch_plan": (_I, [_I] * 4 + [C.POINTER(C.c_int32)]),
     "jb200_ternary_linear_grouped": (_I, [_P, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _I, _P]),
 }

@@ -477,6 +477,7 @@ void jb200_host_decode16_prepared(uint32_t word, uint32_t* out8) { decode16_prep
 int jb200_host_expert_tiles(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out6) {
   return expert_tiles_host(tokens, second, C, E, hidden, sms, out6);
 }
+int jb200_host_mid_ring(int bn, int K, int coarse, int32_t* out4) { return mid_ring_host(bn, K, coarse, out4); }
 int jb200_host_dispatch_plan(int tokens, int C, int hidden, int sms, int32_t* out2) {
   return dispatch_plan_host(tokens, C, hidden, sms, out2);
 }

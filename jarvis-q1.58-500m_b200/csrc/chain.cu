@@ -117,6 +117,25 @@ inline MidTile expert_plan(int tokens, bool second, int C, int E, int hidden, in
   return mid_plan(cut ? 2 * tokens : tokens, E, second ? C : hidden, cut, second ? W2_TILES : W1_TILES, sms);
 }
 
+// Forms and tiles of a call's products.  Chunks of four K-blocks, where the rings of all products that run the same kernel hold them: each
+// finds its code in the instruction cache after the one before, two kernels in turn do not (900 tokens, the out-projection alone in chunks of
+// four: 1694 -> 1728 us).  Up to ALL_ROWS_TOKENS the expert matrices run kernels of their own.
+struct Products {
+  bool mid, mid_qkv, mid_out, coarse, w1_coarse, w2_coarse;
+  MidTile qkv, out, w1, w2;
+  Products(int N, bool small, int C, int E, int hidden, int sms)
+      : mid(!small && N <= MID_TOKENS), mid_qkv(mid || (!small && mid_wave(N, 3 * C, sms))), mid_out(mid || (!small && mid_wave(N, C, sms))),
+        qkv(mid_plan(N, 1, 3 * C, false, QKV_TILES, sms)), out(mid_plan(N, 1, C, false, OUT_TILES, sms)),
+        w1(expert_plan(N, false, C, E, hidden, sms)), w2(expert_plan(N, true, C, E, hidden, sms)) {
+    const bool all_rows = N <= ALL_ROWS_TOKENS;
+    w1_coarse = mid && mid_gemm_coarse_fits(w1.bn_max, C);
+    w2_coarse = mid && mid_gemm_coarse_fits(w2.bn_max, hidden);
+    coarse = (!mid_qkv || mid_gemm_coarse_fits(qkv.bn_max, C)) && (!mid_out || mid_gemm_coarse_fits(out.bn_max, C)) &&
+             (!mid || all_rows || (w1_coarse && w2_coarse));
+    if (!all_rows) w1_coarse = w2_coarse = coarse;
+  }
+};
+
 // What makes the dispatch maps of a call (counts, offsets, slots), and whether the router also leaves the assignments of every expert
 // (`load`), from which the first expert matrix takes its segments while maps and rows are made; without them it takes the maps' offsets.  Up
 // to ALL_ROWS_TOKENS there is no dispatch.  Beyond, maps and rows in one launch: from the ids on any device, or, where the router is a single
@@ -144,12 +163,21 @@ inline Dispatch dispatch_plan(int N, bool small, int sms) {
 
 int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out) {
   if (tokens < 1 || tokens > MID_TOKENS || C < 128 || E < 1 || hidden < 128 || sms < 1 || !out) return 0;
-  const MidTile t = expert_plan(tokens, second != 0, C, E, hidden, sms);
+  const Products g(tokens, false, C, E, hidden, sms);
+  const MidTile& t = second ? g.w2 : g.w1;
   const int K = second ? hidden : C;
+  const bool coarse = second ? g.w2_coarse : g.w1_coarse;
   out[0] = !second && tokens <= ALL_ROWS_TOKENS;
   out[1] = MID_FEATURES; out[2] = t.bn; out[3] = t.bn_max;
-  out[4] = mid_gemm_least_chunks(t.bn, K); out[5] = mid_gemm_least_chunks(t.bn_max, K);
+  out[4] = mid_gemm_ring(t.bn, K, coarse).chunks; out[5] = mid_gemm_ring(t.bn_max, K, coarse).chunks;
   return 1;
+}
+
+int mid_ring_host(int bn, int K, int coarse, int32_t* out) {
+  if (bn < 16 || bn > 256 || bn % 16 != 0 || K < 128 || !out) return 0;
+  const MidRing r = mid_gemm_ring(bn, K, coarse != 0);
+  out[0] = r.chunks; out[1] = r.kb; out[2] = r.tmem_cols; out[3] = r.smem;
+  return r.chunks >= 1;
 }
 
 int dispatch_plan_host(int tokens, int C, int hidden, int sms, int32_t* out) {
@@ -219,22 +247,15 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
   float* x = f->x;
   const int small_tile = N <= 8 ? 8 : 16;
   const bool small = small_form(N, C, hidden);                  // beyond, the tcgen05 form streams K
-  const bool mid = !small && N <= MID_TOKENS, all_rows = N <= ALL_ROWS_TOKENS;
+  const bool all_rows = N <= ALL_ROWS_TOKENS;
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
   const Dispatch by = dispatch_plan(N, small, sms);
-  const MidTile qkv_tile = mid_plan(N, 1, 3 * C, false, QKV_TILES, sms), out_tile = mid_plan(N, 1, C, false, OUT_TILES, sms);
-  const bool mid_qkv = mid || (!small && mid_wave(N, 3 * C, sms)), mid_out = mid || (!small && mid_wave(N, C, sms));
-  const MidTile w1_tile = expert_plan(N, false, C, E, hidden, sms), w2_tile = expert_plan(N, true, C, E, hidden, sms);
-  // Chunks of four K-blocks, where the rings of all products that run the same kernel hold them: each finds its code in the instruction
-  // cache after the one before, two kernels in turn do not (900 tokens, the out-projection alone in chunks of four: 1694 -> 1728 us).
-  const bool w1_coarse = mid && mid_gemm_coarse_fits(w1_tile.bn_max, C), w2_coarse = mid && mid_gemm_coarse_fits(w2_tile.bn_max, hidden);
-  const bool coarse = (!mid_qkv || mid_gemm_coarse_fits(qkv_tile.bn_max, C)) && (!mid_out || mid_gemm_coarse_fits(out_tile.bn_max, C)) &&
-                      (!mid || all_rows || (w1_coarse && w2_coarse));
-  auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G,
-                      const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epi, void* dst, const MidTile& t) {
-    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, counts, routes, epi, dst, t.bn, t.bn_max,
-                           all_rows && G > 1 ? (epi == JB200_EPI_GELU_BF16 ? w1_coarse : w2_coarse) : coarse, st);
+  const Products g(N, small, C, E, hidden, sms);
+  const bool mid = g.mid, mid_qkv = g.mid_qkv, mid_out = g.mid_out;
+  auto mid_gemm = [&](const void* in, int M, int K, const uint8_t* wt, const float* al, int al_rows, int n_out, int G, const int32_t* seg,
+                      const int32_t* counts, const MidRoutes* routes, int epi, void* dst, const MidTile& t, bool coarse) {
+    return launch_mid_gemm(in, M, K, wt, al, al_rows, n_out, G, seg, counts, routes, epi, dst, t.bn, t.bn_max, coarse, st);
   };
 
   // the accumulators and the router's work counters are one block: cleared by the first kernel
@@ -266,7 +287,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, small_tile, st));
     else if (mid_qkv)
-      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, qkv_tile));
+      JB_TRY(mid_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, nullptr, nullptr, JB200_EPI_BF16, qkv, g.qkv, g.coarse));
     else
       JB_TRY(launch_ternary_gemm(xn, N, C, p.w_qkv, p.a_qkv, C, 3 * C, 1, nullptr, JB200_EPI_BF16, qkv, 0, 1, st, nullptr, true));
     // a state updated in place needs one segment per sequence: later segments would read what the last one writes
@@ -277,7 +298,7 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
     if (small)
       JB_TRY(launch_small_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, small_tile, st));
     else if (mid_out)
-      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, out_tile));
+      JB_TRY(mid_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, nullptr, nullptr, JB200_EPI_RESID_F32, x, g.out, g.coarse));
     else
       JB_TRY(launch_ternary_gemm(o, N, C, p.w_out, p.a_out, C, C, 1, nullptr, JB200_EPI_RESID_F32, x, 0, 1, st, nullptr, true));
 
@@ -304,19 +325,19 @@ int forward_layers(const jb200_layer* layers, int n_layers, const jb200_forward*
       if (small)
         JB_TRY(launch_small_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, idx, scatter, JB200_EPI_GELU_BF16, hid, small_tile, st));
       else
-        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, nullptr, &store, JB200_EPI_GELU_BF16, hid, w1_tile));
+        JB_TRY(mid_gemm(xn, N, C, p.w1, p.a1, hidden, hidden, E, nullptr, nullptr, &store, JB200_EPI_GELU_BF16, hid, g.w1, g.w1_coarse));
     } else {
       if (by.maps != Dispatch::METADATA) JB_TRY(launch_dispatch_chain(idx, counts8, xn, N, C, E, counts, offs, scatter, gather, gate_idx, disp, st));
       else JB_TRY(launch_dispatch_gather(xn, gather, 2 * N, N, C, disp, st));
       if (mid)
-        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, by.load ? nullptr : offs, router_load, nullptr, JB200_EPI_GELU_BF16, hid, w1_tile));
+        JB_TRY(mid_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, by.load ? nullptr : offs, router_load, nullptr, JB200_EPI_GELU_BF16, hid, g.w1, g.w1_coarse));
       else
         JB_TRY(launch_ternary_gemm(disp, 2 * N, C, p.w1, p.a1, hidden, hidden, E, offs, JB200_EPI_GELU_BF16, hid, 0, 1, st, nullptr, true, router_load));
     }
     if (small)
       JB_TRY(launch_small_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, nullptr, nullptr, JB200_EPI_BF16, y, small_tile, st));
     else if (mid)
-      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, late_maps ? nullptr : offs, nullptr, late_maps ? &rows_of : nullptr, JB200_EPI_BF16, y, w2_tile));
+      JB_TRY(mid_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, late_maps ? nullptr : offs, nullptr, late_maps ? &rows_of : nullptr, JB200_EPI_BF16, y, g.w2, g.w2_coarse));
     else
       JB_TRY(launch_ternary_gemm(hid, 2 * N, hidden, p.w2, p.a2, C, C, E, offs, JB200_EPI_BF16, y, 0, 1, st, nullptr, true));
 

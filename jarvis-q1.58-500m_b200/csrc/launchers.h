@@ -51,8 +51,11 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
                     const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
                     bool coarse, cudaStream_t stream);
 constexpr int MID_FEATURES = 128;              // out-features of its tiles
+struct MidRing {
+  int chunks, kb, tmem_cols, smem;             // chunks in flight, K-blocks of one, tensor-memory columns and shared memory in use
+};
+MidRing mid_gemm_ring(int bn, int K, bool coarse);      // its ring with token tiles of bn rows; no chunks where K is not a multiple of one
 bool mid_gemm_coarse_fits(int bn, int K);      // `coarse`, chunks of four K-blocks in place of two: where its ring still holds three
-int mid_gemm_least_chunks(int bn, int K);      // what its ring holds at least with token tiles of bn, in chunks of two K-blocks
 int launch_prepare_weights(const uint8_t* packed, size_t n_bytes, uint8_t* prepared, cudaStream_t stream);
 void decode16_host(uint32_t w, uint32_t* out8);
 void decode16_prepared_host(uint32_t w_canonical, uint32_t* out8);
@@ -156,6 +159,7 @@ int launch_step_cluster(const jb200_layer* layers, int n_layers, const jb200_for
                         cudaStream_t stream, bool* taken);
 int launch_cross_entropy(const void* logits, int ld, int n_rows, int V, const int64_t* targets, float* row_loss,
                          const float* aux_a, int stride_a, const float* aux_b, int n_aux, float* loss, cudaStream_t stream);
+int mid_ring_host(int bn, int K, int coarse, int32_t* out);
 int dispatch_plan_host(int tokens, int C, int hidden, int sms, int32_t* out);
 int expert_tiles_host(int tokens, int second, int C, int E, int hidden, int sms, int32_t* out);
 size_t accumulator_bytes(int E);

@@ -481,20 +481,23 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
 constexpr int RING_SMEM = 222 * 1024, RING_LEAST = 3;
 inline int chunk_bytes(int bn, int ck) { return ck * bn * BK * 2; }
 inline int code_boxes(int K) { return std::min((K + BOX_KB * BK - 1) / (BOX_KB * BK), MAX_BOXES); }
-// Chunks in flight: weights in what the accumulator leaves of tensor memory, rows in what the codes leave of shared memory.
-inline int ring_chunks(int bn, int ck, int K) {
-  return std::min({(int(TMEM_COLS) - acc_cols(bn)) / int(ck * KB_COLS), (RING_SMEM - code_boxes(K) * BOX_BYTES) / chunk_bytes(bn, ck),
-                   MAX_CHUNKS, K / (BK * ck)});
-}
 constexpr size_t LEAST_SMEM = 116 * 1024;      // two CTAs of an SM would only wait for each other's tensor memory
 
 }  // namespace
 
-bool mid_gemm_coarse_fits(int bn, int K) { return K % (BK * CK_MOST) == 0 && ring_chunks(bn, CK_MOST, K) >= RING_LEAST; }
-
-int mid_gemm_least_chunks(int bn, int K) {
-  return std::min({(224 * 1024) / (chunk_bytes(MID_FEATURES, 2) + chunk_bytes(bn, 2)), MAX_CHUNKS, K / (BK * 2)});
+// Chunks in flight: weights in what the accumulator leaves of tensor memory, rows in what the codes leave of shared memory.
+MidRing mid_gemm_ring(int bn, int K, bool coarse) {
+  const int ck = coarse ? CK_MOST : 2;
+  MidRing r = {0, ck, 0, 0};
+  if (K % (BK * ck) != 0) return r;
+  r.chunks = std::min({(int(TMEM_COLS) - acc_cols(bn)) / int(ck * KB_COLS), (RING_SMEM - code_boxes(K) * BOX_BYTES) / chunk_bytes(bn, ck),
+                       MAX_CHUNKS, K / (BK * ck)});
+  r.tmem_cols = acc_cols(bn) + r.chunks * ck * int(KB_COLS);
+  r.smem = code_boxes(K) * BOX_BYTES + r.chunks * chunk_bytes(bn, ck) + 1024;       // the base is rounded up to 1024
+  return r;
 }
+
+bool mid_gemm_coarse_fits(int bn, int K) { return mid_gemm_ring(bn, K, true).chunks >= RING_LEAST; }
 
 int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared, const float* alpha, int alpha_rows, int N, int G,
                     const int32_t* seg, const int32_t* counts, const MidRoutes* routes, int epilogue, void* out, int bn, int bn_max,
@@ -513,15 +516,18 @@ int launch_mid_gemm(const void* x_bf16, int M, int K, const uint8_t* w_prepared,
   p.boxes = code_boxes(K);
   p.status = device_status_ptr();
   if (!p.status) return JB200_ERR_CUDA;
-  const int n_kb = K / BK, ck = coarse ? CK_MOST : 2;
+  const int n_kb = K / BK;
+  int ck = 2;
   Maps maps;                                   // [K-block][token][64]: one copy takes the same rows of ck K-blocks
   const cuuint64_t gdim[3] = {cuuint64_t(BK), cuuint64_t(M), cuuint64_t(n_kb)};
   const cuuint64_t gstride[2] = {cuuint64_t(K) * 2, cuuint64_t(BK) * 2};
   size_t smem = LEAST_SMEM;
   for (int i = 0; i < 3; ++i) {
     p.bn[i] = i == 0 ? bn : i == 1 ? (bn + bn_max) / 32 * 16 : bn_max;
-    p.chunks[i] = ring_chunks(p.bn[i], ck, K);
-    smem = std::max(smem, size_t(p.boxes) * BOX_BYTES + size_t(p.chunks[i]) * chunk_bytes(p.bn[i], ck) + 1024);
+    const MidRing ring = mid_gemm_ring(p.bn[i], K, coarse);
+    ck = ring.kb;
+    p.chunks[i] = ring.chunks;
+    smem = std::max(smem, size_t(ring.smem));
     if (i > 0 && p.bn[i] == p.bn[i - 1]) {
       maps.x[i] = maps.x[i - 1];
       continue;

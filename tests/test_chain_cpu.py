@@ -299,23 +299,48 @@ def test_an_edited_layer_alone_is_laid_out_again(step_library):
 @pytest.mark.parametrize("hidden", [1024, 2048, 4096])
 def test_expert_tiles_are_no_larger_than_their_rows(E, hidden):
     """However many tiles the experts need, a token tile ends with the rows there are: the smallest that leaves the launch on half of the
-    SMs (all rows for every expert) or on all of them, else one for all rows."""
-    lib, out = _lib.load(), (C.c_int32 * 6)()
+    SMs (all rows for every expert) or on all of them, else one for all rows.  Its ring is one that the kernel has, in chunks of four
+    K-blocks or of two."""
+    lib, out, of = _lib.load(), (C.c_int32 * 6)(), (C.c_int32 * 4)()
+    rings = lambda tile, K: [of[0] for coarse in (0, 1) if lib.jb200_host_mid_ring(tile, K, coarse, of)]
     up = lambda n: (n + 15) // 16 * 16
     for tokens in range(1, 961):
         assert lib.jb200_host_expert_tiles(tokens, 0, 1024, E, hidden, 148, out) == 1
         all_rows, bm, bn, bn_max, ring, ring_max = out
         rows = tokens if all_rows else -(-2 * tokens // E)
         assert all_rows == (tokens <= 160) and bn <= bn_max <= min(256, up(2 * tokens)) and ring >= ring_max >= 2
+        assert ring in rings(bn, 1024) and ring_max in rings(bn_max, 1024)
         if all_rows:
             tiles = lambda n: hidden // bm * E * -(-tokens // n)
-            assert bn == bn_max <= up(tokens) and ring == min(8, 224 * 1024 // (256 * (bm + bn)))
+            assert bn == bn_max <= up(tokens)
             assert tiles(bn) <= 74 or bn == up(tokens)
             assert bn <= 64 or tiles(bn - 16) > 74
         else:
             assert bn <= up(rows + -(-rows // 8))
         assert lib.jb200_host_expert_tiles(tokens, 1, 1024, E, hidden, 148, out) == 1 and out[2] <= out[3] <= min(256, up(2 * tokens))
+        assert out[4] in rings(out[2], hidden) and out[5] in rings(out[3], hidden)
     assert lib.jb200_host_expert_tiles(961, 0, 1024, E, hidden, 148, out) == 0
+
+
+@pytest.mark.parametrize("K", [128, 256, 384, 1024, 1152, 2048, 8192])
+def test_the_ring_of_the_latency_gemm_fits_its_memories(K):
+    """Accumulator (f32, bn columns in steps of 64) and weights (32 columns a K-block of 64) in the 512 columns of tensor memory; codes (boxes of
+    128 rows x 512 in-features, at most four) and rows (bf16) in 227 KB; never more chunks than K has or the kernel has barriers for."""
+    lib, out = _lib.load(), (C.c_int32 * 4)()
+    for bn in range(16, 257, 16):
+        for coarse in (0, 1):
+            kb = 4 if coarse else 2
+            ok = lib.jb200_host_mid_ring(bn, K, coarse, out)
+            if K % (64 * kb):
+                assert not ok
+                continue
+            boxes, acc, rows = 16384 * min(-(-K // 512), 4), -(-bn // 64) * 64, 128 * bn * kb
+            assert out[1] == kb and out[2] == acc + out[0] * kb * 32 <= 512
+            assert out[3] == boxes + out[0] * rows + 1024 <= 223 * 1024       # beside them control words and the epilogue's row lists, 3 KB
+            assert out[0] <= min(8, K // (64 * kb))
+            # and no chunk is left out that all of them would hold
+            assert out[0] == min(8, K // (64 * kb)) or out[2] + kb * 32 > 512 or out[3] + rows > 223 * 1024
+            assert ok == (out[0] >= 1) and (coarse or out[0] >= min(2, K // 128))
 
 
 @pytest.mark.parametrize("sms", [8, 37, 59, 60, 132, 148, 160])
