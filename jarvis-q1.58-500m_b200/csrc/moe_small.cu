@@ -186,9 +186,16 @@ struct TailShared {
 };
 struct Decay {
   float alpha, mean, var;
+  bool got;                    // false: this warp has given up waiting for the other CTAs
 };
-__device__ __noinline__ void tail_wait_long(uint32_t bar, volatile uint32_t* abort_flag, unsigned int* status) {
-  (void)mbar_wait(bar, 0u, abort_flag, status, JB200_STATUS_LSF_LOAD);
+__device__ __noinline__ bool tail_wait_long(uint32_t bar, volatile uint32_t* abort_flag, unsigned int* status) {
+  return mbar_wait(bar, 0u, abort_flag, status, JB200_STATUS_LSF_LOAD);
+}
+// A CTA may leave when what the others send it has landed.  Behind a cluster barrier (threads that have left count as arrived) all of it is
+// on its way.
+__device__ __noinline__ void tail_landed(uint32_t bar) {
+  for (int i = 0; i < 1000; ++i)
+    if (mbar_try_wait_parked(bar, 0u, 20000u)) return;
 }
 // Ahead of everything else; the CTAs of a cluster have all done it behind the cluster_wait() of tail_decay.
 __device__ __forceinline__ void tail_begin(TailShared& s, int n_cta, uint32_t row_bytes) {
@@ -227,16 +234,17 @@ __device__ __forceinline__ Decay tail_decay(const TailParams& p, Combined c, flo
                  make_uint4(uint32_t(__double2loint(a)), uint32_t(__double2hiint(a)), uint32_t(__double2loint(b)), uint32_t(__double2hiint(b))));
     }
   }
+  bool got = true;
   if (n_cta == 1) __syncthreads();
-  else if (!mbar_try_wait(smem_u32(&s.bar), 0u)) tail_wait_long(smem_u32(&s.bar), &s.abort_flag, p.status);
-  __syncwarp();
+  else if (!mbar_try_wait(smem_u32(&s.bar), 0u)) got = tail_wait_long(smem_u32(&s.bar), &s.abort_flag, p.status);
+  got = __all_sync(0xffffffffu, got);
   double sum = lane < n_cta ? s.all[lane][0] : 0.0, sq = lane < n_cta ? s.all[lane][1] : 0.0;
   for (int o = n_cta > 8 ? 8 : 4; o > 0; o >>= 1) {
     sum += __shfl_xor_sync(0xffffffffu, sum, o);
     sq += __shfl_xor_sync(0xffffffffu, sq, o);
   }
   const float2 mv = moe_act_mean_var(__shfl_sync(0xffffffffu, sum, 0), __shfl_sync(0xffffffffu, sq, 0), p.st.n_el, p.st.inv_el, p.st.inv_el1);
-  return {lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, mv.y), mv.x, mv.y};
+  return {lsf_alpha_from_var(p.alpha_min, p.alpha_max, var_scale, mv.y), mv.x, mv.y, got};
 }
 // The norm's weight, on its way while the kernel ahead runs (what a thread has read into L1 by then is gone behind the grid dependency: read
 // from global memory at the end, the weight took 1.9 us).
@@ -297,6 +305,11 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_step_kernel(const TailPar
   Combined c = {0.f, 0.f};
   if (on) c = combine_row(p, sl.x, sl.y, g, lane, [&](int i, uint4 v) { m[i] = v; });
   const Decay d = tail_decay(p, c, var_scale, sh, rank, n_cta, [] {});
+  if (!d.got) {                // 2 s late: nobody sends anything behind this
+    cluster_arrive();
+    cluster_wait();
+    tail_landed(smem_u32(&sh.bar));
+  }
   const float alpha = d.alpha;
   if (rank == 0 && tid == int(blockDim.x) - 1) tail_scalars(p, l_bal, mu, d);
   if (!on) return;
@@ -473,6 +486,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) tail_scan_kernel(const TailPar
   __syncwarp();
   cluster_arrive();
   cluster_wait();
+  if (!d.got) tail_landed(smem_u32(&sh.bar));
   if (!p.w_norm || !on) return;
 
   // ---- the norm of the warp's token ----
