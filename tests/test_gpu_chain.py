@@ -616,3 +616,17 @@ def test_chain_where_maps_and_rows_come_from_the_ids(C, E, N):
 def test_chain_where_the_attention_products_leave_the_latency_form(B, T):
     """One wave of tiles of 256 rows: q|k|v up to 1536 tokens, the out-projection up to 4608 (148 SMs)."""
     _chain_against_kernels(1024, 4, 2, B, T)
+
+
+@pytest.mark.parametrize("B,T,C", [(2, 300, 1024), (3, 234, 1024), (2, 481, 1024), (3, 500, 128), (5, 473, 1024), (5, 474, 1024)])
+def test_a_token_whose_router_is_nan_where_the_router_leaves_counts_of_eight(B, T, C):
+    """513 to 2368 tokens, and just beyond: the router's counts, the ranks of the dispatch and the segments of the first expert matrix (the
+    latency form's up to 960, the pair form's beyond) agree on where an assignment without an expert goes."""
+    test_both_assignments_of_a_token_whose_router_is_nan_run(B, T, C)
+
+
+@pytest.mark.parametrize("skew", [0.5, 4.0])
+@pytest.mark.parametrize("T", [513, 961, 1500, 2048])
+def test_chain_with_uneven_experts_whose_segments_are_counted_by_the_router(T, skew):
+    """Very long segments and empty ones, from counts, in the latency form and in the pair form."""
+    test_chain_with_uneven_experts(T, skew)
