@@ -776,7 +776,9 @@ int launch_dispatch_chain(const int64_t* topk_idx, const unsigned long long* cou
   JB_REQUIRE(aligned16(topk_idx) && aligned16(x_bf16) && aligned16(dispatched), "dispatch_chain: pointers must be 16-byte aligned");
   static_assert(DISPATCH_IDS_MAX / DISP_THREADS * 2 < 256 && (DISPATCH_EIGHTS_MAX / 8 + DISP_THREADS - 1) / DISP_THREADS * 16 < 256,
                 "a byte per expert and thread");
-  const bool few = n_tokens <= 8 * 148;                    // a wave of CTAs, as small as they go
+  const int sms = sm_count();
+  if (sms <= 0) return JB200_ERR_CUDA;
+  const bool few = n_tokens <= 8 * sms;                    // a wave of CTAs, as small as they go
   auto kernel = counts8 ? (few ? (E == 4 ? dispatch_kernel<4, 8, EIGHTS> : dispatch_kernel<8, 8, EIGHTS>)
                                : (E == 4 ? dispatch_kernel<4, 16, EIGHTS> : dispatch_kernel<8, 16, EIGHTS>))
                         : (E == 4 ? dispatch_kernel<4, 8, IDS> : dispatch_kernel<8, 8, IDS>);
