@@ -92,14 +92,21 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
                       int64_t* __restrict__ topk_idx, float* __restrict__ gates,
                       double* __restrict__ probs_sum, int* __restrict__ top1_hist, int* __restrict__ load,
                       unsigned long long* __restrict__ counts8, bool ahead) {
-  extern __shared__ float w_s[];  // [E][C], [C]
+  extern __shared__ __align__(16) float w_s[];  // [E][C], [C]
   __shared__ float p_acc[ROUTER_THREADS / 32][E];
-  __shared__ int h_acc[E], l_acc[E];
+  __shared__ int h_acc[E], l_acc[PER == 1 ? E : 1];           // (the assignments of every expert are counted in a single pass alone)
   auto stage = [&] {
+    // the norm's weight, four values a thread, travels with the router's rows (behind them it was a round trip more, 0.5 us)
+    const int n4 = 4 * threadIdx.x;
+    const float4 wn = n4 < C ? __ldg(reinterpret_cast<const float4*>(w_norm + n4)) : make_float4(0.f, 0.f, 0.f, 0.f);
     for (int i = threadIdx.x; i < E * C; i += ROUTER_THREADS) w_s[(i / C) * C + router_w_index(i % C)] = __ldg(w_router + i);
-    for (int i = threadIdx.x; i < C; i += ROUTER_THREADS) w_s[E * C + i] = __ldg(w_norm + i);
+    if (n4 < C) *reinterpret_cast<float4*>(w_s + E * C + n4) = wn;
   };
-  if (threadIdx.x < E) h_acc[threadIdx.x] = l_acc[threadIdx.x] = 0;
+  static_assert(4 * ROUTER_THREADS >= 1024, "d_model is at most 1024");
+  if (threadIdx.x < E) {
+    h_acc[threadIdx.x] = 0;
+    if (PER == 1) l_acc[threadIdx.x] = 0;
+  }
   if (ahead) stage();
   pdl_wait();
   pdl_trigger();
@@ -112,19 +119,23 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
   // A warp takes PER tokens per pass: with two, their loads are in flight together, the two dependency chains interleave,
   // and the router weights read from shared memory serve both.  The CTAs are persistent (two per SM) and stride
   // over the tokens, so the router matrix is staged once per CTA.  Where one token a warp is a single pass, it is over sooner (24
-  // layers and head, 600, 900, 1300 tokens 1667 -> 1637, 1848 -> 1803, 2511 -> 2480 us).
+  // layers and head, 600, 900, 1300 tokens 1667 -> 1637, 1848 -> 1803, 2511 -> 2480 us).  By itself, d_model 1024 and four experts, with the norm's
+  // weight staged too and rows loaded side by side: 300, 1184, 2368, 9000, 16,384 tokens 5.4 -> 4.15, 5.5 -> 4.4, 5.7 -> 5.4, 12.4 -> 11.9, 24.4 -> 23.4 us (two a
+  // warp and weights from L1 before); 128 channels +2 to +4 % from 1185 tokens on.
   const int n_items = (n_tokens + PER - 1) / PER;
   for (int item = blockIdx.x * (ROUTER_THREADS / 32) + warp; item < n_items; item += gridDim.x * (ROUTER_THREADS / 32)) {
     const int tok = PER * item;
     float v[PER][4][8], ss[PER], r[PER], acc[PER][E];
+    const float* xr[PER];                                       // a lone last token is processed twice, stored once
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const float* xr = x + size_t(min(tok + k, n_tokens - 1)) * C;     // a lone last token is processed twice, stored once
+    for (int k = 0; k < PER; ++k) xr[k] = x + size_t(tok + k < n_tokens ? tok + k : tok) * C;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int c = (i * 32 + lane) * 8;
-        if (c < C) {
-          const float4 a = __ldg(reinterpret_cast<const float4*>(xr + c)), b = __ldg(reinterpret_cast<const float4*>(xr + c) + 1);
+    for (int i = 0; i < 4; ++i) {
+      const int c = (i * 32 + lane) * 8;
+      if (c < C) {
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const float4 a = __ldg(reinterpret_cast<const float4*>(xr[k] + c)), b = __ldg(reinterpret_cast<const float4*>(xr[k] + c) + 1);
           v[k][i][0] = a.x; v[k][i][1] = a.y; v[k][i][2] = a.z; v[k][i][3] = a.w;
           v[k][i][4] = b.x; v[k][i][5] = b.y; v[k][i][6] = b.z; v[k][i][7] = b.w;
         }
@@ -173,7 +184,7 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
     }
 #pragma unroll
     for (int k = 0; k < PER; ++k)
-      if (k == 0 || tok + k < n_tokens) router_finish<E>(acc[k], lane, tok + k, topk_idx, gates, nullptr, h_acc, p_local, load ? l_acc : nullptr);
+      if (k == 0 || tok + k < n_tokens) router_finish<E>(acc[k], lane, tok + k, topk_idx, gates, nullptr, h_acc, p_local, PER == 1 && load ? l_acc : nullptr);
   }
   if (lane == 0) {
 #pragma unroll
@@ -185,7 +196,7 @@ rmsnorm_router_kernel(const float* __restrict__ x, const float* __restrict__ w_n
     for (int w = 0; w < ROUTER_THREADS / 32; ++w) s += p_acc[w][threadIdx.x];
     if (probs_sum) atomicAdd(&probs_sum[threadIdx.x], double(s));
     if (top1_hist && h_acc[threadIdx.x]) atomicAdd(&top1_hist[threadIdx.x], h_acc[threadIdx.x]);
-    if (load && l_acc[threadIdx.x]) atomicAdd(&load[threadIdx.x], l_acc[threadIdx.x]);
+    if (PER == 1 && load && l_acc[threadIdx.x]) atomicAdd(&load[threadIdx.x], l_acc[threadIdx.x]);
   }
   if (PER == 1 && counts8 && threadIdx.x == 32) {          // single pass: the CTA's eight tokens, a byte per expert
     unsigned long long c = 0;
@@ -698,12 +709,14 @@ int launch_rmsnorm_router(const float* x, const float* w_norm, float eps, void* 
   JB_REQUIRE(aligned16(x) && aligned16(w_norm) && aligned16(xn_bf16) && aligned16(w_router),
              "rmsnorm_router: pointers must be 16-byte aligned");
   if (n_tokens == 0) return JB200_OK;
-  // persistent CTAs, two per SM, striding over the tokens: two per warp and pass, or one where that leaves a single pass
+  // persistent CTAs, two per SM, striding over the tokens: two per warp and pass, or one where that leaves a single pass.  By itself only
+  // while that is one CTA an SM (d_model 1024, four experts, 1184 and 2368 tokens: 4.4 and 5.95 us with one, 5.4 and 5.4 with two); with counts of
+  // eight tokens up to two, for what they save behind it.
   const int sms = sm_count();
   if (sms <= 0) return JB200_ERR_CUDA;
-  const int warps = ROUTER_THREADS / 32, per = n_tokens <= 2 * sms * warps ? 1 : 2;
+  const int warps = ROUTER_THREADS / 32, per = n_tokens <= (counts8 ? 2 : 1) * sms * warps ? 1 : 2;
   const int blocks = std::min((n_tokens + per * warps - 1) / (per * warps), 2 * sms);
-  JB_REQUIRE(!counts8 || (per == 1 && load), "rmsnorm_router: counts of eight tokens need a single pass");
+  JB_REQUIRE((!counts8 && !load) || (counts8 && load && per == 1), "rmsnorm_router: counts need a single pass");
   const size_t smem = size_t(E + 1) * C * sizeof(float);      // the router's rows and the norm's
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(xn_bf16);
   auto kernel = per == 1 ? (E == 4 ? rmsnorm_router_kernel<4, 1> : rmsnorm_router_kernel<8, 1>)

@@ -286,6 +286,23 @@ def test_fused_rmsnorm_router_is_bit_identical_to_the_two_kernels():
         assert torch.equal(h1, h2) and torch.allclose(ps1, ps2, rtol=1e-6)
 
 
+@pytest.mark.parametrize("E,C", [(4, 8), (8, 128), (4, 776), (8, 1024)])
+@pytest.mark.parametrize("N", [1184, 1185, 2368, 2369])
+def test_fused_rmsnorm_router_where_a_warp_begins_to_take_two_tokens(N, E, C):
+    """148 SMs: one token a warp in one CTA an SM, two beyond; even and odd numbers; rows of less than a warp's eight values a lane and of all."""
+    g = torch.Generator().manual_seed(N + C)
+    x, wn = torch.randn(N, C, generator=g).cuda() * 3, (torch.rand(C, generator=g) + 0.5).cuda()
+    wr = (torch.randn(E, C, generator=g) * 0.05).cuda()
+    x[7] = float("nan")
+    hist = torch.zeros(E, dtype=torch.int32, device="cuda")
+    xn1 = ops.rmsnorm(x, wn, 1e-6)
+    idx1, gates1, _ = ops.router_top2(xn1, wr)
+    xn2, idx2, gates2 = ops.rmsnorm_router(x, wn, 1e-6, wr, top1_hist=hist)
+    assert torch.equal(xn1.view(torch.int16), xn2.view(torch.int16)) and torch.equal(idx1, idx2)
+    assert torch.equal(gates1.view(torch.int32), gates2.view(torch.int32))
+    assert torch.equal(hist, torch.bincount(idx1[:, 0].clamp_min(0), minlength=E).int())
+
+
 def test_router_ties_go_to_lower_expert():
     x = torch.zeros(64, 256, dtype=torch.bfloat16)
     w = torch.randn(4, 256)
