@@ -54,7 +54,7 @@ int set_dependent_launch(int on);
 bool dependent_launch_enabled();  // programmatic dependent launch of the library's kernels (jb200_set_dependent_launch)
 
 // Tensor maps are pure functions of their arguments, and a forward encodes the same ones for every layer (~0.4 us of
-// host time each, ten per layer): the last few dozen of a thread are kept and compared by value.  dims / box: `rank`
+// host time each, ten per layer): a forward's worth of them is kept per thread and compared by value.  dims / box: `rank`
 // entries, innermost first; strides: rank - 1 entries in bytes.  `what` names the caller in error messages.
 int encode_tiled(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const void* ptr, const cuuint64_t* dims,
                  const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle,

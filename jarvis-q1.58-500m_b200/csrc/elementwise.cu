@@ -1,6 +1,8 @@
 // Row-wise glue kernels of the block: RMSNorm (jarvis_engine/jarvis_model.py:25-26) and the
 // token-embedding gather (nn.Embedding at jarvis_model.py:452, 498).  Both are pure HBM
 // streaming: one warp per row, 16-byte accesses.
+#include <type_traits>
+
 #include "common.cuh"
 #include "launchers.h"
 
@@ -43,19 +45,20 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* p, const fl
 template <typename TIn, typename TOut, int MAXV, bool AHEAD>
 __global__ void __launch_bounds__(ROW_THREADS) rmsnorm_kernel(const TIn* __restrict__ x, const float* __restrict__ w,
                                                               float eps, TOut* __restrict__ y, int n_rows, int C) {
-  const int row = blockIdx.x * (ROW_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   float wk[AHEAD ? MAXV : 1][8];
   if constexpr (AHEAD) {
 #pragma unroll
     for (int i = 0; i < MAXV; ++i)
       if ((i * 32 + lane) * 8 < C) load8<float>(w + (i * 32 + lane) * 8, wk[i]);
+    __syncwarp();
+    // In a chain before the wait: q|k|v comes next, which reads weights alone ahead of its own, and this kernel is shorter than their decoding
+    // (24 layers and head, 200, 256, 900 tokens, 3 x 777: 988 -> 968, 1021 -> 998, 1688 -> 1675, 2806 -> 2778 us).
+    pdl_trigger();
   }
-  __syncwarp();
-  // In a chain before the wait: q|k|v comes next, which reads weights alone ahead of its own, and this kernel is shorter than their decoding
-  // (24 layers and head, 200, 256, 900 tokens, 3 x 777: 988 -> 968, 1021 -> 998, 1688 -> 1675, 2806 -> 2778 us).
-  if (AHEAD) pdl_trigger();
   pdl_wait();
   if (!AHEAD) pdl_trigger();
+  const int row = blockIdx.x * (ROW_THREADS / 32) + (threadIdx.x >> 5);
   if (row >= n_rows) return;
   const TIn* xr = x + size_t(row) * C;
   TOut* yr = y + size_t(row) * C;
@@ -104,8 +107,9 @@ template <typename TIn, typename TOut>
 int launch_rmsnorm_t(const void* x, const float* w, float eps, void* y, int n_rows, int C, bool ahead, cudaStream_t stream) {
   const int blocks = (n_rows + ROW_THREADS / 32 - 1) / (ROW_THREADS / 32);
   // (beyond a wave of CTAs the registers are better spent on more of them)
-  auto kernel = C > 1024 ? rmsnorm_kernel<TIn, TOut, 16, false>
-                         : ahead && n_rows <= 4096 ? rmsnorm_kernel<TIn, TOut, 4, true> : rmsnorm_kernel<TIn, TOut, 4, false>;
+  auto kernel = C > 1024 ? rmsnorm_kernel<TIn, TOut, 16, false> : rmsnorm_kernel<TIn, TOut, 4, false>;
+  if constexpr (std::is_same_v<TIn, float> && std::is_same_v<TOut, __nv_bfloat16>)       // what a chain has
+    if (ahead && C <= 1024 && n_rows <= 4096) kernel = rmsnorm_kernel<TIn, TOut, 4, true>;
   launch_dep(kernel, blocks, ROW_THREADS, 0, stream, reinterpret_cast<const TIn*>(x), w, eps, reinterpret_cast<TOut*>(y), n_rows, C);
   JB_LAUNCH_CHECK("rmsnorm_kernel");
   return JB200_OK;

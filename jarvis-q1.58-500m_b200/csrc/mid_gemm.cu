@@ -9,7 +9,8 @@
 //     stage there is before the grid dependency is waited for;
 //   - the weights are the MMA's A operand in TENSOR memory: a K = 16 step of N tokens takes 10 + N / 2 cycles, where 128 rows read from
 //     shared memory cost 43 + N / 2 and 64 rows 27 + N / 2 (48 tokens: 34 against 67 and 51).  What the accumulator leaves of the
-//     512 columns holds twelve to fourteen K-blocks, so of K = 1024 nearly all is decoded ahead, when no MMA is in the way of the stores;
+//     512 columns and the rows of shared memory hold fourteen K-blocks of up to 64 rows, of 128, 160 and 256 rows (K = 1024) ten, eight and
+//     four (mid_gemm_ring): of K = 1024 and small tiles nearly all is decoded ahead, when no MMA is in the way of the stores;
 //   - K-blocks travel in chunks of CK: one TMA copy, one barrier wait and one commit per chunk (~290, ~85 and ~45 cycles,
 //     none of which hides behind MMAs: issuing them takes as long as they do), with as many chunks in flight as fit: four K-blocks a
 //     chunk where three of them do, else two (24 layers and head with two -> four: 17, 37, 64, 128, 256 tokens 677 -> 654, 697 -> 675,
@@ -17,8 +18,9 @@
 //   - codes come by TMA, all at once up to K = 2048, in rows of 128 bytes;
 //   - the eight decoder warps become the epilogue; the residual is added by reductions, nothing waits for old values.  Weight
 //     rows are dealt to lanes so that a thread finds four neighbouring out-features of a token: 8- and 16-byte stores, no shuffles.
-// With weights in shared memory, in tiles of 64 or 128 out-features, and codes in registers 24 layers and head as a graph took 881 us at
-// 37 tokens (now 779), 1096 at 128 (904), 1360 at 256 (1181), 2068 at 900 (1849), steps of 64 and 256 sequences 958 (878) and 1699 (1533).
+// Weights from shared memory, in tiles of 64 or 128 out-features and with codes in registers -> in tensor memory, in chunks of two, and
+// nothing else changed: 24 layers and head as a graph 881 -> 779 us at 37 tokens, 1096 -> 904 at 128, 1360 -> 1181 at 256, 2068 -> 1849 at 900, steps
+// of 64 and 256 sequences 958 -> 878 and 1699 -> 1533.  (The chunks of four above were measured after router, dispatch and tails had become shorter.)
 // What is left: the first copy's way (0.5 us after the dependency), 0.17-0.2 us for two K-blocks, epilogue and the end of the grid (0.6 and
 // 0.6-0.9 us), and where the kernel ahead is short, decoding (0.14 us a K-block).  Not kept: sixteen decoder warps (180 to 512 tokens 2-3 %
 // slower: their registers are not free while the kernel ahead runs), one look at all barriers in place of a wait each, commits left out, a pass
@@ -99,7 +101,6 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
         "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // 16 lanes x 16 columns: thread (g, c) of 8 x 4 receives of lanes g (v[4j], v[4j + 1]) and g + 8 (v[4j + 2], v[4j + 3]) the columns
 // 8j + 2c and 8j + 2c + 1.
 __device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
@@ -447,7 +448,7 @@ mid_gemm_kernel(const __grid_constant__ Maps maps, const MidParams p) {
             f32x2_split(lo, x0, x1);
             f32x2_split(hi, x2, x3);
             const bool sw = turn & 1;
-            if (row >= 0)
+            if (row >= 0)          // (addends and sums below 2^-126 become zero, as in small_gemm.cu; TMA's reduction keeps them)
               asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
                            ::"l"(reinterpret_cast<float*>(p.out) + size_t(row) * p.N + feat), "f"(sw ? x1 : x0), "f"(sw ? x0 : x1),
                              "f"(sw ? x3 : x2), "f"(sw ? x2 : x3) : "memory");
