@@ -21,7 +21,10 @@
 // beyond, an expert belongs to four CTAs, which exchange its hidden rows among themselves.
 // Measured (24 layers and the vocabulary head, replayed as a graph, kernel by kernel -> here): 1 sequence 621 -> 494 us, 2 675 -> 517,
 // 4 710 -> 504, 7 715 -> 511, 8 718 -> 630, 16 810 -> 655, 32 937 -> 751, 56 1049 -> 928.  With more tokens a cluster the form
-// loses: every cluster decodes all weights for itself, and shared memory holds eight.
+// loses: every cluster decodes all weights for itself, and shared memory holds eight.  The kernels have become faster since, those for more than
+// sixteen tokens above all: kernel by kernel 1 sequence 572, 2 609, 4 643, 8 657, 12 711, 16 769, 17 602, 20 609, 24 612, 32 637, 40 663, 48 684, 56 713 us, here
+// 492, 508, 503, 633, 633, 656, 657, 662, 690, 743, 788, 844, 927.  So from 17 sequences on the kernels would be the faster form; the line below has not been
+// drawn again.
 // Every value is rounded and every f32 sum ordered as in the kernels this one stands for.  The f64 sums over tokens behind mean and
 // variance, and those of the router's probabilities, are added in another order and rounded to f32 after that: the tests find the
 // results equal bit for bit, and a last bit of those scalars is what could differ.
